@@ -226,3 +226,31 @@ def tolerance(case):
     if case["rows"] > 512 and case["mode"] != "exact" or case["mode"] == "fast":
         return {"rel": 5e-3}    # one 16-bit term per operand
     return {"rel": 1e-4}        # two 16-bit terms per activation, logits of some ten units in a softmax
+
+
+def _activation(name, z):
+    if name == "relu":
+        return z.clamp(min=0)
+    if name == "leaky":
+        return torch.where(z > 0, z, 0.01 * z)
+    if name == "foo52":
+        return torch.where(z > 1, 1 + 0.01 * (z - 1), torch.where(z < 0, 0.01 * z, z))
+    return {"sigmoid": torch.sigmoid, "tanh": torch.tanh, "softmax": lambda v: torch.softmax(v, 1)}[name](z)
+
+
+def exact(case, seed):
+    """The forward pass in 64 bits, on the weights that the loaded file stands for.  Files are compared byte for byte; a
+    training job's result hangs on the order of the library's own shuffles and has no such value."""
+    if case["kind"] not in ("device", "host", "sample"):
+        return None
+    topology = _topology(case)
+    net = _served(case["net"], case["acts"], case["precision"])
+    weights, biases = torch.from_numpy(np.array(net.weights)), torch.from_numpy(np.array(net.biases))
+    a = _inputs(case["rows"], topology[0], seed, uniform=case["net"] == MLP["net"]).double()
+    w_pos = b_pos = 0
+    for fan_in, fan_out, act in zip(topology, topology[1:], case["acts"].split(",")):
+        w = weights[w_pos:w_pos + fan_in * fan_out].cuda().double().view(fan_out, fan_in)
+        a = _activation(act, a @ w.T + biases[b_pos:b_pos + fan_out].cuda().double())
+        w_pos += fan_in * fan_out
+        b_pos += fan_out
+    return a[0].cpu().numpy() if case["kind"] == "sample" else a if case["kind"] == "device" else a.cpu().numpy()
