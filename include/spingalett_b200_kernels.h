@@ -227,6 +227,21 @@ SPGK_API int spgk_layer_wstream(const spgk_layer *L, const spgk_layer *next, con
                                 void *scratch, void *stream);
 SPGK_API int spgk_wstream_status(void *scratch, void *stream);
 
+/* ---- K3i: integer files, a few to a few hundred rows --------------------------
+ * Whole net of INT8 / INT4 / INT2 layers through the 8-bit integer tensor path (tcgen05 kind::i8): activations as
+ * four base-128 digits of a 28-bit fixed-point number per value (scaled by the row's maximum), exact integer sums.
+ * Two kernels per layer: digits of the layer's input, then the layer.  ys[l] receives layer l's output, fp32
+ * [N][layers[l].out]; ACT_SOFTMAX, allowed on the last layer only, is left to spgk_softmax_rows.
+ * Needs 16-byte aligned packed rows, in <= 131072 and N <= SPGK_ISTREAM_MAX_BATCH; other nets: SPGK_E_UNSUPPORTED
+ * (and spgk_istream_scratch_bytes returns 0).
+ * scratch: spgk_istream_scratch_bytes bytes; its first 16640 bytes (status word, counters) ZERO before first use and
+ * left at zero.  They are laid out as in spgk_layer_wstream's scratch, so one buffer may serve both and
+ * spgk_wstream_status reads the status of either. */
+#define SPGK_ISTREAM_MAX_BATCH 512
+SPGK_API size_t spgk_istream_scratch_bytes(const spgk_layer *layers, uint32_t count, uint32_t N);
+SPGK_API int spgk_istream_forward(const spgk_layer *layers, uint32_t count, const float *x, uint32_t ldx, float *const *ys,
+                                  uint32_t N, void *scratch, void *stream);
+
 /* ---- K2: large-batch tcgen05 GEMM layer ----------------------------------
  * C[N][out] = act(bias + w_scale * A[N][in] * W^T) with the accumulator in
  * tensor memory; both operands reach shared memory by TMA (no multicast).

@@ -1,0 +1,642 @@
+// spg_istream.cu -- batches of a few to a few hundred rows on integer files (INT8 / INT4 / INT2): the packed weights
+// stream once per 64 rows through the 8-bit integer tensor path, for nets whose every layer qualifies.
+//
+//   y[n][j] = act(bias[j] + w_scale * sum_k q[j][k] * x[n][k])
+//
+// The 128 rows of the tcgen05.mma tile (kind::i8) are weight rows, its columns are the batch: every activation is a
+// 28-bit fixed-point number V = round(x / S * (2^27-1)), S the row's largest magnitude, held as four signed base-128
+// digits, one column per digit.  Products and sums are exact in int32 (tensor memory) and int64 (recombination), so a
+// layer's only errors are the rounding to 28 bits (2^-28 of the row's maximum) and the final rounding to fp32.
+//
+// What bounds it.  HBM needs 41 us for the 272 MB of the INT4 net 8192-16384-16384-8192-1000.  A 128 x 128 block of
+// weights moves through shared memory as 8 KB packed (in and out), 16 KB of operand (in and out) and C * 128 B of digits
+// (in and out, C = 4 columns per row): 56 KB at 8 rows, 112 KB at 64 rows, 440 and 880 cycles at 128 B/clk -- 51 us and
+// 103 us over the net.  One byte per weight in the operand instead of two is why this path exists beside the 16-bit
+// streaming kernel, which writes and reads 32 KB per such block.
+//
+// Per CTA (one per SM, 15 warps):
+//   warp 0      weight boxes by TMA (128 rows x 128 packed bytes, 128-byte swizzle), ahead of the previous layer's end:
+//               weights depend on nothing
+//   warp 14     digit tiles by TMA ([C] x 128 k), after the staging kernel has finished
+//   warps 6-13  unpack a box into operand tiles (INT4: a nibble moved to the top of its byte is 16q in two's complement;
+//               INT2: 64q; INT8 boxes are the operand as they arrive)
+//   warp 1      issues the MMAs, four K = 32 steps per 128-wide block
+//   warps 2-5   tensor memory -> int64 -> scale, bias, activation -> fp32
+// The work is cut evenly: the (row tile, group of rows, box) units of a layer are numbered tile after tile and CTA c takes
+// units [c U / G, (c+1) U / G), so no SM idles in a last wave (128 tiles on 148 SMs would waste 14 %).  A tile that spans
+// CTAs is summed in int64 by the CTA that finishes last (a counter per tile); integer sums do not depend on the order.
+//
+// Every mbarrier wait is bounded.  Reference: forward / batch_forward layer step, Src/Spingalett.Network.c:218-247,
+// Src/Spingalett.Training.c:327-343, decode of Src/Spingalett.Serialize.c:222-294.
+#include "spg_common.cuh"
+#include "spg_tc.cuh"
+#include <cstdio>
+
+namespace {
+
+using namespace spgtc;
+
+constexpr uint32_t IS_CONV_WARP0 = 6, IS_CONV_WARPS = 8, IS_DIGIT_WARP = IS_CONV_WARP0 + IS_CONV_WARPS;
+constexpr uint32_t IS_THREADS = 32 * (IS_DIGIT_WARP + 1);
+constexpr uint32_t TILE_ROWS = 128;
+constexpr uint32_t BOX_BYTES = 128 * TILE_ROWS;        // one box of packed weights = one operand tile = 16 KB
+constexpr uint32_t GROUP_ROWS = 64;                    // batch rows per pass over the weights: 256 digit columns
+constexpr uint32_t MAX_K = 131072;                     // 64 * 128 * K < 2^31
+constexpr uint32_t MAX_TILES = 4096;                   // counters in the scratch head
+constexpr uint32_t STAGE_THREADS = 1024;
+constexpr double Q27 = 134217727.0;
+
+struct IsParams {
+    uint32_t out, groups, rpg, N, C;                   // rows per group, batch rows, columns of a tile (4 * rpg)
+    uint32_t kbr, boxes;                               // 128-wide k-blocks per box, boxes per row tile
+    uint32_t RS, AS, BS;
+    uint64_t units;                                    // tiles * boxes
+    uint32_t direct; int prec, act;
+    double scale; const float *bias; const double *row_scale;
+    float *y; uint32_t ldy;
+    long long *partial; uint32_t *counters; int32_t *status;
+    uint32_t idesc;
+};
+
+// D[tmem] (+)= A[smem desc] * B[smem desc], signed 8-bit operands, int32 accumulate, one CTA
+__device__ __forceinline__ void umma_i8(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate)
+{
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n\t}"
+        ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(0u) : "memory");
+}
+// int32 accumulator, A and B signed 8-bit, both K-major, M = 128, N = n
+inline uint32_t idesc_i8(uint32_t n) { return (2u << 4) | (1u << 7) | (1u << 10) | ((n >> 3) << 17) | ((128u >> 4) << 24); }
+
+// first unit of CTA c
+__host__ __device__ inline uint64_t unit_start(uint64_t units, uint32_t grid, uint32_t c) { return units * c / grid; }
+
+// ---- staging: fp32 rows -> digit operand -------------------------------------------------------------------------------
+
+// byte of element e (0..15) inside a group of 16 consecutive k, in the order in which the unpacking delivers the weights
+template <int PREC> __host__ __device__ constexpr uint32_t is_position(uint32_t e)
+{
+    return PREC == SPG_P_I4 ? (e & 8u) + (e & 1u) * 4u + ((e & 7u) >> 1)
+         : PREC == SPG_P_I2 ? (e & 3u) * 4u + (e >> 2) : e;
+}
+
+__device__ __forceinline__ void is_load16(float (&f)[16], const float *row, uint32_t k, uint32_t in, uint32_t vec)
+{
+#pragma unroll
+    for (uint32_t i = 0; i < 16; i += 4) {
+        float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (k < in) {
+            if (vec) v = *reinterpret_cast<const float4 *>(row + k + i);
+            else v = make_float4(row[k + i], row[k + i + 1], row[k + i + 2], row[k + i + 3]);
+        }
+        f[i] = v.x; f[i + 1] = v.y; f[i + 2] = v.z; f[i + 3] = v.w;
+    }
+}
+// largest magnitude as an integer: a NaN counts as more than an infinity
+__device__ __forceinline__ uint32_t is_magnitude(const float (&f)[16])
+{
+    uint32_t m = 0;
+#pragma unroll
+    for (uint32_t i = 0; i < 16; i++) m = max(m, __float_as_uint(f[i]) & 0x7FFFFFFFu);
+    return m;
+}
+
+// One CTA per batch row (rows past N and k past `in` become zero digits): the row's maximum, then four digit rows of `ld`
+// bytes, 16 elements per thread and step.  64 rows of 16384: 4 MB in, 4 MB out, a few microseconds, of which the next
+// layer's first weight boxes hide some.  A row with an infinity or a NaN gets a NaN scale and zero digits.
+template <int PREC>
+__global__ void __launch_bounds__(STAGE_THREADS)
+spg_is_stage_kernel(const float *__restrict__ x, uint32_t ldx, uint32_t N, uint32_t in, uint32_t ld, uint32_t vec,
+                    uint8_t *__restrict__ dst, double *__restrict__ row_scale)
+{
+    __shared__ uint32_t s_max[32];
+    spg_grid_trigger();
+    spg_grid_wait();
+    const uint32_t n = blockIdx.x, tid = threadIdx.x;
+    const bool live = n < N;
+    const float *row = x + (uint64_t)(live ? n : 0) * ldx;
+    float f[16];                                       // the thread's first 16 elements are read once; `in` is a multiple of 16
+    is_load16(f, row, 16 * tid, live ? in : 0, vec);
+    uint32_t m = is_magnitude(f);
+    for (uint32_t k = 16 * (tid + STAGE_THREADS); live && k < in; k += 16 * STAGE_THREADS) {
+        float g[16];
+        is_load16(g, row, k, in, vec);
+        m = max(m, is_magnitude(g));
+    }
+    m = __reduce_max_sync(0xffffffffu, m);
+    if ((tid & 31u) == 0) s_max[tid >> 5] = m;
+    __syncthreads();
+    m = __reduce_max_sync(0xffffffffu, s_max[tid & 31u]);
+    const bool finite = m < 0x7F800000u;
+    const double s = (double)__uint_as_float(m);
+    const double inv = finite && m ? Q27 / s : 0.0;
+    if (tid == 0) row_scale[n] = finite ? s / Q27 : (double)__uint_as_float(0x7FC00000u);
+    const bool zero = !live || !finite;
+    for (uint32_t k = 16 * tid; k < ld; k += 16 * STAGE_THREADS) {
+        if (k >= 16 * STAGE_THREADS) is_load16(f, row, k, live ? in : 0, vec);
+        uint32_t w[4][4] = {};
+        if (!zero) {
+#pragma unroll
+            for (uint32_t i = 0; i < 16; i++) {
+                // adding 1.5 * 2^52 leaves the product, rounded to an integer once, in the low word
+                int v = __double2loint(fma((double)f[i], inv, 6755399441055744.0));
+                const uint32_t pos = is_position<PREC>(i);
+#pragma unroll
+                for (uint32_t d = 0; d < 4; d++) {
+                    const int dig = d == 3 ? v : ((v + 64) & 127) - 64;
+                    v = (v - dig) >> 7;
+                    w[d][pos >> 2] |= ((uint32_t)dig & 0xFFu) << (8 * (pos & 3u));
+                }
+            }
+        }
+#pragma unroll
+        for (uint32_t d = 0; d < 4; d++)
+            *reinterpret_cast<uint4 *>(dst + (uint64_t)(4 * n + d) * ld + k) = make_uint4(w[d][0], w[d][1], w[d][2], w[d][3]);
+    }
+}
+
+// ---- the layer ---------------------------------------------------------------------------------------------------------
+
+__device__ __forceinline__ void is_epi_sync() { asm volatile("bar.sync 2, 128;" ::: "memory"); }
+
+__device__ __forceinline__ void is_finish(const IsParams &p, uint32_t n, uint32_t row, float bias, double scale, long long sum)
+{
+    if (row >= p.out || n >= p.N) return;
+    const double v = (double)sum * scale + (double)bias;
+    p.y[(uint64_t)n * p.ldy + row] = spg_activate((float)v, p.act);
+}
+
+// Segments of a CTA: the runs of its units that lie in one tile.
+struct IsSegment { uint64_t u, end; uint32_t tile, k0, k1; };
+__device__ __forceinline__ bool is_next_segment(const IsParams &p, IsSegment &s)
+{
+    if (s.u >= s.end) return false;
+    s.tile = (uint32_t)(s.u / p.boxes);
+    s.k0 = (uint32_t)(s.u - (uint64_t)s.tile * p.boxes);
+    const uint64_t left = s.end - s.u;
+    s.k1 = left < p.boxes - s.k0 ? s.k0 + (uint32_t)left : p.boxes;
+    s.u += s.k1 - s.k0;
+    return true;
+}
+
+// Epilogue role (warps 2..5): thread = one weight row (tensor-memory lane) of the tile, walking the batch rows.
+__device__ __forceinline__ void is_epilogue(const IsParams &p, IsSegment seg, uint32_t tmem_base, uint32_t tfull0, uint32_t tempty0,
+                                            volatile int *abort_flag, int *s_last, double *s_scale, uint32_t warp, uint32_t lane)
+{
+    const uint32_t q = warp & 3u, et = q * 32u + lane;
+    const uint64_t start = seg.u;
+    uint32_t count = 0;
+    spg_grid_wait();
+    for (; is_next_segment(p, seg); count++) {
+        const uint32_t acc = count & 1u, mt = seg.tile / p.groups, n0 = (seg.tile % p.groups) * p.rpg;
+        const bool whole = seg.k1 - seg.k0 == p.boxes;
+        const uint32_t row = mt * TILE_ROWS + et;
+        const float bias = row < p.out ? p.bias[row] : 0.0f;
+        // the group's scales, once per segment into shared memory: a global load per value would be a chain of L2 latencies
+        if (et < p.rpg) s_scale[et] = __ldcg(p.row_scale + n0 + et) * p.scale;
+        is_epi_sync();
+        // a CTA has at most two partial segments: one at the start of its range (slot 0) and one at its end (slot 1)
+        const uint64_t first = (uint64_t)seg.tile * p.boxes + seg.k0;
+        long long *mine = p.partial + ((uint64_t)(2 * blockIdx.x + (first == start ? 0 : 1)) * p.rpg) * TILE_ROWS + et;
+        const bool ok = mbar_wait(tfull0 + 8 * acc, (count >> 1) & 1u, abort_flag, p.status, 9);
+        tc_fence_after();
+        const uint32_t taddr = tmem_base + acc * p.C + ((q * 32u) << 16);
+        for (uint32_t c0 = 0; c0 < p.C; c0 += 16) {
+            uint32_t r[16];
+            tmem_ld16(taddr + c0, r);
+            tmem_ld_wait();
+            if (!ok) continue;
+#pragma unroll
+            for (uint32_t i = 0; i < 4; i++) {
+                const long long v = (((long long)(int)r[4 * i + 3] * 128 + (int)r[4 * i + 2]) * 128 + (int)r[4 * i + 1]) * 128 + (int)r[4 * i];
+                const uint32_t rr = (c0 >> 2) + i;
+                if (whole) is_finish(p, n0 + rr, row, bias, s_scale[rr], v);
+                else __stcg(mine + (uint64_t)rr * TILE_ROWS, v);
+            }
+        }
+        tc_fence_before();
+        mbar_arrive(tempty0 + 8 * acc);                 // the accumulator may be overwritten
+        if (whole) { is_epi_sync(); continue; }         // (the scales of the next segment may replace these)
+        __threadfence();
+        is_epi_sync();
+        if (et == 0) {
+            const uint32_t part = seg.k1 - seg.k0;
+            *s_last = ok && atomicAdd(&p.counters[seg.tile], part) + part == p.boxes;
+        }
+        is_epi_sync();
+        if (*s_last) {
+            __threadfence();
+            // The CTAs that hold units of this tile are consecutive; all but the first have theirs at the start of their range.
+            // Eight rows of three pieces are in flight at a time: the loop is bound by the latency of L2, not by its bytes.
+            const uint64_t t0 = (uint64_t)seg.tile * p.boxes, t1 = t0 + p.boxes;
+            uint32_t c_lo = (uint32_t)(t0 * gridDim.x / p.units);
+            while (c_lo > 0 && unit_start(p.units, gridDim.x, c_lo) > t0) c_lo--;
+            while (unit_start(p.units, gridDim.x, c_lo + 1) <= t0) c_lo++;
+            uint32_t pieces = 1;
+            while (c_lo + pieces < gridDim.x && unit_start(p.units, gridDim.x, c_lo + pieces) < t1) pieces++;
+            const uint64_t piece_step = (uint64_t)2 * p.rpg * TILE_ROWS;
+            const long long *rest = p.partial + (uint64_t)c_lo * piece_step + et;          // slot 0 of the first CTA
+            const long long *head = rest + (unit_start(p.units, gridDim.x, c_lo) == t0 ? 0 : (uint64_t)p.rpg * TILE_ROWS);
+            for (uint32_t r0 = 0; r0 < p.rpg; r0 += 8) {
+                long long sum[8];
+#pragma unroll
+                for (uint32_t i = 0; i < 8; i++) sum[i] = r0 + i < p.rpg ? __ldcg(head + (uint64_t)(r0 + i) * TILE_ROWS) : 0;
+                for (uint32_t c = 1; c < pieces; c += 2) {
+                    const bool two = c + 1 < pieces;
+                    const long long *s0 = rest + c * piece_step, *s1 = rest + (two ? c + 1 : c) * piece_step;
+                    long long v[16];
+#pragma unroll
+                    for (uint32_t i = 0; i < 8; i++) {
+                        v[i] = r0 + i < p.rpg ? __ldcg(s0 + (uint64_t)(r0 + i) * TILE_ROWS) : 0;
+                        v[8 + i] = two && r0 + i < p.rpg ? __ldcg(s1 + (uint64_t)(r0 + i) * TILE_ROWS) : 0;
+                    }
+#pragma unroll
+                    for (uint32_t i = 0; i < 8; i++) sum[i] += v[i] + v[8 + i];
+                }
+#pragma unroll
+                for (uint32_t i = 0; i < 8; i++)
+                    if (r0 + i < p.rpg) is_finish(p, n0 + r0 + i, row, bias, s_scale[r0 + i], sum[i]);
+            }
+            if (et == 0) p.counters[seg.tile] = 0;       // ready for the next layer
+        }
+        is_epi_sync();
+    }
+}
+
+__global__ void __launch_bounds__(IS_THREADS, 1)
+spg_istream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const IsParams p)
+{
+    extern __shared__ uint8_t is_smem_raw[];
+    const uint32_t raw = smem_u32(is_smem_raw);
+    const uint32_t base = (raw + 1023u) & ~1023u;
+    uint8_t *smem = is_smem_raw + (base - raw);
+    // layout: box ring | operand ring (absent for INT8) | digit ring | barriers | flags | scales of a group
+    const uint32_t b_bytes = p.C * 128u;
+    const uint32_t a_off = p.RS * BOX_BYTES;
+    const uint32_t b_off = a_off + (p.direct ? 0u : p.AS * BOX_BYTES);
+    const uint32_t bar_off = b_off + p.BS * b_bytes;
+    const uint32_t rfull0 = base + bar_off, rempty0 = rfull0 + 8 * p.RS;
+    const uint32_t afull0 = rempty0 + 8 * p.RS, aempty0 = afull0 + 8 * p.AS;
+    const uint32_t bfull0 = aempty0 + 8 * p.AS, bempty0 = bfull0 + 8 * p.BS;
+    const uint32_t tfull0 = bempty0 + 8 * p.BS, tempty0 = tfull0 + 16;
+    const uint32_t flag_off = bar_off + 16 * (p.RS + p.AS + p.BS) + 32;
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem + flag_off);
+    volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
+    int *s_last = const_cast<int *>(abort_flag) + 1;
+    double *s_scale = reinterpret_cast<double *>(smem + flag_off + 16);
+
+    const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
+    uint32_t tmem_cols = 32;
+    while (tmem_cols < 2 * p.C) tmem_cols *= 2;          // two accumulators, 512 columns at most
+
+    if (tid == 0) {
+        for (uint32_t s = 0; s < p.RS; s++) { mbar_init(rfull0 + 8 * s, 1); mbar_init(rempty0 + 8 * s, p.direct ? 1 : IS_CONV_WARPS); }
+        for (uint32_t s = 0; s < p.AS; s++) { mbar_init(afull0 + 8 * s, IS_CONV_WARPS / p.AS); mbar_init(aempty0 + 8 * s, 1); }
+        for (uint32_t s = 0; s < p.BS; s++) { mbar_init(bfull0 + 8 * s, 1); mbar_init(bempty0 + 8 * s, 1); }
+        for (uint32_t a = 0; a < 2; a++) { mbar_init(tfull0 + 8 * a, 1); mbar_init(tempty0 + 8 * a, 128); }
+        *abort_flag = 0;
+        mbar_fence_init();
+        prefetch_map(&map_w);
+        prefetch_map(&map_x);
+    }
+    if (warp == 1) tmem_alloc(smem_u32(tmem_slot), tmem_cols);
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem_base = *tmem_slot;
+    spg_grid_trigger();
+
+    const uint32_t abort_addr = smem_u32(const_cast<int *>(abort_flag));
+    IsSegment seg;
+    seg.u = unit_start(p.units, gridDim.x, blockIdx.x);
+    seg.end = unit_start(p.units, gridDim.x, blockIdx.x + 1);
+
+    if (warp == 0) {
+        // ------------------------------ weight boxes ------------------------------
+        // The first ring of boxes goes out before the previous kernel of the stream has ended; every role waits for that end
+        // before its first bounded wait, which would otherwise count somebody else's running time.
+        uint32_t rs = 0, rph = 0;
+        while (is_next_segment(p, seg)) {
+            const int r0 = (int)(seg.tile / p.groups * TILE_ROWS);
+            for (uint32_t b = seg.k0; b < seg.k1; b++) {
+                if (rs == 0 && rph) spg_grid_wait();
+                mbar_wait_uniform(rempty0 + 8 * rs, rph ^ 1u, abort_addr, p.status, 1);
+                if (*abort_flag) goto is_role_done;
+                if (elect_one()) {
+                    mbar_expect_tx(rfull0 + 8 * rs, BOX_BYTES);
+                    tma_load_2d(base + rs * BOX_BYTES, &map_w, rfull0 + 8 * rs, (int)(b * 128u), r0);
+                }
+                __syncwarp();
+                if (++rs == p.RS) { rs = 0; rph ^= 1u; }
+            }
+        }
+    } else if (warp == IS_DIGIT_WARP) {
+        // ------------------------------ digit tiles -------------------------------
+        uint32_t bs = 0, bph = 0;
+        spg_grid_wait();
+        while (is_next_segment(p, seg)) {
+            const int c0 = (int)(seg.tile % p.groups * p.C);
+            for (uint32_t kb = seg.k0 * p.kbr; kb < seg.k1 * p.kbr; kb++) {
+                mbar_wait_uniform(bempty0 + 8 * bs, bph ^ 1u, abort_addr, p.status, 2);
+                if (*abort_flag) goto is_role_done;
+                if (elect_one()) {
+                    mbar_expect_tx(bfull0 + 8 * bs, b_bytes);
+                    tma_load_2d(base + b_off + bs * b_bytes, &map_x, bfull0 + 8 * bs, (int)(kb * 128u), c0);
+                }
+                __syncwarp();
+                if (++bs == p.BS) { bs = 0; bph ^= 1u; }
+            }
+        }
+    } else if (warp == 1) {
+        // ------------------------------ MMA issuer --------------------------------
+        uint32_t rs = 0, rph = 0, as = 0, aph = 0, bs = 0, bph = 0, count = 0;
+        const uint64_t r_desc0 = smem_desc_sw128(base), a_desc0 = smem_desc_sw128(base + a_off), b_desc0 = smem_desc_sw128(base + b_off);
+        const uint32_t b_step = b_bytes >> 4;
+        spg_grid_wait();
+        for (; is_next_segment(p, seg); count++) {
+            const uint32_t acc = count & 1u;
+            mbar_wait_uniform(tempty0 + 8 * acc, ((count >> 1) & 1u) ^ 1u, abort_addr, p.status, 3);
+            if (*abort_flag) goto is_role_done;
+            tc_fence_after();
+            const uint32_t d_tmem = tmem_base + acc * p.C;
+            uint32_t accum = 0;
+            const uint32_t blocks = (seg.k1 - seg.k0) * p.kbr;
+            for (uint32_t kb = 0; kb < blocks; kb++) {
+                uint64_t da;
+                if (p.direct) {
+                    mbar_wait_uniform(rfull0 + 8 * rs, rph, abort_addr, p.status, 4);
+                    da = r_desc0 + (uint64_t)(rs * (BOX_BYTES >> 4));
+                } else {
+                    mbar_wait_uniform(afull0 + 8 * as, aph, abort_addr, p.status, 5);
+                    da = a_desc0 + (uint64_t)(as * (BOX_BYTES >> 4));
+                }
+                mbar_wait_uniform(bfull0 + 8 * bs, bph, abort_addr, p.status, 6);
+                if (*abort_flag) goto is_role_done;
+                tc_fence_after();
+                const uint64_t db = b_desc0 + (uint64_t)(bs * b_step);
+                if (elect_one()) {
+#pragma unroll
+                    for (uint32_t k = 0; k < 4; k++) { umma_i8(d_tmem, da + 2 * k, db + 2 * k, p.idesc, accum); accum = 1; }
+                    umma_commit(bempty0 + 8 * bs);
+                    umma_commit(p.direct ? rempty0 + 8 * rs : aempty0 + 8 * as);
+                }
+                __syncwarp();
+                accum = 1;
+                if (++bs == p.BS) { bs = 0; bph ^= 1u; }
+                if (p.direct) { if (++rs == p.RS) { rs = 0; rph ^= 1u; } }
+                else if (++as == p.AS) { as = 0; aph ^= 1u; }
+            }
+            if (elect_one()) umma_commit(tfull0 + 8 * acc);
+            __syncwarp();
+        }
+    } else if (warp >= IS_CONV_WARP0) {
+        // ------------------------------ unpackers ---------------------------------
+        // AS groups of 8 / AS warps; group g makes the operand tiles of the k-blocks whose running number is g mod AS, always
+        // in ring slot g, so AS tiles are in the making at once and the latency of one (load, unpack, store, proxy fence,
+        // arrive) hides behind the others.  Lanes 0-7 of a quarter warp take eight different rows of a swizzle atom: no bank
+        // conflict on either side.  (Sixteen warps instead of eight: 2 to 5 % slower at every batch size.)
+        if (!p.direct) {
+            const uint32_t wpg = IS_CONV_WARPS / p.AS, TG = 32u * wpg;
+            const uint32_t cw = warp - IS_CONV_WARP0, grp = cw / wpg, ctg = (cw % wpg) * 32u + lane;
+            uint32_t rs = 0, rph = 0, as = 0, aph = 0;
+            uint8_t *atile = smem + a_off + grp * BOX_BYTES;
+            spg_grid_wait();
+            while (is_next_segment(p, seg)) {
+                for (uint32_t b = seg.k0; b < seg.k1; b++) {
+                    const bool okr = mbar_wait(rfull0 + 8 * rs, rph, abort_flag, p.status, 7);
+                    const uint8_t *box = smem + rs * BOX_BYTES;
+                    for (uint32_t j = 0; j < p.kbr; j++) {
+                        if (as == grp) {
+                            const bool ok = okr && mbar_wait(aempty0 + 8 * as, aph ^ 1u, abort_flag, p.status, 8);
+                            if (ok && p.prec == SPG_P_I4) {
+                                // a 128-wide block is pieces 4j .. 4j+3 (16 bytes, 32 nibbles) of each packed row
+                                for (uint32_t u0 = ctg; u0 < 512; u0 += 4 * TG) {
+                                    uint4 w[4];
+#pragma unroll
+                                    for (uint32_t i = 0; i < 4; i++) {
+                                        const uint32_t u = u0 + i * TG, r7 = u & 7u, pc = (u >> 3) & 3u, row = (u >> 5) * 8u + r7;
+                                        w[i] = *reinterpret_cast<const uint4 *>(box + row * 128u + (((4 * j + pc) ^ r7) << 4));
+                                    }
+#pragma unroll
+                                    for (uint32_t i = 0; i < 4; i++) {
+                                        const uint32_t u = u0 + i * TG, r7 = u & 7u, pc = (u >> 3) & 3u, row = (u >> 5) * 8u + r7;
+                                        const uint32_t m = 0xF0F0F0F0u;
+                                        uint4 lo, hi;
+                                        lo.x = (w[i].x << 4) & m; lo.y = w[i].x & m; lo.z = (w[i].y << 4) & m; lo.w = w[i].y & m;
+                                        hi.x = (w[i].z << 4) & m; hi.y = w[i].z & m; hi.z = (w[i].w << 4) & m; hi.w = w[i].w & m;
+                                        *reinterpret_cast<uint4 *>(atile + row * 128u + (((2 * pc) ^ r7) << 4)) = lo;
+                                        *reinterpret_cast<uint4 *>(atile + row * 128u + (((2 * pc + 1) ^ r7) << 4)) = hi;
+                                    }
+                                }
+                            } else if (ok) {
+                                // INT2: pieces 2j, 2j+1 (64 crumbs each), a word of 16 crumbs becomes one 16-byte chunk
+                                for (uint32_t u = ctg; u < 256; u += TG) {
+                                    const uint32_t r7 = u & 7u, pc = (u >> 3) & 1u, row = (u >> 4) * 8u + r7;
+                                    const uint4 v = *reinterpret_cast<const uint4 *>(box + row * 128u + (((2 * j + pc) ^ r7) << 4));
+                                    const uint32_t ws[4] = { v.x, v.y, v.z, v.w };
+#pragma unroll
+                                    for (uint32_t i = 0; i < 4; i++) {
+                                        const uint32_t m = 0xC0C0C0C0u;
+                                        *reinterpret_cast<uint4 *>(atile + row * 128u + (((4 * pc + i) ^ r7) << 4)) =
+                                            make_uint4((ws[i] << 6) & m, (ws[i] << 4) & m, (ws[i] << 2) & m, ws[i] & m);
+                                    }
+                                }
+                            }
+                            fence_async_smem();          // the tensor core reads the tile through the async proxy
+                            __syncwarp();
+                            if (lane == 0) mbar_arrive(afull0 + 8 * as);
+                        }
+                        if (++as == p.AS) { as = 0; aph ^= 1u; }
+                    }
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(rempty0 + 8 * rs);
+                    if (++rs == p.RS) { rs = 0; rph ^= 1u; }
+                }
+            }
+        }
+    } else {
+        is_epilogue(p, seg, tmem_base, tfull0, tempty0, abort_flag, s_last, s_scale, warp, lane);
+    }
+is_role_done:
+    tc_fence_before();
+    __syncthreads();
+    if (*abort_flag) {
+        // a wait gave up: give copies that may still be in flight time to land before the shared memory goes away
+        if (tid == 0) for (int i = 0; i < 256; i++) __nanosleep(1000);
+        __syncthreads();
+    }
+    if (warp == 1) { tc_fence_after(); tmem_free(tmem_base, tmem_cols); }
+}
+
+// ---- host side ---------------------------------------------------------------------------------------------------------
+
+struct IsPlan {
+    uint32_t groups, rpg, C, kbr, boxes, ld, m_tiles, tiles, RS, AS, BS, grid;
+    uint64_t units;
+    size_t partial_bytes, operand_bytes, smem;
+    bool direct, ok;
+};
+
+constexpr size_t IS_HEAD = 256 + 4 * MAX_TILES;        // status word, counters (both zero between calls)
+
+IsPlan is_plan(const spgk_layer *L, uint32_t N, uint32_t sms)
+{
+    IsPlan pl{};
+    const int prec = L->precision;
+    if (prec != SPG_P_I8 && prec != SPG_P_I4 && prec != SPG_P_I2) return pl;
+    if (!L->in || !L->out || L->in > MAX_K || N == 0 || N > SPGK_ISTREAM_MAX_BATCH) return pl;
+    const uint32_t bits = spg_bits_per_elem(prec);
+    if ((L->in * bits) % 128 || ((uintptr_t)L->w & 15u)) return pl;       // TMA: 16-byte aligned packed rows
+    pl.groups = (N + GROUP_ROWS - 1) / GROUP_ROWS;
+    pl.rpg = ((N + pl.groups - 1) / pl.groups + 3u) & ~3u;
+    pl.C = 4 * pl.rpg;
+    pl.kbr = 8u / bits;
+    pl.direct = prec == SPG_P_I8;
+    pl.boxes = (L->in * bits + 1023u) / 1024u;
+    pl.ld = pl.boxes * pl.kbr * 128u;
+    pl.m_tiles = (L->out + TILE_ROWS - 1) / TILE_ROWS;
+    pl.tiles = pl.m_tiles * pl.groups;
+    if (pl.tiles > MAX_TILES) return pl;
+    pl.units = (uint64_t)pl.tiles * pl.boxes;
+    // one CTA per SM, but a tile in about four pieces at most: the sum over more of them costs more than they save
+    const uint64_t want = (uint64_t)pl.tiles * (pl.boxes < 4 ? pl.boxes : 4);
+    pl.grid = want < sms ? (uint32_t)want : sms;
+    // rings: four operand tiles (one per unpacker group), digit tiles up to 96 KB, boxes with the rest
+    const uint32_t b_bytes = pl.C * 128u;
+    pl.AS = pl.direct ? 1 : 4;
+    pl.BS = 96u * 1024 / b_bytes;
+    if (pl.BS > 8) pl.BS = 8;
+    const uint32_t a_bytes = pl.direct ? 0 : pl.AS * BOX_BYTES;
+    pl.RS = (224u * 1024 - a_bytes - pl.BS * b_bytes) / BOX_BYTES;
+    if (pl.RS > 10) pl.RS = 10;
+    pl.smem = 1024 + (size_t)pl.RS * BOX_BYTES + a_bytes + (size_t)pl.BS * b_bytes + 16 * (pl.RS + pl.AS + pl.BS) + 32 + 16 + GROUP_ROWS * sizeof(double);
+    pl.partial_bytes = (size_t)2 * pl.grid * pl.rpg * TILE_ROWS * sizeof(long long);
+    pl.operand_bytes = (size_t)pl.groups * pl.C * pl.ld;
+    pl.ok = pl.smem <= 227u * 1024;
+    return pl;
+}
+
+typedef CUresult (*IsEncodeFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *,
+                               const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
+                               CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+
+// 2-D byte map with 128-byte swizzle, box of 128 bytes x `box_rows`
+int is_map(const void *ptr, uint64_t row_bytes, uint64_t rows, uint32_t box_rows, CUtensorMap *out)
+{
+    static IsEncodeFn fn = []() -> IsEncodeFn {
+        void *f = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &f, cudaEnableDefault, &q) != cudaSuccess || q != cudaDriverEntryPointSuccess) return nullptr;
+        return reinterpret_cast<IsEncodeFn>(f);
+    }();
+    if (!fn) { spgk_set_error("cuTensorMapEncodeTiled", "driver entry point not available"); return SPGK_E_CUDA; }
+    cuuint64_t dims[2] = { row_bytes, rows };
+    cuuint64_t strides[1] = { row_bytes };
+    cuuint32_t box[2] = { 128, box_rows };
+    cuuint32_t estr[2] = { 1, 1 };
+    const CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void *>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                          CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) {
+        char msg[64];
+        snprintf(msg, sizeof msg, "CUresult %d", (int)r);
+        spgk_set_error("cuTensorMapEncodeTiled (integer stream)", msg);
+        return SPGK_E_CUDA;
+    }
+    return SPGK_OK;
+}
+
+// scratch: head | partial sums | digit operand | row scales, each part sized for the largest layer
+struct IsScratch { size_t partial, operand, scales, total; bool ok; };
+IsScratch is_scratch(const spgk_layer *layers, uint32_t count, uint32_t N, uint32_t sms)
+{
+    IsScratch s{};
+    size_t partial = 0, operand = 0, rows = 0;
+    for (uint32_t l = 0; l < count; l++) {
+        if (l + 1 < count && (layers[l].act == SPG_ACT_SOFTMAX || layers[l + 1].in != layers[l].out)) return s;
+        const IsPlan pl = is_plan(&layers[l], N, sms);
+        if (!pl.ok) return s;
+        if (pl.partial_bytes > partial) partial = pl.partial_bytes;
+        if (pl.operand_bytes > operand) operand = pl.operand_bytes;
+        rows = (size_t)pl.groups * pl.rpg;
+    }
+    if (!rows) return s;
+    s.partial = IS_HEAD;
+    s.operand = s.partial + ((partial + 255) & ~(size_t)255);
+    s.scales = s.operand + ((operand + 255) & ~(size_t)255);
+    s.total = s.scales + rows * sizeof(double);
+    s.ok = true;
+    return s;
+}
+
+}  // namespace
+
+extern "C" {
+
+size_t spgk_istream_scratch_bytes(const spgk_layer *layers, uint32_t count, uint32_t N)
+{
+    SpgDeviceProps dp;
+    if (!layers || spg_device_props(&dp) != SPGK_OK || dp.cc != 100) return 0;
+    const IsScratch s = is_scratch(layers, count, N, (uint32_t)dp.sm_count);
+    return s.ok ? s.total : 0;
+}
+
+int spgk_istream_forward(const spgk_layer *layers, uint32_t count, const float *x, uint32_t ldx, float *const *ys, uint32_t N,
+                         void *scratch, void *stream)
+{
+    if (!layers || !x || !ys || !scratch) { spgk_set_error("spgk_istream_forward", "bad argument"); return SPGK_E_ARG; }
+    SpgDeviceProps dp;
+    int rc;
+    if ((rc = spg_device_props(&dp))) return rc;
+    if (dp.cc != 100) return SPGK_E_UNSUPPORTED;                         // tcgen05 / TMEM exist on sm_100 only
+    const uint32_t sms = (uint32_t)dp.sm_count;
+    const IsScratch sc = is_scratch(layers, count, N, sms);
+    if (!sc.ok) return SPGK_E_UNSUPPORTED;
+    {
+        static SpgOncePerDevice once;
+        int dev = 0;
+        SPGK_CUDA(cudaGetDevice(&dev));
+        rc = once.run(dev, [&]() -> int {
+            SPGK_CUDA(cudaFuncSetAttribute(spg_istream_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
+            return SPGK_OK;
+        });
+        if (rc) return rc;
+    }
+    cudaStream_t s = (cudaStream_t)stream;
+    uint8_t *base = reinterpret_cast<uint8_t *>(scratch);
+    uint8_t *operand = base + sc.operand;
+    double *row_scale = reinterpret_cast<double *>(base + sc.scales);
+    const float *xin = x;
+    uint32_t xld = ldx;
+    for (uint32_t l = 0; l < count; l++) {
+        const spgk_layer *L = &layers[l];
+        const IsPlan pl = is_plan(L, N, sms);
+        const uint32_t vec = (((uintptr_t)xin | ((uintptr_t)xld * 4)) & 15u) == 0;
+        auto stage = L->precision == SPG_P_I8 ? spg_is_stage_kernel<SPG_P_I8> : L->precision == SPG_P_I4 ? spg_is_stage_kernel<SPG_P_I4> : spg_is_stage_kernel<SPG_P_I2>;
+        CUtensorMap map_w, map_x;
+        if ((rc = is_map(L->w, (uint64_t)L->in * spg_bits_per_elem(L->precision) / 8, L->out, TILE_ROWS, &map_w))) return rc;
+        if ((rc = is_map(operand, pl.ld, (uint64_t)pl.groups * pl.C, pl.C, &map_x))) return rc;
+        SPGK_CUDA(spg_launch_chained(stage, dim3(pl.groups * pl.rpg), dim3(STAGE_THREADS), 0, s, xin, xld, N, L->in, pl.ld, vec, operand, row_scale));
+        if ((rc = spgk_check_launch("spg_is_stage_kernel"))) return rc;
+        IsParams p{};
+        p.out = L->out; p.groups = pl.groups; p.rpg = pl.rpg; p.N = N; p.C = pl.C;
+        p.kbr = pl.kbr; p.boxes = pl.boxes; p.units = pl.units;
+        p.RS = pl.RS; p.AS = pl.AS; p.BS = pl.BS;
+        p.direct = pl.direct; p.prec = L->precision;
+        p.act = L->act == SPG_ACT_SOFTMAX ? SPG_ACT_NONE : L->act;
+        p.scale = (double)L->w_scale / (L->precision == SPG_P_I4 ? 16.0 : L->precision == SPG_P_I2 ? 64.0 : 1.0);
+        p.bias = L->bias; p.row_scale = row_scale;
+        p.y = ys[l]; p.ldy = L->out;
+        p.status = reinterpret_cast<int32_t *>(base);
+        p.counters = reinterpret_cast<uint32_t *>(base + 256);
+        p.partial = reinterpret_cast<long long *>(base + sc.partial);
+        p.idesc = idesc_i8(pl.C);
+        SPGK_CUDA(spg_launch_chained(spg_istream_kernel, dim3(pl.grid), dim3(IS_THREADS), pl.smem, s, map_w, map_x, p));
+        if ((rc = spgk_check_launch("spg_istream_kernel"))) return rc;
+        xin = ys[l]; xld = L->out;
+    }
+    return SPGK_OK;
+}
+
+}  // extern "C"

@@ -452,6 +452,47 @@ int spg_dev_forward_small(spg_net *n, const float *d_x, uint32_t ldx, uint32_t N
     return SPINGALETT_OK;
 }
 
+/* The integer streaming kernel serves nets of at least this many packed weight bytes, from this many rows on (figures
+ * beside the call in forward_batch_on). */
+#define SPG_ISTREAM_MIN_BYTES ((size_t)64 << 20)
+#define SPG_ISTREAM_MIN_ROWS 7u
+
+/* The whole net on the 8-bit integer streaming kernel, for nets of integer layers that it takes (SPINGALETT_OK with
+ * *d_last == NULL means that it does not take this one and nothing was launched). */
+static int forward_istream(spg_net *n, const float *d_x, uint32_t N, float **d_last, float *d_final)
+{
+    NeuralNetwork *p = &n->pub;
+    *d_last = NULL;
+    size_t packed = 0;
+    for (uint32_t l = 0; l < n->dev_layers; l++) packed += spg_array_bytes((uint64_t)n->klayers[l].in * n->klayers[l].out, (PrecisionMode)n->klayers[l].precision);
+    if (packed < SPG_ISTREAM_MIN_BYTES) return SPINGALETT_OK;
+    const size_t need = spgk_istream_scratch_bytes(n->klayers, n->dev_layers, N);
+    if (!need) return SPINGALETT_OK;
+    int rc = reserve_zeroed(n, &n->d_ws_scratch, &n->ws_scratch_bytes, need, "integer-stream scratch");
+    if (rc) return rc;
+    if (n->small_cap < N || !n->d_small) {
+        spgk_free(n->d_small); n->d_small = NULL; n->small_cap = 0;
+        void *b = NULL;
+        if ((rc = spg_map_kernel_error(spgk_malloc(&b, (size_t)N * p->total_neurons * sizeof(float)), "small-batch workspace"))) return rc;
+        n->d_small = b; n->small_cap = N;
+    }
+    float *ys[n->dev_layers];
+    for (uint32_t l = 0; l < n->dev_layers; l++)
+        ys[l] = (d_final && l + 1 == n->dev_layers) ? d_final : n->d_small + (size_t)N * p->neuron_offsets[l + 1];
+    prof_mark(n);
+    rc = spg_map_kernel_error(spgk_istream_forward(n->klayers, n->dev_layers, d_x, p->topology[0], ys, N, n->d_ws_scratch, n->stream), "layers (integer stream)");
+    prof_mark(n);
+    if (rc) return rc;
+    n->ws_pending = true;
+    const spgk_layer *Ll = &n->klayers[n->dev_layers - 1];
+    float *y = ys[n->dev_layers - 1];
+    if (Ll->act == ACT_SOFTMAX && (rc = spg_map_kernel_error(spgk_softmax_rows(y, Ll->out, N, Ll->out, n->stream), "softmax"))) return rc;
+    /* the name of the family that serves this many rows */
+    spg_note_path(N <= 3 * SPGK_GEMV_MAX_BATCH ? "gemv" : N <= 96 ? "wstream" : "tcgen05");
+    *d_last = y;
+    return SPINGALETT_OK;
+}
+
 /* ------------------------------------------------------------------------ */
 /* large-batch chain                                                         */
 /* ------------------------------------------------------------------------ */
@@ -1037,6 +1078,19 @@ static float *forward_batch_on(spg_net *n, ForwardBatchArgs a)
     /* Up to 8 rows always take the weight-streaming chain; up to 512 rows do so (in groups of at most 128
      * rows, each group streaming the packed weights once) when every layer is eligible for the tensor-core
      * streaming kernel; everything else is the large-batch GEMM chain. */
+    /* Large integer files from a few rows on: the 8-bit integer streaming kernel when it takes every layer.  Large INT4
+     * net: 160 us against 202 us (GEMV) at 8 rows, 257 against 578 us (16-bit streaming kernel) at 64, 615 against
+     * 680 us (GEMM chain) at 256.  FAST asks for one term per operand, which the GEMM chain serves beyond 96 rows. */
+    if (N >= SPG_ISTREAM_MIN_ROWS && N <= SPGK_ISTREAM_MAX_BATCH && spgk_gemv_get_int_path() &&
+        (N <= 96 || spingalett_get_math_mode() != SPINGALETT_MATH_FAST)) {
+        float *d_last = NULL;
+        if (forward_istream(n, d_x, N, &d_last, out_dev ? result : NULL)) return NULL;
+        if (d_last) {
+            if (!out_dev && spg_map_kernel_error(spgk_memcpy_d2h(result, d_last, out_bytes, n->stream), "forward_batch: output copy")) return NULL;
+            if (!(in_dev && out_dev) && finish(n)) return NULL;
+            return result;
+        }
+    }
     /* 9 to 24 rows on a net the GEMV takes whole: groups of 8 rows through the GEMV (0.2 ms per group on the large
      * INT4 net) beat one pass of the tensor-core streaming kernel (0.7 - 0.8 ms there) */
     bool gemv_groups = N > SPGK_GEMV_MAX_BATCH && N <= 3 * SPGK_GEMV_MAX_BATCH;

@@ -1,0 +1,111 @@
+"""The 8-bit integer streaming kernel (spgk_istream_forward): whole nets of INT8 / INT4 / INT2 layers against float64.
+
+The bound per output is derived: an input value is rounded to a multiple of S / (2^27 - 1), S the row's largest magnitude,
+so it is off by less than S * 2^-27.9; products and sums are exact; the result is rounded to fp32 once and the activation
+function (2 ulp) is applied."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+Q = {3: 127.0, 4: 7.0, 5: 1.0}
+
+
+@pytest.fixture()
+def k(spg, has_gpu):
+    assert has_gpu
+    lib, vp = spg.lib(), C.c_void_p
+    lib.spgk_istream_scratch_bytes.argtypes = [C.POINTER(spg.abi.KLayer), C.c_uint32, C.c_uint32]
+    lib.spgk_istream_scratch_bytes.restype = C.c_size_t
+    lib.spgk_istream_forward.argtypes = [C.POINTER(spg.abi.KLayer), C.c_uint32, vp, C.c_uint32, C.POINTER(vp), C.c_uint32, vp, vp]
+    lib.spgk_wstream_status.argtypes = [vp, vp]
+    lib.spgk_error_string.restype = C.c_char_p
+    return lib
+
+
+def _layer(spg, oracle, rng, out, inn, prec, act):
+    import torch
+    raw = oracle.Oracle.encode((rng.standard_normal(out * inn) / np.sqrt(inn)).astype(np.float32), prec)
+    dec = oracle.Oracle.decode(raw, out * inn, prec).astype(np.float64).reshape(out, inn)
+    scale = float(np.frombuffer(raw[:4].tobytes(), np.float32)[0]) / Q[prec]
+    w = torch.from_numpy(np.concatenate([raw[4:], np.zeros(256, np.uint8)])).cuda()
+    bias = rng.standard_normal(out).astype(np.float32) * 0.1
+    b = torch.from_numpy(bias).cuda()
+    return spg.abi.KLayer(w.data_ptr(), b.data_ptr(), scale, inn, out, prec, act), dec, bias, (w, b)
+
+
+def _bound(x, dec, y):
+    return np.abs(x).max(1, keepdims=True) * 2.0 ** -27.9 * np.abs(dec).sum(1) + 4e-7 * np.abs(y) + 1e-30
+
+
+# one row tile and ragged ones, a tile in pieces, one box and several, one group of rows and several, a padded group
+@pytest.mark.parametrize("prec", [3, 4, 5])
+@pytest.mark.parametrize("out,inn,n", [(128, 64, 1), (1, 128, 4), (100, 1024, 2), (1000, 8192, 3), (129, 576, 9), (257, 4096, 17),
+                                       (640, 2048, 64), (300, 1280, 65), (130, 17408, 100), (2500, 1088, 512)])
+def test_layer_against_float64(spg, k, oracle, prec, out, inn, n):
+    import torch
+    rng = np.random.default_rng(out * 31 + inn + n)
+    L, dec, bias, hold = _layer(spg, oracle, rng, out, inn, prec, 6)
+    x = rng.standard_normal((n, inn)).astype(np.float32)
+    x[0] *= 1e-30                                   # rows have scales of their own
+    if n > 2:
+        x[1] = 0.0
+        x[2, inn // 2] = 1e6                        # one large value: the rest of the row keeps what is left of the 28 bits
+    buf = torch.zeros(n * inn + 1, device="cuda")
+    y = torch.full((n + 1, out), -9.0, device="cuda")
+    nbytes = k.spgk_istream_scratch_bytes(C.byref(L), 1, n)
+    assert nbytes > 0
+    scratch = torch.zeros(nbytes, dtype=torch.uint8, device="cuda")
+    ys = (C.c_void_p * 1)(y.data_ptr())
+    want = x.astype(np.float64) @ dec.T + bias
+    for off in (0, 1):                              # 16-byte aligned rows and rows that are not; the second call finds the counters at zero
+        buf[off:off + n * inn] = torch.from_numpy(x.ravel()).cuda()
+        y.fill_(-9.0)
+        assert k.spgk_istream_forward(C.byref(L), 1, buf.data_ptr() + 4 * off, inn, ys, n, scratch.data_ptr(), None) == 0, k.spgk_error_string()
+        assert k.spgk_wstream_status(scratch.data_ptr(), None) == 0, k.spgk_error_string()
+        got = y.cpu().numpy()
+        assert np.all(got[n] == -9.0)
+        assert np.all(np.abs(got[:n] - want) <= _bound(x.astype(np.float64), dec, want)), np.abs(got[:n] - want).max()
+
+
+@pytest.mark.parametrize("precs", [(4, 4, 4), (3, 5, 4)])
+def test_chain_and_rows_that_are_not_finite(spg, k, oracle, precs):
+    import torch
+    rng = np.random.default_rng(5)
+    topo, acts, n = [576, 384, 640, 130], [3, 4, 6], 70      # leaky, foo52, none
+    built = [_layer(spg, oracle, rng, o, i, p, a) for i, o, p, a in zip(topo, topo[1:], precs, acts)]
+    Ls = (spg.abi.KLayer * 3)(*[b[0] for b in built])
+    x = rng.standard_normal((n, topo[0])).astype(np.float32)
+    x[3, 7], x[66, 9] = np.inf, np.nan
+    ys_t = [torch.zeros(n, o, device="cuda") for o in topo[1:]]
+    ys = (C.c_void_p * 3)(*[t.data_ptr() for t in ys_t])
+    scratch = torch.zeros(k.spgk_istream_scratch_bytes(Ls, 3, n), dtype=torch.uint8, device="cuda")
+    xd = torch.from_numpy(x).cuda()
+    assert k.spgk_istream_forward(Ls, 3, xd.data_ptr(), topo[0], ys, n, scratch.data_ptr(), None) == 0, k.spgk_error_string()
+    assert k.spgk_wstream_status(scratch.data_ptr(), None) == 0, k.spgk_error_string()
+    good = np.isfinite(x).all(1)
+    a = x.astype(np.float64)
+    for t, (_, dec, bias, _), act in zip(ys_t, built, acts):
+        a = np.where(good[:, None], a, 0.0)
+        z = a @ dec.T + bias
+        want = {3: np.where(z > 0, z, 0.01 * z), 4: np.where(z > 1, 1 + 0.01 * (z - 1), np.where(z < 0, 0.01 * z, z)), 6: z}[act]
+        got = t.cpu().numpy()
+        assert not np.any(np.isfinite(got[~good]))
+        # a layer is measured on the input that the device had, so that the bound is one layer's (the activations' slopes are at most 1)
+        assert np.all(np.abs(got[good] - want[good]) <= _bound(a, dec, z)[good])
+        a = got.astype(np.float64)
+
+
+def test_what_is_declined(spg, k):
+    import torch
+    w, b = torch.zeros(1 << 16, dtype=torch.uint8, device="cuda"), torch.zeros(64, device="cuda")
+    ok = spg.abi.KLayer(w.data_ptr(), b.data_ptr(), 1.0, 64, 64, 4, 1)
+    assert k.spgk_istream_scratch_bytes(C.byref(ok), 1, 16) > 0
+    assert k.spgk_istream_scratch_bytes(C.byref(ok), 1, 513) == 0
+    for bad in [spg.abi.KLayer(w.data_ptr(), b.data_ptr(), 1.0, 72, 64, 4, 1),        # packed rows of 36 bytes
+                spg.abi.KLayer(w.data_ptr() + 4, b.data_ptr(), 1.0, 64, 64, 4, 1),    # base not 16-byte aligned
+                spg.abi.KLayer(w.data_ptr(), b.data_ptr(), 1.0, 64, 64, 2, 1)]:       # not an integer file
+        assert k.spgk_istream_scratch_bytes(C.byref(bad), 1, 16) == 0
+    pair = (spg.abi.KLayer * 2)(spg.abi.KLayer(w.data_ptr(), b.data_ptr(), 1.0, 64, 64, 4, 5), ok)      # softmax inside the net
+    assert k.spgk_istream_scratch_bytes(pair, 2, 16) == 0
