@@ -234,9 +234,9 @@ SPGK_API int spgk_wstream_status(void *scratch, void *stream);
  * [N][layers[l].out]; ACT_SOFTMAX, allowed on the last layer only, is left to spgk_softmax_rows.
  * Needs 16-byte aligned packed rows, in <= 131072 and N <= SPGK_ISTREAM_MAX_BATCH; other nets: SPGK_E_UNSUPPORTED
  * (and spgk_istream_scratch_bytes returns 0).
- * scratch: spgk_istream_scratch_bytes bytes; its first 16640 bytes (status word, counters) ZERO before first use and
- * left at zero.  They are laid out as in spgk_layer_wstream's scratch, so one buffer may serve both and
- * spgk_wstream_status reads the status of either. */
+ * scratch: spgk_istream_scratch_bytes bytes, ZERO-FILLED before first use (status word, counters and sums are left at
+ * zero, at places that do not depend on N); after a failure that the status reports, zero-filled again.
+ * spgk_wstream_status reads its status. */
 #define SPGK_ISTREAM_MAX_BATCH 512
 SPGK_API size_t spgk_istream_scratch_bytes(const spgk_layer *layers, uint32_t count, uint32_t N);
 SPGK_API int spgk_istream_forward(const spgk_layer *layers, uint32_t count, const float *x, uint32_t ldx, float *const *ys,

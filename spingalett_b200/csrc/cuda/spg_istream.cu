@@ -14,17 +14,19 @@
 // 103 us over the net.  One byte per weight in the operand instead of two is why this path exists beside the 16-bit
 // streaming kernel, which writes and reads 32 KB per such block.
 //
-// Per CTA (one per SM, 15 warps):
+// Per CTA (one per SM, 19 warps):
 //   warp 0      weight boxes by TMA (128 rows x 128 packed bytes, 128-byte swizzle), ahead of the previous layer's end:
 //               weights depend on nothing
-//   warp 14     digit tiles by TMA ([C] x 128 k), after the staging kernel has finished
-//   warps 6-13  unpack a box into operand tiles (INT4: a nibble moved to the top of its byte is 16q in two's complement;
+//   warp 18     digit tiles by TMA ([C] x 128 k), after the staging kernel has finished
+//   warps 10-17 unpack a box into operand tiles (INT4: a nibble moved to the top of its byte is 16q in two's complement;
 //               INT2: 64q; INT8 boxes are the operand as they arrive)
 //   warp 1      issues the MMAs, four K = 32 steps per 128-wide block
-//   warps 2-5   tensor memory -> int64 -> scale, bias, activation -> fp32
+//   warps 2-9   tensor memory -> int64 -> scale, bias, activation -> fp32
 // The work is cut evenly: the (row tile, group of rows, box) units of a layer are numbered tile after tile and CTA c takes
 // units [c U / G, (c+1) U / G), so no SM idles in a last wave (128 tiles on 148 SMs would waste 14 %).  A tile that spans
-// CTAs is summed in int64 by the CTA that finishes last (a counter per tile); integer sums do not depend on the order.
+// CTAs is summed in L2 with 64-bit integer reductions, whose result does not depend on their order, and finished by the CTA
+// that comes last (a counter per tile), which leaves the sums at zero for the next layer.  (Pieces written side by side and
+// read back one after the other cost the last CTA 16 L2 round trips at 64 rows, 11 us of every layer.)
 //
 // Every mbarrier wait is bounded.  Reference: forward / batch_forward layer step, Src/Spingalett.Network.c:218-247,
 // Src/Spingalett.Training.c:327-343, decode of Src/Spingalett.Serialize.c:222-294.
@@ -36,7 +38,7 @@ namespace {
 
 using namespace spgtc;
 
-constexpr uint32_t IS_CONV_WARP0 = 6, IS_CONV_WARPS = 8, IS_DIGIT_WARP = IS_CONV_WARP0 + IS_CONV_WARPS;
+constexpr uint32_t IS_EPI_WARPS = 8, IS_CONV_WARP0 = 2 + IS_EPI_WARPS, IS_CONV_WARPS = 8, IS_DIGIT_WARP = IS_CONV_WARP0 + IS_CONV_WARPS;
 constexpr uint32_t IS_THREADS = 32 * (IS_DIGIT_WARP + 1);
 constexpr uint32_t TILE_ROWS = 128;
 constexpr uint32_t BOX_BYTES = 128 * TILE_ROWS;        // one box of packed weights = one operand tile = 16 KB
@@ -54,7 +56,7 @@ struct IsParams {
     uint32_t direct; int prec, act;
     double scale; const float *bias; const double *row_scale;
     float *y; uint32_t ldy;
-    long long *partial; uint32_t *counters; int32_t *status;
+    unsigned long long *sums; uint32_t *counters; int32_t *status;
     uint32_t idesc;
 };
 
@@ -159,7 +161,7 @@ spg_is_stage_kernel(const float *__restrict__ x, uint32_t ldx, uint32_t N, uint3
 
 // ---- the layer ---------------------------------------------------------------------------------------------------------
 
-__device__ __forceinline__ void is_epi_sync() { asm volatile("bar.sync 2, 128;" ::: "memory"); }
+__device__ __forceinline__ void is_epi_sync() { asm volatile("bar.sync 2, %0;" ::"n"(32 * IS_EPI_WARPS) : "memory"); }
 
 __device__ __forceinline__ void is_finish(const IsParams &p, uint32_t n, uint32_t row, float bias, double scale, long long sum)
 {
@@ -181,12 +183,12 @@ __device__ __forceinline__ bool is_next_segment(const IsParams &p, IsSegment &s)
     return true;
 }
 
-// Epilogue role (warps 2..5): thread = one weight row (tensor-memory lane) of the tile, walking the batch rows.
+// Epilogue role (warps 2..9): thread = one weight row (tensor-memory lane) of the tile; of two warps on the same lanes each
+// takes every other four batch rows.
 __device__ __forceinline__ void is_epilogue(const IsParams &p, IsSegment seg, uint32_t tmem_base, uint32_t tfull0, uint32_t tempty0,
                                             volatile int *abort_flag, int *s_last, double *s_scale, uint32_t warp, uint32_t lane)
 {
-    const uint32_t q = warp & 3u, et = q * 32u + lane;
-    const uint64_t start = seg.u;
+    const uint32_t half = (warp - 2u) >> 2, et = (warp & 3u) * 32u + lane;
     uint32_t count = 0;
     spg_grid_wait();
     for (; is_next_segment(p, seg); count++) {
@@ -195,15 +197,22 @@ __device__ __forceinline__ void is_epilogue(const IsParams &p, IsSegment seg, ui
         const uint32_t row = mt * TILE_ROWS + et;
         const float bias = row < p.out ? p.bias[row] : 0.0f;
         // the group's scales, once per segment into shared memory: a global load per value would be a chain of L2 latencies
-        if (et < p.rpg) s_scale[et] = __ldcg(p.row_scale + n0 + et) * p.scale;
+        if (half == 0 && et < p.rpg) s_scale[et] = __ldcg(p.row_scale + n0 + et) * p.scale;
+        // the sums of a tile in pieces belong to the CTA that holds its first unit: at most one tile that goes on past the end
+        // of a CTA's range starts in it
+        unsigned long long *sums = p.sums + et;
+        if (!whole) {
+            const uint64_t t0 = (uint64_t)seg.tile * p.boxes;
+            uint32_t c = (uint32_t)(t0 * gridDim.x / p.units);
+            while (c > 0 && unit_start(p.units, gridDim.x, c) > t0) c--;
+            while (unit_start(p.units, gridDim.x, c + 1) <= t0) c++;
+            sums += (uint64_t)c * p.rpg * TILE_ROWS;
+        }
         is_epi_sync();
-        // a CTA has at most two partial segments: one at the start of its range (slot 0) and one at its end (slot 1)
-        const uint64_t first = (uint64_t)seg.tile * p.boxes + seg.k0;
-        long long *mine = p.partial + ((uint64_t)(2 * blockIdx.x + (first == start ? 0 : 1)) * p.rpg) * TILE_ROWS + et;
         const bool ok = mbar_wait(tfull0 + 8 * acc, (count >> 1) & 1u, abort_flag, p.status, 9);
         tc_fence_after();
-        const uint32_t taddr = tmem_base + acc * p.C + ((q * 32u) << 16);
-        for (uint32_t c0 = 0; c0 < p.C; c0 += 16) {
+        const uint32_t taddr = tmem_base + acc * p.C + ((et & ~31u) << 16);
+        for (uint32_t c0 = 16 * half; c0 < p.C; c0 += 32) {
             uint32_t r[16];
             tmem_ld16(taddr + c0, r);
             tmem_ld_wait();
@@ -213,7 +222,7 @@ __device__ __forceinline__ void is_epilogue(const IsParams &p, IsSegment seg, ui
                 const long long v = (((long long)(int)r[4 * i + 3] * 128 + (int)r[4 * i + 2]) * 128 + (int)r[4 * i + 1]) * 128 + (int)r[4 * i];
                 const uint32_t rr = (c0 >> 2) + i;
                 if (whole) is_finish(p, n0 + rr, row, bias, s_scale[rr], v);
-                else __stcg(mine + (uint64_t)rr * TILE_ROWS, v);
+                else atomicAdd(sums + (uint64_t)rr * TILE_ROWS, (unsigned long long)v);
             }
         }
         tc_fence_before();
@@ -221,45 +230,29 @@ __device__ __forceinline__ void is_epilogue(const IsParams &p, IsSegment seg, ui
         if (whole) { is_epi_sync(); continue; }         // (the scales of the next segment may replace these)
         __threadfence();
         is_epi_sync();
-        if (et == 0) {
+        if (warp == 2 && lane == 0) {
             const uint32_t part = seg.k1 - seg.k0;
             *s_last = ok && atomicAdd(&p.counters[seg.tile], part) + part == p.boxes;
         }
         is_epi_sync();
         if (*s_last) {
             __threadfence();
-            // The CTAs that hold units of this tile are consecutive; all but the first have theirs at the start of their range.
-            // Eight rows of three pieces are in flight at a time: the loop is bound by the latency of L2, not by its bytes.
-            const uint64_t t0 = (uint64_t)seg.tile * p.boxes, t1 = t0 + p.boxes;
-            uint32_t c_lo = (uint32_t)(t0 * gridDim.x / p.units);
-            while (c_lo > 0 && unit_start(p.units, gridDim.x, c_lo) > t0) c_lo--;
-            while (unit_start(p.units, gridDim.x, c_lo + 1) <= t0) c_lo++;
-            uint32_t pieces = 1;
-            while (c_lo + pieces < gridDim.x && unit_start(p.units, gridDim.x, c_lo + pieces) < t1) pieces++;
-            const uint64_t piece_step = (uint64_t)2 * p.rpg * TILE_ROWS;
-            const long long *rest = p.partial + (uint64_t)c_lo * piece_step + et;          // slot 0 of the first CTA
-            const long long *head = rest + (unit_start(p.units, gridDim.x, c_lo) == t0 ? 0 : (uint64_t)p.rpg * TILE_ROWS);
-            for (uint32_t r0 = 0; r0 < p.rpg; r0 += 8) {
-                long long sum[8];
+            for (uint32_t r0 = 4 * half; r0 < p.rpg; r0 += 32) {               // four groups of four rows in flight
+                long long v[16];
 #pragma unroll
-                for (uint32_t i = 0; i < 8; i++) sum[i] = r0 + i < p.rpg ? __ldcg(head + (uint64_t)(r0 + i) * TILE_ROWS) : 0;
-                for (uint32_t c = 1; c < pieces; c += 2) {
-                    const bool two = c + 1 < pieces;
-                    const long long *s0 = rest + c * piece_step, *s1 = rest + (two ? c + 1 : c) * piece_step;
-                    long long v[16];
-#pragma unroll
-                    for (uint32_t i = 0; i < 8; i++) {
-                        v[i] = r0 + i < p.rpg ? __ldcg(s0 + (uint64_t)(r0 + i) * TILE_ROWS) : 0;
-                        v[8 + i] = two && r0 + i < p.rpg ? __ldcg(s1 + (uint64_t)(r0 + i) * TILE_ROWS) : 0;
-                    }
-#pragma unroll
-                    for (uint32_t i = 0; i < 8; i++) sum[i] += v[i] + v[8 + i];
+                for (uint32_t i = 0; i < 16; i++) {
+                    const uint32_t rr = r0 + (i >> 2) * 8 + (i & 3u);
+                    v[i] = rr < p.rpg ? (long long)__ldcg(sums + (uint64_t)rr * TILE_ROWS) : 0;
                 }
 #pragma unroll
-                for (uint32_t i = 0; i < 8; i++)
-                    if (r0 + i < p.rpg) is_finish(p, n0 + r0 + i, row, bias, s_scale[r0 + i], sum[i]);
+                for (uint32_t i = 0; i < 16; i++) {
+                    const uint32_t rr = r0 + (i >> 2) * 8 + (i & 3u);
+                    if (rr >= p.rpg) continue;
+                    __stcg(sums + (uint64_t)rr * TILE_ROWS, 0ull);
+                    is_finish(p, n0 + rr, row, bias, s_scale[rr], v[i]);
+                }
             }
-            if (et == 0) p.counters[seg.tile] = 0;       // ready for the next layer
+            if (warp == 2 && lane == 0) p.counters[seg.tile] = 0;
         }
         is_epi_sync();
     }
@@ -295,7 +288,7 @@ spg_istream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         for (uint32_t s = 0; s < p.RS; s++) { mbar_init(rfull0 + 8 * s, 1); mbar_init(rempty0 + 8 * s, p.direct ? 1 : IS_CONV_WARPS); }
         for (uint32_t s = 0; s < p.AS; s++) { mbar_init(afull0 + 8 * s, IS_CONV_WARPS / p.AS); mbar_init(aempty0 + 8 * s, 1); }
         for (uint32_t s = 0; s < p.BS; s++) { mbar_init(bfull0 + 8 * s, 1); mbar_init(bempty0 + 8 * s, 1); }
-        for (uint32_t a = 0; a < 2; a++) { mbar_init(tfull0 + 8 * a, 1); mbar_init(tempty0 + 8 * a, 128); }
+        for (uint32_t a = 0; a < 2; a++) { mbar_init(tfull0 + 8 * a, 1); mbar_init(tempty0 + 8 * a, 32 * IS_EPI_WARPS); }
         *abort_flag = 0;
         mbar_fence_init();
         prefetch_map(&map_w);
@@ -475,11 +468,11 @@ is_role_done:
 struct IsPlan {
     uint32_t groups, rpg, C, kbr, boxes, ld, m_tiles, tiles, RS, AS, BS, grid;
     uint64_t units;
-    size_t partial_bytes, operand_bytes, smem;
+    size_t operand_bytes, smem;
     bool direct, ok;
 };
 
-constexpr size_t IS_HEAD = 256 + 4 * MAX_TILES;        // status word, counters (both zero between calls)
+constexpr size_t IS_HEAD = 256 + 4 * MAX_TILES;        // status word, counters; zero between calls, like the sums behind them
 
 IsPlan is_plan(const spgk_layer *L, uint32_t N, uint32_t sms)
 {
@@ -512,7 +505,6 @@ IsPlan is_plan(const spgk_layer *L, uint32_t N, uint32_t sms)
     pl.RS = (224u * 1024 - a_bytes - pl.BS * b_bytes) / BOX_BYTES;
     if (pl.RS > 10) pl.RS = 10;
     pl.smem = 1024 + (size_t)pl.RS * BOX_BYTES + a_bytes + (size_t)pl.BS * b_bytes + 16 * (pl.RS + pl.AS + pl.BS) + 32 + 16 + GROUP_ROWS * sizeof(double);
-    pl.partial_bytes = (size_t)2 * pl.grid * pl.rpg * TILE_ROWS * sizeof(long long);
     pl.operand_bytes = (size_t)pl.groups * pl.C * pl.ld;
     pl.ok = pl.smem <= 227u * 1024;
     return pl;
@@ -547,23 +539,23 @@ int is_map(const void *ptr, uint64_t row_bytes, uint64_t rows, uint32_t box_rows
     return SPGK_OK;
 }
 
-// scratch: head | partial sums | digit operand | row scales, each part sized for the largest layer
-struct IsScratch { size_t partial, operand, scales, total; bool ok; };
+// scratch: head | sums, one slot per CTA, of a size that depends on the device alone (they are zero between calls of any batch
+// size) | digit operand of the largest layer | row scales
+struct IsScratch { size_t sums, operand, scales, total; bool ok; };
 IsScratch is_scratch(const spgk_layer *layers, uint32_t count, uint32_t N, uint32_t sms)
 {
     IsScratch s{};
-    size_t partial = 0, operand = 0, rows = 0;
+    size_t operand = 0, rows = 0;
     for (uint32_t l = 0; l < count; l++) {
         if (l + 1 < count && (layers[l].act == SPG_ACT_SOFTMAX || layers[l + 1].in != layers[l].out)) return s;
         const IsPlan pl = is_plan(&layers[l], N, sms);
         if (!pl.ok) return s;
-        if (pl.partial_bytes > partial) partial = pl.partial_bytes;
         if (pl.operand_bytes > operand) operand = pl.operand_bytes;
         rows = (size_t)pl.groups * pl.rpg;
     }
     if (!rows) return s;
-    s.partial = IS_HEAD;
-    s.operand = s.partial + ((partial + 255) & ~(size_t)255);
+    s.sums = IS_HEAD;
+    s.operand = s.sums + (size_t)sms * GROUP_ROWS * TILE_ROWS * sizeof(long long);
     s.scales = s.operand + ((operand + 255) & ~(size_t)255);
     s.total = s.scales + rows * sizeof(double);
     s.ok = true;
@@ -630,7 +622,7 @@ int spgk_istream_forward(const spgk_layer *layers, uint32_t count, const float *
         p.y = ys[l]; p.ldy = L->out;
         p.status = reinterpret_cast<int32_t *>(base);
         p.counters = reinterpret_cast<uint32_t *>(base + 256);
-        p.partial = reinterpret_cast<long long *>(base + sc.partial);
+        p.sums = reinterpret_cast<unsigned long long *>(base + sc.sums);
         p.idesc = idesc_i8(pl.C);
         SPGK_CUDA(spg_launch_chained(spg_istream_kernel, dim3(pl.grid), dim3(IS_THREADS), pl.smem, s, map_w, map_x, p));
         if ((rc = spgk_check_launch("spg_istream_kernel"))) return rc;

@@ -123,6 +123,7 @@ void spg_dev_release(spg_net *n)
     for (int i = 0; i < 2; i++) { spgk_free(n->d_staged[i]); n->d_staged[i] = NULL; n->staged_bytes[i] = 0; }
     for (int i = 0; i < 2; i++) { spgk_free(n->d_operand[i]); n->d_operand[i] = NULL; n->operand_bytes[i] = 0; }
     spgk_free(n->d_ws_scratch); n->d_ws_scratch = NULL; n->ws_scratch_bytes = 0;
+    spgk_free(n->d_is_scratch); n->d_is_scratch = NULL; n->is_scratch_bytes = 0; n->is_pending = false;
     spgk_free(n->d_rep_idx); n->d_rep_idx = NULL; n->rep_idx_bytes = 0;
     n->auto_calibrated = false;
     n->auto_calls = 0;
@@ -228,6 +229,13 @@ static int finish(spg_net *n)
     if (n->ws_pending) {
         n->ws_pending = false;
         if ((rc = spg_map_kernel_error(spgk_wstream_status(n->d_ws_scratch, n->stream), "weight-stream kernel"))) return rc;
+    }
+    if (n->is_pending) {
+        n->is_pending = false;
+        if ((rc = spg_map_kernel_error(spgk_wstream_status(n->d_is_scratch, n->stream), "integer-stream kernel"))) {
+            spgk_free(n->d_is_scratch); n->d_is_scratch = NULL; n->is_scratch_bytes = 0;      /* its counters may be off zero */
+            return rc;
+        }
     }
     if (n->gemv_pending) {
         n->gemv_pending = false;
@@ -468,7 +476,7 @@ static int forward_istream(spg_net *n, const float *d_x, uint32_t N, float **d_l
     if (packed < SPG_ISTREAM_MIN_BYTES) return SPINGALETT_OK;
     const size_t need = spgk_istream_scratch_bytes(n->klayers, n->dev_layers, N);
     if (!need) return SPINGALETT_OK;
-    int rc = reserve_zeroed(n, &n->d_ws_scratch, &n->ws_scratch_bytes, need, "integer-stream scratch");
+    int rc = reserve_zeroed(n, &n->d_is_scratch, &n->is_scratch_bytes, need, "integer-stream scratch");
     if (rc) return rc;
     if (n->small_cap < N || !n->d_small) {
         spgk_free(n->d_small); n->d_small = NULL; n->small_cap = 0;
@@ -480,10 +488,10 @@ static int forward_istream(spg_net *n, const float *d_x, uint32_t N, float **d_l
     for (uint32_t l = 0; l < n->dev_layers; l++)
         ys[l] = (d_final && l + 1 == n->dev_layers) ? d_final : n->d_small + (size_t)N * p->neuron_offsets[l + 1];
     prof_mark(n);
-    rc = spg_map_kernel_error(spgk_istream_forward(n->klayers, n->dev_layers, d_x, p->topology[0], ys, N, n->d_ws_scratch, n->stream), "layers (integer stream)");
+    rc = spg_map_kernel_error(spgk_istream_forward(n->klayers, n->dev_layers, d_x, p->topology[0], ys, N, n->d_is_scratch, n->stream), "layers (integer stream)");
     prof_mark(n);
     if (rc) return rc;
-    n->ws_pending = true;
+    n->is_pending = true;
     const spgk_layer *Ll = &n->klayers[n->dev_layers - 1];
     float *y = ys[n->dev_layers - 1];
     if (Ll->act == ACT_SOFTMAX && (rc = spg_map_kernel_error(spgk_softmax_rows(y, Ll->out, N, Ll->out, n->stream), "softmax"))) return rc;

@@ -50,6 +50,7 @@ typedef struct spg_net_s {
     void *d_staged[2]; size_t staged_bytes[2];   /* ping-pong staged inputs of the GEMV chain */
     void *d_operand[2]; size_t operand_bytes[2]; /* ping-pong activation operands of the weight-streaming chain */
     void *d_ws_scratch; size_t ws_scratch_bytes; bool ws_pending;
+    void *d_is_scratch; size_t is_scratch_bytes; bool is_pending;    /* integer streaming chain */
     /* AUTO math mode: rows recomputed exactly after the one-term pass */
     uint32_t *d_rep_idx; size_t rep_idx_bytes; float *d_rep_in; size_t rep_in_bytes; float *d_rep_out; size_t rep_out_bytes;
     uint32_t last_repaired; bool auto_calibrated; float auto_theta;
