@@ -460,10 +460,10 @@ int spg_dev_forward_small(spg_net *n, const float *d_x, uint32_t ldx, uint32_t N
     return SPINGALETT_OK;
 }
 
-/* The integer streaming kernel serves nets of at least this many packed weight bytes, from this many rows on (figures
- * beside the call in forward_batch_on). */
-#define SPG_ISTREAM_MIN_BYTES ((size_t)64 << 20)
+/* Rows and packed weight bytes that the integer streaming kernel serves (figures beside the call in forward_batch_on) */
 #define SPG_ISTREAM_MIN_ROWS 7u
+#define SPG_ISTREAM_MAX_ROWS 256u
+#define SPG_ISTREAM_MEDIUM_BYTES ((size_t)4 << 20)      /* least packed size beyond 96 rows */
 
 /* The whole net on the 8-bit integer streaming kernel, for nets of integer layers that it takes (SPINGALETT_OK with
  * *d_last == NULL means that it does not take this one and nothing was launched). */
@@ -473,7 +473,7 @@ static int forward_istream(spg_net *n, const float *d_x, uint32_t N, float **d_l
     *d_last = NULL;
     size_t packed = 0;
     for (uint32_t l = 0; l < n->dev_layers; l++) packed += spg_array_bytes((uint64_t)n->klayers[l].in * n->klayers[l].out, (PrecisionMode)n->klayers[l].precision);
-    if (packed < SPG_ISTREAM_MIN_BYTES) return SPINGALETT_OK;
+    if (N > 96 && packed < SPG_ISTREAM_MEDIUM_BYTES) return SPINGALETT_OK;
     const size_t need = spgk_istream_scratch_bytes(n->klayers, n->dev_layers, N);
     if (!need) return SPINGALETT_OK;
     int rc = reserve_zeroed(n, &n->d_is_scratch, &n->is_scratch_bytes, need, "integer-stream scratch");
@@ -1086,10 +1086,13 @@ static float *forward_batch_on(spg_net *n, ForwardBatchArgs a)
     /* Up to 8 rows always take the weight-streaming chain; up to 512 rows do so (in groups of at most 128
      * rows, each group streaming the packed weights once) when every layer is eligible for the tensor-core
      * streaming kernel; everything else is the large-batch GEMM chain. */
-    /* Large integer files from a few rows on: the 8-bit integer streaming kernel when it takes every layer.  Large INT4
-     * net: 160 us against 202 us (GEMV) at 8 rows, 257 against 578 us (16-bit streaming kernel) at 64, 615 against
-     * 680 us (GEMM chain) at 256.  FAST asks for one term per operand, which the GEMM chain serves beyond 96 rows. */
-    if (N >= SPG_ISTREAM_MIN_ROWS && N <= SPGK_ISTREAM_MAX_BATCH && spgk_gemv_get_int_path() &&
+    /* Integer files from a few rows on: the 8-bit integer streaming kernel when it takes every layer.  Measured, against the
+     * path that served before: large INT4 net 152 us against 204 (GEMV) at 8 rows, 207 against 578 (16-bit streaming kernel)
+     * at 64, 554 against 680 (GEMM chain) at 256; at 6 rows the GEMV is level (155, INT2 131), at 512 the chain is ahead
+     * (945).  Nets of 4 and 12 MB: 38 against 54 and 42 against 65 us at 8 rows, 0.45 of the time or less at 32 to 96,
+     * 0.8 to 0.9 at 128 and 256; of 0.5 MB: 34 against 119 us at 8 rows, but no gain beyond 96.  FAST asks for one term per
+     * operand, which the GEMM chain serves beyond 96 rows. */
+    if (N >= SPG_ISTREAM_MIN_ROWS && N <= SPG_ISTREAM_MAX_ROWS && spgk_gemv_get_int_path() &&
         (N <= 96 || spingalett_get_math_mode() != SPINGALETT_MATH_FAST)) {
         float *d_last = NULL;
         if (forward_istream(n, d_x, N, &d_last, out_dev ? result : NULL)) return NULL;
