@@ -1088,7 +1088,7 @@ static float *forward_batch_on(spg_net *n, ForwardBatchArgs a)
      * streaming kernel; everything else is the large-batch GEMM chain. */
     /* Integer files from a few rows on: the 8-bit integer streaming kernel when it takes every layer.  Measured, against the
      * path that served before: large INT4 net 152 us against 204 (GEMV) at 8 rows, 207 against 578 (16-bit streaming kernel)
-     * at 64, 554 against 680 (GEMM chain) at 256; at 6 rows the GEMV is level (155, INT2 131), at 512 the chain is ahead
+     * at 64, 624 against 684 (GEMM chain) at 256; at 6 rows the GEMV is level (155, INT2 131), at 512 the chain is ahead
      * (945).  Nets of 4 and 12 MB: 38 against 54 and 42 against 65 us at 8 rows, 0.45 of the time or less at 32 to 96,
      * 0.8 to 0.9 at 128 and 256; of 0.5 MB: 34 against 119 us at 8 rows, but no gain beyond 96.  FAST asks for one term per
      * operand, which the GEMM chain serves beyond 96 rows. */
