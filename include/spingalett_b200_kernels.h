@@ -230,6 +230,7 @@ SPGK_API int spgk_wstream_status(void *scratch, void *stream);
 /* ---- K3i: integer files, a few to a few hundred rows --------------------------
  * Whole net of INT8 / INT4 / INT2 layers through the 8-bit integer tensor path (tcgen05 kind::i8): activations as
  * four base-128 digits of a 28-bit fixed-point number per value (scaled by the row's maximum), exact integer sums.
+ * Rows with more than an eighth of their non-zero values below 2^-12 of the maximum hold those in four more digits.
  * Two kernels per layer: digits of the layer's input, then the layer.  ys[l] receives layer l's output, fp32
  * [N][layers[l].out]; ACT_SOFTMAX, allowed on the last layer only, is left to spgk_softmax_rows.
  * Needs 16-byte aligned packed rows, in <= 131072 and N <= SPGK_ISTREAM_MAX_BATCH; other nets: SPGK_E_UNSUPPORTED

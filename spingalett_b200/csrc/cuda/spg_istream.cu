@@ -8,13 +8,23 @@
 // digits, one column per digit.  Products and sums are exact in int32 (tensor memory) and int64 (recombination), so a
 // layer's only errors are the rounding to 28 bits (2^-28 of the row's maximum) and the final rounding to fp32.
 //
+// Rows of wide range.  An element below 2^-12 S keeps less than 16 bits that way, which shows in outputs whose weights on the
+// large elements are zero (a quarter of the INT4 weights of a normal draw are, most of the INT2 ones).  A row in which more
+// than an eighth of the non-zero elements are that small is a wide one: what the rounding left of its small elements is held
+// in four more digits, with the largest such remainder as scale, so they keep 28 bits of that or 56 of S, whichever is finer.
+// When a layer's input has a wide row, every k-block is multiplied with both sets of digits, into both accumulators: weights
+// and unpacking are shared.  Rows of a normal draw, of pixels, or of what the hidden activations make of them are not wide
+// (0.1 to 5 % of small elements; the most for a leaky rectifier, whose slope puts half of a row within 1 % of the other half).
+// Looking for wide rows costs 1 us of a layer (INT4 net 8192-16384-16384-8192-1000: 151 -> 156 us at 8 rows, 201 -> 204 at
+// 64); with one input of 1e6 beside ordinary ones, which makes every row of that net's layers wide: 221, 367, and 954 at 256.
+//
 // What bounds it.  HBM needs 41 us for the 272 MB of the INT4 net 8192-16384-16384-8192-1000.  A 128 x 128 block of
 // weights moves through shared memory as 8 KB packed (in and out), 16 KB of operand (in and out) and C * 128 B of digits
 // (in and out, C = 4 columns per row): 56 KB at 8 rows, 112 KB at 64 rows, 440 and 880 cycles at 128 B/clk -- 51 us and
 // 103 us over the net.  One byte per weight in the operand instead of two is why this path exists beside the 16-bit
 // streaming kernel, which writes and reads 32 KB per such block.
 //
-// Measured: 151 us at 8 rows (GEMV: 201), 207 at 64 (16-bit streaming kernel: 577), 624 at 256 (GEMM chain: 684).  About 10 us
+// Measured: 157 us at 8 rows (GEMV: 201), 211 at 64 (16-bit streaming kernel: 577), 628 at 256 (GEMM chain: 684).  About 10 us
 // of a layer are its start, staging and last sums; the rest goes at 750 cycles per 128-wide block up to 64 rows, the turn of
 // the MMA warp (two waits, four MMAs, two commits): taking out the unpacking, the digit copies or the MMAs alone leaves the
 // time within a few per cent, and so do two or eight operand slots instead of four.
@@ -55,13 +65,15 @@ constexpr double Q27 = 134217727.0;
 
 struct IsParams {
     uint32_t out, groups, rpg, N, C;                   // rows per group, batch rows, columns of a tile (4 * rpg)
+    uint32_t rows;                                     // groups * rpg: rows of scales, a quarter of the rows of one set of digits
     uint32_t kbr, boxes;                               // 128-wide k-blocks per box, boxes per row tile
     uint32_t RS, AS, BS;
     uint64_t units;                                    // tiles * boxes
     uint32_t direct; int prec, act;
     double scale; const float *bias; const double *row_scale;
+    const uint8_t *wide;
     float *y; uint32_t ldy;
-    unsigned long long *sums; uint32_t *counters; int32_t *status;
+    unsigned long long *sums, *sums2; uint32_t *counters; int32_t *status;      // sums2: of the second set of digits
     uint32_t idesc;
 };
 
@@ -73,6 +85,11 @@ __device__ __forceinline__ void umma_i8(uint32_t tmem_d, uint64_t desc_a, uint64
         "setp.ne.b32 p, %4, 0;\n\t"
         "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n\t}"
         ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(0u) : "memory");
+}
+__device__ __forceinline__ void tmem_ld4(uint32_t taddr, uint32_t (&r)[4])
+{
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(taddr) : "memory");
 }
 // int32 accumulator, A and B signed 8-bit, both K-major, M = 128, N = n
 inline uint32_t idesc_i8(uint32_t n) { return (2u << 4) | (1u << 7) | (1u << 10) | ((n >> 3) << 17) | ((128u >> 4) << 24); }
@@ -110,15 +127,83 @@ __device__ __forceinline__ uint32_t is_magnitude(const float (&f)[16])
     return m;
 }
 
+// The element as a fixed-point number: adding 1.5 * 2^52 leaves the product, rounded to an integer once, in the low word
+__device__ __forceinline__ int is_fixed(double v, double inv) { return __double2loint(fma(v, inv, 6755399441055744.0)); }
+// Elements that keep less than 16 bits: not zero and below 2^-12 of the row's maximum
+constexpr int COARSE = 1 << 15;
+
+// The four digits of 16 fixed-point numbers, at `dst` in each of four operand rows
+template <int PREC> __device__ __forceinline__ void is_store16(const int (&fixed)[16], uint8_t *dst, uint32_t ld)
+{
+    uint32_t w[4][4] = {};
+#pragma unroll
+    for (uint32_t i = 0; i < 16; i++) {
+        int v = fixed[i];
+        const uint32_t pos = is_position<PREC>(i);
+#pragma unroll
+        for (uint32_t d = 0; d < 4; d++) {
+            const int dig = d == 3 ? v : ((v + 64) & 127) - 64;
+            v = (v - dig) >> 7;
+            w[d][pos >> 2] |= ((uint32_t)dig & 0xFFu) << (8 * (pos & 3u));
+        }
+    }
+#pragma unroll
+    for (uint32_t d = 0; d < 4; d++) *reinterpret_cast<uint4 *>(dst + (uint64_t)d * ld) = make_uint4(w[d][0], w[d][1], w[d][2], w[d][3]);
+}
+
+// What the first set's rounding left of a coarse element, else 0.  Exact but for the last of 53 bits: `step` is the very
+// number that V is multiplied with later.
+__device__ __forceinline__ double is_left(float x, double inv, double step)
+{
+    const int v = is_fixed((double)x, inv);
+    return x != 0.0f && abs(v) < COARSE ? fma((double)-v, step, (double)x) : 0.0;
+}
+
+// The second set of digits of a wide row: what is left of its coarse elements, with the largest of it as scale.  Returns that
+// scale.  Short loops on purpose: code that ordinary rows never run costs them its way into the instruction cache (unrolled
+// like the first set's it took 1 us of every layer).
+template <int PREC>
+__device__ __noinline__ double is_stage_second(const float *row, uint32_t in, uint32_t ld, double inv, double step, uint8_t *dst)
+{
+    __shared__ double s_left[32];
+    const uint32_t tid = threadIdx.x;
+    double left = 0.0;
+#pragma unroll 1
+    for (uint32_t k = tid; k < in; k += STAGE_THREADS) left = fmax(left, fabs(is_left(row[k], inv, step)));
+#pragma unroll 1
+    for (int o = 16; o > 0; o >>= 1) left = fmax(left, __shfl_xor_sync(0xffffffffu, left, o));
+    if ((tid & 31u) == 0) s_left[tid >> 5] = left;
+    __syncthreads();
+#pragma unroll 1
+    for (uint32_t i = 0; i < 32; i++) left = fmax(left, s_left[i]);
+    const double inv2 = left > 0.0 ? Q27 / left : 0.0;
+#pragma unroll 1
+    for (uint32_t k = tid; k < ld; k += STAGE_THREADS) {
+        int v = k < in ? is_fixed(is_left(row[k], inv, step), inv2) : 0;
+        uint8_t *out = dst + (k & ~15u) + is_position<PREC>(k & 15u);
+#pragma unroll 1
+        for (uint32_t d = 0; d < 4; d++, out += ld) {
+            const int dig = d == 3 ? v : ((v + 64) & 127) - 64;
+            v = (v - dig) >> 7;
+            *out = (uint8_t)dig;
+        }
+    }
+    return left * (1.0 / Q27);
+}
+
 // One CTA per batch row (rows past N and k past `in` become zero digits): the row's maximum, then four digit rows of `ld`
 // bytes, 16 elements per thread and step.  64 rows of 16384: 4 MB in, 4 MB out, a few microseconds, of which the next
 // layer's first weight boxes hide some.  A row with an infinity or a NaN gets a NaN scale and zero digits.
+// row_scale: a scale per row, then a second one per row, which is zero unless the row is a wide one (else its second set of
+// digits, 4 * gridDim.x operand rows further on, is whatever it was: finite, and multiplied with zero).
+// wide: a byte per row, not zero if the row is a wide one.
 template <int PREC>
 __global__ void __launch_bounds__(STAGE_THREADS)
 spg_is_stage_kernel(const float *__restrict__ x, uint32_t ldx, uint32_t N, uint32_t in, uint32_t ld, uint32_t vec,
-                    uint8_t *__restrict__ dst, double *__restrict__ row_scale)
+                    uint8_t *__restrict__ dst, double *__restrict__ row_scale, uint8_t *__restrict__ wide)
 {
     __shared__ uint32_t s_max[32];
+    __shared__ int s_coarse[32];
     spg_grid_trigger();
     spg_grid_wait();
     const uint32_t n = blockIdx.x, tid = threadIdx.x;
@@ -139,39 +224,41 @@ spg_is_stage_kernel(const float *__restrict__ x, uint32_t ldx, uint32_t N, uint3
     const bool finite = m < 0x7F800000u;
     const double s = (double)__uint_as_float(m);
     const double inv = finite && m ? Q27 / s : 0.0;
-    if (tid == 0) row_scale[n] = finite ? s / Q27 : (double)__uint_as_float(0x7FC00000u);
+    const double step = finite ? s * (1.0 / Q27) : (double)__uint_as_float(0x7FC00000u);
     const bool zero = !live || !finite;
+    int coarse = 0;                                    // 8 per coarse element, -1 per element that is not zero
     for (uint32_t k = 16 * tid; k < ld; k += 16 * STAGE_THREADS) {
         if (k >= 16 * STAGE_THREADS) is_load16(f, row, k, live ? in : 0, vec);
-        uint32_t w[4][4] = {};
+        int fixed[16] = {};
         if (!zero) {
 #pragma unroll
             for (uint32_t i = 0; i < 16; i++) {
-                // adding 1.5 * 2^52 leaves the product, rounded to an integer once, in the low word
-                int v = __double2loint(fma((double)f[i], inv, 6755399441055744.0));
-                const uint32_t pos = is_position<PREC>(i);
-#pragma unroll
-                for (uint32_t d = 0; d < 4; d++) {
-                    const int dig = d == 3 ? v : ((v + 64) & 127) - 64;
-                    v = (v - dig) >> 7;
-                    w[d][pos >> 2] |= ((uint32_t)dig & 0xFFu) << (8 * (pos & 3u));
-                }
+                fixed[i] = is_fixed((double)f[i], inv);
+                if (f[i] != 0.0f) coarse += abs(fixed[i]) < COARSE ? 7 : -1;
             }
         }
-#pragma unroll
-        for (uint32_t d = 0; d < 4; d++)
-            *reinterpret_cast<uint4 *>(dst + (uint64_t)(4 * n + d) * ld + k) = make_uint4(w[d][0], w[d][1], w[d][2], w[d][3]);
+        is_store16<PREC>(fixed, dst + (uint64_t)(4 * n) * ld + k, ld);
     }
+    coarse = __reduce_add_sync(0xffffffffu, coarse);
+    double step2 = 0.0;
+    if (__syncthreads_or(coarse > 0)) {                // in no warp's share: not in the row either
+        if ((tid & 31u) == 0) s_coarse[tid >> 5] = coarse;
+        __syncthreads();
+        coarse = __reduce_add_sync(0xffffffffu, s_coarse[tid & 31u]);
+        if (coarse > 0) step2 = is_stage_second<PREC>(row, in, ld, inv, step, dst + (uint64_t)4 * (gridDim.x + n) * ld);
+    }
+    if (tid == 0) { row_scale[n] = step; row_scale[gridDim.x + n] = step2; wide[n] = step2 != 0.0; }
 }
 
 // ---- the layer ---------------------------------------------------------------------------------------------------------
 
 __device__ __forceinline__ void is_epi_sync() { asm volatile("bar.sync 2, %0;" ::"n"(32 * IS_EPI_WARPS) : "memory"); }
 
-__device__ __forceinline__ void is_finish(const IsParams &p, uint32_t n, uint32_t row, float bias, double scale, long long sum)
+// `rest`: bias, and the second set's share
+__device__ __forceinline__ void is_finish(const IsParams &p, uint32_t n, uint32_t row, double rest, double scale, long long sum)
 {
     if (row >= p.out || n >= p.N) return;
-    const double v = (double)sum * scale + (double)bias;
+    const double v = (double)sum * scale + rest;
     p.y[(uint64_t)n * p.ldy + row] = spg_activate((float)v, p.act);
 }
 
@@ -188,46 +275,82 @@ __device__ __forceinline__ bool is_next_segment(const IsParams &p, IsSegment &s)
     return true;
 }
 
+// The sum of four neighbouring columns: the digits of one batch row
+__device__ __forceinline__ long long is_recombine(const uint32_t *r)
+{
+    return (((long long)(int)r[3] * 128 + (int)r[2]) * 128 + (int)r[1]) * 128 + (int)r[0];
+}
+
+// Whether any row of the layer's input is a wide one (a whole warp, after the staging kernel has finished)
+__device__ __forceinline__ bool is_any_wide(const IsParams &p, uint32_t lane)
+{
+    uint32_t wide = 0;
+    for (uint32_t n = 4 * lane; n < p.rows; n += 128) wide |= __ldcg(reinterpret_cast<const uint32_t *>(p.wide + n));
+    return __any_sync(0xffffffffu, wide != 0);
+}
+
 // Epilogue role (warps 2..9): thread = one weight row (tensor-memory lane) of the tile; of two warps on the same lanes each
-// takes every other four batch rows.
-__device__ __forceinline__ void is_epilogue(const IsParams &p, IsSegment seg, uint32_t tmem_base, uint32_t tfull0, uint32_t tempty0,
+// takes every other four batch rows.  `wide`: with the second set of digits, in loops of its own (its branches and registers in
+// the others took 1 to 2 us a layer).
+__device__ __forceinline__ void is_epilogue(const IsParams &p, bool wide, IsSegment seg, uint32_t tmem_base, uint32_t tfull0, uint32_t tempty0,
                                             volatile int *abort_flag, int *s_last, double *s_scale, uint32_t warp, uint32_t lane)
 {
     const uint32_t half = (warp - 2u) >> 2, et = (warp & 3u) * 32u + lane;
     uint32_t count = 0;
-    spg_grid_wait();
     for (; is_next_segment(p, seg); count++) {
-        const uint32_t acc = count & 1u, mt = seg.tile / p.groups, n0 = (seg.tile % p.groups) * p.rpg;
+        // a wide layer's second set takes the second accumulator: no double buffering
+        const uint32_t acc = wide ? 0 : count & 1u, phase = (wide ? count : count >> 1) & 1u, mt = seg.tile / p.groups, n0 = (seg.tile % p.groups) * p.rpg;
         const bool whole = seg.k1 - seg.k0 == p.boxes;
         const uint32_t row = mt * TILE_ROWS + et;
         const float bias = row < p.out ? p.bias[row] : 0.0f;
         // the group's scales, once per segment into shared memory: a global load per value would be a chain of L2 latencies
-        if (half == 0 && et < p.rpg) s_scale[et] = __ldcg(p.row_scale + n0 + et) * p.scale;
+        if (half == 0 && et < p.rpg) {
+            s_scale[et] = __ldcg(p.row_scale + n0 + et) * p.scale;
+            if (wide) s_scale[GROUP_ROWS + et] = __ldcg(p.row_scale + p.rows + n0 + et) * p.scale;
+        }
         // the sums of a tile in pieces belong to the CTA that holds its first unit: at most one tile that goes on past the end
         // of a CTA's range starts in it
-        unsigned long long *sums = p.sums + et;
+        uint64_t slot = et;
         if (!whole) {
             const uint64_t t0 = (uint64_t)seg.tile * p.boxes;
             uint32_t c = (uint32_t)(t0 * gridDim.x / p.units);
             while (c > 0 && unit_start(p.units, gridDim.x, c) > t0) c--;
             while (unit_start(p.units, gridDim.x, c + 1) <= t0) c++;
-            sums += (uint64_t)c * p.rpg * TILE_ROWS;
+            slot += (uint64_t)c * p.rpg * TILE_ROWS;
         }
+        unsigned long long *sums = p.sums + slot, *sums2 = p.sums2 + slot;
         is_epi_sync();
-        const bool ok = mbar_wait(tfull0 + 8 * acc, (count >> 1) & 1u, abort_flag, p.status, 9);
+        const bool ok = mbar_wait(tfull0 + 8 * acc, phase, abort_flag, p.status, 9);
         tc_fence_after();
         const uint32_t taddr = tmem_base + acc * p.C + ((et & ~31u) << 16);
-        for (uint32_t c0 = 16 * half; c0 < p.C; c0 += 32) {
-            uint32_t r[16];
-            tmem_ld16(taddr + c0, r);
-            tmem_ld_wait();
-            if (!ok) continue;
+        if (!wide) {
+            for (uint32_t c0 = 16 * half; c0 < p.C; c0 += 32) {
+                uint32_t r[16];
+                tmem_ld16(taddr + c0, r);
+                tmem_ld_wait();
+                if (!ok) continue;
 #pragma unroll
-            for (uint32_t i = 0; i < 4; i++) {
-                const long long v = (((long long)(int)r[4 * i + 3] * 128 + (int)r[4 * i + 2]) * 128 + (int)r[4 * i + 1]) * 128 + (int)r[4 * i];
-                const uint32_t rr = (c0 >> 2) + i;
-                if (whole) is_finish(p, n0 + rr, row, bias, s_scale[rr], v);
-                else atomicAdd(sums + (uint64_t)rr * TILE_ROWS, (unsigned long long)v);
+                for (uint32_t i = 0; i < 4; i++) {
+                    const long long v = is_recombine(r + 4 * i);
+                    const uint32_t rr = (c0 >> 2) + i;
+                    if (whole) is_finish(p, n0 + rr, row, (double)bias, s_scale[rr], v);
+                    else atomicAdd(sums + (uint64_t)rr * TILE_ROWS, (unsigned long long)v);
+                }
+            }
+        } else {
+#pragma unroll 1
+            for (uint32_t rr = half; rr < p.rpg; rr += 2) {
+                uint32_t r[4], q[4];
+                tmem_ld4(taddr + 4 * rr, r);
+                tmem_ld4(taddr + p.C + 4 * rr, q);
+                tmem_ld_wait();
+                if (!ok) continue;
+                const long long v = is_recombine(r), v2 = is_recombine(q);
+                if (whole) is_finish(p, n0 + rr, row, (double)bias + (double)v2 * s_scale[GROUP_ROWS + rr], s_scale[rr], v);
+                else {
+                    atomicAdd(sums + (uint64_t)rr * TILE_ROWS, (unsigned long long)v);
+                    atomicAdd(sums2 + (uint64_t)rr * TILE_ROWS, (unsigned long long)v2);
+                }
             }
         }
         tc_fence_before();
@@ -242,7 +365,7 @@ __device__ __forceinline__ void is_epilogue(const IsParams &p, IsSegment seg, ui
         is_epi_sync();
         if (*s_last) {
             __threadfence();
-            for (uint32_t r0 = 4 * half; r0 < p.rpg; r0 += 32) {               // four groups of four rows in flight
+            for (uint32_t r0 = 4 * half; !wide && r0 < p.rpg; r0 += 32) {      // four groups of four rows in flight
                 long long v[16];
 #pragma unroll
                 for (uint32_t i = 0; i < 16; i++) {
@@ -254,12 +377,84 @@ __device__ __forceinline__ void is_epilogue(const IsParams &p, IsSegment seg, ui
                     const uint32_t rr = r0 + (i >> 2) * 8 + (i & 3u);
                     if (rr >= p.rpg) continue;
                     __stcg(sums + (uint64_t)rr * TILE_ROWS, 0ull);
-                    is_finish(p, n0 + rr, row, bias, s_scale[rr], v[i]);
+                    is_finish(p, n0 + rr, row, (double)bias, s_scale[rr], v[i]);
                 }
+            }
+#pragma unroll 1
+            for (uint32_t rr = half; wide && rr < p.rpg; rr += 2) {
+                const long long v = (long long)__ldcg(sums + (uint64_t)rr * TILE_ROWS), v2 = (long long)__ldcg(sums2 + (uint64_t)rr * TILE_ROWS);
+                __stcg(sums + (uint64_t)rr * TILE_ROWS, 0ull);
+                __stcg(sums2 + (uint64_t)rr * TILE_ROWS, 0ull);
+                is_finish(p, n0 + rr, row, (double)bias + (double)v2 * s_scale[GROUP_ROWS + rr], s_scale[rr], v);
             }
             if (warp == 2 && lane == 0) p.counters[seg.tile] = 0;
         }
         is_epi_sync();
+    }
+}
+
+// Digit tiles of a CTA that go out before it is known whether the layer has a wide row: one per ring slot at most.  They are
+// the first set's tiles of consecutive blocks, which is the order of a layer without wide rows; in a wide one, where the sets
+// alternate, they are thrown away.
+__device__ __forceinline__ uint32_t is_early_tiles(const IsParams &p, const IsSegment &seg)
+{
+    const uint64_t tiles = (seg.end - seg.u) * p.kbr;
+    return tiles < p.BS ? (uint32_t)tiles : p.BS;
+}
+
+// MMA role (warp 1): SETS sets of digits per 128-wide block of weights (a number known to the compiler: the warp's turn bounds
+// the kernel, and a counted loop over the sets took 3 us of the 65 that 256 rows of a 4096-4096-1024 net take)
+struct IsBars { uint32_t rfull0, rempty0, afull0, aempty0, bfull0, bempty0, tfull0, tempty0; };
+template <uint32_t SETS>
+__device__ __forceinline__ void is_mma(const IsParams &p, IsSegment seg, const IsBars &bar, uint64_t a_desc0, uint64_t b_desc0, uint32_t tmem_base,
+                                       uint32_t abort_addr, volatile int *abort_flag)
+{
+    uint32_t rs = 0, rph = 0, as = 0, aph = 0, bs = 0, bph = 0, count = 0;
+    const uint32_t b_step = p.C * 128u >> 4;
+    if (SETS == 2) {
+        const uint32_t early = is_early_tiles(p, seg);
+        for (uint32_t i = 0; i < early; i++) {
+            mbar_wait_uniform(bar.bfull0 + 8 * bs, bph, abort_addr, p.status, 10);
+            if (*abort_flag) return;
+            if (elect_one()) mbar_arrive(bar.bempty0 + 8 * bs);
+            __syncwarp();
+            if (++bs == p.BS) { bs = 0; bph ^= 1u; }
+        }
+    }
+    for (; is_next_segment(p, seg); count++) {
+        const uint32_t acc = SETS == 2 ? 0 : count & 1u, phase = (SETS == 2 ? count : count >> 1) & 1u;
+        mbar_wait_uniform(bar.tempty0 + 8 * acc, phase ^ 1u, abort_addr, p.status, 3);
+        if (*abort_flag) return;
+        tc_fence_after();
+        const uint32_t d_tmem = tmem_base + acc * p.C;
+        uint32_t accum = 0;
+        const uint32_t blocks = (seg.k1 - seg.k0) * p.kbr;
+        for (uint32_t kb = 0; kb < blocks; kb++) {
+            if (p.direct) mbar_wait_uniform(bar.rfull0 + 8 * rs, rph, abort_addr, p.status, 4);
+            else mbar_wait_uniform(bar.afull0 + 8 * as, aph, abort_addr, p.status, 5);
+            const uint64_t da = a_desc0 + (uint64_t)((p.direct ? rs : as) * (BOX_BYTES >> 4));
+#pragma unroll
+            for (uint32_t set = 0; set < SETS; set++) {
+                mbar_wait_uniform(bar.bfull0 + 8 * bs, bph, abort_addr, p.status, 6);
+                if (*abort_flag) return;
+                tc_fence_after();
+                const uint64_t db = b_desc0 + (uint64_t)(bs * b_step);
+                if (elect_one()) {
+                    uint32_t acc_in = accum;
+#pragma unroll
+                    for (uint32_t k = 0; k < 4; k++) { umma_i8(d_tmem + set * p.C, da + 2 * k, db + 2 * k, p.idesc, acc_in); acc_in = 1; }
+                    umma_commit(bar.bempty0 + 8 * bs);
+                    if (set + 1 == SETS) umma_commit(p.direct ? bar.rempty0 + 8 * rs : bar.aempty0 + 8 * as);
+                }
+                __syncwarp();
+                if (++bs == p.BS) { bs = 0; bph ^= 1u; }
+            }
+            accum = 1;
+            if (p.direct) { if (++rs == p.RS) { rs = 0; rph ^= 1u; } }
+            else if (++as == p.AS) { as = 0; aph ^= 1u; }
+        }
+        if (elect_one()) umma_commit(bar.tfull0 + 8 * acc);
+        __syncwarp();
     }
 }
 
@@ -270,7 +465,7 @@ spg_istream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     const uint32_t raw = smem_u32(is_smem_raw);
     const uint32_t base = (raw + 1023u) & ~1023u;
     uint8_t *smem = is_smem_raw + (base - raw);
-    // layout: box ring | operand ring (absent for INT8) | digit ring | barriers | flags | scales of a group
+    // layout: box ring | operand ring (absent for INT8) | digit ring | barriers | flags | scales of a group, both sets
     const uint32_t b_bytes = p.C * 128u;
     const uint32_t a_off = p.RS * BOX_BYTES;
     const uint32_t b_off = a_off + (p.direct ? 0u : p.AS * BOX_BYTES);
@@ -332,63 +527,40 @@ spg_istream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         }
     } else if (warp == IS_DIGIT_WARP) {
         // ------------------------------ digit tiles -------------------------------
-        uint32_t bs = 0, bph = 0;
+        uint32_t bs = 0, bph = 0, early = is_early_tiles(p, seg);
+        auto load = [&](uint32_t kb, uint32_t row) {
+            mbar_wait_uniform(bempty0 + 8 * bs, bph ^ 1u, abort_addr, p.status, 2);
+            if (*abort_flag) return;
+            if (elect_one()) {
+                mbar_expect_tx(bfull0 + 8 * bs, b_bytes);
+                tma_load_2d(base + b_off + bs * b_bytes, &map_x, bfull0 + 8 * bs, (int)(kb * 128u), (int)row);
+            }
+            __syncwarp();
+            if (++bs == p.BS) { bs = 0; bph ^= 1u; }
+        };
         spg_grid_wait();
+        IsSegment ahead = seg;
+        for (uint32_t left = early; left && is_next_segment(p, ahead);)
+            for (uint32_t kb = ahead.k0 * p.kbr; left && kb < ahead.k1 * p.kbr; kb++, left--) load(kb, ahead.tile % p.groups * p.C);
+        const uint32_t sets = is_any_wide(p, lane) ? 2 : 1;
+        if (sets == 2) early = 0;
         while (is_next_segment(p, seg)) {
-            const int c0 = (int)(seg.tile % p.groups * p.C);
+            const uint32_t c0 = seg.tile % p.groups * p.C;
             for (uint32_t kb = seg.k0 * p.kbr; kb < seg.k1 * p.kbr; kb++) {
-                mbar_wait_uniform(bempty0 + 8 * bs, bph ^ 1u, abort_addr, p.status, 2);
-                if (*abort_flag) goto is_role_done;
-                if (elect_one()) {
-                    mbar_expect_tx(bfull0 + 8 * bs, b_bytes);
-                    tma_load_2d(base + b_off + bs * b_bytes, &map_x, bfull0 + 8 * bs, (int)(kb * 128u), c0);
+                if (early) { early--; continue; }                              // has gone out
+                for (uint32_t set = 0; set < sets; set++) {
+                    load(kb, c0 + set * 4 * p.rows);
+                    if (*abort_flag) goto is_role_done;
                 }
-                __syncwarp();
-                if (++bs == p.BS) { bs = 0; bph ^= 1u; }
             }
         }
     } else if (warp == 1) {
         // ------------------------------ MMA issuer --------------------------------
-        uint32_t rs = 0, rph = 0, as = 0, aph = 0, bs = 0, bph = 0, count = 0;
-        const uint64_t r_desc0 = smem_desc_sw128(base), a_desc0 = smem_desc_sw128(base + a_off), b_desc0 = smem_desc_sw128(base + b_off);
-        const uint32_t b_step = b_bytes >> 4;
+        const IsBars bar = { rfull0, rempty0, afull0, aempty0, bfull0, bempty0, tfull0, tempty0 };
+        const uint64_t a_desc0 = smem_desc_sw128(p.direct ? base : base + a_off), b_desc0 = smem_desc_sw128(base + b_off);
         spg_grid_wait();
-        for (; is_next_segment(p, seg); count++) {
-            const uint32_t acc = count & 1u;
-            mbar_wait_uniform(tempty0 + 8 * acc, ((count >> 1) & 1u) ^ 1u, abort_addr, p.status, 3);
-            if (*abort_flag) goto is_role_done;
-            tc_fence_after();
-            const uint32_t d_tmem = tmem_base + acc * p.C;
-            uint32_t accum = 0;
-            const uint32_t blocks = (seg.k1 - seg.k0) * p.kbr;
-            for (uint32_t kb = 0; kb < blocks; kb++) {
-                uint64_t da;
-                if (p.direct) {
-                    mbar_wait_uniform(rfull0 + 8 * rs, rph, abort_addr, p.status, 4);
-                    da = r_desc0 + (uint64_t)(rs * (BOX_BYTES >> 4));
-                } else {
-                    mbar_wait_uniform(afull0 + 8 * as, aph, abort_addr, p.status, 5);
-                    da = a_desc0 + (uint64_t)(as * (BOX_BYTES >> 4));
-                }
-                mbar_wait_uniform(bfull0 + 8 * bs, bph, abort_addr, p.status, 6);
-                if (*abort_flag) goto is_role_done;
-                tc_fence_after();
-                const uint64_t db = b_desc0 + (uint64_t)(bs * b_step);
-                if (elect_one()) {
-#pragma unroll
-                    for (uint32_t k = 0; k < 4; k++) { umma_i8(d_tmem, da + 2 * k, db + 2 * k, p.idesc, accum); accum = 1; }
-                    umma_commit(bempty0 + 8 * bs);
-                    umma_commit(p.direct ? rempty0 + 8 * rs : aempty0 + 8 * as);
-                }
-                __syncwarp();
-                accum = 1;
-                if (++bs == p.BS) { bs = 0; bph ^= 1u; }
-                if (p.direct) { if (++rs == p.RS) { rs = 0; rph ^= 1u; } }
-                else if (++as == p.AS) { as = 0; aph ^= 1u; }
-            }
-            if (elect_one()) umma_commit(tfull0 + 8 * acc);
-            __syncwarp();
-        }
+        if (is_any_wide(p, lane)) is_mma<2>(p, seg, bar, a_desc0, b_desc0, tmem_base, abort_addr, abort_flag);
+        else is_mma<1>(p, seg, bar, a_desc0, b_desc0, tmem_base, abort_addr, abort_flag);
     } else if (warp >= IS_CONV_WARP0) {
         // ------------------------------ unpackers ---------------------------------
         // AS groups of 8 / AS warps; group g makes the operand tiles of the k-blocks whose running number is g mod AS, always
@@ -455,7 +627,15 @@ spg_istream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
             }
         }
     } else {
-        is_epilogue(p, seg, tmem_base, tfull0, tempty0, abort_flag, s_last, s_scale, warp, lane);
+        spg_grid_wait();
+        if (warp == 2) {                                  // one warp looks for all eight
+            const bool wide = is_any_wide(p, lane);
+            if (lane == 0) *s_last = wide;
+        }
+        is_epi_sync();
+        const bool wide = *s_last != 0;
+        is_epi_sync();
+        is_epilogue(p, wide, seg, tmem_base, tfull0, tempty0, abort_flag, s_last, s_scale, warp, lane);
     }
 is_role_done:
     tc_fence_before();
@@ -509,8 +689,8 @@ IsPlan is_plan(const spgk_layer *L, uint32_t N, uint32_t sms)
     const uint32_t a_bytes = pl.direct ? 0 : pl.AS * BOX_BYTES;
     pl.RS = (224u * 1024 - a_bytes - pl.BS * b_bytes) / BOX_BYTES;
     if (pl.RS > 10) pl.RS = 10;
-    pl.smem = 1024 + (size_t)pl.RS * BOX_BYTES + a_bytes + (size_t)pl.BS * b_bytes + 16 * (pl.RS + pl.AS + pl.BS) + 32 + 16 + GROUP_ROWS * sizeof(double);
-    pl.operand_bytes = (size_t)pl.groups * pl.C * pl.ld;
+    pl.smem = 1024 + (size_t)pl.RS * BOX_BYTES + a_bytes + (size_t)pl.BS * b_bytes + 16 * (pl.RS + pl.AS + pl.BS) + 32 + 16 + 2 * GROUP_ROWS * sizeof(double);
+    pl.operand_bytes = 2 * (size_t)pl.groups * pl.C * pl.ld;              // both sets of digits
     pl.ok = pl.smem <= 227u * 1024;
     return pl;
 }
@@ -544,9 +724,10 @@ int is_map(const void *ptr, uint64_t row_bytes, uint64_t rows, uint32_t box_rows
     return SPGK_OK;
 }
 
-// scratch: head | sums, one slot per CTA, of a size that depends on the device alone (they are zero between calls of any batch
-// size) | digit operand of the largest layer | row scales
-struct IsScratch { size_t sums, operand, scales, total; bool ok; };
+// scratch: head | sums, one slot per CTA and set of digits, of a size that depends on the device alone (they are zero between
+// calls of any batch size): 19.4 MB on 148 SMs | digit operand of the largest layer | row scales |
+// a byte per row
+struct IsScratch { size_t sums, sums2, operand, scales, wide, total; bool ok; };
 IsScratch is_scratch(const spgk_layer *layers, uint32_t count, uint32_t N, uint32_t sms)
 {
     IsScratch s{};
@@ -560,9 +741,11 @@ IsScratch is_scratch(const spgk_layer *layers, uint32_t count, uint32_t N, uint3
     }
     if (!rows) return s;
     s.sums = IS_HEAD;
-    s.operand = s.sums + (size_t)sms * GROUP_ROWS * TILE_ROWS * sizeof(long long);
+    s.sums2 = s.sums + (size_t)sms * GROUP_ROWS * TILE_ROWS * sizeof(long long);
+    s.operand = s.sums2 + (s.sums2 - s.sums);
     s.scales = s.operand + ((operand + 255) & ~(size_t)255);
-    s.total = s.scales + rows * sizeof(double);
+    s.wide = s.scales + 2 * rows * sizeof(double);
+    s.total = s.wide + rows;
     s.ok = true;
     return s;
 }
@@ -613,21 +796,22 @@ int spgk_istream_forward(const spgk_layer *layers, uint32_t count, const float *
         auto stage = L->precision == SPG_P_I8 ? spg_is_stage_kernel<SPG_P_I8> : L->precision == SPG_P_I4 ? spg_is_stage_kernel<SPG_P_I4> : spg_is_stage_kernel<SPG_P_I2>;
         CUtensorMap map_w, map_x;
         if ((rc = is_map(L->w, (uint64_t)L->in * spg_bits_per_elem(L->precision) / 8, L->out, TILE_ROWS, &map_w))) return rc;
-        if ((rc = is_map(operand, pl.ld, (uint64_t)pl.groups * pl.C, pl.C, &map_x))) return rc;
-        SPGK_CUDA(spg_launch_chained(stage, dim3(pl.groups * pl.rpg), dim3(STAGE_THREADS), 0, s, xin, xld, N, L->in, pl.ld, vec, operand, row_scale));
+        if ((rc = is_map(operand, pl.ld, 2 * (uint64_t)pl.groups * pl.C, pl.C, &map_x))) return rc;
+        SPGK_CUDA(spg_launch_chained(stage, dim3(pl.groups * pl.rpg), dim3(STAGE_THREADS), 0, s, xin, xld, N, L->in, pl.ld, vec, operand, row_scale, base + sc.wide));
         if ((rc = spgk_check_launch("spg_is_stage_kernel"))) return rc;
         IsParams p{};
-        p.out = L->out; p.groups = pl.groups; p.rpg = pl.rpg; p.N = N; p.C = pl.C;
+        p.out = L->out; p.groups = pl.groups; p.rpg = pl.rpg; p.N = N; p.C = pl.C; p.rows = pl.groups * pl.rpg;
         p.kbr = pl.kbr; p.boxes = pl.boxes; p.units = pl.units;
         p.RS = pl.RS; p.AS = pl.AS; p.BS = pl.BS;
         p.direct = pl.direct; p.prec = L->precision;
         p.act = L->act == SPG_ACT_SOFTMAX ? SPG_ACT_NONE : L->act;
         p.scale = (double)L->w_scale / (L->precision == SPG_P_I4 ? 16.0 : L->precision == SPG_P_I2 ? 64.0 : 1.0);
-        p.bias = L->bias; p.row_scale = row_scale;
+        p.bias = L->bias; p.row_scale = row_scale; p.wide = base + sc.wide;
         p.y = ys[l]; p.ldy = L->out;
         p.status = reinterpret_cast<int32_t *>(base);
         p.counters = reinterpret_cast<uint32_t *>(base + 256);
         p.sums = reinterpret_cast<unsigned long long *>(base + sc.sums);
+        p.sums2 = reinterpret_cast<unsigned long long *>(base + sc.sums2);
         p.idesc = idesc_i8(pl.C);
         SPGK_CUDA(spg_launch_chained(spg_istream_kernel, dim3(pl.grid), dim3(IS_THREADS), pl.smem, s, map_w, map_x, p));
         if ((rc = spgk_check_launch("spg_istream_kernel"))) return rc;

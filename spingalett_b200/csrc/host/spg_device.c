@@ -464,6 +464,7 @@ int spg_dev_forward_small(spg_net *n, const float *d_x, uint32_t ldx, uint32_t N
 #define SPG_ISTREAM_MIN_ROWS 7u
 #define SPG_ISTREAM_MAX_ROWS 256u
 #define SPG_ISTREAM_MEDIUM_BYTES ((size_t)4 << 20)      /* least packed size beyond 96 rows */
+#define SPG_ISTREAM_EXACT_ROWS 24u                      /* most rows in EXACT mode */
 
 /* The whole net on the 8-bit integer streaming kernel, for nets of integer layers that it takes (SPINGALETT_OK with
  * *d_last == NULL means that it does not take this one and nothing was launched). */
@@ -1087,13 +1088,16 @@ static float *forward_batch_on(spg_net *n, ForwardBatchArgs a)
      * rows, each group streaming the packed weights once) when every layer is eligible for the tensor-core
      * streaming kernel; everything else is the large-batch GEMM chain. */
     /* Integer files from a few rows on: the 8-bit integer streaming kernel when it takes every layer.  Measured, against the
-     * path that served before: large INT4 net 152 us against 204 (GEMV) at 8 rows, 207 against 578 (16-bit streaming kernel)
-     * at 64, 624 against 684 (GEMM chain) at 256; at 6 rows the GEMV is level (155, INT2 131), at 512 the chain is ahead
+     * path that served before: large INT4 net 157 us against 204 (GEMV) at 8 rows, 211 against 578 (16-bit streaming kernel)
+     * at 64, 628 against 684 (GEMM chain) at 256; at 6 rows the GEMV is level (155, INT2 131), at 512 the chain is ahead
      * (945).  Nets of 4 and 12 MB: 38 against 54 and 42 against 65 us at 8 rows, 0.45 of the time or less at 32 to 96,
      * 0.8 to 0.9 at 128 and 256; of 0.5 MB: 34 against 119 us at 8 rows, but no gain beyond 96.  FAST asks for one term per
-     * operand, which the GEMM chain serves beyond 96 rows. */
+     * operand, which the GEMM chain serves beyond 96 rows.  EXACT promises 16 bits of every single value, which this kernel's
+     * fixed-point numbers hold for all but the few smallest of a row: beyond 24 rows (up to there the alternative is the GEMV,
+     * whose fixed-point numbers are coarser) EXACT stays with the kernels that feed two 16-bit terms. */
+    const SpingalettMathMode mode = spingalett_get_math_mode();
     if (N >= SPG_ISTREAM_MIN_ROWS && N <= SPG_ISTREAM_MAX_ROWS && spgk_gemv_get_int_path() &&
-        (N <= 96 || spingalett_get_math_mode() != SPINGALETT_MATH_FAST)) {
+        (N <= 96 || mode != SPINGALETT_MATH_FAST) && (N <= SPG_ISTREAM_EXACT_ROWS || mode != SPINGALETT_MATH_EXACT)) {
         float *d_last = NULL;
         if (forward_istream(n, d_x, N, &d_last, out_dev ? result : NULL)) return NULL;
         if (d_last) {

@@ -2,7 +2,8 @@
 
 The bound per output is derived: an input value is rounded to a multiple of S / (2^27 - 1), S the row's largest magnitude,
 so it is off by less than S * 2^-27.9; products and sums are exact; the result is rounded to fp32 once and the activation
-function (2 ulp) is applied."""
+function (2 ulp) is applied.  In a row of wide range (more than an eighth of its non-zero values below 2^-12 S) those values
+are off by less than 2^-27.9 of the largest thing that the first rounding left of any of them."""
 import ctypes as C
 
 import numpy as np
@@ -24,19 +25,35 @@ def k(spg, has_gpu):
     return lib
 
 
-def _layer(spg, oracle, rng, out, inn, prec, act):
+def _layer(spg, oracle, rng, out, inn, prec, act, unused=None):
+    """A layer whose odd outputs take nothing from the inputs `unused`."""
     import torch
-    raw = oracle.Oracle.encode((rng.standard_normal(out * inn) / np.sqrt(inn)).astype(np.float32), prec)
-    dec = oracle.Oracle.decode(raw, out * inn, prec).astype(np.float64).reshape(out, inn)
-    scale = float(np.frombuffer(raw[:4].tobytes(), np.float32)[0]) / Q[prec]
+    vals = (rng.standard_normal((out, inn)) / np.sqrt(inn)).astype(np.float32)
+    if unused is not None:
+        vals[1::2, unused] = 0.0
+    raw = oracle.Oracle.encode(vals.ravel(), prec)
+    scale = float(np.float32(np.frombuffer(raw[:4].tobytes(), np.float32)[0] / Q[prec]))
+    # the decoded weights before their own rounding to fp32, which the bounds below leave no room for
+    dec = np.rint(oracle.Oracle.decode(raw, out * inn, prec).astype(np.float64).reshape(out, inn) / scale) * scale
     w = torch.from_numpy(np.concatenate([raw[4:], np.zeros(256, np.uint8)])).cuda()
     bias = rng.standard_normal(out).astype(np.float32) * 0.1
     b = torch.from_numpy(bias).cuda()
     return spg.abi.KLayer(w.data_ptr(), b.data_ptr(), scale, inn, out, prec, act), dec, bias, (w, b)
 
 
+def _is_wide(x):
+    """Rows of wide range, and which of their values are small ones (a value within a rounding of 2^-12 S may go either way)."""
+    s = np.abs(x).max(1, keepdims=True)
+    coarse = (x != 0) & (np.abs(x) < s * 2.0 ** -12)
+    return 8 * coarse.sum(1) > (x != 0).sum(1), coarse
+
+
 def _bound(x, dec, y):
-    return np.abs(x).max(1, keepdims=True) * 2.0 ** -27.9 * np.abs(dec).sum(1) + 4e-7 * np.abs(y) + 1e-30
+    s = np.abs(x).max(1, keepdims=True) * 2.0 ** -27.9
+    wide, coarse = _is_wide(x)
+    left = np.where(coarse, np.minimum(np.abs(x), s), 0.0).max(1, keepdims=True)
+    off = np.where(wide[:, None] & coarse, left * 2.0 ** -27.9, np.where(x != 0, s, 0.0))
+    return off @ np.abs(dec).T + 4e-7 * np.abs(y) + 1e-30
 
 
 # one row tile and ragged ones, a tile in pieces, one box and several, one group of rows and several, a padded group
@@ -46,12 +63,12 @@ def _bound(x, dec, y):
 def test_layer_against_float64(spg, k, oracle, prec, out, inn, n):
     import torch
     rng = np.random.default_rng(out * 31 + inn + n)
-    L, dec, bias, hold = _layer(spg, oracle, rng, out, inn, prec, 6)
+    L, dec, bias, hold = _layer(spg, oracle, rng, out, inn, prec, 6, unused=inn // 2)
     x = rng.standard_normal((n, inn)).astype(np.float32)
     x[0] *= 1e-30                                   # rows have scales of their own
     if n > 2:
         x[1] = 0.0
-        x[2, inn // 2] = 1e6                        # one large value: the rest of the row keeps what is left of the 28 bits
+        x[2, inn // 2] = 1e6                        # one large value, which half of the outputs do not use
     buf = torch.zeros(n * inn + 1, device="cuda")
     y = torch.full((n + 1, out), -9.0, device="cuda")
     nbytes = k.spgk_istream_scratch_bytes(C.byref(L), 1, n)
@@ -109,3 +126,66 @@ def test_what_is_declined(spg, k):
         assert k.spgk_istream_scratch_bytes(C.byref(bad), 1, 16) == 0
     pair = (spg.abi.KLayer * 2)(spg.abi.KLayer(w.data_ptr(), b.data_ptr(), 1.0, 64, 64, 4, 5), ok)      # softmax inside the net
     assert k.spgk_istream_scratch_bytes(pair, 2, 16) == 0
+
+
+# values on two and on three scales, an eighth of small ones and one more, a row of one value, next to ordinary rows
+@pytest.mark.parametrize("prec", [3, 4, 5])
+@pytest.mark.parametrize("out,inn,n", [(70, 576, 7), (500, 2048, 33), (130, 17408, 80)])
+def test_rows_of_wide_range(spg, k, oracle, prec, out, inn, n):
+    import torch
+    rng = np.random.default_rng(out + inn + n)
+    few = slice(0, 5)
+    L, dec, bias, hold = _layer(spg, oracle, rng, out, inn, prec, 6, unused=few)
+    x = rng.choice([-1.0, 1.0], (n, inn)) * rng.uniform(1.0, 2.0, (n, inn))
+    x[0, few] *= 1e7
+    x[1, few], x[1, 5:inn // 2] = x[1, few] * 1e20, x[1, 5:inn // 2] * 1e-9
+    x[2, :inn // 8] *= 1e-6                         # as many small ones as a row may have that is not a wide one
+    x[3, :inn // 8 + 1] *= 1e-6
+    x[4] = 0.0
+    x[4, 1] = -3.0
+    x[5, few] *= 1e-38                              # few small ones, denormal
+    x[6, 3] = 3e38
+    x = x.astype(np.float32)
+    wide, _ = _is_wide(x.astype(np.float64))
+    assert wide[[0, 1, 3, 6]].all() and not wide[[2, 4, 5]].any() and not wide[7:].any()
+    scratch = torch.zeros(k.spgk_istream_scratch_bytes(C.byref(L), 1, n), dtype=torch.uint8, device="cuda")
+    y = torch.zeros(n, out, device="cuda")
+    ys = (C.c_void_p * 1)(y.data_ptr())
+    for rows in (np.arange(n), np.roll(np.arange(n), 2), np.flatnonzero(~wide)):        # the last: back to ordinary rows alone
+        xr = x[rows]
+        xd = torch.from_numpy(xr).cuda()
+        assert k.spgk_istream_forward(C.byref(L), 1, xd.data_ptr(), inn, ys, len(rows), scratch.data_ptr(), None) == 0, k.spgk_error_string()
+        assert k.spgk_wstream_status(scratch.data_ptr(), None) == 0, k.spgk_error_string()
+        want = xr.astype(np.float64) @ dec.T + bias
+        err = np.abs(y.cpu().numpy()[:len(rows)] - want)
+        assert np.all(err <= _bound(xr.astype(np.float64), dec, want)), err.max(1)
+
+
+@pytest.mark.parametrize("mode", ["auto", "exact"])
+@pytest.mark.parametrize("n", [8, 25, 64, 200])
+def test_one_large_input_that_has_no_weight(spg, has_gpu, tmp_path, mode, n):
+    """One input of 1e3 to 1e30 beside 4095 ordinary ones; every weight on it is zero.  The other inputs have to keep the 16
+    bits that two bf16 terms hold (each off by less than 2^-18 of itself, independently): 8 standard deviations of their sum, and
+    2^-24 of a partial sum of ordinary size for each time a tensor core adds 16 products to it (twice 4096 products in EXACT)."""
+    a = spg.abi
+    topo = [4096, 2048]
+    net = spg.Network.build(topo, [a.ACT_LEAKY_RELU], a.WEIGHT_INITIALIZATION_HE, seed=11)
+    w = net.weights.reshape(topo[1], topo[0])
+    w[:, 77] = 0.0
+    net.save(str(tmp_path / "m.nn"), a.PRECISION_INT4)
+    net.free()
+    net = spg.Network.load(str(tmp_path / "m.nn"))
+    w, b = net.weights.reshape(topo[1], topo[0]).astype(np.float64), net.biases.astype(np.float64)
+    assert not w[:, 77].any()
+    x = np.random.default_rng(n).standard_normal((n, topo[0])).astype(np.float32)
+    x[:, 77] = 10.0 ** (3 + np.arange(n) % 28)
+    spg.set_math_mode(a.MATH_AUTO if mode == "auto" else a.MATH_EXACT)
+    try:
+        got = net.forward_batch(x)
+    finally:
+        spg.set_math_mode(a.MATH_AUTO)
+    z = x.astype(np.float64) @ w.T + b
+    tol = (8 * 2.0 ** -18 + 2 * 4096 / 16 * 2.0 ** -24) * np.sqrt((x.astype(np.float64) ** 2 * (np.arange(topo[0]) != 77)) @ (w ** 2).T)
+    err = np.abs(got - np.where(z > 0, z, 0.01 * z))
+    assert np.all(err <= tol), (err / tol).max(1)
+    net.free()
