@@ -20,7 +20,7 @@ no collective), so scaling is weak: `value` is all ranks' rows per second.
   roofline  the dominant kernel of the path that ran (config.path): the one-launch
             three-layer kernel or the per-layer tcgen05 GEMM -- algorithmic FLOPs of
             its launches / their summed device time (event pairs recorded by the
-            library around each launch), against the measured bf16 peak; the GEMV or
+            library around each launch), against the measured bf16 peak; the GEMV or a
             weight-streaming kernel for small batches -- packed weight bytes / time,
             against the measured HBM bandwidth
   cpu_baseline  the reference's own CPU forward (built from its sources into
@@ -71,6 +71,19 @@ def algorithmic_bytes(topo, dtype, batch):
     return total + batch * topo[0] * 4 + batch * topo[-1] * 4
 METRIC = "mlp_forward_samples_per_sec"
 PRECS = ["fp32", "fp16", "bf16", "int8", "int4", "int2"]
+
+
+def arithmetic(path, dtype, math):
+    """What the path that ran (spingalett_last_path) computes with."""
+    if path == "istream" or path == "gemv" and dtype in ("int8", "int4", "int2"):
+        return "s8 digits x s8 -> s32 (exact sums of 28-bit fixed-point activations)"
+    if path in ("gemv", "wstream"):
+        return "bf16 terms x bf16 -> f32 (exact products)"
+    return {"exact": "bf16(hi+lo)xbf16->f32", "fast": "f16xf16->f32", "auto": "f16xf16->f32 + exact recompute of low-margin rows"}[math]
+
+
+KERNEL_OF_PATH = {"gemv": "spg_gemv_kernel", "istream": "spg_istream_kernel", "wstream": "spg_wstream_kernel", "tcgen05": "spg_gemm_tc_kernel",
+                  "tcgen05-fused": "spg_mlp3_fused_kernel", "simt": "spg_layer_simt_kernel"}
 
 
 def parse():
@@ -540,11 +553,7 @@ def main():
     value = batch * world / (dev_ms * 1e-3)
     e2e_value = batch * world / (e2e_ms * 1e-3)
     passes = 2 if args.math == "exact" else 1
-    compute = {"exact": "bf16(hi+lo)xbf16->f32", "fast": "f16xf16->f32", "auto": "f16xf16->f32 + exact recompute of low-margin rows"}[args.math]
-    if path_taken == "gemv" and args.dtype in ("int8", "int4", "int2"):
-        compute = "s8 digits x s8 -> s32 (exact sums of 28-bit fixed-point activations)"
-    elif path_taken in ("gemv", "wstream"):
-        compute = "bf16 terms x bf16 -> f32 (exact products)"
+    compute = arithmetic(path_taken, args.dtype, args.math)
     line = {
         "metric": METRIC, "value": value, "unit": "samples/s", "n_gpus": world, "steps": args.steps, "warmup": max(3, args.warmup),
         "ms_per_step": dev_ms, "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
@@ -571,7 +580,7 @@ def main():
             traffic = json.load(open(tpath)).get(f"{args.workload}_{args.dtype}_{args.math}_{batch}")
         line["roofline"] = {"bound": "tensor", "achieved": achieved, "peak": pk["bf16_tflops"], "unit": "TFLOP/s",
                             "frac": achieved / pk["bf16_tflops"], "traffic": traffic,
-                            "kernel": "spg_mlp3_fused_kernel" if fused else "spg_gemm_tc_kernel",
+                            "kernel": KERNEL_OF_PATH[path_taken],
                             "launches": int(k_cnt), "kernel_ms_per_step": k_ms_eff / args.steps,
                             "peak_source": pk["source"] + " burst bf16", "tensor_passes_per_product": passes,
                             "executed_frac": achieved * passes / pk["bf16_tflops"],
@@ -585,15 +594,18 @@ def main():
         achieved = nbytes * args.steps / (k_ms * 1e-3) / 1e9
         traffic = None
         tpath = os.path.join(ROOT, "profiles", "gemv_traffic.json")
-        if os.path.exists(tpath):
+        if path_taken == "gemv" and os.path.exists(tpath):
             traffic = json.load(open(tpath)).get(f"{args.workload}_{args.dtype}_{batch}")
         line["roofline"] = {"bound": "hbm", "achieved": achieved, "peak": pk["hbm_gbs"], "unit": "GB/s",
                             "frac": achieved / pk["hbm_gbs"], "traffic": traffic,
-                            "kernel": "spg_wstream_kernel" if path_taken == "wstream" else "spg_gemv_kernel",
+                            "kernel": KERNEL_OF_PATH[path_taken],
                             "launches": int(k_cnt), "kernel_ms_per_step": k_ms / args.steps,
                             "algorithmic_bytes_per_step": nbytes, "peak_source": pk["source"] + " copy bandwidth",
                             "whole_step_frac": nbytes / (dev_ms * 1e-3) / 1e9 / pk["hbm_gbs"],
-                            "note": "frac: event pairs around each layer kernel in a separate pass (events keep a layer from "
+                            "note": "frac: the packed weights once per step over an event pair around the staging and layer kernels of all "
+                                    "layers; the weights are streamed once per 64 rows"
+                                    if path_taken == "istream" else
+                                    "frac: event pairs around each layer kernel in a separate pass (events keep a layer from "
                                     "prefetching weights under the previous one); whole_step_frac: algorithmic bytes / ms_per_step "
                                     "of the timed loop, staging and softmax included"}
     if (args.all_dtypes or args.workload == "mlp") and not args.one_dtype:

@@ -237,11 +237,12 @@ SPGK_API int spgk_wstream_status(void *scratch, void *stream);
  * (and spgk_istream_scratch_bytes returns 0).
  * scratch: spgk_istream_scratch_bytes bytes, ZERO-FILLED before first use (status word, counters and sums are left at
  * zero, at places that do not depend on N); after a failure that the status reports, zero-filled again.
- * spgk_wstream_status reads its status. */
+ * spgk_istream_status waits for the stream and reads its status. */
 #define SPGK_ISTREAM_MAX_BATCH 512
 SPGK_API size_t spgk_istream_scratch_bytes(const spgk_layer *layers, uint32_t count, uint32_t N);
 SPGK_API int spgk_istream_forward(const spgk_layer *layers, uint32_t count, const float *x, uint32_t ldx, float *const *ys,
                                   uint32_t N, void *scratch, void *stream);
+SPGK_API int spgk_istream_status(void *scratch, void *stream);
 
 /* ---- K2: large-batch tcgen05 GEMM layer ----------------------------------
  * C[N][out] = act(bias + w_scale * A[N][in] * W^T) with the accumulator in

@@ -820,4 +820,19 @@ int spgk_istream_forward(const spgk_layer *layers, uint32_t count, const float *
     return SPGK_OK;
 }
 
+int spgk_istream_status(void *scratch, void *stream)
+{
+    int32_t h = 0;
+    SPGK_CUDA(cudaMemcpyAsync(&h, scratch, sizeof h, cudaMemcpyDeviceToHost, (cudaStream_t)stream));
+    SPGK_CUDA(cudaStreamSynchronize((cudaStream_t)stream));
+    if (h != 0) {
+        char msg[96];
+        snprintf(msg, sizeof msg, "bounded wait %d gave up inside the integer streaming kernel", (int)h);
+        spgk_set_error("spg_istream_kernel", msg);
+        SPGK_CUDA(cudaMemsetAsync(scratch, 0, sizeof h, (cudaStream_t)stream));
+        return SPGK_E_TIMEOUT;
+    }
+    return SPGK_OK;
+}
+
 }  // extern "C"

@@ -232,7 +232,7 @@ static int finish(spg_net *n)
     }
     if (n->is_pending) {
         n->is_pending = false;
-        if ((rc = spg_map_kernel_error(spgk_wstream_status(n->d_is_scratch, n->stream), "integer-stream kernel"))) {
+        if ((rc = spg_map_kernel_error(spgk_istream_status(n->d_is_scratch, n->stream), "integer-stream kernel"))) {
             spgk_free(n->d_is_scratch); n->d_is_scratch = NULL; n->is_scratch_bytes = 0;      /* its counters may be off zero */
             return rc;
         }
@@ -496,8 +496,7 @@ static int forward_istream(spg_net *n, const float *d_x, uint32_t N, float **d_l
     const spgk_layer *Ll = &n->klayers[n->dev_layers - 1];
     float *y = ys[n->dev_layers - 1];
     if (Ll->act == ACT_SOFTMAX && (rc = spg_map_kernel_error(spgk_softmax_rows(y, Ll->out, N, Ll->out, n->stream), "softmax"))) return rc;
-    /* the name of the family that serves this many rows */
-    spg_note_path(N <= 3 * SPGK_GEMV_MAX_BATCH ? "gemv" : N <= 96 ? "wstream" : "tcgen05");
+    spg_note_path("istream");
     *d_last = y;
     return SPINGALETT_OK;
 }

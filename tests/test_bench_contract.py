@@ -41,6 +41,13 @@ def test_reference_arm_runs_on_rank_zero_only():
     assert r.returncode == 0 and r.stdout.strip() == ""
 
 
+def test_the_line_names_what_the_path_runs():
+    import bench
+    for path, kernel, dtype in (("istream", "spg_istream_kernel", "s8 digits"), ("wstream", "spg_wstream_kernel", "bf16 terms"),
+                                ("gemv", "spg_gemv_kernel", "s8 digits"), ("tcgen05", "spg_gemm_tc_kernel", "f16xf16")):
+        assert bench.KERNEL_OF_PATH[path] == kernel and bench.arithmetic(path, "int4", "auto").startswith(dtype)
+
+
 def test_defaults_follow_the_workload():
     sys.path.insert(0, ROOT)
     import bench

@@ -78,14 +78,15 @@ def test_wide_bf16_mlp_batch_16384(spg, w_net, mode):
         spg.set_math_mode(spg.abi.MATH_AUTO)
 
 
-@pytest.mark.parametrize("n", [1, 8, 20, 64, 128, 256])
+@pytest.mark.parametrize("n", [1, 6, 8, 20, 64, 128, 256])
 def test_large_int4_mlp_batch_sweep(spg, l_net, n):
     net, onet = l_net
     x = nets.normal_inputs(n, nets.L_TOPO[0], seed=100 + n)
     spg.set_math_mode(spg.abi.MATH_EXACT)
     got = net.forward_batch(x)
-    # 9..24 rows: GEMV in groups of 8; up to 96 rows: one pass of the streaming kernel; beyond: the GEMM chain on kept operands
-    assert spg.last_path() == ("gemv" if n <= 24 else "wstream" if n <= 96 else "tcgen05")
+    # up to 6 rows: GEMV; up to 24 (in EXACT): the integer streaming kernel; up to 96: the 16-bit streaming kernel; beyond: the
+    # GEMM chain on kept operands
+    assert spg.last_path() == ("gemv" if n <= 6 else "istream" if n <= 24 else "wstream" if n <= 96 else "tcgen05")
     rows = np.arange(n) if n <= 64 else np.random.default_rng(2).choice(n, 64, replace=False)
     want = onet.forward_batch(x[rows])
     agree, err = nets.parity(got[rows], want)
@@ -95,7 +96,7 @@ def test_large_int4_mlp_batch_sweep(spg, l_net, n):
         one = net.forward(x[0])                                  # the reference's single-sample entry point
         assert np.abs(one - want[0]).max() <= 2e-5
     if n <= 24:
-        # the integer-digit GEMV (default for integer files) against the bf16-term GEMV on the whole chain
+        # the integer kernels (GEMV up to 6 rows, streaming kernel beyond) against the bf16-term GEMV on the whole chain
         lib = spg.lib()
         lib.spgk_gemv_set_int_path(0)
         try:

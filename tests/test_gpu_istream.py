@@ -20,7 +20,7 @@ def k(spg, has_gpu):
     lib.spgk_istream_scratch_bytes.argtypes = [C.POINTER(spg.abi.KLayer), C.c_uint32, C.c_uint32]
     lib.spgk_istream_scratch_bytes.restype = C.c_size_t
     lib.spgk_istream_forward.argtypes = [C.POINTER(spg.abi.KLayer), C.c_uint32, vp, C.c_uint32, C.POINTER(vp), C.c_uint32, vp, vp]
-    lib.spgk_wstream_status.argtypes = [vp, vp]
+    lib.spgk_istream_status.argtypes = [vp, vp]
     lib.spgk_error_string.restype = C.c_char_p
     return lib
 
@@ -80,7 +80,7 @@ def test_layer_against_float64(spg, k, oracle, prec, out, inn, n):
         buf[off:off + n * inn] = torch.from_numpy(x.ravel()).cuda()
         y.fill_(-9.0)
         assert k.spgk_istream_forward(C.byref(L), 1, buf.data_ptr() + 4 * off, inn, ys, n, scratch.data_ptr(), None) == 0, k.spgk_error_string()
-        assert k.spgk_wstream_status(scratch.data_ptr(), None) == 0, k.spgk_error_string()
+        assert k.spgk_istream_status(scratch.data_ptr(), None) == 0, k.spgk_error_string()
         got = y.cpu().numpy()
         assert np.all(got[n] == -9.0)
         assert np.all(np.abs(got[:n] - want) <= _bound(x.astype(np.float64), dec, want)), np.abs(got[:n] - want).max()
@@ -100,7 +100,7 @@ def test_chain_and_rows_that_are_not_finite(spg, k, oracle, precs):
     scratch = torch.zeros(k.spgk_istream_scratch_bytes(Ls, 3, n), dtype=torch.uint8, device="cuda")
     xd = torch.from_numpy(x).cuda()
     assert k.spgk_istream_forward(Ls, 3, xd.data_ptr(), topo[0], ys, n, scratch.data_ptr(), None) == 0, k.spgk_error_string()
-    assert k.spgk_wstream_status(scratch.data_ptr(), None) == 0, k.spgk_error_string()
+    assert k.spgk_istream_status(scratch.data_ptr(), None) == 0, k.spgk_error_string()
     good = np.isfinite(x).all(1)
     a = x.astype(np.float64)
     for t, (_, dec, bias, _), act in zip(ys_t, built, acts):
@@ -155,7 +155,7 @@ def test_rows_of_wide_range(spg, k, oracle, prec, out, inn, n):
         xr = x[rows]
         xd = torch.from_numpy(xr).cuda()
         assert k.spgk_istream_forward(C.byref(L), 1, xd.data_ptr(), inn, ys, len(rows), scratch.data_ptr(), None) == 0, k.spgk_error_string()
-        assert k.spgk_wstream_status(scratch.data_ptr(), None) == 0, k.spgk_error_string()
+        assert k.spgk_istream_status(scratch.data_ptr(), None) == 0, k.spgk_error_string()
         want = xr.astype(np.float64) @ dec.T + bias
         err = np.abs(y.cpu().numpy()[:len(rows)] - want)
         assert np.all(err <= _bound(xr.astype(np.float64), dec, want)), err.max(1)
