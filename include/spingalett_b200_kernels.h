@@ -236,7 +236,8 @@ SPGK_API int spgk_wstream_status(void *scratch, void *stream);
  * Needs 16-byte aligned packed rows, in <= 131072 and N <= SPGK_ISTREAM_MAX_BATCH; other nets: SPGK_E_UNSUPPORTED
  * (and spgk_istream_scratch_bytes returns 0).
  * scratch: spgk_istream_scratch_bytes bytes, ZERO-FILLED before first use (status word, counters and sums are left at
- * zero, at places that do not depend on N); after a failure that the status reports, zero-filled again.
+ * zero, at places that do not depend on N); after a failure that the status reports, zero-filled again.  Until the
+ * status has been read, every output after the failure is NaN.
  * spgk_istream_status waits for the stream and reads its status. */
 #define SPGK_ISTREAM_MAX_BATCH 512
 SPGK_API size_t spgk_istream_scratch_bytes(const spgk_layer *layers, uint32_t count, uint32_t N);

@@ -291,8 +291,9 @@ __device__ __forceinline__ bool is_any_wide(const IsParams &p, uint32_t lane)
 
 // Epilogue role (warps 2..9): thread = one weight row (tensor-memory lane) of the tile; of two warps on the same lanes each
 // takes every other four batch rows.  `wide`: with the second set of digits, in loops of its own (its branches and registers in
-// the others took 1 to 2 us a layer).
-__device__ __forceinline__ void is_epilogue(const IsParams &p, bool wide, IsSegment seg, uint32_t tmem_base, uint32_t tfull0, uint32_t tempty0,
+// the others took 1 to 2 us a layer).  `dirty`: a launch before this one failed and nobody has read its status yet, so the sums and
+// counters cannot be relied on.
+__device__ __forceinline__ void is_epilogue(const IsParams &p, bool wide, bool dirty, IsSegment seg, uint32_t tmem_base, uint32_t tfull0, uint32_t tempty0,
                                             volatile int *abort_flag, int *s_last, double *s_scale, uint32_t warp, uint32_t lane)
 {
     const uint32_t half = (warp - 2u) >> 2, et = (warp & 3u) * 32u + lane;
@@ -320,7 +321,7 @@ __device__ __forceinline__ void is_epilogue(const IsParams &p, bool wide, IsSegm
         }
         unsigned long long *sums = p.sums + slot, *sums2 = p.sums2 + slot;
         is_epi_sync();
-        const bool ok = mbar_wait(tfull0 + 8 * acc, phase, abort_flag, p.status, 9);
+        const bool ok = mbar_wait(tfull0 + 8 * acc, phase, abort_flag, p.status, 9) && !dirty;
         tc_fence_after();
         const uint32_t taddr = tmem_base + acc * p.C + ((et & ~31u) << 16);
         if (!wide) {
@@ -355,12 +356,19 @@ __device__ __forceinline__ void is_epilogue(const IsParams &p, bool wide, IsSegm
         }
         tc_fence_before();
         mbar_arrive(tempty0 + 8 * acc);                 // the accumulator may be overwritten
-        if (whole) { is_epi_sync(); continue; }         // (the scales of the next segment may replace these)
-        __threadfence();
-        is_epi_sync();
+        if (!whole) __threadfence();
+        is_epi_sync();                                  // (also: the scales of the next segment may replace these)
+        const bool failed = !ok || *abort_flag;
+        if (failed) {
+            // a wait gave up, here or before: nothing in the output that could pass for a result
+#pragma unroll 1
+            for (uint32_t rr = half; rr < p.rpg; rr += 2)
+                if (row < p.out && n0 + rr < p.N) p.y[(uint64_t)(n0 + rr) * p.ldy + row] = __uint_as_float(0x7FC00000u);
+        }
+        if (whole) continue;
         if (warp == 2 && lane == 0) {
             const uint32_t part = seg.k1 - seg.k0;
-            *s_last = ok && atomicAdd(&p.counters[seg.tile], part) + part == p.boxes;
+            *s_last = !failed && atomicAdd(&p.counters[seg.tile], part) + part == p.boxes;
         }
         is_epi_sync();
         if (*s_last) {
@@ -629,13 +637,14 @@ spg_istream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     } else {
         spg_grid_wait();
         if (warp == 2) {                                  // one warp looks for all eight
+            const int32_t failed = __ldcg(p.status);      // by an earlier launch: its sums and counters are still about
             const bool wide = is_any_wide(p, lane);
-            if (lane == 0) *s_last = wide;
+            if (lane == 0) *s_last = (wide ? 1 : 0) | (failed ? 2 : 0);
         }
         is_epi_sync();
-        const bool wide = *s_last != 0;
+        const int found = *s_last;
         is_epi_sync();
-        is_epilogue(p, wide, seg, tmem_base, tfull0, tempty0, abort_flag, s_last, s_scale, warp, lane);
+        is_epilogue(p, found & 1, found & 2, seg, tmem_base, tfull0, tempty0, abort_flag, s_last, s_scale, warp, lane);
     }
 is_role_done:
     tc_fence_before();

@@ -114,6 +114,33 @@ def test_chain_and_rows_that_are_not_finite(spg, k, oracle, precs):
         a = got.astype(np.float64)
 
 
+@pytest.mark.parametrize("n", [1, 70])
+def test_outputs_after_a_failure_are_nan_until_its_status_is_read(spg, k, oracle, n):
+    """The status word a failed launch leaves (set here by the host): what its sums and counters hold must not come out as a
+    result, not even through a rectifier, in any layer."""
+    import torch
+    rng = np.random.default_rng(n)
+    topo = [256, 4096, 300]
+    built = [_layer(spg, oracle, rng, o, i, 4, 1) for i, o in zip(topo, topo[1:])]
+    Ls = (spg.abi.KLayer * 2)(*[b[0] for b in built])
+    x = torch.from_numpy(rng.standard_normal((n, topo[0])).astype(np.float32)).cuda()
+    ys_t = [torch.zeros(n + 1, o, device="cuda") for o in topo[1:]]
+    ys = (C.c_void_p * 2)(*[t.data_ptr() for t in ys_t])
+    scratch = torch.zeros(k.spgk_istream_scratch_bytes(Ls, 2, n), dtype=torch.uint8, device="cuda")
+    scratch[0] = 9
+    for _ in range(2):
+        assert k.spgk_istream_forward(Ls, 2, x.data_ptr(), topo[0], ys, n, scratch.data_ptr(), None) == 0, k.spgk_error_string()
+        torch.cuda.synchronize()
+        for t in ys_t:
+            assert bool(t[:n].isnan().all()) and not bool(t[n].any())
+            t.zero_()
+    assert k.spgk_istream_status(scratch.data_ptr(), None) == -4 and b"bounded wait 9 gave up inside the integer" in k.spgk_error_string()
+    scratch.zero_()
+    assert k.spgk_istream_forward(Ls, 2, x.data_ptr(), topo[0], ys, n, scratch.data_ptr(), None) == 0, k.spgk_error_string()
+    assert k.spgk_istream_status(scratch.data_ptr(), None) == 0
+    assert all(bool(t[:n].isfinite().all()) for t in ys_t)
+
+
 def test_what_is_declined(spg, k):
     import torch
     w, b = torch.zeros(1 << 16, dtype=torch.uint8, device="cuda"), torch.zeros(64, device="cuda")
