@@ -221,9 +221,8 @@ fail:
 static void prof_collect(spg_net *n);
 static void prof_mark(spg_net *n);
 
-/* Wait for the net's stream, then surface a bounded-wait failure reported by a
- * tensor-core kernel and fold the timing events in. */
-static int finish(spg_net *n)
+/* Waits for the small-batch kernels whose status words have not been read yet and surfaces a bounded-wait failure. */
+static int settle_small(spg_net *n)
 {
     int rc;
     if (n->ws_pending) {
@@ -241,6 +240,15 @@ static int finish(spg_net *n)
         n->gemv_pending = false;
         if ((rc = spg_map_kernel_error(spgk_gemv_status(n->d_gemv_scratch, n->stream), "GEMV"))) return rc;
     }
+    return SPINGALETT_OK;
+}
+
+/* Wait for the net's stream, then surface a bounded-wait failure reported by a
+ * tensor-core kernel and fold the timing events in. */
+static int finish(spg_net *n)
+{
+    int rc = settle_small(n);
+    if (rc) return rc;
     if (n->status_pending) {
         n->status_pending = false;
         if ((rc = spg_map_kernel_error(spgk_gemm_tc_status(n->d_status, n->stream), "tcgen05 GEMM"))) return rc;
@@ -338,11 +346,14 @@ static int reserve(void **buf, size_t *have, size_t need, const char *what)
 /* small-batch chain                                                         */
 /* ------------------------------------------------------------------------ */
 
-/* device buffer that must start zero-filled (status words, ticket counters) */
+/* device buffer that must start zero-filled (status words, ticket counters); a status that nobody has read yet goes to the
+ * caller before the buffer it lies in is replaced */
 static int reserve_zeroed(spg_net *n, void **buf, size_t *have, size_t need, const char *what)
 {
     if (!need || (*have >= need && *buf)) return SPINGALETT_OK;
-    int rc = reserve(buf, have, need, what);
+    int rc = *buf ? settle_small(n) : SPINGALETT_OK;
+    if (rc) return rc;
+    rc = reserve(buf, have, need, what);
     if (rc) return rc;
     return spg_map_kernel_error(spgk_memset(*buf, 0, need, n->stream), what);
 }

@@ -371,3 +371,23 @@ def test_row_shares_of_the_device_fan_out_cover_the_batch_once(spg):
             assert max(sizes) - min(sizes) <= 1
             assert spans == [spg.shard_rows(rows, shares, g) for g in range(shares)]
     assert lib.spingalett_set_devices(None, 0) == 0
+
+
+def test_a_failure_is_reported_when_its_status_buffer_is_replaced(tmp_path):
+    """tests/c/unread_status.c: the library's host sources on fake kernels."""
+    import re
+    import subprocess
+    host = os.path.join(ROOT, "spingalett_b200", "csrc", "host")
+    objs = []
+    for src in sorted(f for f in os.listdir(host) if f.endswith(".c")) + [os.path.join(ROOT, "tests", "c", "unread_status.c")]:
+        objs.append(str(tmp_path / (os.path.basename(src) + ".o")))
+        subprocess.run(["gcc", "-std=c2x", "-O1", "-D_GNU_SOURCE", "-I", os.path.join(ROOT, "include"), "-I", host, "-c", os.path.join(host, src),
+                        "-o", objs[-1]], check=True)
+    names = subprocess.run(["nm"] + objs, capture_output=True, text=True, check=True).stdout
+    missing = set(re.findall(r" U (spgk?_\w+)", names)) - set(re.findall(r" [TtDBbCR] (spgk?_\w+)", names))
+    stubs = tmp_path / "stubs.c"
+    stubs.write_text("".join(f"long {name}(void) {{ return 0; }}\n" for name in sorted(missing)))
+    exe = str(tmp_path / "unread_status")
+    subprocess.run(["gcc", "-std=c2x", "-O1", *objs, str(stubs), "-o", exe, "-lpthread", "-ldl", "-lm"], check=True)
+    r = subprocess.run([exe, str(tmp_path / "net.nn")], capture_output=True, text=True, timeout=60)
+    assert r.returncode == 0 and r.stdout.endswith("reported\n"), (r.returncode, r.stdout, r.stderr)
