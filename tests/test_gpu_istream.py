@@ -216,3 +216,79 @@ def test_one_large_input_that_has_no_weight(spg, has_gpu, tmp_path, mode, n):
     err = np.abs(got - np.where(z > 0, z, 0.01 * z))
     assert np.all(err <= tol), (err / tol).max(1)
     net.free()
+
+
+def _loaded(spg, tmp_path, topo, acts, prec, seed=3):
+    net = spg.Network.build(topo, acts, spg.abi.WEIGHT_INITIALIZATION_HE, seed=seed)
+    net.save(str(tmp_path / "m.nn"), prec)
+    net.free()
+    return spg.Network.load(str(tmp_path / "m.nn"))
+
+
+@pytest.mark.parametrize("prec", [3, 4, 5])
+def test_one_net_over_batches_of_changing_size(spg, has_gpu, tmp_path, prec):
+    """The counters and sums of a net's scratch are at zero after every call, wherever the next batch's plan looks for them: a
+    sequence that grows, shrinks, changes the number of groups and meets wide rows in between, on host and device buffers.
+    Bound: both layers' 28 bits and fp32 rounding, eight deviations of the sums of independent errors."""
+    import torch
+    a = spg.abi
+    topo = [4096, 4096, 130]
+    net = _loaded(spg, tmp_path, topo, [a.ACT_RELU, a.ACT_LEAKY_RELU], prec)
+    w = [torch.from_numpy(v.astype(np.float64)).cuda() for v in np.split(net.weights, [topo[0] * topo[1]])]
+    b = [torch.from_numpy(v.astype(np.float64)).cuda() for v in np.split(net.biases, [topo[1]])]
+    w = [v.view(o, i) for v, i, o in zip(w, topo, topo[1:])]
+    net.set_stream(torch.cuda.current_stream().cuda_stream)
+    for step, n in enumerate([200, 7, 65, 8, 256, 33, 200, 96, 97]):
+        x = torch.randn(n, topo[0], generator=torch.Generator("cuda").manual_seed(n + step), device="cuda")
+        if step in (2, 5):
+            x[n // 2, 9] = 1e5
+        if step % 2:
+            got = torch.from_numpy(net.forward_batch(x.cpu().numpy())).cuda()
+        else:
+            got = torch.empty(n, topo[-1], device="cuda")
+            net.forward_batch_ptr(x.data_ptr(), n, got.data_ptr())
+            net.synchronize()
+        assert spg.last_path() == "istream"
+        h, tol = x.double(), torch.zeros_like(x, dtype=torch.float64)
+        for w_, b_, slope in zip(w, b, (0.0, 0.01)):
+            z, w2 = h @ w_.T + b_, (w_ ** 2).T
+            fixed = h.abs().amax(1, keepdim=True) * 2.0 ** -27.9 * w2.sum(0).sqrt()
+            # tol: of one value so far, eight deviations; the second term is the rounding of the weights compared with to fp32
+            tol = 8 * (fixed + 2.0 ** -24 * (h ** 2 @ w2).sqrt()) + (tol ** 2 @ w2).sqrt() + 4e-7 * z.abs()
+            h = torch.where(z > 0, z, slope * z)
+        err = (got.double() - h).abs()
+        assert bool((err <= tol + 1e-30).all()), (step, n, float((err / tol).max()))
+    net.free()
+
+
+def test_the_rows_widths_and_modes_that_take_the_path(spg, has_gpu, tmp_path):
+    """Just inside and just outside of every line that the dispatch draws."""
+    a, lib = spg.abi, spg.lib()
+    modes = {"auto": a.MATH_AUTO, "exact": a.MATH_EXACT, "fast": a.MATH_FAST}
+    small, medium, less = [128, 64, 10], [4096, 2048], [4096, 2047]                  # 4 MB of INT4, and not quite
+    soft = [a.ACT_RELU, a.ACT_SOFTMAX]
+    for topo, acts, prec, rows in [
+            (small, soft, 3, {("auto", 6): 0, ("auto", 7): 1, ("auto", 96): 1, ("auto", 97): 0, ("exact", 24): 1, ("exact", 25): 0, ("fast", 96): 1}),
+            (small, soft, 4, {("auto", 7): 1}), (small, soft, 5, {("auto", 7): 1}), (small, soft, 1, {("auto", 7): 0}), (small, soft, 0, {("auto", 7): 0}),
+            (medium, soft[1:], 4, {("auto", 97): 1, ("auto", 256): 1, ("auto", 257): 0, ("exact", 97): 0, ("fast", 97): 0}),
+            (less, soft[1:], 4, {("auto", 96): 1, ("auto", 97): 0}),
+            ([72, 64, 10], soft, 4, {("auto", 16): 0}),                                 # packed rows of 36 bytes
+            ([128, 72, 10], soft, 4, {("auto", 16): 0}),                                # the same, in the second layer
+            (small, [a.ACT_SOFTMAX, a.ACT_SOFTMAX], 4, {("auto", 16): 0})]:
+        net = _loaded(spg, tmp_path, topo, acts, prec)
+        for (mode, n), takes in rows.items():
+            spg.set_math_mode(modes[mode])
+            try:
+                y = net.forward_batch(np.random.default_rng(n).standard_normal((n, topo[0])).astype(np.float32))
+            finally:
+                spg.set_math_mode(a.MATH_AUTO)
+            assert (spg.last_path() == "istream") == bool(takes), (topo, prec, mode, n, spg.last_path())
+            assert np.all(np.isfinite(y))
+            if takes and n == 7:
+                lib.spgk_gemv_set_int_path(0)
+                try:
+                    other = net.forward_batch(np.random.default_rng(n).standard_normal((n, topo[0])).astype(np.float32))
+                finally:
+                    lib.spgk_gemv_set_int_path(1)
+                assert spg.last_path() != "istream" and np.abs(other - y).max() <= 1e-4      # two bf16 terms: 2^-17 of a value
+        net.free()

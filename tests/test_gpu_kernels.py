@@ -190,6 +190,46 @@ def test_gemv_against_float64(spg, k, oracle, prec, int_path, out, inn, n):
     k.spgk_gemv_set_int_path(1)
 
 
+@pytest.mark.parametrize("prec", [3, 4, 5])
+@pytest.mark.parametrize("n", [7, 8])
+def test_integer_gemv_chain_against_float64(spg, k, oracle, prec, n):
+    """A whole net in one launch on the integer path, at the batch sizes where forward_batch takes another kernel.  A layer is
+    judged on the input the device had: off by less than 2^-28 of the layer's bound of its input,
+    max|bias| + scale * qmax * sum|x| of the layer before (for the first layer: its largest magnitude)."""
+    import torch
+    vp = C.c_void_p
+    k.spgk_gemv_forward_chain.argtypes = [C.POINTER(spg.abi.KLayer), C.c_uint32, vp, C.c_uint32, C.POINTER(vp), C.c_uint32, vp, vp, vp, vp]
+    k.spgk_gemv_staged_bytes.argtypes, k.spgk_gemv_staged_bytes.restype = [C.c_uint32, C.c_uint32], C.c_size_t
+    k.spgk_gemv_status.argtypes = [vp, vp]
+    rng = np.random.default_rng(n)
+    topo, q = [1024, 2048, 512, 130], {3: 127.0, 4: 7.0, 5: 1.0}[prec]
+    Ls, decs, biases, hold = [], [], [], []
+    for inn, out in zip(topo, topo[1:]):
+        raw = oracle.Oracle.encode((rng.standard_normal(out * inn) / np.sqrt(inn)).astype(np.float32), prec)
+        scale = float(np.float32(np.frombuffer(raw[:4].tobytes(), np.float32)[0] / q))
+        decs.append(np.rint(oracle.Oracle.decode(raw, out * inn, prec).astype(np.float64).reshape(out, inn) / scale) * scale)
+        biases.append(rng.standard_normal(out).astype(np.float32) * 0.1)
+        hold.append((torch.from_numpy(np.concatenate([raw[4:], np.zeros(256, np.uint8)])).cuda(), torch.from_numpy(biases[-1]).cuda()))
+        Ls.append(spg.abi.KLayer(hold[-1][0].data_ptr(), hold[-1][1].data_ptr(), scale, inn, out, prec, 3, float(np.abs(biases[-1]).max())))
+    arr = (spg.abi.KLayer * 3)(*Ls)
+    x = rng.standard_normal((n, topo[0])).astype(np.float32)
+    xd = torch.from_numpy(x).cuda()
+    ys_t = [torch.zeros(n, o, device="cuda") for o in topo[1:]]
+    ys = (vp * 3)(*[t.data_ptr() for t in ys_t])
+    staged = [torch.zeros(max(k.spgk_gemv_staged_bytes(i, n) for i in topo[:-1]), dtype=torch.uint8, device="cuda") for _ in range(2)]
+    scratch = torch.zeros(max(k.spgk_gemv_scratch_bytes(C.byref(L), n) for L in Ls), dtype=torch.uint8, device="cuda")
+    assert k.spgk_gemv_forward_chain(arr, 3, xd.data_ptr(), topo[0], ys, n, staged[0].data_ptr(), staged[1].data_ptr(), scratch.data_ptr(), None) == 0, k.spgk_error_string()
+    assert k.spgk_gemv_status(scratch.data_ptr(), None) == 0
+    a, reach = x.astype(np.float64), np.abs(x).max(1, keepdims=True)
+    for t, L, dec, bias in zip(ys_t, Ls, decs, biases):
+        z = a @ dec.T + bias
+        want, got = np.where(z > 0, z, 0.01 * z), t.cpu().numpy().astype(np.float64)
+        bound = reach * 2.0 ** -27.9 * np.abs(dec).sum(1) + 4e-7 * np.abs(z) + 2.0 ** -23 * (np.abs(bias) + np.abs(z - bias))
+        assert np.all(np.abs(got - want) <= bound), (np.abs(got - want) / bound).max()
+        reach = np.abs(bias).max() + L.w_scale * q * (1.0 + 2.0 ** -20) * np.abs(a).sum(1, keepdims=True)
+        a = got
+
+
 def test_gemv_declines_unaligned_rows(spg, k):
     import torch
     payload = torch.zeros(4096, dtype=torch.uint8, device="cuda")
