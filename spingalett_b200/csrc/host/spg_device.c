@@ -358,16 +358,21 @@ static int reserve_zeroed(spg_net *n, void **buf, size_t *have, size_t need, con
     return spg_map_kernel_error(spgk_memset(*buf, 0, need, n->stream), what);
 }
 
+/* fp32 activations of every layer of N rows */
+static int activations_reserve(spg_net *n, uint32_t N)
+{
+    if (n->small_cap >= N && n->d_small) return SPINGALETT_OK;
+    spgk_free(n->d_small); n->d_small = NULL; n->small_cap = 0;
+    void *b = NULL;
+    const int rc = spg_map_kernel_error(spgk_malloc(&b, (size_t)N * n->pub.total_neurons * sizeof(float)), "small-batch workspace");
+    if (rc == SPINGALETT_OK) { n->d_small = b; n->small_cap = N; }
+    return rc;
+}
+
 static int small_reserve(spg_net *n, uint32_t N)
 {
-    NeuralNetwork *p = &n->pub;
-    if (n->small_cap < N || !n->d_small) {
-        spgk_free(n->d_small); n->d_small = NULL; n->small_cap = 0;
-        void *b = NULL;
-        int rc = spg_map_kernel_error(spgk_malloc(&b, (size_t)N * p->total_neurons * sizeof(float)), "small-batch workspace");
-        if (rc) return rc;
-        n->d_small = b; n->small_cap = N;
-    }
+    int rc = activations_reserve(n, N);
+    if (rc) return rc;
     size_t gemv = 0, staged = 0, ws = 0, operand = 0;
     for (uint32_t l = 0; l < n->dev_layers; l++) {
         const spgk_layer *L = &n->klayers[l];
@@ -382,7 +387,6 @@ static int small_reserve(spg_net *n, uint32_t N)
         if (s > ws) ws = s;
         if (s && (s = spgk_wstream_operand_bytes(L->in, N)) > operand) operand = s;
     }
-    int rc;
     for (int i = 0; i < 2; i++) {
         if (staged && (rc = reserve(&n->d_staged[i], &n->staged_bytes[i], staged, "gemv staged input"))) return rc;
         if (operand && (rc = reserve(&n->d_operand[i], &n->operand_bytes[i], operand, "activation operand"))) return rc;
@@ -489,13 +493,7 @@ static int forward_istream(spg_net *n, const float *d_x, uint32_t N, float **d_l
     const size_t need = spgk_istream_scratch_bytes(n->klayers, n->dev_layers, N);
     if (!need) return SPINGALETT_OK;
     int rc = reserve_zeroed(n, &n->d_is_scratch, &n->is_scratch_bytes, need, "integer-stream scratch");
-    if (rc) return rc;
-    if (n->small_cap < N || !n->d_small) {
-        spgk_free(n->d_small); n->d_small = NULL; n->small_cap = 0;
-        void *b = NULL;
-        if ((rc = spg_map_kernel_error(spgk_malloc(&b, (size_t)N * p->total_neurons * sizeof(float)), "small-batch workspace"))) return rc;
-        n->d_small = b; n->small_cap = N;
-    }
+    if (rc || (rc = activations_reserve(n, N))) return rc;
     float *ys[n->dev_layers];
     for (uint32_t l = 0; l < n->dev_layers; l++)
         ys[l] = (d_final && l + 1 == n->dev_layers) ? d_final : n->d_small + (size_t)N * p->neuron_offsets[l + 1];
@@ -1094,10 +1092,12 @@ static float *forward_batch_on(spg_net *n, ForwardBatchArgs a)
         } else if (spg_map_kernel_error(spgk_memcpy_h2d(n->d_in32, a.inputs, in_bytes, n->stream), "forward_batch: input copy")) return NULL;
     }
 
-    /* Up to 8 rows always take the weight-streaming chain; up to 512 rows do so (in groups of at most 128
-     * rows, each group streaming the packed weights once) when every layer is eligible for the tensor-core
-     * streaming kernel; everything else is the large-batch GEMM chain. */
-    /* Integer files from a few rows on: the 8-bit integer streaming kernel when it takes every layer.  Measured, against the
+    /* Integer files take the 8-bit integer streaming kernel from a few rows on, when it takes every layer.  Of what is left, up
+     * to 8 rows go layer by layer (GEMV first), up to 512 rows in groups of at most 128 through the 16-bit streaming kernel when
+     * it takes every layer, each group streaming the packed weights once; everything else is the large-batch GEMM chain.
+     *
+     * The line at 7 rows is where the large INT4 net crosses; small nets are ahead at 7 already (0.63 of the time and less) and
+     * where they cross has not been looked for.  Measured, against the
      * path that served before: large INT4 net 157 us against 204 (GEMV) at 8 rows, 211 against 578 (16-bit streaming kernel)
      * at 64, 628 against 684 (GEMM chain) at 256; at 6 rows the GEMV is level (155, INT2 131), at 512 the chain is ahead
      * (945).  Nets of 4 and 12 MB: 38 against 54 and 42 against 65 us at 8 rows, 0.45 of the time or less at 32 to 96,
@@ -1117,7 +1117,7 @@ static float *forward_batch_on(spg_net *n, ForwardBatchArgs a)
         }
     }
     /* 9 to 24 rows on a net the GEMV takes whole: groups of 8 rows through the GEMV (0.2 ms per group on the large
-     * INT4 net) beat one pass of the tensor-core streaming kernel (0.7 - 0.8 ms there) */
+     * INT4 net, when it still came here) beat one pass of the tensor-core streaming kernel (0.7 - 0.8 ms there) */
     bool gemv_groups = N > SPGK_GEMV_MAX_BATCH && N <= 3 * SPGK_GEMV_MAX_BATCH;
     for (uint32_t l = 0; l < n->dev_layers && gemv_groups; l++)
         if (!spgk_gemv_scratch_bytes(&n->klayers[l], SPGK_GEMV_MAX_BATCH)) gemv_groups = false;
