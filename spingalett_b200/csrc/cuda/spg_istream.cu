@@ -15,19 +15,22 @@
 // When a layer's input has a wide row, every k-block is multiplied with both sets of digits, into both accumulators: weights
 // and unpacking are shared.  Rows of a normal draw, of pixels, or of what the hidden activations make of them are not wide
 // (0.1 to 5 % of small elements; the most for a leaky rectifier, whose slope puts half of a row within 1 % of the other half).
-// Looking for wide rows costs 1 us of a layer (INT4 net 8192-16384-16384-8192-1000: 151 -> 156 us at 8 rows, 201 -> 204 at
+// Looking for wide rows costs about 1 us of a layer (INT4 net 8192-16384-16384-8192-1000: 151 -> 156 us at 8 rows, 201 -> 204 at
 // 64); with one input of 1e6 beside ordinary ones, which makes every row of that net's layers wide: 221, 367, and 954 at 256.
 //
 // What bounds it.  HBM needs 41 us for the 272 MB of the INT4 net 8192-16384-16384-8192-1000.  A 128 x 128 block of
 // weights moves through shared memory as 8 KB packed (in and out), 16 KB of operand (in and out) and C * 128 B of digits
-// (in and out, C = 4 columns per row): 56 KB at 8 rows, 112 KB at 64 rows, 440 and 880 cycles at 128 B/clk -- 51 us and
-// 103 us over the net.  One byte per weight in the operand instead of two is why this path exists beside the 16-bit
-// streaming kernel, which writes and reads 32 KB per such block.
+// (in and out, C = 4 columns per row): 56 KB at 8 rows, 112 KB at 64 rows, 440 and 880 cycles at 128 B/clk -- 53 us and
+// 106 us over the net, whose busiest SMs have 237 such blocks.  One byte per weight in the operand instead of two is why this
+// path exists beside the 16-bit streaming kernel, which writes and reads 32 KB per such block.
 //
-// Measured: 157 us at 8 rows (GEMV: 201), 211 at 64 (16-bit streaming kernel: 577), 628 at 256 (GEMM chain: 684).  About 10 us
-// of a layer are its start, staging and last sums; the rest goes at 750 cycles per 128-wide block up to 64 rows, the turn of
-// the MMA warp (two waits, four MMAs, two commits): taking out the unpacking, the digit copies or the MMAs alone leaves the
-// time within a few per cent, and so do two or eight operand slots instead of four.
+// Measured: 157 us at 8 rows (GEMV: 201), 211 at 64 (16-bit streaming kernel: 577), 628 at 256 (GEMM chain: 684).  From
+// layers of 32 to 166 blocks a CTA: at 8 rows 825 cycles a block and 14 us a layer (154 us for the net), at 64 rows 1000 and
+// 21 (207 us).  INT8, whose boxes need no unpacking, takes 725 cycles at 8 rows, 5.4 TB/s.  INT4 and INT2 are bound there by a
+// block's way through unpackers and MMA warp -- DRAM 29 %, shared memory 22 %, tensor pipe 6 %, issue slots 24 % of their peaks;
+// taking out the unpacking, the digit copies or the MMAs alone left the time within a few per cent, and so did two or eight
+// operand slots instead of four.  At 64 rows the tensor pipe needs 514 of the 1000 cycles and every CTA draws 32 KB of digits
+// a block from L2.  The 14 to 21 us of a layer are staging, the first boxes and tiles, and the last sums.
 //
 // Per CTA (one per SM, 19 warps):
 //   warp 0      weight boxes by TMA (128 rows x 128 packed bytes, 128-byte swizzle), ahead of the previous layer's end:
