@@ -1052,6 +1052,8 @@ static float *forward_batch_on(spg_net *n, ForwardBatchArgs a)
         result = n->h_out;
     }
     if (N == 0) return result;
+    /* rows recomputed by this call: none unless the recomputation of a large batch says otherwise */
+    if (spingalett_get_math_mode() == SPINGALETT_MATH_AUTO) { n->count_slots_used = 0; n->count_pending = false; n->last_repaired = 0; }
 
     const float *d_x = a.inputs;
     const bool in_dev = spgk_is_device_pointer(a.inputs) == 1;
@@ -1141,7 +1143,7 @@ static float *forward_batch_on(spg_net *n, ForwardBatchArgs a)
             if (reserve((void **)&n->d_out32, &n->out32_bytes, out_bytes, "forward_batch: output staging")) return NULL;
             d_out = n->d_out32;
         }
-        n->count_slot = 0; n->count_slots_used = 0;
+        n->count_slot = 0;
         if (pipelined) {
             /* compute on chunk c starts as soon as its copy has landed, while the copies of the later chunks go on */
             /* copy c is queued before compute c-1 is launched, so a pageable source (whose copies block the host)

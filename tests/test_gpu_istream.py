@@ -261,6 +261,25 @@ def test_one_net_over_batches_of_changing_size(spg, has_gpu, tmp_path, prec):
     net.free()
 
 
+@pytest.mark.parametrize("n", [1, 64, 200, 400])
+def test_a_small_auto_batch_recomputes_no_rows(spg, has_gpu, tmp_path, n):
+    """spingalett_last_repaired is about the last AUTO call, also when that one had nothing to recompute."""
+    a, lib = spg.abi, spg.lib()
+    net = _loaded(spg, tmp_path, [4096, 2048, 10], [a.ACT_RELU, a.ACT_SOFTMAX], 4)
+    x = np.random.default_rng(n).standard_normal((2048, 4096)).astype(np.float32)
+    lib.spingalett_set_auto_margin(5.0)
+    try:
+        for read in (True, False):
+            net.forward_batch(x)
+            if read:
+                assert lib.spingalett_last_repaired(net._h) > 0
+            net.forward_batch(x[:n])
+            assert lib.spingalett_last_repaired(net._h) == 0, (read, spg.last_path())
+    finally:
+        lib.spingalett_set_auto_margin(0.0)
+    net.free()
+
+
 def test_the_rows_widths_and_modes_that_take_the_path(spg, has_gpu, tmp_path):
     """Just inside and just outside of every line that the dispatch draws."""
     a, lib = spg.abi, spg.lib()
