@@ -580,7 +580,7 @@ def main():
             traffic = json.load(open(tpath)).get(f"{args.workload}_{args.dtype}_{args.math}_{batch}")
         line["roofline"] = {"bound": "tensor", "achieved": achieved, "peak": pk["bf16_tflops"], "unit": "TFLOP/s",
                             "frac": achieved / pk["bf16_tflops"], "traffic": traffic,
-                            "kernel": KERNEL_OF_PATH[path_taken],
+                            "kernel": KERNEL_OF_PATH.get(path_taken, path_taken),
                             "launches": int(k_cnt), "kernel_ms_per_step": k_ms_eff / args.steps,
                             "peak_source": pk["source"] + " burst bf16", "tensor_passes_per_product": passes,
                             "executed_frac": achieved * passes / pk["bf16_tflops"],
@@ -598,7 +598,7 @@ def main():
             traffic = json.load(open(tpath)).get(f"{args.workload}_{args.dtype}_{batch}")
         line["roofline"] = {"bound": "hbm", "achieved": achieved, "peak": pk["hbm_gbs"], "unit": "GB/s",
                             "frac": achieved / pk["hbm_gbs"], "traffic": traffic,
-                            "kernel": KERNEL_OF_PATH[path_taken],
+                            "kernel": KERNEL_OF_PATH.get(path_taken, path_taken),
                             "launches": int(k_cnt), "kernel_ms_per_step": k_ms / args.steps,
                             "algorithmic_bytes_per_step": nbytes, "peak_source": pk["source"] + " copy bandwidth",
                             "whole_step_frac": nbytes / (dev_ms * 1e-3) / 1e9 / pk["hbm_gbs"],
