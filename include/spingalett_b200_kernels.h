@@ -267,6 +267,7 @@ SPGK_API int spgk_istream_status(void *scratch, void *stream);
  * layer needs spgk_softmax_rows afterwards.
  * status: dev int32 the kernel reports a bounded wait that gave up in; read it
  * with spgk_gemm_tc_status() (which synchronises the stream).
+ * Products that fit the device in one wave of smaller tiles run in a kernel that also cuts K (spg_gemm_split.cu).
  * Does batch_forward()'s layer step, reference Training.c:318-343. */
 SPGK_API int spgk_gemm_tc_supported(const spgk_layer *L);
 SPGK_API uint32_t spgk_gemm_tc_softmax_max(void);

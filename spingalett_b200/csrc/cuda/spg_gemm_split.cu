@@ -1,0 +1,432 @@
+// spg_gemm_split.cu -- the tensor-core layer of spg_gemm_tc.cu for products of few tiles.
+//
+//   C[M][N] = act(bias + scale * sum over passes  A_pa[M][K] * W_pw[N][K]^T)
+//
+// A product of a few hundred rows has a handful of 128 x 256 tiles: most SMs idle while each busy one walks the whole K
+// range, and its epilogue turns 256 columns into output with nothing to hide behind.  Here a tile is 128 x BN with BN down
+// to 16, and a cluster of up to eight CTAs shares it: CTA r multiplies the r-th part of the k-blocks, hands the partial
+// sums of every row to the CTA that owns the row (distributed shared memory, 128 / S rows each), and each CTA finishes its
+// own rows: sum in CTA order, scale, bias, activation or softmax, store.  The result does not depend on timing.
+//
+// A k-block brings all planes of both operands at once (hi and lo of the activations, of the weights where they have two)
+// and every pass multiplies what is there, so a two-term product moves three tiles where the pass-by-pass walk moves four.
+//
+// What bounds it: latency.  At 256 rows of a 784-512-1000-10 net a layer takes 5.2 us of about 9500 cycles: 1000 of set-up (under
+// the layer before), 2900 until the first k-block has landed, 1500 to 2400 for the rest, 800 to 2200 for handing the sums over,
+// 1100 to 1900 for the cluster barrier, 1100 to 2100 to finish the rows.  With more rows the operands come to weigh, at 47 bytes
+// a cycle and SM.  The tensor pipe is idle most of the time.
+// Measured against the persistent kernel, a layer with two terms an activation (us): 256 rows 784 -> 512 19.3 -> 6.5 and
+// 1000 -> 10 11.6 -> 6.2; 1000 rows 784 -> 512 19.6 -> 8.8 and 2048 -> 2048 32.1 -> 23.7; 3000 rows 301 -> 777 14.7 -> 9.5 and
+// 777 -> 333 19.7 -> 10.2.  Whole nets: 784-512-1000-10 at 256 rows 49.8 -> 22.8; 301-777-333-129-37 at 3001 rows 64.7 -> 38.9; the
+// recomputation of some 950 of 65536 rows 46 -> 30.
+//
+// Every wait on an mbarrier is bounded as in spg_gemm_tc.cu; the cluster barriers are reached by every thread on every path.
+#include "spg_common.cuh"
+#include "spg_tc.cuh"
+#include "spg_gemm.cuh"
+#include <cmath>
+
+namespace {
+
+using namespace spgtc;
+
+constexpr uint32_t TM = 128, TK = 64;
+constexpr uint32_t A_BYTES = TM * TK * 2;
+constexpr uint32_t EPI = 8;
+constexpr uint32_t THREADS = 64 + 32 * EPI;
+constexpr uint32_t MAX_STAGES = 6, MAX_SPLIT = 8, MAX_BN = 192;
+
+struct SplitParams {
+    uint32_t M, N, kblocks, BN, S, stages;
+    uint32_t m_tiles, n_tiles;
+    uint32_t a_parts, w_parts, stage_bytes;
+    uint32_t idesc;
+    float scale; const float *bias; int act, softmax;
+    void *out16; uint32_t ldo16; uint64_t o_plane; int out_parts, type16;
+    float *out32; uint32_t ldo32; const uint32_t *out_rows;
+    float margin_theta; uint32_t *margin_idx, *margin_count;
+    const uint32_t *m_limit;
+    int32_t *status;
+};
+
+__device__ __forceinline__ void load_planes(uint32_t dst, const CUtensorMap *map, uint32_t bar, int k, int row)
+{
+    asm volatile(
+        "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
+        ::"r"(dst), "l"(map), "r"(bar), "r"(k), "r"(row), "r"(0) : "memory");
+}
+__device__ __forceinline__ void store_remote4(uint32_t addr, const uint32_t *r)
+{
+    asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]) : "memory");
+}
+
+// a load that stays where it is written, ahead of the waits
+__device__ __forceinline__ float load_early(const float *p)
+{
+    float v;
+    asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(v) : "l"(p));
+    return v;
+}
+
+__device__ __forceinline__ void add4(float4 &s, const float *p)
+{
+    const float4 a = *reinterpret_cast<const float4 *>(p);
+    s.x += a.x; s.y += a.y; s.z += a.z; s.w += a.w;
+}
+// the S partial sums of four neighbouring outputs, `step` floats apart, added in CTA order
+__device__ __forceinline__ float4 sum_parts(const float *at, uint32_t step, uint32_t S)
+{
+    float4 s = *reinterpret_cast<const float4 *>(at);
+    if (S > 1) add4(s, at + step);
+    if (S > 2) { add4(s, at + 2 * step); add4(s, at + 3 * step); }
+    if (S > 4) { add4(s, at + 4 * step); add4(s, at + 5 * step); add4(s, at + 6 * step); add4(s, at + 7 * step); }
+    return s;
+}
+
+// What a thread finishes of a tile: four neighbouring columns (col..) of every lanes_y-th of the rows that its CTA owns.
+// recv: their sums, [part][own row][BN], columns of neighbouring rows in another order (swz).
+struct Mine { const float *recv; uint32_t own, row0, rows, col, cx, cy, lanes_y; float4 bias; };
+
+__device__ __forceinline__ float4 logits4(const SplitParams &p, const Mine &m, uint32_t rl)
+{
+    const float4 s = sum_parts(m.recv + rl * p.BN + (m.cx ^ ((rl & 3u) * 4)), m.own * p.BN, p.S);
+    return make_float4(fmaf(s.x, p.scale, m.bias.x), fmaf(s.y, p.scale, m.bias.y), fmaf(s.z, p.scale, m.bias.z), fmaf(s.w, p.scale, m.bias.w));
+}
+__device__ __forceinline__ void write4(const SplitParams &p, uint32_t row, uint32_t col, float4 v)
+{
+    float *o = p.out32 + (uint64_t)(p.out_rows ? p.out_rows[row] : row) * p.ldo32 + col;
+    if (col + 4 <= p.N && (reinterpret_cast<uintptr_t>(o) & 15u) == 0) { *reinterpret_cast<float4 *>(o) = v; return; }
+    if (col < p.N) o[0] = v.x;
+    if (col + 1 < p.N) o[1] = v.y;
+    if (col + 2 < p.N) o[2] = v.z;
+    if (col + 3 < p.N) o[3] = v.w;
+}
+template <typename T16> __device__ __forceinline__ uint32_t round2(float &a, float &b)      // the pair in 16 bits; a, b: what is left of them
+{
+    union { uint32_t q; T16 h[2]; } pk;
+    if constexpr (__is_same(T16, __half)) { pk.h[0] = __float2half_rn(a); pk.h[1] = __float2half_rn(b); a -= __half2float(pk.h[0]); b -= __half2float(pk.h[1]); }
+    else { pk.h[0] = __float2bfloat16_rn(a); pk.h[1] = __float2bfloat16_rn(b); a -= __bfloat162float(pk.h[0]); b -= __bfloat162float(pk.h[1]); }
+    return pk.q;
+}
+template <int ACT, typename T16>
+__device__ __forceinline__ void finish_rows(const SplitParams &p, const Mine &m)
+{
+    // The loop is kept small on purpose: a CTA runs it a few times only, and every line of code comes from L2 first (unrolled by
+    // four and with the activation chosen inside, 128 x 144 tanh outputs took 29000 cycles, with this loop 8000).
+    T16 *o16 = reinterpret_cast<T16 *>(p.out16) + (uint64_t)(m.row0 + m.cy) * p.ldo16 + m.col;
+    const uint64_t step = (uint64_t)m.lanes_y * p.ldo16;
+    const bool in16 = p.out16 && m.col < p.ldo16;              // (ldo16 is a multiple of 8: a group of four lies inside or outside it)
+    const uint32_t live = m.rows > m.row0 ? min(m.own, m.rows - m.row0) : 0;
+#pragma unroll 1
+    for (uint32_t rl = m.cy; rl < live; rl += m.lanes_y, o16 += step) {
+        float4 v = logits4(p, m, rl);
+        v.x = spg_activate(v.x, ACT); v.y = spg_activate(v.y, ACT); v.z = spg_activate(v.z, ACT); v.w = spg_activate(v.w, ACT);
+        if (p.out32) write4(p, m.row0 + rl, m.col, v);
+        if (in16) {
+            uint2 q;
+            q.x = round2<T16>(v.x, v.y); q.y = round2<T16>(v.z, v.w);
+            *reinterpret_cast<uint2 *>(o16) = q;
+            if (p.out_parts > 1) {
+                q.x = round2<T16>(v.x, v.y); q.y = round2<T16>(v.z, v.w);
+                *reinterpret_cast<uint2 *>(o16 + p.o_plane) = q;
+            }
+        }
+    }
+}
+
+// Softmax rows: the BN / 4 lanes that hold a row (a power of two of them) are neighbours in a warp; formulas and margin test as
+// in spg_gemm_tc.cu's epilogue.  Every lane makes the same number of rounds.
+__device__ __forceinline__ void finish_softmax(const SplitParams &p, const Mine &m)
+{
+    const uint32_t lanes = p.BN >> 2;
+#pragma unroll 1
+    for (uint32_t rl = m.cy; rl - m.cy < m.own; rl += m.lanes_y) {
+        const uint32_t row = m.row0 + rl;
+        const bool live = rl < m.own && row < m.rows;
+        const float4 z = logits4(p, m, rl < m.own ? rl : 0);
+        float v[4] = { z.x, z.y, z.z, z.w };
+        float mx = -FLT_MAX, second = -FLT_MAX;
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+            if (m.col + i < p.N) { if (v[i] > mx) { second = mx; mx = v[i]; } else if (v[i] > second) second = v[i]; }
+#pragma unroll 1
+        for (uint32_t o = lanes >> 1; o > 0; o >>= 1) {
+            const float m2 = __shfl_xor_sync(0xffffffffu, mx, o), s2 = __shfl_xor_sync(0xffffffffu, second, o);
+            second = fmaxf(fminf(mx, m2), fmaxf(second, s2));
+            mx = fmaxf(mx, m2);
+        }
+        float sum = 0.0f;
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            v[i] = m.col + i < p.N ? expf(v[i] - mx) : 0.0f;
+            sum += v[i];
+        }
+#pragma unroll 1
+        for (uint32_t o = lanes >> 1; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+        if (m.col == 0 && live && p.margin_idx && p.N >= 2 && (!(mx - second >= p.margin_theta) || !(sum < FLT_MAX)))
+            p.margin_idx[atomicAdd(p.margin_count, 1u)] = row;
+        const float inv = sum > 0.0f ? 1.0f / sum : 1.0f;
+        if (live) write4(p, row, m.col, make_float4(v[0] * inv, v[1] * inv, v[2] * inv, v[3] * inv));
+    }
+}
+
+template <typename T16> __device__ __forceinline__ void finish(const SplitParams &p, const Mine &m)
+{
+    switch (p.act) {                                           // the same for every thread
+        case SPG_ACT_RELU:    finish_rows<SPG_ACT_RELU, T16>(p, m); break;
+        case SPG_ACT_LEAKY:   finish_rows<SPG_ACT_LEAKY, T16>(p, m); break;
+        case SPG_ACT_FOO52:   finish_rows<SPG_ACT_FOO52, T16>(p, m); break;
+        case SPG_ACT_TANH:    finish_rows<SPG_ACT_TANH, T16>(p, m); break;
+        case SPG_ACT_SIGMOID: finish_rows<SPG_ACT_SIGMOID, T16>(p, m); break;
+        default:              finish_rows<SPG_ACT_NONE, T16>(p, m); break;
+    }
+}
+
+__global__ void __launch_bounds__(THREADS, 1)
+spg_gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w, const SplitParams p)
+{
+    extern __shared__ __align__(1024) uint8_t smem[];          // (1024: the swizzle atoms of the operand tiles)
+    const uint32_t base = smem_u32(smem);
+    const uint32_t recv_off = p.stages * p.stage_bytes, bar_off = recv_off + TM * p.BN * 4;
+    const uint32_t full0 = base + bar_off, empty0 = full0 + 8 * MAX_STAGES, tfull = empty0 + 8 * MAX_STAGES;
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem + bar_off + 16 * MAX_STAGES + 8);
+    volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
+    const uint32_t abort_addr = smem_u32(const_cast<int *>(abort_flag));
+    const uint32_t warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31u;
+    const uint32_t tmem_cols = p.BN <= 32 ? 32 : p.BN <= 64 ? 64 : p.BN <= 128 ? 128 : 256;       // a power of two
+
+    if (threadIdx.x == 0) {
+        for (uint32_t s = 0; s < p.stages; s++) { mbar_init(full0 + 8 * s, 1); mbar_init(empty0 + 8 * s, 1); }
+        mbar_init(tfull, 1);
+        *abort_flag = 0;
+        mbar_fence_init();
+        prefetch_map(&map_a);
+        prefetch_map(&map_w);
+    }
+    if (warp == 1) tmem_alloc(smem_u32(tmem_slot), tmem_cols);
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync();                                            // the other CTAs of the cluster are there: their shared memory may be written
+    tc_fence_after();
+    const uint32_t tmem = *tmem_slot;
+    spg_grid_trigger();
+    spg_grid_wait();
+
+    const uint32_t rows = spg_limit_rows(p.M, p.m_limit);
+    const uint32_t tiles = (rows + TM - 1) / TM * p.n_tiles, rank = cluster_rank(), clusters = gridDim.x / p.S;
+    const uint32_t kb0 = rank * p.kblocks / p.S, kb1 = (rank + 1) * p.kblocks / p.S;
+    const uint32_t own = TM / p.S;                             // rows of a tile that this CTA finishes
+    const uint32_t passes = 1 + (p.a_parts > 1) + (p.w_parts > 1);
+    const uint32_t w_off = p.a_parts * A_BYTES, w_plane = p.BN * TK * 2;
+    const uint32_t groups = p.BN >> 2, lanes_y = THREADS / groups, cx = threadIdx.x % groups * 4, cy = threadIdx.x / groups;
+    uint32_t it = 0, round = 0;                                // k-blocks and tiles so far
+    for (uint32_t t = blockIdx.x / p.S; t < tiles; t += clusters, round++) {
+        // neighbouring clusters take the column tiles of the same rows
+        const uint32_t mt = t / p.n_tiles, nt = t % p.n_tiles;
+        const uint32_t col = nt * p.BN + cx;                   // this thread's columns when the tile is finished; their biases are under way from here
+        float4 bias = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (col < p.N) bias.x = load_early(p.bias + col);
+        if (col + 1 < p.N) bias.y = load_early(p.bias + col + 1);
+        if (col + 2 < p.N) bias.z = load_early(p.bias + col + 2);
+        if (col + 3 < p.N) bias.w = load_early(p.bias + col + 3);
+        if (warp == 0) {
+            for (uint32_t kb = kb0; kb < kb1; kb++, it++) {
+                const uint32_t s = it % p.stages, ph = (it / p.stages) & 1u, st = base + s * p.stage_bytes;
+                mbar_wait_uniform(empty0 + 8 * s, ph ^ 1u, abort_addr, p.status, 51);
+                if (elect_one()) {
+                    mbar_expect_tx(full0 + 8 * s, p.stage_bytes);
+                    load_planes(st, &map_a, full0 + 8 * s, (int)(kb * TK), (int)(mt * TM));
+                    load_planes(st + w_off, &map_w, full0 + 8 * s, (int)(kb * TK), (int)(nt * p.BN));
+                }
+                __syncwarp();
+            }
+        } else if (warp == 1) {
+            for (uint32_t kb = kb0; kb < kb1; kb++, it++) {
+                const uint32_t s = it % p.stages, ph = (it / p.stages) & 1u, st = base + s * p.stage_bytes;
+                mbar_wait_uniform(full0 + 8 * s, ph, abort_addr, p.status, 52);
+                tc_fence_after();
+                // hi*hi, then the corrections lo*hi and hi*lo (lo*lo is below fp32 resolution)
+                for (uint32_t ps = 0; ps < passes; ps++) {
+                    const bool a_lo = ps == 1 && p.a_parts > 1, w_lo = ps > 0 && !a_lo;
+                    const uint64_t da = smem_desc_sw128(st + (a_lo ? A_BYTES : 0)), db = smem_desc_sw128(st + w_off + (w_lo ? w_plane : 0));
+                    if (elect_one()) {
+#pragma unroll
+                        for (uint32_t k = 0; k < TK / 16; k++) umma_f16(tmem, da + 2 * k, db + 2 * k, p.idesc, (kb != kb0 || (ps | k)) ? 1u : 0u);
+                    }
+                    __syncwarp();
+                }
+                if (elect_one()) {
+                    umma_commit(empty0 + 8 * s);
+                    if (kb + 1 == kb1) umma_commit(tfull);
+                }
+                __syncwarp();
+            }
+        } else {
+            // partial sums -> the CTA that owns the row: thread = one row, the two warps on a quadrant take 16 columns in turn
+            const uint32_t q = warp & 3u, half = (warp - 2u) >> 2, row = q * 32u + lane, swz = (row & 3u) * 4;    // neighbouring rows on other banks
+            mbar_wait(tfull, round & 1u, abort_flag, p.status, 53);
+            tc_fence_after();
+            const uint32_t dst = mapa(base + recv_off + (rank * own + row % own) * p.BN * 4, row / own);
+            for (uint32_t c = 16 * half; c < p.BN; c += 32) {
+                uint32_t r[16];
+                tmem_ld16(tmem + c + ((q * 32u) << 16), r);
+                tmem_ld_wait();
+#pragma unroll
+                for (int i = 0; i < 16; i += 4) store_remote4(dst + ((c + i) ^ swz) * 4, r + i);
+            }
+            tc_fence_before();
+        }
+        cluster_sync();                                        // every partial sum of this cluster's tile is in place
+        tc_fence_after();
+        const Mine mine = { reinterpret_cast<const float *>(smem + recv_off), own, mt * TM + rank * own, rows, col, cx, cy, lanes_y, bias };
+        if (cy < lanes_y) {                                    // (a power of two of groups leaves no thread out)
+            if (p.softmax) finish_softmax(p, mine);
+            else if (p.type16 == SPGK_T_F16) finish<__half>(p, mine);
+            else finish<__nv_bfloat16>(p, mine);
+        }
+        if (t + clusters < tiles) cluster_sync();              // read before the next tile's sums replace them (the same decision in every CTA of the cluster)
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 1) { tc_fence_after(); tmem_free(tmem, tmem_cols); }
+}
+
+struct SplitPlan { uint32_t BN, S, stages, smem; };
+
+uint32_t split_smem(uint32_t BN, uint32_t stages, uint32_t stage_bytes)
+{
+    return stages * stage_bytes + TM * BN * 4 + 16 * MAX_STAGES + 32;
+}
+
+// clusters of 1, 2, 4 and 8 CTAs that the device holds at one CTA an SM (0: none)
+struct AtOnce { uint32_t n[4]; };
+int clusters_at_once(int dev, AtOnce &out)
+{
+    static SpgOncePerDevice once;
+    static AtOnce known[SPG_MAX_DEVICES];
+    const int rc = once.run(dev, [&]() -> int {
+        for (int i = 0; i < 4; i++) {
+            cudaLaunchConfig_t cfg = {};
+            cfg.gridDim = dim3(1u << i); cfg.blockDim = dim3(THREADS); cfg.dynamicSmemBytes = 160 * 1024;
+            cudaLaunchAttribute attr[1];
+            attr[0].id = cudaLaunchAttributeClusterDimension;
+            attr[0].val.clusterDim.x = 1u << i; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+            cfg.attrs = attr; cfg.numAttrs = 1;
+            int n = 0;
+            if (cudaOccupancyMaxActiveClusters(&n, spg_gemm_split_kernel, &cfg) != cudaSuccess) { cudaGetLastError(); n = 0; }
+            known[dev].n[i] = n > 0 ? (uint32_t)n : 0u;
+        }
+        return SPGK_OK;
+    });
+    if (rc == SPGK_OK) out = known[dev];
+    return rc;
+}
+
+// The split of a product whose row count only the device knows.  The caller's guess of the count changes from call to call
+// and must not change the order of the sums, so the split depends on the layer alone: as many CTAs a tile as 1024 rows
+// leave SMs for.
+uint32_t fixed_split(uint32_t N, uint32_t kblocks, uint32_t sm_count)
+{
+    const uint32_t tiles = 8 * ((N + 63) / 64);
+    uint32_t S = 1;
+    while (S < MAX_SPLIT && 2 * S <= kblocks && 2 * S * tiles <= sm_count) S <<= 1;
+    return S;
+}
+
+// Which products come here, and how they are cut: those for which some tile width and split fit on the device in one wave
+// (one CTA an SM), at the width and split that the estimate below makes cheapest.  Measured for 24 products (32 to 3000 rows,
+// 10 to 2048 columns, 301 to 2048 inputs) over every width and split: the estimate picked the fastest or one within 8 % of it,
+// and none was slower than the persistent kernel, which overlaps epilogues with the next tile's products and is the better one
+// as soon as tiles come in waves.
+//
+// Tile width and split of the cheapest arrangement; only_S: that split and no other, if not zero.  one_wave: only what the
+// device holds at once (false if nothing fits).
+bool split_plan(const AtOnce &at, uint32_t rows, uint32_t N, uint32_t kblocks, uint32_t a_parts, uint32_t w_parts, bool softmax, uint32_t only_S, bool one_wave,
+                size_t smem_max, SplitPlan &best)
+{
+    const uint32_t mt = (rows + TM - 1) / TM;
+    uint32_t lo = 16, hi = N < MAX_BN ? (N + 15u) & ~15u : MAX_BN;
+    if (softmax) {                                              // a row in one tile, on a power of two of lanes
+        while (lo < N) lo <<= 1;
+        if (lo > 128) return false;
+        hi = lo;
+    }
+    uint64_t best_cost = ~0ull;
+    for (uint32_t BN = lo; BN <= hi; BN += 16) {
+        const uint32_t nt = (N + BN - 1) / BN, stage = a_parts * A_BYTES + w_parts * BN * TK * 2;
+        const uint64_t tiles = (uint64_t)mt * nt;
+        for (uint32_t i = 0, S = 1; S <= MAX_SPLIT && S <= kblocks; i++, S <<= 1) {
+            if ((only_S && S != only_S) || !at.n[i] || (one_wave && tiles > at.n[i])) continue;
+            const uint32_t kb = (kblocks + S - 1) / S;
+            // cycles of a tile (measured, 128 CTAs at work): operands at 47 bytes a cycle; partial sums into their owner's shared
+            // memory at 55 (the own one), 24, 21 and 13, and out of it at 60; a cluster barrier
+            static const uint32_t push[4] = { 55, 24, 21, 13 };
+            const uint64_t cost = (1500 + (uint64_t)kb * stage / 47 + TM * BN * 4 / push[i] + TM * BN * 4 / 60 + (S > 1 ? 1200 : 0)) * ((tiles + at.n[i] - 1) / at.n[i]);
+            if (cost >= best_cost) continue;
+            uint32_t stages = !one_wave || kb > MAX_STAGES ? MAX_STAGES : kb;
+            while (stages > 1 && split_smem(BN, stages, stage) > smem_max) stages--;
+            if (split_smem(BN, stages, stage) > smem_max || (stages == 1 && kb > 1)) continue;
+            best_cost = cost;
+            best = { BN, S, stages, split_smem(BN, stages, stage) };
+        }
+    }
+    return best_cost != ~0ull;
+}
+
+}  // namespace
+
+int spg_gemm_split_try(const SpgGemmArgs &a, const SpgDeviceProps &dp, int dev)
+{
+    if (a.w_type16 != a.type16) return SPGK_E_UNSUPPORTED;
+    const uint32_t kblocks = (a.L->in + TK - 1) / TK;
+    static SpgOncePerDevice once;
+    int rc = once.run(dev, [&]() -> int {
+        SPGK_CUDA(cudaFuncSetAttribute(spg_gemm_split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dp.smem_optin));
+        return SPGK_OK;
+    });
+    if (rc) return rc;
+    // the rows to arrange for: where only the device knows, those of the call before and what a selection by chance varies
+    uint32_t rows = a.N, only_S = 0;
+    if (spg_tls_rows_limit) {
+        rows = spg_tls_rows_expected ? spg_tls_rows_expected + 4u * (uint32_t)sqrtf((float)spg_tls_rows_expected) : 1024;
+        if (rows > a.N) rows = a.N;
+        only_S = fixed_split(a.L->out, kblocks, (uint32_t)dp.sm_count);
+    }
+    AtOnce at;
+    if ((rc = clusters_at_once(dev, at))) return rc;
+    SplitPlan plan;
+    // (an unsplit tile is summed in the order of the persistent kernel: either may run)
+    if (!split_plan(at, rows, a.L->out, kblocks, (uint32_t)a.a_parts, (uint32_t)a.w_parts, a.softmax_fused != 0, only_S, only_S < 2,
+                    dp.smem_optin, plan)) return SPGK_E_UNSUPPORTED;
+
+    SplitParams p{};
+    p.M = a.N; p.N = a.L->out; p.kblocks = kblocks; p.BN = plan.BN; p.S = plan.S; p.stages = plan.stages;
+    p.n_tiles = (a.L->out + p.BN - 1) / p.BN; p.m_tiles = (a.N + TM - 1) / TM;
+    p.a_parts = (uint32_t)a.a_parts; p.w_parts = (uint32_t)a.w_parts; p.stage_bytes = p.a_parts * A_BYTES + p.w_parts * p.BN * TK * 2;
+    p.idesc = idesc_f16((uint32_t)a.type16, (uint32_t)a.w_type16, p.BN);
+    p.scale = a.L->w_scale; p.bias = a.L->bias;
+    p.act = a.L->act == SPG_ACT_SOFTMAX ? SPG_ACT_NONE : a.L->act;
+    p.softmax = a.softmax_fused ? 1 : 0;
+    p.out16 = a.out16; p.ldo16 = a.ldo16; p.o_plane = a.o_plane; p.out_parts = a.out_parts; p.type16 = a.type16;
+    p.out32 = a.out32; p.ldo32 = a.ldo32; p.out_rows = spg_tls_out_rows;
+    if (p.softmax && spg_tls_margin_idx) { p.margin_theta = spg_tls_margin_theta; p.margin_idx = spg_tls_margin_idx; p.margin_count = spg_tls_margin_count; }
+    p.m_limit = spg_tls_rows_limit;
+    p.status = a.status;
+    CUtensorMap map_a, map_w;
+    if ((rc = spg_gemm_map(&map_a, a.a16, a.type16, a.L->in, a.N, a.lda, a.a_plane, a.a_parts, TM, p.a_parts))) return rc;
+    if ((rc = spg_gemm_map(&map_w, a.w16, a.w_type16, a.L->in, a.L->out, a.ldw, a.w_plane, a.w_parts, p.BN, p.w_parts))) return rc;
+
+    const uint64_t tiles = (uint64_t)p.m_tiles * p.n_tiles;
+    const uint32_t at_once = at.n[p.S == 1 ? 0 : p.S == 2 ? 1 : p.S == 4 ? 2 : 3];
+    const uint32_t clusters = tiles < at_once ? (uint32_t)tiles : at_once;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(clusters * p.S); cfg.blockDim = dim3(THREADS); cfg.dynamicSmemBytes = plan.smem; cfg.stream = (cudaStream_t)a.stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = p.S; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr; cfg.numAttrs = 2;
+    SPGK_CUDA(cudaLaunchKernelEx(&cfg, spg_gemm_split_kernel, map_a, map_w, p));
+    return spgk_check_launch("spg_gemm_split_kernel");
+}

@@ -14,11 +14,14 @@
 // accumulator is double-buffered in TMEM so the epilogue of tile i overlaps the
 // main loop of tile i+1.
 //
+// Products that fit the device in one wave of smaller tiles run in spg_gemm_split.cu instead.
+//
 // Every wait on an mbarrier is bounded: when the bound is hit the CTA records a
 // code in `status`, raises a shared abort flag that all roles poll, drains, frees
 // its tensor memory and returns; the launcher turns that into SPGK_E_TIMEOUT.
 #include "spg_common.cuh"
 #include "spg_tc.cuh"
+#include "spg_gemm.cuh"
 #include <cuda.h>
 #include <cstdio>
 #include <mutex>
@@ -721,9 +724,18 @@ EncodeTiledFn encode_fn()
     return fn;
 }
 
-// 3-D map over `parts` planes of a row-major [rows][ld] 16-bit matrix whose first K columns are valid.
-int make_map(CUtensorMap *map, const void *base, int type16, uint32_t K, uint32_t rows, uint32_t ld, uint64_t plane,
-             int parts, uint32_t box_rows)
+uint32_t pick_bn(uint32_t out)
+{
+    if (out > 128) return 256;
+    uint32_t bn = 16;
+    while (bn < out) bn <<= 1;
+    return bn;
+}
+
+}  // namespace
+
+int spg_gemm_map(CUtensorMap *map, const void *base, int type16, uint32_t K, uint32_t rows, uint32_t ld, uint64_t plane, int parts,
+                 uint32_t box_rows, uint32_t box_planes)
 {
     EncodeTiledFn fn = encode_fn();
     if (!fn) { spgk_set_error("cuTensorMapEncodeTiled", "driver entry point not available"); return SPGK_E_CUDA; }
@@ -735,7 +747,7 @@ int make_map(CUtensorMap *map, const void *base, int type16, uint32_t K, uint32_
     cuuint64_t plane_bytes = parts > 1 ? plane * 2 : (cuuint64_t)rows * ld * 2;
     plane_bytes = (plane_bytes + 15) & ~(cuuint64_t)15;
     cuuint64_t strides[2] = { (cuuint64_t)ld * 2, plane_bytes };
-    cuuint32_t box[3] = { BK, box_rows, 1 };
+    cuuint32_t box[3] = { BK, box_rows, box_planes };
     cuuint32_t estr[3] = { 1, 1, 1 };
     CUresult r = fn(map, type16 == SPGK_T_F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3,
                     const_cast<void *>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
@@ -748,16 +760,6 @@ int make_map(CUtensorMap *map, const void *base, int type16, uint32_t K, uint32_
     }
     return SPGK_OK;
 }
-
-uint32_t pick_bn(uint32_t out)
-{
-    if (out > 128) return 256;
-    uint32_t bn = 16;
-    while (bn < out) bn <<= 1;
-    return bn;
-}
-
-}  // namespace
 
 extern "C" {
 
@@ -847,10 +849,16 @@ static int gemm_launch(const spgk_layer *L,
     {
         const int prc = spg_device_props(&dp);
         if (prc) return prc;
-        // the opt-in for large dynamic shared memory is a per-device function attribute
-        static SpgOncePerDevice once;
         int dev = 0;
         SPGK_CUDA(cudaGetDevice(&dev));
+        if (!head) {
+            const SpgGemmArgs args = { L, w16, ldw, w_plane, w_parts, w_type16, a16, lda, a_plane, a_parts, type16, out16, ldo16, o_plane,
+                                       out_parts, out32, ldo32, N, softmax_fused, status, stream };
+            const int rc = spg_gemm_split_try(args, dp, dev);
+            if (rc != SPGK_E_UNSUPPORTED) return rc;
+        }
+        // the opt-in for large dynamic shared memory is a per-device function attribute
+        static SpgOncePerDevice once;
         const int orc = once.run(dev, [&]() -> int {
             SPGK_CUDA(cudaFuncSetAttribute(spg_gemm_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dp.smem_optin));
             return SPGK_OK;
@@ -905,16 +913,16 @@ static int gemm_launch(const spgk_layer *L,
     p.out_rows = spg_tls_out_rows;
 
     CUtensorMap map_a, map_w;
-    int rc = make_map(&map_a, a16, type16, L->in, N, lda, a_plane, a_parts, BM);
+    int rc = spg_gemm_map(&map_a, a16, type16, L->in, N, lda, a_plane, a_parts, BM, 1);
     if (rc) return rc;
-    rc = make_map(&map_w, w16, w_type16, L->in, L->out, ldw, w_plane, w_parts, p.BN);
+    rc = spg_gemm_map(&map_w, w16, w_type16, L->in, L->out, ldw, w_plane, w_parts, p.BN, 1);
     if (rc) return rc;
 
     // 16-bit output through TMA stores when it is one plane and the tiles are wide enough for 64-column patches
     CUtensorMap map_o = map_a;
     p.tma_store = (out16 && out_parts == 1 && p.BN >= 128 && !softmax_fused && !head) ? 1 : 0;
     if (p.tma_store) {
-        rc = make_map(&map_o, out16, type16, ldo16, N, ldo16, o_plane, 1, 32);
+        rc = spg_gemm_map(&map_o, out16, type16, ldo16, N, ldo16, o_plane, 1, 32, 1);
         if (rc) return rc;
     }
     const uint32_t tiles = p.own_rows ? p.m_tiles : p.m_tiles * p.n_tiles;   // with a head or a wide softmax a CTA owns whole row tiles
