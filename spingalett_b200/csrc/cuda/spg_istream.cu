@@ -24,13 +24,11 @@
 // 106 us over the net, whose busiest SMs have 237 such blocks.  One byte per weight in the operand instead of two is why this
 // path exists beside the 16-bit streaming kernel, which writes and reads 32 KB per such block.
 //
-// Measured: 157 us at 8 rows (GEMV: 201), 211 at 64 (16-bit streaming kernel: 577), 628 at 256 (GEMM chain: 684).  From
-// layers of 32 to 166 blocks a CTA: at 8 rows 825 cycles a block and 14 us a layer (154 us for the net), at 64 rows 1000 and
-// 21 (207 us).  INT8, whose boxes need no unpacking, takes 725 cycles at 8 rows, 5.4 TB/s.  INT4 and INT2 are bound there by a
-// block's way through unpackers and MMA warp -- DRAM 29 %, shared memory 22 %, tensor pipe 6 %, issue slots 24 % of their peaks;
-// taking out the unpacking, the digit copies or the MMAs alone left the time within a few per cent, and so did two or eight
-// operand slots instead of four.  At 64 rows the tensor pipe needs 514 of the 1000 cycles and every CTA draws 32 KB of digits
-// a block from L2.  The 14 to 21 us of a layer are staging, the first boxes and tiles, and the last sums.
+// Measured: 125 us at 8 rows (GEMV: 201), 188 at 64 (16-bit streaming kernel: 577), 561 at 256 (GEMM chain: 684).  A block of
+// INT4 takes 480 cycles at 8 rows, of which the MMA warp's own turn is all (operand tiles changing hands one at a time: 810),
+// and 750 at 64 (900), where every CTA draws 32 KB of digits a block from L2 at 43 bytes a cycle; the tensor pipe would need
+// 512.  INT8, whose boxes need no unpacking, takes 725 cycles at 8 rows, 5.4 TB/s.  The rest of a layer is staging, the first
+// boxes and tiles, and the last sums (1 us at 8 rows, 3 at 64).
 //
 // Per CTA (one per SM, 19 warps):
 //   warp 0      weight boxes by TMA (128 rows x 128 packed bytes, 128-byte swizzle), ahead of the previous layer's end:
@@ -70,7 +68,8 @@ struct IsParams {
     uint32_t out, groups, rpg, N, C;                   // rows per group, batch rows, columns of a tile (4 * rpg)
     uint32_t rows;                                     // groups * rpg: rows of scales, a quarter of the rows of one set of digits
     uint32_t kbr, boxes;                               // 128-wide k-blocks per box, boxes per row tile
-    uint32_t RS, AS, BS;
+    uint32_t RS, AS, BS;                               // ring slots: boxes, operand (G blocks each), digits (GB blocks each)
+    uint32_t G, GB;
     uint64_t units;                                    // tiles * boxes
     uint32_t direct; int prec, act;
     double scale; const float *bias; const double *row_scale;
@@ -258,11 +257,11 @@ spg_is_stage_kernel(const float *__restrict__ x, uint32_t ldx, uint32_t N, uint3
 __device__ __forceinline__ void is_epi_sync() { asm volatile("bar.sync 2, %0;" ::"n"(32 * IS_EPI_WARPS) : "memory"); }
 
 // `rest`: bias, and the second set's share
+template <int ACT>
 __device__ __forceinline__ void is_finish(const IsParams &p, uint32_t n, uint32_t row, double rest, double scale, long long sum)
 {
-    if (row >= p.out || n >= p.N) return;
-    const double v = (double)sum * scale + rest;
-    p.y[(uint64_t)n * p.ldy + row] = spg_activate((float)v, p.act);
+    const float v = spg_activate((float)((double)sum * scale + rest), ACT);
+    if (row < p.out && n < p.N) p.y[(uint64_t)n * p.ldy + row] = v;
 }
 
 // Segments of a CTA: the runs of its units that lie in one tile.
@@ -294,8 +293,11 @@ __device__ __forceinline__ bool is_any_wide(const IsParams &p, uint32_t lane)
 
 // Epilogue role (warps 2..9): thread = one weight row (tensor-memory lane) of the tile; of two warps on the same lanes each
 // takes every other four batch rows.  `wide`: with the second set of digits, in loops of its own (its branches and registers in
-// the others took 1 to 2 us a layer).  `dirty`: a launch before this one failed and nobody has read its status yet, so the sums and
+// the others took 1 to 2 us a layer).  Turning a sum into an output is a chain of some 450 cycles (two conversions of 100 and 75
+// among them) and a scheduler has two of these warps: only values side by side hide it, so the activation is chosen outside and
+// nothing in the chain branches (with the choice inside, the last sums of a tile took 17500 cycles at 64 rows).  `dirty`: a launch before this one failed and nobody has read its status yet, so the sums and
 // counters cannot be relied on.
+template <int ACT>
 __device__ __forceinline__ void is_epilogue(const IsParams &p, bool wide, bool dirty, IsSegment seg, uint32_t tmem_base, uint32_t tfull0, uint32_t tempty0,
                                             volatile int *abort_flag, int *s_last, double *s_scale, uint32_t warp, uint32_t lane)
 {
@@ -333,12 +335,14 @@ __device__ __forceinline__ void is_epilogue(const IsParams &p, bool wide, bool d
                 tmem_ld16(taddr + c0, r);
                 tmem_ld_wait();
                 if (!ok) continue;
+                if (whole) {
 #pragma unroll
-                for (uint32_t i = 0; i < 4; i++) {
-                    const long long v = is_recombine(r + 4 * i);
-                    const uint32_t rr = (c0 >> 2) + i;
-                    if (whole) is_finish(p, n0 + rr, row, (double)bias, s_scale[rr], v);
-                    else atomicAdd(sums + (uint64_t)rr * TILE_ROWS, (unsigned long long)v);
+                    for (uint32_t i = 0; i < 4; i++)
+                        is_finish<ACT>(p, n0 + (c0 >> 2) + i, row, (double)bias, s_scale[(c0 >> 2) + i], is_recombine(r + 4 * i));
+                } else {
+#pragma unroll
+                    for (uint32_t i = 0; i < 4; i++)
+                        atomicAdd(sums + (uint64_t)((c0 >> 2) + i) * TILE_ROWS, (unsigned long long)is_recombine(r + 4 * i));
                 }
             }
         } else {
@@ -350,7 +354,7 @@ __device__ __forceinline__ void is_epilogue(const IsParams &p, bool wide, bool d
                 tmem_ld_wait();
                 if (!ok) continue;
                 const long long v = is_recombine(r), v2 = is_recombine(q);
-                if (whole) is_finish(p, n0 + rr, row, (double)bias + (double)v2 * s_scale[GROUP_ROWS + rr], s_scale[rr], v);
+                if (whole) is_finish<ACT>(p, n0 + rr, row, (double)bias + (double)v2 * s_scale[GROUP_ROWS + rr], s_scale[rr], v);
                 else {
                     atomicAdd(sums + (uint64_t)rr * TILE_ROWS, (unsigned long long)v);
                     atomicAdd(sums2 + (uint64_t)rr * TILE_ROWS, (unsigned long long)v2);
@@ -386,9 +390,9 @@ __device__ __forceinline__ void is_epilogue(const IsParams &p, bool wide, bool d
 #pragma unroll
                 for (uint32_t i = 0; i < 16; i++) {
                     const uint32_t rr = r0 + (i >> 2) * 8 + (i & 3u);
-                    if (rr >= p.rpg) continue;
-                    __stcg(sums + (uint64_t)rr * TILE_ROWS, 0ull);
-                    is_finish(p, n0 + rr, row, (double)bias, s_scale[rr], v[i]);
+                    const bool live = rr < p.rpg;
+                    if (live) __stcg(sums + (uint64_t)rr * TILE_ROWS, 0ull);
+                    is_finish<ACT>(p, live ? n0 + rr : p.N, row, (double)bias, s_scale[live ? rr : 0], v[i]);
                 }
             }
 #pragma unroll 1
@@ -396,7 +400,7 @@ __device__ __forceinline__ void is_epilogue(const IsParams &p, bool wide, bool d
                 const long long v = (long long)__ldcg(sums + (uint64_t)rr * TILE_ROWS), v2 = (long long)__ldcg(sums2 + (uint64_t)rr * TILE_ROWS);
                 __stcg(sums + (uint64_t)rr * TILE_ROWS, 0ull);
                 __stcg(sums2 + (uint64_t)rr * TILE_ROWS, 0ull);
-                is_finish(p, n0 + rr, row, (double)bias + (double)v2 * s_scale[GROUP_ROWS + rr], s_scale[rr], v);
+                is_finish<ACT>(p, n0 + rr, row, (double)bias + (double)v2 * s_scale[GROUP_ROWS + rr], s_scale[rr], v);
             }
             if (warp == 2 && lane == 0) p.counters[seg.tile] = 0;
         }
@@ -404,26 +408,30 @@ __device__ __forceinline__ void is_epilogue(const IsParams &p, bool wide, bool d
     }
 }
 
-// Digit tiles of a CTA that go out before it is known whether the layer has a wide row: one per ring slot at most.  They are
-// the first set's tiles of consecutive blocks, which is the order of a layer without wide rows; in a wide one, where the sets
-// alternate, they are thrown away.
-__device__ __forceinline__ uint32_t is_early_tiles(const IsParams &p, const IsSegment &seg)
+// Digit slots of a CTA that go out before it is known whether the layer has a wide row: the ring at most.  They are the first
+// set's of consecutive blocks, which is the order of a layer without wide rows; in a wide one, where the sets alternate, they
+// are thrown away.
+__device__ __forceinline__ uint32_t is_early_slots(const IsParams &p, const IsSegment &seg)
 {
-    const uint64_t tiles = (seg.end - seg.u) * p.kbr;
-    return tiles < p.BS ? (uint32_t)tiles : p.BS;
+    const uint64_t slots = (seg.end - seg.u) * p.kbr / p.GB;
+    return slots < p.BS ? (uint32_t)slots : p.BS;
 }
 
-// MMA role (warp 1): SETS sets of digits per 128-wide block of weights (a number known to the compiler: the warp's turn bounds
-// the kernel, and a counted loop over the sets took 3 us of the 65 that 256 rows of a 4096-4096-1024 net take)
+// MMA role (warp 1): SETS sets of digits per 128-wide block of weights.  The warp's own turn bounds the kernel at small
+// batches: a wait costs it some 100 cycles even when there is nothing to wait for, a commit as much, an MMA 45 to 128.  So
+// operand tiles change hands G blocks at a time and digit tiles GB (a divisor of G), and all three are numbers known to the
+// compiler (a counted loop over the sets took 3 us of the 65 that 256 rows of a 4096-4096-1024 net take).  At 8 rows of INT4 a
+// block then takes the warp 480 cycles; it took 810 one at a time.
 struct IsBars { uint32_t rfull0, rempty0, afull0, aempty0, bfull0, bempty0, tfull0, tempty0; };
-template <uint32_t SETS>
+template <uint32_t SETS, uint32_t G, uint32_t GB>
 __device__ __forceinline__ void is_mma(const IsParams &p, IsSegment seg, const IsBars &bar, uint64_t a_desc0, uint64_t b_desc0, uint32_t tmem_base,
                                        uint32_t abort_addr, volatile int *abort_flag)
 {
-    uint32_t rs = 0, rph = 0, as = 0, aph = 0, bs = 0, bph = 0, count = 0;
-    const uint32_t b_step = p.C * 128u >> 4;
+    uint32_t as = 0, aph = 0, bs = 0, bph = 0, count = 0;      // G = 1: the boxes are the operand
+    const uint32_t b_step = p.C * 128u >> 4, slots = G == 1 ? p.RS : p.AS;
+    const uint32_t full0 = G == 1 ? bar.rfull0 : bar.afull0, empty0 = G == 1 ? bar.rempty0 : bar.aempty0;
     if (SETS == 2) {
-        const uint32_t early = is_early_tiles(p, seg);
+        const uint32_t early = is_early_slots(p, seg);
         for (uint32_t i = 0; i < early; i++) {
             mbar_wait_uniform(bar.bfull0 + 8 * bs, bph, abort_addr, p.status, 10);
             if (*abort_flag) return;
@@ -439,30 +447,33 @@ __device__ __forceinline__ void is_mma(const IsParams &p, IsSegment seg, const I
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + acc * p.C;
         uint32_t accum = 0;
-        const uint32_t blocks = (seg.k1 - seg.k0) * p.kbr;
-        for (uint32_t kb = 0; kb < blocks; kb++) {
-            if (p.direct) mbar_wait_uniform(bar.rfull0 + 8 * rs, rph, abort_addr, p.status, 4);
-            else mbar_wait_uniform(bar.afull0 + 8 * as, aph, abort_addr, p.status, 5);
-            const uint64_t da = a_desc0 + (uint64_t)((p.direct ? rs : as) * (BOX_BYTES >> 4));
+        const uint32_t turns = (seg.k1 - seg.k0) * p.kbr / G;  // (kbr is a multiple of G)
+        for (uint32_t turn = 0; turn < turns; turn++) {
+            mbar_wait_uniform(full0 + 8 * as, aph, abort_addr, p.status, G == 1 ? 4 : 5);
+            const uint64_t da = a_desc0 + (uint64_t)(as * G * (BOX_BYTES >> 4));
 #pragma unroll
-            for (uint32_t set = 0; set < SETS; set++) {
-                mbar_wait_uniform(bar.bfull0 + 8 * bs, bph, abort_addr, p.status, 6);
-                if (*abort_flag) return;
-                tc_fence_after();
-                const uint64_t db = b_desc0 + (uint64_t)(bs * b_step);
-                if (elect_one()) {
-                    uint32_t acc_in = accum;
+            for (uint32_t j = 0; j < G; j += GB) {
 #pragma unroll
-                    for (uint32_t k = 0; k < 4; k++) { umma_i8(d_tmem + set * p.C, da + 2 * k, db + 2 * k, p.idesc, acc_in); acc_in = 1; }
-                    umma_commit(bar.bempty0 + 8 * bs);
-                    if (set + 1 == SETS) umma_commit(p.direct ? bar.rempty0 + 8 * rs : bar.aempty0 + 8 * as);
+                for (uint32_t set = 0; set < SETS; set++) {
+                    mbar_wait_uniform(bar.bfull0 + 8 * bs, bph, abort_addr, p.status, 6);
+                    if (*abort_flag) return;
+                    tc_fence_after();
+                    const uint64_t db = b_desc0 + (uint64_t)(bs * GB * b_step);
+                    if (elect_one()) {
+#pragma unroll
+                        for (uint32_t i = 0; i < GB; i++)
+#pragma unroll
+                            for (uint32_t k = 0; k < 4; k++)
+                                umma_i8(d_tmem + set * p.C, da + (j + i) * (BOX_BYTES >> 4) + 2 * k, db + i * b_step + 2 * k, p.idesc, j + i + k ? 1u : accum);
+                        umma_commit(bar.bempty0 + 8 * bs);
+                        if (j + GB == G && set + 1 == SETS) umma_commit(empty0 + 8 * as);
+                    }
+                    __syncwarp();
+                    if (++bs == p.BS) { bs = 0; bph ^= 1u; }
                 }
-                __syncwarp();
-                if (++bs == p.BS) { bs = 0; bph ^= 1u; }
             }
             accum = 1;
-            if (p.direct) { if (++rs == p.RS) { rs = 0; rph ^= 1u; } }
-            else if (++as == p.AS) { as = 0; aph ^= 1u; }
+            if (++as == slots) { as = 0; aph ^= 1u; }
         }
         if (elect_one()) umma_commit(bar.tfull0 + 8 * acc);
         __syncwarp();
@@ -479,8 +490,8 @@ spg_istream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     // layout: box ring | operand ring (absent for INT8) | digit ring | barriers | flags | scales of a group, both sets
     const uint32_t b_bytes = p.C * 128u;
     const uint32_t a_off = p.RS * BOX_BYTES;
-    const uint32_t b_off = a_off + (p.direct ? 0u : p.AS * BOX_BYTES);
-    const uint32_t bar_off = b_off + p.BS * b_bytes;
+    const uint32_t b_off = a_off + (p.direct ? 0u : p.AS * p.G * BOX_BYTES);
+    const uint32_t bar_off = b_off + p.BS * p.GB * b_bytes;
     const uint32_t rfull0 = base + bar_off, rempty0 = rfull0 + 8 * p.RS;
     const uint32_t afull0 = rempty0 + 8 * p.RS, aempty0 = afull0 + 8 * p.AS;
     const uint32_t bfull0 = aempty0 + 8 * p.AS, bempty0 = bfull0 + 8 * p.BS;
@@ -538,13 +549,14 @@ spg_istream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         }
     } else if (warp == IS_DIGIT_WARP) {
         // ------------------------------ digit tiles -------------------------------
-        uint32_t bs = 0, bph = 0, early = is_early_tiles(p, seg);
+        uint32_t bs = 0, bph = 0, early = is_early_slots(p, seg);
         auto load = [&](uint32_t kb, uint32_t row) {
             mbar_wait_uniform(bempty0 + 8 * bs, bph ^ 1u, abort_addr, p.status, 2);
             if (*abort_flag) return;
             if (elect_one()) {
-                mbar_expect_tx(bfull0 + 8 * bs, b_bytes);
-                tma_load_2d(base + b_off + bs * b_bytes, &map_x, bfull0 + 8 * bs, (int)(kb * 128u), (int)row);
+                mbar_expect_tx(bfull0 + 8 * bs, p.GB * b_bytes);
+                for (uint32_t i = 0; i < p.GB; i++)
+                    tma_load_2d(base + b_off + (bs * p.GB + i) * b_bytes, &map_x, bfull0 + 8 * bs, (int)((kb + i) * 128u), (int)row);
             }
             __syncwarp();
             if (++bs == p.BS) { bs = 0; bph ^= 1u; }
@@ -552,12 +564,12 @@ spg_istream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         spg_grid_wait();
         IsSegment ahead = seg;
         for (uint32_t left = early; left && is_next_segment(p, ahead);)
-            for (uint32_t kb = ahead.k0 * p.kbr; left && kb < ahead.k1 * p.kbr; kb++, left--) load(kb, ahead.tile % p.groups * p.C);
+            for (uint32_t kb = ahead.k0 * p.kbr; left && kb < ahead.k1 * p.kbr; kb += p.GB, left--) load(kb, ahead.tile % p.groups * p.C);
         const uint32_t sets = is_any_wide(p, lane) ? 2 : 1;
         if (sets == 2) early = 0;
         while (is_next_segment(p, seg)) {
             const uint32_t c0 = seg.tile % p.groups * p.C;
-            for (uint32_t kb = seg.k0 * p.kbr; kb < seg.k1 * p.kbr; kb++) {
+            for (uint32_t kb = seg.k0 * p.kbr; kb < seg.k1 * p.kbr; kb += p.GB) {
                 if (early) { early--; continue; }                              // has gone out
                 for (uint32_t set = 0; set < sets; set++) {
                     load(kb, c0 + set * 4 * p.rows);
@@ -570,17 +582,22 @@ spg_istream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         const IsBars bar = { rfull0, rempty0, afull0, aempty0, bfull0, bempty0, tfull0, tempty0 };
         const uint64_t a_desc0 = smem_desc_sw128(p.direct ? base : base + a_off), b_desc0 = smem_desc_sw128(base + b_off);
         spg_grid_wait();
-        if (is_any_wide(p, lane)) is_mma<2>(p, seg, bar, a_desc0, b_desc0, tmem_base, abort_addr, abort_flag);
-        else is_mma<1>(p, seg, bar, a_desc0, b_desc0, tmem_base, abort_addr, abort_flag);
+#define IS_MMA(SETSV, GV, GBV) is_mma<SETSV, GV, GBV>(p, seg, bar, a_desc0, b_desc0, tmem_base, abort_addr, abort_flag)
+        const bool wide = is_any_wide(p, lane);
+        if (p.direct) { if (wide) IS_MMA(2, 1, 1); else IS_MMA(1, 1, 1); }
+        else if (p.GB == 1) { if (wide) IS_MMA(2, 2, 1); else IS_MMA(1, 2, 1); }
+        else { if (wide) IS_MMA(2, 2, 2); else IS_MMA(1, 2, 2); }
+#undef IS_MMA
     } else if (warp >= IS_CONV_WARP0) {
         // ------------------------------ unpackers ---------------------------------
-        // AS groups of 8 / AS warps; group g makes the operand tiles of the k-blocks whose running number is g mod AS, always
-        // in ring slot g, so AS tiles are in the making at once and the latency of one (load, unpack, store, proxy fence,
-        // arrive) hides behind the others.  Lanes 0-7 of a quarter warp take eight different rows of a swizzle atom: no bank
+        // A group of warps for each of the AS * G operand tiles that the ring holds; group g makes the tiles of the k-blocks whose
+        // running number is g mod AS * G, always in place g, so that many tiles are in the making at once and the latency of one
+        // (load, unpack, store, proxy fence, arrive: 600 cycles) hides behind the others.  Lanes 0-7 of a quarter warp take eight different rows of a swizzle atom: no bank
         // conflict on either side.  (Sixteen warps instead of eight: 2 to 5 % slower at every batch size.)
         if (!p.direct) {
-            const uint32_t wpg = IS_CONV_WARPS / p.AS, TG = 32u * wpg;
+            const uint32_t tiles = p.AS * p.G, wpg = IS_CONV_WARPS / tiles, TG = 32u * wpg;
             const uint32_t cw = warp - IS_CONV_WARP0, grp = cw / wpg, ctg = (cw % wpg) * 32u + lane;
+            const uint32_t afull = afull0 + 8 * (grp / p.G), aempty = aempty0 + 8 * (grp / p.G);
             uint32_t rs = 0, rph = 0, as = 0, aph = 0;
             uint8_t *atile = smem + a_off + grp * BOX_BYTES;
             spg_grid_wait();
@@ -590,7 +607,7 @@ spg_istream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                     const uint8_t *box = smem + rs * BOX_BYTES;
                     for (uint32_t j = 0; j < p.kbr; j++) {
                         if (as == grp) {
-                            const bool ok = okr && mbar_wait(aempty0 + 8 * as, aph ^ 1u, abort_flag, p.status, 8);
+                            const bool ok = okr && mbar_wait(aempty, aph ^ 1u, abort_flag, p.status, 8);
                             if (ok && p.prec == SPG_P_I4) {
                                 // a 128-wide block is pieces 4j .. 4j+3 (16 bytes, 32 nibbles) of each packed row
                                 for (uint32_t u0 = ctg; u0 < 512; u0 += 4 * TG) {
@@ -627,9 +644,9 @@ spg_istream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                             }
                             fence_async_smem();          // the tensor core reads the tile through the async proxy
                             __syncwarp();
-                            if (lane == 0) mbar_arrive(afull0 + 8 * as);
+                            if (lane == 0) mbar_arrive(afull);
                         }
-                        if (++as == p.AS) { as = 0; aph ^= 1u; }
+                        if (++as == tiles) { as = 0; aph ^= 1u; }
                     }
                     __syncwarp();
                     if (lane == 0) mbar_arrive(rempty0 + 8 * rs);
@@ -647,7 +664,16 @@ spg_istream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         is_epi_sync();
         const int found = *s_last;
         is_epi_sync();
-        is_epilogue(p, found & 1, found & 2, seg, tmem_base, tfull0, tempty0, abort_flag, s_last, s_scale, warp, lane);
+#define IS_EPI(ACTV) is_epilogue<ACTV>(p, found & 1, found & 2, seg, tmem_base, tfull0, tempty0, abort_flag, s_last, s_scale, warp, lane)
+        switch (p.act) {
+            case SPG_ACT_RELU:    IS_EPI(SPG_ACT_RELU); break;
+            case SPG_ACT_LEAKY:   IS_EPI(SPG_ACT_LEAKY); break;
+            case SPG_ACT_FOO52:   IS_EPI(SPG_ACT_FOO52); break;
+            case SPG_ACT_TANH:    IS_EPI(SPG_ACT_TANH); break;
+            case SPG_ACT_SIGMOID: IS_EPI(SPG_ACT_SIGMOID); break;
+            default:              IS_EPI(SPG_ACT_NONE); break;
+        }
+#undef IS_EPI
     }
 is_role_done:
     tc_fence_before();
@@ -663,7 +689,7 @@ is_role_done:
 // ---- host side ---------------------------------------------------------------------------------------------------------
 
 struct IsPlan {
-    uint32_t groups, rpg, C, kbr, boxes, ld, m_tiles, tiles, RS, AS, BS, grid;
+    uint32_t groups, rpg, C, kbr, boxes, ld, m_tiles, tiles, RS, AS, BS, G, GB, grid;
     uint64_t units;
     size_t operand_bytes, smem;
     bool direct, ok;
@@ -693,15 +719,18 @@ IsPlan is_plan(const spgk_layer *L, uint32_t N, uint32_t sms)
     // one CTA per SM, but a tile in about four pieces at most: the sum over more of them costs more than they save
     const uint64_t want = (uint64_t)pl.tiles * (pl.boxes < 4 ? pl.boxes : 4);
     pl.grid = want < sms ? (uint32_t)want : sms;
-    // rings: four operand tiles (one per unpacker group), digit tiles up to 96 KB, boxes with the rest
+    // rings: operand tiles in two slots of G blocks, digit tiles up to 96 KB (in pairs up to 32 rows), boxes with the rest
     const uint32_t b_bytes = pl.C * 128u;
-    pl.AS = pl.direct ? 1 : 4;
+    pl.G = pl.direct ? 1 : 2;
+    pl.AS = pl.direct ? 1 : 2;
+    pl.GB = pl.direct || b_bytes > 16384 ? 1 : 2;
     pl.BS = 96u * 1024 / b_bytes;
     if (pl.BS > 8) pl.BS = 8;
-    const uint32_t a_bytes = pl.direct ? 0 : pl.AS * BOX_BYTES;
-    pl.RS = (224u * 1024 - a_bytes - pl.BS * b_bytes) / BOX_BYTES;
+    pl.BS /= pl.GB;
+    const uint32_t a_bytes = pl.direct ? 0 : pl.AS * pl.G * BOX_BYTES;
+    pl.RS = (224u * 1024 - a_bytes - pl.BS * pl.GB * b_bytes) / BOX_BYTES;
     if (pl.RS > 10) pl.RS = 10;
-    pl.smem = 1024 + (size_t)pl.RS * BOX_BYTES + a_bytes + (size_t)pl.BS * b_bytes + 16 * (pl.RS + pl.AS + pl.BS) + 32 + 16 + 2 * GROUP_ROWS * sizeof(double);
+    pl.smem = 1024 + (size_t)pl.RS * BOX_BYTES + a_bytes + (size_t)pl.BS * pl.GB * b_bytes + 16 * (pl.RS + pl.AS + pl.BS) + 32 + 16 + 2 * GROUP_ROWS * sizeof(double);
     pl.operand_bytes = 2 * (size_t)pl.groups * pl.C * pl.ld;              // both sets of digits
     pl.ok = pl.smem <= 227u * 1024;
     return pl;
@@ -814,7 +843,7 @@ int spgk_istream_forward(const spgk_layer *layers, uint32_t count, const float *
         IsParams p{};
         p.out = L->out; p.groups = pl.groups; p.rpg = pl.rpg; p.N = N; p.C = pl.C; p.rows = pl.groups * pl.rpg;
         p.kbr = pl.kbr; p.boxes = pl.boxes; p.units = pl.units;
-        p.RS = pl.RS; p.AS = pl.AS; p.BS = pl.BS;
+        p.RS = pl.RS; p.AS = pl.AS; p.BS = pl.BS; p.G = pl.G; p.GB = pl.GB;
         p.direct = pl.direct; p.prec = L->precision;
         p.act = L->act == SPG_ACT_SOFTMAX ? SPG_ACT_NONE : L->act;
         p.scale = (double)L->w_scale / (L->precision == SPG_P_I4 ? 16.0 : L->precision == SPG_P_I2 ? 64.0 : 1.0);
