@@ -51,34 +51,45 @@ size_t spg_array_bytes(uint64_t count, PrecisionMode p)
     }
 }
 
+/* elements lo .. hi-1 of an array; src: its first element (behind the abs-max of an integer format).  The integer formats have
+ * 256, 16 or 4 values: the table holds (q / Q) * amax for each of them. */
+typedef struct { const uint8_t *src; PrecisionMode p; float *dst; const float *table; } decode_ctx;
+static void decode_slice(void *ctx, size_t lo, size_t hi)
+{
+    const decode_ctx *c = ctx;
+    const uint8_t *src = c->src;
+    const float *table = c->table;
+    float *dst = c->dst;
+    switch (c->p) {
+        case PRECISION_FLOAT32: memcpy(dst + lo, src + 4 * lo, 4 * (hi - lo)); break;
+        case PRECISION_FP16:
+        case PRECISION_BFLOAT16:
+            for (size_t i = lo; i < hi; i++) {
+                uint16_t h; memcpy(&h, src + 2 * i, 2);
+                dst[i] = c->p == PRECISION_FP16 ? dec_f16(h) : float_of((uint32_t)h << 16);
+            }
+            break;
+        case PRECISION_INT8: for (size_t i = lo; i < hi; i++) dst[i] = table[src[i]]; break;
+        case PRECISION_INT4: for (size_t i = lo; i < hi; i++) dst[i] = table[(src[i >> 1] >> ((i & 1) * 4)) & 0xF]; break;
+        default:             for (size_t i = lo; i < hi; i++) dst[i] = table[(src[i >> 2] >> ((i & 3) * 2)) & 3]; break;
+    }
+}
+
 void spg_decode_array(const uint8_t *src, uint64_t count, PrecisionMode p, float *dst)
 {
-    if (p == PRECISION_FLOAT32) { memcpy(dst, src, 4 * count); return; }
-    if (p == PRECISION_FP16 || p == PRECISION_BFLOAT16) {
-        for (uint64_t i = 0; i < count; i++) {
-            uint16_t h; memcpy(&h, src + 2 * i, 2);
-            dst[i] = p == PRECISION_FP16 ? dec_f16(h) : float_of((uint32_t)h << 16);
-        }
-        return;
-    }
-    float amax; memcpy(&amax, src, 4);
-    src += 4;
-    if (!(amax > 0.0f)) { memset(dst, 0, 4 * count); return; }
-    if (p == PRECISION_INT8) {
-        for (uint64_t i = 0; i < count; i++) dst[i] = ((float)(int8_t)src[i] / 127.0f) * amax;
-    } else if (p == PRECISION_INT4) {
-        for (uint64_t i = 0; i < count; i++) {
-            int v = (src[i >> 1] >> ((i & 1) * 4)) & 0xF;
-            if (v & 8) v -= 16;
-            dst[i] = ((float)v / 7.0f) * amax;
-        }
-    } else {
-        for (uint64_t i = 0; i < count; i++) {
-            int v = (src[i >> 2] >> ((i & 3) * 2)) & 3;
-            if (v & 2) v -= 4;
-            dst[i] = (float)v * amax;
+    float table[256];
+    if (p >= PRECISION_INT8) {
+        float amax; memcpy(&amax, src, 4);
+        src += 4;
+        if (!(amax > 0.0f)) { memset(dst, 0, 4 * count); return; }
+        const int values = p == PRECISION_INT8 ? 256 : p == PRECISION_INT4 ? 16 : 4;
+        for (int v = 0; v < values; v++) {
+            const float q = (float)(v < values / 2 ? v : v - values);
+            table[v] = p == PRECISION_INT2 ? q * amax : (q / spg_precision_q(p)) * amax;
         }
     }
+    decode_ctx c = { src, p, dst, table };
+    spg_bulk(decode_slice, &c, (size_t)count, 4096, (size_t)1 << 18);
 }
 
 size_t spg_encode_array(const float *src, uint64_t count, PrecisionMode p, uint8_t *dst)

@@ -91,7 +91,7 @@ static void shadows_release(spg_net *n)
 
 void spg_dev_invalidate(spg_net *n) { shadows_release(n); if (n->dev_ready) spg_dev_release(n); }
 
-static int bind_device(spg_net *n)
+int spg_dev_bind(spg_net *n)
 {
     if (n->device < 0) {
         int count = 0;
@@ -161,7 +161,7 @@ int spg_dev_ensure(spg_net *n)
     if (n->dev_ready) return spg_map_kernel_error(spgk_set_device(n->device), "bind device");
     NeuralNetwork *p = &n->pub;
     if (p->layers < 2) { spg_set_error(SPINGALETT_ERR_INVALID, "network has no weight layer"); return SPINGALETT_ERR_INVALID; }
-    int rc = bind_device(n);
+    int rc = spg_dev_bind(n);
     if (rc) return rc;
     uint32_t wl = p->layers - 1;
     n->d_w = calloc(wl, sizeof *n->d_w);
@@ -902,45 +902,6 @@ int spg_dev_forward_large(spg_net *n, const float *d_x, uint32_t N, float *d_out
 
 static float *forward_batch_on(spg_net *n, ForwardBatchArgs a);
 
-/* A pageable source is copied into page-locked staging by several host threads at once: one thread (what a cudaMemcpy
- * from pageable memory amounts to) moves about 11 GB/s, a third of what the host link takes. */
-#define SPG_STAGE_THREADS 16    /* most; SPINGALETT_STAGE_THREADS in the environment asks for fewer */
-typedef struct { char *dst; const char *src; size_t bytes; } stage_job;
-static void *stage_worker(void *arg)
-{
-    stage_job *j = arg;
-    memcpy(j->dst, j->src, j->bytes);
-    return NULL;
-}
-static void stage_copy(void *dst, const void *src, size_t bytes)
-{
-    static int want = 0;
-    if (!want) {
-        const char *e = getenv("SPINGALETT_STAGE_THREADS");
-        const long cores = sysconf(_SC_NPROCESSORS_ONLN);
-        want = e && atoi(e) > 0 ? atoi(e) : (cores >= 16 ? 8 : cores >= 4 ? (int)(cores / 2) : 1);
-        if (want > SPG_STAGE_THREADS) want = SPG_STAGE_THREADS;
-    }
-    int nt = want;
-    if (bytes < ((size_t)4 << 20)) nt = 1;
-    pthread_t th[SPG_STAGE_THREADS];
-    stage_job jobs[SPG_STAGE_THREADS];
-    const size_t share = ((bytes / (size_t)nt) + 4095) & ~(size_t)4095;
-    int started = 0;
-    for (int t = 1; t < nt; t++) {
-        const size_t off = (size_t)t * share;
-        if (off >= bytes) break;
-        jobs[t] = (stage_job){ (char *)dst + off, (const char *)src + off, bytes - off < share ? bytes - off : share };
-        if (pthread_create(&th[t], NULL, stage_worker, &jobs[t]) != 0) {        /* no thread: this one copies the rest */
-            memcpy((char *)dst + off, (const char *)src + off, bytes - off);
-            break;
-        }
-        started = t;
-    }
-    memcpy(dst, src, bytes < share || nt == 1 ? bytes : share);
-    for (int t = 1; t <= started; t++) pthread_join(th[t], NULL);
-}
-
 /* a replica record for device `dev`: shares the host arrays and the packed payload of `n`, owns its device image */
 static spg_net *shadow_for(spg_net *n, int slot, int dev)
 {
@@ -1151,15 +1112,22 @@ static float *forward_batch_on(spg_net *n, ForwardBatchArgs a)
             for (uint32_t c = 0; c <= chunks; c++) {
                 if (c < chunks) {
                     const size_t r0 = (size_t)c * chunk_rows, rows = N - r0 < chunk_rows ? N - r0 : chunk_rows;
-                    const float *src = a.inputs + r0 * in0;
-                    if (staged) {
-                        /* the staging buffer of chunk c was last read by the copy of chunk c-2 */
-                        if (c >= 2 && spg_map_kernel_error(spgk_event_sync(n->copy_ev[c - 1]), "forward_batch: staging")) return NULL;
-                        stage_copy(n->h_chunk[c & 1], src, rows * in0 * sizeof(float));
-                        src = n->h_chunk[c & 1];
+                    /* the staging buffer of chunk c was last read by the copy of chunk c-2; a staged chunk goes out in two
+                       pieces, so that the link has work while the second is staged */
+                    if (staged && c >= 2 && spg_map_kernel_error(spgk_event_sync(n->copy_ev[c - 1]), "forward_batch: staging")) return NULL;
+                    const size_t piece = staged ? (rows / 2 + 7) & ~(size_t)7 : rows;      /* (8 rows: the copy's 32-byte boundaries) */
+                    int rc = SPINGALETT_OK;
+                    for (size_t p0 = 0; p0 < rows && !rc; p0 += piece) {
+                        const size_t pr = rows - p0 < piece ? rows - p0 : piece;
+                        const float *src = a.inputs + (r0 + p0) * in0;
+                        if (staged) {
+                            float *at = n->h_chunk[c & 1] + p0 * in0;
+                            spg_stage_copy(at, src, pr * in0 * sizeof(float));
+                            src = at;
+                        }
+                        rc = spg_map_kernel_error(spgk_memcpy_h2d(n->d_in32 + (r0 + p0) * in0, src, pr * in0 * sizeof(float), n->copy_stream), "forward_batch: input copy");
                     }
-                    if (spg_map_kernel_error(spgk_memcpy_h2d(n->d_in32 + r0 * in0, src, rows * in0 * sizeof(float), n->copy_stream),
-                                             "forward_batch: input copy") ||
+                    if (rc ||
                         spg_map_kernel_error(spgk_event_record(n->copy_ev[c + 1], n->copy_stream), "forward_batch: pipeline")) return NULL;
                 }
                 if (c >= 1) {

@@ -23,6 +23,7 @@
 typedef struct spg_net_s {
     NeuralNetwork pub;          /* MUST stay first: &net->pub == (NeuralNetwork *)net */
     uint32_t magic;
+    uint64_t expect_w, expect_b;    /* elements that pub.weights / biases were made for ahead of the layers (zeros beyond the layers so far) */
 
     /* Weights as stored.  For a net read from a .nn file these are the packed
      * arrays of the file (without the abs-max prefix, which is kept in
@@ -109,6 +110,10 @@ SPG_HIDDEN float spg_rand_uniform_pm1(void);
 SPG_HIDDEN float spg_rand_normal(void);
 SPG_HIDDEN uint32_t spg_rand_u32(void);
 SPG_HIDDEN void spg_shuffle(uint32_t *idx, uint32_t n);
+/* bulk.c */
+typedef void (*spg_slice_fn)(void *ctx, size_t lo, size_t hi);
+SPG_HIDDEN void spg_bulk(spg_slice_fn fn, void *ctx, size_t n, size_t grain, size_t least);
+SPG_HIDDEN void spg_stage_copy(void *dst, const void *src, size_t bytes);
 /* codec.c */
 SPG_HIDDEN size_t spg_array_bytes(uint64_t count, PrecisionMode p);
 SPG_HIDDEN void spg_decode_array(const uint8_t *src, uint64_t count, PrecisionMode p, float *dst);
@@ -116,9 +121,11 @@ SPG_HIDDEN size_t spg_encode_array(const float *src, uint64_t count, PrecisionMo
 SPG_HIDDEN float spg_precision_q(PrecisionMode p);
 /* network.c */
 SPG_HIDDEN int spg_net_ensure_train_arrays(spg_net *n);
+SPG_HIDDEN bool spg_net_expect(spg_net *n, uint64_t weights, uint64_t biases);
 SPG_HIDDEN void spg_net_drop_payload(spg_net *n);
 /* device.c */
 SPG_HIDDEN int spg_dev_ensure(spg_net *n);           /* upload if needed */
+SPG_HIDDEN int spg_dev_bind(spg_net *n);             /* the net's device, made current */
 SPG_HIDDEN void spg_dev_release(spg_net *n);
 SPG_HIDDEN void spg_dev_invalidate(spg_net *n);
 SPG_HIDDEN int spg_dev_forward_small(spg_net *n, const float *d_x, uint32_t ldx, uint32_t N, float **d_last, float *d_final);

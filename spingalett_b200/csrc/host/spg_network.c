@@ -38,6 +38,23 @@ static bool grow_f32(float **arr, uint64_t old_count, uint64_t new_count)
     return true;
 }
 
+/* Makes the parameter arrays of an empty net for the layers that are about to be appended: untouched zero pages, which the
+ * loader's threads then fill, instead of arrays that every layer extends and clears. */
+bool spg_net_expect(spg_net *pn, uint64_t weights, uint64_t biases)
+{
+    NeuralNetwork *n = &pn->pub;
+    if (n->weights || n->biases) return true;
+    n->weights = zeros_f32(weights);
+    n->biases = zeros_f32(biases);
+    if (!n->weights || !n->biases) {
+        free(n->weights); free(n->biases);
+        n->weights = n->biases = NULL;
+        return false;
+    }
+    pn->expect_w = weights; pn->expect_b = biases;
+    return true;
+}
+
 static void recompute_offsets(NeuralNetwork *n)
 {
     uint64_t no = 0, wo = 0, bo = 0;
@@ -128,7 +145,10 @@ void layer_struct_arguments(LayerArgs args)
     bool ok = topo && noff && woff && boff && (!has_weights || acts);
     ok = ok && grow_f32(&n->neurons, old_n, old_n + args.neurons_amount);
     if (ok && has_weights) {
-        ok = grow_f32(&n->weights, old_w, old_w + add_w) && grow_f32(&n->biases, old_b, old_b + add_b);
+        ok = (old_w + add_w <= pn->expect_w || grow_f32(&n->weights, old_w, old_w + add_w)) &&
+             (old_b + add_b <= pn->expect_b || grow_f32(&n->biases, old_b, old_b + add_b));
+        if (ok && old_w + add_w > pn->expect_w) pn->expect_w = 0;      /* grown past what was made ahead: as without it */
+        if (ok && old_b + add_b > pn->expect_b) pn->expect_b = 0;
         /* arrays that only exist once training has run keep their contents too */
         if (ok && n->grad_weights)
             ok = grow_f32(&n->grad_weights, old_w, old_w + add_w) && grow_f32(&n->grad_biases, old_b, old_b + add_b) &&

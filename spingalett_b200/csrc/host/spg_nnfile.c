@@ -13,6 +13,8 @@
 #include <stdio.h>
 #include <stdlib.h>
 #include <string.h>
+#include <errno.h>
+#include <unistd.h>
 
 typedef struct { const uint8_t *p; size_t len, pos; } cursor;
 
@@ -24,6 +26,19 @@ static bool take(cursor *c, void *dst, size_t n)
     return true;
 }
 
+/* bytes lo .. hi-1 of a regular file; a read that fails or comes up short is noted */
+typedef struct { int fd; uint8_t *buf; int failed; } read_ctx;
+static void read_slice(void *ctx, size_t lo, size_t hi)
+{
+    read_ctx *c = ctx;
+    while (lo < hi) {
+        const ssize_t got = pread(c->fd, c->buf + lo, hi - lo, (off_t)lo);
+        if (got < 0 && errno == EINTR) continue;
+        if (got <= 0) { __atomic_store_n(&c->failed, 1, __ATOMIC_RELAXED); return; }
+        lo += (size_t)got;
+    }
+}
+
 static uint8_t *slurp(const char *path, size_t *len)
 {
     FILE *f = fopen(path, "rb");
@@ -33,12 +48,23 @@ static uint8_t *slurp(const char *path, size_t *len)
         long sz = ftell(f);
         if (sz >= 0 && fseek(f, 0, SEEK_SET) == 0) {
             buf = malloc((size_t)sz + 1);
-            if (buf && fread(buf, 1, (size_t)sz, f) != (size_t)sz) { free(buf); buf = NULL; }
+            if (buf) {
+                read_ctx c = { fileno(f), buf, 0 };
+                spg_bulk(read_slice, &c, (size_t)sz, 4096, (size_t)1 << 20);
+                if (c.failed) { free(buf); buf = NULL; }
+            }
             *len = (size_t)sz;
         }
     }
     fclose(f);
     return buf;
+}
+
+typedef struct { uint8_t *dst; const uint8_t *src; } keep_ctx;
+static void keep_slice(void *ctx, size_t lo, size_t hi)
+{
+    const keep_ctx *c = ctx;
+    memcpy(c->dst + lo, c->src + lo, hi - lo);
 }
 
 /* read one stored array: decode to fp32 and optionally keep the packed bytes */
@@ -54,7 +80,8 @@ static bool read_array(cursor *c, uint32_t count, PrecisionMode p, float *dst, u
         *keep_bytes = nbytes - skip;
         *keep = malloc(*keep_bytes ? *keep_bytes : 1);
         if (!*keep) return false;
-        memcpy(*keep, src + skip, *keep_bytes);
+        keep_ctx k = { *keep, src + skip };
+        spg_bulk(keep_slice, &k, *keep_bytes, 4096, (size_t)1 << 20);
     }
     c->pos += nbytes;
     return true;
@@ -100,6 +127,16 @@ NeuralNetwork *load_spingalett(const char *filename)
     net = new_spingalett_struct_arguments((NeuralNetworkArgs){ .loss_func = (LossFunction)loss });
     if (!net) { spg_set_error(SPINGALETT_ERR_ALLOC, "load: network creation failed"); goto fail; }
     net->time_step = time_step;
+    /* the parameter arrays in one go, if the file is long enough to fill them (a topology that the file does not bear out
+       allocates layer by layer, as far as that goes) */
+    uint64_t all_w = 0, all_b = 0;
+    bool sane = true;
+    for (uint32_t l = 0; l + 1 < layers && sane; l++) {
+        all_w += (uint64_t)topo[l] * topo[l + 1];
+        all_b += topo[l + 1];
+        sane = topo[l] && topo[l + 1] && all_w < (uint64_t)1 << 40 && spg_array_bytes(all_w, prec) <= c.len;
+    }
+    if (sane && !spg_net_expect(spg_priv(net), all_w, all_b)) { spg_set_error(SPINGALETT_ERR_ALLOC, "load: network creation failed"); goto fail; }
     for (uint32_t l = 0; l < layers; l++) {
         layer_struct_arguments((LayerArgs){ .net = net, .neurons_amount = topo[l],
                                             .act_func = l ? (ActivationFunction)acts[l - 1] : ACT_SIGMOID,

@@ -233,7 +233,7 @@ void train_struct_arguments(TrainArgs a)
         p->time_step = 0;
         spg_log(LOG_INFO, "Optimizer state reset");
     }
-    if (spg_dev_ensure(n) != SPINGALETT_OK) return;          /* binds the device (and validates it exists) */
+    if (spg_dev_bind(n) != SPINGALETT_OK) return;            /* (the image for inference is not needed here, and stale after this) */
 
     /* STRATEGY_SAMPLE is a batch of one sample per update, in the caller's order (Training.c:894-897, :78-250) */
     const bool mini = a.training_strategy == STRATEGY_SMALL_BATCH, online = a.training_strategy == STRATEGY_SAMPLE;
@@ -292,10 +292,15 @@ void train_struct_arguments(TrainArgs a)
     /* the host arrays are the truth between calls (callers may edit them): upload them every time */
     DEV(spgk_memcpy_h2d(t->params, p->weights, tw * 4, st), "train: upload weights");
     DEV(spgk_memcpy_h2d(t->params + tw, p->biases, tb * 4, st), "train: upload biases");
-    DEV(spgk_memcpy_h2d(t->m, p->opt_m_weights, tw * 4, st), "train: upload m");
-    DEV(spgk_memcpy_h2d(t->m + tw, p->opt_m_biases, tb * 4, st), "train: upload m");
-    DEV(spgk_memcpy_h2d(t->v, p->opt_v_weights, tw * 4, st), "train: upload v");
-    DEV(spgk_memcpy_h2d(t->v + tw, p->opt_v_biases, tb * 4, st), "train: upload v");
+    if (a.reset_optimizer) {                                 /* cleared above: nothing to copy */
+        DEV(spgk_memset(t->m, 0, np * 4, st), "train: clear m");
+        DEV(spgk_memset(t->v, 0, np * 4, st), "train: clear v");
+    } else {
+        DEV(spgk_memcpy_h2d(t->m, p->opt_m_weights, tw * 4, st), "train: upload m");
+        DEV(spgk_memcpy_h2d(t->m + tw, p->opt_m_biases, tb * 4, st), "train: upload m");
+        DEV(spgk_memcpy_h2d(t->v, p->opt_v_weights, tw * 4, st), "train: upload v");
+        DEV(spgk_memcpy_h2d(t->v + tw, p->opt_v_biases, tb * 4, st), "train: upload v");
+    }
     DEV(spgk_memcpy_h2d(t->data_x, a.inputs, (size_t)a.sample_count * in0 * 4, st), "train: upload inputs");
     DEV(spgk_memcpy_h2d(t->data_t, a.targets, (size_t)a.sample_count * outw * 4, st), "train: upload targets");
     DEV(spgk_memset(t->grads, 0, np * 4, st), "train: clear gradients");
