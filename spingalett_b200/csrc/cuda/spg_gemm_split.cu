@@ -20,7 +20,8 @@
 // 777 -> 333 19.7 -> 10.2.  Whole nets: 784-512-1000-10 at 256 rows 49.8 -> 22.8; 301-777-333-129-37 at 3001 rows 64.7 -> 38.9; the
 // recomputation of some 950 of 65536 rows 46 -> 30.
 //
-// Every wait on an mbarrier is bounded as in spg_gemm_tc.cu; the cluster barriers are reached by every thread on every path.
+// Every wait on an mbarrier is bounded as in spg_gemm_tc.cu; the cluster barriers are reached by every thread on every path, by
+// whole warps (they are of the aligned kind).
 #include "spg_common.cuh"
 #include "spg_tc.cuh"
 #include "spg_gemm.cuh"
@@ -265,6 +266,7 @@ spg_gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
             // partial sums -> the CTA that owns the row: thread = one row, the two warps on a quadrant take 16 columns in turn
             const uint32_t q = warp & 3u, half = (warp - 2u) >> 2, row = q * 32u + lane, swz = (row & 3u) * 4;    // neighbouring rows on other banks
             mbar_wait(tfull, round & 1u, abort_flag, p.status, 53);
+            __syncwarp();                                      // each lane has waited in a loop of its own; what follows is for whole warps
             tc_fence_after();
             const uint32_t dst = mapa(base + recv_off + (rank * own + row % own) * p.BN * 4, row / own);
             for (uint32_t c = 16 * half; c < p.BN; c += 32) {
@@ -284,6 +286,7 @@ spg_gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
             else if (p.type16 == SPGK_T_F16) finish<__half>(p, mine);
             else finish<__nv_bfloat16>(p, mine);
         }
+        __syncwarp();                                          // lanes finish different numbers of rows; the barrier is for whole warps
         if (t + clusters < tiles) cluster_sync();              // read before the next tile's sums replace them (the same decision in every CTA of the cluster)
     }
     tc_fence_before();
