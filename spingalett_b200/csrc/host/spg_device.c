@@ -1115,7 +1115,7 @@ static float *forward_batch_on(spg_net *n, ForwardBatchArgs a)
                     /* the staging buffer of chunk c was last read by the copy of chunk c-2; a staged chunk goes out in two
                        pieces, so that the link has work while the second is staged */
                     if (staged && c >= 2 && spg_map_kernel_error(spgk_event_sync(n->copy_ev[c - 1]), "forward_batch: staging")) return NULL;
-                    const size_t piece = staged ? (rows / 2 + 7) & ~(size_t)7 : rows;      /* (8 rows: the copy's 32-byte boundaries) */
+                    const size_t piece = staged ? ((rows + 1) / 2 + 7) & ~(size_t)7 : rows;      /* (8 rows at least: the copy's 32-byte boundaries) */
                     int rc = SPINGALETT_OK;
                     for (size_t p0 = 0; p0 < rows && !rc; p0 += piece) {
                         const size_t pr = rows - p0 < piece ? rows - p0 : piece;

@@ -209,6 +209,23 @@ def test_pageable_host_batch_through_the_staged_pipeline(spg, oracle, monkeypatc
     net.free()
 
 
+@pytest.mark.parametrize("width", [20, 96])
+@pytest.mark.parametrize("tail", [1, 2, 7, 8, 9, 17])
+def test_staged_pipeline_with_a_short_last_chunk(spg, width, tail):
+    """Two chunks and a few rows: from pageable and from page-locked memory the same rows."""
+    import torch
+    net = spg.Network.build([width, 40, 5], [spg.abi.ACT_RELU, spg.abi.ACT_SIGMOID], spg.abi.WEIGHT_INITIALIZATION_NONE)
+    rng = np.random.default_rng(tail)
+    net.weights[:] = rng.standard_normal(net.weights.size).astype(np.float32) / 6
+    x = rng.random((2 * 16384 + tail, width), dtype=np.float32)
+    got = net.forward_batch(x)
+    assert np.array_equal(got, net.forward_batch(torch.from_numpy(x).pin_memory().numpy()))
+    w1, w2 = net.weights[:width * 40].reshape(40, width).astype(np.float64), net.weights[width * 40:].reshape(5, 40).astype(np.float64)
+    want = 1 / (1 + np.exp(-np.maximum(x @ w1.T, 0) @ w2.T))
+    assert np.abs(got - want).max() <= 1e-3
+    net.free()
+
+
 @pytest.mark.parametrize("which", ["chain", "one-launch"])
 def test_auto_margin_is_measured_again_every_1024_large_calls(spg, oracle, tmp_path_factory, which):
     """The AUTO margin is calibrated on the first large batch and measured again on every 1024th large call, where it can

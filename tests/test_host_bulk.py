@@ -1,7 +1,13 @@
 """Files whose arrays are long enough to be read and decoded by several threads (bulk.c): every precision, counts that are no
-multiple of anything, any number of threads, and files that end early."""
+multiple of anything, any number of threads, and files that end early; host batches that are staged in pieces."""
+import os
+import re
+import subprocess
+
 import numpy as np
 import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 TOPOLOGY = [1033, 1117, 3]
 COUNTS = [1033 * 1117, 1117 * 3]
@@ -67,3 +73,25 @@ def test_a_file_that_ends_early(spg, tmp_path, name):
     after = spg.Network(net)
     assert np.array_equal(after.weights[:COUNTS[0]], before.weights[:COUNTS[0]])
     assert not after.biases[-TOPOLOGY[2]:].any()
+
+
+def on_fake_kernels(tmp_path, program):
+    """The library's host sources and tests/c/<program>.c, with a stub for every kernel call that the program does not fake."""
+    host = os.path.join(ROOT, "spingalett_b200", "csrc", "host")
+    sources = [os.path.join(host, f) for f in sorted(os.listdir(host)) if f.endswith(".c")] + [os.path.join(ROOT, "tests", "c", program + ".c")]
+    objs = []
+    for src in sources:
+        objs.append(str(tmp_path / (os.path.basename(src) + ".o")))
+        subprocess.run(["gcc", "-std=c2x", "-O1", "-D_GNU_SOURCE", "-I", os.path.join(ROOT, "include"), "-I", host, "-c", src, "-o", objs[-1]], check=True)
+    names = subprocess.run(["nm"] + objs, capture_output=True, text=True, check=True).stdout
+    missing = set(re.findall(r" U (spgk?_\w+)", names)) - set(re.findall(r" [TtDBbCR] (spgk?_\w+)", names))
+    stubs = tmp_path / "stubs.c"
+    stubs.write_text("".join(f"long {name}(void) {{ return 0; }}\n" for name in sorted(missing)))
+    exe = str(tmp_path / program)
+    subprocess.run(["gcc", "-std=c2x", "-O1", *objs, str(stubs), "-o", exe, "-lpthread", "-ldl", "-lm"], check=True)
+    return exe
+
+
+def test_short_last_chunks_are_staged_whole(tmp_path):
+    r = subprocess.run([on_fake_kernels(tmp_path, "staged_pieces")], capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0 and r.stdout == "all staged\n", (r.returncode, r.stdout, r.stderr)
