@@ -84,6 +84,6 @@ static void copy_slice(void *ctx, size_t lo, size_t hi)
 void spg_stage_copy(void *dst, const void *src, size_t bytes)
 {
     copy_ctx c = { dst, src };
-    if (bytes < ((size_t)4 << 20)) memcpy(dst, src, bytes);
+    if (bytes < SPG_STAGE_THREADED) memcpy(dst, src, bytes);
     else spg_bulk(copy_slice, &c, bytes, 4096, (size_t)1 << 20);
 }

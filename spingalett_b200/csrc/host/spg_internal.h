@@ -113,6 +113,7 @@ SPG_HIDDEN void spg_shuffle(uint32_t *idx, uint32_t n);
 /* bulk.c */
 typedef void (*spg_slice_fn)(void *ctx, size_t lo, size_t hi);
 SPG_HIDDEN void spg_bulk(spg_slice_fn fn, void *ctx, size_t n, size_t grain, size_t least);
+#define SPG_STAGE_THREADED ((size_t)4 << 20)         /* bytes from which spg_stage_copy takes several threads */
 SPG_HIDDEN void spg_stage_copy(void *dst, const void *src, size_t bytes);
 /* codec.c */
 SPG_HIDDEN size_t spg_array_bytes(uint64_t count, PrecisionMode p);

@@ -1,4 +1,5 @@
-/* Staged host batches with short last chunks: every row arrives, in copies that get somewhere.  Host code of the library on fake
+/* Staged host batches with short last chunks: every row arrives, in copies that get somewhere, and a chunk is only cut where
+ * its pieces are long enough to be staged by several threads (4 MB).  Host code of the library on fake
  * kernels, as in unread_status.c; "device memory" is the heap, and the fake copy looks at what it is given. */
 #include <stdio.h>
 #include <stdlib.h>
@@ -29,6 +30,8 @@ int spgk_memcpy_h2d(void *d, const void *h, size_t bytes, void *s)
     if (g_in) {
         if (!bytes || ++g_copies > 64) fail("a copy of nothing");
         if (g_at + bytes > g_rows * g_row_bytes || memcmp(h, (const char *)g_in + g_at, bytes) != 0) fail("wrong rows staged");
+        const size_t chunk = g_at / g_row_bytes / CHUNK, rows = g_rows - chunk * CHUNK < CHUNK ? g_rows - chunk * CHUNK : CHUNK;
+        if (bytes != rows * g_row_bytes && bytes < (size_t)4 << 20) fail("a piece for one thread");
         g_at += bytes;
     }
     memcpy(d, h, bytes);
@@ -38,7 +41,7 @@ int spgk_memcpy_h2d(void *d, const void *h, size_t bytes, void *s)
 int main(void)
 {
     spingalett_set_verbose(false);
-    static const uint32_t tails[] = { 1, 2, 7, 8, 9, 15, 16, 17, 1234, 16383, 16384 }, widths[] = { 1, 20, 96, 300 };
+    static const uint32_t tails[] = { 1, 2, 7, 8, 9, 15, 16, 17, 1234, 16383, 16384 }, widths[] = { 1, 20, 96, 128, 300 };
     for (size_t w = 0; w < sizeof widths / sizeof *widths; w++) {
         NeuralNetwork *net = new_spingalett();
         layer(.net = net, .neurons_amount = widths[w], .act_func = ACT_SIGMOID);
