@@ -398,8 +398,10 @@ int spg_gemm_split_try(const SpgGemmArgs &a, const SpgDeviceProps &dp, int dev)
     AtOnce at;
     if ((rc = clusters_at_once(dev, at))) return rc;
     SplitPlan plan;
-    // (an unsplit tile is summed in the order of the persistent kernel: either may run)
-    if (!split_plan(at, rows, a.L->out, kblocks, (uint32_t)a.a_parts, (uint32_t)a.w_parts, a.softmax_fused != 0, only_S, only_S < 2,
+    // An unsplit tile is summed in the order of the persistent kernel, so either may run; but not where a softmax follows, whose own
+    // sum that kernel takes in another order: rows counted on the device always come here then, whatever the guess.
+    const bool one_wave = only_S == 0 || (only_S == 1 && !a.softmax_fused);
+    if (!split_plan(at, rows, a.L->out, kblocks, (uint32_t)a.a_parts, (uint32_t)a.w_parts, a.softmax_fused != 0, only_S, one_wave,
                     dp.smem_optin, plan)) return SPGK_E_UNSUPPORTED;
 
     SplitParams p{};

@@ -139,3 +139,24 @@ def test_rows_counted_on_the_device_do_not_hang_on_the_guess(spg, lib, N, K, row
     rest = np.ones(cap + 1, bool)
     rest[where[:rows]] = False
     assert np.all(results[0][rest] == -3.0)
+
+
+@pytest.mark.parametrize("N,K", [(10, 60), (37, 64), (128, 24), (10, 1000)])
+def test_a_softmax_of_counted_rows_does_not_hang_on_the_guess(spg, lib, N, K):
+    """Guesses on both sides of what the device holds at once, with K in one piece and in several: same bits."""
+    import torch
+    cap, rows = 24000, 21000
+    z, _, run = product(spg, lib, rows, N, K, 2, 1, 1, 5, softmax=1, cap=cap, seed=N)
+    n = torch.tensor([rows], dtype=torch.int32, device="cuda")
+    results = []
+    try:
+        for guess in (0, 100, 5000, 18000, 21000, cap):
+            lib.spgk_set_dynamic_rows(n.data_ptr(), guess)
+            results.append(run(0)[1])
+    finally:
+        lib.spgk_set_dynamic_rows(None, 0)
+    for r in results[1:]:
+        assert np.array_equal(results[0], r)
+    e = np.exp(z - z.max(1, keepdims=True))
+    assert np.abs(results[0][:rows] - (e / e.sum(1, keepdims=True))[:rows]).max() <= 1e-4
+    assert np.all(results[0][rows:] == -3.0)
