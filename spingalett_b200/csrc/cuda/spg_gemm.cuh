@@ -19,5 +19,6 @@ struct SpgGemmArgs {
 int spg_gemm_map(CUtensorMap *map, const void *base, int type16, uint32_t K, uint32_t rows, uint32_t ld, uint64_t plane, int parts,
                  uint32_t box_rows, uint32_t box_planes);
 
-// Launches the few-tiles kernel if it has an arrangement for this product, else SPGK_E_UNSUPPORTED (nothing launched).
-int spg_gemm_split_try(const SpgGemmArgs &a, const SpgDeviceProps &dp, int dev);
+// Launches the few-tiles kernel if it has an arrangement for this product.  SPGK_E_UNSUPPORTED: the persistent kernel is needed, for
+// row counts above `served` (0: for all, nothing was launched).
+int spg_gemm_split_try(const SpgGemmArgs &a, const SpgDeviceProps &dp, int dev, uint32_t &served);

@@ -8,6 +8,9 @@
 // sums of every row to the CTA that owns the row (distributed shared memory, 128 / S rows each), and each CTA finishes its
 // own rows: sum in CTA order, scale, bias, activation or softmax, store.  The result does not depend on timing.
 //
+// Where only the device knows the row count, it also decides there whether K is cut: beyond a number of rows that hangs on the
+// layer alone the clusters would have to take tile after tile, and every CTA walks the whole of K for tiles of its own instead.
+//
 // A k-block brings all planes of both operands at once (hi and lo of the activations, of the weights where they have two)
 // and every pass multiplies what is there, so a two-term product moves three tiles where the pass-by-pass walk moves four.
 //
@@ -47,6 +50,8 @@ struct SplitParams {
     float *out32; uint32_t ldo32; const uint32_t *out_rows;
     float margin_theta; uint32_t *margin_idx, *margin_count;
     const uint32_t *m_limit;
+    uint32_t above, upto;         // other row counts than above < rows <= upto are left to another launch
+    uint32_t cut_rows;            // rows up to which a cluster shares a tile; with more, each of its CTAs takes tiles of its own
     int32_t *status;
 };
 
@@ -86,11 +91,11 @@ __device__ __forceinline__ float4 sum_parts(const float *at, uint32_t step, uint
 
 // What a thread finishes of a tile: four neighbouring columns (col..) of every lanes_y-th of the rows that its CTA owns.
 // recv: their sums, [part][own row][BN], columns of neighbouring rows in another order (swz).
-struct Mine { const float *recv; uint32_t own, row0, rows, col, cx, cy, lanes_y; float4 bias; };
+struct Mine { const float *recv; uint32_t S, own, row0, rows, col, cx, cy, lanes_y; float4 bias; };
 
 __device__ __forceinline__ float4 logits4(const SplitParams &p, const Mine &m, uint32_t rl)
 {
-    const float4 s = sum_parts(m.recv + rl * p.BN + (m.cx ^ ((rl & 3u) * 4)), m.own * p.BN, p.S);
+    const float4 s = sum_parts(m.recv + rl * p.BN + (m.cx ^ ((rl & 3u) * 4)), m.own * p.BN, m.S);
     return make_float4(fmaf(s.x, p.scale, m.bias.x), fmaf(s.y, p.scale, m.bias.y), fmaf(s.z, p.scale, m.bias.z), fmaf(s.w, p.scale, m.bias.w));
 }
 __device__ __forceinline__ void write4(const SplitParams &p, uint32_t row, uint32_t col, float4 v)
@@ -210,18 +215,22 @@ spg_gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
     cluster_sync();                                            // the other CTAs of the cluster are there: their shared memory may be written
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
+    // a tile shared by the cluster (divisions ahead of the wait, where nobody waits for them)
+    const uint32_t me = cluster_rank(), passes = 1 + (p.a_parts > 1) + (p.w_parts > 1);
+    uint32_t S = p.S, rank = me, kb0 = me * p.kblocks / S, kb1 = (me + 1) * p.kblocks / S;
+    uint32_t own = TM / S, first = blockIdx.x / S, step = gridDim.x / S;      // own: rows of a tile that this CTA finishes
+    const uint32_t w_off = p.a_parts * A_BYTES, w_plane = p.BN * TK * 2;
+    const uint32_t groups = p.BN >> 2, lanes_y = THREADS / groups, cx = threadIdx.x % groups * 4, cy = threadIdx.x / groups;
     spg_grid_trigger();
     spg_grid_wait();
 
     const uint32_t rows = spg_limit_rows(p.M, p.m_limit);
-    const uint32_t tiles = (rows + TM - 1) / TM * p.n_tiles, rank = cluster_rank(), clusters = gridDim.x / p.S;
-    const uint32_t kb0 = rank * p.kblocks / p.S, kb1 = (rank + 1) * p.kblocks / p.S;
-    const uint32_t own = TM / p.S;                             // rows of a tile that this CTA finishes
-    const uint32_t passes = 1 + (p.a_parts > 1) + (p.w_parts > 1);
-    const uint32_t w_off = p.a_parts * A_BYTES, w_plane = p.BN * TK * 2;
-    const uint32_t groups = p.BN >> 2, lanes_y = THREADS / groups, cx = threadIdx.x % groups * 4, cy = threadIdx.x / groups;
+    const uint32_t tiles = rows > p.above && rows <= p.upto ? (rows + TM - 1) / TM * p.n_tiles : 0;
+    const bool cut = rows <= p.cut_rows;                       // (the same in every CTA)
+    if (!cut) { S = 1; rank = 0; kb0 = 0; kb1 = p.kblocks; own = TM; first = blockIdx.x; step = gridDim.x; }
+    const auto together = [cut] { if (cut) cluster_sync(); else __syncthreads(); };      // all that work on a tile
     uint32_t it = 0, round = 0;                                // k-blocks and tiles so far
-    for (uint32_t t = blockIdx.x / p.S; t < tiles; t += clusters, round++) {
+    for (uint32_t t = first; t < tiles; t += step, round++) {
         // neighbouring clusters take the column tiles of the same rows
         const uint32_t mt = t / p.n_tiles, nt = t % p.n_tiles;
         const uint32_t col = nt * p.BN + cx;                   // this thread's columns when the tile is finished; their biases are under way from here
@@ -268,7 +277,7 @@ spg_gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
             mbar_wait(tfull, round & 1u, abort_flag, p.status, 53);
             __syncwarp();                                      // each lane has waited in a loop of its own; what follows is for whole warps
             tc_fence_after();
-            const uint32_t dst = mapa(base + recv_off + (rank * own + row % own) * p.BN * 4, row / own);
+            const uint32_t dst = mapa(base + recv_off + (rank * own + row % own) * p.BN * 4, cut ? row / own : me);
             for (uint32_t c = 16 * half; c < p.BN; c += 32) {
                 uint32_t r[16];
                 tmem_ld16(tmem + c + ((q * 32u) << 16), r);
@@ -278,16 +287,16 @@ spg_gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
             }
             tc_fence_before();
         }
-        cluster_sync();                                        // every partial sum of this cluster's tile is in place
+        together();                                            // every partial sum of the tile is in place
         tc_fence_after();
-        const Mine mine = { reinterpret_cast<const float *>(smem + recv_off), own, mt * TM + rank * own, rows, col, cx, cy, lanes_y, bias };
+        const Mine mine = { reinterpret_cast<const float *>(smem + recv_off), S, own, mt * TM + rank * own, rows, col, cx, cy, lanes_y, bias };
         if (cy < lanes_y) {                                    // (a power of two of groups leaves no thread out)
             if (p.softmax) finish_softmax(p, mine);
             else if (p.type16 == SPGK_T_F16) finish<__half>(p, mine);
             else finish<__nv_bfloat16>(p, mine);
         }
         __syncwarp();                                          // lanes finish different numbers of rows; the barrier is for whole warps
-        if (t + clusters < tiles) cluster_sync();              // read before the next tile's sums replace them (the same decision in every CTA of the cluster)
+        if (t + step < tiles) together();                      // read before the next tile's sums replace them (the same decision in all that share it)
     }
     tc_fence_before();
     __syncthreads();
@@ -325,9 +334,31 @@ int clusters_at_once(int dev, AtOnce &out)
     return rc;
 }
 
+// Cycles of a tile (measured, 128 CTAs at work): 7000 for set-up, the first operands and the way from tile to tile; operands at 47
+// bytes a cycle; partial sums into their owner's shared memory at 55 (the own one), 24, 21 and 13, and out of it at 60; a cluster
+// barrier.  (The first number only matters where tiles come in waves: what each further wave took beyond the rest.)
+uint64_t tile_cycles(uint32_t BN, uint32_t i, uint32_t kblocks, uint32_t stage)
+{
+    static const uint32_t push[4] = { 55, 24, 21, 13 };
+    const uint32_t S = 1u << i, kb = (kblocks + S - 1) / S;
+    return 7000 + (uint64_t)kb * stage / 47 + TM * BN * 4 / push[i] + TM * BN * 4 / 60 + (S > 1 ? 1200 : 0);
+}
+
+uint32_t stage_size(uint32_t BN, uint32_t a_parts, uint32_t w_parts) { return a_parts * A_BYTES + w_parts * BN * TK * 2; }
+
+// The tile widths that a layer may have, in steps of 16
+struct Widths { uint32_t lo, hi; };
+Widths widths(uint32_t N, bool softmax)
+{
+    if (!softmax) return { 16, N < MAX_BN ? (N + 15u) & ~15u : MAX_BN };
+    uint32_t bn = 16;                                           // a row in one tile, on a power of two of lanes
+    while (bn < N) bn <<= 1;
+    return { bn, bn };
+}
+
 // The split of a product whose row count only the device knows.  The caller's guess of the count changes from call to call
-// and must not change the order of the sums, so the split depends on the layer alone: as many CTAs a tile as 1024 rows
-// leave SMs for.
+// and must not change the order of the sums, so what decides it is the layer, and the count itself: as many CTAs a tile as 1024
+// rows leave SMs for, up to a count that hangs on the layer alone (cut_rows).
 uint32_t fixed_split(uint32_t N, uint32_t kblocks, uint32_t sm_count)
 {
     const uint32_t tiles = 8 * ((N + 63) / 64);
@@ -336,35 +367,39 @@ uint32_t fixed_split(uint32_t N, uint32_t kblocks, uint32_t sm_count)
     return S;
 }
 
+// Rows up to which the device cuts K, tiles at their widest: as many waves of cut tiles as take about as long as one tile uncut.
+// Measured on either side of it (us): 1000 -> 10 at 3500 rows 10.9 cut and 14.7 not, at 4600 15.3 and 14.7, at 8000 24.4 and 18;
+// 4096 -> 128 at 4600 38.6 and 53, at 8000 67.5 and 53; 784 -> 512 at 2300 12.9 and 22, at 8000 34.9 and 25.
+uint32_t cut_rows(const AtOnce &at, uint32_t i, uint32_t N, uint32_t kblocks, uint32_t a_parts, uint32_t w_parts, bool softmax)
+{
+    const uint32_t BN = widths(N, softmax).hi, stage = stage_size(BN, a_parts, w_parts);
+    const uint64_t cut = tile_cycles(BN, i, kblocks, stage), uncut = tile_cycles(BN, 0, kblocks, stage);
+    const uint32_t waves = (uint32_t)((uncut + cut / 2) / cut);
+    return (waves ? waves : 1) * at.n[i] / ((N + BN - 1) / BN) * TM;
+}
+
 // Which products come here, and how they are cut: those for which some tile width and split fit on the device in one wave
 // (one CTA an SM), at the width and split that the estimate below makes cheapest.  Measured for 24 products (32 to 3000 rows,
 // 10 to 2048 columns, 301 to 2048 inputs) over every width and split: the estimate picked the fastest or one within 8 % of it,
 // and none was slower than the persistent kernel, which overlaps epilogues with the next tile's products and is the better one
 // as soon as tiles come in waves.
 //
-// Tile width and split of the cheapest arrangement; only_S: that split and no other, if not zero.  one_wave: only what the
+// Tile width and split of the cheapest arrangement; only_i: that split and no other, if not negative.  one_wave: only what the
 // device holds at once (false if nothing fits).
-bool split_plan(const AtOnce &at, uint32_t rows, uint32_t N, uint32_t kblocks, uint32_t a_parts, uint32_t w_parts, bool softmax, uint32_t only_S, bool one_wave,
+bool split_plan(const AtOnce &at, uint32_t rows, uint32_t N, uint32_t kblocks, uint32_t a_parts, uint32_t w_parts, bool softmax, int only_i, bool one_wave,
                 size_t smem_max, SplitPlan &best)
 {
     const uint32_t mt = (rows + TM - 1) / TM;
-    uint32_t lo = 16, hi = N < MAX_BN ? (N + 15u) & ~15u : MAX_BN;
-    if (softmax) {                                              // a row in one tile, on a power of two of lanes
-        while (lo < N) lo <<= 1;
-        if (lo > 128) return false;
-        hi = lo;
-    }
+    const Widths w = widths(N, softmax);
+    if (softmax && w.hi > 128) return false;
     uint64_t best_cost = ~0ull;
-    for (uint32_t BN = lo; BN <= hi; BN += 16) {
-        const uint32_t nt = (N + BN - 1) / BN, stage = a_parts * A_BYTES + w_parts * BN * TK * 2;
+    for (uint32_t BN = w.lo; BN <= w.hi; BN += 16) {
+        const uint32_t nt = (N + BN - 1) / BN, stage = stage_size(BN, a_parts, w_parts);
         const uint64_t tiles = (uint64_t)mt * nt;
         for (uint32_t i = 0, S = 1; S <= MAX_SPLIT && S <= kblocks; i++, S <<= 1) {
-            if ((only_S && S != only_S) || !at.n[i] || (one_wave && tiles > at.n[i])) continue;
+            if ((only_i >= 0 && i != (uint32_t)only_i) || !at.n[i] || (one_wave && tiles > at.n[i])) continue;
             const uint32_t kb = (kblocks + S - 1) / S;
-            // cycles of a tile (measured, 128 CTAs at work): operands at 47 bytes a cycle; partial sums into their owner's shared
-            // memory at 55 (the own one), 24, 21 and 13, and out of it at 60; a cluster barrier
-            static const uint32_t push[4] = { 55, 24, 21, 13 };
-            const uint64_t cost = (1500 + (uint64_t)kb * stage / 47 + TM * BN * 4 / push[i] + TM * BN * 4 / 60 + (S > 1 ? 1200 : 0)) * ((tiles + at.n[i] - 1) / at.n[i]);
+            const uint64_t cost = tile_cycles(BN, i, kblocks, stage) * ((tiles + at.n[i] - 1) / at.n[i]);
             if (cost >= best_cost) continue;
             uint32_t stages = !one_wave || kb > MAX_STAGES ? MAX_STAGES : kb;
             while (stages > 1 && split_smem(BN, stages, stage) > smem_max) stages--;
@@ -376,38 +411,15 @@ bool split_plan(const AtOnce &at, uint32_t rows, uint32_t N, uint32_t kblocks, u
     return best_cost != ~0ull;
 }
 
-}  // namespace
+// which row counts a launch serves, and up to which K is cut
+struct Counts { uint32_t above, upto, cut; };
 
-int spg_gemm_split_try(const SpgGemmArgs &a, const SpgDeviceProps &dp, int dev)
+int split_launch(const SpgGemmArgs &a, const AtOnce &at, const SplitPlan &plan, const Counts &counts)
 {
-    if (a.w_type16 != a.type16) return SPGK_E_UNSUPPORTED;
-    const uint32_t kblocks = (a.L->in + TK - 1) / TK;
-    static SpgOncePerDevice once;
-    int rc = once.run(dev, [&]() -> int {
-        SPGK_CUDA(cudaFuncSetAttribute(spg_gemm_split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dp.smem_optin));
-        return SPGK_OK;
-    });
-    if (rc) return rc;
-    // the rows to arrange for: where only the device knows, those of the call before and what a selection by chance varies
-    uint32_t rows = a.N, only_S = 0;
-    if (spg_tls_rows_limit) {
-        rows = spg_tls_rows_expected ? spg_tls_rows_expected + 4u * (uint32_t)sqrtf((float)spg_tls_rows_expected) : 1024;
-        if (rows > a.N) rows = a.N;
-        only_S = fixed_split(a.L->out, kblocks, (uint32_t)dp.sm_count);
-    }
-    AtOnce at;
-    if ((rc = clusters_at_once(dev, at))) return rc;
-    SplitPlan plan;
-    // An unsplit tile is summed in the order of the persistent kernel, so either may run; but not where a softmax follows, whose own
-    // sum that kernel takes in another order: rows counted on the device always come here then, whatever the guess.
-    const bool one_wave = only_S == 0 || (only_S == 1 && !a.softmax_fused);
-    if (!split_plan(at, rows, a.L->out, kblocks, (uint32_t)a.a_parts, (uint32_t)a.w_parts, a.softmax_fused != 0, only_S, one_wave,
-                    dp.smem_optin, plan)) return SPGK_E_UNSUPPORTED;
-
     SplitParams p{};
-    p.M = a.N; p.N = a.L->out; p.kblocks = kblocks; p.BN = plan.BN; p.S = plan.S; p.stages = plan.stages;
+    p.M = a.N; p.N = a.L->out; p.kblocks = (a.L->in + TK - 1) / TK; p.BN = plan.BN; p.S = plan.S; p.stages = plan.stages;
     p.n_tiles = (a.L->out + p.BN - 1) / p.BN; p.m_tiles = (a.N + TM - 1) / TM;
-    p.a_parts = (uint32_t)a.a_parts; p.w_parts = (uint32_t)a.w_parts; p.stage_bytes = p.a_parts * A_BYTES + p.w_parts * p.BN * TK * 2;
+    p.a_parts = (uint32_t)a.a_parts; p.w_parts = (uint32_t)a.w_parts; p.stage_bytes = stage_size(p.BN, p.a_parts, p.w_parts);
     p.idesc = idesc_f16((uint32_t)a.type16, (uint32_t)a.w_type16, p.BN);
     p.scale = a.L->w_scale; p.bias = a.L->bias;
     p.act = a.L->act == SPG_ACT_SOFTMAX ? SPG_ACT_NONE : a.L->act;
@@ -416,8 +428,10 @@ int spg_gemm_split_try(const SpgGemmArgs &a, const SpgDeviceProps &dp, int dev)
     p.out32 = a.out32; p.ldo32 = a.ldo32; p.out_rows = spg_tls_out_rows;
     if (p.softmax && spg_tls_margin_idx) { p.margin_theta = spg_tls_margin_theta; p.margin_idx = spg_tls_margin_idx; p.margin_count = spg_tls_margin_count; }
     p.m_limit = spg_tls_rows_limit;
+    p.above = counts.above; p.upto = counts.upto; p.cut_rows = counts.cut;
     p.status = a.status;
     CUtensorMap map_a, map_w;
+    int rc;
     if ((rc = spg_gemm_map(&map_a, a.a16, a.type16, a.L->in, a.N, a.lda, a.a_plane, a.a_parts, TM, p.a_parts))) return rc;
     if ((rc = spg_gemm_map(&map_w, a.w16, a.w_type16, a.L->in, a.L->out, a.ldw, a.w_plane, a.w_parts, p.BN, p.w_parts))) return rc;
 
@@ -434,4 +448,52 @@ int spg_gemm_split_try(const SpgGemmArgs &a, const SpgDeviceProps &dp, int dev)
     cfg.attrs = attr; cfg.numAttrs = 2;
     SPGK_CUDA(cudaLaunchKernelEx(&cfg, spg_gemm_split_kernel, map_a, map_w, p));
     return spgk_check_launch("spg_gemm_split_kernel");
+}
+
+}  // namespace
+
+int spg_gemm_split_try(const SpgGemmArgs &a, const SpgDeviceProps &dp, int dev, uint32_t &served)
+{
+    served = 0;
+    if (a.w_type16 != a.type16) return SPGK_E_UNSUPPORTED;
+    static SpgOncePerDevice once;
+    int rc = once.run(dev, [&]() -> int {
+        SPGK_CUDA(cudaFuncSetAttribute(spg_gemm_split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dp.smem_optin));
+        return SPGK_OK;
+    });
+    if (rc) return rc;
+    AtOnce at;
+    if ((rc = clusters_at_once(dev, at))) return rc;
+    const uint32_t N = a.L->out, kblocks = (a.L->in + TK - 1) / TK, a_parts = (uint32_t)a.a_parts, w_parts = (uint32_t)a.w_parts;
+    const bool softmax = a.softmax_fused != 0;
+    SplitPlan plan;
+    if (!spg_tls_rows_limit) {
+        if (!split_plan(at, a.N, N, kblocks, a_parts, w_parts, softmax, -1, true, dp.smem_optin, plan)) return SPGK_E_UNSUPPORTED;
+        return split_launch(a, at, plan, { 0, ~0u, ~0u });
+    }
+
+    // Rows counted on the device: arranged for those of the call before and what a selection by chance varies.  The guess steers
+    // the tile width, and which launch serves counts at which K is not cut; the sums are the same for any guess.
+    uint32_t seen = spg_tls_rows_expected ? spg_tls_rows_expected : 1024;
+    if (seen > a.N) seen = a.N;
+    uint32_t rows = seen + 4u * (uint32_t)sqrtf((float)seen);
+    if (rows > a.N) rows = a.N;
+    int i = 0;
+    for (uint32_t S = fixed_split(N, kblocks, (uint32_t)dp.sm_count); S > 1; S >>= 1) i++;
+    if (i == 0) {
+        // An unsplit tile is summed in the order of the persistent kernel, so either may run; but not where a softmax follows, whose
+        // own sum that kernel takes in another order: rows counted on the device always come here then.
+        if (!split_plan(at, rows, N, kblocks, a_parts, w_parts, softmax, 0, !softmax, dp.smem_optin, plan)) return SPGK_E_UNSUPPORTED;
+        return split_launch(a, at, plan, { 0, ~0u, ~0u });
+    }
+    const uint32_t limit = cut_rows(at, (uint32_t)i, N, kblocks, a_parts, w_parts, softmax);
+    if (!split_plan(at, rows < limit ? rows : limit, N, kblocks, a_parts, w_parts, softmax, i, false, dp.smem_optin, plan)) return SPGK_E_UNSUPPORTED;
+    if (seen <= limit) return split_launch(a, at, plan, { 0, ~0u, limit });
+    // Many rows: K whole and tile after tile, by a launch made for that.  It follows this one, and either finds that the count is
+    // not its own: 2 us, against 784 -> 512 at 65536 rows in 252 us here and 116 there.  Again, a softmax has its own order of sums.
+    if ((rc = split_launch(a, at, plan, { 0, limit, limit }))) return rc;
+    served = limit;
+    if (!softmax) return SPGK_E_UNSUPPORTED;
+    if (!split_plan(at, rows, N, kblocks, a_parts, w_parts, true, 0, false, dp.smem_optin, plan)) return SPGK_E_UNSUPPORTED;
+    return split_launch(a, at, plan, { limit, ~0u, ~0u });
 }

@@ -65,7 +65,8 @@ struct GemmParams {
     float margin_theta; uint32_t *margin_idx, *margin_count;
     const uint32_t *out_rows;     // optional scatter of the fp32 output rows   // fused-softmax rows with top-two logit gap < theta are appended here (optional)
     int tma_store;                // 16-bit output leaves through TMA stores (one plane, tiles at least 128 wide)
-    const uint32_t *m_limit;      // optional device-resident row count: the kernel works on min(M, *m_limit) rows
+    const uint32_t *m_limit;      // optional device-resident row count: the kernel works on min(M, *m_limit) rows ...
+    uint32_t m_above;             // ... or on none, if they are no more than this (spg_gemm_split_kernel has them)
 };
 
 struct RowLimit { uint32_t m_tiles, group_m; };   // tile counts for the rows actually present (<= the launch's capacity)
@@ -568,6 +569,7 @@ spg_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
     if (p.m_limit) {
         const uint32_t m = *reinterpret_cast<const volatile uint32_t *>(p.m_limit);
         rows = m < rows ? m : rows;
+        if (rows <= p.m_above) rows = 0;
     }
     RowLimit rl;
     rl.m_tiles = (rows + BM - 1) / BM;
@@ -846,6 +848,7 @@ static int gemm_launch(const spgk_layer *L,
     }
     if (N == 0) return SPGK_OK;
     SpgDeviceProps dp;
+    uint32_t served = 0;
     {
         const int prc = spg_device_props(&dp);
         if (prc) return prc;
@@ -854,7 +857,7 @@ static int gemm_launch(const spgk_layer *L,
         if (!head) {
             const SpgGemmArgs args = { L, w16, ldw, w_plane, w_parts, w_type16, a16, lda, a_plane, a_parts, type16, out16, ldo16, o_plane,
                                        out_parts, out32, ldo32, N, softmax_fused, status, stream };
-            const int rc = spg_gemm_split_try(args, dp, dev);
+            const int rc = spg_gemm_split_try(args, dp, dev, served);
             if (rc != SPGK_E_UNSUPPORTED) return rc;
         }
         // the opt-in for large dynamic shared memory is a per-device function attribute
@@ -908,7 +911,7 @@ static int gemm_launch(const spgk_layer *L,
     p.out16 = out16; p.ldo16 = ldo16; p.o_plane = o_plane; p.out_parts = out_parts; p.type16 = type16;
     p.out32 = out32; p.ldo32 = ldo32;
     p.status = status;
-    p.m_limit = spg_tls_rows_limit;
+    p.m_limit = spg_tls_rows_limit; p.m_above = served;
     if ((softmax_fused || (head && head->act == SPG_ACT_SOFTMAX)) && spg_tls_margin_idx) { p.margin_theta = spg_tls_margin_theta; p.margin_idx = spg_tls_margin_idx; p.margin_count = spg_tls_margin_count; }
     p.out_rows = spg_tls_out_rows;
 

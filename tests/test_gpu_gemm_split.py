@@ -160,3 +160,27 @@ def test_a_softmax_of_counted_rows_does_not_hang_on_the_guess(spg, lib, N, K):
     e = np.exp(z - z.max(1, keepdims=True))
     assert np.abs(results[0][:rows] - (e / e.sum(1, keepdims=True))[:rows]).max() <= 1e-4
     assert np.all(results[0][rows:] == -3.0)
+
+
+@pytest.mark.parametrize("N,K,rows", [(512, 784, (1500, 3072, 3073, 20000)), (256, 2048, (1500, 4096, 4700, 24000)), (128, 130, (2100, 24000)),
+                                      (100, 1000, (1900, 2100, 4300)), (777, 301, (4800, 9000))])
+def test_counts_beyond_what_the_device_holds_at_once(spg, lib, N, K, rows):
+    """K is cut up to a count that hangs on the layer alone: same bits for any guess on either side of it, in all outputs."""
+    import torch
+    cap = 24000
+    z, size, run = product(spg, lib, cap, N, K, 2, 1, 1, 1, seed=N)
+    want = np.maximum(z, 0)
+    try:
+        for count in rows:
+            n = torch.tensor([count], dtype=torch.int32, device="cuda")
+            results = []
+            for guess in (0, 100, count, cap):
+                lib.spgk_set_dynamic_rows(n.data_ptr(), guess)
+                results.append(run(2))
+            for o16, o32 in results[1:]:
+                assert np.array_equal(results[0][0], o16) and np.array_equal(results[0][1], o32), count
+            o16, o32 = results[0]
+            assert np.all(np.abs(o32[:count] - want[:count]) <= bound(K) * size[:count] + 1e-6 * np.maximum(1, want[:count]))
+            assert np.all(o32[count:] == -3.0) and np.all(o16[:, count:] == 7.0)
+    finally:
+        lib.spgk_set_dynamic_rows(None, 0)
