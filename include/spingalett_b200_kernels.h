@@ -470,6 +470,8 @@ SPGK_API int spgk_nccl_abort(void *comm);
  * spgk_selftest_bounded_wait: launches one small kernel that waits on a barrier nobody arrives on with the kernels' own
  *   bounded waits and `limit` attempts (<= 4096; each attempt may suspend the warp for 20 us); the kernel returns by itself,
  *   status3[0] holds the wait's code, and the call returns SPGK_E_TIMEOUT exactly as a GEMM whose wait gave up does.
+ * spgk_selftest_impatient: the calling thread's products of few tiles (spg_gemm_split.cu) take the wait for a finished tile as given
+ *   up as soon as they come to it, with copies and products under way: outputs stay as they were and the status word says so.
  * spgk_selftest_timed_call: host only: a call that answers after answer_ms under the rendezvous timeout wrapper with a
  *   limit of timeout_ms: 0 or SPGK_E_TIMEOUT.
  * spgk_selftest_once_per_device: host only: the once-per-device bookkeeping of the launchers over `devices` fake indices and
@@ -477,6 +479,7 @@ SPGK_API int spgk_nccl_abort(void *comm);
 SPGK_API void spgk_fail_malloc_after(int k);
 SPGK_API int spgk_mem_info(size_t *free_bytes, size_t *total_bytes);
 SPGK_API int spgk_selftest_bounded_wait(int32_t *status3, uint32_t limit, void *stream);
+SPGK_API void spgk_selftest_impatient(int on);
 SPGK_API int spgk_selftest_timed_call(int answer_ms, int timeout_ms);
 SPGK_API int spgk_selftest_once_per_device(int devices, int calls, int fail_first);
 

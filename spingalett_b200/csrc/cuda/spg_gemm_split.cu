@@ -24,11 +24,15 @@
 // recomputation of some 950 of 65536 rows 46 -> 30.
 //
 // Every wait on an mbarrier is bounded as in spg_gemm_tc.cu; the cluster barriers are reached by every thread on every path, by
-// whole warps (they are of the aligned kind).
+// whole warps (they are of the aligned kind).  A wait that gave up in one CTA is known to its whole cluster before anybody finishes
+// a row: that tile's outputs are left as they were, copies and products under way are awaited (again with a bound), and the
+// cluster returns.
 #include "spg_common.cuh"
 #include "spg_tc.cuh"
 #include "spg_gemm.cuh"
 #include <cmath>
+
+static thread_local bool spg_tls_impatient = false;            // spgk_selftest_impatient
 
 namespace {
 
@@ -50,6 +54,7 @@ struct SplitParams {
     float *out32; uint32_t ldo32; const uint32_t *out_rows;
     float margin_theta; uint32_t *margin_idx, *margin_count;
     const uint32_t *m_limit;
+    int impatient;                // (the check of the failure path) a finished tile is given up before it is waited for
     uint32_t above, upto;         // other row counts than above < rows <= upto are left to another launch
     uint32_t cut_rows;            // rows up to which a cluster shares a tile; with more, each of its CTAs takes tiles of its own
     int32_t *status;
@@ -64,6 +69,10 @@ __device__ __forceinline__ void load_planes(uint32_t dst, const CUtensorMap *map
 __device__ __forceinline__ void store_remote4(uint32_t addr, const uint32_t *r)
 {
     asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]) : "memory");
+}
+__device__ __forceinline__ void store_remote(uint32_t addr, uint32_t v)
+{
+    asm volatile("st.shared::cluster.b32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
 }
 
 // a load that stays where it is written, ahead of the waits
@@ -197,14 +206,14 @@ spg_gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
     const uint32_t full0 = base + bar_off, empty0 = full0 + 8 * MAX_STAGES, tfull = empty0 + 8 * MAX_STAGES;
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem + bar_off + 16 * MAX_STAGES + 8);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
-    const uint32_t abort_addr = smem_u32(const_cast<int *>(abort_flag));
+    const uint32_t abort_addr = smem_u32(const_cast<int *>(abort_flag)), drain_addr = abort_addr + 4;      // (drain: the flag of the last waits)
     const uint32_t warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31u;
     const uint32_t tmem_cols = p.BN <= 32 ? 32 : p.BN <= 64 ? 64 : p.BN <= 128 ? 128 : 256;       // a power of two
 
     if (threadIdx.x == 0) {
         for (uint32_t s = 0; s < p.stages; s++) { mbar_init(full0 + 8 * s, 1); mbar_init(empty0 + 8 * s, 1); }
         mbar_init(tfull, 1);
-        *abort_flag = 0;
+        abort_flag[0] = abort_flag[1] = 0;
         mbar_fence_init();
         prefetch_map(&map_a);
         prefetch_map(&map_w);
@@ -229,7 +238,7 @@ spg_gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
     const bool cut = rows <= p.cut_rows;                       // (the same in every CTA)
     if (!cut) { S = 1; rank = 0; kb0 = 0; kb1 = p.kblocks; own = TM; first = blockIdx.x; step = gridDim.x; }
     const auto together = [cut] { if (cut) cluster_sync(); else __syncthreads(); };      // all that work on a tile
-    uint32_t it = 0, round = 0;                                // k-blocks and tiles so far
+    uint32_t it = 0, round = 0, sent = 0;                      // k-blocks and tiles so far; k-blocks that the electing lane has sent for
     for (uint32_t t = first; t < tiles; t += step, round++) {
         // neighbouring clusters take the column tiles of the same rows
         const uint32_t mt = t / p.n_tiles, nt = t % p.n_tiles;
@@ -243,7 +252,8 @@ spg_gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
             for (uint32_t kb = kb0; kb < kb1; kb++, it++) {
                 const uint32_t s = it % p.stages, ph = (it / p.stages) & 1u, st = base + s * p.stage_bytes;
                 mbar_wait_uniform(empty0 + 8 * s, ph ^ 1u, abort_addr, p.status, 51);
-                if (elect_one()) {
+                if (elect_one() && !*abort_flag) {
+                    sent = it + 1;
                     mbar_expect_tx(full0 + 8 * s, p.stage_bytes);
                     load_planes(st, &map_a, full0 + 8 * s, (int)(kb * TK), (int)(mt * TM));
                     load_planes(st + w_off, &map_w, full0 + 8 * s, (int)(kb * TK), (int)(nt * p.BN));
@@ -274,20 +284,26 @@ spg_gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
         } else {
             // partial sums -> the CTA that owns the row: thread = one row, the two warps on a quadrant take 16 columns in turn
             const uint32_t q = warp & 3u, half = (warp - 2u) >> 2, row = q * 32u + lane, swz = (row & 3u) * 4;    // neighbouring rows on other banks
-            mbar_wait(tfull, round & 1u, abort_flag, p.status, 53);
+            const bool ok = !p.impatient && mbar_wait(tfull, round & 1u, abort_flag, p.status, 53);
+            if (p.impatient) { *abort_flag = 1; atomicCAS(p.status, 0, 53); }
             __syncwarp();                                      // each lane has waited in a loop of its own; what follows is for whole warps
             tc_fence_after();
             const uint32_t dst = mapa(base + recv_off + (rank * own + row % own) * p.BN * 4, cut ? row / own : me);
-            for (uint32_t c = 16 * half; c < p.BN; c += 32) {
-                uint32_t r[16];
-                tmem_ld16(tmem + c + ((q * 32u) << 16), r);
-                tmem_ld_wait();
+            if (__all_sync(0xffffffffu, ok)) {
+                for (uint32_t c = 16 * half; c < p.BN; c += 32) {
+                    uint32_t r[16];
+                    tmem_ld16(tmem + c + ((q * 32u) << 16), r);
+                    tmem_ld_wait();
 #pragma unroll
-                for (int i = 0; i < 16; i += 4) store_remote4(dst + ((c + i) ^ swz) * 4, r + i);
+                    for (int i = 0; i < 16; i += 4) store_remote4(dst + ((c + i) ^ swz) * 4, r + i);
+                }
             }
             tc_fence_before();
         }
+        if (*abort_flag && lane < S) store_remote(mapa(abort_addr, cut ? lane : me), 1);
+        __syncwarp();
         together();                                            // every partial sum of the tile is in place
+        if (*abort_flag) break;                                // (the same in every CTA of the cluster: nobody waits between its two barriers)
         tc_fence_after();
         const Mine mine = { reinterpret_cast<const float *>(smem + recv_off), S, own, mt * TM + rank * own, rows, col, cx, cy, lanes_y, bias };
         if (cy < lanes_y) {                                    // (a power of two of groups leaves no thread out)
@@ -297,6 +313,14 @@ spg_gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
         }
         __syncwarp();                                          // lanes finish different numbers of rows; the barrier is for whole warps
         if (t + step < tiles) together();                      // read before the next tile's sums replace them (the same decision in all that share it)
+    }
+    if (*abort_flag) {
+        // shared and tensor memory are given back when nothing writes to them any more
+        sent = __reduce_max_sync(0xffffffffu, sent);
+        if (warp == 0)
+            for (uint32_t i = sent > p.stages ? sent - p.stages : 0; i < sent; i++)
+                mbar_wait_uniform(full0 + 8 * (i % p.stages), (i / p.stages) & 1u, drain_addr, p.status, 54);
+        else if (warp == 1) mbar_wait_uniform(tfull, round & 1u, drain_addr, p.status, 55);
     }
     tc_fence_before();
     __syncthreads();
@@ -429,6 +453,7 @@ int split_launch(const SpgGemmArgs &a, const AtOnce &at, const SplitPlan &plan, 
     if (p.softmax && spg_tls_margin_idx) { p.margin_theta = spg_tls_margin_theta; p.margin_idx = spg_tls_margin_idx; p.margin_count = spg_tls_margin_count; }
     p.m_limit = spg_tls_rows_limit;
     p.above = counts.above; p.upto = counts.upto; p.cut_rows = counts.cut;
+    p.impatient = spg_tls_impatient ? 1 : 0;
     p.status = a.status;
     CUtensorMap map_a, map_w;
     int rc;
@@ -497,3 +522,5 @@ int spg_gemm_split_try(const SpgGemmArgs &a, const SpgDeviceProps &dp, int dev, 
     if (!split_plan(at, rows, N, kblocks, a_parts, w_parts, true, 0, false, dp.smem_optin, plan)) return SPGK_E_UNSUPPORTED;
     return split_launch(a, at, plan, { limit, ~0u, ~0u });
 }
+
+extern "C" void spgk_selftest_impatient(int on) { spg_tls_impatient = on != 0; }

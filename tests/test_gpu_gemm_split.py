@@ -7,6 +7,7 @@ import pytest
 
 pytestmark = pytest.mark.gpu
 
+TIMEOUT = -4                                           # SPGK_E_TIMEOUT
 ACT = {6: lambda v: v, 1: lambda v: np.maximum(v, 0), 3: lambda v: np.where(v > 0, v, 0.01 * v), 2: np.tanh,
        0: lambda v: 1 / (1 + np.exp(-v)), 4: lambda v: np.where(v > 1, 1 + 0.01 * (v - 1), np.where(v < 0, 0.01 * v, v))}
 
@@ -53,14 +54,15 @@ def product(spg, lib, M, N, K, a_parts, w_parts, t16, act, softmax=0, cap=None, 
     z = x * 0.75 + bias.double().cpu().numpy()
     size = 0.75 * (np.abs(A).sum(0) @ np.abs(W).sum(0).T) + np.abs(z)      # what the sum's rounding errors are relative to
 
-    def run(out_parts):
+    def run(out_parts, fails=False):
         o16 = torch.full((2, cap, ldo), 7.0, dtype=dt, device="cuda")
         o32 = torch.full((cap + 1, N), -3.0, device="cuda")
         rc = lib.spgk_layer_gemm_tc(C.byref(layer), w.data_ptr(), ld, N * ld, w_parts, t16, a.data_ptr(), ld, cap * ld, a_parts, t16,
                                     o16.data_ptr() if out_parts else None, ldo, cap * ldo, max(out_parts, 1), o32.data_ptr(), N, cap, softmax,
                                     status.data_ptr(), None)
         assert rc == 0, lib.spgk_error_string()
-        assert lib.spgk_gemm_tc_status(status.data_ptr(), None) == 0, lib.spgk_error_string()
+        rc = lib.spgk_gemm_tc_status(status.data_ptr(), None)
+        assert rc == (TIMEOUT if fails else 0), (rc, lib.spgk_error_string())
         return o16.double().cpu().numpy()[:, :, :N], o32.cpu().numpy()
     run.bias = bias                                    # `layer` holds its address only
     return z, size, run
@@ -184,3 +186,27 @@ def test_counts_beyond_what_the_device_holds_at_once(spg, lib, N, K, rows):
             assert np.all(o32[count:] == -3.0) and np.all(o16[:, count:] == 7.0)
     finally:
         lib.spgk_set_dynamic_rows(None, 0)
+
+
+@pytest.mark.parametrize("M,N,K,softmax", [(200, 1000, 512, 0), (256, 512, 784, 0), (300, 129, 1024, 0), (64, 2048, 2048, 0), (130, 10, 1000, 1), (1, 1, 1, 0)])
+def test_a_wait_that_gave_up_leaves_the_outputs_alone(spg, lib, M, N, K, softmax):
+    """Every tile's wait is given up: nothing is written or listed, the status says so, and the next call is sound."""
+    import torch
+    z, size, run = product(spg, lib, M, N, K, 2, 1, 1, 5 if softmax else 6, softmax=softmax)
+    idx, count = torch.zeros(M, dtype=torch.int32, device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
+    lib.spgk_set_margin_sink(1e30, idx.data_ptr(), count.data_ptr())
+    try:
+        for _ in range(2):
+            lib.spgk_selftest_impatient(1)
+            o16, o32 = run(0 if softmax else 2, fails=True)
+            assert np.all(o32 == -3.0) and np.all(o16 == 7.0) and int(count) == 0
+            lib.spgk_selftest_impatient(0)
+            o32 = run(0 if softmax else 2)[1][:M]
+            if softmax:
+                assert int(count) == M and np.allclose(o32.sum(1), 1, atol=1e-5)
+                count.zero_()
+            else:
+                assert np.all(np.abs(o32 - z) <= bound(K) * size + 1e-6)
+    finally:
+        lib.spgk_selftest_impatient(0)
+        lib.spgk_set_margin_sink(0.0, None, None)
