@@ -14,6 +14,10 @@ struct SpgGemmArgs {
     uint32_t N; int softmax_fused; int32_t *status; void *stream;
 };
 
+// what the calling thread's last product ran as (spgk_gemm_tc_arrangement)
+struct SpgGemmArrangement { uint32_t few_tiles, columns, split, stages; };
+extern thread_local SpgGemmArrangement spg_tls_arrangement;
+
 // 3-D tensor map over `parts` planes of a row-major [rows][ld] 16-bit matrix whose first K columns are valid; a box is 64
 // columns x box_rows x box_planes
 int spg_gemm_map(CUtensorMap *map, const void *base, int type16, uint32_t K, uint32_t rows, uint32_t ld, uint64_t plane, int parts,

@@ -472,6 +472,7 @@ int split_launch(const SpgGemmArgs &a, const AtOnce &at, const SplitPlan &plan, 
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr; cfg.numAttrs = 2;
     SPGK_CUDA(cudaLaunchKernelEx(&cfg, spg_gemm_split_kernel, map_a, map_w, p));
+    spg_tls_arrangement = { 1, p.BN, p.S, p.stages };
     return spgk_check_launch("spg_gemm_split_kernel");
 }
 

@@ -27,6 +27,8 @@
 #include <mutex>
 #include <type_traits>
 
+thread_local SpgGemmArrangement spg_tls_arrangement;
+
 namespace {
 
 constexpr uint32_t BM = 128;            // rows of C per tile (UMMA M)
@@ -932,6 +934,7 @@ static int gemm_launch(const spgk_layer *L,
     const uint32_t grid = tiles < (uint32_t)sm_count ? tiles : (uint32_t)sm_count;
     const size_t smem = 1024 + (size_t)stages * stage_bytes + p.stg_bytes + 8 * (2 * stages + 8) + 64;
     SPGK_CUDA(spg_launch_chained(spg_gemm_tc_kernel, dim3(grid), dim3(NUM_THREADS), smem, (cudaStream_t)stream, map_a, map_w, map_o, p));
+    spg_tls_arrangement = { 0, p.BN, 1, p.stages };
     return spgk_check_launch("spg_gemm_tc_kernel");
 }
 
@@ -944,6 +947,12 @@ int spgk_layer_gemm_tc(const spgk_layer *L,
 {
     return gemm_launch(L, w16, ldw, w_plane, w_parts, w_type16, a16, lda, a_plane, a_parts, type16,
                        out16, ldo16, o_plane, out_parts, out32, ldo32, N, softmax_fused, status, stream, nullptr, nullptr);
+}
+
+void spgk_gemm_tc_arrangement(uint32_t out[4])
+{
+    const SpgGemmArrangement &a = spg_tls_arrangement;
+    out[0] = a.few_tiles; out[1] = a.columns; out[2] = a.split; out[3] = a.stages;
 }
 
 int spgk_layer_gemm_tc_head(const spgk_layer *L,

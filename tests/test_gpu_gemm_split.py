@@ -22,8 +22,17 @@ def lib(spg):
     lib.spgk_set_dynamic_rows.argtypes = [vp, C.c_uint32]
     lib.spgk_set_output_rows.argtypes = [vp]
     lib.spgk_set_margin_sink.argtypes = [C.c_float, vp, vp]
+    lib.spgk_gemm_tc_arrangement.argtypes = [C.POINTER(C.c_uint32 * 4)]
+    lib.spgk_gemm_tc_arrangement.restype = None
     lib.spgk_error_string.restype = C.c_char_p
     return lib
+
+
+def arrangement(lib):
+    """Of the last launch: few-tiles kernel or not, columns of a tile, CTAs that share one, stages of the operand ring."""
+    out = (C.c_uint32 * 4)()
+    lib.spgk_gemm_tc_arrangement(C.byref(out))
+    return tuple(out)
 
 
 def planes(x, dt, parts):
@@ -74,8 +83,11 @@ def bound(K):
     return (K + 12) * 2.0 ** -23
 
 
-@pytest.mark.parametrize("M,N,K", [(1, 1, 1), (1, 16, 8), (9, 17, 63), (127, 33, 64), (128, 128, 65), (129, 10, 1000), (200, 1000, 512), (256, 512, 784),
-                                   (300, 129, 1024), (1025, 100, 129), (3001, 777, 301), (3001, 37, 129), (64, 2048, 2048)])
+SIZES = [(1, 1, 1), (1, 16, 8), (9, 17, 63), (127, 33, 64), (128, 128, 65), (129, 10, 1000), (200, 1000, 512), (256, 512, 784),
+         (300, 129, 1024), (1025, 100, 129), (3001, 777, 301), (3001, 37, 129), (64, 2048, 2048), (700, 512, 512)]
+
+
+@pytest.mark.parametrize("M,N,K", SIZES)
 @pytest.mark.parametrize("t16,a_parts,w_parts", [(0, 1, 1), (0, 2, 1), (1, 2, 1), (1, 2, 2), (1, 1, 2)])
 def test_products_of_few_tiles(spg, lib, M, N, K, t16, a_parts, w_parts):
     act = (6, 1, 3, 2, 0, 4)[(M + N + K) % 6]
@@ -83,6 +95,7 @@ def test_products_of_few_tiles(spg, lib, M, N, K, t16, a_parts, w_parts):
     want = ACT[act](z)
     for out_parts in (1, 2):
         o16, o32 = run(out_parts)
+        assert arrangement(lib)[0] == 1
         # (1e-6: the activation's own rounding; none of them stretches a difference)
         assert np.all(np.abs(o32[:M] - want) <= bound(K) * size + 1e-6 * np.maximum(1, np.abs(want)))
         assert np.all(o32[M] == -3.0)
@@ -91,6 +104,18 @@ def test_products_of_few_tiles(spg, lib, M, N, K, t16, a_parts, w_parts):
         assert np.all(np.abs(o16[:out_parts].sum(0) - o32[:M]) <= 1.01 * eps * np.abs(o32[:M]) + tiny)
         if out_parts == 1:
             assert np.all(o16[1] == 7.0)
+
+
+def test_the_sizes_meet_every_arrangement(spg, lib):
+    met = set()
+    for M, N, K in SIZES:
+        for parts in ((1, 1), (2, 1), (2, 2)):
+            product(spg, lib, M, N, K, *parts, 1, 6)[2](1)
+            met.add(arrangement(lib))
+    columns = {a[1] for a in met}
+    assert {a[0] for a in met} == {1} and {a[2] for a in met} == {1, 2, 4, 8}
+    assert any(c & (c - 1) for c in columns) and any(320 % (c // 4) for c in columns)      # (of 320 threads, some have no row)
+    assert min(columns) == 16 and max(columns) >= 128 and len({a[3] for a in met}) >= 3
 
 
 @pytest.mark.parametrize("M,N,K", [(1, 2, 8), (130, 10, 1000), (256, 16, 64), (257, 17, 130), (500, 64, 64), (40, 128, 700), (3, 100, 256)])
@@ -155,6 +180,7 @@ def test_a_softmax_of_counted_rows_does_not_hang_on_the_guess(spg, lib, N, K):
         for guess in (0, 100, 5000, 18000, 21000, cap):
             lib.spgk_set_dynamic_rows(n.data_ptr(), guess)
             results.append(run(0)[1])
+            assert arrangement(lib)[0] == 1
     finally:
         lib.spgk_set_dynamic_rows(None, 0)
     for r in results[1:]:
@@ -172,6 +198,7 @@ def test_counts_beyond_what_the_device_holds_at_once(spg, lib, N, K, rows):
     cap = 24000
     z, size, run = product(spg, lib, cap, N, K, 2, 1, 1, 1, seed=N)
     want = np.maximum(z, 0)
+    kernels = set()
     try:
         for count in rows:
             n = torch.tensor([count], dtype=torch.int32, device="cuda")
@@ -179,6 +206,7 @@ def test_counts_beyond_what_the_device_holds_at_once(spg, lib, N, K, rows):
             for guess in (0, 100, count, cap):
                 lib.spgk_set_dynamic_rows(n.data_ptr(), guess)
                 results.append(run(2))
+                kernels.add(arrangement(lib)[0])
             for o16, o32 in results[1:]:
                 assert np.array_equal(results[0][0], o16) and np.array_equal(results[0][1], o32), count
             o16, o32 = results[0]
@@ -186,6 +214,7 @@ def test_counts_beyond_what_the_device_holds_at_once(spg, lib, N, K, rows):
             assert np.all(o32[count:] == -3.0) and np.all(o16[:, count:] == 7.0)
     finally:
         lib.spgk_set_dynamic_rows(None, 0)
+    assert kernels == {0, 1}                           # few rows expected, and many
 
 
 @pytest.mark.parametrize("M,N,K,softmax", [(200, 1000, 512, 0), (256, 512, 784, 0), (300, 129, 1024, 0), (64, 2048, 2048, 0), (130, 10, 1000, 1), (1, 1, 1, 0)])
