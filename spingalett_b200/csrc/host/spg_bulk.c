@@ -5,6 +5,7 @@
  * memcpy, 3.7 with stores that do not read the destination first, 2.8 with twelve threads. */
 #include "spg_internal.h"
 #include <pthread.h>
+#include <stdatomic.h>
 #include <stdlib.h>
 #include <string.h>
 #include <unistd.h>
@@ -12,7 +13,9 @@
 #include <immintrin.h>
 #endif
 
-#define SPG_BULK_THREADS 16    /* most; SPINGALETT_STAGE_THREADS in the environment asks for another number of them */
+#define SPG_BULK_THREADS 16    /* most for a caller; SPINGALETT_STAGE_THREADS in the environment asks for another number of them */
+
+static atomic_int g_callers;   /* calls with several threads that are at work in the process */
 
 typedef struct { spg_slice_fn fn; void *ctx; size_t lo, hi; } slice;
 
@@ -23,21 +26,18 @@ static void *slice_worker(void *arg)
     return NULL;
 }
 
-static int bulk_threads(void)
+/* The cores are shared by all callers: a batch cut over several devices has one for each of them. */
+static int bulk_threads(int callers)
 {
     const char *e = getenv("SPINGALETT_STAGE_THREADS");
     const long cores = sysconf(_SC_NPROCESSORS_ONLN);
-    int want = e && atoi(e) > 0 ? atoi(e) : (int)(cores - cores / 4);      /* three quarters: the caller's program lives here too */
+    int want = e && atoi(e) > 0 ? atoi(e) : (int)(cores - cores / 4) / callers;      /* three quarters: the caller's program lives here too */
     if (want < 1) want = 1;
     return want > SPG_BULK_THREADS ? SPG_BULK_THREADS : want;
 }
 
-/* fn over [0, n) in slices that start at multiples of `grain`; a thread for every `least` of n at most */
-void spg_bulk(spg_slice_fn fn, void *ctx, size_t n, size_t grain, size_t least)
+static void run_slices(spg_slice_fn fn, void *ctx, size_t n, size_t grain, size_t nt)
 {
-    size_t nt = n / least;
-    if (nt > 1) { const size_t most = (size_t)bulk_threads(); if (nt > most) nt = most; }
-    if (nt < 2) { fn(ctx, 0, n); return; }
     const size_t share = ((n + nt - 1) / nt + grain - 1) / grain * grain;
     pthread_t th[SPG_BULK_THREADS];
     slice sl[SPG_BULK_THREADS];
@@ -50,6 +50,18 @@ void spg_bulk(spg_slice_fn fn, void *ctx, size_t n, size_t grain, size_t least)
     }
     fn(ctx, 0, share < n ? share : n);
     for (size_t t = 1; t <= started; t++) pthread_join(th[t], NULL);
+}
+
+/* fn over [0, n) in slices that start at multiples of `grain`; a thread for every `least` of n at most */
+void spg_bulk(spg_slice_fn fn, void *ctx, size_t n, size_t grain, size_t least)
+{
+    size_t nt = n / least;
+    if (nt < 2) { fn(ctx, 0, n); return; }
+    const size_t most = (size_t)bulk_threads(atomic_fetch_add(&g_callers, 1) + 1);
+    if (nt > most) nt = most;
+    if (nt < 2) fn(ctx, 0, n);
+    else run_slices(fn, ctx, n, grain, nt);
+    atomic_fetch_sub(&g_callers, 1);
 }
 
 #if defined(__x86_64__)

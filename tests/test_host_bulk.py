@@ -95,3 +95,16 @@ def on_fake_kernels(tmp_path, program):
 def test_short_last_chunks_are_staged_whole(tmp_path):
     r = subprocess.run([on_fake_kernels(tmp_path, "staged_pieces")], capture_output=True, text=True, timeout=120)
     assert r.returncode == 0 and r.stdout == "all staged\n", (r.returncode, r.stdout, r.stderr)
+
+
+@pytest.mark.parametrize("asked", ["", "5"])
+def test_callers_at_the_same_time_share_the_cores(tmp_path, asked):
+    host, exe = os.path.join(ROOT, "spingalett_b200", "csrc", "host"), str(tmp_path / "bulk_callers")
+    subprocess.run(["gcc", "-std=c2x", "-O1", "-D_GNU_SOURCE", "-I", os.path.join(ROOT, "include"), "-I", host, os.path.join(host, "spg_bulk.c"),
+                    os.path.join(ROOT, "tests", "c", "bulk_callers.c"), "-o", exe, "-lpthread"], check=True)
+    r = subprocess.run([exe], capture_output=True, text=True, timeout=60, env={**os.environ, "SPINGALETT_STAGE_THREADS": asked})
+    first, during, after = map(int, r.stdout.split())
+    cores = os.sysconf("SC_NPROCESSORS_ONLN")
+    most = int(asked) if asked else max(1, min(16, cores - cores // 4))
+    assert (first, after) == (most, most)
+    assert during == (most if asked else max(1, min(16, (cores - cores // 4) // 2)))
