@@ -404,12 +404,23 @@ uint32_t cut_rows(const AtOnce &at, uint32_t i, uint32_t N, uint32_t kblocks, ui
 
 // Which products come here, and how they are cut: those for which some tile width and split fit on the device in one wave
 // (one CTA an SM), at the width and split that the estimate below makes cheapest.  Measured for 24 products (32 to 3000 rows,
-// 10 to 2048 columns, 301 to 2048 inputs) over every width and split: the estimate picked the fastest or one within 8 % of it,
-// and none was slower than the persistent kernel, which overlaps epilogues with the next tile's products and is the better one
-// as soon as tiles come in waves.
+// 10 to 2048 columns, 301 to 2048 inputs) over every width and split: the estimate picked the fastest or one within 8 % of it.
+// Against the persistent kernel, which overlaps epilogues with the next tile's products and is the better one as soon as tiles
+// come in waves: 1296 products of 130 to 16000 rows, 256 to 24576 columns, 128 to 16384 inputs, weights from HBM.  Cut tiles take
+// 0.1 to 0.8 of its time.  Uncut ones 0.5 to 1, but for those that behind() names: with a deeper ring and wider tiles it
+// streams long operands faster.
 //
+// Whether an uncut tile is behind: one term an operand 1.02 to 1.22 of the persistent kernel's time above 144 columns (three
+// stages), 0.91 to 1.1 from 2048 inputs on; two terms above 160 columns (two stages) 0.82 to 1 up to 4096 inputs, 1.01 to 1.17
+// beyond; three terms never.
+bool behind(uint32_t BN, uint32_t kblocks, uint32_t planes)
+{
+    if (planes == 2) return BN > 144 || kblocks >= 32;
+    return planes == 3 && BN > 160 && kblocks > 64;
+}
+
 // Tile width and split of the cheapest arrangement; only_i: that split and no other, if not negative.  one_wave: only what the
-// device holds at once (false if nothing fits).
+// device holds at once (false if nothing fits, or if what fits is behind the persistent kernel).
 bool split_plan(const AtOnce &at, uint32_t rows, uint32_t N, uint32_t kblocks, uint32_t a_parts, uint32_t w_parts, bool softmax, int only_i, bool one_wave,
                 size_t smem_max, SplitPlan &best)
 {
@@ -432,7 +443,8 @@ bool split_plan(const AtOnce &at, uint32_t rows, uint32_t N, uint32_t kblocks, u
             best = { BN, S, stages, split_smem(BN, stages, stage) };
         }
     }
-    return best_cost != ~0ull;
+    if (best_cost == ~0ull) return false;
+    return !one_wave || best.S > 1 || !behind(best.BN, kblocks, a_parts + w_parts);
 }
 
 // which row counts a launch serves, and up to which K is cut

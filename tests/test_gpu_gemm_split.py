@@ -239,3 +239,12 @@ def test_a_wait_that_gave_up_leaves_the_outputs_alone(spg, lib, M, N, K, softmax
     finally:
         lib.spgk_selftest_impatient(0)
         lib.spgk_set_margin_sink(0.0, None, None)
+
+
+@pytest.mark.parametrize("M,N,K,a_parts,few", [(1500, 2000, 256, 1, 0), (1500, 2000, 256, 2, 1), (700, 3000, 1984, 1, 1), (700, 3000, 2040, 1, 0),
+                                               (1500, 2000, 4096, 2, 1), (1500, 2000, 4104, 2, 0), (130, 512, 4104, 1, 1)])
+def test_long_or_wide_uncut_tiles_are_left_to_the_persistent_kernel(spg, lib, M, N, K, a_parts, few):
+    z, size, run = product(spg, lib, M, N, K, a_parts, 1, 1, 6)
+    o32 = run(0)[1]
+    assert arrangement(lib)[0] == few
+    assert np.all(np.abs(o32[:M] - z) <= bound(K) * size + 1e-6)
