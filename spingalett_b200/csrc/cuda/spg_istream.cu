@@ -15,8 +15,9 @@
 // When a layer's input has a wide row, every k-block is multiplied with both sets of digits, into both accumulators: weights
 // and unpacking are shared.  Rows of a normal draw, of pixels, or of what the hidden activations make of them are not wide
 // (0.1 to 5 % of small elements; the most for a leaky rectifier, whose slope puts half of a row within 1 % of the other half).
-// Looking for wide rows costs about 1 us of a layer (INT4 net 8192-16384-16384-8192-1000: 151 -> 156 us at 8 rows, 201 -> 204 at
-// 64); with one input of 1e6 beside ordinary ones, which makes every row of that net's layers wide: 221, 367, and 954 at 256.
+// Looking for wide rows costs about 1 us of a layer; with one input of 1e6 beside ordinary ones, which makes every row of that net's
+// layers wide, the INT4 net 8192-16384-16384-8192-1000 takes 185 us instead of 127 at 8 rows, 353 instead of 177 at 64, 1034
+// instead of 492 at 256 (one batch again and again).
 //
 // What bounds it.  HBM needs 41 us for the 272 MB of the INT4 net 8192-16384-16384-8192-1000.  A 128 x 128 block of
 // weights moves through shared memory as 8 KB packed (in and out), 16 KB of operand (in and out) and C * 128 B of digits
@@ -24,10 +25,11 @@
 // 106 us over the net, whose busiest SMs have 237 such blocks.  One byte per weight in the operand instead of two is why this
 // path exists beside the 16-bit streaming kernel, which writes and reads 32 KB per such block.
 //
-// Measured: 125 us at 8 rows (GEMV: 201), 188 at 64 (16-bit streaming kernel: 577), 561 at 256 (GEMM chain: 684).  A block of
+// Measured: 125 us at 8 rows (GEMV: 201), 188 at 64 (16-bit streaming kernel: 577), 555 at 256 (GEMM chain: 684).  A block of
 // INT4 takes 480 cycles at 8 rows, of which the MMA warp's own turn is all (operand tiles changing hands one at a time: 810),
 // and 750 at 64 (900), where every CTA draws 32 KB of digits a block from L2 at 43 bytes a cycle; the tensor pipe would need
-// 512.  INT8, whose boxes need no unpacking, takes 725 cycles at 8 rows, 5.4 TB/s.  The rest of a layer is staging, the first
+// 512.  From layers of 32 to 166 blocks with weights from HBM: 530 cycles a block and 14 us a layer at 8 rows, 870 and 16 at 64.
+// INT8, whose boxes need no unpacking, takes 700 cycles at 8 rows, 5.5 TB/s.  The rest of a layer is staging, the first
 // boxes and tiles, and the last sums (1 us at 8 rows, 3 at 64).
 //
 // Per CTA (one per SM, 19 warps):

@@ -791,7 +791,8 @@ int spg_dev_forward_large(spg_net *n, const float *d_x, uint32_t N, float *d_out
     if (!softmax_out) return large_chain(n, d_x, N, d_out, true);
     /* Few rows: the chain is bound by streaming the weights (or by latency), where the exact chain's second pass over K
      * is nearly free, while the one-term pass plus the recomputation chain costs two chains: 0.70 ms against 1.05 ms at
-     * 256 rows of the large INT4 net, 1.00 against 1.20 at 512 (the curves cross near 700 rows). */
+     * 256 rows of the large INT4 net, 1.00 against 1.20 at 512 (the curves crossed near 700 rows; drawn before products of few
+     * tiles had a kernel of their own). */
     if (N <= SPG_AUTO_EXACT_ROWS) return large_chain(n, d_x, N, d_out, true);
 
     int rc;
@@ -862,7 +863,7 @@ int spg_dev_forward_large(spg_net *n, const float *d_x, uint32_t N, float *d_out
         if ((rc = reserve((void **)&n->d_rep_out, &n->rep_out_bytes, (size_t)N * outw * 4, "repair outputs"))) return rc;
     }
     /* The flagged rows are a percent or two of the batch, so either repair is one latency-bound pass over a handful of
-     * tiles.  Measured on the benchmark MLP at 65536 rows: the per-layer exact chain takes 67 us, the one-launch kernel
+     * tiles.  Measured on the benchmark MLP at 65536 rows: the per-layer exact chain takes 30 us, the one-launch kernel
      * in pair mode 93 us (a single 128-row tile runs its 13 + 32 k-blocks and six epilogues back to back), so the chain
      * is the default; SPINGALETT_REPAIR=fused selects the other for comparisons. */
     static int repair_fused = -1;
@@ -1059,12 +1060,13 @@ static float *forward_batch_on(spg_net *n, ForwardBatchArgs a)
      * to 8 rows go layer by layer (GEMV first), up to 512 rows in groups of at most 128 through the 16-bit streaming kernel when
      * it takes every layer, each group streaming the packed weights once; everything else is the large-batch GEMM chain.
      *
-     * The line at 7 rows is where the large INT4 net crosses; small nets are ahead at 7 already (0.63 of the time and less) and
-     * where they cross has not been looked for.  Measured, against the
-     * path that served before: large INT4 net 157 us against 204 (GEMV) at 8 rows, 211 against 578 (16-bit streaming kernel)
-     * at 64, 628 against 684 (GEMM chain) at 256; at 6 rows the GEMV is level (155, INT2 131), at 512 the chain is ahead
-     * (945).  Nets of 4 and 12 MB: 38 against 54 and 42 against 65 us at 8 rows, 0.45 of the time or less at 32 to 96,
-     * 0.8 to 0.9 at 128 and 256; of 0.5 MB: 34 against 119 us at 8 rows, but no gain beyond 96.  FAST asks for one term per
+     * Measured, against the path that served before: large INT4 net 126 us against 204 (GEMV) at 8 rows, 188 against 578
+     * (16-bit streaming kernel) at 64, 555 against 684 (GEMM chain) at 256.  Nets of 4 and 12 MB: 33 against 54 and 36 against
+     * 65 us at 8 rows, 0.45 of the time or less at 32 to 96; of 0.5 MB: 32 against 119 us at 8 rows.  The lines were drawn where
+     * the curves of older kernels crossed: the one at 7 rows when 8 rows took 157 us here (the GEMV: 155 at 6, INT2 132), the
+     * ones at 96 rows and 4 MB before products of few tiles had a kernel of their own (0.5 MB: 41 us here at 96 rows, 22 on the
+     * GEMM chain at 128; 4 MB: 51 here at 128), the one at 256 with the chain at 945 us for 512 rows (now 876).  Where today's
+     * cross has not been looked for.  FAST asks for one term per
      * operand, which the GEMM chain serves beyond 96 rows.  EXACT promises 16 bits of every single value, which this kernel's
      * fixed-point numbers hold for all but the few smallest of a row: beyond 24 rows (up to there the alternative is the GEMV,
      * whose fixed-point numbers are coarser) EXACT stays with the kernels that feed two 16-bit terms. */
