@@ -112,8 +112,8 @@ SPGK_API int spgk_softmax_rows(float *y, uint32_t ldy, uint32_t N, uint32_t widt
  * this thread -- spgk_split16, spgk_gather_rows, spgk_scatter_rows, spgk_softmax_rows, spgk_layer_gemm_tc --
  * treat their row argument as a capacity and work on min(rows, *ptr) rows, *ptr being read by the kernels
  * when they run, so a selection made on the device (spgk_margin_select) can be followed up without a host
- * round trip.  `expected` is the caller's guess of the count (0 = none); it only steers tile shapes.  NULL
- * switches it off.  (No reference counterpart.) */
+ * round trip.  `expected` is the caller's guess of the count (0 = none); it steers tile shapes and which
+ * kernel is ready for many rows, results do not hang on it.  NULL switches it off.  (No reference counterpart.) */
 SPGK_API void spgk_set_dynamic_rows(const uint32_t *rows_dev, uint32_t expected);
 /* After spgk_set_margin_sink(theta, idx, count) the next spgk_layer_gemm_tc calls of this thread that finish a
  * softmax row in their epilogue (softmax_fused = 1) do the work of spgk_margin_select on the way: rows whose two
@@ -267,7 +267,8 @@ SPGK_API int spgk_istream_status(void *scratch, void *stream);
  * layer needs spgk_softmax_rows afterwards.
  * status: dev int32 the kernel reports a bounded wait that gave up in; read it
  * with spgk_gemm_tc_status() (which synchronises the stream).
- * Products that fit the device in one wave of smaller tiles run in a kernel that also cuts K (spg_gemm_split.cu).
+ * Products that fit the device in one wave of smaller tiles run in a kernel that also cuts K (spg_gemm_split.cu); where only
+ * the device knows the row count, that count decides there.
  * Does batch_forward()'s layer step, reference Training.c:318-343. */
 SPGK_API int spgk_gemm_tc_supported(const spgk_layer *L);
 SPGK_API uint32_t spgk_gemm_tc_softmax_max(void);
