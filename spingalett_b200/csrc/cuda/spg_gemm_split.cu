@@ -248,6 +248,7 @@ spg_gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
         if (col + 1 < p.N) bias.y = load_early(p.bias + col + 1);
         if (col + 2 < p.N) bias.z = load_early(p.bias + col + 2);
         if (col + 3 < p.N) bias.w = load_early(p.bias + col + 3);
+        bool gone = false;                                     // a wait of this warp gave up
         if (warp == 0) {
             for (uint32_t kb = kb0; kb < kb1; kb++, it++) {
                 const uint32_t s = it % p.stages, ph = (it / p.stages) & 1u, st = base + s * p.stage_bytes;
@@ -289,7 +290,8 @@ spg_gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
             __syncwarp();                                      // each lane has waited in a loop of its own; what follows is for whole warps
             tc_fence_after();
             const uint32_t dst = mapa(base + recv_off + (rank * own + row % own) * p.BN * 4, cut ? row / own : me);
-            if (__all_sync(0xffffffffu, ok)) {
+            gone = !__all_sync(0xffffffffu, ok);
+            if (!gone) {
                 for (uint32_t c = 16 * half; c < p.BN; c += 32) {
                     uint32_t r[16];
                     tmem_ld16(tmem + c + ((q * 32u) << 16), r);
@@ -300,7 +302,8 @@ spg_gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
             }
             tc_fence_before();
         }
-        if (*abort_flag && lane < S) store_remote(mapa(abort_addr, cut ? lane : me), 1);
+        if (warp < 2) gone = *abort_flag;
+        if (gone && lane < S) store_remote(mapa(abort_addr, cut ? lane : me), 1);
         __syncwarp();
         together();                                            // every partial sum of the tile is in place
         if (*abort_flag) break;                                // (the same in every CTA of the cluster: nobody waits between its two barriers)
