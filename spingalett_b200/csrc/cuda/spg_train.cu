@@ -7,11 +7,11 @@
 //   delta_l   = (delta_{l+1} W_l) * act'(a_l)            batch_compute_deltas     :374-393
 //   gW_l      = s * delta_{l+1}^T a_l,  gB_l = s * colsum batch_accumulate_gradients :396-419
 //   Adam      eps inside the square root                  SIMD.c:279-328
-// Everything is fp32, as in the reference.  The step is latency-bound (about
-// 1.2 GFLOP per 256-row batch of the 784-512-1000-10 MLP), so the GEMMs are a
-// plain shared-memory tiled fp32 kernel with the three operand layouts the step
-// needs and the elementwise work fused into its epilogue.
-#include "spg_common.cuh"
+// Everything is fp32, as in the reference.  Large products are a plain
+// shared-memory tiled fp32 kernel with the three operand layouts the step needs
+// and the elementwise work fused into its epilogue; smaller ones, and the output
+// end of a step, are in spg_train_mma.cu.
+#include "spg_train.cuh"
 #include <dlfcn.h>
 #include <chrono>
 #include <condition_variable>
@@ -25,8 +25,6 @@
 namespace {
 
 constexpr int TK = 16;      // k depth of a staged tile; the CTA tile is TS x TS, (TS/4)^2 threads with 4x4 outputs each
-
-enum { GEMM_FWD = 0, GEMM_DELTA = 1, GEMM_GRAD = 2 };
 
 // Four consecutive floats at `base`: one 128-bit load when `vec`, else element-wise with zeros where the row is
 // outside the matrix (`row_ok` false) or the element index first+j reaches `limit`.
@@ -59,8 +57,8 @@ spg_train_gemm_kernel(const float *__restrict__ A, uint32_t lda, const float *__
 {
     constexpr int TM = TS, TN = TS, NT = (TS / 4) * (TS / 4), Q = TS / 4;     // Q: groups of four per tile row along m or n
     constexpr int R = TS * TK / 4 / NT;                                       // groups per thread per operand
-    constexpr bool a_km = MODE == GEMM_GRAD;                    // A stored [K][M] (contiguous in m); otherwise [M][K]
-    constexpr bool b_nk = MODE == GEMM_FWD;                     // B stored [N][K] (contiguous in k); otherwise [K][N]
+    constexpr bool a_km = MODE == TRAIN_GRAD;                    // A stored [K][M] (contiguous in m); otherwise [M][K]
+    constexpr bool b_nk = MODE == TRAIN_FWD;                     // B stored [N][K] (contiguous in k); otherwise [K][N]
     static_assert(KS == 1 || (KS - 1) * NT * 20 <= KS * 2 * TK * (TS + 4), "the partial sums reuse the staging memory");
     __shared__ __align__(16) float sm[KS][2][TK][TS + 4];
     const uint32_t slice = threadIdx.x / NT, tid = threadIdx.x % NT, tx = tid % Q, ty = tid / Q;
@@ -77,7 +75,7 @@ spg_train_gemm_kernel(const float *__restrict__ A, uint32_t lda, const float *__
     float4 ra[R], rb[R];
     // MODE 2 with `colsum`: the CTAs of the first tile column also sum their A tile over k, colsum[m] = alpha * sum_k A[k][m]
     // (the bias gradient beside the weight gradient); one thread per group of four m carries those sums
-    const bool cs = MODE == GEMM_GRAD && colsum != nullptr && blockIdx.x == 0 && tx == 0;
+    const bool cs = MODE == TRAIN_GRAD && colsum != nullptr && blockIdx.x == 0 && tx == 0;
     float bs[4] = { 0.0f, 0.0f, 0.0f, 0.0f };
 
     auto fetch = [&](uint32_t k0) {
@@ -177,171 +175,22 @@ spg_train_gemm_kernel(const float *__restrict__ A, uint32_t lda, const float *__
             const uint32_t n = n0 + tx * 4 + j;
             if (n >= N) continue;
             float v = acc[i][j];
-            if (MODE == GEMM_FWD) v = spg_activate(v + bias[n], act);
-            else if (MODE == GEMM_DELTA) v *= spg_derivative(aux[(uint64_t)m * ldaux + n], act);
+            if (MODE == TRAIN_FWD) v = spg_activate(v + bias[n], act);
+            else if (MODE == TRAIN_DELTA) v *= spg_derivative(aux[(uint64_t)m * ldaux + n], act);
             else v *= alpha;
             C[(uint64_t)m * ldc + n] = v;
         }
     }
 }
 
-// ---- the same three products on the tensor cores, with fp32-level error -------------------------------------------------
-// An fp32 value x is split into hi = tf32(x) and lo = tf32(x - hi); a*b is formed as a_lo*b_hi + a_hi*b_lo + a_hi*b_hi by
-// three mma.m16n8k8.tf32 with fp32 accumulation (the dropped a_lo*b_lo term is below 2^-22 of the product).  CTA tile
-// 32 x 32, KS k-slices of two warps each (a warp owns 16 rows x 32 columns of the slice's partial sum); staging, slice
-// order and the fixed-order addition of the partial sums are those of spg_train_gemm_kernel.  The staged tiles have a
-// pitch of 40 floats, which makes the fragment reads As[k][m], k = lane%4 (+4), m = lane/4 (+8), conflict-free.
-__device__ __forceinline__ void tf32_split(float x, uint32_t &hi, uint32_t &lo)
-{
-    asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(hi) : "f"(x));
-    asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(lo) : "f"(x - __uint_as_float(hi)));
-}
-
-__device__ __forceinline__ void mma_tf32(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1)
-{
-    asm volatile("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-
-template <int MODE, int KS>
-__global__ void __launch_bounds__(64 * KS)
-spg_train_mma_kernel(const float *__restrict__ A, uint32_t lda, const float *__restrict__ B, uint32_t ldb,
-                     float *__restrict__ C, uint32_t ldc, uint32_t M, uint32_t N, uint32_t K,
-                     float alpha, const float *__restrict__ bias, const float *__restrict__ aux, uint32_t ldaux, int act,
-                     float *__restrict__ colsum)
-{
-    constexpr int TS = 32, NT = 64, Q = 8, R = 2, P = TS + 8;
-    constexpr bool a_km = MODE == GEMM_GRAD;
-    constexpr bool b_nk = MODE == GEMM_FWD;
-    static_assert((KS - 1) * (NT * 16 + TS) <= KS * 2 * TK * P, "the partial sums reuse the staging memory");
-    __shared__ __align__(16) float sm[KS][2][TK][P];
-    const uint32_t slice = threadIdx.x / NT, tid = threadIdx.x % NT, lane = tid & 31u, mh = tid >> 5, g = lane >> 2, t = lane & 3u;
-    float (*As)[P] = sm[slice][0];
-    float (*Bs)[P] = sm[slice][1];
-    const uint32_t m0 = blockIdx.y * TS, n0 = blockIdx.x * TS;
-    const bool a_al = (lda & 3u) == 0 && (reinterpret_cast<uintptr_t>(A) & 15u) == 0 && m0 + TS <= M;
-    const bool b_al = (ldb & 3u) == 0 && (reinterpret_cast<uintptr_t>(B) & 15u) == 0 && n0 + TS <= N;
-    float acc[4][4];                                            // [8-column block][fragment register]
-#pragma unroll
-    for (int i = 0; i < 4; i++)
-#pragma unroll
-        for (int j = 0; j < 4; j++) acc[i][j] = 0.0f;
-    float4 ra[R], rb[R];
-    const bool cs = MODE == GEMM_GRAD && colsum != nullptr && blockIdx.x == 0 && tid < (uint32_t)TS;    // thread tid sums column m0+tid
-    float bsum = 0.0f;
-
-    auto fetch = [&](uint32_t k0) {
-        const bool whole = k0 + TK <= K;
-#pragma unroll
-        for (int r = 0; r < R; r++) {
-            const uint32_t i = tid + r * NT;
-            if (a_km) {
-                const uint32_t k = i / Q, m = (i % Q) * 4;
-                ra[r] = train_load4(A + (uint64_t)(k0 + k) * lda + m0 + m, a_al && whole, k0 + k < K, m0 + m, M);
-            } else {
-                const uint32_t m = i / (TK / 4), k = (i % (TK / 4)) * 4;
-                ra[r] = train_load4(A + (uint64_t)(m0 + m) * lda + k0 + k, a_al && whole, m0 + m < M, k0 + k, K);
-            }
-            if (b_nk) {
-                const uint32_t n = i / (TK / 4), k = (i % (TK / 4)) * 4;
-                rb[r] = train_load4(B + (uint64_t)(n0 + n) * ldb + k0 + k, b_al && whole, n0 + n < N, k0 + k, K);
-            } else {
-                const uint32_t k = i / Q, n = (i % Q) * 4;
-                rb[r] = train_load4(B + (uint64_t)(k0 + k) * ldb + n0 + n, b_al && whole, k0 + k < K, n0 + n, N);
-            }
-        }
-    };
-    auto stage = [&]() {
-#pragma unroll
-        for (int r = 0; r < R; r++) {
-            const uint32_t i = tid + r * NT;
-            if (a_km) {
-                *reinterpret_cast<float4 *>(&As[i / Q][(i % Q) * 4]) = ra[r];
-            } else {
-                const uint32_t m = i / (TK / 4), k = (i % (TK / 4)) * 4;
-                As[k][m] = ra[r].x; As[k + 1][m] = ra[r].y; As[k + 2][m] = ra[r].z; As[k + 3][m] = ra[r].w;
-            }
-            if (b_nk) {
-                const uint32_t n = i / (TK / 4), k = (i % (TK / 4)) * 4;
-                Bs[k][n] = rb[r].x; Bs[k + 1][n] = rb[r].y; Bs[k + 2][n] = rb[r].z; Bs[k + 3][n] = rb[r].w;
-            } else {
-                *reinterpret_cast<float4 *>(&Bs[i / Q][(i % Q) * 4]) = rb[r];
-            }
-        }
-    };
-
-    fetch(slice * TK);
-    for (uint32_t kb = 0; kb < K; kb += KS * TK) {
-        stage();
-        __syncthreads();
-        if (kb + KS * TK < K) fetch(kb + (KS + slice) * TK);
-#pragma unroll
-        for (int ks = 0; ks < TK; ks += 8) {
-            uint32_t ah[4], al[4];
-            tf32_split(As[ks + t][mh * 16 + g], ah[0], al[0]);
-            tf32_split(As[ks + t][mh * 16 + g + 8], ah[1], al[1]);
-            tf32_split(As[ks + t + 4][mh * 16 + g], ah[2], al[2]);
-            tf32_split(As[ks + t + 4][mh * 16 + g + 8], ah[3], al[3]);
-#pragma unroll
-            for (int nb = 0; nb < 4; nb++) {
-                uint32_t bh0, bl0, bh1, bl1;
-                tf32_split(Bs[ks + t][nb * 8 + g], bh0, bl0);
-                tf32_split(Bs[ks + t + 4][nb * 8 + g], bh1, bl1);
-                mma_tf32(acc[nb], al, bh0, bh1);
-                mma_tf32(acc[nb], ah, bl0, bl1);
-                mma_tf32(acc[nb], ah, bh0, bh1);
-            }
-        }
-        if (cs) {
-#pragma unroll
-            for (int k = 0; k < TK; k++) bsum += As[k][tid];
-        }
-        __syncthreads();
-    }
-    {
-        float *red = &sm[0][0][0][0];
-        if (slice > 0) {
-#pragma unroll
-            for (int i = 0; i < 16; i++) red[(slice - 1) * (NT * 16 + TS) + i * NT + tid] = acc[i >> 2][i & 3];
-            if (cs) red[(slice - 1) * (NT * 16 + TS) + NT * 16 + tid] = bsum;
-        }
-        __syncthreads();
-        if (slice > 0) return;
-        for (int sl = 0; sl < KS - 1; sl++) {
-#pragma unroll
-            for (int i = 0; i < 16; i++) acc[i >> 2][i & 3] += red[sl * (NT * 16 + TS) + i * NT + tid];
-            if (cs) bsum += red[sl * (NT * 16 + TS) + NT * 16 + tid];
-        }
-    }
-    if (cs && m0 + tid < M) colsum[m0 + tid] = alpha * bsum;
-#pragma unroll
-    for (int nb = 0; nb < 4; nb++) {
-#pragma unroll
-        for (int c = 0; c < 4; c++) {
-            const uint32_t m = m0 + mh * 16 + g + (c >> 1) * 8, n = n0 + nb * 8 + 2 * t + (c & 1);
-            if (m >= M || n >= N) continue;
-            float v = acc[nb][c];
-            if (MODE == GEMM_FWD) v = spg_activate(v + bias[n], act);
-            else if (MODE == GEMM_DELTA) v *= spg_derivative(aux[(uint64_t)m * ldaux + n], act);
-            else v *= alpha;
-            C[(uint64_t)m * ldc + n] = v;
-        }
-    }
-}
-
-// Forward product of a narrow layer (N <= 16 outputs, e.g. the class scores): one warp per row of A, the lanes striding
-// over k, every lane keeping N partial sums that a shuffle tree adds at the end.  The N rows of B are read by every warp
-// and stay in L1.  C[m][n] = act(sum_k A[m][k] B[n][k] + bias[n]).
-// FUSE 1 / 2 make it the whole output end of a training step in one launch: the row's softmax (1) or sigmoid (2) is formed
-// in the warp, C gets the activation, delta[m][n] = C[m][n] - T[m][n], and the row's cross-entropy is added to *loss when
-// loss is not null (same formulas as spg_softmax_rows_kernel and spg_ce_delta_kernel).
-template <bool VEC, int FUSE>
+// Forward product of a narrow layer (N <= 16 outputs): one warp per row of A, the lanes striding over k, every lane keeping N
+// partial sums that a shuffle tree adds at the end.  The N rows of B are read by every warp and stay in L1.
+// C[m][n] = act(sum_k A[m][k] B[n][k] + bias[n]).
+template <bool VEC>
 __global__ void __launch_bounds__(256)
 spg_train_fwd_narrow_kernel(const float *__restrict__ A, uint32_t lda, const float *__restrict__ B, uint32_t ldb,
                             float *__restrict__ C, uint32_t ldc, uint32_t M, uint32_t N, uint32_t K,
-                            const float *__restrict__ bias, int act, const float *__restrict__ T, float *__restrict__ delta,
-                            float *loss)
+                            const float *__restrict__ bias, int act)
 {
     const uint32_t lane = threadIdx.x & 31u, m = blockIdx.x * 8u + (threadIdx.x >> 5);
     if (m >= M) return;
@@ -377,39 +226,7 @@ spg_train_fwd_narrow_kernel(const float *__restrict__ A, uint32_t lda, const flo
 #pragma unroll
     for (int n = 0; n < 16; n++)
         if (lane == (uint32_t)n) v = acc[n];
-    const bool mine = lane < N;
-    const float z = mine ? v + bias[lane] : 0.0f;
-    if (FUSE == 0) {
-        if (mine) C[(uint64_t)m * ldc + lane] = spg_activate(z, act);
-        return;
-    }
-    float o;
-    if (FUSE == 1) {
-        const float mx = spg_warp_max(mine ? z : -FLT_MAX);
-        const float e = mine ? expf(z - mx) : 0.0f;
-        const float sum = spg_warp_sum(e);
-        o = sum > 0.0f ? e * (1.0f / sum) : e;
-    } else {
-        o = spg_activate(z, SPG_ACT_SIGMOID);
-    }
-    float local = 0.0f;
-    if (mine) {
-        const float tg = T[(uint64_t)m * N + lane];
-        C[(uint64_t)m * ldc + lane] = o;
-        delta[(uint64_t)m * N + lane] = o - tg;
-        if (loss) {
-            if (FUSE == 2) {
-                const float c = fminf(fmaxf(o, 1e-9f), 1.0f - 1e-9f);
-                local = -(tg * logf(c) + (1.0f - tg) * logf(1.0f - c));
-            } else {
-                local = -tg * logf(fmaxf(o, 1e-9f));
-            }
-        }
-    }
-    if (loss) {
-        local = spg_warp_sum(local);
-        if (lane == 0) atomicAdd(loss, local);
-    }
+    if (lane < N) C[(uint64_t)m * ldc + lane] = spg_activate(v + bias[lane], act);
 }
 
 // delta = a - t over `count` elements; optionally adds the cross-entropy of each row to *loss
@@ -683,36 +500,29 @@ static int train_gemm(int mode, const float *A, uint32_t lda, const float *B, ui
                       uint32_t M, uint32_t N, uint32_t K, float alpha, const float *bias, const float *aux, uint32_t ldaux,
                       int act, float *colsum, void *stream)
 {
-    if (!A || !B || !C || M == 0 || N == 0 || K == 0 || (mode == GEMM_FWD && !bias) || (mode == GEMM_DELTA && !aux)) {
+    if (!A || !B || !C || M == 0 || N == 0 || K == 0 || (mode == TRAIN_FWD && !bias) || (mode == TRAIN_DELTA && !aux)) {
         spgk_set_error("spgk_train_gemm", "bad argument");
         return SPGK_E_ARG;
     }
     cudaStream_t s = (cudaStream_t)stream;
-    if (act == SPG_ACT_SOFTMAX && mode == GEMM_FWD) act = SPG_ACT_NONE;      // softmax rows are finished separately
-    if (mode != GEMM_FWD && mode != GEMM_DELTA && mode != GEMM_GRAD) { spgk_set_error("spgk_train_gemm", "unknown mode"); return SPGK_E_ARG; }
-    if (mode == GEMM_FWD && N <= 16u) {
+    if (act == SPG_ACT_SOFTMAX && mode == TRAIN_FWD) act = SPG_ACT_NONE;      // softmax rows are finished separately
+    if (mode != TRAIN_FWD && mode != TRAIN_DELTA && mode != TRAIN_GRAD) { spgk_set_error("spgk_train_gemm", "unknown mode"); return SPGK_E_ARG; }
+    if (mode == TRAIN_FWD && N <= 16u) {
         const bool vec = (K & 3u) == 0 && (lda & 3u) == 0 && (ldb & 3u) == 0 &&
                          ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(B)) & 15u) == 0;
-        if (vec) spg_train_fwd_narrow_kernel<true, 0><<<(M + 7) / 8, 256, 0, s>>>(A, lda, B, ldb, C, ldc, M, N, K, bias, act, nullptr, nullptr, nullptr);
-        else spg_train_fwd_narrow_kernel<false, 0><<<(M + 7) / 8, 256, 0, s>>>(A, lda, B, ldb, C, ldc, M, N, K, bias, act, nullptr, nullptr, nullptr);
+        if (vec) spg_train_fwd_narrow_kernel<true><<<(M + 7) / 8, 256, 0, s>>>(A, lda, B, ldb, C, ldc, M, N, K, bias, act);
+        else spg_train_fwd_narrow_kernel<false><<<(M + 7) / 8, 256, 0, s>>>(A, lda, B, ldb, C, ldc, M, N, K, bias, act);
         return spgk_check_launch("spg_train_fwd_narrow_kernel");
     }
     // Products of at least 148 64 x 64 tiles: the SIMT kernel with that tile.  Smaller ones - on a 256-row step of a
-    // 784-512-1000-10 network that is every product - take 32 x 32 tiles on the tensor cores with the k range of a tile
-    // split over four two-warp slices of the CTA, eight when there are at most 32 tiles.
-    const uint32_t tiles64 = ((N + 63) / 64) * ((M + 63) / 64), tiles32 = ((N + 31) / 32) * ((M + 31) / 32);
-    const int shape = tiles64 >= 148u ? 0 : tiles32 > 32u ? 1 : 2;
-#define SPG_TRAIN_ARGS A, lda, B, ldb, C, ldc, M, N, K, alpha, bias, aux, ldaux, act, colsum
-#define SPG_TRAIN_SHAPES(MODEV) \
-    do { const dim3 g32((N + 31) / 32, (M + 31) / 32); \
-         if (shape == 0) spg_train_gemm_kernel<MODEV, 64, 1><<<dim3((N + 63) / 64, (M + 63) / 64), 256, 0, s>>>(SPG_TRAIN_ARGS); \
-         else if (shape == 1) spg_train_mma_kernel<MODEV, 4><<<g32, 256, 0, s>>>(SPG_TRAIN_ARGS); \
-         else spg_train_mma_kernel<MODEV, 8><<<g32, 512, 0, s>>>(SPG_TRAIN_ARGS); } while (0)
-    if (mode == GEMM_FWD) SPG_TRAIN_SHAPES(GEMM_FWD);
-    else if (mode == GEMM_DELTA) SPG_TRAIN_SHAPES(GEMM_DELTA);
-    else SPG_TRAIN_SHAPES(GEMM_GRAD);
-#undef SPG_TRAIN_SHAPES
-#undef SPG_TRAIN_ARGS
+    // 784-512-1000-10 network that is every product - take 32 x 32 tiles on the tensor cores.
+    const uint32_t tiles64 = ((N + 63) / 64) * ((M + 63) / 64);
+    if (tiles64 < 148u)
+        return spg_train_product(mode, SpgTrainProduct{ A, B, C, lda, ldb, ldc, M, N, K, alpha, bias, aux, ldaux, act, colsum }, s);
+    const dim3 grid((N + 63) / 64, (M + 63) / 64);
+    if (mode == TRAIN_FWD) spg_train_gemm_kernel<TRAIN_FWD, 64, 1><<<grid, 256, 0, s>>>(A, lda, B, ldb, C, ldc, M, N, K, alpha, bias, aux, ldaux, act, colsum);
+    else if (mode == TRAIN_DELTA) spg_train_gemm_kernel<TRAIN_DELTA, 64, 1><<<grid, 256, 0, s>>>(A, lda, B, ldb, C, ldc, M, N, K, alpha, bias, aux, ldaux, act, colsum);
+    else spg_train_gemm_kernel<TRAIN_GRAD, 64, 1><<<grid, 256, 0, s>>>(A, lda, B, ldb, C, ldc, M, N, K, alpha, bias, aux, ldaux, act, colsum);
     return spgk_check_launch("spg_train_gemm_kernel");
 }
 
@@ -727,26 +537,7 @@ int spgk_train_grad(const float *delta, uint32_t ldd, const float *a, uint32_t l
                     uint32_t out, uint32_t in, uint32_t rows, float scale, void *stream)
 {
     if (!gb) { spgk_set_error("spgk_train_grad", "bad argument"); return SPGK_E_ARG; }
-    return train_gemm(GEMM_GRAD, delta, ldd, a, lda, gw, ldg, out, in, rows, scale, nullptr, nullptr, 0, 0, gb, stream);
-}
-
-int spgk_train_output(const float *x, uint32_t ldx, const float *w, uint32_t ldw, const float *bias, float *y, const float *t,
-                      float *delta, float *loss, uint32_t rows, uint32_t out, uint32_t in, int sigmoid_output, void *stream)
-{
-    if (!x || !w || !bias || !y || !t || !delta || rows == 0 || in == 0 || out == 0 || out > 16u) {
-        spgk_set_error("spgk_train_output", "bad argument");
-        return SPGK_E_ARG;
-    }
-    cudaStream_t s = (cudaStream_t)stream;
-    const bool vec = (in & 3u) == 0 && (ldx & 3u) == 0 && (ldw & 3u) == 0 &&
-                     ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w)) & 15u) == 0;
-    const dim3 grid((rows + 7) / 8);
-#define SPG_OUT_LAUNCH(VECV, FUSEV) \
-    spg_train_fwd_narrow_kernel<VECV, FUSEV><<<grid, 256, 0, s>>>(x, ldx, w, ldw, y, out, rows, out, in, bias, 0, t, delta, loss)
-    if (sigmoid_output) { if (vec) SPG_OUT_LAUNCH(true, 2); else SPG_OUT_LAUNCH(false, 2); }
-    else { if (vec) SPG_OUT_LAUNCH(true, 1); else SPG_OUT_LAUNCH(false, 1); }
-#undef SPG_OUT_LAUNCH
-    return spgk_check_launch("spg_train_fwd_narrow_kernel");
+    return train_gemm(TRAIN_GRAD, delta, ldd, a, lda, gw, ldg, out, in, rows, scale, nullptr, nullptr, 0, 0, gb, stream);
 }
 
 // ---- device step state and graph replay of a training step --------------------------------------------------------------
