@@ -77,12 +77,14 @@ def arithmetic(path, dtype, math):
     """What the path that ran (spingalett_last_path) computes with."""
     if path == "istream" or path == "gemv" and dtype in ("int8", "int4", "int2"):
         return "s8 digits x s8 -> s32 (exact sums of 28-bit fixed-point activations)"
+    if path == "rows":
+        return "f64 products and sums"
     if path in ("gemv", "wstream"):
         return "bf16 terms x bf16 -> f32 (exact products)"
     return {"exact": "bf16(hi+lo)xbf16->f32", "fast": "f16xf16->f32", "auto": "f16xf16->f32 + exact recompute of low-margin rows"}[math]
 
 
-KERNEL_OF_PATH = {"gemv": "spg_gemv_kernel", "istream": "spg_istream_kernel", "wstream": "spg_wstream_kernel", "tcgen05": "spg_gemm_tc_kernel",
+KERNEL_OF_PATH = {"rows": "spg_rows_kernel", "gemv": "spg_gemv_kernel", "istream": "spg_istream_kernel", "wstream": "spg_wstream_kernel", "tcgen05": "spg_gemm_tc_kernel",
                   "tcgen05-fused": "spg_mlp3_fused_kernel", "simt": "spg_layer_simt_kernel"}
 
 

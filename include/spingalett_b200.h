@@ -406,6 +406,7 @@ SPINGALETT_API void spingalett_profile_read(NeuralNetwork *net, double *kernel_m
 
 /* Number of kernels this library has launched in the calling process, and the
  * name of the compute path the last batched/forward call took ("gemv",
+ * "rows" -- nets of few weights on up to eight rows --,
  * "istream" -- integer files through the 8-bit integer tensor path --, "wstream",
  * "tcgen05", "tcgen05-fused" -- the three-layer net in one launch --, "simt").  For benchmarks and tests. */
 SPINGALETT_API uint64_t spingalett_kernel_launches(void);

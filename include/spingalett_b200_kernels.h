@@ -97,6 +97,19 @@ SPGK_API int spgk_stream_wait_event(void *stream, void *event);
 SPGK_API int spgk_layer_simt(const spgk_layer *L, const float *x, uint32_t ldx,
                              float *y, uint32_t ldy, uint32_t N, void *stream);
 
+/* ---- a small net on one to eight rows -------------------------------------
+ * Every layer of the net (any precision, width and alignment), one chained launch each, sums of four in fp32 and their sum in 64 bits; the row softmax of a
+ * layer that has one is applied (a hidden one too).  ys[l]: fp32 [N][layers[l].out].  Fast for nets that fit L2 many times over.
+ * Does forward()'s layer loop, reference Network.c:218-247. */
+#define SPGK_ROWS_MAX_BATCH 8u
+SPGK_API int spgk_rows_forward(const spgk_layer *layers, uint32_t count, const float *x, uint32_t ldx, float *const *ys, uint32_t N,
+                               void *stream);
+/* One sample the same way, from and to page-locked host memory: host and dev hold the input and then every layer's outputs, one behind the
+ * other; the input is read from host, the outputs are written to dev and to host (there once the stream has been waited for).
+ * SPGK_E_UNSUPPORTED, and nothing launched, for a softmax of more than 128 outputs. */
+#define SPGK_ROWS_MAX_LAYERS 64u
+SPGK_API int spgk_rows_sample(const spgk_layer *layers, uint32_t count, float *host, float *dev, void *stream);
+
 /* ---- softmax over rows, in place ----------------------------------------
  * Reference Activation.c:5-21 per row: max from -FLT_MAX, expf(x-max), scale
  * by 1/sum only if sum > 0.  width <= 65535. */

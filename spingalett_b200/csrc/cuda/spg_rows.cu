@@ -1,0 +1,253 @@
+// spg_rows.cu -- one to eight rows through a small net, any precision, any width, any alignment.
+//
+//   y[n][j] = act(bias[j] + w_scale * sum_k q[j][k] * x[n][k])
+//
+// A net of a few megabytes lives in L2 and a forward pass of a sample is a chain of latencies: what a layer costs is a launch,
+// the way to its input and a sum.  A warp takes an output.  Its weights depend on nothing, so the first 1024 of its row are in
+// registers, decoded, before the layer before it has ended (programmatic dependent launch); then come the input (8 neighbouring
+// values a lane, all loads of a round in flight), the products, four of them added in fp32 and the fours in 64 bits, and a shuffle
+// tree.  (Every product in 64 bits: as accurate as the last rounding allows, and 2 to 4 us slower from six rows on, a conversion
+// runs at 14 a cycle and SM.)
+//
+// What bounds it: 3 us a layer of launch, two L2 latencies and the tree; beyond four rows the loads of the inputs.  Before (the
+// weight-streaming GEMV, made to keep HBM busy, or the general kernel where rows are no multiple of 16 bytes) and now, us a call:
+// 784-512-1000-10 at one row fp32 29.8 -> 10, INT8 45 -> 10, INT4 24.7 -> 9.4; at eight rows fp32 90 -> 12, INT4 115 -> 10;
+// 301-777-333-129-37 fp32 at one row 22.6 -> 12.4, at eight 103 -> 18.5; 1024-1024-1024-1024-16 BF16 35 -> 12 and 117 -> 23.
+// forward() of one sample 57 -> 36 (28 of them launches, device time and the wait).  Error against 64 bits 5e-8 to 2e-7 (before:
+// 1e-7 to 5e-6).  An input that travels as a parameter of the first launch instead of through the fetch kernel: level.
+//
+// Reference: forward's layer step, Src/Spingalett.Network.c:218-247; decode of Src/Spingalett.Serialize.c:222-294.
+#include "spg_common.cuh"
+#include <type_traits>
+
+namespace {
+
+constexpr uint32_t GROUP = 8, ROUNDS = 4, SPAN = 32 * GROUP * ROUNDS;      // neighbours a lane takes, groups a lane has in flight, elements a warp has
+constexpr uint32_t LAST_WARPS = 32, LAST_MAX = 128;                        // the layer whose row softmax is finished in the CTA
+
+struct RowsParams {
+    const void *w; const float *bias; float scale; uint32_t in, out; int act;
+    const float *x; uint32_t ldx; float *y; uint32_t ldy; uint32_t N;
+    float *copy;                           // a second place for the outputs of row 0 (page-locked host memory), or null
+    uint32_t vec_w, vec_x;                 // groups of eight weights / inputs lie on their own alignment
+};
+
+// the weights e .. e + 7 of the matrix, as stored
+template <int PREC> __device__ __forceinline__ void decode8(const void *w, uint64_t e, float (&q)[8])
+{
+    if constexpr (PREC == SPG_P_F32) {
+        const float4 *p = reinterpret_cast<const float4 *>(reinterpret_cast<const float *>(w) + e);
+        const float4 a = __ldg(p), b = __ldg(p + 1);
+        q[0] = a.x; q[1] = a.y; q[2] = a.z; q[3] = a.w; q[4] = b.x; q[5] = b.y; q[6] = b.z; q[7] = b.w;
+    } else if constexpr (PREC == SPG_P_F16 || PREC == SPG_P_BF16) {
+        const uint4 v = __ldg(reinterpret_cast<const uint4 *>(reinterpret_cast<const uint16_t *>(w) + e));
+        const uint32_t u[4] = { v.x, v.y, v.z, v.w };
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+            const uint32_t h = u[i >> 1] >> ((i & 1) * 16) & 0xFFFFu;
+            q[i] = PREC == SPG_P_F16 ? __half2float(__ushort_as_half((unsigned short)h)) : __uint_as_float(h << 16);
+        }
+    } else if constexpr (PREC == SPG_P_I8) {
+        const uint2 v = __ldg(reinterpret_cast<const uint2 *>(reinterpret_cast<const int8_t *>(w) + e));
+#pragma unroll
+        for (int i = 0; i < 8; i++) q[i] = (float)((int)((i < 4 ? v.x : v.y) << (24 - 8 * (i & 3))) >> 24);
+    } else if constexpr (PREC == SPG_P_I4) {
+        const uint32_t v = __ldg(reinterpret_cast<const uint32_t *>(reinterpret_cast<const uint8_t *>(w) + (e >> 1)));
+#pragma unroll
+        for (int i = 0; i < 8; i++) q[i] = (float)((int)(v << (28 - 4 * i)) >> 28);
+    } else {
+        const uint32_t v = __ldg(reinterpret_cast<const uint16_t *>(reinterpret_cast<const uint8_t *>(w) + (e >> 2)));
+#pragma unroll
+        for (int i = 0; i < 8; i++) q[i] = (float)((int)(v << (30 - 2 * i)) >> 30);
+    }
+}
+
+// Output j for rows n0 .. n0 + NB - 1 (rows from N on read as the last one): the sums, in every lane.  `wait`: the input is what
+// the launch before this one writes, and nobody has waited for it yet.
+template <int PREC, int NB> __device__ __forceinline__ void dot(const RowsParams &p, uint32_t j, uint32_t n0, bool wait, uint32_t lane, double (&sum)[NB])
+{
+    const uint64_t row = (uint64_t)j * p.in;
+    double acc[NB][2];
+#pragma unroll
+    for (int b = 0; b < NB; b++) acc[b][0] = acc[b][1] = 0.0;
+#pragma unroll 1
+    for (uint32_t k0 = 0; k0 < p.in; k0 += SPAN) {
+        float q[ROUNDS][GROUP];
+#pragma unroll
+        for (uint32_t u = 0; u < ROUNDS; u++) {
+            const uint32_t k = k0 + (u * 32 + lane) * GROUP;
+            if (p.vec_w && k < p.in) decode8<PREC>(p.w, row + k, q[u]);        // (then `in` is a multiple of eight)
+            else {
+#pragma unroll
+                for (uint32_t i = 0; i < GROUP; i++) q[u][i] = k + i < p.in ? spg_decode_elem(p.w, row + k + i, PREC) : 0.0f;
+            }
+        }
+        if (wait) { spg_grid_wait(); wait = false; }
+#pragma unroll
+        for (uint32_t u = 0; u < ROUNDS; u++) {
+            const uint32_t k = k0 + (u * 32 + lane) * GROUP;
+            if (k0 + u * 32 * GROUP >= p.in) break;                             // (the same for the whole warp)
+#pragma unroll
+            for (int b = 0; b < NB; b++) {
+                const float *x = p.x + (uint64_t)min(n0 + b, p.N - 1) * p.ldx + k;
+                float v[GROUP];
+                if (p.vec_x && k + GROUP <= p.in) {
+                    const float4 lo = *reinterpret_cast<const float4 *>(x), hi = *reinterpret_cast<const float4 *>(x + 4);
+                    v[0] = lo.x; v[1] = lo.y; v[2] = lo.z; v[3] = lo.w; v[4] = hi.x; v[5] = hi.y; v[6] = hi.z; v[7] = hi.w;
+                } else {
+#pragma unroll
+                    for (uint32_t i = 0; i < GROUP; i++) v[i] = k + i < p.in ? x[i] : 0.0f;
+                }
+#pragma unroll
+                for (uint32_t h = 0; h < 2; h++) {
+                    float four = q[u][4 * h] * v[4 * h];
+#pragma unroll
+                    for (uint32_t i = 4 * h + 1; i < 4 * h + 4; i++) four = fmaf(q[u][i], v[i], four);
+                    acc[b][h] += (double)four;
+                }
+            }
+        }
+    }
+#pragma unroll
+    for (int b = 0; b < NB; b++) {
+        sum[b] = acc[b][0] + acc[b][1];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) sum[b] += __shfl_xor_sync(0xffffffffu, sum[b], o);
+    }
+}
+
+__device__ __forceinline__ float value(const RowsParams &p, uint32_t j, double sum) { return (float)(sum * (double)p.scale + (double)p.bias[j]); }
+
+template <int PREC, int NB>
+__global__ void __launch_bounds__(256)
+spg_rows_kernel(const RowsParams p)
+{
+    const uint32_t lane = threadIdx.x & 31u, j = blockIdx.x * 8 + (threadIdx.x >> 5);
+    spg_grid_trigger();
+    if (j >= p.out) return;
+    double sum[NB];
+    const uint32_t n0 = blockIdx.y * NB;
+    dot<PREC, NB>(p, j, n0, true, lane, sum);
+    double mine = sum[0];
+#pragma unroll
+    for (int b = 1; b < NB; b++) if (lane == (uint32_t)b) mine = sum[b];
+    if (lane < NB && n0 + lane < p.N) {
+        const float y = spg_activate(value(p, j, mine), p.act);
+        p.y[(uint64_t)(n0 + lane) * p.ldy + j] = y;
+        if (p.copy && n0 + lane == 0) p.copy[j] = y;
+    }
+}
+
+// The last layer with a softmax of at most LAST_MAX outputs: one CTA a row, its warps take the outputs in turn; formulas of
+// spg_softmax_rows_kernel.
+template <int PREC>
+__global__ void __launch_bounds__(32 * LAST_WARPS)
+spg_rows_softmax_kernel(const RowsParams p)
+{
+    __shared__ float z[LAST_MAX];
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, n = blockIdx.x;
+    spg_grid_trigger();
+    for (uint32_t j = warp; j < p.out; j += LAST_WARPS) {
+        double sum[1];
+        dot<PREC, 1>(p, j, n, j == warp, lane, sum);
+        if (lane == 0) z[j] = value(p, j, sum[0]);
+    }
+    __syncthreads();
+    if (warp) return;
+    spg_grid_wait();                       // (an output that no warp had: this row is written after the layer before has ended all the same)
+    float mx = -FLT_MAX, sum = 0.0f;
+    for (uint32_t j = lane; j < p.out; j += 32) if (z[j] > mx) mx = z[j];
+    mx = spg_warp_max(mx);
+    for (uint32_t j = lane; j < p.out; j += 32) { z[j] = expf(z[j] - mx); sum += z[j]; }
+    sum = spg_warp_sum(sum);
+    const float inv = sum > 0.0f ? 1.0f / sum : 1.0f;
+    for (uint32_t j = lane; j < p.out; j += 32) {
+        p.y[(uint64_t)n * p.ldy + j] = z[j] * inv;
+        if (p.copy && n == 0) p.copy[j] = z[j] * inv;
+    }
+}
+
+// a sample from page-locked host memory
+__global__ void __launch_bounds__(256)
+spg_rows_fetch_kernel(const float *src, float *dst, uint32_t count)
+{
+    const uint32_t i = blockIdx.x * 256 + threadIdx.x;
+    spg_grid_trigger();
+    const float v = i < count ? src[i] : 0.0f;
+    spg_grid_wait();                       // what is in dst may still be read
+    if (i < count) dst[i] = v;
+}
+
+template <int PREC> cudaError_t launch(const RowsParams &p, bool softmax, cudaStream_t s)
+{
+    if (softmax) return spg_launch_chained(spg_rows_softmax_kernel<PREC>, dim3(p.N), dim3(32 * LAST_WARPS), 0, s, p);
+    // one row of the batch a warp up to four rows, two beyond (weights decoded once for both): 784-512-1000-10 at 4 rows 9.7 against 11.5 us,
+    // at 6 rows 12.9 against 10.9
+    if (p.N <= 4) return spg_launch_chained(spg_rows_kernel<PREC, 1>, dim3((p.out + 7) / 8, p.N), dim3(256), 0, s, p);
+    return spg_launch_chained(spg_rows_kernel<PREC, 2>, dim3((p.out + 7) / 8, (p.N + 1) / 2), dim3(256), 0, s, p);
+}
+
+}  // namespace
+
+// calls f with the layer's precision as a constant
+template <typename F> static cudaError_t with_precision(int precision, F f)
+{
+    switch (precision) {
+        case SPG_P_F32:  return f(std::integral_constant<int, SPG_P_F32>());
+        case SPG_P_F16:  return f(std::integral_constant<int, SPG_P_F16>());
+        case SPG_P_BF16: return f(std::integral_constant<int, SPG_P_BF16>());
+        case SPG_P_I8:   return f(std::integral_constant<int, SPG_P_I8>());
+        case SPG_P_I4:   return f(std::integral_constant<int, SPG_P_I4>());
+        default:         return f(std::integral_constant<int, SPG_P_I2>());
+    }
+}
+
+static int rows_chain(const spgk_layer *layers, uint32_t count, const float *x, uint32_t ldx, float *const *ys, float *const *copies, uint32_t N, void *stream)
+{
+    for (uint32_t l = 0; l < count; l++) {
+        const spgk_layer *L = &layers[l];
+        const bool softmax = L->act == SPG_ACT_SOFTMAX, fused = softmax && L->out <= LAST_MAX;
+        RowsParams p;
+        p.w = L->w; p.bias = L->bias; p.scale = L->w_scale; p.in = L->in; p.out = L->out; p.act = softmax ? SPG_ACT_NONE : L->act;
+        p.x = x; p.ldx = ldx; p.y = ys[l]; p.ldy = L->out; p.N = N; p.copy = copies ? copies[l] : nullptr;
+        p.vec_w = (L->in % 8 == 0 && ((uintptr_t)L->w & 15u) == 0) ? 1u : 0u;
+        p.vec_x = (((uintptr_t)x | ((uintptr_t)ldx * 4)) & 15u) == 0 ? 1u : 0u;
+        SPGK_CUDA(with_precision(L->precision, [&](auto prec) { return launch<prec.value>(p, fused, (cudaStream_t)stream); }));
+        int rc = spgk_check_launch("spg_rows_kernel");
+        if (rc) return rc;
+        if (softmax && !fused && (rc = spgk_softmax_rows(ys[l], L->out, N, L->out, stream))) return rc;
+        x = ys[l]; ldx = L->out;
+    }
+    return SPGK_OK;
+}
+
+static bool layers_ok(const spgk_layer *layers, uint32_t count)
+{
+    for (uint32_t l = 0; l < count; l++) {
+        const spgk_layer *L = &layers[l];
+        if (!L->w || !L->bias || L->in == 0 || L->out == 0 || (unsigned)L->precision >= SPG_P_COUNT) return false;
+    }
+    return true;
+}
+
+extern "C" int spgk_rows_forward(const spgk_layer *layers, uint32_t count, const float *x, uint32_t ldx, float *const *ys, uint32_t N, void *stream)
+{
+    if (!layers || !x || !ys || N == 0 || N > SPGK_ROWS_MAX_BATCH || !layers_ok(layers, count)) { spgk_set_error("spgk_rows_forward", "bad argument"); return SPGK_E_ARG; }
+    for (uint32_t l = 0; l < count; l++) if (!ys[l]) { spgk_set_error("spgk_rows_forward", "bad argument"); return SPGK_E_ARG; }
+    return rows_chain(layers, count, x, ldx, ys, nullptr, N, stream);
+}
+
+extern "C" int spgk_rows_sample(const spgk_layer *layers, uint32_t count, float *host, float *dev, void *stream)
+{
+    if (!layers || !host || !dev || count == 0 || count > SPGK_ROWS_MAX_LAYERS || !layers_ok(layers, count)) { spgk_set_error("spgk_rows_sample", "bad argument"); return SPGK_E_ARG; }
+    float *ys[SPGK_ROWS_MAX_LAYERS], *copies[SPGK_ROWS_MAX_LAYERS];
+    uint64_t at = layers[0].in;
+    for (uint32_t l = 0; l < count; l++) {
+        if (layers[l].act == SPG_ACT_SOFTMAX && layers[l].out > LAST_MAX) return SPGK_E_UNSUPPORTED;
+        ys[l] = dev + at; copies[l] = host + at;
+        at += layers[l].out;
+    }
+    SPGK_CUDA(spg_launch_chained(spg_rows_fetch_kernel, dim3((layers[0].in + 255) / 256), dim3(256), 0, (cudaStream_t)stream, host, dev, layers[0].in));
+    const int rc = spgk_check_launch("spg_rows_fetch_kernel");
+    return rc ? rc : rows_chain(layers, count, dev, layers[0].in, ys, copies, 1, stream);
+}

@@ -403,16 +403,42 @@ static bool all_wstream(const spg_net *n, uint32_t N)
     return true;
 }
 
+/* Up to eight rows of a net of few weights go warp by warp from L2, whatever their precision, widths and alignment.  The lines lie where the
+ * curves cross (us a call, this kernel / what served before): 0.9 million weights 10 / 25 to 45 at one row, 12 / 90 to 162 at eight; 7.3
+ * million INT8 weights 18.6 / 20.6 at one row, 35 / 43 at six; 8.0 million BF16 ones in rows of odd lengths 26 / 27 and 76 / 95; 25
+ * million INT2 weights 148 / 49 at six.  (At seven and eight rows forward_batch asks the integer streaming kernel first.) */
+#define SPG_ROWS_MAX_WEIGHTS ((uint64_t)8 << 20)
+
+static bool few_weights(const spg_net *n)
+{
+    uint64_t count = 0;
+    for (uint32_t l = 0; l < n->dev_layers; l++) count += (uint64_t)n->klayers[l].in * n->klayers[l].out;
+    return count <= SPG_ROWS_MAX_WEIGHTS;
+}
+
 /* Small / medium batches (fp32 activations between layers; every layer streams its packed weights once).
- * Per layer, in order of preference: the weight-streaming tcgen05 kernel, the mma.sync GEMV (<= 8 rows),
- * the general SIMT kernel.  d_x == NULL means the caller already placed the input rows in slot 0 of the
+ * Nets of few weights on up to 8 rows: spg_rows.cu.  Otherwise per layer, in order of preference: the weight-streaming
+ * tcgen05 kernel, the mma.sync GEMV (<= 8 rows), the general SIMT kernel.  d_x == NULL means the caller already placed the input rows in slot 0 of the
  * workspace (after a reservation-only call, see forward()). */
 int spg_dev_forward_small(spg_net *n, const float *d_x, uint32_t ldx, uint32_t N, float **d_last, float *d_final)
 {
     NeuralNetwork *p = &n->pub;
-    int rc = small_reserve(n, N);
+    const bool rows = N <= SPGK_ROWS_MAX_BATCH && few_weights(n);
+    int rc = rows ? activations_reserve(n, N) : small_reserve(n, N);
     if (rc) return rc;
     if (!d_last) return SPINGALETT_OK;          /* reservation only */
+    if (rows) {
+        float *ys[n->dev_layers];
+        for (uint32_t l = 0; l < n->dev_layers; l++)
+            ys[l] = (d_final && l + 1 == n->dev_layers) ? d_final : n->d_small + (size_t)N * p->neuron_offsets[l + 1];
+        prof_mark(n);
+        rc = spg_map_kernel_error(spgk_rows_forward(n->klayers, n->dev_layers, d_x ? d_x : n->d_small, d_x ? ldx : p->topology[0], ys, N, n->stream), "layers (small net)");
+        prof_mark(n);
+        if (rc) return rc;
+        spg_note_path("rows");
+        *d_last = ys[n->dev_layers - 1];
+        return SPINGALETT_OK;
+    }
     const float *x = d_x ? d_x : n->d_small;
     uint32_t xld = d_x ? ldx : p->topology[0];
     const char *path = NULL;
@@ -472,6 +498,27 @@ int spg_dev_forward_small(spg_net *n, const float *d_x, uint32_t ldx, uint32_t N
     }
     spg_note_path(path ? path : "none");
     *d_last = d_final ? d_final : n->d_small + (size_t)N * p->neuron_offsets[p->layers - 1];
+    return SPINGALETT_OK;
+}
+
+/* One sample of a net of few weights, from h_io (page-locked: the input, then room for every layer's outputs) and back into it, without a
+ * copy on either side: *taken says whether anything was launched. */
+int spg_dev_forward_sample(spg_net *n, float *h_io, bool *taken)
+{
+    *taken = false;
+    if (!few_weights(n) || n->dev_layers > SPGK_ROWS_MAX_LAYERS) return SPINGALETT_OK;
+    int rc = activations_reserve(n, 1);
+    if (rc) return rc;
+    prof_mark(n);
+    rc = spgk_rows_sample(n->klayers, n->dev_layers, h_io, n->d_small, n->stream);
+    prof_mark(n);
+    if (rc == SPGK_E_UNSUPPORTED) {
+        if (n->prof_used >= 2) n->prof_used -= 2;          /* nothing was launched between the two marks */
+        return SPINGALETT_OK;
+    }
+    if ((rc = spg_map_kernel_error(rc, "forward (small net)"))) return rc;
+    spg_note_path("rows");
+    *taken = true;
     return SPINGALETT_OK;
 }
 
@@ -1057,7 +1104,7 @@ static float *forward_batch_on(spg_net *n, ForwardBatchArgs a)
     }
 
     /* Integer files take the 8-bit integer streaming kernel from a few rows on, when it takes every layer.  Of what is left, up
-     * to 8 rows go layer by layer (GEMV first), up to 512 rows in groups of at most 128 through the 16-bit streaming kernel when
+     * to 8 rows go through spg_dev_forward_small (nets of few weights warp by warp, others GEMV first), up to 512 rows in groups of at most 128 through the 16-bit streaming kernel when
      * it takes every layer, each group streaming the packed weights once; everything else is the large-batch GEMM chain.
      *
      * Measured, against the path that served before: large INT4 net 126 us against 204 (GEMV) at 8 rows, 188 against 578

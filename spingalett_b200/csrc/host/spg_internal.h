@@ -130,6 +130,7 @@ SPG_HIDDEN int spg_dev_bind(spg_net *n);             /* the net's device, made c
 SPG_HIDDEN void spg_dev_release(spg_net *n);
 SPG_HIDDEN void spg_dev_invalidate(spg_net *n);
 SPG_HIDDEN int spg_dev_forward_small(spg_net *n, const float *d_x, uint32_t ldx, uint32_t N, float **d_last, float *d_final);
+SPG_HIDDEN int spg_dev_forward_sample(spg_net *n, float *h_io, bool *taken);
 SPG_HIDDEN int spg_dev_forward_large(spg_net *n, const float *d_x, uint32_t N, float *d_out);
 SPG_HIDDEN int spg_map_kernel_error(int rc, const char *where);
 /* train.c */

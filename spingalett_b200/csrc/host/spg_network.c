@@ -251,13 +251,17 @@ float *forward_struct_arguments(ForwardArgs args)
         pn->h_stage = p; pn->h_stage_bytes = need;
     }
     memcpy(pn->h_stage, args.input, (size_t)n->topology[0] * sizeof(float));
-    /* the workspace holds every layer's activations; slot 0 is the input */
-    if (spg_dev_forward_small(pn, NULL, 0, 1, NULL, NULL) != SPINGALETT_OK) return NULL;      /* reserve */
-    if (spg_map_kernel_error(spgk_memcpy_h2d(pn->d_small, pn->h_stage, (size_t)n->topology[0] * sizeof(float), pn->stream),
-                             "forward: input copy")) return NULL;
-    float *d_last = NULL;
-    if (spg_dev_forward_small(pn, NULL, 0, 1, &d_last, NULL) != SPINGALETT_OK) return NULL;
-    if (spg_map_kernel_error(spgk_memcpy_d2h(pn->h_stage, pn->d_small, need, pn->stream), "forward: copy back")) return NULL;
+    bool taken;
+    if (spg_dev_forward_sample(pn, pn->h_stage, &taken) != SPINGALETT_OK) return NULL;
+    if (!taken) {
+        /* the workspace holds every layer's activations; slot 0 is the input */
+        if (spg_dev_forward_small(pn, NULL, 0, 1, NULL, NULL) != SPINGALETT_OK) return NULL;      /* reserve */
+        if (spg_map_kernel_error(spgk_memcpy_h2d(pn->d_small, pn->h_stage, (size_t)n->topology[0] * sizeof(float), pn->stream),
+                                 "forward: input copy")) return NULL;
+        float *d_last = NULL;
+        if (spg_dev_forward_small(pn, NULL, 0, 1, &d_last, NULL) != SPINGALETT_OK) return NULL;
+        if (spg_map_kernel_error(spgk_memcpy_d2h(pn->h_stage, pn->d_small, need, pn->stream), "forward: copy back")) return NULL;
+    }
     if (spg_map_kernel_error(spgk_stream_sync(pn->stream), "forward: sync")) return NULL;
     memcpy(n->neurons, pn->h_stage, need);
     return n->neurons + n->neuron_offsets[n->layers - 1];
