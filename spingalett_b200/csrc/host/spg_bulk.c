@@ -8,6 +8,7 @@
 #include <stdatomic.h>
 #include <stdlib.h>
 #include <string.h>
+#include <sys/mman.h>
 #include <unistd.h>
 #if defined(__x86_64__)
 #include <immintrin.h>
@@ -99,3 +100,27 @@ void spg_stage_copy(void *dst, const void *src, size_t bytes)
     if (bytes < SPG_STAGE_THREADED) memcpy(dst, src, bytes);
     else spg_bulk(copy_slice, &c, bytes, 4096, (size_t)1 << 20);
 }
+
+/* Long fresh memory in pages of 2 MB where the system has them: it is filled once, and a page fault for every 4 KB of 100 MB takes as long
+ * as filling it. */
+void spg_large_pages(void *p, size_t bytes)
+{
+    const uintptr_t page = (uintptr_t)2 << 20, lo = ((uintptr_t)p + page - 1) & ~(page - 1), hi = ((uintptr_t)p + bytes) & ~(page - 1);
+    if (p && hi > lo) madvise((void *)lo, hi - lo, MADV_HUGEPAGE);
+}
+
+/* into memory that the host reads next */
+static void plain_slice(void *ctx, size_t lo, size_t hi)
+{
+    const copy_ctx *c = ctx;
+    memcpy(c->dst + lo, c->src + lo, hi - lo);
+}
+
+void spg_bulk_copy(void *dst, const void *src, size_t bytes)
+{
+    copy_ctx c = { dst, src };
+    spg_bulk(plain_slice, &c, bytes, 4096, (size_t)1 << 20);
+}
+
+static void zero_slice(void *ctx, size_t lo, size_t hi) { memset((char *)ctx + lo, 0, hi - lo); }
+void spg_bulk_zero(void *dst, size_t bytes) { spg_bulk(zero_slice, dst, bytes, 4096, (size_t)1 << 20); }

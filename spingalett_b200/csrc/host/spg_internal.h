@@ -115,6 +115,21 @@ typedef void (*spg_slice_fn)(void *ctx, size_t lo, size_t hi);
 SPG_HIDDEN void spg_bulk(spg_slice_fn fn, void *ctx, size_t n, size_t grain, size_t least);
 #define SPG_STAGE_THREADED ((size_t)4 << 20)         /* bytes from which spg_stage_copy takes several threads */
 SPG_HIDDEN void spg_stage_copy(void *dst, const void *src, size_t bytes);
+SPG_HIDDEN void spg_bulk_copy(void *dst, const void *src, size_t bytes);
+SPG_HIDDEN void spg_bulk_zero(void *dst, size_t bytes);
+SPG_HIDDEN void spg_large_pages(void *p, size_t bytes);
+/* stage.c */
+#define SPG_STAGE_PIECE ((size_t)8 << 20)
+typedef struct { void *piece[2], *landed[2], *stream; bool busy[2]; int turn; } spg_stager;      /* two page-locked pieces on a stream */
+typedef bool (*spg_sink_fn)(void *ctx, size_t at, const void *piece, size_t n);
+SPG_HIDDEN int spg_stager_open(spg_stager *s, void *stream);
+SPG_HIDDEN void spg_stager_close(spg_stager *s);                                   /* waits for what is under way */
+SPG_HIDDEN int spg_stager_settle(spg_stager *s);
+SPG_HIDDEN int spg_stager_up(spg_stager *s, void *dev, const void *src, size_t bytes);
+typedef struct { const void *dev; size_t bytes; void *ctx; } spg_segment;                       /* device memory and where it goes */
+SPG_HIDDEN int spg_stager_down(spg_stager *s, spg_sink_fn sink, const spg_segment *seg, int count);
+SPG_HIDDEN bool spg_sink_array(void *ctx, size_t at, const void *piece, size_t n);
+SPG_HIDDEN void spg_stage_users(int change);
 /* codec.c */
 SPG_HIDDEN size_t spg_array_bytes(uint64_t count, PrecisionMode p);
 SPG_HIDDEN void spg_decode_array(const uint8_t *src, uint64_t count, PrecisionMode p, float *dst);

@@ -51,6 +51,7 @@ bool spg_net_expect(spg_net *pn, uint64_t weights, uint64_t biases)
         n->weights = n->biases = NULL;
         return false;
     }
+    spg_large_pages(n->weights, (size_t)weights * sizeof(float));
     pn->expect_w = weights; pn->expect_b = biases;
     return true;
 }
@@ -87,6 +88,7 @@ NeuralNetwork *new_spingalett_struct_arguments(NeuralNetworkArgs args)
     n->pub.loss_func = args.loss_func;
     n->store_precision = PRECISION_FLOAT32;
     n->device = -1;
+    spg_stage_users(1);
     return &n->pub;
 }
 
@@ -303,5 +305,6 @@ void free_network(NeuralNetwork *n)
     free(n->topology); free(n->act_func);
     pn->magic = 0;
     free(pn);
+    spg_stage_users(-1);
     spg_log(LOG_DEBUG, "Memory freed.");
 }

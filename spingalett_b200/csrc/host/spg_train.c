@@ -42,6 +42,10 @@ typedef struct {
     size_t cap[12];                          /* bytes held by each of the buffers above, in declaration order */
     uint64_t np;                             /* parameters the flat buffers were sized for */
     void *stream;                            /* a stream of the library's own for nets that sit on the legacy default stream */
+    float *h_words;                          /* page-locked: status words (page-locking a kilobyte takes up to 2 ms, giving it back 0.6) */
+    uint32_t *h_order[2];                    /* page-locked: the shuffled orders of this epoch and the next, on their way to `idx` */
+    void *order_ev[2];
+    size_t order_cap;                        /* samples the orders have room for */
 } train_state;
 
 /* process-wide communicator for the gradient exchange */
@@ -112,7 +116,37 @@ static void state_free(train_state *t)
                      t->idx, t->words };
     for (size_t i = 0; i < sizeof bufs / sizeof bufs[0]; i++) spgk_free(bufs[i]);
     spgk_stream_destroy(t->stream);
+    spgk_host_free(t->h_words);
+    for (int i = 0; i < 2; i++) {
+        spgk_host_free(t->h_order[i]);
+        if (t->order_ev[i]) spgk_event_destroy(t->order_ev[i]);
+    }
     free(t);
+}
+
+/* room for the shuffled orders of two epochs */
+static int orders_reserve(train_state *t, uint32_t samples)
+{
+    for (int i = 0; i < 2; i++) {
+        int rc;
+        if (t->order_cap < samples) { spgk_host_free(t->h_order[i]); t->h_order[i] = NULL; }
+        void *h = NULL;
+        if (!t->h_order[i] && (rc = spg_map_kernel_error(spgk_host_alloc(&h, (size_t)samples * 4), "train: shuffle order"))) { t->order_cap = 0; return rc; }
+        if (h) t->h_order[i] = h;
+        if (!t->order_ev[i] && (rc = spg_map_kernel_error(spgk_event_create(&t->order_ev[i]), "train: shuffle order"))) return rc;
+    }
+    if (t->order_cap < samples) t->order_cap = samples;
+    return SPINGALETT_OK;
+}
+
+/* The caller's arrays to the device: long pageable ones through page-locked pieces (opened when the first one comes), others by a plain copy */
+static int train_upload(spg_stager *stage, bool *staged, void *dev, const void *src, size_t bytes, void *st)
+{
+    if (bytes >= SPG_STAGE_THREADED && spgk_is_device_pointer(src) != 1 && spgk_is_pinned_host_pointer(src) != 1) {
+        if (!*staged) *staged = spg_stager_open(stage, st) == SPGK_OK;
+        if (*staged) return spg_stager_up(stage, dev, src, bytes);
+    }
+    return spgk_memcpy_h2d(dev, src, bytes, st);
 }
 
 void spg_train_release(spg_net *n)
@@ -226,8 +260,8 @@ void train_struct_arguments(TrainArgs a)
     spg_net *n = spg_priv(p);
     if (spg_net_ensure_train_arrays(n) != SPINGALETT_OK) return;
     if (a.reset_optimizer) {
-        memset(p->opt_m_weights, 0, p->total_weights * sizeof(float));
-        memset(p->opt_v_weights, 0, p->total_weights * sizeof(float));
+        spg_bulk_zero(p->opt_m_weights, p->total_weights * sizeof(float));
+        spg_bulk_zero(p->opt_v_weights, p->total_weights * sizeof(float));
         memset(p->opt_m_biases, 0, p->total_biases * sizeof(float));
         memset(p->opt_v_biases, 0, p->total_biases * sizeof(float));
         p->time_step = 0;
@@ -265,7 +299,8 @@ void train_struct_arguments(TrainArgs a)
     }
     void *st = n->stream;
     uint32_t *order = NULL;
-    float *h_pinned = NULL;
+    spg_stager stage;
+    bool staged = false;                     /* `stage` is open */
     bool failed = true;
     void *graph_exec = NULL;                 /* the step as an executable CUDA graph, once captured */
     bool graph_failed = false, in_capture = false;
@@ -281,28 +316,34 @@ void train_struct_arguments(TrainArgs a)
         if (state_reserve(t, 8, (void **)&t->batch_x, (size_t)batch * in0 * 4, "train: batch inputs") ||
             state_reserve(t, 9, (void **)&t->batch_t, (size_t)batch * outw * 4, "train: batch targets")) goto fail;
         if (state_reserve(t, 10, (void **)&t->idx, (size_t)a.sample_count * 4, "train: shuffle order")) goto fail;
+        if (orders_reserve(t, a.sample_count)) goto fail;
         order = malloc((size_t)a.sample_count * sizeof *order);
         if (!order) { spg_set_error(SPINGALETT_ERR_ALLOC, "Mini-batch allocation failed"); goto fail; }
         for (uint32_t i = 0; i < a.sample_count; i++) order[i] = i;
     }
     float *d_loss = t->words, *d_sumsq = t->words + 2, *d_agree = t->words + 8;
     int *d_flag = (int *)(t->words + 1);
-    DEV(spgk_host_alloc((void **)&h_pinned, 1024), "train: pinned words");
+    if (!t->h_words) {
+        void *h = NULL;
+        DEV(spgk_host_alloc(&h, 1024), "train: pinned words");
+        t->h_words = h;
+    }
+    float *const h_pinned = t->h_words;
 
     /* the host arrays are the truth between calls (callers may edit them): upload them every time */
-    DEV(spgk_memcpy_h2d(t->params, p->weights, tw * 4, st), "train: upload weights");
+    DEV(train_upload(&stage, &staged, t->params, p->weights, tw * 4, st), "train: upload weights");
     DEV(spgk_memcpy_h2d(t->params + tw, p->biases, tb * 4, st), "train: upload biases");
     if (a.reset_optimizer) {                                 /* cleared above: nothing to copy */
         DEV(spgk_memset(t->m, 0, np * 4, st), "train: clear m");
         DEV(spgk_memset(t->v, 0, np * 4, st), "train: clear v");
     } else {
-        DEV(spgk_memcpy_h2d(t->m, p->opt_m_weights, tw * 4, st), "train: upload m");
+        DEV(train_upload(&stage, &staged, t->m, p->opt_m_weights, tw * 4, st), "train: upload m");
         DEV(spgk_memcpy_h2d(t->m + tw, p->opt_m_biases, tb * 4, st), "train: upload m");
-        DEV(spgk_memcpy_h2d(t->v, p->opt_v_weights, tw * 4, st), "train: upload v");
+        DEV(train_upload(&stage, &staged, t->v, p->opt_v_weights, tw * 4, st), "train: upload v");
         DEV(spgk_memcpy_h2d(t->v + tw, p->opt_v_biases, tb * 4, st), "train: upload v");
     }
-    DEV(spgk_memcpy_h2d(t->data_x, a.inputs, (size_t)a.sample_count * in0 * 4, st), "train: upload inputs");
-    DEV(spgk_memcpy_h2d(t->data_t, a.targets, (size_t)a.sample_count * outw * 4, st), "train: upload targets");
+    DEV(train_upload(&stage, &staged, t->data_x, a.inputs, (size_t)a.sample_count * in0 * 4, st), "train: upload inputs");
+    DEV(train_upload(&stage, &staged, t->data_t, a.targets, (size_t)a.sample_count * outw * 4, st), "train: upload targets");
     DEV(spgk_memset(t->grads, 0, np * 4, st), "train: clear gradients");
 
     if (s_world > 1) {
@@ -396,9 +437,13 @@ void train_struct_arguments(TrainArgs a)
         if (need_loss || graph_mode) DEV(spgk_memset(d_loss, 0, 4, st), "train: clear loss");
         float *const loss_ptr = (need_loss || graph_mode) ? d_loss : NULL;      /* a replayed step always adds to the loss word */
         if (mini) {
+            /* the order goes out from one of two page-locked buffers, so that this thread need not wait for the epoch before */
+            const int b = (int)(epoch & 1);
             spg_shuffle(order, a.sample_count);
-            DEV(spgk_memcpy_h2d(t->idx, order, (size_t)a.sample_count * 4, st), "train: upload order");
-            DEV(train_sync(st), "train: order sync");        /* `order` is reshuffled next epoch */
+            if (epoch > 2) DEV(s_world > 1 ? train_sync(st) : spgk_event_sync(t->order_ev[b]), "train: order sync");
+            memcpy(t->h_order[b], order, (size_t)a.sample_count * 4);
+            DEV(spgk_memcpy_h2d(t->idx, t->h_order[b], (size_t)a.sample_count * 4, st), "train: upload order");
+            DEV(spgk_event_record(t->order_ev[b], st), "train: upload order");
         }
         const uint32_t nb = (a.sample_count + batch - 1) / batch;
         for (uint32_t bi = 0; bi < nb; bi++) {
@@ -562,15 +607,18 @@ void train_struct_arguments(TrainArgs a)
     }
     if (fused_x) DEV(spgk_xchg_gather(s_xchg, st), "train: gather gradients and optimiser state");
     /* host mirrors of everything the reference leaves in the public struct */
-    DEV(spgk_memcpy_d2h(p->weights, P, tw * 4, st), "train: weights to host");
     DEV(spgk_memcpy_d2h(p->biases, P + tw, tb * 4, st), "train: biases to host");
-    DEV(spgk_memcpy_d2h(p->grad_weights, G, tw * 4, st), "train: gradients to host");
     DEV(spgk_memcpy_d2h(p->grad_biases, G + tw, tb * 4, st), "train: gradients to host");
-    DEV(spgk_memcpy_d2h(p->opt_m_weights, M, tw * 4, st), "train: m to host");
     DEV(spgk_memcpy_d2h(p->opt_m_biases, M + tw, tb * 4, st), "train: m to host");
-    DEV(spgk_memcpy_d2h(p->opt_v_weights, V, tw * 4, st), "train: v to host");
     DEV(spgk_memcpy_d2h(p->opt_v_biases, V + tw, tb * 4, st), "train: v to host");
     DEV(train_sync(st), "train: final sync");
+    const spg_segment back[4] = { { P, tw * 4, p->weights }, { G, tw * 4, p->grad_weights }, { M, tw * 4, p->opt_m_weights }, { V, tw * 4, p->opt_v_weights } };
+    if (tw * 16 >= SPG_STAGE_THREADED && !staged) staged = spg_stager_open(&stage, st) == SPGK_OK;
+    if (staged) DEV(spg_stager_down(&stage, spg_sink_array, back, 4), "train: arrays to host");
+    else {
+        for (int i = 0; i < 4; i++) DEV(spgk_memcpy_d2h(back[i].ctx, back[i].dev, back[i].bytes, st), "train: arrays to host");
+        DEV(train_sync(st), "train: final sync");
+    }
     if (fused_x) DEV(spgk_xchg_status(s_xchg, st), "train: gradient exchange");
     spg_log(LOG_INFO, "Training completed.");
     failed = false;
@@ -580,7 +628,7 @@ fail:
     spgk_graph_destroy(graph_exec);
     spgk_train_use_state(NULL);
     free(order);
-    spgk_host_free(h_pinned);
+    if (staged) spg_stager_close(&stage);
     n->live_params = n->live_m = n->live_v = NULL;
     if (failed) spg_train_release(n);          /* after an error nothing of the device state is trusted */
     if (failed && s_xchg) { spgk_xchg_destroy(s_xchg); s_xchg = NULL; }
