@@ -71,6 +71,7 @@ SPGK_API int spgk_memcpy_d2h(void *host, const void *dev, size_t bytes, void *st
 SPGK_API int spgk_memcpy_d2d(void *dst, const void *src, size_t bytes, void *stream);
 SPGK_API int spgk_memset(void *dev, int value, size_t bytes, void *stream);
 SPGK_API int spgk_stream_sync(void *stream);
+SPGK_API int spgk_stream_capturing(void *stream);             /* 1 while launches on it are being captured into a graph */
 /* 1 if ptr is device (or managed) memory, 0 if host, <0 on error */
 SPGK_API int spgk_is_device_pointer(const void *ptr);
 SPGK_API int spgk_is_pinned_host_pointer(const void *ptr);   /* 1: page-locked host memory, 0: pageable or unknown */
@@ -136,6 +137,8 @@ SPGK_API void spgk_set_margin_sink(float theta, uint32_t *idx, uint32_t *count);
 /* After spgk_set_output_rows(idx) the fp32 output of this thread's spgk_layer_gemm_tc calls is scattered: row r of the
  * result is written to row idx[r] of out32 (the counterpart of spgk_split16_rows).  NULL switches it off. */
 SPGK_API void spgk_set_output_rows(const uint32_t *rows_idx);
+/* *host = *count; *count = 0.  host: page-locked host memory, there once the stream has been waited for. */
+SPGK_API int spgk_count_take(uint32_t *count, uint32_t *host, void *stream);
 SPGK_API int spgk_margin_select(const float *probs, uint32_t ldp, uint32_t N, uint32_t width, float theta,
                                 uint32_t *idx, uint32_t *count, void *stream);
 /* max over rows of the change in the top-two log gap between a fast and an exact result (float bits in *max_bits,

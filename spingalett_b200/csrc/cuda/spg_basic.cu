@@ -116,6 +116,12 @@ int spgk_host_alloc(void **host, size_t bytes)
     return SPGK_OK;
 }
 int spgk_host_free(void *host) { if (host) SPGK_CUDA(cudaFreeHost(host)); return SPGK_OK; }
+int spgk_stream_capturing(void *stream)
+{
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing((cudaStream_t)stream, &st) != cudaSuccess) { cudaGetLastError(); return 0; }
+    return st != cudaStreamCaptureStatusNone;
+}
 int spgk_memcpy_h2d(void *dev, const void *host, size_t bytes, void *stream)
 {
     SPGK_CUDA(cudaMemcpyAsync(dev, host, bytes, cudaMemcpyHostToDevice, (cudaStream_t)stream));
@@ -333,6 +339,15 @@ spg_scatter_rows_kernel(const float *__restrict__ src, const uint32_t *__restric
     }
 }
 
+// a device-resident count to page-locked host memory, and back to zero
+__global__ void spg_count_take_kernel(uint32_t *count, uint32_t *host)
+{
+    spg_grid_trigger();
+    spg_grid_wait();
+    *host = *count;
+    *count = 0u;
+}
+
 // fp32 -> `parts` 16-bit planes (term p = round(x - sum of earlier terms)).
 template <typename T16>
 __device__ __forceinline__ T16 spg_to16(float v);
@@ -462,6 +477,13 @@ int spgk_scatter_rows(const float *src, const uint32_t *idx, float *dst, uint32_
     uint32_t blocks = (uint32_t)((total + 255) / 256 < 148ull * 8 ? (total + 255) / 256 : 148ull * 8);
     SPGK_CUDA(spg_launch_chained(spg_scatter_rows_kernel, dim3(blocks), dim3(256), 0, (cudaStream_t)stream, src, idx, dst, rows, width, ldd, spg_tls_rows_limit));
     return spgk_check_launch("spg_scatter_rows_kernel");
+}
+
+int spgk_count_take(uint32_t *count, uint32_t *host, void *stream)
+{
+    if (!count || !host) { spgk_set_error("spgk_count_take", "bad argument"); return SPGK_E_ARG; }
+    SPGK_CUDA(spg_launch_chained(spg_count_take_kernel, dim3(1), dim3(1), 0, (cudaStream_t)stream, count, host));
+    return spgk_check_launch("spg_count_take_kernel");
 }
 
 int spgk_split16(const float *x, uint32_t ldx, uint32_t N, uint32_t in, void *dst, uint32_t ld16,

@@ -542,7 +542,7 @@ spg_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
     // the warp index through a shuffle: provably warp-uniform, so the role code below keeps uniform values in uniform registers
     const uint32_t warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31u;
     const uint32_t abort_addr = smem_u32(const_cast<int *>(abort_flag));
-    const uint32_t tmem_cols = 2 * p.BN < 32 ? 32 : 2 * p.BN;       // power of two: BN in {16,32,64,128,256}
+    const uint32_t tmem_cols = 2 * p.BN <= 32 ? 32u : 1u << (32 - __clz(2 * p.BN - 1));      // a power of two for two accumulators: BN in {16,32,64,96,128,192,256}
 
     if (threadIdx.x == 0) {
         for (uint32_t s = 0; s < p.stages; s++) { mbar_init(full0 + 8 * s, 1); mbar_init(empty0 + 8 * s, 1); }
@@ -875,11 +875,18 @@ static int gemm_launch(const spgk_layer *L,
     GemmParams p{};
     p.M = N; p.N = L->out; p.K = L->in;
     p.BN = pick_bn(L->out);
-    // a device-resident row count usually means a small selection of a large batch: when the caller's estimate of
-    // it gives fewer tiles than SMs, narrower tiles spread the work (at the price of re-reading the rows more often)
-    if (spg_tls_rows_limit && spg_tls_rows_expected && !softmax_fused) {
+    uint32_t width = p.BN;
+    // a device-resident row count usually means a small selection of a large batch: of the widths down to 64, the one whose waves of tiles take
+    // the shortest for the caller's estimate of it (a wave takes as long as its width, and 32 columns more for what goes on beside the products)
+    if (spg_tls_rows_limit && spg_tls_rows_expected && !softmax_fused && p.BN > 64) {
         const uint32_t mt = (spg_tls_rows_expected + BM - 1) / BM;
-        while (p.BN > 64 && mt * ((L->out + p.BN - 1) / p.BN) < (uint32_t)sm_count) p.BN >>= 1;
+        uint32_t best = 0xFFFFFFFFu;
+        for (uint32_t bn : { 256u, 192u, 128u, 96u, 64u }) {
+            if (bn > p.BN) continue;
+            const uint32_t waves = (mt * ((L->out + bn - 1) / bn) + sm_count - 1) / sm_count, cost = waves * (bn + 32u);
+            if (cost < best) { best = cost; width = bn; }
+        }
+        p.BN = width;
     }
     p.kblocks = (L->in + BK - 1) / BK;
     // passes: hi*hi first, then the correction terms (lo*hi, hi*lo); lo*lo is below fp32 resolution
@@ -923,9 +930,9 @@ static int gemm_launch(const spgk_layer *L,
     rc = spg_gemm_map(&map_w, w16, w_type16, L->in, L->out, ldw, w_plane, w_parts, p.BN, 1);
     if (rc) return rc;
 
-    // 16-bit output through TMA stores when it is one plane and the tiles are wide enough for 64-column patches
+    // 16-bit output through TMA stores when it is one plane and a warp's columns are whole 64-column patches
     CUtensorMap map_o = map_a;
-    p.tma_store = (out16 && out_parts == 1 && p.BN >= 128 && !softmax_fused && !head) ? 1 : 0;
+    p.tma_store = (out16 && out_parts == 1 && p.BN % 128 == 0 && !softmax_fused && !head) ? 1 : 0;
     if (p.tma_store) {
         rc = spg_gemm_map(&map_o, out16, type16, ldo16, N, ldo16, o_plane, 1, 32, 1);
         if (rc) return rc;

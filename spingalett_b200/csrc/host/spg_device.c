@@ -843,18 +843,24 @@ int spg_dev_forward_large(spg_net *n, const float *d_x, uint32_t N, float *d_out
     if (N <= SPG_AUTO_EXACT_ROWS) return large_chain(n, d_x, N, d_out, true);
 
     int rc;
+    /* the list of rows stands behind a head of 256 bytes: [0] the number of rows, which every call leaves at zero, [8] the calibration's word */
+    const uint32_t *const list_before = n->d_rep_idx;
     if ((rc = reserve((void **)&n->d_rep_idx, &n->rep_idx_bytes, (size_t)N * 4 + 256, "repair index"))) return rc;
-    uint32_t *d_count = n->d_rep_idx + N;
+    uint32_t *const d_count = n->d_rep_idx, *const d_rows = n->d_rep_idx + 64;
+    if (n->d_rep_idx != list_before) n->count_clean = false;
+    /* (a call that is being captured runs later, and more than once, whatever happens in between: it clears the count itself) */
+    const bool captured = spgk_stream_capturing(n->stream) != 0, clean_before = n->count_clean;
+    if ((!clean_before || captured) && (rc = spg_map_kernel_error(spgk_memset(d_count, 0, 4, n->stream), "repair count clear"))) return rc;
+    n->count_clean = false;
     float theta = spingalett_get_auto_margin();
     if (theta <= 0.0f && n->auto_calibrated) theta = n->auto_theta;
     /* with the margin known in advance, the softmax epilogue of the last layer picks the rows out itself */
     const spgk_layer *Llast = &n->klayers[n->dev_layers - 1];
     const bool sink = theta > 0.0f && (fused || spgk_gemm_tc_softmax_fusable(Llast->out, N, 0));
-    if (sink && (rc = spg_map_kernel_error(spgk_memset(d_count, 0, 4, n->stream), "repair count clear"))) return rc;
     if (fused) {
-        rc = fused_pass(n, d_x, N, d_out, false, NULL, NULL, 0, theta, sink ? n->d_rep_idx : NULL, sink ? d_count : NULL);
+        rc = fused_pass(n, d_x, N, d_out, false, NULL, NULL, 0, theta, sink ? d_rows : NULL, sink ? d_count : NULL);
     } else {
-        if (sink) spgk_set_margin_sink(theta, n->d_rep_idx, d_count);
+        if (sink) spgk_set_margin_sink(theta, d_rows, d_count);
         rc = large_chain(n, d_x, N, d_out, false);
         spgk_set_margin_sink(0.0f, NULL, NULL);
     }
@@ -887,13 +893,11 @@ int spg_dev_forward_large(spg_net *n, const float *d_x, uint32_t N, float *d_out
         }
         theta = n->auto_theta;
     }
-    if (!sink) {
-        if ((rc = spg_map_kernel_error(spgk_memset(d_count, 0, 4, n->stream), "repair count clear"))) return rc;
-        if ((rc = spg_map_kernel_error(spgk_margin_select(d_out, outw, N, outw, theta, n->d_rep_idx, d_count, n->stream), "margin check"))) return rc;
-    }
+    if (!sink && (rc = spg_map_kernel_error(spgk_margin_select(d_out, outw, N, outw, theta, d_rows, d_count, n->stream), "margin check"))) return rc;
     /* The row count stays on the device: the gather, the exact chain and the scatter below are launched for
-     * N rows of capacity and read the count when they run, so the call needs no host round trip.  A copy
-     * travels to pinned host memory for spingalett_last_repaired(). */
+     * N rows of capacity and read the count when they run, so the call needs no host round trip.  A last kernel
+     * writes it to pinned host memory for spingalett_last_repaired() and clears it for the next call: a copy behind
+     * this call and a memset in front of the next cost the stream 13 us, it costs 3. */
     if (!n->h_count) {
         void *h = NULL;
         if ((rc = spg_map_kernel_error(spgk_host_alloc(&h, 256), "repair count (host)"))) return rc;
@@ -902,7 +906,7 @@ int spg_dev_forward_large(spg_net *n, const float *d_x, uint32_t N, float *d_out
     }
     uint32_t *h_slot = n->h_count + n->count_slot;
     const uint32_t expected = n->count_seen ? *(volatile uint32_t *)h_slot : 0;    /* the count of the call before: a guide to tile shapes only */
-    /* (the copy is queued behind the repair kernels: nothing sits between the one-term pass and the repair, so the
+    /* (the count is taken behind the repair kernels: nothing sits between the one-term pass and the repair, so the
      * repair's prologue overlaps the tail of the pass under programmatic dependent launch) */
     if (n->count_slot + 1 > n->count_slots_used) n->count_slots_used = n->count_slot + 1;
     if (Llast->act == ACT_SOFTMAX && Llast->out > spgk_gemm_tc_softmax_max()) {
@@ -918,28 +922,28 @@ int spg_dev_forward_large(spg_net *n, const float *d_x, uint32_t N, float *d_out
     if (fused && repair_fused && n->klayers[0].precision != PRECISION_FLOAT32) {
         /* files whose weights are exact in 16 bits: the flagged rows again through the same kernel, each as a
          * hi/lo pair of tile rows, written over their one-term results */
-        if ((rc = fused_pass(n, d_x, N, d_out, true, n->d_rep_idx, d_count, expected, 0.0f, NULL, NULL))) return rc;
-        if ((rc = spg_map_kernel_error(spgk_memcpy_d2h(h_slot, d_count, 4, n->stream), "repair count"))) return rc;
-        n->count_pending = true; n->count_seen = true;
+        if ((rc = fused_pass(n, d_x, N, d_out, true, d_rows, d_count, expected, 0.0f, NULL, NULL))) return rc;
+        if ((rc = spg_map_kernel_error(spgk_count_take(d_count, h_slot, n->stream), "repair count"))) return rc;
+        n->count_pending = true; n->count_seen = true; n->count_clean = captured ? clean_before : true;
         return SPINGALETT_OK;
     }
     spgk_set_dynamic_rows(d_count, expected);
     dynamic_rows = true;
     if (Llast->act != ACT_SOFTMAX || Llast->out <= spgk_gemm_tc_softmax_max()) {
         /* the split reads the flagged rows in place and the last layer's epilogue writes them back in place */
-        repair_rows = n->d_rep_idx;
+        repair_rows = d_rows;
         rc = large_chain(n, d_x, N, d_out, true);
         repair_rows = NULL;
     } else {
-        rc = spg_map_kernel_error(spgk_gather_rows(d_x, n->d_rep_idx, n->d_rep_in, N, in0, n->stream), "repair gather");
+        rc = spg_map_kernel_error(spgk_gather_rows(d_x, d_rows, n->d_rep_in, N, in0, n->stream), "repair gather");
         if (!rc) rc = large_chain(n, n->d_rep_in, N, n->d_rep_out, true);
-        if (!rc) rc = spg_map_kernel_error(spgk_scatter_rows(n->d_rep_out, n->d_rep_idx, d_out, N, outw, outw, n->stream), "repair scatter");
+        if (!rc) rc = spg_map_kernel_error(spgk_scatter_rows(n->d_rep_out, d_rows, d_out, N, outw, outw, n->stream), "repair scatter");
     }
     spgk_set_dynamic_rows(NULL, 0);
     dynamic_rows = false;
     if (rc) return rc;
-    if ((rc = spg_map_kernel_error(spgk_memcpy_d2h(h_slot, d_count, 4, n->stream), "repair count"))) return rc;
-    n->count_pending = true; n->count_seen = true;
+    if ((rc = spg_map_kernel_error(spgk_count_take(d_count, h_slot, n->stream), "repair count"))) return rc;
+    n->count_pending = true; n->count_seen = true; n->count_clean = captured ? clean_before : true;
     spg_note_path(fused_pass_ran ? "tcgen05-fused" : "tcgen05");
     return SPINGALETT_OK;
 }

@@ -57,7 +57,7 @@ typedef struct spg_net_s {
     uint32_t last_repaired; bool auto_calibrated; float auto_theta;
     uint8_t bf16_fits_f16;                /* BF16 file: 0 not looked at yet, 1 every weight is within fp16's range, 2 not */
     uint32_t auto_calls;                  /* large AUTO calls since the calibration: every SPG_AUTO_RECAL-th one measures again */
-    uint32_t *h_count; bool count_pending, count_seen;      /* pinned: [slot] repaired-row counts of the last AUTO call (one slot per pipelined chunk) */
+    uint32_t *h_count; bool count_pending, count_seen, count_clean;      /* pinned: [slot] repaired-row counts of the last AUTO call (one slot per pipelined chunk) */
     uint32_t count_slot, count_slots_used;
     void *copy_stream; void *copy_ev[SPG_PIPE_MAX + 1];      /* host-input pipeline: copies run ahead of compute */
     float *h_chunk[2]; size_t h_chunk_bytes;                /* page-locked staging for pageable inputs: two chunks */
