@@ -303,7 +303,7 @@ SPGK_API int spgk_layer_gemm_tc(const spgk_layer *L,
                                 float *out32, uint32_t ldo32,
                                 uint32_t N, int softmax_fused, int32_t *status, void *stream);
 /* How the calling thread's last launch of a product was arranged: whether the few-tiles kernel took it, columns of a tile, CTAs
- * that share one, stages of the operand ring.  (For tests and measurements.) */
+ * that share one (2 outside the few-tiles kernel: the kernel on pairs of CTAs), stages of the operand ring.  (For tests and measurements.) */
 SPGK_API void spgk_gemm_tc_arrangement(uint32_t out[4]);
 /* The same layer with the network's narrow last layer ("head", at most 16 outputs) finished in its epilogue:
  * each epilogue thread keeps the head's dot products of its row in registers (fp32 FMAs against head weights

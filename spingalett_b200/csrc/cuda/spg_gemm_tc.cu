@@ -67,6 +67,7 @@ struct GemmParams {
     float margin_theta; uint32_t *margin_idx, *margin_count;
     const uint32_t *out_rows;     // optional scatter of the fp32 output rows   // fused-softmax rows with top-two logit gap < theta are appended here (optional)
     int tma_store;                // 16-bit output leaves through TMA stores (one plane, tiles at least 128 wide)
+    uint32_t a_terms, w_terms;    // pairs of CTAs: terms of a stage
     const uint32_t *m_limit;      // optional device-resident row count: the kernel works on min(M, *m_limit) rows ...
     uint32_t m_above;             // ... or on none, if they are no more than this (spg_gemm_split_kernel has them)
 };
@@ -121,6 +122,18 @@ __device__ __forceinline__ void my_tile(const GemmParams &p, const RowLimit &rl,
 {
     if (p.own_rows) { m_tile = blockIdx.x + (i / p.n_tiles) * gridDim.x; n_tile = i % p.n_tiles; }
     else tile_coords(p, rl, blockIdx.x + i * gridDim.x, m_tile, n_tile);
+}
+
+// The same for a pair of CTAs, whose tiles are 256 rows high (the row tiles of `rl` then too): this CTA's half is row tile 2 * that + rank.
+__device__ __forceinline__ uint32_t pair_tile_count(const GemmParams &p, const RowLimit &rl)
+{
+    const uint32_t total = rl.m_tiles * p.n_tiles, pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
+    return total > pair ? (total - pair + pairs - 1) / pairs : 0;
+}
+__device__ __forceinline__ void pair_tile(const GemmParams &p, const RowLimit &rl, uint32_t i, uint32_t &m_tile, uint32_t &n_tile)
+{
+    tile_coords(p, rl, (blockIdx.x >> 1) + i * (gridDim.x >> 1), m_tile, n_tile);
+    m_tile = 2 * m_tile + (blockIdx.x & 1u);
 }
 
 template <typename T16> __device__ __forceinline__ uint32_t pack2(float a, float b);
@@ -220,7 +233,7 @@ __device__ __forceinline__ void store_patch(const GemmParams &p, uint32_t rows, 
 // Epilogue role.  Warp w reads TMEM lanes 32*(w%4).. (its quadrant) and, of the tile's BN columns,
 // the half selected by (w-2)/4; each thread therefore owns one row of C and walks its columns in
 // chunks of 32 (two tcgen05.ld in flight per wait).
-template <int ACT, int HP>
+template <int ACT, int HP, bool PAIR = false>
 __device__ __forceinline__ void epilogue_loop(const GemmParams &p, const RowLimit &rl, uint32_t rows, uint32_t tmem_base, uint32_t tfull0, uint32_t tempty0,
                                               volatile int *abort_flag, uint32_t warp, uint32_t lane, uint8_t *stage,
                                               const CUtensorMap *map_o, uint32_t hx0)
@@ -228,7 +241,7 @@ __device__ __forceinline__ void epilogue_loop(const GemmParams &p, const RowLimi
     uint8_t *stg = stage + (warp - 2u) * PATCH_BYTES;          // 1024-byte aligned: a swizzle atom is 8 rows x 128 bytes
     const uint32_t stg_addr = smem_u32(stg);
     const uint32_t q = warp & 3u, half = (warp - 2u) >> 2;
-    const uint32_t ntile = my_tile_count(p, rl);
+    const uint32_t ntile = PAIR ? pair_tile_count(p, rl) : my_tile_count(p, rl);
     const uint32_t span = p.BN >= 32 ? p.BN / 2 : p.BN;            // columns per warp
     const uint32_t c_begin = p.BN >= 32 ? half * span : 0;
     const bool idle = p.BN < 32 && half == 1;                      // a 16-wide tile has work for one warp per quadrant
@@ -238,7 +251,7 @@ __device__ __forceinline__ void epilogue_loop(const GemmParams &p, const RowLimi
     float *xch = reinterpret_cast<float *>(stage + p.stg_bytes - 4 * 2 * 32 * 16 * 4) ;   // head mode: [parity][quadrant][lane][16] exchange
     for (uint32_t tcount = 0; tcount < ntile; tcount++) {
         uint32_t mt, nt;
-        my_tile(p, rl, tcount, mt, nt);
+        if (PAIR) pair_tile(p, rl, tcount, mt, nt); else my_tile(p, rl, tcount, mt, nt);
         const uint32_t acc = tcount & 1u, acc_ph = (tcount >> 1) & 1u;
         if (!mbar_wait(tfull0 + 8 * acc, acc_ph, abort_flag, p.status, 4)) break;
         tc_fence_after();
@@ -324,7 +337,10 @@ __device__ __forceinline__ void epilogue_loop(const GemmParams &p, const RowLimi
             }
         }
         tc_fence_before();
-        mbar_arrive(tempty0 + 8 * acc);                            // every epilogue thread hands the accumulator back
+        if (PAIR) {
+            __syncwarp();
+            if (lane == 0) spgtc::mbar_arrive_cluster(tempty0 + 8 * acc);      // a barrier of the pair's first CTA
+        } else mbar_arrive(tempty0 + 8 * acc);                     // every epilogue thread hands the accumulator back
         if (HP > 0 && nt == p.n_tiles - 1) {
             // The row is complete: the warp of the upper column half hands its sums to the warp of the lower half
             // (same rows), which adds bias, applies the head's activation or softmax and writes the outputs.
@@ -673,6 +689,147 @@ spg_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
     }
 }
 
+// ---- pairs of CTAs ---------------------------------------------------------------------------------------------------------------
+// Products of more tiles than the GPU has SMs: a pair (cluster of two, cta_group::2) has tiles of 256 rows.  Each CTA holds its own 128 rows of
+// every term of A and half of W's rows, and a stage holds all terms of a 64-deep k-block, so that none is fetched twice.
+//
+// What bounds the kernel of single CTAs is the way from L2: it delivers 64 bytes a cycle to an SM, a [128 x 64] and a [256 x 64] tile are 48 KB
+// for 512 cycles of products, and with two terms W comes twice.  Here it is 32 KB for 512 cycles with one term and 48 KB for 1024 with two.
+// Single CTAs and pairs, us: 16384 rows, 8192 x 8192, one term 1645 -> 1561 (1.41 PFLOP/s, as much as the power limit leaves cuBLAS); 8192 rows,
+// two terms 1550 -> 1322 (1.66); 65536 rows, 512 x 784, one term 64.7 -> 52.7, two 122.9 -> 89.1, both operands in two 162 -> 115; 1000 x 512, two
+// terms 143.7 -> 129.3 (its outputs); 2560 rows, 2048 x 2048, one term 31.9 -> 31.3, two 58.2 -> 51.1.
+__device__ __forceinline__ void tma_load_3d_pair(uint32_t dst, const CUtensorMap *map, uint32_t leader_bar, int c0, int c1, int c2)
+{
+    asm volatile(
+        "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
+        ::"r"(dst), "l"(map), "r"(leader_bar), "r"(c0), "r"(c1), "r"(c2) : "memory");
+}
+
+__global__ void __launch_bounds__(NUM_THREADS, 1)
+spg_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w,
+                     const __grid_constant__ CUtensorMap map_o, const GemmParams p)
+{
+    extern __shared__ uint8_t smem_raw[];
+    const uint32_t raw = smem_u32(smem_raw);
+    const uint32_t base = (raw + 1023u) & ~1023u;                    // (the same offset in both CTAs)
+    uint8_t *smem = smem_raw + (base - raw);
+
+    const uint32_t w_bytes = p.BN * BK;                              // half of W's rows, 16-bit
+    const uint32_t stage_bytes = p.a_terms * A_TILE_BYTES + p.w_terms * w_bytes;
+    const uint32_t stg_off = p.stages * stage_bytes, bar_off = stg_off + p.stg_bytes;
+    // barrier table: full[stages], empty[stages], tmem_full[2], tmem_empty[2]
+    const uint32_t full0 = base + bar_off, empty0 = full0 + 8 * p.stages, tfull0 = empty0 + 8 * p.stages, tempty0 = tfull0 + 16;
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem + bar_off + 16 * p.stages + 32);
+    volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
+    const uint32_t abort_addr = smem_u32(const_cast<int *>(abort_flag));
+
+    const uint32_t warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31u;
+    const uint32_t rank = spgtc::cluster_rank();
+    const uint32_t lead_full0 = spgtc::mapa(full0, 0), lead_tempty0 = spgtc::mapa(tempty0, 0);
+    constexpr uint32_t TMEM_COLS = 512;
+
+    if (threadIdx.x == 0) {
+        for (uint32_t s = 0; s < p.stages; s++) { mbar_init(full0 + 8 * s, 1); mbar_init(empty0 + 8 * s, 1); }
+        for (uint32_t a = 0; a < 2; a++) { mbar_init(tfull0 + 8 * a, 1); mbar_init(tempty0 + 8 * a, 2 * EPI_WARPS); }
+        *abort_flag = 0;
+        spgtc::mbar_fence_init();
+        spgtc::prefetch_map(&map_a);
+        spgtc::prefetch_map(&map_w);
+    }
+    if (warp == 1) spgtc::tmem_alloc_pair(smem_u32(tmem_slot), TMEM_COLS);
+    tc_fence_before();
+    spgtc::cluster_sync();                                           // both CTAs' barriers exist before anyone arrives on them
+    tc_fence_after();
+    const uint32_t tmem_base = *tmem_slot;
+    spg_grid_trigger();
+    spg_grid_wait();
+    uint32_t rows = p.M;
+    if (p.m_limit) {
+        const uint32_t m = *reinterpret_cast<const volatile uint32_t *>(p.m_limit);
+        rows = m < rows ? m : rows;
+        if (rows <= p.m_above) rows = 0;
+    }
+    RowLimit rl;
+    rl.m_tiles = (rows + 2 * BM - 1) / (2 * BM);
+    rl.group_m = (rl.m_tiles && p.group_m > rl.m_tiles) ? rl.m_tiles : p.group_m;
+    const uint32_t ntile = pair_tile_count(p, rl);
+
+    if (warp == 0) {
+        // ------------------------------ TMA producer: this CTA's rows; everything counts on the first CTA's barrier ------------------------------
+        uint32_t it = 0;
+        for (uint32_t ti = 0; ti < ntile; ti++) {
+            uint32_t mt, nt;
+            pair_tile(p, rl, ti, mt, nt);
+            for (uint32_t kb = 0; kb < p.kblocks; kb++, it++) {
+                const uint32_t s = it % p.stages, ph = (it / p.stages) & 1u;
+                spgtc::mbar_wait_uniform_cluster(empty0 + 8 * s, ph ^ 1u, abort_addr, p.status, 1, WAIT_LIMIT);
+                if (elect_one()) {
+                    if (rank == 0) mbar_arrive_expect_tx(full0 + 8 * s, 2 * stage_bytes);
+                    const uint32_t at = base + s * stage_bytes;
+                    for (uint32_t t = 0; t < p.a_terms; t++)
+                        tma_load_3d_pair(at + t * A_TILE_BYTES, &map_a, lead_full0 + 8 * s, (int)(kb * BK), (int)(mt * BM), (int)t);
+                    for (uint32_t t = 0; t < p.w_terms; t++)
+                        tma_load_3d_pair(at + p.a_terms * A_TILE_BYTES + t * w_bytes, &map_w, lead_full0 + 8 * s, (int)(kb * BK),
+                                         (int)(nt * p.BN + rank * (p.BN / 2)), (int)t);
+                }
+                __syncwarp();
+            }
+        }
+    } else if (warp == 1) {
+        if (rank == 0) {
+            // ------------------------------ MMA issuer for both CTAs ------------------------------
+            uint32_t it = 0;
+            for (uint32_t tcount = 0; tcount < ntile; tcount++) {
+                const uint32_t acc = tcount & 1u, acc_ph = (tcount >> 1) & 1u;
+                spgtc::mbar_wait_uniform_cluster(tempty0 + 8 * acc, acc_ph ^ 1u, abort_addr, p.status, 2, WAIT_LIMIT);
+                tc_fence_after();
+                const uint32_t d_tmem = tmem_base + acc * p.BN;
+                for (uint32_t kb = 0; kb < p.kblocks; kb++, it++) {
+                    const uint32_t s = it % p.stages, ph = (it / p.stages) & 1u;
+                    spgtc::mbar_wait_uniform_cluster(full0 + 8 * s, ph, abort_addr, p.status, 3, WAIT_LIMIT);
+                    tc_fence_after();
+                    const uint32_t at = base + s * stage_bytes, w_at = at + p.a_terms * A_TILE_BYTES;
+                    if (elect_one()) {
+                        for (uint32_t ps = 0; ps < p.npass; ps++) {
+                            const uint64_t da = make_smem_desc(at + p.pass_a[ps] * A_TILE_BYTES), db = make_smem_desc(w_at + p.pass_w[ps] * w_bytes);
+#pragma unroll
+                            for (uint32_t k = 0; k < BK / UMMA_K; k++)
+                                spgtc::umma_f16_pair(d_tmem, da + 2 * k, db + 2 * k, p.idesc, (kb | ps | k) ? 1u : 0u);
+                        }
+                        spgtc::umma_commit_pair(empty0 + 8 * s);
+                        if (kb + 1 == p.kblocks) spgtc::umma_commit_pair(tfull0 + 8 * acc);
+                    }
+                    __syncwarp();
+                }
+            }
+        }
+    } else {
+        uint8_t *stage = smem + stg_off;
+#define SPG_EPI(ACTV) epilogue_loop<ACTV, 0, true>(p, rl, rows, tmem_base, tfull0, lead_tempty0, abort_flag, warp, lane, stage, &map_o, 0)
+        switch (p.act) {
+            case SPG_ACT_RELU:     SPG_EPI(SPG_ACT_RELU); break;
+            case SPG_ACT_LEAKY:    SPG_EPI(SPG_ACT_LEAKY); break;
+            case SPG_ACT_FOO52:    SPG_EPI(SPG_ACT_FOO52); break;
+            case SPG_ACT_TANH:     SPG_EPI(SPG_ACT_TANH); break;
+            case SPG_ACT_SIGMOID:  SPG_EPI(SPG_ACT_SIGMOID); break;
+            default:               SPG_EPI(SPG_ACT_NONE); break;
+        }
+#undef SPG_EPI
+    }
+
+    tc_fence_before();
+    __syncthreads();
+    if (*abort_flag && threadIdx.x == 0) {
+        // a wait gave up: tiles that may still be in flight get time to land before the shared memory goes away
+        for (int i = 0; i < 256; i++) __nanosleep(1000);
+    }
+    spgtc::cluster_sync();               // neither CTA leaves while the other's products may read its shared memory or its warps arrive on its barriers
+    if (warp == 1) {
+        tc_fence_after();
+        spgtc::tmem_free_pair(tmem_base, TMEM_COLS);
+    }
+}
+
 // ---------------------------------------------------------------------------------
 // 16-bit weight operand preparation: any stored precision -> `parts` planes of
 // [out][ldw] 16-bit values (plane 0 = round(q), plane 1 = round(q - plane 0)).
@@ -866,6 +1023,7 @@ static int gemm_launch(const spgk_layer *L,
         static SpgOncePerDevice once;
         const int orc = once.run(dev, [&]() -> int {
             SPGK_CUDA(cudaFuncSetAttribute(spg_gemm_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dp.smem_optin));
+            SPGK_CUDA(cudaFuncSetAttribute(spg_gemm_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dp.smem_optin));
             return SPGK_OK;
         });
         if (orc) return orc;
@@ -876,14 +1034,19 @@ static int gemm_launch(const spgk_layer *L,
     p.M = N; p.N = L->out; p.K = L->in;
     p.BN = pick_bn(L->out);
     uint32_t width = p.BN;
+    // pairs of CTAs for what fills the GPU with its widest tiles, going by the caller's estimate of a device-resident row count, and has at least
+    // eight stages of products a tile: 4864 rows, 1024 x 256, one term 14.0 us against 13.1; 20000 rows, 300 x 128, two terms 22.5 against 22.9
+    const uint32_t rows_guess = spg_tls_rows_limit ? (spg_tls_rows_expected < N ? spg_tls_rows_expected : N) : N;
+    const uint32_t products = (L->in + BK - 1) / BK * (a_parts + w_parts - 1);
+    const bool pair = !softmax_fused && !head && p.BN == 256 && products >= 8u && (uint64_t)((rows_guess + BM - 1) / BM) * ((L->out + 255) / 256) > (uint64_t)sm_count && sm_count >= 2;
     // a device-resident row count usually means a small selection of a large batch: of the widths down to 64, the one whose waves of tiles take
     // the shortest for the caller's estimate of it (a wave takes as long as its width, and 32 columns more for what goes on beside the products)
     if (spg_tls_rows_limit && spg_tls_rows_expected && !softmax_fused && p.BN > 64) {
-        const uint32_t mt = (spg_tls_rows_expected + BM - 1) / BM;
+        const uint32_t high = pair ? 2 * BM : BM, at_once = pair ? sm_count / 2 : sm_count, mt = (rows_guess + high - 1) / high;
         uint32_t best = 0xFFFFFFFFu;
         for (uint32_t bn : { 256u, 192u, 128u, 96u, 64u }) {
             if (bn > p.BN) continue;
-            const uint32_t waves = (mt * ((L->out + bn - 1) / bn) + sm_count - 1) / sm_count, cost = waves * (bn + 32u);
+            const uint32_t waves = (mt * ((L->out + bn - 1) / bn) + at_once - 1) / at_once, cost = waves * (bn + 32u);
             if (cost < best) { best = cost; width = bn; }
         }
         p.BN = width;
@@ -894,7 +1057,8 @@ static int gemm_launch(const spgk_layer *L,
     p.pass_a[p.npass] = 0; p.pass_w[p.npass] = 0; p.npass++;
     if (a_parts > 1) { p.pass_a[p.npass] = 1; p.pass_w[p.npass] = 0; p.npass++; }
     if (w_parts > 1) { p.pass_a[p.npass] = 0; p.pass_w[p.npass] = 1; p.npass++; }
-    const uint32_t stage_bytes = A_TILE_BYTES + p.BN * BK * 2;
+    p.a_terms = a_parts; p.w_terms = w_parts;
+    const uint32_t stage_bytes = pair ? a_parts * A_TILE_BYTES + w_parts * p.BN * BK : A_TILE_BYTES + p.BN * BK * 2;
     if (head) {
         p.head_w = head_w; p.head_bias = head->bias; p.head_scale = head->w_scale; p.head_out = head->out; p.head_hp = head_hp(head);
         p.head_softmax = head->act == SPG_ACT_SOFTMAX ? 1 : 0;
@@ -911,7 +1075,8 @@ static int gemm_launch(const spgk_layer *L,
     p.m_tiles = (N + BM - 1) / BM;
     p.n_tiles = (L->out + p.BN - 1) / p.BN;
     p.group_m = p.m_tiles < 16 ? p.m_tiles : 16;
-    p.idesc = (1u << 4) | ((uint32_t)type16 << 7) | ((uint32_t)w_type16 << 10) | ((p.BN >> 3) << 17) | ((BM >> 4) << 24);
+    if (pair) p.group_m = 8;                                 // (tiles of 256 rows)
+    p.idesc = (1u << 4) | ((uint32_t)type16 << 7) | ((uint32_t)w_type16 << 10) | ((p.BN >> 3) << 17) | (((pair ? 2 * BM : BM) >> 4) << 24);
     p.scale = L->w_scale; p.bias = L->bias;
     p.act = L->act == SPG_ACT_SOFTMAX ? SPG_ACT_NONE : L->act;
     p.softmax = softmax_fused ? 1 : 0;
@@ -927,7 +1092,7 @@ static int gemm_launch(const spgk_layer *L,
     CUtensorMap map_a, map_w;
     int rc = spg_gemm_map(&map_a, a16, type16, L->in, N, lda, a_plane, a_parts, BM, 1);
     if (rc) return rc;
-    rc = spg_gemm_map(&map_w, w16, w_type16, L->in, L->out, ldw, w_plane, w_parts, p.BN, 1);
+    rc = spg_gemm_map(&map_w, w16, w_type16, L->in, L->out, ldw, w_plane, w_parts, pair ? p.BN / 2 : p.BN, 1);
     if (rc) return rc;
 
     // 16-bit output through TMA stores when it is one plane and a warp's columns are whole 64-column patches
@@ -940,6 +1105,20 @@ static int gemm_launch(const spgk_layer *L,
     const uint32_t tiles = p.own_rows ? p.m_tiles : p.m_tiles * p.n_tiles;   // with a head or a wide softmax a CTA owns whole row tiles
     const uint32_t grid = tiles < (uint32_t)sm_count ? tiles : (uint32_t)sm_count;
     const size_t smem = 1024 + (size_t)stages * stage_bytes + p.stg_bytes + 8 * (2 * stages + 8) + 64;
+    if (pair) {
+        const uint32_t pair_tiles = (p.m_tiles + 1) / 2 * p.n_tiles, pairs = pair_tiles < (uint32_t)sm_count / 2 ? pair_tiles : (uint32_t)sm_count / 2;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(2 * pairs); cfg.blockDim = dim3(NUM_THREADS); cfg.dynamicSmemBytes = smem; cfg.stream = (cudaStream_t)stream;
+        cudaLaunchAttribute attr[2];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+        attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[1].val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = attr; cfg.numAttrs = 2;
+        SPGK_CUDA(cudaLaunchKernelEx(&cfg, spg_gemm_pair_kernel, map_a, map_w, map_o, p));
+        spg_tls_arrangement = { 0, p.BN, 2, p.stages };
+        return spgk_check_launch("spg_gemm_pair_kernel");
+    }
     SPGK_CUDA(spg_launch_chained(spg_gemm_tc_kernel, dim3(grid), dim3(NUM_THREADS), smem, (cudaStream_t)stream, map_a, map_w, map_o, p));
     spg_tls_arrangement = { 0, p.BN, 1, p.stages };
     return spgk_check_launch("spg_gemm_tc_kernel");
