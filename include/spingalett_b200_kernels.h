@@ -395,6 +395,10 @@ SPGK_API int spgk_ce_delta(const float *a, const float *t, float *delta, uint64_
 SPGK_API int spgk_col_sums(const float *d, uint32_t rows, uint32_t cols, float scale, float *out, void *stream);
 SPGK_API int spgk_train_grad(const float *delta, uint32_t ldd, const float *a, uint32_t lda, float *gw, uint32_t ldg,
                              float *gb, uint32_t out, uint32_t in, uint32_t rows, float scale, void *stream);
+/* the gradients of two layers over the same rows, in one launch where the two products are cut alike: the results of two spgk_train_grad calls
+ * with dense operands ([rows][out], [rows][in], [out][in]) */
+typedef struct { const float *delta, *a; float *gw, *gb; uint32_t out, in; } spgk_train_gradients;
+SPGK_API int spgk_train_grad2(const spgk_train_gradients *a, const spgk_train_gradients *b, uint32_t rows, float scale, void *stream);
 SPGK_API int spgk_gather_rows(const float *src, const uint32_t *idx, float *dst, uint32_t rows, uint32_t width,
                               void *stream);
 SPGK_API int spgk_gather_rows2(const float *src_a, uint32_t width_a, float *dst_a, const float *src_b, uint32_t width_b,
@@ -437,6 +441,9 @@ SPGK_API size_t spgk_train_state_bytes(void);
 SPGK_API int spgk_train_state_reset(void *state, void *stream);
 SPGK_API int spgk_train_state_step(void *state, uint32_t steps_per_epoch, uint32_t batch, float b1, float b2, void *stream);
 SPGK_API void spgk_train_use_state(const void *state);
+/* spgk_train_use_state, and spgk_gather_rows2 and the update move the record on themselves (no spgk_train_state_step): for steps that are one
+ * gather, products and one update */
+SPGK_API void spgk_train_move_state(void *state, uint32_t steps_per_epoch, uint32_t batch, float b1, float b2);
 SPGK_API int spgk_graph_begin(void *stream);
 SPGK_API int spgk_graph_end(void *stream, void **exec);
 SPGK_API int spgk_graph_launch(void *exec, void *stream);

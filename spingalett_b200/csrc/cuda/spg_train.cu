@@ -292,31 +292,48 @@ spg_gather_rows_kernel(const float *__restrict__ src, const uint32_t *__restrict
 // arguments every time and can be replayed as a CUDA graph: the position in the epoch (first row of the step in the
 // shuffled order) and Adam's running powers of beta1 / beta2 with the bias corrections made of them.  The host
 // computes the same values with the same fp32 operations (Training.c:480-500), so both ways give the same bits.
+// A step that gathers its rows and ends with one of the update kernels here needs no launch of its own for it: the gather reads `step` and makes
+// this step's corrections (which only the update reads), the update moves `step` on (which only the gather reads).
 struct SpgStepState { uint32_t step, start; float b1pow, b2pow, mf, vf; };
+struct SpgStepMove { SpgStepState *state; uint32_t steps_per_epoch, batch; float b1, b2; };
+
+__device__ __forceinline__ void move_corrections(const SpgStepMove &mv)
+{
+    SpgStepState *st = mv.state;
+    st->b1pow *= mv.b1;
+    st->b2pow *= mv.b2;
+    st->mf = 1.0f / (1.0f - st->b1pow);
+    st->vf = 1.0f / (1.0f - st->b2pow);
+}
+
+__device__ __forceinline__ void move_step(const SpgStepMove &mv) { mv.state->step = mv.state->step + 1 == mv.steps_per_epoch ? 0u : mv.state->step + 1; }
 
 // first launch of a step: this step's values, then the position moves on
 __global__ void spg_train_state_kernel(SpgStepState *st, uint32_t steps_per_epoch, uint32_t batch, float b1, float b2)
 {
     st->start = st->step * batch;
     st->step = st->step + 1 == steps_per_epoch ? 0u : st->step + 1;
-    st->b1pow *= b1;
-    st->b2pow *= b2;
-    st->mf = 1.0f / (1.0f - st->b1pow);
-    st->vf = 1.0f / (1.0f - st->b2pow);
+    move_corrections(SpgStepMove{ st, steps_per_epoch, batch, b1, b2 });
 }
 
 struct SpgGraph { cudaGraphExec_t exec; uint32_t nodes; };
 
 // the device step state that the launchers below hand to their kernels (NULL: arguments come from the host)
 thread_local const SpgStepState *tls_step_state = nullptr;
+thread_local SpgStepMove tls_step_move = {};            // .state: the gather and the update move the record on
 
 // gather the same rows of two tables (a mini-batch's inputs and targets) in one launch
 __global__ void __launch_bounds__(256)
 spg_gather_rows2_kernel(const float *__restrict__ src_a, uint32_t wa, float *__restrict__ dst_a, const float *__restrict__ src_b,
                         uint32_t wb, float *__restrict__ dst_b, const uint32_t *__restrict__ idx, uint32_t rows,
-                        const SpgStepState *__restrict__ state)
+                        const SpgStepState *state, const SpgStepMove mv)
 {
-    if (state) idx += state->start;                    // the step's first row of the shuffled order, kept on the device
+    spg_grid_wait();
+    spg_grid_trigger();
+    if (mv.state) {
+        idx += mv.state->step * mv.batch;
+        if (blockIdx.x == 0 && threadIdx.x == 0) move_corrections(mv);
+    } else if (state) idx += state->start;             // the step's first row of the shuffled order, kept on the device
     const uint32_t w = wa + wb;
     const uint64_t total = (uint64_t)rows * w;
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (uint64_t)gridDim.x * blockDim.x) {
@@ -332,9 +349,12 @@ spg_gather_rows2_kernel(const float *__restrict__ src_a, uint32_t wa, float *__r
 // m = b1*m + (1-b1)*g ; v = b2*v + (1-b2)*g*g ; w -= lr * (m*mf) / sqrt(v*vf + eps).
 __global__ void __launch_bounds__(256)
 spg_adam_kernel(float *__restrict__ w, float *__restrict__ m, float *__restrict__ v, const float *__restrict__ g, uint64_t n,
-                float lr, float b1, float b2, float mf, float vf, float eps, float gscale, const SpgStepState *__restrict__ state)
+                float lr, float b1, float b2, float mf, float vf, float eps, float gscale, const SpgStepState *state, const SpgStepMove mv)
 {
+    spg_grid_wait();
+    spg_grid_trigger();
     if (state) { mf = state->mf; vf = state->vf; }     // bias corrections of this step, advanced on the device
+    if (mv.state && blockIdx.x == 0 && threadIdx.x == 0) move_step(mv);
     const float omb1 = 1.0f - b1, omb2 = 1.0f - b2;
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
         const float gi = g[i] * gscale;
@@ -408,9 +428,12 @@ spg_sumsq_kernel(const float *__restrict__ g, uint64_t n, float *out)
 __global__ void __launch_bounds__(256)
 spg_optimizer_kernel(int kind, float *__restrict__ w, float *__restrict__ m, float *__restrict__ v, const float *__restrict__ g,
                      uint64_t n, uint64_t n_w, float lr, float momentum, float b1, float b2, float mf, float vf, float eps,
-                     float decay, float gscale, const float *sumsq, float max_norm, const SpgStepState *__restrict__ state)
+                     float decay, float gscale, const float *sumsq, float max_norm, const SpgStepState *state, const SpgStepMove mv)
 {
+    spg_grid_wait();
+    spg_grid_trigger();
     if (state) { mf = state->mf; vf = state->vf; }
+    if (mv.state && blockIdx.x == 0 && threadIdx.x == 0) move_step(mv);
     float gs = gscale;
     if (sumsq) {
         const float norm = sqrtf(*sumsq) * gscale;
@@ -516,9 +539,8 @@ static int train_gemm(int mode, const float *A, uint32_t lda, const float *B, ui
     }
     // Products of at least 148 64 x 64 tiles: the SIMT kernel with that tile.  Smaller ones - on a 256-row step of a
     // 784-512-1000-10 network that is every product - take 32 x 32 tiles on the tensor cores.
-    const uint32_t tiles64 = ((N + 63) / 64) * ((M + 63) / 64);
-    if (tiles64 < 148u)
-        return spg_train_product(mode, SpgTrainProduct{ A, B, C, lda, ldb, ldc, M, N, K, alpha, bias, aux, ldaux, act, colsum }, s);
+    const SpgTrainProduct p = { A, B, C, lda, ldb, ldc, M, N, K, alpha, bias, aux, ldaux, act, colsum };
+    if (spg_train_one_kernel(p)) return spg_train_product(mode, p, s);
     const dim3 grid((N + 63) / 64, (M + 63) / 64);
     if (mode == TRAIN_FWD) spg_train_gemm_kernel<TRAIN_FWD, 64, 1><<<grid, 256, 0, s>>>(A, lda, B, ldb, C, ldc, M, N, K, alpha, bias, aux, ldaux, act, colsum);
     else if (mode == TRAIN_DELTA) spg_train_gemm_kernel<TRAIN_DELTA, 64, 1><<<grid, 256, 0, s>>>(A, lda, B, ldb, C, ldc, M, N, K, alpha, bias, aux, ldaux, act, colsum);
@@ -531,6 +553,28 @@ int spgk_train_gemm(int mode, const float *A, uint32_t lda, const float *B, uint
                     int act, void *stream)
 {
     return train_gemm(mode, A, lda, B, ldb, C, ldc, M, N, K, alpha, bias, aux, ldaux, act, nullptr, stream);
+}
+
+int spgk_train_grad2(const spgk_train_gradients *a, const spgk_train_gradients *b, uint32_t rows, float scale, void *stream)
+{
+    SpgTrainProduct p[2];
+    const spgk_train_gradients *g[2] = { a, b };
+    for (int i = 0; i < 2; i++) {
+        if (!g[i] || !g[i]->delta || !g[i]->a || !g[i]->gw || !g[i]->gb || g[i]->out == 0 || g[i]->in == 0 || rows == 0) {
+            spgk_set_error("spgk_train_grad2", "bad argument");
+            return SPGK_E_ARG;
+        }
+        p[i] = SpgTrainProduct{ g[i]->delta, g[i]->a, g[i]->gw, g[i]->out, g[i]->in, g[i]->in, g[i]->out, g[i]->in, rows, scale, nullptr, nullptr, 0, 0, g[i]->gb };
+    }
+    if (spg_train_one_kernel(p[0]) && spg_train_one_kernel(p[1])) {
+        const int rc = spg_train_two_gradients(p[0], p[1], (cudaStream_t)stream);
+        if (rc != SPGK_E_UNSUPPORTED) return rc;
+    }
+    for (int i = 0; i < 2; i++) {
+        const int rc = spgk_train_grad(g[i]->delta, g[i]->out, g[i]->a, g[i]->in, g[i]->gw, g[i]->in, g[i]->gb, g[i]->out, g[i]->in, rows, scale, stream);
+        if (rc) return rc;
+    }
+    return SPGK_OK;
 }
 
 int spgk_train_grad(const float *delta, uint32_t ldd, const float *a, uint32_t lda, float *gw, uint32_t ldg, float *gb,
@@ -563,7 +607,14 @@ int spgk_train_state_step(void *state, uint32_t steps_per_epoch, uint32_t batch,
 
 // from now on spgk_gather_rows2 (row offset), spgk_adam and spgk_optimizer_step (bias corrections) of this thread take
 // those values from `state` instead of their arguments; NULL switches back
-void spgk_train_use_state(const void *state) { tls_step_state = static_cast<const SpgStepState *>(state); }
+void spgk_train_use_state(const void *state) { tls_step_state = static_cast<const SpgStepState *>(state); tls_step_move = {}; }
+
+// ... and those launches move the record on themselves, without spgk_train_state_step: a step is then a gather, its products and one update
+void spgk_train_move_state(void *state, uint32_t steps_per_epoch, uint32_t batch, float b1, float b2)
+{
+    tls_step_state = static_cast<const SpgStepState *>(state);
+    tls_step_move = { static_cast<SpgStepState *>(state), steps_per_epoch, batch, b1, b2 };
+}
 
 // Stream capture of a step's launches into a graph, and its replay.  begin .. end must enclose only launches and
 // memsets on `stream`; end returns the executable graph (NULL and an error code if the capture did not come off).
@@ -609,8 +660,8 @@ int spgk_gather_rows2(const float *src_a, uint32_t width_a, float *dst_a, const 
 {
     if (!src_a || !dst_a || !src_b || !dst_b || !idx) { spgk_set_error("spgk_gather_rows2", "bad argument"); return SPGK_E_ARG; }
     if (rows == 0 || width_a + width_b == 0) return SPGK_OK;
-    spg_gather_rows2_kernel<<<blocks_for((uint64_t)rows * (width_a + width_b)), 256, 0, (cudaStream_t)stream>>>(
-        src_a, width_a, dst_a, src_b, width_b, dst_b, idx, rows, tls_step_state);
+    SPGK_CUDA(spg_launch_chained(spg_gather_rows2_kernel, dim3(blocks_for((uint64_t)rows * (width_a + width_b))), dim3(256), 0, (cudaStream_t)stream,
+        src_a, width_a, dst_a, src_b, width_b, dst_b, idx, rows, tls_step_state, tls_step_move));
     return spgk_check_launch("spg_gather_rows2_kernel");
 }
 
@@ -642,7 +693,8 @@ int spgk_adam(float *w, float *m, float *v, const float *g, uint64_t n, float lr
 {
     if (!w || !m || !v || !g) { spgk_set_error("spgk_adam", "bad argument"); return SPGK_E_ARG; }
     if (n == 0) return SPGK_OK;
-    spg_adam_kernel<<<blocks_for(n), 256, 0, (cudaStream_t)stream>>>(w, m, v, g, n, lr, b1, b2, mf, vf, eps, gscale, tls_step_state);
+    SPGK_CUDA(spg_launch_chained(spg_adam_kernel, dim3(blocks_for(n)), dim3(256), 0, (cudaStream_t)stream, w, m, v, g, n, lr, b1, b2, mf, vf, eps, gscale,
+                                 tls_step_state, tls_step_move));
     return spgk_check_launch("spg_adam_kernel");
 }
 
@@ -675,8 +727,8 @@ int spgk_optimizer_step(int kind, float *w, float *m, float *v, const float *g, 
         return SPGK_E_ARG;
     }
     if (n == 0) return SPGK_OK;
-    spg_optimizer_kernel<<<blocks_for(n), 256, 0, (cudaStream_t)stream>>>(kind, w, m, v, g, n, n_weights, lr, momentum, b1, b2, mf, vf,
-                                                                         eps, decay, gscale, sumsq_dev, max_norm, tls_step_state);
+    SPGK_CUDA(spg_launch_chained(spg_optimizer_kernel, dim3(blocks_for(n)), dim3(256), 0, (cudaStream_t)stream, kind, w, m, v, g, n, n_weights, lr, momentum,
+                                 b1, b2, mf, vf, eps, decay, gscale, sumsq_dev, max_norm, tls_step_state, tls_step_move));
     return spgk_check_launch("spg_optimizer_kernel");
 }
 

@@ -20,5 +20,9 @@ struct SpgTrainProduct {
     float *colsum;
 };
 
+// whether the tensor-core kernel takes a product: fewer than 148 tiles of 64 x 64
+inline bool spg_train_one_kernel(const SpgTrainProduct &p) { return ((p.N + 63) / 64) * ((p.M + 63) / 64) < 148u; }
+// two gradients in one launch; SPGK_E_UNSUPPORTED, and nothing launched, for products that are cut differently
+int spg_train_two_gradients(const SpgTrainProduct &a, const SpgTrainProduct &b, cudaStream_t s);
 // any of the three, on the tensor cores with fp32-level error (spg_train_mma.cu)
 int spg_train_product(int mode, const SpgTrainProduct &p, cudaStream_t s);

@@ -17,7 +17,7 @@
 // activation and stores.  tcgen05 would lift the first bound, but adds in another order and wants both terms of both operands written back
 // to shared memory.  One launch behind another, before (register-staged tiles, one barrier of the CTA a slice) and now: 512 x 784 forward,
 // 256 rows 16.5 -> 10.0 us, 1000 x 512 forward 18.0 -> 10.2, 512 x 1000 delta 16.4 -> 12.1, 1000 x 512 gradient 14.4 -> 10.7; the step of
-// the 784-512-1000-10 net 98 -> 68 us.  Three and four slots: level alone, 4 us slower in the step.  A ring that the whole CTA shares, one
+// the 784-512-1000-10 net 98 -> 68 us (65 to 68 with the gradients of its first two layers in one launch, 15 us instead of 17).  Three and four slots: level alone, 4 us slower in the step.  A ring that the whole CTA shares, one
 // barrier a stage: 0.5 to 2 us slower each, the warps then load, split and multiply in step.
 #include "spg_train.cuh"
 
@@ -235,30 +235,55 @@ spg_train_mma_kernel(const SpgTrainProduct p)
     product_tile<MODE, V, WARPS>(p, blockIdx.x, sm);
 }
 
+// the gradients of two layers: what the second leaves idle of the GPU's last wave the first has filled already
+template <int V, int WARPS>
+__global__ void __launch_bounds__(WARPS * 32)
+spg_train_grad2_kernel(const SpgTrainProduct a, const SpgTrainProduct b, uint32_t tiles_a)
+{
+    extern __shared__ __align__(16) float sm[];
+    spg_grid_wait();
+    spg_grid_trigger();
+    const bool first = blockIdx.x < tiles_a;
+    product_tile<TRAIN_GRAD, V, WARPS>(first ? a : b, first ? blockIdx.x : blockIdx.x - tiles_a, sm);
+}
+
 uint32_t tiles(const SpgTrainProduct &p) { return ((p.M + TILE - 1) / TILE) * ((p.N + TILE - 1) / TILE); }
 
-template <int MODE, int V, int WARPS>
-int launch(const SpgTrainProduct &p, cudaStream_t s)
+// Launches on `count` tiles.  CTAs are started while the launch before is still running, on whatever SM has room: so that they do not pile up there,
+// a CTA takes the shared memory that leaves an SM room for its even share of them (1 KB of each goes to the system).
+template <typename Kernel, typename... Args>
+int launch_tiles(SpgOncePerDevice &once, Kernel kernel, uint32_t count, int warps, cudaStream_t s, const Args &...args)
 {
-    static SpgOncePerDevice once;
-    constexpr size_t ring = 4 * ring_floats(WARPS);
-    static_assert(sum_floats(WARPS) <= ring_floats(WARPS), "the partial sums take the place of the rings");
+    const size_t ring = 4 * ring_floats(warps);
     int device = 0;
     SpgDeviceProps props;
     SPGK_CUDA(cudaGetDevice(&device));
     int rc = spg_device_props(&props);
     if (rc) return rc;
     rc = once.run(device, [&] {
-        SPGK_CUDA(cudaFuncSetAttribute(spg_train_mma_kernel<MODE, V, WARPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)props.smem_optin));
+        SPGK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)props.smem_optin));
         return SPGK_OK;
     });
     if (rc) return rc;
-    // CTAs are started while the launch before is still running, on whatever SM has room: so that they do not pile up there, a CTA takes
-    // the shared memory that leaves an SM room for its even share of them (1 KB of each goes to the system).
-    const uint32_t share = (tiles(p) + props.sm_count - 1) / props.sm_count;
+    const uint32_t share = (count + props.sm_count - 1) / props.sm_count;
     const size_t room = (props.smem_optin + 1024) / share - 1024 & ~(size_t)127, bytes = share < 8 && room > ring ? room : ring;
-    SPGK_CUDA(spg_launch_chained(spg_train_mma_kernel<MODE, V, WARPS>, dim3(tiles(p)), dim3(WARPS * 32), bytes, s, p));
+    SPGK_CUDA(spg_launch_chained(kernel, dim3(count), dim3(warps * 32), bytes, s, args...));
     return spgk_check_launch("spg_train_mma_kernel");
+}
+
+template <int MODE, int V, int WARPS>
+int launch(const SpgTrainProduct &p, cudaStream_t s)
+{
+    static SpgOncePerDevice once;
+    static_assert(sum_floats(WARPS) <= ring_floats(WARPS), "the partial sums take the place of the rings");
+    return launch_tiles(once, spg_train_mma_kernel<MODE, V, WARPS>, tiles(p), WARPS, s, p);
+}
+
+template <int V, int WARPS>
+int launch_grad2(const SpgTrainProduct &a, const SpgTrainProduct &b, cudaStream_t s)
+{
+    static SpgOncePerDevice once;
+    return launch_tiles(once, spg_train_grad2_kernel<V, WARPS>, tiles(a) + tiles(b), WARPS, s, a, b, tiles(a));
 }
 
 // ---- the output end of a step, for at most 16 outputs -----------------------------------------------------------------------
@@ -350,10 +375,22 @@ spg_train_output_kernel(const OutputArgs p)
 
 }  // namespace
 
-int spg_train_product(int mode, const SpgTrainProduct &p, cudaStream_t s)
+static bool on_lines(const SpgTrainProduct &p)
 {
     const auto lines = [](const void *q, uint32_t ld) { return ((uintptr_t)q & 15u) == 0 && (ld & 3u) == 0; };
-    const bool vec = lines(p.A, p.lda) && lines(p.B, p.ldb);
+    return lines(p.A, p.lda) && lines(p.B, p.ldb);
+}
+
+int spg_train_two_gradients(const SpgTrainProduct &a, const SpgTrainProduct &b, cudaStream_t s)
+{
+    const bool vec = on_lines(a), few = tiles(a) <= 32u;
+    if (vec != on_lines(b) || few != (tiles(b) <= 32u)) return SPGK_E_UNSUPPORTED;
+    return few ? (vec ? launch_grad2<4, 8>(a, b, s) : launch_grad2<1, 8>(a, b, s)) : (vec ? launch_grad2<4, 4>(a, b, s) : launch_grad2<1, 4>(a, b, s));
+}
+
+int spg_train_product(int mode, const SpgTrainProduct &p, cudaStream_t s)
+{
+    const bool vec = on_lines(p);
     const bool few = tiles(p) <= 32u;      // eight warps a tile instead of four: 10 x 1000 over 256 rows 4.2 against 4.8 us, 30 x 60 over 1000 9.6 against 11
 #define SPG_PRODUCT(MODE) (few ? (vec ? launch<MODE, 4, 8>(p, s) : launch<MODE, 1, 8>(p, s)) : (vec ? launch<MODE, 4, 4>(p, s) : launch<MODE, 1, 4>(p, s)))
     return mode == TRAIN_FWD ? SPG_PRODUCT(TRAIN_FWD) : mode == TRAIN_DELTA ? SPG_PRODUCT(TRAIN_DELTA) : SPG_PRODUCT(TRAIN_GRAD);

@@ -427,9 +427,11 @@ void train_struct_arguments(TrainArgs a)
     { const char *e = getenv("SPINGALETT_TRAIN_GRAPH"); if (e && *e == '0') graph_mode = false; }
     void *step_state = (void *)(t->words + 128);      /* clear of the loss / flag / norm words and of the rank-agreement floats */
     uint64_t steps_done = 0;
+    const bool moving = graph_mode && mini && s_world == 1;          /* the gather and the update move the record on */
     if (graph_mode) {
         DEV(spgk_train_state_reset(step_state, st), "train: step state");
-        spgk_train_use_state(step_state);
+        if (moving) spgk_train_move_state(step_state, steps_per_epoch, batch, a.beta1, a.beta2);
+        else spgk_train_use_state(step_state);
     }
     for (size_t epoch = 1; epoch <= a.epochs; epoch++) {
         const bool need_loss = should_report(epoch, a.epochs, a.report_interval) ||
@@ -465,7 +467,7 @@ void train_struct_arguments(TrainArgs a)
                 if (spgk_graph_begin(st) == SPGK_OK) in_capture = true;
                 else { spingalett_clear_error(); graph_failed = true; capture = false; }
             }
-            if (graph_mode) SDEV(spgk_train_state_step(step_state, steps_per_epoch, batch, a.beta1, a.beta2, st), "train: step state");
+            if (graph_mode && !moving) SDEV(spgk_train_state_step(step_state, steps_per_epoch, batch, a.beta1, a.beta2, st), "train: step state");
             if (mini) {
                 /* (with the device record the kernel adds the step's first row itself) */
                 SDEV(spgk_gather_rows2(t->data_x, in0, t->batch_x, t->data_t, outw, t->batch_t, graph_mode ? t->idx : t->idx + start, cur, st),
@@ -507,8 +509,17 @@ void train_struct_arguments(TrainArgs a)
                 const uint32_t fi = p->topology[l], fo = p->topology[l + 1];
                 const float *dl = t->deltas + (size_t)cur * p->neuron_offsets[l + 1];
                 const float *al = l == 0 ? bx : t->acts + (size_t)cur * p->neuron_offsets[l];
-                SDEV(spgk_train_grad(dl, fo, al, fi, G + p->weight_offsets[l], fi, G + tw + p->bias_offsets[l],
-                                    fo, fi, cur, gs, st), "train: gradients");
+                const bool alone = s_world > 1 && !fused_x;              /* every layer's gradients cross the links as soon as they are there */
+                if (l > 1 || alone || last == 1)
+                    SDEV(spgk_train_grad(dl, fo, al, fi, G + p->weight_offsets[l], fi, G + tw + p->bias_offsets[l],
+                                        fo, fi, cur, gs, st), "train: gradients");
+                else if (l == 0) {                                       /* those of the first two layers in one launch */
+                    const spgk_train_gradients both[2] = {
+                        { t->deltas + (size_t)cur * p->neuron_offsets[2], t->acts + (size_t)cur * p->neuron_offsets[1], G + p->weight_offsets[1],
+                          G + tw + p->bias_offsets[1], p->topology[2], p->topology[1] },
+                        { dl, al, G, G + tw + p->bias_offsets[0], fo, fi } };
+                    SDEV(spgk_train_grad2(&both[0], &both[1], cur, gs, st), "train: gradients");
+                }
                 if (s_world > 1 && !fused_x) {
                     SDEV(spgk_event_record(s_ev_ready, st), "train: exchange order");
                     SDEV(spgk_stream_wait_event(s_ar_stream, s_ev_ready), "train: exchange order");

@@ -47,6 +47,28 @@ def test_products_against_float64(spg, rows, fi, fo):
     assert np.all(np.abs(sums[:fo] - gs * D.sum(0)) <= gs * (rows + 2) * EPS * np.abs(D).sum(0)) and sums[fo] == -7.0
 
 
+@pytest.mark.parametrize("rows,w0,w1,w2", [(256, 784, 512, 1000), (100, 301, 333, 129), (32, 24, 50, 10), (7, 36, 1024, 40), (300, 1024, 1024, 20)])
+def test_two_layers_gradients_in_one_launch(spg, rows, w0, w1, w2):
+    """The same bits as one launch each, for products that are cut alike and for those that are not."""
+    import torch
+    lib = spg.lib()
+
+    class Gradients(C.Structure):
+        _fields_ = [("delta", vp), ("a", vp), ("gw", vp), ("gb", vp), ("out", u32), ("in_", u32)]
+    lib.spgk_train_grad2.argtypes = [C.POINTER(Gradients), C.POINTER(Gradients), u32, f32, vp]
+    lib.spgk_train_grad.argtypes = [vp, u32, vp, u32, vp, u32, vp, u32, u32, u32, f32, vp]
+    rng = np.random.default_rng(rows)
+    d1, d2, x, h = dev(*(rng.standard_normal((rows, w)).astype(np.float32) for w in (w1, w2, w0, w1)))
+    one, two = ([torch.full(s, -7.0, device="cuda") for s in ((w2, w1), (w2,), (w1, w0), (w1,))] for _ in range(2))
+    a = Gradients(d2.data_ptr(), h.data_ptr(), one[0].data_ptr(), one[1].data_ptr(), w2, w1)
+    b = Gradients(d1.data_ptr(), x.data_ptr(), one[2].data_ptr(), one[3].data_ptr(), w1, w0)
+    assert lib.spgk_train_grad2(C.byref(a), C.byref(b), rows, 0.25, None) == 0
+    assert lib.spgk_train_grad(d2.data_ptr(), w2, h.data_ptr(), w1, two[0].data_ptr(), w1, two[1].data_ptr(), w2, w1, rows, 0.25, None) == 0
+    assert lib.spgk_train_grad(d1.data_ptr(), w1, x.data_ptr(), w0, two[2].data_ptr(), w0, two[3].data_ptr(), w1, w0, rows, 0.25, None) == 0
+    for p, q in zip(one, two):
+        assert torch.equal(p, q) and not torch.any(p == -7.0)
+
+
 # inputs around a lane's four, a warp's 128 and the 1024 of a round; one and two outputs a warp; an odd number of rows
 @pytest.mark.parametrize("sigmoid", [0, 1])
 @pytest.mark.parametrize("rows,fi,fo", [(1, 1, 1), (2, 4, 8), (3, 127, 9), (5, 128, 16), (255, 1000, 10), (4, 1023, 3), (2, 1024, 16), (3, 1028, 10), (3, 2049, 10)])
