@@ -25,10 +25,11 @@
 // 106 us over the net, whose busiest SMs have 237 such blocks.  One byte per weight in the operand instead of two is why this
 // path exists beside the 16-bit streaming kernel, which writes and reads 32 KB per such block.
 //
-// Measured: 125 us at 8 rows (GEMV: 201), 188 at 64 (16-bit streaming kernel: 577), 555 at 256 (GEMM chain: 684).  A block of
-// INT4 takes 480 cycles at 8 rows, of which the MMA warp's own turn is all (operand tiles changing hands one at a time: 810),
-// and 750 at 64 (900), where every CTA draws 32 KB of digits a block from L2 at 43 bytes a cycle; the tensor pipe would need
-// 512.  From layers of 32 to 166 blocks with weights from HBM: 530 cycles a block and 14 us a layer at 8 rows, 870 and 16 at 64.
+// Measured: 125 us at 8 rows (GEMV: 201), 166 at 64 (16-bit streaming kernel: 577), 460 at 256 (GEMM chain: 684).  A block of
+// INT4 takes 480 cycles at 8 rows, of which the MMA warp's own turn is all (operand tiles changing hands one at a time: 810).
+// At 64 rows a CTA alone draws 32 KB of digits a block from L2, at 43 bytes a cycle: 750 cycles; the tensor pipe would need
+// 512.  Large layers of more than 32 rows a group therefore run on pairs of CTAs (cta_group::2), each with half of the digits:
+// INT4 176 -> 166 us at 64 rows, 257 -> 229 at 96, 552 -> 460 at 256; INT2 452 -> 404, INT8 656 -> 568 at 256.  From layers of 32 to 166 blocks with weights from HBM: 530 cycles a block and 14 us a layer at 8 rows, 870 and 16 at 64.
 // INT8, whose boxes need no unpacking, takes 700 cycles at 8 rows, 5.5 TB/s.  The rest of a layer is staging, the first
 // boxes and tiles, and the last sums (1 us at 8 rows, 3 at 64).
 //
@@ -61,6 +62,7 @@ constexpr uint32_t IS_THREADS = 32 * (IS_DIGIT_WARP + 1);
 constexpr uint32_t TILE_ROWS = 128;
 constexpr uint32_t BOX_BYTES = 128 * TILE_ROWS;        // one box of packed weights = one operand tile = 16 KB
 constexpr uint32_t GROUP_ROWS = 64;                    // batch rows per pass over the weights: 256 digit columns
+constexpr uint32_t IS_PAIR_ROWS = 32, IS_PAIR_BLOCKS = 32;
 constexpr uint32_t MAX_K = 131072;                     // 64 * 128 * K < 2^31
 constexpr uint32_t MAX_TILES = 4096;                   // counters in the scratch head
 constexpr uint32_t STAGE_THREADS = 1024;
@@ -95,8 +97,17 @@ __device__ __forceinline__ void tmem_ld4(uint32_t taddr, uint32_t (&r)[4])
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(taddr) : "memory");
 }
-// int32 accumulator, A and B signed 8-bit, both K-major, M = 128, N = n
-inline uint32_t idesc_i8(uint32_t n) { return (2u << 4) | (1u << 7) | (1u << 10) | ((n >> 3) << 17) | ((128u >> 4) << 24); }
+// ... over the two CTAs of a pair: 128 rows of A each, half of B's rows each
+__device__ __forceinline__ void umma_i8_pair(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate)
+{
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::i8 [%0], %1, %2, %3, {%5, %5, %5, %5, %5, %5, %5, %5}, p;\n\t}"
+        ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(0u) : "memory");
+}
+// int32 accumulator, A and B signed 8-bit, both K-major, m x n
+inline uint32_t idesc_i8(uint32_t m, uint32_t n) { return (2u << 4) | (1u << 7) | (1u << 10) | ((n >> 3) << 17) | ((m >> 4) << 24); }
 
 // first unit of CTA c
 __host__ __device__ inline uint64_t unit_start(uint64_t units, uint32_t grid, uint32_t c) { return units * c / grid; }
@@ -299,17 +310,18 @@ __device__ __forceinline__ bool is_any_wide(const IsParams &p, uint32_t lane)
 // among them) and a scheduler has two of these warps: only values side by side hide it, so the activation is chosen outside and
 // nothing in the chain branches (with the choice inside, the last sums of a tile took 17500 cycles at 64 rows).  `dirty`: a launch before this one failed and nobody has read its status yet, so the sums and
 // counters cannot be relied on.
-template <int ACT>
+template <int ACT, bool PAIR>
 __device__ __forceinline__ void is_epilogue(const IsParams &p, bool wide, bool dirty, IsSegment seg, uint32_t tmem_base, uint32_t tfull0, uint32_t tempty0,
                                             volatile int *abort_flag, int *s_last, double *s_scale, uint32_t warp, uint32_t lane)
 {
     const uint32_t half = (warp - 2u) >> 2, et = (warp & 3u) * 32u + lane;
+    const uint32_t cta = PAIR ? blockIdx.x & 1u : 0u, teams = PAIR ? gridDim.x >> 1 : gridDim.x;      // teams: pairs, or CTAs alone
     uint32_t count = 0;
     for (; is_next_segment(p, seg); count++) {
         // a wide layer's second set takes the second accumulator: no double buffering
         const uint32_t acc = wide ? 0 : count & 1u, phase = (wide ? count : count >> 1) & 1u, mt = seg.tile / p.groups, n0 = (seg.tile % p.groups) * p.rpg;
         const bool whole = seg.k1 - seg.k0 == p.boxes;
-        const uint32_t row = mt * TILE_ROWS + et;
+        const uint32_t row = (PAIR ? 2 * mt + cta : mt) * TILE_ROWS + et;
         const float bias = row < p.out ? p.bias[row] : 0.0f;
         // the group's scales, once per segment into shared memory: a global load per value would be a chain of L2 latencies
         if (half == 0 && et < p.rpg) {
@@ -321,10 +333,10 @@ __device__ __forceinline__ void is_epilogue(const IsParams &p, bool wide, bool d
         uint64_t slot = et;
         if (!whole) {
             const uint64_t t0 = (uint64_t)seg.tile * p.boxes;
-            uint32_t c = (uint32_t)(t0 * gridDim.x / p.units);
-            while (c > 0 && unit_start(p.units, gridDim.x, c) > t0) c--;
-            while (unit_start(p.units, gridDim.x, c + 1) <= t0) c++;
-            slot += (uint64_t)c * p.rpg * TILE_ROWS;
+            uint32_t c = (uint32_t)(t0 * teams / p.units);
+            while (c > 0 && unit_start(p.units, teams, c) > t0) c--;
+            while (unit_start(p.units, teams, c + 1) <= t0) c++;
+            slot += (uint64_t)(PAIR ? 2 * c + cta : c) * p.rpg * TILE_ROWS;
         }
         unsigned long long *sums = p.sums + slot, *sums2 = p.sums2 + slot;
         is_epi_sync();
@@ -364,7 +376,10 @@ __device__ __forceinline__ void is_epilogue(const IsParams &p, bool wide, bool d
             }
         }
         tc_fence_before();
-        mbar_arrive(tempty0 + 8 * acc);                 // the accumulator may be overwritten
+        if (PAIR) {                                     // the accumulator may be overwritten
+            __syncwarp();
+            if (lane == 0) mbar_arrive_cluster(tempty0 + 8 * acc);
+        } else mbar_arrive(tempty0 + 8 * acc);
         if (!whole) __threadfence();
         is_epi_sync();                                  // (also: the scales of the next segment may replace these)
         const bool failed = !ok || *abort_flag;
@@ -377,7 +392,7 @@ __device__ __forceinline__ void is_epilogue(const IsParams &p, bool wide, bool d
         if (whole) continue;
         if (warp == 2 && lane == 0) {
             const uint32_t part = seg.k1 - seg.k0;
-            *s_last = !failed && atomicAdd(&p.counters[seg.tile], part) + part == p.boxes;
+            *s_last = !failed && atomicAdd(&p.counters[PAIR ? 2 * seg.tile + cta : seg.tile], part) + part == p.boxes;
         }
         is_epi_sync();
         if (*s_last) {
@@ -404,7 +419,7 @@ __device__ __forceinline__ void is_epilogue(const IsParams &p, bool wide, bool d
                 __stcg(sums2 + (uint64_t)rr * TILE_ROWS, 0ull);
                 is_finish<ACT>(p, n0 + rr, row, (double)bias + (double)v2 * s_scale[GROUP_ROWS + rr], s_scale[rr], v);
             }
-            if (warp == 2 && lane == 0) p.counters[seg.tile] = 0;
+            if (warp == 2 && lane == 0) p.counters[PAIR ? 2 * seg.tile + cta : seg.tile] = 0;
         }
         is_epi_sync();
     }
@@ -425,19 +440,22 @@ __device__ __forceinline__ uint32_t is_early_slots(const IsParams &p, const IsSe
 // compiler (a counted loop over the sets took 3 us of the 65 that 256 rows of a 4096-4096-1024 net take).  At 8 rows of INT4 a
 // block then takes the warp 480 cycles; it took 810 one at a time.
 struct IsBars { uint32_t rfull0, rempty0, afull0, aempty0, bfull0, bempty0, tfull0, tempty0; };
-template <uint32_t SETS, uint32_t G, uint32_t GB>
+template <uint32_t SETS, uint32_t G, uint32_t GB, bool PAIR>
 __device__ __forceinline__ void is_mma(const IsParams &p, IsSegment seg, const IsBars &bar, uint64_t a_desc0, uint64_t b_desc0, uint32_t tmem_base,
                                        uint32_t abort_addr, volatile int *abort_flag)
 {
     uint32_t as = 0, aph = 0, bs = 0, bph = 0, count = 0;      // G = 1: the boxes are the operand
-    const uint32_t b_step = p.C * 128u >> 4, slots = G == 1 ? p.RS : p.AS;
+    const uint32_t b_step = p.C * 128u >> (PAIR ? 5 : 4), slots = G == 1 ? p.RS : p.AS;
     const uint32_t full0 = G == 1 ? bar.rfull0 : bar.afull0, empty0 = G == 1 ? bar.rempty0 : bar.aempty0;
     if (SETS == 2) {
         const uint32_t early = is_early_slots(p, seg);
         for (uint32_t i = 0; i < early; i++) {
             mbar_wait_uniform(bar.bfull0 + 8 * bs, bph, abort_addr, p.status, 10);
             if (*abort_flag) return;
-            if (elect_one()) mbar_arrive(bar.bempty0 + 8 * bs);
+            if (elect_one()) {
+                mbar_arrive(bar.bempty0 + 8 * bs);
+                if (PAIR) mbar_arrive_cluster(mapa(bar.bempty0 + 8 * bs, 1));
+            }
             __syncwarp();
             if (++bs == p.BS) { bs = 0; bph ^= 1u; }
         }
@@ -466,9 +484,10 @@ __device__ __forceinline__ void is_mma(const IsParams &p, IsSegment seg, const I
                         for (uint32_t i = 0; i < GB; i++)
 #pragma unroll
                             for (uint32_t k = 0; k < 4; k++)
-                                umma_i8(d_tmem + set * p.C, da + (j + i) * (BOX_BYTES >> 4) + 2 * k, db + i * b_step + 2 * k, p.idesc, j + i + k ? 1u : accum);
-                        umma_commit(bar.bempty0 + 8 * bs);
-                        if (j + GB == G && set + 1 == SETS) umma_commit(empty0 + 8 * as);
+                                PAIR ? umma_i8_pair(d_tmem + set * p.C, da + (j + i) * (BOX_BYTES >> 4) + 2 * k, db + i * b_step + 2 * k, p.idesc, j + i + k ? 1u : accum)
+                                     : umma_i8(d_tmem + set * p.C, da + (j + i) * (BOX_BYTES >> 4) + 2 * k, db + i * b_step + 2 * k, p.idesc, j + i + k ? 1u : accum);
+                        PAIR ? umma_commit_pair(bar.bempty0 + 8 * bs) : umma_commit(bar.bempty0 + 8 * bs);
+                        if (j + GB == G && set + 1 == SETS) PAIR ? umma_commit_pair(empty0 + 8 * as) : umma_commit(empty0 + 8 * as);
                     }
                     __syncwarp();
                     if (++bs == p.BS) { bs = 0; bph ^= 1u; }
@@ -477,11 +496,14 @@ __device__ __forceinline__ void is_mma(const IsParams &p, IsSegment seg, const I
             accum = 1;
             if (++as == slots) { as = 0; aph ^= 1u; }
         }
-        if (elect_one()) umma_commit(bar.tfull0 + 8 * acc);
+        if (elect_one()) PAIR ? umma_commit_pair(bar.tfull0 + 8 * acc) : umma_commit(bar.tfull0 + 8 * acc);
         __syncwarp();
     }
 }
 
+// PAIR: clusters of two.  A pair's tiles are 256 weight rows high; each CTA has its own 128 (boxes, unpacking, accumulator, epilogue as alone) and
+// half of the digit columns, and the first one's MMA warp issues for both.  The barriers it waits on live in its shared memory.
+template <bool PAIR>
 __global__ void __launch_bounds__(IS_THREADS, 1)
 spg_istream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const IsParams p)
 {
@@ -490,7 +512,7 @@ spg_istream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     const uint32_t base = (raw + 1023u) & ~1023u;
     uint8_t *smem = is_smem_raw + (base - raw);
     // layout: box ring | operand ring (absent for INT8) | digit ring | barriers | flags | scales of a group, both sets
-    const uint32_t b_bytes = p.C * 128u;
+    const uint32_t b_bytes = p.C * (PAIR ? 64u : 128u);
     const uint32_t a_off = p.RS * BOX_BYTES;
     const uint32_t b_off = a_off + (p.direct ? 0u : p.AS * p.G * BOX_BYTES);
     const uint32_t bar_off = b_off + p.BS * p.GB * b_bytes;
@@ -505,30 +527,34 @@ spg_istream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     double *s_scale = reinterpret_cast<double *>(smem + flag_off + 16);
 
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
+    const uint32_t cta = PAIR ? cluster_rank() : 0u, team = PAIR ? blockIdx.x >> 1 : blockIdx.x, teams = PAIR ? gridDim.x >> 1 : gridDim.x;
     uint32_t tmem_cols = 32;
     while (tmem_cols < 2 * p.C) tmem_cols *= 2;          // two accumulators, 512 columns at most
 
     if (tid == 0) {
         for (uint32_t s = 0; s < p.RS; s++) { mbar_init(rfull0 + 8 * s, 1); mbar_init(rempty0 + 8 * s, p.direct ? 1 : IS_CONV_WARPS); }
-        for (uint32_t s = 0; s < p.AS; s++) { mbar_init(afull0 + 8 * s, IS_CONV_WARPS / p.AS); mbar_init(aempty0 + 8 * s, 1); }
+        for (uint32_t s = 0; s < p.AS; s++) { mbar_init(afull0 + 8 * s, (PAIR ? 2 : 1) * IS_CONV_WARPS / p.AS); mbar_init(aempty0 + 8 * s, 1); }
         for (uint32_t s = 0; s < p.BS; s++) { mbar_init(bfull0 + 8 * s, 1); mbar_init(bempty0 + 8 * s, 1); }
-        for (uint32_t a = 0; a < 2; a++) { mbar_init(tfull0 + 8 * a, 1); mbar_init(tempty0 + 8 * a, 32 * IS_EPI_WARPS); }
+        for (uint32_t a = 0; a < 2; a++) { mbar_init(tfull0 + 8 * a, 1); mbar_init(tempty0 + 8 * a, PAIR ? 2 * IS_EPI_WARPS : 32 * IS_EPI_WARPS); }
         *abort_flag = 0;
         mbar_fence_init();
         prefetch_map(&map_w);
         prefetch_map(&map_x);
     }
-    if (warp == 1) tmem_alloc(smem_u32(tmem_slot), tmem_cols);
+    if (warp == 1) PAIR ? tmem_alloc_pair(smem_u32(tmem_slot), tmem_cols) : tmem_alloc(smem_u32(tmem_slot), tmem_cols);
     tc_fence_before();
-    __syncthreads();
+    if (PAIR) cluster_sync();                            // both CTAs' barriers exist before anyone arrives on them
+    else __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    const uint32_t lead_rfull0 = PAIR ? mapa(rfull0, 0) : rfull0, lead_bfull0 = PAIR ? mapa(bfull0, 0) : bfull0;
+    const uint32_t lead_tempty0 = PAIR ? mapa(tempty0, 0) : tempty0;
     spg_grid_trigger();
 
     const uint32_t abort_addr = smem_u32(const_cast<int *>(abort_flag));
     IsSegment seg;
-    seg.u = unit_start(p.units, gridDim.x, blockIdx.x);
-    seg.end = unit_start(p.units, gridDim.x, blockIdx.x + 1);
+    seg.u = unit_start(p.units, teams, team);
+    seg.end = unit_start(p.units, teams, team + 1);
 
     if (warp == 0) {
         // ------------------------------ weight boxes ------------------------------
@@ -536,14 +562,19 @@ spg_istream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         // before its first bounded wait, which would otherwise count somebody else's running time.
         uint32_t rs = 0, rph = 0;
         while (is_next_segment(p, seg)) {
-            const int r0 = (int)(seg.tile / p.groups * TILE_ROWS);
+            const int r0 = (int)((PAIR ? 2 * (seg.tile / p.groups) + cta : seg.tile / p.groups) * TILE_ROWS);
             for (uint32_t b = seg.k0; b < seg.k1; b++) {
                 if (rs == 0 && rph) spg_grid_wait();
                 mbar_wait_uniform(rempty0 + 8 * rs, rph ^ 1u, abort_addr, p.status, 1);
                 if (*abort_flag) goto is_role_done;
                 if (elect_one()) {
-                    mbar_expect_tx(rfull0 + 8 * rs, BOX_BYTES);
-                    tma_load_2d(base + rs * BOX_BYTES, &map_w, rfull0 + 8 * rs, (int)(b * 128u), r0);
+                    if (PAIR && p.direct) {              // the boxes are the operand: the issuer waits for both CTAs'
+                        if (cta == 0) mbar_expect_tx(rfull0 + 8 * rs, 2 * BOX_BYTES);
+                        tma_load_2d_pair(base + rs * BOX_BYTES, &map_w, lead_rfull0 + 8 * rs, (int)(b * 128u), r0);
+                    } else {
+                        mbar_expect_tx(rfull0 + 8 * rs, BOX_BYTES);
+                        tma_load_2d(base + rs * BOX_BYTES, &map_w, rfull0 + 8 * rs, (int)(b * 128u), r0);
+                    }
                 }
                 __syncwarp();
                 if (++rs == p.RS) { rs = 0; rph ^= 1u; }
@@ -556,9 +587,12 @@ spg_istream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
             mbar_wait_uniform(bempty0 + 8 * bs, bph ^ 1u, abort_addr, p.status, 2);
             if (*abort_flag) return;
             if (elect_one()) {
-                mbar_expect_tx(bfull0 + 8 * bs, p.GB * b_bytes);
-                for (uint32_t i = 0; i < p.GB; i++)
-                    tma_load_2d(base + b_off + (bs * p.GB + i) * b_bytes, &map_x, bfull0 + 8 * bs, (int)((kb + i) * 128u), (int)row);
+                if (cta == 0) mbar_expect_tx(bfull0 + 8 * bs, (PAIR ? 2 : 1) * p.GB * b_bytes);
+                for (uint32_t i = 0; i < p.GB; i++) {
+                    const uint32_t dst = base + b_off + (bs * p.GB + i) * b_bytes;
+                    if (PAIR) tma_load_2d_pair(dst, &map_x, lead_bfull0 + 8 * bs, (int)((kb + i) * 128u), (int)(row + cta * (p.C / 2)));
+                    else tma_load_2d(dst, &map_x, bfull0 + 8 * bs, (int)((kb + i) * 128u), (int)row);
+                }
             }
             __syncwarp();
             if (++bs == p.BS) { bs = 0; bph ^= 1u; }
@@ -584,7 +618,8 @@ spg_istream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         const IsBars bar = { rfull0, rempty0, afull0, aempty0, bfull0, bempty0, tfull0, tempty0 };
         const uint64_t a_desc0 = smem_desc_sw128(p.direct ? base : base + a_off), b_desc0 = smem_desc_sw128(base + b_off);
         spg_grid_wait();
-#define IS_MMA(SETSV, GV, GBV) is_mma<SETSV, GV, GBV>(p, seg, bar, a_desc0, b_desc0, tmem_base, abort_addr, abort_flag)
+        if (cta) goto is_role_done;                      // the first CTA issues for both
+#define IS_MMA(SETSV, GV, GBV) is_mma<SETSV, GV, GBV, PAIR>(p, seg, bar, a_desc0, b_desc0, tmem_base, abort_addr, abort_flag)
         const bool wide = is_any_wide(p, lane);
         if (p.direct) { if (wide) IS_MMA(2, 1, 1); else IS_MMA(1, 1, 1); }
         else if (p.GB == 1) { if (wide) IS_MMA(2, 2, 1); else IS_MMA(1, 2, 1); }
@@ -599,7 +634,7 @@ spg_istream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         if (!p.direct) {
             const uint32_t tiles = p.AS * p.G, wpg = IS_CONV_WARPS / tiles, TG = 32u * wpg;
             const uint32_t cw = warp - IS_CONV_WARP0, grp = cw / wpg, ctg = (cw % wpg) * 32u + lane;
-            const uint32_t afull = afull0 + 8 * (grp / p.G), aempty = aempty0 + 8 * (grp / p.G);
+            const uint32_t afull = PAIR ? mapa(afull0 + 8 * (grp / p.G), 0) : afull0 + 8 * (grp / p.G), aempty = aempty0 + 8 * (grp / p.G);
             uint32_t rs = 0, rph = 0, as = 0, aph = 0;
             uint8_t *atile = smem + a_off + grp * BOX_BYTES;
             spg_grid_wait();
@@ -646,7 +681,7 @@ spg_istream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                             }
                             fence_async_smem();          // the tensor core reads the tile through the async proxy
                             __syncwarp();
-                            if (lane == 0) mbar_arrive(afull);
+                            if (lane == 0) PAIR ? mbar_arrive_cluster(afull) : mbar_arrive(afull);
                         }
                         if (++as == tiles) { as = 0; aph ^= 1u; }
                     }
@@ -666,7 +701,7 @@ spg_istream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         is_epi_sync();
         const int found = *s_last;
         is_epi_sync();
-#define IS_EPI(ACTV) is_epilogue<ACTV>(p, found & 1, found & 2, seg, tmem_base, tfull0, tempty0, abort_flag, s_last, s_scale, warp, lane)
+#define IS_EPI(ACTV) is_epilogue<ACTV, PAIR>(p, found & 1, found & 2, seg, tmem_base, tfull0, lead_tempty0, abort_flag, s_last, s_scale, warp, lane)
         switch (p.act) {
             case SPG_ACT_RELU:    IS_EPI(SPG_ACT_RELU); break;
             case SPG_ACT_LEAKY:   IS_EPI(SPG_ACT_LEAKY); break;
@@ -685,7 +720,8 @@ is_role_done:
         if (tid == 0) for (int i = 0; i < 256; i++) __nanosleep(1000);
         __syncthreads();
     }
-    if (warp == 1) { tc_fence_after(); tmem_free(tmem_base, tmem_cols); }
+    if (PAIR) cluster_sync();                            // neither CTA leaves while the other's products read its shared memory or its warps arrive there
+    if (warp == 1) { tc_fence_after(); PAIR ? tmem_free_pair(tmem_base, tmem_cols) : tmem_free(tmem_base, tmem_cols); }
 }
 
 // ---- host side ---------------------------------------------------------------------------------------------------------
@@ -694,7 +730,7 @@ struct IsPlan {
     uint32_t groups, rpg, C, kbr, boxes, ld, m_tiles, tiles, RS, AS, BS, G, GB, grid;
     uint64_t units;
     size_t operand_bytes, smem;
-    bool direct, ok;
+    bool direct, pair, ok;
 };
 
 constexpr size_t IS_HEAD = 256 + 4 * MAX_TILES;        // status word, counters; zero between calls, like the sums behind them
@@ -709,20 +745,28 @@ IsPlan is_plan(const spgk_layer *L, uint32_t N, uint32_t sms)
     if ((L->in * bits) % 128 || ((uintptr_t)L->w & 15u)) return pl;       // TMA: 16-byte aligned packed rows
     pl.groups = (N + GROUP_ROWS - 1) / GROUP_ROWS;
     pl.rpg = ((N + pl.groups - 1) / pl.groups + 3u) & ~3u;
+    // Pairs of CTAs where the digits are most of what an SM draws from L2 (more than 32 rows a group; up to 32 rows pairs were level or behind by 7 %)
+    // and the layer is a long one: 32 blocks for an SM, or 8192 inputs (1024-4096-4096-1000, 2 to 28 blocks an SM: 52.4 us in pairs against 51.3 at
+    // 64 rows; 8192 x 1000, 3.4 blocks: the net around it 166 us against 171 with this layer alone on single CTAs).  INT8, which 64 rows stream
+    // at the rate of HBM, only from the second group on (40 rows: 170 against 167 us, 72 rows: 253 against 261).
+    const uint64_t blocks = (uint64_t)((L->out + TILE_ROWS - 1) / TILE_ROWS) * ((L->in + 127u) / 128u) * pl.groups;
+    pl.pair = pl.rpg > IS_PAIR_ROWS && (blocks >= (uint64_t)IS_PAIR_BLOCKS * sms || L->in >= 8192u) && L->out > TILE_ROWS && sms >= 2 && (prec != SPG_P_I8 || pl.groups > 1);
+    if (pl.pair) pl.rpg = (pl.rpg + 7u) & ~7u;                            // (a pair's product takes multiples of 32 columns)
     pl.C = 4 * pl.rpg;
     pl.kbr = 8u / bits;
     pl.direct = prec == SPG_P_I8;
     pl.boxes = (L->in * bits + 1023u) / 1024u;
     pl.ld = pl.boxes * pl.kbr * 128u;
-    pl.m_tiles = (L->out + TILE_ROWS - 1) / TILE_ROWS;
+    const uint32_t high = pl.pair ? 2 * TILE_ROWS : TILE_ROWS;
+    pl.m_tiles = (L->out + high - 1) / high;
     pl.tiles = pl.m_tiles * pl.groups;
-    if (pl.tiles > MAX_TILES) return pl;
+    if (pl.tiles > (pl.pair ? MAX_TILES / 2 : MAX_TILES)) return pl;     // (a pair's tile has two counters)
     pl.units = (uint64_t)pl.tiles * pl.boxes;
     // one CTA per SM, but a tile in about four pieces at most: the sum over more of them costs more than they save
     const uint64_t want = (uint64_t)pl.tiles * (pl.boxes < 4 ? pl.boxes : 4);
-    pl.grid = want < sms ? (uint32_t)want : sms;
+    pl.grid = pl.pair ? 2 * (want < sms / 2 ? (uint32_t)want : sms / 2) : want < sms ? (uint32_t)want : sms;
     // rings: operand tiles in two slots of G blocks, digit tiles up to 96 KB (in pairs up to 32 rows), boxes with the rest
-    const uint32_t b_bytes = pl.C * 128u;
+    const uint32_t b_bytes = pl.C * (pl.pair ? 64u : 128u);
     pl.G = pl.direct ? 1 : 2;
     pl.AS = pl.direct ? 1 : 2;
     pl.GB = pl.direct || b_bytes > 16384 ? 1 : 2;
@@ -780,7 +824,7 @@ IsScratch is_scratch(const spgk_layer *layers, uint32_t count, uint32_t N, uint3
         const IsPlan pl = is_plan(&layers[l], N, sms);
         if (!pl.ok) return s;
         if (pl.operand_bytes > operand) operand = pl.operand_bytes;
-        rows = (size_t)pl.groups * pl.rpg;
+        if ((size_t)pl.groups * pl.rpg > rows) rows = (size_t)pl.groups * pl.rpg;
     }
     if (!rows) return s;
     s.sums = IS_HEAD;
@@ -821,7 +865,8 @@ int spgk_istream_forward(const spgk_layer *layers, uint32_t count, const float *
         int dev = 0;
         SPGK_CUDA(cudaGetDevice(&dev));
         rc = once.run(dev, [&]() -> int {
-            SPGK_CUDA(cudaFuncSetAttribute(spg_istream_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
+            SPGK_CUDA(cudaFuncSetAttribute(spg_istream_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
+            SPGK_CUDA(cudaFuncSetAttribute(spg_istream_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
             return SPGK_OK;
         });
         if (rc) return rc;
@@ -839,7 +884,7 @@ int spgk_istream_forward(const spgk_layer *layers, uint32_t count, const float *
         auto stage = L->precision == SPG_P_I8 ? spg_is_stage_kernel<SPG_P_I8> : L->precision == SPG_P_I4 ? spg_is_stage_kernel<SPG_P_I4> : spg_is_stage_kernel<SPG_P_I2>;
         CUtensorMap map_w, map_x;
         if ((rc = is_map(L->w, (uint64_t)L->in * spg_bits_per_elem(L->precision) / 8, L->out, TILE_ROWS, &map_w))) return rc;
-        if ((rc = is_map(operand, pl.ld, 2 * (uint64_t)pl.groups * pl.C, pl.C, &map_x))) return rc;
+        if ((rc = is_map(operand, pl.ld, 2 * (uint64_t)pl.groups * pl.C, pl.pair ? pl.C / 2 : pl.C, &map_x))) return rc;
         SPGK_CUDA(spg_launch_chained(stage, dim3(pl.groups * pl.rpg), dim3(STAGE_THREADS), 0, s, xin, xld, N, L->in, pl.ld, vec, operand, row_scale, base + sc.wide));
         if ((rc = spgk_check_launch("spg_is_stage_kernel"))) return rc;
         IsParams p{};
@@ -855,8 +900,19 @@ int spgk_istream_forward(const spgk_layer *layers, uint32_t count, const float *
         p.counters = reinterpret_cast<uint32_t *>(base + 256);
         p.sums = reinterpret_cast<unsigned long long *>(base + sc.sums);
         p.sums2 = reinterpret_cast<unsigned long long *>(base + sc.sums2);
-        p.idesc = idesc_i8(pl.C);
-        SPGK_CUDA(spg_launch_chained(spg_istream_kernel, dim3(pl.grid), dim3(IS_THREADS), pl.smem, s, map_w, map_x, p));
+        p.idesc = idesc_i8(pl.pair ? 2 * TILE_ROWS : TILE_ROWS, pl.C);
+        if (pl.pair) {
+            cudaLaunchConfig_t cfg = {};
+            cfg.gridDim = dim3(pl.grid); cfg.blockDim = dim3(IS_THREADS); cfg.dynamicSmemBytes = pl.smem; cfg.stream = s;
+            cudaLaunchAttribute attr[2];
+            attr[0].id = cudaLaunchAttributeClusterDimension;
+            attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+            attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+            attr[1].val.programmaticStreamSerializationAllowed = 1;
+            cfg.attrs = attr; cfg.numAttrs = 2;
+            SPGK_CUDA(cudaLaunchKernelEx(&cfg, spg_istream_kernel<true>, map_w, map_x, p));
+        } else
+            SPGK_CUDA(spg_launch_chained(spg_istream_kernel<false>, dim3(pl.grid), dim3(IS_THREADS), pl.smem, s, map_w, map_x, p));
         if ((rc = spgk_check_launch("spg_istream_kernel"))) return rc;
         xin = ys[l]; xld = L->out;
     }
