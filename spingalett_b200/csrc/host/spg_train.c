@@ -42,8 +42,8 @@ typedef struct {
     size_t cap[12];                          /* bytes held by each of the buffers above, in declaration order */
     uint64_t np;                             /* parameters the flat buffers were sized for */
     void *stream;                            /* a stream of the library's own for nets that sit on the legacy default stream */
-    float *h_words;                          /* page-locked: status words (page-locking a kilobyte takes up to 2 ms, giving it back 0.6) */
-    uint32_t *h_order[2];                    /* page-locked: the shuffled orders of this epoch and the next, on their way to `idx` */
+    float *h_words;                          /* page-locked block: status words (page-locking a kilobyte takes up to 2 ms, giving it back 0.6) ... */
+    uint32_t *h_order[2];                    /* ... and in it the shuffled orders of this epoch and the next, on their way to `idx` */
     void *order_ev[2];
     size_t order_cap;                        /* samples the orders have room for */
 } train_state;
@@ -117,25 +117,25 @@ static void state_free(train_state *t)
     for (size_t i = 0; i < sizeof bufs / sizeof bufs[0]; i++) spgk_free(bufs[i]);
     spgk_stream_destroy(t->stream);
     spgk_host_free(t->h_words);
-    for (int i = 0; i < 2; i++) {
-        spgk_host_free(t->h_order[i]);
-        if (t->order_ev[i]) spgk_event_destroy(t->order_ev[i]);
-    }
+    for (int i = 0; i < 2; i++) if (t->order_ev[i]) spgk_event_destroy(t->order_ev[i]);
     free(t);
 }
 
-/* room for the shuffled orders of two epochs */
-static int orders_reserve(train_state *t, uint32_t samples)
+/* the page-locked block: 1 KB of words, then room for the shuffled orders of two epochs (0 samples: none) */
+static int pinned_reserve(train_state *t, uint32_t samples)
 {
-    for (int i = 0; i < 2; i++) {
-        int rc;
-        if (t->order_cap < samples) { spgk_host_free(t->h_order[i]); t->h_order[i] = NULL; }
+    int rc;
+    if (t->h_words && t->order_cap < samples) { spgk_host_free(t->h_words); t->h_words = NULL; }
+    if (!t->h_words) {
         void *h = NULL;
-        if (!t->h_order[i] && (rc = spg_map_kernel_error(spgk_host_alloc(&h, (size_t)samples * 4), "train: shuffle order"))) { t->order_cap = 0; return rc; }
-        if (h) t->h_order[i] = h;
-        if (!t->order_ev[i] && (rc = spg_map_kernel_error(spgk_event_create(&t->order_ev[i]), "train: shuffle order"))) return rc;
+        t->order_cap = 0;
+        if ((rc = spg_map_kernel_error(spgk_host_alloc(&h, 1024 + 2 * (size_t)samples * 4), "train: pinned words"))) return rc;
+        t->h_words = h; t->order_cap = samples;
     }
-    if (t->order_cap < samples) t->order_cap = samples;
+    for (int i = 0; i < 2; i++) {
+        t->h_order[i] = (uint32_t *)(void *)(t->h_words + 256) + (size_t)i * t->order_cap;
+        if (samples && !t->order_ev[i] && (rc = spg_map_kernel_error(spgk_event_create(&t->order_ev[i]), "train: shuffle order"))) return rc;
+    }
     return SPINGALETT_OK;
 }
 
@@ -316,18 +316,13 @@ void train_struct_arguments(TrainArgs a)
         if (state_reserve(t, 8, (void **)&t->batch_x, (size_t)batch * in0 * 4, "train: batch inputs") ||
             state_reserve(t, 9, (void **)&t->batch_t, (size_t)batch * outw * 4, "train: batch targets")) goto fail;
         if (state_reserve(t, 10, (void **)&t->idx, (size_t)a.sample_count * 4, "train: shuffle order")) goto fail;
-        if (orders_reserve(t, a.sample_count)) goto fail;
         order = malloc((size_t)a.sample_count * sizeof *order);
         if (!order) { spg_set_error(SPINGALETT_ERR_ALLOC, "Mini-batch allocation failed"); goto fail; }
         for (uint32_t i = 0; i < a.sample_count; i++) order[i] = i;
     }
     float *d_loss = t->words, *d_sumsq = t->words + 2, *d_agree = t->words + 8;
     int *d_flag = (int *)(t->words + 1);
-    if (!t->h_words) {
-        void *h = NULL;
-        DEV(spgk_host_alloc(&h, 1024), "train: pinned words");
-        t->h_words = h;
-    }
+    if (pinned_reserve(t, mini ? a.sample_count : 0)) goto fail;
     float *const h_pinned = t->h_words;
 
     /* the host arrays are the truth between calls (callers may edit them): upload them every time */
