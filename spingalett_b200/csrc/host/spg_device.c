@@ -124,7 +124,7 @@ void spg_dev_release(spg_net *n)
     for (int i = 0; i < 2; i++) { spgk_free(n->d_operand[i]); n->d_operand[i] = NULL; n->operand_bytes[i] = 0; }
     spgk_free(n->d_ws_scratch); n->d_ws_scratch = NULL; n->ws_scratch_bytes = 0;
     spgk_free(n->d_is_scratch); n->d_is_scratch = NULL; n->is_scratch_bytes = 0; n->is_pending = false;
-    spgk_free(n->d_rep_idx); n->d_rep_idx = NULL; n->rep_idx_bytes = 0;
+    spgk_free(n->d_rep_idx); n->d_rep_idx = NULL; n->rep_idx_bytes = 0; n->count_clean = false;
     n->auto_calibrated = false;
     n->auto_calls = 0;
     n->bf16_fits_f16 = 0;
@@ -844,10 +844,10 @@ int spg_dev_forward_large(spg_net *n, const float *d_x, uint32_t N, float *d_out
 
     int rc;
     /* the list of rows stands behind a head of 256 bytes: [0] the number of rows, which every call leaves at zero, [8] the calibration's word */
-    const uint32_t *const list_before = n->d_rep_idx;
-    if ((rc = reserve((void **)&n->d_rep_idx, &n->rep_idx_bytes, (size_t)N * 4 + 256, "repair index"))) return rc;
+    const size_t list_bytes = (size_t)N * 4 + 256;
+    if (n->rep_idx_bytes < list_bytes) n->count_clean = false;       /* (by its size: a list that has grown may lie where it lay before) */
+    if ((rc = reserve((void **)&n->d_rep_idx, &n->rep_idx_bytes, list_bytes, "repair index"))) return rc;
     uint32_t *const d_count = n->d_rep_idx, *const d_rows = n->d_rep_idx + 64;
-    if (n->d_rep_idx != list_before) n->count_clean = false;
     /* (a call that is being captured runs later, and more than once, whatever happens in between: it clears the count itself) */
     const bool captured = spgk_stream_capturing(n->stream) != 0, clean_before = n->count_clean;
     if ((!clean_before || captured) && (rc = spg_map_kernel_error(spgk_memset(d_count, 0, 4, n->stream), "repair count clear"))) return rc;
