@@ -470,6 +470,7 @@ int spg_dev_forward_small(spg_net *n, const float *d_x, uint32_t ldx, uint32_t N
         /* up to 8 rows: the mma.sync GEMV first (measured faster there), then the tcgen05 streaming kernel;
          * more rows: the streaming kernel only */
         const char *used = "gemv";
+        const spgk_layer *streams = NULL;
         int k = SPGK_E_UNSUPPORTED;
         prof_mark(n);
         if (N <= SPGK_GEMV_MAX_BATCH) {
@@ -478,10 +479,12 @@ int spg_dev_forward_small(spg_net *n, const float *d_x, uint32_t ldx, uint32_t N
         }
         if (k == SPGK_E_UNSUPPORTED) {
             used = "wstream";
-            k = spgk_layer_wstream(L, next, operand, n->d_operand[(l + 1) & 1], x, xld, y, L->out, N, n->d_ws_scratch, n->stream);
+            /* the next layer's operand too, if it comes here: the buffers have room for the layers that do */
+            streams = next && !(N <= SPGK_GEMV_MAX_BATCH && spgk_gemv_scratch_bytes(next, N)) ? next : NULL;
+            k = spgk_layer_wstream(L, streams, operand, n->d_operand[(l + 1) & 1], x, xld, y, L->out, N, n->d_ws_scratch, n->stream);
             if (k == SPGK_OK) n->ws_pending = true;
         }
-        operand = (k == SPGK_OK && used[0] == 'w' && next && spgk_wstream_stages_next(L, next, N)) ? n->d_operand[(l + 1) & 1] : NULL;
+        operand = (k == SPGK_OK && streams && spgk_wstream_stages_next(L, streams, N)) ? n->d_operand[(l + 1) & 1] : NULL;
         staged = (k == SPGK_OK && used[0] == 'g' && next && spgk_gemv_chain_stages_next(L, next, N)) ? n->d_staged[(l + 1) & 1] : NULL;
         prof_mark(n);
         if (k == SPGK_E_UNSUPPORTED) {
