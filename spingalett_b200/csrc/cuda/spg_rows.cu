@@ -62,6 +62,18 @@ template <int PREC> __device__ __forceinline__ void decode8(const void *w, uint6
     }
 }
 
+// One sum with every product and sum in 64 bits.  Integer weights are multiplied before their scale: in fp32 a sum of four is then out of range for inputs
+// from 6.7e35 on, where a weight times an input is not.
+template <int PREC> __device__ __forceinline__ double dot_in_double(const void *w, uint64_t row, const float *x, uint32_t in, uint32_t lane)
+{
+    double sum = 0.0;
+#pragma unroll 1
+    for (uint32_t k = lane; k < in; k += 32) sum += (double)spg_decode_elem(w, row + k, PREC) * (double)x[k];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    return sum;
+}
+
 // Output j for rows n0 .. n0 + NB - 1 (rows from N on read as the last one): the sums, in every lane.  `wait`: the input is what
 // the launch before this one writes, and nobody has waited for it yet.
 template <int PREC, int NB> __device__ __forceinline__ void dot(const RowsParams &p, uint32_t j, uint32_t n0, bool wait, uint32_t lane, double (&sum)[NB])
@@ -113,6 +125,8 @@ template <int PREC, int NB> __device__ __forceinline__ void dot(const RowsParams
         sum[b] = acc[b][0] + acc[b][1];
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) sum[b] += __shfl_xor_sync(0xffffffffu, sum[b], o);
+        if constexpr (PREC >= SPG_P_I8)
+            if (!isfinite(sum[b])) sum[b] = dot_in_double<PREC>(p.w, row, p.x + (uint64_t)min(n0 + b, p.N - 1) * p.ldx, p.in, lane);      // (the same in every lane)
     }
 }
 

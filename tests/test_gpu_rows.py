@@ -70,6 +70,37 @@ def test_small_net_against_float64(spg, prec, widths):
             assert np.all(got[0][n] == -3.0) and np.all(got[1][n] == -3.0)
 
 
+@pytest.mark.parametrize("prec", [3, 4, 5])
+@pytest.mark.parametrize("n", [1, 4, 7])
+def test_integer_weights_times_large_inputs(spg, prec, n):
+    """Inputs up to 1e38: a stored weight times an input is out of fp32's range, a weight times an input is not.  Rows with values that are not
+    finite keep them to themselves."""
+    import torch
+    lib = spg.lib()
+    lib.spgk_rows_forward.argtypes = [C.POINTER(spg.abi.KLayer), C.c_uint32, C.c_void_p, C.c_uint32, C.POINTER(C.c_void_p), C.c_uint32, C.c_void_p]
+    rng = np.random.default_rng(prec * 10 + n)
+    inn, out = 1100, 41
+    raw, q = matrix(rng, out, inn, prec)
+    scale = float(np.float32(1 / (np.abs(q).max() * inn)))          # no sum is larger than its largest input
+    bias = rng.standard_normal(out).astype(np.float32)
+    dw, db = torch.from_numpy(np.concatenate([raw, np.zeros(64, np.uint8)])).cuda(), torch.from_numpy(bias).cuda()
+    layer = spg.abi.KLayer(dw.data_ptr(), db.data_ptr(), scale, inn, out, prec, 6)
+    x = (rng.standard_normal((n, inn)) * 2e37).astype(np.float32)
+    x[n // 2] *= np.float32(1e-37)
+    x[n - 1, :2] = np.float32(1e38), np.float32(-1e38)
+    if n == 7:
+        x[2, 5], x[4, 6] = np.inf, np.nan
+    w = np.asarray(q, np.float64).reshape(out, inn) * scale
+    dx, y = torch.from_numpy(x).cuda(), torch.full((n + 1, out), -3.0, device="cuda")
+    assert lib.spgk_rows_forward(C.byref(layer), 1, dx.data_ptr(), inn, (C.c_void_p * 1)(y.data_ptr()), n, None) == 0
+    torch.cuda.synchronize()
+    got, a = y.cpu().numpy(), x.astype(np.float64)
+    good = np.isfinite(x).all(1)
+    want = a[good] @ w.T + bias
+    assert np.all(np.abs(got[:n][good] - want) <= 2.0 ** -22 * (np.abs(a[good]) @ np.abs(w).T) + 2.0 ** -23 * np.abs(want))
+    assert not np.isfinite(got[:n][~good]).any() and np.all(got[n] == -3.0)
+
+
 @pytest.mark.parametrize("topo,last", [([784, 512, 10], 5), ([301, 77, 128], 5), ([33, 40, 129], 5), ([7, 1], 0)])
 def test_a_sample_from_host_memory_gives_what_a_batch_of_one_gives(spg, topo, last):
     """forward() (input and outputs of every layer through page-locked memory; wider softmax rows by copies) against forward_batch."""
