@@ -107,7 +107,7 @@ SPGK_API int spgk_rows_forward(const spgk_layer *layers, uint32_t count, const f
                                void *stream);
 /* One sample the same way, from and to page-locked host memory: host and dev hold the input and then every layer's outputs, one behind the
  * other; the input is read from host, the outputs are written to dev and to host (there once the stream has been waited for).
- * SPGK_E_UNSUPPORTED, and nothing launched, for a softmax of more than 128 outputs. */
+ * SPGK_E_UNSUPPORTED, and nothing launched, for a softmax that needs a launch of its own (more than 128 outputs, or too many products for a CTA). */
 #define SPGK_ROWS_MAX_LAYERS 64u
 SPGK_API int spgk_rows_sample(const spgk_layer *layers, uint32_t count, float *host, float *dev, void *stream);
 

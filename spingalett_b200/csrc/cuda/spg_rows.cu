@@ -7,7 +7,8 @@
 // registers, decoded, before the layer before it has ended (programmatic dependent launch); then come the input (8 neighbouring
 // values a lane, all loads of a round in flight), the products, four of them added in fp32 and the fours in 64 bits, and a shuffle
 // tree.  (Every product in 64 bits: as accurate as the last rounding allows, and 2 to 4 us slower from six rows on, a conversion
-// runs at 14 a cycle and SM.)
+// runs at 14 a cycle and SM.)  A warp takes 1.2 to 1.7 us for 1024 elements of a row, so rows of more than 2048 are shared by four or eight
+// warps: one row of 65536-64-10 INT8 109 -> 18 us, of 4096-10 8.8 -> 5.
 //
 // What bounds it: 3 us a layer of launch, two L2 latencies and the tree; beyond four rows the loads of the inputs.  Before (the
 // weight-streaming GEMV, made to keep HBM busy, or the general kernel where rows are no multiple of 16 bytes) and now, us a call:
@@ -22,17 +23,24 @@
 
 namespace {
 
-constexpr uint32_t GROUP = 8, ROUNDS = 4, SPAN = 32 * GROUP * ROUNDS;      // neighbours a lane takes, groups a lane has in flight, elements a warp has
+constexpr uint32_t GROUP = 8, TURN = 32 * GROUP, SPAN = 4 * TURN;          // neighbours a lane takes, elements that a warp takes side by side, and that it has in flight
+constexpr uint32_t LONG_ROW = 2 * SPAN;                                    // inputs beyond which several warps share an output
 constexpr uint32_t LAST_WARPS = 32, LAST_MAX = 128;                        // the layer whose row softmax is finished in the CTA
 
 struct RowsParams {
-    const void *w; const float *bias; float scale; uint32_t in, out; int act;
+    const void *w; const float *bias; double scale; uint32_t in, out; int act;
     const float *x; uint32_t ldx; float *y; uint32_t ldy; uint32_t N;
     float *copy;                           // a second place for the outputs of row 0 (page-locked host memory), or null
     uint32_t vec_w, vec_x;                 // groups of eight weights / inputs lie on their own alignment
+    uint32_t parts;                        // warps that share an output: 1, 2, 4 or 8
 };
 
-// the weights e .. e + 7 of the matrix, as stored
+// Integer weights are multiplied before their scale, which a large input times a weight of 128 would not survive in fp32: they are taken as
+// multiples of 2^-9, 2^-5 and 2^-3 (INT8, INT4, INT2), so that four products add up to no more than the largest input; the scale makes up for it.
+template <int PREC> constexpr int UNIT = PREC == SPG_P_I8 ? 9 : PREC == SPG_P_I4 ? 5 : PREC == SPG_P_I2 ? 3 : 0;
+template <int PREC> constexpr float ONE = 1.0f / (float)(1 << UNIT<PREC>);
+
+// the weights e .. e + 7 of the matrix, in those units
 template <int PREC> __device__ __forceinline__ void decode8(const void *w, uint64_t e, float (&q)[8])
 {
     if constexpr (PREC == SPG_P_F32) {
@@ -50,55 +58,44 @@ template <int PREC> __device__ __forceinline__ void decode8(const void *w, uint6
     } else if constexpr (PREC == SPG_P_I8) {
         const uint2 v = __ldg(reinterpret_cast<const uint2 *>(reinterpret_cast<const int8_t *>(w) + e));
 #pragma unroll
-        for (int i = 0; i < 8; i++) q[i] = (float)((int)((i < 4 ? v.x : v.y) << (24 - 8 * (i & 3))) >> 24);
+        for (int i = 0; i < 8; i++) q[i] = (float)((int)((i < 4 ? v.x : v.y) << (24 - 8 * (i & 3))) >> 24) * ONE<PREC>;
     } else if constexpr (PREC == SPG_P_I4) {
         const uint32_t v = __ldg(reinterpret_cast<const uint32_t *>(reinterpret_cast<const uint8_t *>(w) + (e >> 1)));
 #pragma unroll
-        for (int i = 0; i < 8; i++) q[i] = (float)((int)(v << (28 - 4 * i)) >> 28);
+        for (int i = 0; i < 8; i++) q[i] = (float)((int)(v << (28 - 4 * i)) >> 28) * ONE<PREC>;
     } else {
         const uint32_t v = __ldg(reinterpret_cast<const uint16_t *>(reinterpret_cast<const uint8_t *>(w) + (e >> 2)));
 #pragma unroll
-        for (int i = 0; i < 8; i++) q[i] = (float)((int)(v << (30 - 2 * i)) >> 30);
+        for (int i = 0; i < 8; i++) q[i] = (float)((int)(v << (30 - 2 * i)) >> 30) * ONE<PREC>;
     }
 }
 
-// One sum with every product and sum in 64 bits.  Integer weights are multiplied before their scale: in fp32 a sum of four is then out of range for inputs
-// from 6.7e35 on, where a weight times an input is not.
-template <int PREC> __device__ __forceinline__ double dot_in_double(const void *w, uint64_t row, const float *x, uint32_t in, uint32_t lane)
-{
-    double sum = 0.0;
-#pragma unroll 1
-    for (uint32_t k = lane; k < in; k += 32) sum += (double)spg_decode_elem(w, row + k, PREC) * (double)x[k];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-    return sum;
-}
-
-// Output j for rows n0 .. n0 + NB - 1 (rows from N on read as the last one): the sums, in every lane.  `wait`: the input is what
-// the launch before this one writes, and nobody has waited for it yet.
-template <int PREC, int NB> __device__ __forceinline__ void dot(const RowsParams &p, uint32_t j, uint32_t n0, bool wait, uint32_t lane, double (&sum)[NB])
+// Output j for rows n0 .. n0 + NB - 1 (rows from N on read as the last one): the sums of every parts-th span from the part-th on, in every
+// lane.  `wait`: the input is what the launch before this one writes, and nobody has waited for it yet.
+template <int PREC, int NB, uint32_t TURNS = SPAN / TURN>
+__device__ __forceinline__ void dot(const RowsParams &p, uint32_t j, uint32_t n0, uint32_t part, uint32_t parts, bool wait, uint32_t lane, double (&sum)[NB])
 {
     const uint64_t row = (uint64_t)j * p.in;
     double acc[NB][2];
 #pragma unroll
     for (int b = 0; b < NB; b++) acc[b][0] = acc[b][1] = 0.0;
 #pragma unroll 1
-    for (uint32_t k0 = 0; k0 < p.in; k0 += SPAN) {
-        float q[ROUNDS][GROUP];
+    for (uint32_t k0 = part * (TURNS * TURN); k0 < p.in; k0 += parts * (TURNS * TURN)) {
+        float q[TURNS][GROUP];
 #pragma unroll
-        for (uint32_t u = 0; u < ROUNDS; u++) {
-            const uint32_t k = k0 + (u * 32 + lane) * GROUP;
+        for (uint32_t u = 0; u < TURNS; u++) {
+            const uint32_t k = k0 + u * TURN + lane * GROUP;
             if (p.vec_w && k < p.in) decode8<PREC>(p.w, row + k, q[u]);        // (then `in` is a multiple of eight)
             else {
 #pragma unroll
-                for (uint32_t i = 0; i < GROUP; i++) q[u][i] = k + i < p.in ? spg_decode_elem(p.w, row + k + i, PREC) : 0.0f;
+                for (uint32_t i = 0; i < GROUP; i++) q[u][i] = k + i < p.in ? spg_decode_elem(p.w, row + k + i, PREC) * ONE<PREC> : 0.0f;
             }
         }
         if (wait) { spg_grid_wait(); wait = false; }
 #pragma unroll
-        for (uint32_t u = 0; u < ROUNDS; u++) {
-            const uint32_t k = k0 + (u * 32 + lane) * GROUP;
-            if (k0 + u * 32 * GROUP >= p.in) break;                             // (the same for the whole warp)
+        for (uint32_t u = 0; u < TURNS; u++) {
+            const uint32_t k = k0 + u * TURN + lane * GROUP;
+            if (k0 + u * TURN >= p.in) break;                             // (the same for the whole warp)
 #pragma unroll
             for (int b = 0; b < NB; b++) {
                 const float *x = p.x + (uint64_t)min(n0 + b, p.N - 1) * p.ldx + k;
@@ -125,26 +122,33 @@ template <int PREC, int NB> __device__ __forceinline__ void dot(const RowsParams
         sum[b] = acc[b][0] + acc[b][1];
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) sum[b] += __shfl_xor_sync(0xffffffffu, sum[b], o);
-        if constexpr (PREC >= SPG_P_I8)
-            if (!isfinite(sum[b])) sum[b] = dot_in_double<PREC>(p.w, row, p.x + (uint64_t)min(n0 + b, p.N - 1) * p.ldx, p.in, lane);      // (the same in every lane)
     }
 }
 
-__device__ __forceinline__ float value(const RowsParams &p, uint32_t j, double sum) { return (float)(sum * (double)p.scale + (double)p.bias[j]); }
+__device__ __forceinline__ float value(const RowsParams &p, uint32_t j, double sum) { return (float)(sum * p.scale + (double)p.bias[j]); }
 
-template <int PREC, int NB>
+// FORM: 0 rows of any length, a warp an output; 1 rows of at most 256; 2 several warps an output
+template <int PREC, int NB, int FORM>
 __global__ void __launch_bounds__(256)
 spg_rows_kernel(const RowsParams p)
 {
-    const uint32_t lane = threadIdx.x & 31u, j = blockIdx.x * 8 + (threadIdx.x >> 5);
+    constexpr bool LONG = FORM == 2;
+    __shared__ double shared[LONG ? 8 : 1][NB];
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, parts = LONG ? p.parts : 1u, j = (blockIdx.x * 8 + warp) / parts, part = warp % parts;
     spg_grid_trigger();
-    if (j >= p.out) return;
+    if (!LONG && j >= p.out) return;
     double sum[NB];
     const uint32_t n0 = blockIdx.y * NB;
-    dot<PREC, NB>(p, j, n0, true, lane, sum);
+    dot<PREC, NB, FORM == 1 ? 1 : SPAN / TURN>(p, LONG ? min(j, p.out - 1) : j, n0, part, parts, true, lane, sum);
     double mine = sum[0];
 #pragma unroll
     for (int b = 1; b < NB; b++) if (lane == (uint32_t)b) mine = sum[b];
+    if (LONG) {
+        if (lane < NB) shared[warp][lane] = mine;
+        __syncthreads();
+        if (part || j >= p.out) return;
+        if (lane < NB) for (uint32_t i = 1; i < parts; i++) mine += shared[warp + i][lane];
+    }
     if (lane < NB && n0 + lane < p.N) {
         const float y = spg_activate(value(p, j, mine), p.act);
         p.y[(uint64_t)(n0 + lane) * p.ldy + j] = y;
@@ -163,7 +167,7 @@ spg_rows_softmax_kernel(const RowsParams p)
     spg_grid_trigger();
     for (uint32_t j = warp; j < p.out; j += LAST_WARPS) {
         double sum[1];
-        dot<PREC, 1>(p, j, n, j == warp, lane, sum);
+        dot<PREC, 1>(p, j, n, 0, 1, j == warp, lane, sum);
         if (lane == 0) z[j] = value(p, j, sum[0]);
     }
     __syncthreads();
@@ -192,13 +196,16 @@ spg_rows_fetch_kernel(const float *src, float *dst, uint32_t count)
     if (i < count) dst[i] = v;
 }
 
-template <int PREC> cudaError_t launch(const RowsParams &p, bool softmax, cudaStream_t s)
+template <int PREC> cudaError_t launch(RowsParams p, bool softmax, cudaStream_t s)
 {
+    p.scale *= (double)(1 << UNIT<PREC>);
     if (softmax) return spg_launch_chained(spg_rows_softmax_kernel<PREC>, dim3(p.N), dim3(32 * LAST_WARPS), 0, s, p);
     // one row of the batch a warp up to four rows, two beyond (weights decoded once for both): 784-512-1000-10 at 4 rows 9.7 against 11.5 us,
     // at 6 rows 12.9 against 10.9
-    if (p.N <= 4) return spg_launch_chained(spg_rows_kernel<PREC, 1>, dim3((p.out + 7) / 8, p.N), dim3(256), 0, s, p);
-    return spg_launch_chained(spg_rows_kernel<PREC, 2>, dim3((p.out + 7) / 8, (p.N + 1) / 2), dim3(256), 0, s, p);
+    const uint32_t each = 8 / p.parts, ctas = (p.out + each - 1) / each;
+    const auto kernel = p.N <= 4 ? (p.parts > 1 ? spg_rows_kernel<PREC, 1, 2> : p.in <= TURN ? spg_rows_kernel<PREC, 1, 1> : spg_rows_kernel<PREC, 1, 0>)
+                                 : (p.parts > 1 ? spg_rows_kernel<PREC, 2, 2> : p.in <= TURN ? spg_rows_kernel<PREC, 2, 1> : spg_rows_kernel<PREC, 2, 0>);
+    return spg_launch_chained(kernel, dim3(ctas, p.N <= 4 ? p.N : (p.N + 1) / 2), dim3(256), 0, s, p);
 }
 
 }  // namespace
@@ -216,15 +223,30 @@ template <typename F> static cudaError_t with_precision(int precision, F f)
     }
 }
 
+// Whether the softmax is finished in one CTA a row: while a warp has at most three of the outputs and four spans.  Its time less that of all
+// CTAs' products and a softmax kernel, us, by spans of a row x outputs a warp: 2 x 1 -3.9, 1 x 2 -1.4, 1 x 3 -0.9, 4 x 1 -0.1, 2 x 2 0.9, 1 x 4 1.8,
+// 2 x 4 8.4, 8 x 1 7.6; for a sample, where it saves two copies, -7.7, -4.4, 1.2, -6.0, -5.6, 2.0, 1.8, 4.4.
+static bool softmax_in_cta(const spgk_layer *L)
+{
+    const uint32_t each = (L->out + LAST_WARPS - 1) / LAST_WARPS, spans = (L->in - 1) / SPAN + 1;
+    return L->act == SPG_ACT_SOFTMAX && L->out <= LAST_MAX && each <= 3 && (uint64_t)each * spans <= 4;
+}
+
 static int rows_chain(const spgk_layer *layers, uint32_t count, const float *x, uint32_t ldx, float *const *ys, float *const *copies, uint32_t N, void *stream)
 {
+    SpgDeviceProps dp;
+    const int prc = spg_device_props(&dp);
+    if (prc) return prc;
     for (uint32_t l = 0; l < count; l++) {
         const spgk_layer *L = &layers[l];
-        const bool softmax = L->act == SPG_ACT_SOFTMAX, fused = softmax && L->out <= LAST_MAX;
+        const bool softmax = L->act == SPG_ACT_SOFTMAX, fused = softmax_in_cta(L);
         RowsParams p;
         p.w = L->w; p.bias = L->bias; p.scale = L->w_scale; p.in = L->in; p.out = L->out; p.act = softmax ? SPG_ACT_NONE : L->act;
         p.x = x; p.ldx = ldx; p.y = ys[l]; p.ldy = L->out; p.N = N; p.copy = copies ? copies[l] : nullptr;
         p.vec_w = (L->in % 8 == 0 && ((uintptr_t)L->w & 15u) == 0) ? 1u : 0u;
+        // (as long as there are warps to spare: 4096-1000 FP16 at four rows 14.9 us with a warp an output, 19.0 with four)
+        p.parts = 1;
+        for (const uint64_t warps = (uint64_t)L->out * (N <= 4 ? N : (N + 1) / 2); L->in > LONG_ROW && p.parts < 8 && p.parts * SPAN < L->in && 2 * p.parts * warps <= 32ull * dp.sm_count;) p.parts *= 2;
         p.vec_x = (((uintptr_t)x | ((uintptr_t)ldx * 4)) & 15u) == 0 ? 1u : 0u;
         SPGK_CUDA(with_precision(L->precision, [&](auto prec) { return launch<prec.value>(p, fused, (cudaStream_t)stream); }));
         int rc = spgk_check_launch("spg_rows_kernel");
@@ -257,7 +279,7 @@ extern "C" int spgk_rows_sample(const spgk_layer *layers, uint32_t count, float 
     float *ys[SPGK_ROWS_MAX_LAYERS], *copies[SPGK_ROWS_MAX_LAYERS];
     uint64_t at = layers[0].in;
     for (uint32_t l = 0; l < count; l++) {
-        if (layers[l].act == SPG_ACT_SOFTMAX && layers[l].out > LAST_MAX) return SPGK_E_UNSUPPORTED;
+        if (layers[l].act == SPG_ACT_SOFTMAX && !softmax_in_cta(&layers[l])) return SPGK_E_UNSUPPORTED;
         ys[l] = dev + at; copies[l] = host + at;
         at += layers[l].out;
     }

@@ -404,16 +404,34 @@ static bool all_wstream(const spg_net *n, uint32_t N)
 }
 
 /* Up to eight rows of a net of few weights go warp by warp from L2, whatever their precision, widths and alignment.  The lines lie where the
- * curves cross (us a call, this kernel / what served before): 0.9 million weights 10 / 25 to 45 at one row, 12 / 90 to 162 at eight; 7.3
- * million INT8 weights 18.6 / 20.6 at one row, 35 / 43 at six; 8.0 million BF16 ones in rows of odd lengths 26 / 27 and 76 / 95; 25
- * million INT2 weights 148 / 49 at six.  (At seven and eight rows forward_batch asks the integer streaming kernel first.) */
+ * kernel meets what serves otherwise (us a call, this kernel / the GEMV or the general kernels), in weights a layer on average, since every
+ * layer costs the others a launch or a chain's step: nets of integers at two rows or more 4 Mi (one layer of 4.1 million INT4 weights at
+ * four rows 15 / 18, of 5.1 million 23 / 18, of 8.4 million 24 / 19, at one row 12 / 36; two layers of 8.3 million 27 / 28, three 33 / 50);
+ * rows of odd lengths, which are loaded one by one, 3 Mi (INT4 in one layer of 4 million 29 / 21 at four rows, two layers of 6.1 million 44
+ * / 60), of fp32 at five to seven rows 2 Mi (three layers of 6.5 million 75 / 71, of 8.1 million 99 / 78; 98 / 254 at eight).  Every output is a
+ * warp, which is much beside the streaming kernel's way with short rows of integers: 64-65536-32 in INT4 126 / 93 at four rows, 64-32768-100 68 / 62.  25
+ * million INT2 weights take 148 / 49 at six rows. */
 #define SPG_ROWS_MAX_WEIGHTS ((uint64_t)8 << 20)
+#define SPG_ROWS_MAX_OUTPUTS 65535u                 /* of a layer of integers */
 
-static bool few_weights(const spg_net *n)
+static bool few_weights(const spg_net *n, uint32_t N)
 {
+    const PrecisionMode prec = n->klayers[0].precision;
+    const bool integers = prec >= PRECISION_INT8;
     uint64_t count = 0;
-    for (uint32_t l = 0; l < n->dev_layers; l++) count += (uint64_t)n->klayers[l].in * n->klayers[l].out;
-    return count <= SPG_ROWS_MAX_WEIGHTS;
+    uint32_t widest = 0;
+    bool odd = false, streams = true;           /* some rows are no multiple of a lane's eight values; all are whole 16 bytes of integers */
+    for (uint32_t l = 0; l < n->dev_layers; l++) {
+        const spgk_layer *L = &n->klayers[l];
+        odd = odd || L->in % 8;
+        streams = streams && integers && L->in % (16u << (prec - PRECISION_INT8)) == 0;
+        if (L->out > widest) widest = L->out;
+        count += (uint64_t)L->in * L->out;
+    }
+    if (streams && widest > SPG_ROWS_MAX_OUTPUTS) return false;
+    const uint64_t mi = (uint64_t)1 << 20;
+    const uint64_t each = odd ? (prec == PRECISION_FLOAT32 && N > 4 && N < 8 ? 2 * mi : 3 * mi) : integers && N > 1 ? 4 * mi : SPG_ROWS_MAX_WEIGHTS;
+    return count <= SPG_ROWS_MAX_WEIGHTS && count <= each * n->dev_layers;
 }
 
 /* Small / medium batches (fp32 activations between layers; every layer streams its packed weights once).
@@ -423,7 +441,7 @@ static bool few_weights(const spg_net *n)
 int spg_dev_forward_small(spg_net *n, const float *d_x, uint32_t ldx, uint32_t N, float **d_last, float *d_final)
 {
     NeuralNetwork *p = &n->pub;
-    const bool rows = N <= SPGK_ROWS_MAX_BATCH && few_weights(n);
+    const bool rows = N <= SPGK_ROWS_MAX_BATCH && few_weights(n, N);
     int rc = rows ? activations_reserve(n, N) : small_reserve(n, N);
     if (rc) return rc;
     if (!d_last) return SPINGALETT_OK;          /* reservation only */
@@ -509,7 +527,7 @@ int spg_dev_forward_small(spg_net *n, const float *d_x, uint32_t ldx, uint32_t N
 int spg_dev_forward_sample(spg_net *n, float *h_io, bool *taken)
 {
     *taken = false;
-    if (!few_weights(n) || n->dev_layers > SPGK_ROWS_MAX_LAYERS) return SPINGALETT_OK;
+    if (!few_weights(n, 1) || n->dev_layers > SPGK_ROWS_MAX_LAYERS) return SPINGALETT_OK;
     int rc = activations_reserve(n, 1);
     if (rc) return rc;
     prof_mark(n);

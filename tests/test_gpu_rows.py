@@ -1,5 +1,6 @@
 """One to eight rows of a small net (spg_rows.cu): every precision, widths around a lane's eight values and a warp's 1024, rows that
-start in the middle of a byte, softmax rows finished in the kernel (up to 128 outputs) and behind it."""
+start in the middle of a byte, rows that several warps share, softmax rows finished in the kernel (up to 128 outputs) and behind it; which
+nets go there."""
 import ctypes as C
 
 import numpy as np
@@ -29,7 +30,7 @@ def matrix(rng, out, inn, prec):
 
 
 @pytest.mark.parametrize("prec", range(6))
-@pytest.mark.parametrize("widths", [(1, 1, 2), (7, 9, 3), (8, 16, 128), (301, 77, 129), (1023, 33, 10), (1024, 40, 64), (1032, 8, 5), (2049, 17, 1)])
+@pytest.mark.parametrize("widths", [(1, 1, 2), (7, 9, 3), (8, 16, 128), (301, 77, 129), (1023, 33, 10), (1024, 40, 64), (1032, 8, 5), (2049, 17, 1), (2048, 2056, 70), (4096, 9, 100), (9001, 3, 128)])
 def test_small_net_against_float64(spg, prec, widths):
     import torch
     lib = spg.lib()
@@ -46,7 +47,7 @@ def test_small_net_against_float64(spg, prec, widths):
         keep += [dw, db]
         layers[l] = spg.abi.KLayer(dw.data_ptr(), db.data_ptr(), scale, inn, out, prec, act)
         values.append((np.asarray(w, np.float64).reshape(out, inn) * scale, bias.astype(np.float64)))
-    for n in (1, 2, 3, 8):
+    for n in (1, 2, 3, 4, 5, 7, 8):                     # (one row of the batch a warp up to four, two beyond, the last of an odd number alone)
         for pad in (0, 1):                              # rows of the input that lie on 16 bytes, and rows that do not
             ldx = widths[0] + pad
             x = rng.standard_normal((n, ldx)).astype(np.float32)
@@ -72,14 +73,15 @@ def test_small_net_against_float64(spg, prec, widths):
 
 @pytest.mark.parametrize("prec", [3, 4, 5])
 @pytest.mark.parametrize("n", [1, 4, 7])
-def test_integer_weights_times_large_inputs(spg, prec, n):
+@pytest.mark.parametrize("inn", [1100, 3000, 9000])
+def test_integer_weights_times_large_inputs(spg, prec, n, inn):
     """Inputs up to 1e38: a stored weight times an input is out of fp32's range, a weight times an input is not.  Rows with values that are not
     finite keep them to themselves."""
     import torch
     lib = spg.lib()
     lib.spgk_rows_forward.argtypes = [C.POINTER(spg.abi.KLayer), C.c_uint32, C.c_void_p, C.c_uint32, C.POINTER(C.c_void_p), C.c_uint32, C.c_void_p]
     rng = np.random.default_rng(prec * 10 + n)
-    inn, out = 1100, 41
+    out = 41
     raw, q = matrix(rng, out, inn, prec)
     scale = float(np.float32(1 / (np.abs(q).max() * inn)))          # no sum is larger than its largest input
     bias = rng.standard_normal(out).astype(np.float32)
@@ -101,7 +103,7 @@ def test_integer_weights_times_large_inputs(spg, prec, n):
     assert not np.isfinite(got[:n][~good]).any() and np.all(got[n] == -3.0)
 
 
-@pytest.mark.parametrize("topo,last", [([784, 512, 10], 5), ([301, 77, 128], 5), ([33, 40, 129], 5), ([7, 1], 0)])
+@pytest.mark.parametrize("topo,last", [([784, 512, 10], 5), ([301, 77, 128], 5), ([40, 4100, 100], 5), ([4100, 97], 5), ([33, 40, 129], 5), ([7, 1], 0)])
 def test_a_sample_from_host_memory_gives_what_a_batch_of_one_gives(spg, topo, last):
     """forward() (input and outputs of every layer through page-locked memory; wider softmax rows by copies) against forward_batch."""
     net = spg.Network.build(topo, [1] * (len(topo) - 2) + [last], spg.abi.WEIGHT_INITIALIZATION_NONE)
@@ -117,4 +119,36 @@ def test_a_sample_from_host_memory_gives_what_a_batch_of_one_gives(spg, topo, la
             w, b = net.weights[:topo[0] * topo[1]].reshape(topo[1], topo[0]).astype(np.float64), net.biases[:topo[1]].astype(np.float64)
             hidden = np.maximum(w @ x[0].astype(np.float64) + b, 0)
             assert np.all(np.abs(neurons[topo[0]:topo[0] + topo[1]] - hidden) <= 2.0 ** -24 * hidden + 2.0 ** -22 * (np.abs(w) @ np.abs(x[0]) + np.abs(b)))
+    net.free()
+
+
+# on either side of the lines: weights a layer (integers at two rows and more, rows of odd lengths), weights in all, outputs of a layer of streamed rows.  64-65536-34
+# goes to two other kernels by turns.
+@pytest.mark.parametrize("topo,precision,n,rows", [([4096, 1024], "int4", 8, False), ([4096, 1024], "int4", 6, True), ([4096, 1032], "int8", 1, True), ([4096, 1032], "int8", 2, False),
+                                                   ([4096, 1032], "fp16", 8, True), ([1001, 3142], "int2", 2, True), ([1001, 3143], "int2", 2, False),
+                                                   ([1001, 2095], "fp32", 5, True), ([1001, 2096], "fp32", 5, False), ([1001, 2096], "fp32", 8, True), ([2048, 2048, 2048], "bf16", 3, True),
+                                                   ([2048, 2048, 2056], "bf16", 3, False), ([64, 65535, 32], "int4", 2, True), ([64, 65536, 34], "int4", 2, False), ([48, 65536, 34], "int4", 2, True),
+                                                   ([64, 65536, 32], "fp32", 2, True)])
+def test_which_nets_go_there(spg, tmp_path, topo, precision, n, rows):
+    net = spg.Network.build(topo, [2] * (len(topo) - 2) + [6], spg.abi.WEIGHT_INITIALIZATION_NONE)
+    rng = np.random.default_rng(sum(topo))
+    net.weights[:] = rng.standard_normal(net.weights.size, dtype=np.float32) / 32
+    net.biases[:] = rng.standard_normal(net.biases.size, dtype=np.float32) / 8
+    net.save(str(tmp_path / "net.nn"), spg.abi.PRECISION_NAMES[precision])
+    net.free()
+    net = spg.Network.load(str(tmp_path / "net.nn"))
+    x = rng.standard_normal((n, topo[0])).astype(np.float32)
+    got = net.forward_batch(x)
+    assert (spg.last_path() == "rows") == rows
+    a, off, at, bt = x.astype(np.float64), 0.0, 0, 0
+    for l, (i, o) in enumerate(zip(topo, topo[1:])):
+        w, b = net.weights[at:at + i * o].reshape(o, i).astype(np.float64), net.biases[bt:bt + o]
+        # every kernel: values to 16 bits at least, weights exact, tanh no steeper than 1
+        off = off @ np.abs(w).T if l else 0.0
+        off = off + 2.0 ** -15 * (np.abs(a) @ np.abs(w).T) + 2.0 ** -20
+        a = a @ w.T + b
+        if l + 2 < len(topo):
+            a = np.tanh(a)
+        at, bt = at + i * o, bt + o
+    assert np.all(np.abs(got - a) <= off)
     net.free()
