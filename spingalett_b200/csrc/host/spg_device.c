@@ -446,15 +446,21 @@ int spg_dev_forward_small(spg_net *n, const float *d_x, uint32_t ldx, uint32_t N
     if (rc) return rc;
     if (!d_last) return SPINGALETT_OK;          /* reservation only */
     if (rows) {
-        float *ys[n->dev_layers];
-        for (uint32_t l = 0; l < n->dev_layers; l++)
-            ys[l] = (d_final && l + 1 == n->dev_layers) ? d_final : n->d_small + (size_t)N * p->neuron_offsets[l + 1];
+        float *ys[SPGK_ROWS_MAX_LAYERS];
+        const float *x = d_x ? d_x : n->d_small;
+        uint32_t xld = d_x ? ldx : p->topology[0], count;
         prof_mark(n);
-        rc = spg_map_kernel_error(spgk_rows_forward(n->klayers, n->dev_layers, d_x ? d_x : n->d_small, d_x ? ldx : p->topology[0], ys, N, n->stream), "layers (small net)");
+        for (uint32_t l0 = 0; l0 < n->dev_layers && !rc; l0 += count) {
+            count = n->dev_layers - l0 < SPGK_ROWS_MAX_LAYERS ? n->dev_layers - l0 : SPGK_ROWS_MAX_LAYERS;
+            for (uint32_t i = 0; i < count; i++)
+                ys[i] = (d_final && l0 + i + 1 == n->dev_layers) ? d_final : n->d_small + (size_t)N * p->neuron_offsets[l0 + i + 1];
+            rc = spg_map_kernel_error(spgk_rows_forward(n->klayers + l0, count, x, xld, ys, N, n->stream), "layers (small net)");
+            x = *d_last = ys[count - 1];
+            xld = n->klayers[l0 + count - 1].out;
+        }
         prof_mark(n);
         if (rc) return rc;
         spg_note_path("rows");
-        *d_last = ys[n->dev_layers - 1];
         return SPINGALETT_OK;
     }
     const float *x = d_x ? d_x : n->d_small;
