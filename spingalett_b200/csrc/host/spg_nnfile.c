@@ -14,7 +14,6 @@
 #include <stdlib.h>
 #include <string.h>
 #include <errno.h>
-#include <fcntl.h>
 #include <unistd.h>
 
 typedef struct { const uint8_t *p; size_t len, pos; } cursor;
@@ -314,13 +313,6 @@ void save_spingalett_struct_arguments(SaveArgs a)
         if (wc > maxc) maxc = wc;
         if (n->topology[l + 1] > maxc) maxc = n->topology[l + 1];
     }
-    /* Room for the whole file at once.  (Without it ext4, which allocates late, writes a file that replaced another out to the disk
-     * when it is closed: 25 MB take 6 to 14 ms instead of 3.)  Where it cannot be had, the writes will say so. */
-    uint64_t size = h + 4ull * n->layers + (n->layers - 1);
-    for (uint32_t l = 0; l + 1 < n->layers; l++)
-        size += (has_opt ? 3u : 1u) * (uint64_t)(spg_array_bytes((uint32_t)(n->topology[l] * n->topology[l + 1]), a.precision) + spg_array_bytes(n->topology[l + 1], a.precision));
-    const bool asked = size >= (1u << 20);
-    if (asked && fallocate(fileno(f), FALLOC_FL_KEEP_SIZE, 0, (off_t)size) != 0) spg_log(LOG_DEBUG, "save: no room reserved");
     uint8_t *scratch = malloc((size_t)maxc * 4 + 8);
     float *zeros = NULL;
     if (has_opt && !n->opt_m_weights) zeros = calloc(maxc, sizeof(float));   /* never trained: state is all zero */
@@ -358,10 +350,6 @@ void save_spingalett_struct_arguments(SaveArgs a)
     }
     dev_encoder_close(&de);
     free(scratch); free(zeros);
-    if (!ok && asked && fflush(f) == 0) {
-        const off_t end = lseek(fileno(f), 0, SEEK_CUR);
-        if (end >= 0 && ftruncate(fileno(f), end) != 0) spg_log(LOG_DEBUG, "save: reserved room stays with the file");
-    }
     if (fclose(f) != 0) ok = false;
     if (!ok) {
         spg_set_error(SPINGALETT_ERR_INVALID, "save: write error (disk full?)");
