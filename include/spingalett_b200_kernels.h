@@ -260,6 +260,9 @@ SPGK_API size_t spgk_istream_scratch_bytes(const spgk_layer *layers, uint32_t co
 SPGK_API int spgk_istream_forward(const spgk_layer *layers, uint32_t count, const float *x, uint32_t ldx, float *const *ys,
                                   uint32_t N, void *scratch, void *stream);
 SPGK_API int spgk_istream_status(void *scratch, void *stream);
+/* How a layer is arranged on a GPU of `sms` SMs (0: the current device's): CTAs that share a tile, batch rows a group, tiles, CTAs.  Returns whether
+ * the kernel takes the layer.  (For tests and measurements; needs no GPU if `sms` is given.) */
+SPGK_API int spgk_istream_arrangement(const spgk_layer *L, uint32_t N, uint32_t sms, uint32_t out[4]);
 
 /* ---- K2: large-batch tcgen05 GEMM layer ----------------------------------
  * C[N][out] = act(bias + w_scale * A[N][in] * W^T) with the accumulator in

@@ -62,7 +62,7 @@ constexpr uint32_t IS_THREADS = 32 * (IS_DIGIT_WARP + 1);
 constexpr uint32_t TILE_ROWS = 128;
 constexpr uint32_t BOX_BYTES = 128 * TILE_ROWS;        // one box of packed weights = one operand tile = 16 KB
 constexpr uint32_t GROUP_ROWS = 64;                    // batch rows per pass over the weights: 256 digit columns
-constexpr uint32_t IS_PAIR_ROWS = 32, IS_PAIR_BLOCKS = 32;
+constexpr uint32_t IS_PAIR_ROWS = 32, IS_PAIR_BLOCKS = 16;
 constexpr uint32_t MAX_K = 131072;                     // 64 * 128 * K < 2^31
 constexpr uint32_t MAX_TILES = 4096;                   // counters in the scratch head
 constexpr uint32_t STAGE_THREADS = 1024;
@@ -735,6 +735,9 @@ struct IsPlan {
 
 constexpr size_t IS_HEAD = 256 + 4 * MAX_TILES;        // status word, counters; zero between calls, like the sums behind them
 
+// one CTA (or pair) per SM (or two), but a tile in about four pieces at most: the sum over more of them costs more than they save
+uint32_t is_ctas(uint64_t tiles, uint32_t boxes, uint32_t most) { const uint64_t want = tiles * (boxes < 4 ? boxes : 4); return want < most ? (uint32_t)want : most; }
+
 IsPlan is_plan(const spgk_layer *L, uint32_t N, uint32_t sms)
 {
     IsPlan pl{};
@@ -745,26 +748,25 @@ IsPlan is_plan(const spgk_layer *L, uint32_t N, uint32_t sms)
     if ((L->in * bits) % 128 || ((uintptr_t)L->w & 15u)) return pl;       // TMA: 16-byte aligned packed rows
     pl.groups = (N + GROUP_ROWS - 1) / GROUP_ROWS;
     pl.rpg = ((N + pl.groups - 1) / pl.groups + 3u) & ~3u;
+    pl.kbr = 8u / bits;
+    pl.boxes = (L->in * bits + 1023u) / 1024u;
     // Pairs of CTAs where the digits are most of what an SM draws from L2 (more than 32 rows a group; up to 32 rows pairs were level or behind by 7 %)
-    // and the layer is a long one: 32 blocks for an SM, or 8192 inputs (1024-4096-4096-1000, 2 to 28 blocks an SM: 52.4 us in pairs against 51.3 at
-    // 64 rows; 8192 x 1000, 3.4 blocks: the net around it 166 us against 171 with this layer alone on single CTAs).  INT8, which 64 rows stream
-    // at the rate of HBM, only from the second group on (40 rows: 170 against 167 us, 72 rows: 253 against 261).
-    const uint64_t blocks = (uint64_t)((L->out + TILE_ROWS - 1) / TILE_ROWS) * ((L->in + 127u) / 128u) * pl.groups;
-    pl.pair = pl.rpg > IS_PAIR_ROWS && (blocks >= (uint64_t)IS_PAIR_BLOCKS * sms || L->in >= 8192u) && L->out > TILE_ROWS && sms >= 2 && (prec != SPG_P_I8 || pl.groups > 1);
+    // and a CTA alone would have at least 16 blocks in a row.  Pairs over single CTAs in 340 layers of 2048 to 16384 inputs and 512 to 16384 outputs at
+    // 40 to 256 rows, weights from HBM, by blocks in a row, INT4: 4 to 8 1.02, 8 to 16 0.99, 16 to 32 0.96, 32 to 64 0.94, beyond 0.92 (INT2 the
+    // same; INT8 1.02, 1.02, 0.98, 1.00, 0.96).  INT8, which 64 rows stream at the rate of HBM, only from the second group on (40 rows: 170 against 167 us, 72
+    // rows: 253 against 261).
+    const uint64_t alone = (uint64_t)((L->out + TILE_ROWS - 1) / TILE_ROWS) * pl.groups, ctas = is_ctas(alone, pl.boxes, sms);
+    pl.pair = pl.rpg > IS_PAIR_ROWS && alone * pl.boxes * pl.kbr >= IS_PAIR_BLOCKS * ctas && L->out > TILE_ROWS && sms >= 2 && (prec != SPG_P_I8 || pl.groups > 1);
     if (pl.pair) pl.rpg = (pl.rpg + 7u) & ~7u;                            // (a pair's product takes multiples of 32 columns)
     pl.C = 4 * pl.rpg;
-    pl.kbr = 8u / bits;
     pl.direct = prec == SPG_P_I8;
-    pl.boxes = (L->in * bits + 1023u) / 1024u;
     pl.ld = pl.boxes * pl.kbr * 128u;
     const uint32_t high = pl.pair ? 2 * TILE_ROWS : TILE_ROWS;
     pl.m_tiles = (L->out + high - 1) / high;
     pl.tiles = pl.m_tiles * pl.groups;
     if (pl.tiles > (pl.pair ? MAX_TILES / 2 : MAX_TILES)) return pl;     // (a pair's tile has two counters)
     pl.units = (uint64_t)pl.tiles * pl.boxes;
-    // one CTA per SM, but a tile in about four pieces at most: the sum over more of them costs more than they save
-    const uint64_t want = (uint64_t)pl.tiles * (pl.boxes < 4 ? pl.boxes : 4);
-    pl.grid = pl.pair ? 2 * (want < sms / 2 ? (uint32_t)want : sms / 2) : want < sms ? (uint32_t)want : sms;
+    pl.grid = pl.pair ? 2 * is_ctas(pl.tiles, pl.boxes, sms / 2) : is_ctas(pl.tiles, pl.boxes, sms);
     // rings: operand tiles in two slots of G blocks, digit tiles up to 96 KB (in pairs up to 32 rows), boxes with the rest
     const uint32_t b_bytes = pl.C * (pl.pair ? 64u : 128u);
     pl.G = pl.direct ? 1 : 2;
@@ -840,6 +842,15 @@ IsScratch is_scratch(const spgk_layer *layers, uint32_t count, uint32_t N, uint3
 }  // namespace
 
 extern "C" {
+
+int spgk_istream_arrangement(const spgk_layer *L, uint32_t N, uint32_t sms, uint32_t out[4])
+{
+    SpgDeviceProps dp;
+    if (!L || (!sms && spg_device_props(&dp) != SPGK_OK)) return 0;
+    const IsPlan pl = is_plan(L, N, sms ? sms : (uint32_t)dp.sm_count);
+    out[0] = pl.pair ? 2 : 1; out[1] = pl.rpg; out[2] = pl.tiles; out[3] = pl.grid;
+    return pl.ok ? 1 : 0;
+}
 
 size_t spgk_istream_scratch_bytes(const spgk_layer *layers, uint32_t count, uint32_t N)
 {
