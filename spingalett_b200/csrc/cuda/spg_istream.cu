@@ -754,9 +754,10 @@ IsPlan is_plan(const spgk_layer *L, uint32_t N, uint32_t sms)
     // and a CTA alone would have at least 16 blocks in a row.  Pairs over single CTAs in 340 layers of 2048 to 16384 inputs and 512 to 16384 outputs at
     // 40 to 256 rows, weights from HBM, by blocks in a row, INT4: 4 to 8 1.02, 8 to 16 0.99, 16 to 32 0.96, 32 to 64 0.94, beyond 0.92 (INT2 the
     // same; INT8 1.02, 1.02, 0.98, 1.00, 0.96).  INT8, which 64 rows stream at the rate of HBM, only from the second group on (40 rows: 170 against 167 us, 72
-    // rows: 253 against 261).
+    // rows: 253 against 261).  A pair's tile has two counters.
     const uint64_t alone = (uint64_t)((L->out + TILE_ROWS - 1) / TILE_ROWS) * pl.groups, ctas = is_ctas(alone, pl.boxes, sms);
-    pl.pair = pl.rpg > IS_PAIR_ROWS && alone * pl.boxes * pl.kbr >= IS_PAIR_BLOCKS * ctas && L->out > TILE_ROWS && sms >= 2 && (prec != SPG_P_I8 || pl.groups > 1);
+    const uint64_t paired = (uint64_t)((L->out + 2 * TILE_ROWS - 1) / (2 * TILE_ROWS)) * pl.groups;
+    pl.pair = pl.rpg > IS_PAIR_ROWS && 2 * paired <= MAX_TILES && alone * pl.boxes * pl.kbr >= IS_PAIR_BLOCKS * ctas && L->out > TILE_ROWS && sms >= 2 && (prec != SPG_P_I8 || pl.groups > 1);
     if (pl.pair) pl.rpg = (pl.rpg + 7u) & ~7u;                            // (a pair's product takes multiples of 32 columns)
     pl.C = 4 * pl.rpg;
     pl.direct = prec == SPG_P_I8;
@@ -764,7 +765,7 @@ IsPlan is_plan(const spgk_layer *L, uint32_t N, uint32_t sms)
     const uint32_t high = pl.pair ? 2 * TILE_ROWS : TILE_ROWS;
     pl.m_tiles = (L->out + high - 1) / high;
     pl.tiles = pl.m_tiles * pl.groups;
-    if (pl.tiles > (pl.pair ? MAX_TILES / 2 : MAX_TILES)) return pl;     // (a pair's tile has two counters)
+    if (pl.tiles > MAX_TILES) return pl;
     pl.units = (uint64_t)pl.tiles * pl.boxes;
     pl.grid = pl.pair ? 2 * is_ctas(pl.tiles, pl.boxes, sms / 2) : is_ctas(pl.tiles, pl.boxes, sms);
     // rings: operand tiles in two slots of G blocks, digit tiles up to 96 KB (in pairs up to 32 rows), boxes with the rest

@@ -31,6 +31,16 @@ def test_which_layers_go_to_pairs(spg, prec, out, inn, n, pair):
     assert tiles == -(-out // (128 << pair)) * -(-n // 64) and ctas <= 148 and ctas % shared == 0
 
 
+@pytest.mark.parametrize("prec", [3, 4, 5])
+@pytest.mark.parametrize("out,inn,n,shared", [
+    (128 * 2 * 682, 4096, 192, 2),                            # 2046 pairs' tiles: two counters each
+    (128 * 2 * 682 + 1, 4096, 192, 1),                        # 2049, and 4095 of single CTAs
+    (128 * 1365, 4096, 192, 1), (128 * 1365 + 1, 4096, 192, None), (128 * 4096, 64, 32, 1), (128 * 4096 + 1, 64, 32, None)])
+def test_layers_of_as_many_tiles_as_there_are_counters(spg, prec, out, inn, n, shared):
+    got = arrangement(spg, prec, out, inn, n, sms=148)
+    assert (got and got[0]) == shared and (not got or got[2] * got[0] <= 4096)
+
+
 # one output into a pair's first CTA, whole pairs, two into its second; a padded group; packed rows that end inside a box
 @gpu
 @pytest.mark.parametrize("prec", [3, 4, 5])
