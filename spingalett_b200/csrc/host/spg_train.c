@@ -121,20 +121,22 @@ static void state_free(train_state *t)
     free(t);
 }
 
-/* the page-locked block: 1 KB of words, then room for the shuffled orders of two epochs (0 samples: none) */
+/* the page-locked block: 1 KB of words, then room for the shuffled orders of two epochs (0 samples: none); the words alone where there is no
+ * more to be had */
 static int pinned_reserve(train_state *t, uint32_t samples)
 {
     int rc;
     if (t->h_words && t->order_cap < samples) { spgk_host_free(t->h_words); t->h_words = NULL; }
     if (!t->h_words) {
         void *h = NULL;
-        t->order_cap = 0;
-        if ((rc = spg_map_kernel_error(spgk_host_alloc(&h, 1024 + 2 * (size_t)samples * 4), "train: pinned words"))) return rc;
-        t->h_words = h; t->order_cap = samples;
+        t->order_cap = samples;
+        if (samples && spgk_host_alloc(&h, 1024 + 2 * (size_t)samples * 4) != SPGK_OK) { h = NULL; t->order_cap = 0; }
+        if (!h && (rc = spg_map_kernel_error(spgk_host_alloc(&h, 1024), "train: pinned words"))) return rc;
+        t->h_words = h;
     }
     for (int i = 0; i < 2; i++) {
-        t->h_order[i] = (uint32_t *)(void *)(t->h_words + 256) + (size_t)i * t->order_cap;
-        if (samples && !t->order_ev[i] && (rc = spg_map_kernel_error(spgk_event_create(&t->order_ev[i]), "train: shuffle order"))) return rc;
+        t->h_order[i] = t->order_cap ? (uint32_t *)(void *)(t->h_words + 256) + (size_t)i * t->order_cap : NULL;
+        if (t->order_cap && !t->order_ev[i] && (rc = spg_map_kernel_error(spgk_event_create(&t->order_ev[i]), "train: shuffle order"))) return rc;
     }
     return SPINGALETT_OK;
 }
@@ -434,13 +436,18 @@ void train_struct_arguments(TrainArgs a)
         if (need_loss || graph_mode) DEV(spgk_memset(d_loss, 0, 4, st), "train: clear loss");
         float *const loss_ptr = (need_loss || graph_mode) ? d_loss : NULL;      /* a replayed step always adds to the loss word */
         if (mini) {
-            /* the order goes out from one of two page-locked buffers, so that this thread need not wait for the epoch before */
+            /* the order goes out from one of two page-locked buffers, where they are to be had, so that this thread need not wait for the epoch before */
             const int b = (int)(epoch & 1);
             spg_shuffle(order, a.sample_count);
-            if (epoch > 2) DEV(s_world > 1 ? train_sync(st) : spgk_event_sync(t->order_ev[b]), "train: order sync");
-            memcpy(t->h_order[b], order, (size_t)a.sample_count * 4);
-            DEV(spgk_memcpy_h2d(t->idx, t->h_order[b], (size_t)a.sample_count * 4, st), "train: upload order");
-            DEV(spgk_event_record(t->order_ev[b], st), "train: upload order");
+            if (t->h_order[b]) {
+                if (epoch > 2) DEV(s_world > 1 ? train_sync(st) : spgk_event_sync(t->order_ev[b]), "train: order sync");
+                memcpy(t->h_order[b], order, (size_t)a.sample_count * 4);
+                DEV(spgk_memcpy_h2d(t->idx, t->h_order[b], (size_t)a.sample_count * 4, st), "train: upload order");
+                DEV(spgk_event_record(t->order_ev[b], st), "train: upload order");
+            } else {
+                DEV(spgk_memcpy_h2d(t->idx, order, (size_t)a.sample_count * 4, st), "train: upload order");
+                DEV(train_sync(st), "train: order sync");        /* `order` is reshuffled next epoch */
+            }
         }
         const uint32_t nb = (a.sample_count + batch - 1) / batch;
         for (uint32_t bi = 0; bi < nb; bi++) {
