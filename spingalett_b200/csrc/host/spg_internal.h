@@ -120,11 +120,10 @@ SPG_HIDDEN void spg_bulk_zero(void *dst, size_t bytes);
 SPG_HIDDEN void spg_large_pages(void *p, size_t bytes);
 /* stage.c */
 #define SPG_STAGE_PIECE ((size_t)8 << 20)
-typedef struct { void *piece[2], *landed[2], *stream; bool busy[2]; int turn; } spg_stager;      /* two page-locked pieces on a stream */
+typedef struct { void *piece[2], *landed[2], *stream; bool busy[2], unsure; int turn; } spg_stager;      /* two page-locked pieces on a stream; unsure: a copy may be under way that no event tells of */
 typedef bool (*spg_sink_fn)(void *ctx, size_t at, const void *piece, size_t n);
 SPG_HIDDEN int spg_stager_open(spg_stager *s, void *stream);
 SPG_HIDDEN void spg_stager_close(spg_stager *s);                                   /* waits for what is under way */
-SPG_HIDDEN int spg_stager_settle(spg_stager *s);
 SPG_HIDDEN int spg_stager_up(spg_stager *s, void *dev, const void *src, size_t bytes);
 typedef struct { const void *dev; size_t bytes; void *ctx; } spg_segment;                       /* device memory and where it goes */
 SPG_HIDDEN int spg_stager_down(spg_stager *s, spg_sink_fn sink, const spg_segment *seg, int count);

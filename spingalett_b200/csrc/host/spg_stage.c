@@ -57,31 +57,37 @@ int spg_stager_open(spg_stager *s, void *stream)
     return SPGK_OK;
 }
 
+/* waits for the copy from or to a piece */
+static int stager_wait(spg_stager *s, int i)
+{
+    if (!s->busy[i]) return SPGK_OK;
+    s->busy[i] = false;
+    const int rc = spgk_event_sync(s->landed[i]);
+    if (rc) s->unsure = true;
+    return rc;
+}
+
+/* a copy from or to a piece has been queued */
+static int stager_queued(spg_stager *s, int i)
+{
+    const int rc = spgk_event_record(s->landed[i], s->stream);
+    if (rc) s->unsure = true;
+    else s->busy[i] = true;
+    return rc;
+}
+
 /* the piece whose turn it is, once the device has done with what it held */
 static int stager_turn(spg_stager *s, int *turn)
 {
     const int i = *turn = s->turn;
     s->turn ^= 1;
-    if (!s->busy[i]) return SPGK_OK;
-    s->busy[i] = false;
-    return spgk_event_sync(s->landed[i]);
-}
-
-int spg_stager_settle(spg_stager *s)
-{
-    int first = SPGK_OK;
-    for (int i = 0; i < 2; i++)
-        if (s->busy[i]) {
-            s->busy[i] = false;
-            const int rc = spgk_event_sync(s->landed[i]);
-            if (rc && !first) first = rc;
-        }
-    return first;
+    return stager_wait(s, i);
 }
 
 void spg_stager_close(spg_stager *s)
 {
-    const bool idle = spg_stager_settle(s) == SPGK_OK;
+    for (int i = 0; i < 2; i++) stager_wait(s, i);
+    const bool idle = !s->unsure || spgk_stream_sync(s->stream) == SPGK_OK;
     for (int i = 0; i < 2; i++) {
         if (s->landed[i]) spgk_event_destroy(s->landed[i]);
         if (idle) piece_return(s->piece[i]);
@@ -98,8 +104,7 @@ int spg_stager_up(spg_stager *s, void *dev, const void *src, size_t bytes)
         int i, rc = stager_turn(s, &i);
         if (rc) return rc;
         spg_stage_copy(s->piece[i], (const char *)src + at, n);
-        if ((rc = spgk_memcpy_h2d((char *)dev + at, s->piece[i], n, s->stream)) || (rc = spgk_event_record(s->landed[i], s->stream))) return rc;
-        s->busy[i] = true;
+        if ((rc = spgk_memcpy_h2d((char *)dev + at, s->piece[i], n, s->stream)) || (rc = stager_queued(s, i))) return rc;
     }
     return SPGK_OK;
 }
@@ -119,12 +124,10 @@ int spg_stager_down(spg_stager *s, spg_sink_fn sink, const spg_segment *seg, int
             now.seg = g; now.at = at; now.n = seg[g].bytes - at < SPG_STAGE_PIECE ? seg[g].bytes - at : SPG_STAGE_PIECE;
             at += now.n;
             if ((rc = stager_turn(s, &now.piece)) || (rc = spgk_memcpy_d2h(s->piece[now.piece], (const char *)seg[g].dev + now.at, now.n, s->stream)) ||
-                (rc = spgk_event_record(s->landed[now.piece], s->stream))) return rc;
-            s->busy[now.piece] = true;
+                (rc = stager_queued(s, now.piece))) return rc;
         }
         if (before.piece >= 0) {
-            s->busy[before.piece] = false;
-            if ((rc = spgk_event_sync(s->landed[before.piece]))) return rc;
+            if ((rc = stager_wait(s, before.piece))) return rc;
             if (!sink(seg[before.seg].ctx, before.at, s->piece[before.piece], before.n)) return SPGK_E_ARG;
         }
         if (now.piece < 0) return SPGK_OK;

@@ -122,6 +122,11 @@ def test_orders_of_a_training_call_without_page_locked_memory(tmp_path):
     assert r.returncode == 0 and r.stdout == "every order\n", (r.returncode, r.stdout, r.stderr)
 
 
+def test_pieces_in_use_are_not_handed_out(tmp_path):
+    r = subprocess.run([on_fake_kernels(tmp_path, "pieces")], capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0 and r.stdout == "every piece at rest\n", (r.returncode, r.stdout, r.stderr)
+
+
 @pytest.mark.parametrize("asked", ["", "5"])
 def test_callers_at_the_same_time_share_the_cores(tmp_path, asked):
     host, exe = os.path.join(ROOT, "spingalett_b200", "csrc", "host"), str(tmp_path / "bulk_callers")
