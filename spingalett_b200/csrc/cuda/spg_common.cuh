@@ -23,6 +23,7 @@ int  spgk_check_launch(const char *kernel_name);
     do {                                                                         \
         cudaError_t e__ = (call);                                                \
         if (e__ != cudaSuccess) {                                                \
+            cudaGetLastError();     /* reported here: not the next launch's */   \
             spgk_set_error(#call, cudaGetErrorString(e__));                      \
             return e__ == cudaErrorMemoryAllocation ? SPGK_E_NOMEM : SPGK_E_CUDA; \
         }                                                                        \

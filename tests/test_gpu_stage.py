@@ -1,5 +1,6 @@
 """Arrays that go to and from the device through page-locked pieces of 8 MB (spg_stage.c): lengths around a piece, saved files byte for byte against
 the host encoder, trained nets bit for bit against copies of page-locked arrays."""
+import ctypes as C
 import os
 
 import numpy as np
@@ -52,3 +53,17 @@ def test_training_from_pageable_and_page_locked_arrays_is_the_same(spg, samples)
         net.free()
     for a, b in zip(*got):
         assert np.any(a != 0) and np.array_equal(a, b)
+
+
+def test_a_failed_allocation_is_not_the_next_launchs_error(spg):
+    """Room for pieces, orders and encoders is asked for and done without where there is none: the failure must not be left for a launch to find."""
+    lib = spg.lib()
+    lib.spgk_malloc.argtypes = [C.POINTER(C.c_void_p), C.c_size_t]
+    net = spg.Network.build([40, 30, 10], [spg.abi.ACT_RELU, spg.abi.ACT_SOFTMAX], spg.abi.WEIGHT_INITIALIZATION_NONE)
+    net.weights[:] = 1.0
+    x = np.ones((3, 40), np.float32)
+    want = net.forward_batch(x)
+    p = C.c_void_p()
+    assert lib.spgk_malloc(C.byref(p), 1 << 50) != 0
+    assert np.array_equal(net.forward_batch(x), want)
+    net.free()
