@@ -78,7 +78,7 @@ def arithmetic(path, dtype, math):
     if path == "istream" or path == "gemv" and dtype in ("int8", "int4", "int2"):
         return "s8 digits x s8 -> s32 (exact sums of 28-bit fixed-point activations)"
     if path == "rows":
-        return "f64 products and sums"
+        return "f32 products and sums of four, f64 sums of those"
     if path in ("gemv", "wstream"):
         return "bf16 terms x bf16 -> f32 (exact products)"
     return {"exact": "bf16(hi+lo)xbf16->f32", "fast": "f16xf16->f32", "auto": "f16xf16->f32 + exact recompute of low-margin rows"}[math]
@@ -86,6 +86,13 @@ def arithmetic(path, dtype, math):
 
 KERNEL_OF_PATH = {"rows": "spg_rows_kernel", "gemv": "spg_gemv_kernel", "istream": "spg_istream_kernel", "wstream": "spg_wstream_kernel", "tcgen05": "spg_gemm_tc_kernel",
                   "tcgen05-fused": "spg_mlp3_fused_kernel", "simt": "spg_layer_simt_kernel"}
+
+
+def kernels(path, topo, batch):
+    """The path's kernel, and with it the one on pairs of CTAs where layers have more 128 x 256 tiles than the GPU has SMs."""
+    name = KERNEL_OF_PATH.get(path, path)
+    pairs = path == "tcgen05" and any(-(-batch // 128) * -(-b // 256) > 148 and a >= 512 and b > 128 for a, b in zip(topo, topo[1:]))
+    return "spg_gemm_pair_kernel, " + name if pairs else name
 
 
 def parse():
@@ -582,7 +589,7 @@ def main():
             traffic = json.load(open(tpath)).get(f"{args.workload}_{args.dtype}_{args.math}_{batch}")
         line["roofline"] = {"bound": "tensor", "achieved": achieved, "peak": pk["bf16_tflops"], "unit": "TFLOP/s",
                             "frac": achieved / pk["bf16_tflops"], "traffic": traffic,
-                            "kernel": KERNEL_OF_PATH.get(path_taken, path_taken),
+                            "kernel": kernels(path_taken, args.topo, batch),
                             "launches": int(k_cnt), "kernel_ms_per_step": k_ms_eff / args.steps,
                             "peak_source": pk["source"] + " burst bf16", "tensor_passes_per_product": passes,
                             "executed_frac": achieved * passes / pk["bf16_tflops"],
@@ -600,7 +607,7 @@ def main():
             traffic = json.load(open(tpath)).get(f"{args.workload}_{args.dtype}_{batch}")
         line["roofline"] = {"bound": "hbm", "achieved": achieved, "peak": pk["hbm_gbs"], "unit": "GB/s",
                             "frac": achieved / pk["hbm_gbs"], "traffic": traffic,
-                            "kernel": KERNEL_OF_PATH.get(path_taken, path_taken),
+                            "kernel": kernels(path_taken, args.topo, batch),
                             "launches": int(k_cnt), "kernel_ms_per_step": k_ms / args.steps,
                             "algorithmic_bytes_per_step": nbytes, "peak_source": pk["source"] + " copy bandwidth",
                             "whole_step_frac": nbytes / (dev_ms * 1e-3) / 1e9 / pk["hbm_gbs"],

@@ -27,9 +27,10 @@ def test_products_of_many_tiles(spg, lib, M, N, K, t16, a_parts, w_parts):  # no
             assert np.all(o16[1] == 7.0)
 
 
-@pytest.mark.parametrize("N,K", [(2048, 300), (8200, 200)])
-def test_counted_rows(spg, lib, N, K):  # noqa: F811
-    """Any count under any guess, on pairs (whose width hangs on the guess) and on single CTAs: same bits, nothing beyond the count."""
+@pytest.mark.parametrize("N,K,shared", [(2048, 300, {1, 2}), (8200, 200, {2})])
+def test_counted_rows(spg, lib, N, K, shared):  # noqa: F811
+    """Any count under any guess, on pairs (whose width hangs on the guess) and, where a guess gives few tiles, on single CTAs: same bits, nothing beyond
+    the count."""
     import torch
     cap = 2600
     z, size, run = product(spg, lib, cap, N, K, 2, 1, 1, 1, seed=N)
@@ -50,4 +51,4 @@ def test_counted_rows(spg, lib, N, K):  # noqa: F811
             assert np.all(o32[count:] == -3.0) and np.all(o16[:, count:] == 7.0)
     finally:
         lib.spgk_set_dynamic_rows(None, 0)
-    assert {s for _, s in seen} >= {2} and len(seen) >= 2
+    assert {s for _, s in seen} == shared and len(seen) >= 2, seen
