@@ -40,7 +40,17 @@ struct RowsParams {
 template <int PREC> constexpr int UNIT = PREC == SPG_P_I8 ? 9 : PREC == SPG_P_I4 ? 5 : PREC == SPG_P_I2 ? 3 : 0;
 template <int PREC> constexpr float ONE = 1.0f / (float)(1 << UNIT<PREC>);
 
-// the weights e .. e + 7 of the matrix, in those units
+// weight e of the matrix in those units
+template <int PREC> __device__ __forceinline__ float decode1(const void *w, uint64_t e)
+{
+    if constexpr (PREC == SPG_P_I4)
+        return (float)(int)((uint32_t)reinterpret_cast<const uint8_t *>(w)[e >> 1] << (28 - 4 * (uint32_t)(e & 1)) & 0xF0000000u) * (ONE<PREC> / (1u << 28));
+    else if constexpr (PREC == SPG_P_I2)
+        return (float)(int)((uint32_t)reinterpret_cast<const uint8_t *>(w)[e >> 2] << (30 - 2 * (uint32_t)(e & 3)) & 0xC0000000u) * (ONE<PREC> / (1u << 30));
+    else return spg_decode_elem(w, e, PREC) * ONE<PREC>;
+}
+
+// the weights e .. e + 7
 template <int PREC> __device__ __forceinline__ void decode8(const void *w, uint64_t e, float (&q)[8])
 {
     if constexpr (PREC == SPG_P_F32) {
@@ -88,7 +98,7 @@ __device__ __forceinline__ void dot(const RowsParams &p, uint32_t j, uint32_t n0
             if (p.vec_w && k < p.in) decode8<PREC>(p.w, row + k, q[u]);        // (then `in` is a multiple of eight)
             else {
 #pragma unroll
-                for (uint32_t i = 0; i < GROUP; i++) q[u][i] = k + i < p.in ? spg_decode_elem(p.w, row + k + i, PREC) * ONE<PREC> : 0.0f;
+                for (uint32_t i = 0; i < GROUP; i++) q[u][i] = k + i < p.in ? decode1<PREC>(p.w, row + k + i) : 0.0f;
             }
         }
         if (wait) { spg_grid_wait(); wait = false; }
