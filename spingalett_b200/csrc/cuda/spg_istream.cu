@@ -25,11 +25,12 @@
 // 106 us over the net, whose busiest SMs have 237 such blocks.  One byte per weight in the operand instead of two is why this
 // path exists beside the 16-bit streaming kernel, which writes and reads 32 KB per such block.
 //
-// Measured: 125 us at 8 rows (GEMV: 201), 166 at 64 (16-bit streaming kernel: 577), 460 at 256 (GEMM chain: 684).  A block of
-// INT4 takes 480 cycles at 8 rows, of which the MMA warp's own turn is all (operand tiles changing hands one at a time: 810).
+// Measured, large INT4 net, inputs new in every call: 125 us at 8 rows (GEMV: 201), 171 at 64 (16-bit streaming kernel: 577), 498 at 256 (GEMM chain:
+// 684).  A block of INT4 takes 480 cycles at 8 rows, of which the MMA warp's own turn is all (operand tiles changing hands one at a time: 810).
 // At 64 rows a CTA alone draws 32 KB of digits a block from L2, at 43 bytes a cycle: 750 cycles; the tensor pipe would need
-// 512.  Large layers of more than 32 rows a group therefore run on pairs of CTAs (cta_group::2), each with half of the digits:
-// INT4 176 -> 166 us at 64 rows, 257 -> 229 at 96, 552 -> 460 at 256; INT2 452 -> 404, INT8 656 -> 568 at 256.  From layers of 32 to 166 blocks with weights from HBM: 530 cycles a block and 14 us a layer at 8 rows, 870 and 16 at 64.
+// 512.  Layers of more than 32 rows a group in which a CTA has many blocks in a row therefore run on pairs of CTAs (cta_group::2), each with half of the
+// digits: a layer of 16384 x 8192 at 40, 64, 96, 256 rows 40.0 -> 35.5, 42.1 -> 40.6, 61 -> 56, 114 -> 104 us, its tensor pipe 69 % busy at 64 rows
+// while it runs; the net 187 -> 171 us at 64 rows, 554 -> 498 at 256; with twelve batches in turn INT4 167 and 443, INT2 163 and 406, INT8 181 and 524.  From layers of 32 to 166 blocks with weights from HBM: 530 cycles a block and 14 us a layer at 8 rows, 870 and 16 at 64.
 // INT8, whose boxes need no unpacking, takes 700 cycles at 8 rows, 5.5 TB/s.  The rest of a layer is staging, the first
 // boxes and tiles, and the last sums (1 us at 8 rows, 3 at 64).
 //

@@ -7,13 +7,14 @@
 // registers, decoded, before the layer before it has ended (programmatic dependent launch); then come the input (8 neighbouring
 // values a lane, all loads of a round in flight), the products, four of them added in fp32 and the fours in 64 bits, and a shuffle
 // tree.  (Every product in 64 bits: as accurate as the last rounding allows, and 2 to 4 us slower from six rows on, a conversion
-// runs at 14 a cycle and SM.)  A warp takes 1.2 to 1.7 us for 1024 elements of a row, so rows of more than 2048 are shared by four or eight
-// warps: one row of 65536-64-10 INT8 109 -> 18 us, of 4096-10 8.8 -> 5.
+// runs at 14 a cycle and SM.)  A warp takes 1.2 to 1.7 us for 1024 elements of a row, so rows of more than 2048 are shared by up to eight
+// warps: 65536-64-10 INT8 at one row 110 -> 18 us, 4096-1000 12.9 -> 8.7.  Rows of at most 256 have a kernel that has no more than those in
+// flight (30 to 61 registers instead of 56 to 70): 250-250-250-250-10 in 0.9 of the time.
 //
 // What bounds it: 3 us a layer of launch, two L2 latencies and the tree; beyond four rows the loads of the inputs.  Before (the
 // weight-streaming GEMV, made to keep HBM busy, or the general kernel where rows are no multiple of 16 bytes) and now, us a call:
-// 784-512-1000-10 at one row fp32 29.8 -> 10, INT8 45 -> 10, INT4 24.7 -> 9.4; at eight rows fp32 90 -> 12, INT4 115 -> 10;
-// 301-777-333-129-37 fp32 at one row 22.6 -> 12.4, at eight 103 -> 18.5; 1024-1024-1024-1024-16 BF16 35 -> 12 and 117 -> 23.
+// 784-512-1000-10 at one row fp32 31.6 -> 8.0, INT8 46 -> 7.8, INT4 26 -> 7.9; at eight rows fp32 90 -> 12, INT4 118 -> 10.4;
+// 301-777-333-129-37 fp32 at one row 22.6 -> 12 to 17, at eight 103 -> 19; 1024-1024-1024-1024-16 BF16 35 -> 12.5 and 117 -> 23.
 // forward() of one sample 57 -> 36 (28 of them launches, device time and the wait).  Error against 64 bits 5e-8 to 2e-7 (before:
 // 1e-7 to 5e-6).  An input that travels as a parameter of the first launch instead of through the fetch kernel: level.
 //

@@ -1138,8 +1138,8 @@ static float *forward_batch_on(spg_net *n, ForwardBatchArgs a)
      * to 8 rows go through spg_dev_forward_small (nets of few weights warp by warp, others GEMV first), up to 512 rows in groups of at most 128 through the 16-bit streaming kernel when
      * it takes every layer, each group streaming the packed weights once; everything else is the large-batch GEMM chain.
      *
-     * Measured, against the path that served before: large INT4 net 126 us against 204 (GEMV) at 8 rows, 188 against 578
-     * (16-bit streaming kernel) at 64, 555 against 684 (GEMM chain) at 256.  Nets of 4 and 12 MB: 33 against 54 and 36 against
+     * Measured, against the path that served before: large INT4 net 125 us against 204 (GEMV) at 8 rows, 171 against 578
+     * (16-bit streaming kernel) at 64, 498 against 684 (GEMM chain) at 256.  Nets of 4 and 12 MB: 33 against 54 and 36 against
      * 65 us at 8 rows, 0.45 of the time or less at 32 to 96; of 0.5 MB: 32 against 119 us at 8 rows.  The lines were drawn where
      * the curves of older kernels crossed: the one at 7 rows when 8 rows took 157 us here (the GEMV: 155 at 6, INT2 132), the
      * ones at 96 rows and 4 MB before products of few tiles had a kernel of their own (0.5 MB: 41 us here at 96 rows, 22 on the
