@@ -67,6 +67,7 @@ struct GemmParams {
     float margin_theta; uint32_t *margin_idx, *margin_count;
     const uint32_t *out_rows;     // optional scatter of the fp32 output rows   // fused-softmax rows with top-two logit gap < theta are appended here (optional)
     int tma_store;                // 16-bit output leaves through TMA stores (one plane, tiles at least 128 wide)
+    uint32_t vec32;               // rows of the fp32 output lie on 16 bytes
     uint32_t a_terms, w_terms;    // pairs of CTAs: terms of a stage
     const uint32_t *m_limit;      // optional device-resident row count: the kernel works on min(M, *m_limit) rows ...
     uint32_t m_above;             // ... or on none, if they are no more than this (spg_gemm_split_kernel has them)
@@ -176,7 +177,7 @@ __device__ __forceinline__ void finish16(const GemmParams &p, const uint32_t (&r
 __device__ __forceinline__ void write32(const GemmParams &p, uint32_t row, uint32_t col0, const float (&v)[16])
 {
     float *o = p.out32 + (uint64_t)(p.out_rows ? p.out_rows[row] : row) * p.ldo32 + col0;
-    if ((p.ldo32 & 3u) == 0 && col0 + 16 <= p.N) {
+    if (p.vec32 && col0 + 16 <= p.N) {
 #pragma unroll
         for (int i = 0; i < 16; i += 4)
             *reinterpret_cast<float4 *>(o + i) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
@@ -469,7 +470,7 @@ __device__ __forceinline__ void epilogue_softmax_wide(const GemmParams &p, const
             const uint32_t col0 = nt * p.BN, cols = p.N - col0 < p.BN ? p.N - col0 : p.BN;
             const uint32_t taddr = tmem_base + acc * p.BN + ((q * 32u) << 16);
             float *orow_ptr = p.out32 + (uint64_t)orow * p.ldo32 + col0;
-            const bool vec = (p.ldo32 & 3u) == 0 && (reinterpret_cast<uintptr_t>(p.out32) & 15u) == 0;      // 16-byte stores (BN is a multiple of 4)
+            const bool vec = p.vec32;                                    // (BN is a multiple of 4)
             for (uint32_t c0 = 0; c0 < cols; c0 += 16) {
                 uint32_t r[16];
                 tmem_ld16(taddr + c0, r);
@@ -1084,6 +1085,7 @@ static int gemm_launch(const spgk_layer *L,
     p.own_rows = (head || (softmax_fused && p.n_tiles != 1)) ? 1u : 0u;
     p.out16 = out16; p.ldo16 = ldo16; p.o_plane = o_plane; p.out_parts = out_parts; p.type16 = type16;
     p.out32 = out32; p.ldo32 = ldo32;
+    p.vec32 = (ldo32 & 3u) == 0 && ((uintptr_t)out32 & 15u) == 0;
     p.status = status;
     p.m_limit = spg_tls_rows_limit; p.m_above = served;
     if ((softmax_fused || (head && head->act == SPG_ACT_SOFTMAX)) && spg_tls_margin_idx) { p.margin_theta = spg_tls_margin_theta; p.margin_idx = spg_tls_margin_idx; p.margin_count = spg_tls_margin_count; }
