@@ -408,7 +408,7 @@ SPINGALETT_API void spingalett_profile_read(NeuralNetwork *net, double *kernel_m
  * name of the compute path the last batched/forward call took ("gemv",
  * "rows" -- nets of few weights on up to eight rows --,
  * "istream" -- integer files through the 8-bit integer tensor path --, "wstream",
- * "tcgen05", "tcgen05-fused" -- the three-layer net in one launch --, "simt").  For benchmarks and tests. */
+ * "tcgen05", "tcgen05-fused" -- the one-term pass of a three-layer net in one launch --, "simt").  For benchmarks and tests. */
 SPINGALETT_API uint64_t spingalett_kernel_launches(void);
 SPINGALETT_API const char *spingalett_last_path(void);
 

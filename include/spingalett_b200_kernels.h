@@ -323,6 +323,22 @@ SPGK_API int spgk_layer_gemm_tc_head(const spgk_layer *L,
                                      const void *a16, uint32_t lda, uint64_t a_plane, int a_parts, int type16,
                                      const spgk_layer *head, const float *head_w, float *out32, uint32_t ldo32,
                                      uint32_t N, int32_t *status, void *stream);
+/* A whole net of 2 to SPGK_CHAIN_MAX_LAYERS layers on N rows in one launch (spg_chain.cu), for batches too small to fill the device layer by
+ * layer.  spgk_chain_plan decides how (SPGK_E_UNSUPPORTED: not at all) and says how much scratch that takes and what it is estimated
+ * to cost; spgk_chain_forward launches it.
+ *   w16/ldw/w_plane/w_parts: every layer's 16-bit weight operand as for spgk_layer_gemm_tc; a_parts: terms of an activation (type16);
+ *   x: fp32 rows, row r of the batch at x_rows[r] where x_rows is given; y: fp32 rows (spgk_set_output_rows);
+ *   softmax_fused: the last layer's softmax is applied here (at most 128 columns), else a softmax layer leaves logits;
+ *   weights_ready: no kernel in front of this one in the stream writes w16 or a bias (they are read under its tail).
+ * Honours spgk_set_dynamic_rows and spgk_set_margin_sink.  A row's result depends on neither N nor the plan. */
+#define SPGK_CHAIN_MAX_LAYERS 8
+typedef struct { uint32_t C, R, clusters, exchange_bytes; uint64_t scratch_bytes; float us, layered_us; } spgk_chain;
+SPGK_API int spgk_chain_plan(const spgk_layer *layers, uint32_t count, uint32_t N, int w_parts, int a_parts, int softmax_fused, spgk_chain *plan);
+SPGK_API int spgk_chain_forward(const spgk_chain *plan, const spgk_layer *layers, uint32_t count, const void *const *w16, const uint32_t *ldw,
+                                const uint64_t *w_plane, int w_parts, int type16, int a_parts, const float *x, uint32_t ldx, const uint32_t *x_rows,
+                                uint32_t N, float *y, uint32_t ldy, int softmax_fused, int weights_ready, void *scratch, int32_t *status, void *stream);
+/* (checks) CTAs of a cluster and rows of a block of the calling thread's last spgk_chain_forward */
+SPGK_API void spgk_chain_arrangement(uint32_t out[2]);
 SPGK_API int spgk_gemm_tc_status(int32_t *status, void *stream);
 
 /* ---- K2f: a three-layer MLP in one launch (large batches) ----------------------
@@ -352,6 +368,8 @@ SPGK_API int spgk_gemm_tc_status(int32_t *status, void *stream);
  * spgk_mlp3_supported() == 0 (other depths, hidden width above 512, head wider than 16, unaligned
  * input rows) means: run the layers one by one with spgk_layer_gemm_tc. */
 SPGK_API int spgk_mlp3_supported(const spgk_layer *L1, const spgk_layer *L2, const spgk_layer *L3, uint32_t ldx);
+/* an estimate of its microseconds for N rows */
+SPGK_API float spgk_mlp3_us(const spgk_layer *L1, const spgk_layer *L2, uint32_t N);
 SPGK_API size_t spgk_mlp3_params_bytes(const spgk_layer *L1, const spgk_layer *L2, const spgk_layer *L3);
 SPGK_API int spgk_mlp3_params(const spgk_layer *L1, const spgk_layer *L2, const spgk_layer *L3, int type16, float *dst, void *stream);
 SPGK_API int spgk_mlp3_forward(const spgk_layer *L1, const void *w1_16, uint32_t ldw1,

@@ -26,3 +26,6 @@ int spg_gemm_map(CUtensorMap *map, const void *base, int type16, uint32_t K, uin
 // Launches the few-tiles kernel if it has an arrangement for this product.  SPGK_E_UNSUPPORTED: the persistent kernel is needed, for
 // row counts above `served` (0: for all, nothing was launched).
 int spg_gemm_split_try(const SpgGemmArgs &a, const SpgDeviceProps &dp, int dev, uint32_t &served);
+
+// spgk_selftest_impatient
+bool spg_gemm_impatient();

@@ -539,4 +539,5 @@ int spg_gemm_split_try(const SpgGemmArgs &a, const SpgDeviceProps &dp, int dev, 
     return split_launch(a, at, plan, { limit, ~0u, ~0u });
 }
 
+bool spg_gemm_impatient() { return spg_tls_impatient; }
 extern "C" void spgk_selftest_impatient(int on) { spg_tls_impatient = on != 0; }

@@ -966,6 +966,18 @@ int spgk_mlp3_supported(const spgk_layer *L1, const spgk_layer *L2, const spgk_l
     return (dp.cc == 100 && dp.smem_optin >= SMEM_TOTAL) ? 1 : 0;
 }
 
+// 1024 to 18000 rows (one tile a pair) in us: 784-512-1000-10 31, 784-256-256-10 18, 256-256-256-10 12.5, 64-64-64-4 8.2, 512-512-512-16 21.5,
+// 1024-512-1024-16 33.8, 128-512-1000-10 24.5; every further tile of a pair 0.55 to 0.85 of that
+float spgk_mlp3_us(const spgk_layer *L1, const spgk_layer *L2, uint32_t N)
+{
+    SpgDeviceProps dp;
+    if (!L1 || !L2 || spg_device_props(&dp) != SPGK_OK || dp.sm_count < 2) return 0.0f;
+    const float kb1 = (float)((L1->in + BK - 1) / BK), kb2 = (float)((L1->out + BK - 1) / BK), ch1 = (float)((L1->out + 255u) / 256u), ch2 = (float)((L2->out + 255u) / 256u);
+    const float tile = 0.35f * (kb1 * (1.0f + 0.5f * ch1) + kb2 * ch2) + 1.5f * ch2;
+    const uint32_t tiles = (N + 255u) / 256u, pairs = (uint32_t)dp.sm_count / 2;
+    return 6.5f + tile * (float)((tiles + pairs - 1) / pairs);
+}
+
 size_t spgk_mlp3_params_bytes(const spgk_layer *L1, const spgk_layer *L2, const spgk_layer *L3)
 {
     if (!L1 || !L2 || !L3) return 0;

@@ -137,6 +137,7 @@ void spg_dev_release(spg_net *n)
         spgk_free(n->d_act32[i]); n->d_act32[i] = NULL;
     }
     n->act16_bytes = 0; n->act32_bytes = 0;
+    spgk_free(n->d_chain); n->d_chain = NULL; n->chain_bytes = 0;
     spgk_free(n->d_status); n->d_status = NULL;
     spgk_free(n->d_w16); n->d_w16 = NULL; n->w16_bytes = 0;
     spgk_free(n->d_head_w); n->d_head_w = NULL;
@@ -698,6 +699,63 @@ static bool bf16_file_as_f16(spg_net *n)
 static _Thread_local bool dynamic_rows = false;      /* true around the repair chain of the AUTO mode */
 static _Thread_local const uint32_t *repair_rows = NULL;   /* repair chain: input row i is row repair_rows[i] of d_x, and its result goes back there */
 
+/* 16-bit flavour of a chain: the file's own 16-bit type when it has one (exact weights); otherwise fp16 for the one-term mode (11
+ * significant bits) and bf16 for the two-term mode (fp32 range, 16 bits over two terms). */
+static int chain_type(spg_net *n, bool exact)
+{
+    const int prec = n->klayers[0].precision;
+    if (prec == PRECISION_FP16) return SPGK_T_F16;
+    if (prec == PRECISION_BFLOAT16) return exact || !bf16_file_as_f16(n) ? SPGK_T_BF16 : SPGK_T_F16;
+    return exact ? SPGK_T_BF16 : SPGK_T_F16;
+}
+
+/* The whole net in one launch: whether it takes this net and as many rows sooner than the layers one by one would, and how.  (Weights that
+ * are not kept as 16-bit operands, and softmax rows that do not end in it, stay with those.) */
+#define SPG_CHAIN_SOFTMAX 128u
+static int whole_plan(spg_net *n, uint32_t N, bool exact, spgk_chain *plan, bool *takes)
+{
+    *takes = false;
+    *plan = (spgk_chain){ 0 };
+    const uint32_t layers = n->dev_layers;
+    const spgk_layer *last = &n->klayers[layers - 1];
+    const bool softmax = last->act == ACT_SOFTMAX;
+    if (layers > SPGK_CHAIN_MAX_LAYERS || (softmax && last->out > SPG_CHAIN_SOFTMAX)) return SPINGALETT_OK;
+    for (uint32_t l = 0; l + 1 < layers; l++) if (n->klayers[l].act == ACT_SOFTMAX) return SPINGALETT_OK;
+    if (!weights_keepable(n, chain_type(n, exact), exact)) return SPINGALETT_OK;
+    const int rc = spgk_chain_plan(n->klayers, layers, N, exact && last->precision == PRECISION_FLOAT32 ? 2 : 1, exact ? 2 : 1, softmax, plan);
+    if (rc == SPGK_E_UNSUPPORTED) return SPINGALETT_OK;
+    *takes = rc == SPGK_OK && plan->clusters && plan->us <= plan->layered_us;
+    return spg_map_kernel_error(rc, "net in one launch");
+}
+
+static int whole_net(spg_net *n, const spgk_chain *plan, const float *d_x, uint32_t N, float *d_out, bool exact)
+{
+    const uint32_t layers = n->dev_layers;
+    const spgk_layer *last = &n->klayers[layers - 1];
+    const int type = chain_type(n, exact), parts = exact ? 2 : 1, w_parts = exact && last->precision == PRECISION_FLOAT32 ? 2 : 1;
+    int rc = reserve(&n->d_chain, &n->chain_bytes, (size_t)plan->scratch_bytes, "operands between layers");
+    if (rc) return rc;
+    const void *w16[SPGK_CHAIN_MAX_LAYERS];
+    uint32_t ldw[SPGK_CHAIN_MAX_LAYERS];
+    uint64_t w_plane[SPGK_CHAIN_MAX_LAYERS];
+    bool ready = true;                          /* no operand is made in front of this launch */
+    for (uint32_t l = 0; l < layers; l++) {
+        const bool there = spgk_weights16_direct(&n->klayers[l], type) || (n->d_w16c[type] && n->d_w16c[type][l]);
+        if ((rc = kept_weight_operand(n, type, l, w_parts, true, &w16[l], &ldw[l], &w_plane[l]))) return rc;
+        ready = ready && there;
+    }
+    if (!dynamic_rows) prof_mark(n);            /* the timing marks cover the full passes, not the repair of a few rows */
+    spgk_set_output_rows(repair_rows);
+    rc = spg_map_kernel_error(spgk_chain_forward(plan, n->klayers, layers, w16, ldw, w_plane, w_parts, type, parts, d_x, n->pub.topology[0], repair_rows,
+                                                 N, d_out, last->out, last->act == ACT_SOFTMAX, ready, n->d_chain, n->d_status, n->stream), "net in one launch");
+    spgk_set_output_rows(NULL);
+    if (!dynamic_rows) prof_mark(n);
+    if (rc) return rc;
+    n->status_pending = true;
+    spg_note_path("tcgen05");
+    return SPINGALETT_OK;
+}
+
 static int large_chain(spg_net *n, const float *d_x, uint32_t N, float *d_out, bool exact)
 {
     NeuralNetwork *p = &n->pub;
@@ -706,14 +764,12 @@ static int large_chain(spg_net *n, const float *d_x, uint32_t N, float *d_out, b
     for (uint32_t l = 0; l + 1 < n->dev_layers; l++) tc = tc && n->klayers[l].act != ACT_SOFTMAX;   /* softmax only as the last layer */
     if (!tc) return large_simt(n, d_x, N, d_out);
 
-    const int prec = n->klayers[0].precision;
-    /* 16-bit flavour: the file's own 16-bit type when it has one (exact
-     * weights); otherwise fp16 for the one-term mode (11 significant bits) and
-     * bf16 for the two-term mode (fp32 range, 16 bits over two terms). */
-    const int type = prec == PRECISION_FP16 ? SPGK_T_F16
-                   : prec == PRECISION_BFLOAT16 ? ((exact || !bf16_file_as_f16(n)) ? SPGK_T_BF16 : SPGK_T_F16)
-                   : exact ? SPGK_T_BF16 : SPGK_T_F16;
-    const int parts = exact ? 2 : 1;
+    spgk_chain whole;
+    bool takes;
+    int rc = whole_plan(n, N, exact, &whole, &takes);
+    if (rc) return rc;
+    if (takes) return whole_net(n, &whole, d_x, N, d_out, exact);
+    const int type = chain_type(n, exact), parts = exact ? 2 : 1;
     uint32_t maxld = 0;
     for (uint32_t l = 0; l + 1 < p->layers; l++) if (round8(p->topology[l]) > maxld) maxld = round8(p->topology[l]);
     const uint64_t plane = (uint64_t)N * maxld;
@@ -722,7 +778,7 @@ static int large_chain(spg_net *n, const float *d_x, uint32_t N, float *d_out, b
         for (int i = 0; i < 2; i++) { spgk_free(n->d_act16[i]); n->d_act16[i] = NULL; }
         n->act16_bytes = 0;
         for (int i = 0; i < 2; i++) {
-            int rc = spg_map_kernel_error(spgk_malloc(&n->d_act16[i], need), "16-bit activation workspace");
+            rc = spg_map_kernel_error(spgk_malloc(&n->d_act16[i], need), "16-bit activation workspace");
             if (rc) return rc;
         }
         n->act16_bytes = need;
@@ -739,7 +795,6 @@ static int large_chain(spg_net *n, const float *d_x, uint32_t N, float *d_out, b
         }
     }
     const bool keep = wtotal && wtotal <= SPG_W16_KEEP_MAX;
-    int rc;
     if (!keep && wneed && (rc = reserve(&n->d_w16, &n->w16_bytes, wneed, "16-bit weight operand scratch"))) return rc;
     rc = spg_map_kernel_error(spgk_split16_rows(d_x, p->topology[0], repair_rows, N, p->topology[0], n->d_act16[0],
                                                 round8(p->topology[0]), plane, parts, type, n->stream), "input split");
@@ -816,6 +871,19 @@ static bool fused_eligible(spg_net *n, const float *d_x, uint32_t N)
     return weights_keepable(n, fast_type(n), false);
 }
 
+/* Nets that the chains take at any number of rows: every layer on the tensor cores, 16-bit operands well inside L2 */
+#define SPG_LIGHT_BYTES ((uint64_t)64 << 20)
+static bool light_operands(spg_net *n)
+{
+    uint64_t bytes = 0;
+    for (uint32_t l = 0; l < n->dev_layers; l++) {
+        const spgk_layer *L = &n->klayers[l];
+        if (!spgk_gemm_tc_supported(L) || (L->act == ACT_SOFTMAX && l + 1 < n->dev_layers)) return false;
+        bytes += (uint64_t)L->in * L->out * (L->precision == PRECISION_FLOAT32 ? 4 : 2);
+    }
+    return bytes <= SPG_LIGHT_BYTES && bytes <= SPG_W16_KEEP_MAX;
+}
+
 /* one launch over N rows (or over the rows of a device-resident list): the one-term pass, or with pairs the
  * two-term recomputation of the listed rows written over their one-term results */
 static int fused_pass(spg_net *n, const float *d_x, uint32_t N, float *d_out, bool pairs,
@@ -859,9 +927,22 @@ int spg_dev_forward_large(spg_net *n, const float *d_x, uint32_t N, float *d_out
     const uint32_t in0 = p->topology[0], outw = p->topology[p->layers - 1];
     const bool softmax_out = p->act_func[p->layers - 2] == ACT_SOFTMAX && outw >= 2;
     /* a three-layer net with a narrow last layer runs its one-term passes as ONE kernel (no activation matrix in HBM) */
-    const bool fused = fused_eligible(n, d_x, N);
+    int rc;
+    spgk_chain whole = { 0 };
+    bool takes, fused = fused_eligible(n, d_x, N);
+    const char *const one_launch = fused ? "tcgen05-fused" : "tcgen05";        /* (the name of its path, on whichever kernel) */
+    const float fused_us = fused ? spgk_mlp3_us(&n->klayers[0], &n->klayers[1], N) : 0.0f;
+    if (fused && mode != SPINGALETT_MATH_EXACT) {
+        /* some thousand rows are too few pairs of tiles for it: 2000 rows of the benchmark MLP 31 us there, 18 as a chain of one launch */
+        if ((rc = whole_plan(n, N, false, &whole, &takes))) return rc;
+        if (takes && whole.us < fused_us) fused = false;
+    }
     if (mode == SPINGALETT_MATH_FAST && fused) return fused_pass(n, d_x, N, d_out, false, NULL, NULL, 0, 0.0f, NULL, NULL);
-    if (mode != SPINGALETT_MATH_AUTO) return large_chain(n, d_x, N, d_out, mode == SPINGALETT_MATH_EXACT);
+    if (mode != SPINGALETT_MATH_AUTO) {
+        rc = large_chain(n, d_x, N, d_out, mode == SPINGALETT_MATH_EXACT);
+        if (!rc && mode == SPINGALETT_MATH_FAST && whole.clusters) spg_note_path(one_launch);
+        return rc;
+    }
     if (!softmax_out) return large_chain(n, d_x, N, d_out, true);
     /* Few rows: the chain is bound by streaming the weights (or by latency), where the exact chain's second pass over K
      * is nearly free, while the one-term pass plus the recomputation chain costs two chains: 0.70 ms against 1.05 ms at
@@ -869,7 +950,6 @@ int spg_dev_forward_large(spg_net *n, const float *d_x, uint32_t N, float *d_out
      * tiles had a kernel of their own). */
     if (N <= SPG_AUTO_EXACT_ROWS) return large_chain(n, d_x, N, d_out, true);
 
-    int rc;
     /* the list of rows stands behind a head of 256 bytes: [0] the number of rows, which every call leaves at zero, [8] the calibration's word */
     const size_t list_bytes = (size_t)N * 4 + 256;
     if (n->rep_idx_bytes < list_bytes) n->count_clean = false;       /* (by its size: a list that has grown may lie where it lay before) */
@@ -893,7 +973,6 @@ int spg_dev_forward_large(spg_net *n, const float *d_x, uint32_t N, float *d_out
     }
     if (rc) return rc;
     if (strncmp(spingalett_last_path(), "tcgen05", 7) != 0) return SPINGALETT_OK;  /* the fp32 chain ran: nothing to repair */
-    const bool fused_pass_ran = fused;
     theta = spingalett_get_auto_margin();
     if (theta <= 0.0f) {
         /* Self-calibration, once per device image of the net: run both modes on up to 2048 rows, measure the
@@ -971,7 +1050,7 @@ int spg_dev_forward_large(spg_net *n, const float *d_x, uint32_t N, float *d_out
     if (rc) return rc;
     if ((rc = spg_map_kernel_error(spgk_count_take(d_count, h_slot, n->stream), "repair count"))) return rc;
     n->count_pending = true; n->count_seen = true; n->count_clean = captured ? clean_before : true;
-    spg_note_path(fused_pass_ran ? "tcgen05-fused" : "tcgen05");
+    spg_note_path(one_launch);
     return SPINGALETT_OK;
 }
 
@@ -1168,7 +1247,11 @@ static float *forward_batch_on(spg_net *n, ForwardBatchArgs a)
     /* from about a hundred rows on the GEMM chain on kept 16-bit operands (0.70 ms at 128 and at 256 rows of the large
      * INT4 net, two-term) beats the streaming kernel (0.58 ms at 64 rows, 0.88 ms at 128, 1.77 ms for the two passes of
      * 256) whenever those operands fit the keep budget */
-    const bool chain_kept = N > 96 && weights_keepable(n, fast_type(n), false) && weights_keepable(n, SPGK_T_BF16, true);
+    /* ... and at any number of rows when those operands are small: the streaming kernel's groups take 100 to 350 us (three layers of 2048: 137 us at
+     * 33 rows, 264 at 96, against 27 on the chain; 784-512-1000-10 in bf16 114 and 240 against 13).  Like that kernel they then use two terms
+     * in any mode. */
+    const bool light = N > SPGK_GEMV_MAX_BATCH && light_operands(n), light_exact = light && N <= 96 && all_wstream(n, N);
+    const bool chain_kept = light || (N > 96 && weights_keepable(n, fast_type(n), false) && weights_keepable(n, SPGK_T_BF16, true));
     if (N <= SPGK_GEMV_MAX_BATCH || gemv_groups || (N <= 512 && !chain_kept && all_wstream(n, N < group ? N : group))) {
         for (uint32_t r0 = 0; r0 < N; r0 += group) {
             const uint32_t rows = N - r0 < group ? N - r0 : group;
@@ -1221,7 +1304,7 @@ static float *forward_batch_on(spg_net *n, ForwardBatchArgs a)
                     if (rc) return NULL;
                 }
             }
-        } else if (spg_dev_forward_large(n, d_x, N, d_out)) return NULL;
+        } else if (light_exact ? large_chain(n, d_x, N, d_out, true) : spg_dev_forward_large(n, d_x, N, d_out)) return NULL;
         if (!out_dev && spg_map_kernel_error(spgk_memcpy_d2h(result, d_out, out_bytes, n->stream), "forward_batch: output copy")) return NULL;
     }
     /* device-to-device calls are stream-ordered like any CUDA library call: the caller

@@ -66,6 +66,7 @@ typedef struct spg_net_s {
     float *d_in32;  size_t in32_bytes;      /* staging for host inputs */
     float *d_out32; size_t out32_bytes;     /* fp32 outputs of the last layer */
     void  *d_act16[2]; size_t act16_bytes;  /* ping-pong 16-bit activation planes */
+    void  *d_chain; size_t chain_bytes;     /* operands between the layers of a net in one launch */
     float *d_act32[2]; size_t act32_bytes;  /* ping-pong fp32 activations (SIMT chain) */
     int32_t *d_status; bool status_pending;
     void *d_w16; size_t w16_bytes;         /* 16-bit weight operand of the layer in flight */
