@@ -19,26 +19,26 @@
 // layers wide, the INT4 net 8192-16384-16384-8192-1000 takes 185 us instead of 127 at 8 rows, 353 instead of 177 at 64, 1034
 // instead of 492 at 256 (one batch again and again).
 //
-// What bounds it.  HBM needs 41 us for the 272 MB of the INT4 net 8192-16384-16384-8192-1000.  A 128 x 128 block of
-// weights moves through shared memory as 8 KB packed (in and out), 16 KB of operand (in and out) and C * 128 B of digits
-// (in and out, C = 4 columns per row): 56 KB at 8 rows, 112 KB at 64 rows, 440 and 880 cycles at 128 B/clk -- 53 us and
-// 106 us over the net, whose busiest SMs have 237 such blocks.  One byte per weight in the operand instead of two is why this
-// path exists beside the 16-bit streaming kernel, which writes and reads 32 KB per such block.
+// Where the operand lies.  A product of 128 x C x 32 with both operands in shared memory takes 73 cycles at C = 32 and 172 at 256, with the
+// weights in tensor memory 43 and 139 (the tensor pipe itself needs 16 and 128); and a 128 x 128 block's 16 KB of operand would go through shared memory
+// twice beside its 8 KB of packed bytes and its digits.  So the unpackers store to tensor memory: 256 columns hold eight blocks, beside two
+// accumulators of up to 128 columns (32 rows) or one of up to 256.  Only where a layer turns out wide and needs two of more than 128 do operand tiles
+// go through shared memory.  INT8 boxes are the operand as they arrive.
 //
-// Measured, large INT4 net, inputs new in every call: 125 us at 8 rows (GEMV: 201), 171 at 64 (16-bit streaming kernel: 577), 498 at 256 (GEMM chain:
-// 684).  A block of INT4 takes 480 cycles at 8 rows, of which the MMA warp's own turn is all (operand tiles changing hands one at a time: 810).
-// At 64 rows a CTA alone draws 32 KB of digits a block from L2, at 43 bytes a cycle: 750 cycles; the tensor pipe would need
-// 512.  Layers of more than 32 rows a group in which a CTA has many blocks in a row therefore run on pairs of CTAs (cta_group::2), each with half of the
-// digits: a layer of 16384 x 8192 at 40, 64, 96, 256 rows 40.0 -> 35.5, 42.1 -> 40.6, 61 -> 56, 114 -> 104 us, its tensor pipe 69 % busy at 64 rows
-// while it runs; the net 187 -> 171 us at 64 rows, 554 -> 498 at 256; with twelve batches in turn INT4 167 and 443, INT2 163 and 406, INT8 181 and 524.  From layers of 32 to 166 blocks with weights from HBM: 530 cycles a block and 14 us a layer at 8 rows, 870 and 16 at 64.
-// INT8, whose boxes need no unpacking, takes 700 cycles at 8 rows, 5.5 TB/s.  The rest of a layer is staging, the first
-// boxes and tiles, and the last sums (1 us at 8 rows, 3 at 64).
+// What bounds it.  HBM needs 41 us for the 272 MB of the INT4 net 8192-16384-16384-8192-1000, whose busiest SMs have 237 blocks: 366 cycles a
+// block.  Measured in the layer 16384 x 16384: 375 cycles a block at 8 rows (6.2 TB/s; 480 with the operand in shared memory), 435 at 32 rows, 560 at 64
+// (746; the tensor pipe's own 512, pairs of CTAs).  The rest of the net's time lies between the blocks, 16 us a layer at 8 rows: last
+// sums 4 to 10, the staging kernel and its two boundaries 8, first digit tiles 3.
+//
+// Measured, large INT4 net, inputs new in every call, before and since: 8 rows 125 -> 116 us (GEMV: 201), 64 rows 172 -> 162 (16-bit streaming kernel: 577),
+// 256 rows 498 -> 466 (GEMM chain: 684).  Layers of more than 32 rows a group in which a CTA has many blocks in a row run on pairs of CTAs
+// (cta_group::2), each with half of the digits, of which a CTA alone would draw 32 KB a block from L2.
 //
 // Per CTA (one per SM, 19 warps):
 //   warp 0      weight boxes by TMA (128 rows x 128 packed bytes, 128-byte swizzle), ahead of the previous layer's end:
 //               weights depend on nothing
 //   warp 18     digit tiles by TMA ([C] x 128 k), after the staging kernel has finished
-//   warps 10-17 unpack a box into operand tiles (INT4: a nibble moved to the top of its byte is 16q in two's complement;
+//   warps 10-17 unpack a box into operand tiles in tensor memory (INT4: a nibble moved to the top of its byte is 16q in two's complement;
 //               INT2: 64q; INT8 boxes are the operand as they arrive)
 //   warp 1      issues the MMAs, four K = 32 steps per 128-wide block
 //   warps 2-9   tensor memory -> int64 -> scale, bias, activation -> fp32
@@ -64,6 +64,7 @@ constexpr uint32_t TILE_ROWS = 128;
 constexpr uint32_t BOX_BYTES = 128 * TILE_ROWS;        // one box of packed weights = one operand tile = 16 KB
 constexpr uint32_t GROUP_ROWS = 64;                    // batch rows per pass over the weights: 256 digit columns
 constexpr uint32_t IS_PAIR_ROWS = 32, IS_PAIR_BLOCKS = 16;
+constexpr uint32_t IS_A_COLUMN = 256, IS_A_SLOTS = 4;   // operand tiles in tensor memory: slots of two blocks, 32 columns each
 constexpr uint32_t MAX_K = 131072;                     // 64 * 128 * K < 2^31
 constexpr uint32_t MAX_TILES = 4096;                   // counters in the scratch head
 constexpr uint32_t STAGE_THREADS = 1024;
@@ -73,7 +74,7 @@ struct IsParams {
     uint32_t out, groups, rpg, N, C;                   // rows per group, batch rows, columns of a tile (4 * rpg)
     uint32_t rows;                                     // groups * rpg: rows of scales, a quarter of the rows of one set of digits
     uint32_t kbr, boxes;                               // 128-wide k-blocks per box, boxes per row tile
-    uint32_t RS, AS, BS;                               // ring slots: boxes, operand (G blocks each), digits (GB blocks each)
+    uint32_t RS, AS, BS, bars;                         // ring slots: boxes, operand in shared memory (G blocks each), digits (GB blocks each); barriers of operand slots
     uint32_t G, GB;
     uint64_t units;                                    // tiles * boxes
     uint32_t direct; int prec, act;
@@ -106,6 +107,37 @@ __device__ __forceinline__ void umma_i8_pair(uint32_t tmem_d, uint64_t desc_a, u
         "setp.ne.b32 p, %4, 0;\n\t"
         "tcgen05.mma.cta_group::2.kind::i8 [%0], %1, %2, %3, {%5, %5, %5, %5, %5, %5, %5, %5}, p;\n\t}"
         ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(0u) : "memory");
+}
+// ... with A in tensor memory: 32 rows' bytes of K = 32 are eight columns
+__device__ __forceinline__ void umma_i8_tmem(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate)
+{
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::i8 [%0], [%1], %2, %3, {%5, %5, %5, %5}, p;\n\t}"
+        ::"r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(0u) : "memory");
+}
+__device__ __forceinline__ void umma_i8_tmem_pair(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate)
+{
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::i8 [%0], [%1], %2, %3, {%5, %5, %5, %5, %5, %5, %5, %5}, p;\n\t}"
+        ::"r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(0u) : "memory");
+}
+// 32 columns of this warp's 32 lanes
+__device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&r)[32])
+{
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,"
+        "%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};"
+        ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]),
+        "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]), "r"(r[18]), "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]),
+        "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31]) : "memory");
+}
+__device__ __forceinline__ void mbar_arrive_by(uint32_t bar, uint32_t count)
+{
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(count) : "memory");
 }
 // int32 accumulator, A and B signed 8-bit, both K-major, m x n
 inline uint32_t idesc_i8(uint32_t m, uint32_t n) { return (2u << 4) | (1u << 7) | (1u << 10) | ((n >> 3) << 17) | ((m >> 4) << 24); }
@@ -268,6 +300,11 @@ spg_is_stage_kernel(const float *__restrict__ x, uint32_t ldx, uint32_t N, uint3
 
 // ---- the layer ---------------------------------------------------------------------------------------------------------
 
+// Operand tiles go to tensor memory, beside one accumulator of up to 256 columns or two of up to 128, unless both sets of digits need more
+// columns than that (or the boxes are the operand).
+__device__ __forceinline__ bool is_in_tmem(const IsParams &p, bool wide) { return !p.direct && !(wide && p.C > 128); }
+__device__ __forceinline__ bool is_one_accumulator(const IsParams &p, bool wide) { return wide || (!p.direct && p.C > 128); }
+
 __device__ __forceinline__ void is_epi_sync() { asm volatile("bar.sync 2, %0;" ::"n"(32 * IS_EPI_WARPS) : "memory"); }
 
 // `rest`: bias, and the second set's share
@@ -317,10 +354,10 @@ __device__ __forceinline__ void is_epilogue(const IsParams &p, bool wide, bool d
 {
     const uint32_t half = (warp - 2u) >> 2, et = (warp & 3u) * 32u + lane;
     const uint32_t cta = PAIR ? blockIdx.x & 1u : 0u, teams = PAIR ? gridDim.x >> 1 : gridDim.x;      // teams: pairs, or CTAs alone
+    const bool one = is_one_accumulator(p, wide);      // (a wide layer's second set takes the second accumulator)
     uint32_t count = 0;
     for (; is_next_segment(p, seg); count++) {
-        // a wide layer's second set takes the second accumulator: no double buffering
-        const uint32_t acc = wide ? 0 : count & 1u, phase = (wide ? count : count >> 1) & 1u, mt = seg.tile / p.groups, n0 = (seg.tile % p.groups) * p.rpg;
+        const uint32_t acc = one ? 0 : count & 1u, phase = (one ? count : count >> 1) & 1u, mt = seg.tile / p.groups, n0 = (seg.tile % p.groups) * p.rpg;
         const bool whole = seg.k1 - seg.k0 == p.boxes;
         const uint32_t row = (PAIR ? 2 * mt + cta : mt) * TILE_ROWS + et;
         const float bias = row < p.out ? p.bias[row] : 0.0f;
@@ -435,18 +472,18 @@ __device__ __forceinline__ uint32_t is_early_slots(const IsParams &p, const IsSe
     return slots < p.BS ? (uint32_t)slots : p.BS;
 }
 
-// MMA role (warp 1): SETS sets of digits per 128-wide block of weights.  The warp's own turn bounds the kernel at small
-// batches: a wait costs it some 100 cycles even when there is nothing to wait for, a commit as much, an MMA 45 to 128.  So
-// operand tiles change hands G blocks at a time and digit tiles GB (a divisor of G), and all three are numbers known to the
-// compiler (a counted loop over the sets took 3 us of the 65 that 256 rows of a 4096-4096-1024 net take).  At 8 rows of INT4 a
-// block then takes the warp 480 cycles; it took 810 one at a time.
+// MMA role (warp 1): SETS sets of digits per 128-wide block of weights.  A wait costs the warp some 70 cycles even when there is nothing to wait
+// for, a commit as much.  So operand tiles change hands G blocks at a time and digit tiles GB (a divisor of G), and all three are numbers
+// known to the compiler (a counted loop over the sets took 3 us of the 65 that 256 rows of a 4096-4096-1024 net take).
+// TMEM: the operand tiles lie in tensor memory.
 struct IsBars { uint32_t rfull0, rempty0, afull0, aempty0, bfull0, bempty0, tfull0, tempty0; };
-template <uint32_t SETS, uint32_t G, uint32_t GB, bool PAIR>
+template <uint32_t SETS, uint32_t G, uint32_t GB, bool PAIR, bool TMEM>
 __device__ __forceinline__ void is_mma(const IsParams &p, IsSegment seg, const IsBars &bar, uint64_t a_desc0, uint64_t b_desc0, uint32_t tmem_base,
                                        uint32_t abort_addr, volatile int *abort_flag)
 {
     uint32_t as = 0, aph = 0, bs = 0, bph = 0, count = 0;      // G = 1: the boxes are the operand
-    const uint32_t b_step = p.C * 128u >> (PAIR ? 5 : 4), slots = G == 1 ? p.RS : p.AS;
+    const uint32_t b_step = p.C * 128u >> (PAIR ? 5 : 4), slots = TMEM ? IS_A_SLOTS : G == 1 ? p.RS : p.AS;
+    const bool one = SETS == 2 || (TMEM && p.C > 128);
     const uint32_t full0 = G == 1 ? bar.rfull0 : bar.afull0, empty0 = G == 1 ? bar.rempty0 : bar.aempty0;
     if (SETS == 2) {
         const uint32_t early = is_early_slots(p, seg);
@@ -462,7 +499,7 @@ __device__ __forceinline__ void is_mma(const IsParams &p, IsSegment seg, const I
         }
     }
     for (; is_next_segment(p, seg); count++) {
-        const uint32_t acc = SETS == 2 ? 0 : count & 1u, phase = (SETS == 2 ? count : count >> 1) & 1u;
+        const uint32_t acc = one ? 0 : count & 1u, phase = (one ? count : count >> 1) & 1u;
         mbar_wait_uniform(bar.tempty0 + 8 * acc, phase ^ 1u, abort_addr, p.status, 3);
         if (*abort_flag) return;
         tc_fence_after();
@@ -472,6 +509,7 @@ __device__ __forceinline__ void is_mma(const IsParams &p, IsSegment seg, const I
         for (uint32_t turn = 0; turn < turns; turn++) {
             mbar_wait_uniform(full0 + 8 * as, aph, abort_addr, p.status, G == 1 ? 4 : 5);
             const uint64_t da = a_desc0 + (uint64_t)(as * G * (BOX_BYTES >> 4));
+            const uint32_t ta = tmem_base + IS_A_COLUMN + as * G * 32;
 #pragma unroll
             for (uint32_t j = 0; j < G; j += GB) {
 #pragma unroll
@@ -485,7 +523,9 @@ __device__ __forceinline__ void is_mma(const IsParams &p, IsSegment seg, const I
                         for (uint32_t i = 0; i < GB; i++)
 #pragma unroll
                             for (uint32_t k = 0; k < 4; k++)
-                                PAIR ? umma_i8_pair(d_tmem + set * p.C, da + (j + i) * (BOX_BYTES >> 4) + 2 * k, db + i * b_step + 2 * k, p.idesc, j + i + k ? 1u : accum)
+                                if (TMEM) PAIR ? umma_i8_tmem_pair(d_tmem + set * p.C, ta + (j + i) * 32 + 8 * k, db + i * b_step + 2 * k, p.idesc, j + i + k ? 1u : accum)
+                                               : umma_i8_tmem(d_tmem + set * p.C, ta + (j + i) * 32 + 8 * k, db + i * b_step + 2 * k, p.idesc, j + i + k ? 1u : accum);
+                                else PAIR ? umma_i8_pair(d_tmem + set * p.C, da + (j + i) * (BOX_BYTES >> 4) + 2 * k, db + i * b_step + 2 * k, p.idesc, j + i + k ? 1u : accum)
                                      : umma_i8(d_tmem + set * p.C, da + (j + i) * (BOX_BYTES >> 4) + 2 * k, db + i * b_step + 2 * k, p.idesc, j + i + k ? 1u : accum);
                         PAIR ? umma_commit_pair(bar.bempty0 + 8 * bs) : umma_commit(bar.bempty0 + 8 * bs);
                         if (j + GB == G && set + 1 == SETS) PAIR ? umma_commit_pair(empty0 + 8 * as) : umma_commit(empty0 + 8 * as);
@@ -518,10 +558,10 @@ spg_istream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     const uint32_t b_off = a_off + (p.direct ? 0u : p.AS * p.G * BOX_BYTES);
     const uint32_t bar_off = b_off + p.BS * p.GB * b_bytes;
     const uint32_t rfull0 = base + bar_off, rempty0 = rfull0 + 8 * p.RS;
-    const uint32_t afull0 = rempty0 + 8 * p.RS, aempty0 = afull0 + 8 * p.AS;
-    const uint32_t bfull0 = aempty0 + 8 * p.AS, bempty0 = bfull0 + 8 * p.BS;
+    const uint32_t afull0 = rempty0 + 8 * p.RS, aempty0 = afull0 + 8 * p.bars;
+    const uint32_t bfull0 = aempty0 + 8 * p.bars, bempty0 = bfull0 + 8 * p.BS;
     const uint32_t tfull0 = bempty0 + 8 * p.BS, tempty0 = tfull0 + 16;
-    const uint32_t flag_off = bar_off + 16 * (p.RS + p.AS + p.BS) + 32;
+    const uint32_t flag_off = bar_off + 16 * (p.RS + p.bars + p.BS) + 32;
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem + flag_off);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
     int *s_last = const_cast<int *>(abort_flag) + 1;
@@ -530,11 +570,11 @@ spg_istream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
     const uint32_t cta = PAIR ? cluster_rank() : 0u, team = PAIR ? blockIdx.x >> 1 : blockIdx.x, teams = PAIR ? gridDim.x >> 1 : gridDim.x;
     uint32_t tmem_cols = 32;
-    while (tmem_cols < 2 * p.C) tmem_cols *= 2;          // two accumulators, 512 columns at most
+    while (tmem_cols < (p.direct ? 2 * p.C : 512u)) tmem_cols *= 2;      // two accumulators, 512 columns at most
 
     if (tid == 0) {
         for (uint32_t s = 0; s < p.RS; s++) { mbar_init(rfull0 + 8 * s, 1); mbar_init(rempty0 + 8 * s, p.direct ? 1 : IS_CONV_WARPS); }
-        for (uint32_t s = 0; s < p.AS; s++) { mbar_init(afull0 + 8 * s, (PAIR ? 2 : 1) * IS_CONV_WARPS / p.AS); mbar_init(aempty0 + 8 * s, 1); }
+        for (uint32_t s = 0; s < p.bars; s++) { mbar_init(afull0 + 8 * s, (PAIR ? 2 : 1) * IS_CONV_WARPS / 2); mbar_init(aempty0 + 8 * s, 1); }      // (half of the unpackers a slot)
         for (uint32_t s = 0; s < p.BS; s++) { mbar_init(bfull0 + 8 * s, 1); mbar_init(bempty0 + 8 * s, 1); }
         for (uint32_t a = 0; a < 2; a++) { mbar_init(tfull0 + 8 * a, 1); mbar_init(tempty0 + 8 * a, PAIR ? 2 * IS_EPI_WARPS : 32 * IS_EPI_WARPS); }
         *abort_flag = 0;
@@ -620,11 +660,12 @@ spg_istream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         const uint64_t a_desc0 = smem_desc_sw128(p.direct ? base : base + a_off), b_desc0 = smem_desc_sw128(base + b_off);
         spg_grid_wait();
         if (cta) goto is_role_done;                      // the first CTA issues for both
-#define IS_MMA(SETSV, GV, GBV) is_mma<SETSV, GV, GBV, PAIR>(p, seg, bar, a_desc0, b_desc0, tmem_base, abort_addr, abort_flag)
+#define IS_MMA(SETSV, GV, GBV, TMEMV) is_mma<SETSV, GV, GBV, PAIR, TMEMV>(p, seg, bar, a_desc0, b_desc0, tmem_base, abort_addr, abort_flag)
         const bool wide = is_any_wide(p, lane);
-        if (p.direct) { if (wide) IS_MMA(2, 1, 1); else IS_MMA(1, 1, 1); }
-        else if (p.GB == 1) { if (wide) IS_MMA(2, 2, 1); else IS_MMA(1, 2, 1); }
-        else { if (wide) IS_MMA(2, 2, 2); else IS_MMA(1, 2, 2); }
+        if (p.direct) { if (wide) IS_MMA(2, 1, 1, false); else IS_MMA(1, 1, 1, false); }
+        else if (!is_in_tmem(p, wide)) { if (p.GB == 1) IS_MMA(2, 2, 1, false); else IS_MMA(2, 2, 2, false); }
+        else if (p.GB == 1) { if (wide) IS_MMA(2, 2, 1, true); else IS_MMA(1, 2, 1, true); }
+        else { if (wide) IS_MMA(2, 2, 2, true); else IS_MMA(1, 2, 2, true); }
 #undef IS_MMA
     } else if (warp >= IS_CONV_WARP0) {
         // ------------------------------ unpackers ---------------------------------
@@ -632,13 +673,71 @@ spg_istream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         // running number is g mod AS * G, always in place g, so that many tiles are in the making at once and the latency of one
         // (load, unpack, store, proxy fence, arrive: 600 cycles) hides behind the others.  Lanes 0-7 of a quarter warp take eight different rows of a swizzle atom: no bank
         // conflict on either side.  (Sixteen warps instead of eight: 2 to 5 % slower at every batch size.)
-        if (!p.direct) {
+        if (!p.direct) spg_grid_wait();
+        const bool in_tmem = !p.direct && is_in_tmem(p, p.C > 128 && is_any_wide(p, lane));
+        if (in_tmem) {
+            // Four warps make the two blocks of a slot, a lane a weight row; the other four make the next slot's.  A row's packed bytes are whole in
+            // the box, so a lane reads them, unpacks them and stores 32 columns a block.
+            const uint32_t set = (warp - IS_CONV_WARP0) >> 2, quadrant = warp & 3u, row = quadrant * 32 + lane, r7 = row & 7u;
+            const bool nibbles = p.prec == SPG_P_I4;
+            const uint32_t turns = nibbles ? 1 : 2;      // slots of a box
+            const uint32_t tmem_a = tmem_base + IS_A_COLUMN + ((quadrant * 32) << 16);
+            uint32_t rs = 0, rph = 0, as = 0, aph = 0, turn = 0;
+            while (is_next_segment(p, seg)) {
+                for (uint32_t b = seg.k0; b < seg.k1; b++) {
+                    const uint8_t *box = smem + rs * BOX_BYTES + row * 128u;
+                    bool mine = false;
+                    for (uint32_t t = 0; t < turns; t++, turn++) {
+                        if ((turn & 1u) == set) {
+                            bool ok = mine || mbar_wait(rfull0 + 8 * rs, rph, abort_flag, p.status, 7);
+                            mine = true;
+                            ok = ok && mbar_wait(aempty0 + 8 * as, aph ^ 1u, abort_flag, p.status, 8);
+                            __syncwarp();
+                            tc_fence_after();
+                            if (__all_sync(0xffffffffu, ok)) {
+#pragma unroll
+                                for (uint32_t j = 0; j < 2; j++) {
+                                    uint32_t r[32];
+                                    if (nibbles) {
+#pragma unroll
+                                        for (uint32_t pc = 0; pc < 4; pc++) {
+                                            const uint4 w = *reinterpret_cast<const uint4 *>(box + (((4 * j + pc) ^ r7) << 4));
+                                            const uint32_t m = 0xF0F0F0F0u, ws[4] = { w.x, w.y, w.z, w.w };
+#pragma unroll
+                                            for (uint32_t i = 0; i < 4; i++) { r[8 * pc + 2 * i] = (ws[i] << 4) & m; r[8 * pc + 2 * i + 1] = ws[i] & m; }
+                                        }
+                                    } else {
+#pragma unroll
+                                        for (uint32_t pc = 0; pc < 2; pc++) {
+                                            const uint4 w = *reinterpret_cast<const uint4 *>(box + (((4 * t + 2 * j + pc) ^ r7) << 4));
+                                            const uint32_t m = 0xC0C0C0C0u, ws[4] = { w.x, w.y, w.z, w.w };
+#pragma unroll
+                                            for (uint32_t i = 0; i < 4; i++) {
+                                                r[16 * pc + 4 * i] = (ws[i] << 6) & m; r[16 * pc + 4 * i + 1] = (ws[i] << 4) & m;
+                                                r[16 * pc + 4 * i + 2] = (ws[i] << 2) & m; r[16 * pc + 4 * i + 3] = ws[i] & m;
+                                            }
+                                        }
+                                    }
+                                    tmem_st32(tmem_a + as * 64 + j * 32, r);
+                                }
+                                asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                            }
+                            tc_fence_before();
+                            __syncwarp();
+                            if (lane == 0) PAIR ? mbar_arrive_cluster(mapa(afull0 + 8 * as, 0)) : mbar_arrive(afull0 + 8 * as);
+                        }
+                        if (++as == IS_A_SLOTS) { as = 0; aph ^= 1u; }
+                    }
+                    if (mine && lane == 0) mbar_arrive_by(rempty0 + 8 * rs, nibbles ? 2 : 1);      // (eight arrivals a box)
+                    if (++rs == p.RS) { rs = 0; rph ^= 1u; }
+                }
+            }
+        } else if (!p.direct) {
             const uint32_t tiles = p.AS * p.G, wpg = IS_CONV_WARPS / tiles, TG = 32u * wpg;
             const uint32_t cw = warp - IS_CONV_WARP0, grp = cw / wpg, ctg = (cw % wpg) * 32u + lane;
             const uint32_t afull = PAIR ? mapa(afull0 + 8 * (grp / p.G), 0) : afull0 + 8 * (grp / p.G), aempty = aempty0 + 8 * (grp / p.G);
             uint32_t rs = 0, rph = 0, as = 0, aph = 0;
             uint8_t *atile = smem + a_off + grp * BOX_BYTES;
-            spg_grid_wait();
             while (is_next_segment(p, seg)) {
                 for (uint32_t b = seg.k0; b < seg.k1; b++) {
                     const bool okr = mbar_wait(rfull0 + 8 * rs, rph, abort_flag, p.status, 7);
@@ -728,7 +827,7 @@ is_role_done:
 // ---- host side ---------------------------------------------------------------------------------------------------------
 
 struct IsPlan {
-    uint32_t groups, rpg, C, kbr, boxes, ld, m_tiles, tiles, RS, AS, BS, G, GB, grid;
+    uint32_t groups, rpg, C, kbr, boxes, ld, m_tiles, tiles, RS, AS, BS, bars, G, GB, grid;
     uint64_t units;
     size_t operand_bytes, smem;
     bool direct, pair, ok;
@@ -772,7 +871,8 @@ IsPlan is_plan(const spgk_layer *L, uint32_t N, uint32_t sms)
     // rings: operand tiles in two slots of G blocks, digit tiles up to 96 KB (in pairs up to 32 rows), boxes with the rest
     const uint32_t b_bytes = pl.C * (pl.pair ? 64u : 128u);
     pl.G = pl.direct ? 1 : 2;
-    pl.AS = pl.direct ? 1 : 2;
+    pl.AS = pl.direct ? 1 : pl.C > 128 ? 2 : 0;      // (in shared memory only for layers that turn out wide)
+    pl.bars = pl.direct ? 1 : IS_A_SLOTS;
     pl.GB = pl.direct || b_bytes > 16384 ? 1 : 2;
     pl.BS = 96u * 1024 / b_bytes;
     if (pl.BS > 8) pl.BS = 8;
@@ -780,7 +880,7 @@ IsPlan is_plan(const spgk_layer *L, uint32_t N, uint32_t sms)
     const uint32_t a_bytes = pl.direct ? 0 : pl.AS * pl.G * BOX_BYTES;
     pl.RS = (224u * 1024 - a_bytes - pl.BS * pl.GB * b_bytes) / BOX_BYTES;
     if (pl.RS > 10) pl.RS = 10;
-    pl.smem = 1024 + (size_t)pl.RS * BOX_BYTES + a_bytes + (size_t)pl.BS * pl.GB * b_bytes + 16 * (pl.RS + pl.AS + pl.BS) + 32 + 16 + 2 * GROUP_ROWS * sizeof(double);
+    pl.smem = 1024 + (size_t)pl.RS * BOX_BYTES + a_bytes + (size_t)pl.BS * pl.GB * b_bytes + 16 * (pl.RS + pl.bars + pl.BS) + 32 + 16 + 2 * GROUP_ROWS * sizeof(double);
     pl.operand_bytes = 2 * (size_t)pl.groups * pl.C * pl.ld;              // both sets of digits
     pl.ok = pl.smem <= 227u * 1024;
     return pl;
@@ -903,7 +1003,7 @@ int spgk_istream_forward(const spgk_layer *layers, uint32_t count, const float *
         IsParams p{};
         p.out = L->out; p.groups = pl.groups; p.rpg = pl.rpg; p.N = N; p.C = pl.C; p.rows = pl.groups * pl.rpg;
         p.kbr = pl.kbr; p.boxes = pl.boxes; p.units = pl.units;
-        p.RS = pl.RS; p.AS = pl.AS; p.BS = pl.BS; p.G = pl.G; p.GB = pl.GB;
+        p.RS = pl.RS; p.AS = pl.AS; p.BS = pl.BS; p.bars = pl.bars; p.G = pl.G; p.GB = pl.GB;
         p.direct = pl.direct; p.prec = L->precision;
         p.act = L->act == SPG_ACT_SOFTMAX ? SPG_ACT_NONE : L->act;
         p.scale = (double)L->w_scale / (L->precision == SPG_P_I4 ? 16.0 : L->precision == SPG_P_I2 ? 64.0 : 1.0);
