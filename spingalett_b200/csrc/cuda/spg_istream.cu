@@ -64,6 +64,7 @@ constexpr uint32_t TILE_ROWS = 128;
 constexpr uint32_t BOX_BYTES = 128 * TILE_ROWS;        // one box of packed weights = one operand tile = 16 KB
 constexpr uint32_t GROUP_ROWS = 64;                    // batch rows per pass over the weights: 256 digit columns
 constexpr uint32_t IS_PAIR_ROWS = 32, IS_PAIR_BLOCKS = 16;
+constexpr uint32_t IS_EARLY_BOXES = 4;
 constexpr uint32_t IS_A_COLUMN = 256, IS_A_SLOTS = 4;   // operand tiles in tensor memory: slots of two blocks, 32 columns each
 constexpr uint32_t MAX_K = 131072;                     // 64 * 128 * K < 2^31
 constexpr uint32_t MAX_TILES = 4096;                   // counters in the scratch head
@@ -76,7 +77,7 @@ struct IsParams {
     uint32_t kbr, boxes;                               // 128-wide k-blocks per box, boxes per row tile
     uint32_t RS, AS, BS, bars;                         // ring slots: boxes, operand in shared memory (G blocks each), digits (GB blocks each); barriers of operand slots
     uint32_t G, GB;
-    uint64_t units;                                    // tiles * boxes
+    uint32_t units;                                    // tiles * boxes (4096 * 1024 at most: times the number of CTAs still 32 bits)
     uint32_t direct; int prec, act;
     double scale; const float *bias; const double *row_scale;
     const uint8_t *wide;
@@ -143,7 +144,7 @@ __device__ __forceinline__ void mbar_arrive_by(uint32_t bar, uint32_t count)
 inline uint32_t idesc_i8(uint32_t m, uint32_t n) { return (2u << 4) | (1u << 7) | (1u << 10) | ((n >> 3) << 17) | ((m >> 4) << 24); }
 
 // first unit of CTA c
-__host__ __device__ inline uint64_t unit_start(uint64_t units, uint32_t grid, uint32_t c) { return units * c / grid; }
+__host__ __device__ inline uint32_t unit_start(uint32_t units, uint32_t grid, uint32_t c) { return units * c / grid; }
 
 // ---- staging: fp32 rows -> digit operand -------------------------------------------------------------------------------
 
@@ -316,14 +317,14 @@ __device__ __forceinline__ void is_finish(const IsParams &p, uint32_t n, uint32_
 }
 
 // Segments of a CTA: the runs of its units that lie in one tile.
-struct IsSegment { uint64_t u, end; uint32_t tile, k0, k1; };
+struct IsSegment { uint32_t u, end, tile, k0, k1; };
 __device__ __forceinline__ bool is_next_segment(const IsParams &p, IsSegment &s)
 {
     if (s.u >= s.end) return false;
-    s.tile = (uint32_t)(s.u / p.boxes);
-    s.k0 = (uint32_t)(s.u - (uint64_t)s.tile * p.boxes);
-    const uint64_t left = s.end - s.u;
-    s.k1 = left < p.boxes - s.k0 ? s.k0 + (uint32_t)left : p.boxes;
+    s.tile = s.u / p.boxes;
+    s.k0 = s.u - s.tile * p.boxes;
+    const uint32_t left = s.end - s.u;
+    s.k1 = left < p.boxes - s.k0 ? s.k0 + left : p.boxes;
     s.u += s.k1 - s.k0;
     return true;
 }
@@ -370,8 +371,8 @@ __device__ __forceinline__ void is_epilogue(const IsParams &p, bool wide, bool d
         // of a CTA's range starts in it
         uint64_t slot = et;
         if (!whole) {
-            const uint64_t t0 = (uint64_t)seg.tile * p.boxes;
-            uint32_t c = (uint32_t)(t0 * teams / p.units);
+            const uint32_t t0 = seg.tile * p.boxes;
+            uint32_t c = t0 * teams / p.units;
             while (c > 0 && unit_start(p.units, teams, c) > t0) c--;
             while (unit_start(p.units, teams, c + 1) <= t0) c++;
             slot += (uint64_t)(PAIR ? 2 * c + cta : c) * p.rpg * TILE_ROWS;
@@ -468,8 +469,8 @@ __device__ __forceinline__ void is_epilogue(const IsParams &p, bool wide, bool d
 // are thrown away.
 __device__ __forceinline__ uint32_t is_early_slots(const IsParams &p, const IsSegment &seg)
 {
-    const uint64_t slots = (seg.end - seg.u) * p.kbr / p.GB;
-    return slots < p.BS ? (uint32_t)slots : p.BS;
+    const uint32_t slots = (seg.end - seg.u) * p.kbr / p.GB;
+    return slots < p.BS ? slots : p.BS;
 }
 
 // MMA role (warp 1): SETS sets of digits per 128-wide block of weights.  A wait costs the warp some 70 cycles even when there is nothing to wait
@@ -599,13 +600,15 @@ spg_istream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
 
     if (warp == 0) {
         // ------------------------------ weight boxes ------------------------------
-        // The first ring of boxes goes out before the previous kernel of the stream has ended; every role waits for that end
-        // before its first bounded wait, which would otherwise count somebody else's running time.
-        uint32_t rs = 0, rph = 0;
+        // The first boxes go out before the previous kernel of the stream has ended; every role waits for that end before its first bounded wait,
+        // which would otherwise count somebody else's running time.  Not a whole ring of boxes: 24 MB of weights from HBM are in the way of the few
+        // loads that the staging kernel and the first digit tiles hang on (large INT4 net at 8 and 64 rows, boxes of ten that go early: none 118.8 / 158.5
+        // us, two 115.9 / 158.3, four 113.9 / 157.3, ten 114.8 / 160.1; asking L2 for up to 48 more each 121 / 169).
+        uint32_t rs = 0, rph = 0, sent = 0;
         while (is_next_segment(p, seg)) {
             const int r0 = (int)((PAIR ? 2 * (seg.tile / p.groups) + cta : seg.tile / p.groups) * TILE_ROWS);
             for (uint32_t b = seg.k0; b < seg.k1; b++) {
-                if (rs == 0 && rph) spg_grid_wait();
+                if (sent++ == IS_EARLY_BOXES) spg_grid_wait();
                 mbar_wait_uniform(rempty0 + 8 * rs, rph ^ 1u, abort_addr, p.status, 1);
                 if (*abort_flag) goto is_role_done;
                 if (elect_one()) {
@@ -828,7 +831,7 @@ is_role_done:
 
 struct IsPlan {
     uint32_t groups, rpg, C, kbr, boxes, ld, m_tiles, tiles, RS, AS, BS, bars, G, GB, grid;
-    uint64_t units;
+    uint32_t units;
     size_t operand_bytes, smem;
     bool direct, pair, ok;
 };
@@ -866,7 +869,7 @@ IsPlan is_plan(const spgk_layer *L, uint32_t N, uint32_t sms)
     pl.m_tiles = (L->out + high - 1) / high;
     pl.tiles = pl.m_tiles * pl.groups;
     if (pl.tiles > MAX_TILES) return pl;
-    pl.units = (uint64_t)pl.tiles * pl.boxes;
+    pl.units = pl.tiles * pl.boxes;
     pl.grid = pl.pair ? 2 * is_ctas(pl.tiles, pl.boxes, sms / 2) : is_ctas(pl.tiles, pl.boxes, sms);
     // rings: operand tiles in two slots of G blocks, digit tiles up to 96 KB (in pairs up to 32 rows), boxes with the rest
     const uint32_t b_bytes = pl.C * (pl.pair ? 64u : 128u);
