@@ -551,8 +551,11 @@ int spg_dev_forward_sample(spg_net *n, float *h_io, bool *taken)
 }
 
 /* Rows and packed weight bytes that the integer streaming kernel serves (figures beside the call in forward_batch_on) */
-#define SPG_ISTREAM_MIN_ROWS 7u
-#define SPG_ISTREAM_MAX_ROWS 256u
+#define SPG_ISTREAM_MIN_ROWS 3u
+#define SPG_ISTREAM_LIGHT_MIN_ROWS 7u                   /* least rows in EXACT mode, and of nets that the small-net kernel takes */
+#define SPG_ISTREAM_MEDIUM_ROWS 256u
+#define SPG_ISTREAM_MAX_ROWS 448u
+#define SPG_ISTREAM_LARGE_BYTES ((size_t)40 << 20)      /* least packed size beyond 256 rows */
 #define SPG_ISTREAM_MEDIUM_BYTES ((size_t)4 << 20)      /* least packed size beyond 96 rows */
 #define SPG_ISTREAM_EXACT_ROWS 24u                      /* most rows in EXACT mode */
 
@@ -564,7 +567,7 @@ static int forward_istream(spg_net *n, const float *d_x, uint32_t N, float **d_l
     *d_last = NULL;
     size_t packed = 0;
     for (uint32_t l = 0; l < n->dev_layers; l++) packed += spg_array_bytes((uint64_t)n->klayers[l].in * n->klayers[l].out, (PrecisionMode)n->klayers[l].precision);
-    if (N > 96 && packed < SPG_ISTREAM_MEDIUM_BYTES) return SPINGALETT_OK;
+    if ((N > 96 && packed < SPG_ISTREAM_MEDIUM_BYTES) || (N > SPG_ISTREAM_MEDIUM_ROWS && packed < SPG_ISTREAM_LARGE_BYTES)) return SPINGALETT_OK;
     const size_t need = spgk_istream_scratch_bytes(n->klayers, n->dev_layers, N);
     if (!need) return SPINGALETT_OK;
     int rc = reserve_zeroed(n, &n->d_is_scratch, &n->is_scratch_bytes, need, "integer-stream scratch");
@@ -1215,20 +1218,18 @@ static float *forward_batch_on(spg_net *n, ForwardBatchArgs a)
 
     /* Integer files take the 8-bit integer streaming kernel from a few rows on, when it takes every layer.  Of what is left, up
      * to 8 rows go through spg_dev_forward_small (nets of few weights warp by warp, others GEMV first), up to 512 rows in groups of at most 128 through the 16-bit streaming kernel when
-     * it takes every layer, each group streaming the packed weights once; everything else is the large-batch GEMM chain.
+     * it takes every layer and the net's 16-bit operands are large, each group streaming the packed weights once; everything else is the chain.
      *
-     * Measured, against the path that served before: large INT4 net 125 us against 204 (GEMV) at 8 rows, 171 against 578
-     * (16-bit streaming kernel) at 64, 498 against 684 (GEMM chain) at 256.  Nets of 4 and 12 MB: 33 against 54 and 36 against
-     * 65 us at 8 rows, 0.45 of the time or less at 32 to 96; of 0.5 MB: 32 against 119 us at 8 rows.  The lines were drawn where
-     * the curves of older kernels crossed: the one at 7 rows when 8 rows took 157 us here (the GEMV: 155 at 6, INT2 132), the
-     * ones at 96 rows and 4 MB before products of few tiles had a kernel of their own (0.5 MB: 41 us here at 96 rows, 22 on the
-     * GEMM chain at 128; 4 MB: 51 here at 128), the one at 256 with the chain at 945 us for 512 rows (now 876).  Where today's
-     * cross has not been looked for.  FAST asks for one term per
-     * operand, which the GEMM chain serves beyond 96 rows.  EXACT promises 16 bits of every single value, which this kernel's
+     * Where the lines lie, us a call, this kernel / what serves otherwise, 8192-16384-16384-8192-1000 in INT4 and INT8, 8192-8192-8192-1000 in INT4:
+     * 2 rows 109 / 79, 140 / 112, 54 / 38 (GEMV); 3 rows 109 / 114, 141 / 137, 54 / 58; 4 rows 109 / 113, 141 / 138, 54 / 57; 6 rows 110 / 154, 143 / 163, 55 / 69.
+     * 260 rows 444 / 714, 569 / 719, 158 / 256 (chain); 448 rows 667 / 825, 890 / 925, 223 / 256; 512 rows 779 / 753, 994 / 1014, 252 / 259.  Smaller nets beyond 256 rows:
+     * 4096-8192-8192-256 in INT4 (49 MB) 130 / 331, 4096-4096-4096-1000 in INT8 (35 MB) 95 / 95 at 260 rows and 121 / 109 at 448, in INT4 (17 MB) 94 / 96 and 121 / 108.
+     * The lines at 96 rows and 4 MB were drawn before today's chains (0.5 MB: 41 us here at 96 rows); its sums are the more exact ones.  FAST asks for one term per
+     * operand, which the chain serves beyond 96 rows.  EXACT promises 16 bits of every single value, which this kernel's
      * fixed-point numbers hold for all but the few smallest of a row: beyond 24 rows (up to there the alternative is the GEMV,
-     * whose fixed-point numbers are coarser) EXACT stays with the kernels that feed two 16-bit terms. */
+     * whose fixed-point numbers are coarser) EXACT stays with the kernels that feed two 16-bit terms, and below 7 with the GEMV. */
     const SpingalettMathMode mode = spingalett_get_math_mode();
-    if (N >= SPG_ISTREAM_MIN_ROWS && N <= SPG_ISTREAM_MAX_ROWS && spgk_gemv_get_int_path() &&
+    if (N >= SPG_ISTREAM_MIN_ROWS && N <= SPG_ISTREAM_MAX_ROWS && (N >= SPG_ISTREAM_LIGHT_MIN_ROWS || (mode != SPINGALETT_MATH_EXACT && !few_weights(n, N))) && spgk_gemv_get_int_path() &&
         (N <= 96 || mode != SPINGALETT_MATH_FAST) && (N <= SPG_ISTREAM_EXACT_ROWS || mode != SPINGALETT_MATH_EXACT)) {
         float *d_last = NULL;
         if (forward_istream(n, d_x, N, &d_last, out_dev ? result : NULL)) return NULL;

@@ -33,3 +33,33 @@ def test_operand_tiles(spg, k, oracle, out, inn, n, prec, wide):  # noqa: F811
         got = y.cpu().numpy()
         assert np.all(np.abs(got[:n] - want) <= _bound(x, dec, want)) and np.all(got[n] == -9.0), again
     del hold
+
+
+def test_few_rows_and_many(spg, oracle, tmp_path):
+    """The lines at 3 rows (nets that the small-net kernel does not take, not in EXACT) and at 448 rows of large nets: the same answers on either side, as
+    the kernels that serve there in EXACT give them."""
+    a = spg.abi
+    for topo, prec, lines in [([4096, 4096, 500], a.PRECISION_INT4, {2: 0, 3: 1, 6: 1}), ([2048, 3072, 2048], a.PRECISION_INT8, {3: 1, 5: 1}),
+                              ([512, 512, 10], a.PRECISION_INT8, {3: 0, 6: 0, 7: 1}),
+                              ([8192, 10240], a.PRECISION_INT4, {257: 1, 448: 1, 449: 0}), ([8192, 10112], a.PRECISION_INT4, {256: 1, 257: 0})]:
+        net = spg.Network.build(topo, [a.ACT_TANH] * (len(topo) - 1), a.WEIGHT_INITIALIZATION_NONE)
+        rng = np.random.default_rng(len(topo))
+        net.weights[:] = rng.standard_normal(net.weights.size, dtype=np.float32) / np.sqrt(topo[0])
+        path = str(tmp_path / "net.nn")
+        net.save(path, prec)
+        net.free()
+        net = spg.Network.load(path)
+        for n, takes in lines.items():
+            x = rng.standard_normal((n, topo[0]), dtype=np.float32)
+            spg.set_math_mode(a.MATH_AUTO)
+            y = net.forward_batch(x)
+            assert (spg.last_path() == "istream") == bool(takes), (topo, n, spg.last_path())
+            spg.set_math_mode(a.MATH_EXACT)
+            try:
+                other = net.forward_batch(x)
+            finally:
+                spg.set_math_mode(a.MATH_AUTO)
+            assert np.abs(other - y).max() <= 1e-4, (topo, n)          # two bf16 terms: 2^-17 of a value, sums of a few units
+            if takes and n < 7:
+                assert spg.last_path() != "istream"
+        net.free()
