@@ -78,6 +78,8 @@ typedef struct spg_net_s {
 
     float *h_out; size_t h_out_bytes;       /* library-owned pinned output buffer */
     float *h_stage; size_t h_stage_bytes;   /* pinned staging for forward() */
+    void *sample_graph; uint32_t sample_calls;      /* forward()'s launches as a graph, calls before there is one */
+    const float *sample_io, *sample_dev;    /* the buffers it refers to */
 
     /* optional kernel timing (spingalett_profile): event pairs around the layer kernels */
     bool prof_on; void **prof_ev; uint32_t prof_cap, prof_used;
