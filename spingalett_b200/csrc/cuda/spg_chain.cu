@@ -18,12 +18,12 @@
 // What bounds it: latency.  256 rows of 784-512-1000-10 in INT4, clusters of 8 on 32 rows each, in cycles: first rows of the input
 // 2700, all of them in shared memory 6000, first layer multiplied 9800 (a product of 128 x 64 x 16 takes 65 cycles, 58 of them whatever
 // its width, to fetch the weights from shared memory), its outputs in the other CTAs 14200 (1200 of it for the release of the stores),
-// second layer 17400, last layer's sums 20000, rows put together 23500; 2 us from the end to the next launch's first load.  With
+// second layer 17400, last layer's sums 20000, rows put together 23500 (with sixteen epilogue warps; eight save 1200); 2 us from the end to the next launch's first load.  With
 // more rows the epilogues' instructions weigh: 3001 rows of 301-777-333-129-37, clusters of 4 on 96 rows, spend half of the time there.
 //
-// Measured against layer by layer (us): 784-512-1000-10 at 256 rows 22.9 -> 14.3 (INT4), 22.0 -> 17.8 (fp32, three products a term), 1500 rows
-// 29 -> 20; 301-777-333-129-37 at 3001 rows 39.2 -> 32.1; 100-65-130-7 at 3000 rows 25.5 -> 13.9; 1024-256-256-256-10 at 12000 rows 76 -> 38;
-// 128-128-128-128-128-128 at 256 rows 39 -> 14.  Against the 16-bit streaming kernel at 33 rows: 784-512-1000-10 in BF16 114 -> 13.
+// Measured against layer by layer (us): 784-512-1000-10 at 256 rows 22.9 -> 13.7 (INT4), 22.0 -> 16.9 (fp32, three products a term), 1500 rows
+// 29 -> 20; 301-777-333-129-37 at 3001 rows 39.2 -> 32.1; 100-65-130-7 at 3000 rows 25.5 -> 13.4; 1024-256-256-256-10 at 12000 rows 76 -> 38;
+// 128-128-128-128-128-128 at 256 rows 39 -> 14.  Against the 16-bit streaming kernel at 33 rows: 784-512-1000-10 in BF16 114 -> 12.
 // Tried: four rows a round of the epilogue instead of eight (560 cycles a round of four, eight little more), the input's loads ahead of the
 // fence that hands a tile on (the fence waits for them), one k-block a stage (waits and commits, 400 cycles a stage, twice as often).
 //
@@ -41,7 +41,7 @@ using namespace spgtc;
 constexpr uint32_t TK = 64, TM = 128;                          // of a weight tile
 constexpr uint32_t KG = 2;                                     // k-blocks that change hands at once
 constexpr uint32_t MAX_LAYERS = SPGK_CHAIN_MAX_LAYERS, MAX_C = 8, MAX_R = 256, MAX_RING = 12;
-constexpr uint32_t EPI = 16, EPI_THREADS = 32 * EPI, THREADS = 128 + EPI_THREADS;
+constexpr uint32_t threads_of(uint32_t epi) { return 128 + 32 * epi; }
 constexpr uint32_t TAIL_MAX = 128, MAX_MT = 4;                 // outputs of a last layer whose sums are put together
 constexpr uint32_t COUNTED_C = 4;                              // CTAs of a cluster where only the device knows the number of rows
 constexpr uint32_t BAR_BYTES = 8 * (5 * MAX_RING + 6) + 32;
@@ -88,7 +88,7 @@ __device__ __forceinline__ void arrive_release_cluster(uint32_t addr)
     asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(addr) : "memory");
 }
 __device__ __forceinline__ void fence_async_global() { asm volatile("fence.proxy.async.global;" ::: "memory"); }
-__device__ __forceinline__ void epi_sync() { asm volatile("bar.sync 1, %0;" ::"n"(EPI_THREADS) : "memory"); }
+template <uint32_t EPI> __device__ __forceinline__ void epi_sync() { asm volatile("bar.sync 1, %0;" ::"n"(32 * EPI) : "memory"); }
 
 // (relaxed: who waits reads nothing that was written before; a release would wait for the outputs' stores, 1400 cycles)
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); }
@@ -181,7 +181,6 @@ template <int ACT, int N> __device__ __forceinline__ void activate(float (&v)[N]
 // One output of eight rows: four from a place in sixteen rows on, and the four sixteen further on, or the first four again where the block has
 // no more.  (A warp's instructions hang on one another: eight rows take little longer than four, 560 cycles.)  The accumulators' sums in
 // their order.
-constexpr uint32_t ROUND = 2 * EPI;
 template <int AP>
 __device__ __forceinline__ void sums8(const Slice &s, uint32_t taddr, uint32_t more, float (&v)[8])
 {
@@ -216,7 +215,7 @@ __device__ __forceinline__ void finish8(const Slice &s, uint32_t taddr, uint32_t
 
 // A layer's outputs become the next one's operand: [k-block][plane][row] of 128 bytes.  Lane pairs trade rows so that each writes
 // two neighbouring values at once.  Columns beyond the layer's outputs get the activation of zero, whose weights are zeros.
-template <int ACT, typename T16, int AP>
+template <int ACT, typename T16, int AP, uint32_t EPI>
 __device__ __forceinline__ void to_operand(const Slice &s, uint8_t *next, uint32_t k0, uint32_t next_k, uint32_t plane)
 {
     const uint32_t odd = s.lane & 1u;
@@ -230,7 +229,7 @@ __device__ __forceinline__ void to_operand(const Slice &s, uint8_t *next, uint32
         // of rows c + odd and c + 2 + odd, where c is a multiple of 8; four rows on another 16 bytes
         const uint32_t at = swizzled(odd, k & 63u) ^ ((4 * s.g & 4u) << 4);
 #pragma unroll 1
-        for (uint32_t c = 4 * s.g; c < s.n; c += ROUND, taddr += ROUND, dst += ROUND * 128) {
+        for (uint32_t c = 4 * s.g; c < s.n; c += 2 * EPI, taddr += 2 * EPI, dst += 2 * EPI * 128) {
             const bool two = c + EPI < s.n;
             float v[8];
             finish8<ACT, AP>(s, taddr, two ? EPI : 0, bias, v);
@@ -249,7 +248,7 @@ __device__ __forceinline__ void to_operand(const Slice &s, uint8_t *next, uint32
     }
 }
 
-template <int ACT, int AP>
+template <int ACT, int AP, uint32_t EPI>
 __device__ __forceinline__ void to_output(const ChainParams &p, const Slice &s)
 {
 #pragma unroll 1
@@ -259,7 +258,7 @@ __device__ __forceinline__ void to_output(const ChainParams &p, const Slice &s)
         const float bias = t == 0 ? s.bias[0] : t == 1 ? s.bias[1] : t == 2 ? s.bias[2] : s.bias[3];
         const uint32_t taddr = s.tmem + t * s.mains * AP * s.n;
 #pragma unroll 1
-        for (uint32_t c = 4 * s.g; c < s.n; c += ROUND) {
+        for (uint32_t c = 4 * s.g; c < s.n; c += 2 * EPI) {
             float v[8];
             finish8<ACT, AP>(s, taddr + c, c + EPI < s.n ? EPI : 0, bias, v);
 #pragma unroll
@@ -274,11 +273,11 @@ __device__ __forceinline__ void to_output(const ChainParams &p, const Slice &s)
 // A narrow last layer: every CTA has multiplied its own outputs of the layer before, which nobody else needs then, by their part of K.  The
 // sums of a row go to the CTA that puts the row together: rows r * R / P and on are CTA r's, of P.  owners: where a row's sums begin there, and
 // the barrier that counts them; part: from there to this CTA's.
-template <int AP> __device__ __forceinline__ void to_owners(const Slice &s, const uint2 *owners, uint32_t part, uint32_t bar)
+template <int AP, uint32_t EPI> __device__ __forceinline__ void to_owners(const Slice &s, const uint2 *owners, uint32_t part, uint32_t bar)
 {
     part += s.o * 4;
 #pragma unroll 1
-    for (uint32_t c = 4 * s.g; c < s.n; c += ROUND) {
+    for (uint32_t c = 4 * s.g; c < s.n; c += 2 * EPI) {
         const uint32_t more = c + EPI < s.n ? EPI : 0;
         float v[8];
         sums8<AP>(s, s.tmem + c, more, v);                     // (by whole warps)
@@ -297,7 +296,7 @@ template <int AP> __device__ __forceinline__ void to_owners(const Slice &s, cons
 
 // ... which adds them in CTA order and finishes the rows, a warp a row; formulas and margin test of the softmax as in the epilogues of the
 // layer kernels
-template <int PER>                                             // outputs of a lane
+template <int PER, uint32_t EPI>                               // PER: outputs of a lane
 __device__ __forceinline__ void put_together(const ChainParams &p, int act, uint32_t out, float scale, const float (&bias)[MAX_MT], const float *parts, uint32_t first, uint32_t count,
                                              uint32_t end, uint32_t w, uint32_t lane)
 {
@@ -352,7 +351,7 @@ __device__ __forceinline__ void put_together(const ChainParams &p, int act, uint
 
 // The block's rows of the input as operand tiles: a warp rounds eight rows of a stage at a time, four columns a lane, so that it waits and
 // hands on once for them.  (A fence waits for the loads that are under way: none is then.)  VEC: rows lie on 16 bytes and end on a group of four.
-template <typename T16, int AP, bool VEC>
+template <typename T16, int AP, bool VEC, uint32_t EPI>
 __device__ __forceinline__ bool round_input(const ChainParams &p, uint32_t block0, uint32_t rows, uint32_t in, uint32_t stages, uint32_t w, uint32_t lane, uint8_t *tiles,
                                             uint32_t a_empty, uint32_t a_conv, Ring ring, volatile int *abort_flag)
 {
@@ -404,8 +403,8 @@ __device__ __forceinline__ bool round_input(const ChainParams &p, uint32_t block
 }
 
 // AP, WP: 16-bit terms of an activation and of a weight
-template <typename T16, int AP, int WP>
-__global__ void __launch_bounds__(THREADS, 1)
+template <typename T16, int AP, int WP, uint32_t EPI>
+__global__ void __launch_bounds__(threads_of(EPI), 1)
 spg_chain_kernel(const __grid_constant__ ChainParams p)
 {
     extern __shared__ __align__(1024) uint8_t smem[];
@@ -433,7 +432,7 @@ spg_chain_kernel(const __grid_constant__ ChainParams p)
     }
     uint2 *const owners = reinterpret_cast<uint2 *>(smem + owners_off);
     if (p.tail)
-        for (uint32_t r = threadIdx.x; r < p.R; r += THREADS) {
+        for (uint32_t r = threadIdx.x; r < p.R; r += 128 + 32 * EPI) {
             const uint32_t owner = ((r + 1) * p.tail - 1) / p.R, first = owner * p.R / p.tail;
             owners[r] = make_uint2(mapa(base + parts_off, owner) + (r - first) * p.l[p.layers - 1].out * 4, mapa(parts_bar, owner));
         }
@@ -607,8 +606,8 @@ spg_chain_kernel(const __grid_constant__ ChainParams p)
                 if (w == 0 && lane == 0) mbar_expect_tx(parts_bar + 8 * (round & 1u), p.tail * row_count * p.l[last].out * 4);
             }
             if (share(0, o0) && ok) {
-                if (p.vec4) ok = round_input<T16, AP, true>(p, b * p.R, rows, p.l[0].in, p.l[0].stages, w, lane, smem + a_off, a_empty, a_conv, ring, abort_flag);
-                else ok = round_input<T16, AP, false>(p, b * p.R, rows, p.l[0].in, p.l[0].stages, w, lane, smem + a_off, a_empty, a_conv, ring, abort_flag);
+                if (p.vec4) ok = round_input<T16, AP, true, EPI>(p, b * p.R, rows, p.l[0].in, p.l[0].stages, w, lane, smem + a_off, a_empty, a_conv, ring, abort_flag);
+                else ok = round_input<T16, AP, false, EPI>(p, b * p.R, rows, p.l[0].in, p.l[0].stages, w, lane, smem + a_off, a_empty, a_conv, ring, abort_flag);
                 for (uint32_t st = 0; st < p.l[0].stages; st++) ring.next(p.SA);
             }
             for (uint32_t l = 0; l < p.layers; l++) {
@@ -640,7 +639,7 @@ spg_chain_kernel(const __grid_constant__ ChainParams p)
                 if (p.tail && l + 1 == last) {
                     if (idle) continue;
                     // (every copy into the activation ring has been used up: its memory holds the CTA's own outputs until they are multiplied)
-#define SPG_CHAIN_CALL(A) to_operand<A, T16, AP>(s, smem + a_off, o0, tail_k, p.R * 128)
+#define SPG_CHAIN_CALL(A) to_operand<A, T16, AP, EPI>(s, smem + a_off, o0, tail_k, p.R * 128)
                     SPG_CHAIN_ACTS(s.act, SPG_CHAIN_CALL)
 #undef SPG_CHAIN_CALL
                     fence_async_smem();
@@ -650,13 +649,13 @@ spg_chain_kernel(const __grid_constant__ ChainParams p)
                 } else if (l < last) {
                     const uint32_t next_k = p.l[l + 1].kblocks * TK, plane = p.R * 128;
                     uint8_t *next = p.scratch + (uint64_t)(2 * cluster + (e & 1u)) * p.exchange_bytes;
-#define SPG_CHAIN_CALL(A) to_operand<A, T16, AP>(s, next, 0, next_k, plane)
+#define SPG_CHAIN_CALL(A) to_operand<A, T16, AP, EPI>(s, next, 0, next_k, plane)
                     SPG_CHAIN_ACTS(s.act, SPG_CHAIN_CALL)
 #undef SPG_CHAIN_CALL
                     // columns of the last k-block that no CTA's tiles reach
                     if (ok && me == 0 && L.covered < next_k) {
                         const uint32_t pieces = (next_k - L.covered) >> 3, total = pieces * p.R * AP;
-                        for (uint32_t i = threadIdx.x - 128; i < total; i += EPI_THREADS) {
+                        for (uint32_t i = threadIdx.x - 128; i < total; i += 32 * EPI) {
                             const uint32_t k = L.covered + i % pieces * 8, r = i / pieces % p.R, a = i / pieces / p.R;
                             *reinterpret_cast<uint4 *>(next + (uint64_t)((k >> 6) * AP + a) * plane + swizzled(r, k & 63u)) = make_uint4(0, 0, 0, 0);
                         }
@@ -664,13 +663,13 @@ spg_chain_kernel(const __grid_constant__ ChainParams p)
                     __syncwarp();
                     fence_async_global();
                     tc_fence_before();
-                    epi_sync();
+                    epi_sync<EPI>();
                     if (w == 0 && lane < C && !*abort_flag) arrive_release_cluster(mapa(ready, lane));
                     e++;
                 } else if (p.tail) {
                     if (idle) continue;
                     const uint32_t part = p.tail_rows * L.out * 4, at = (round & 1u) * p.tail * part;
-                    if (s.tiles) to_owners<AP>(s, owners, at + me * part, 8 * (round & 1u));
+                    if (s.tiles) to_owners<AP, EPI>(s, owners, at + me * part, 8 * (round & 1u));
                     __syncwarp();
                     ok = ok && wait_cluster(parts_bar + 8 * (round & 1u), (round >> 1) & 1u, abort_flag, p.status, 73);
                     ok = __all_sync(0xffffffffu, ok);
@@ -678,13 +677,13 @@ spg_chain_kernel(const __grid_constant__ ChainParams p)
                     __syncwarp();
                     if (b + clusters >= blocks) { cluster_arrive(); arrived = true; }       // nothing goes to another CTA any more
                     const float *parts = reinterpret_cast<const float *>(smem + parts_off + at);
-                    if (ok && s.out <= 32) put_together<1>(p, s.act, s.out, s.scale, s.bias, parts, s.first + row0, row_count, s.end, w, lane);
-                    else if (ok) put_together<TAIL_MAX / 32>(p, s.act, s.out, s.scale, s.bias, parts, s.first + row0, row_count, s.end, w, lane);
+                    if (ok && s.out <= 32) put_together<1, EPI>(p, s.act, s.out, s.scale, s.bias, parts, s.first + row0, row_count, s.end, w, lane);
+                    else if (ok) put_together<TAIL_MAX / 32, EPI>(p, s.act, s.out, s.scale, s.bias, parts, s.first + row0, row_count, s.end, w, lane);
                     __syncwarp();
                     // (nobody sends its sums of the next block while a row of this one is still read, here or in a neighbour that waits for them)
-                    if (b + clusters < blocks) epi_sync();
+                    if (b + clusters < blocks) epi_sync<EPI>();
                 } else {
-#define SPG_CHAIN_CALL(A) to_output<A, AP>(p, s)
+#define SPG_CHAIN_CALL(A) to_output<A, AP, EPI>(p, s)
                     SPG_CHAIN_ACTS(s.act, SPG_CHAIN_CALL)
 #undef SPG_CHAIN_CALL
                 }
@@ -718,6 +717,16 @@ spg_chain_kernel(const __grid_constant__ ChainParams p)
     if (warp == 1) { tc_fence_after(); tmem_free(tmem, p.tmem_cols); }
 }
 
+using Kernel = void (*)(const ChainParams);
+template <uint32_t EPI> Kernel variant_of(int terms, int type16)
+{
+    if (terms > 2) return spg_chain_kernel<__nv_bfloat16, 2, 2, EPI>;
+    if (terms > 1) return type16 == SPGK_T_F16 ? spg_chain_kernel<__half, 2, 1, EPI> : spg_chain_kernel<__nv_bfloat16, 2, 1, EPI>;
+    return type16 == SPGK_T_F16 ? spg_chain_kernel<__half, 1, 1, EPI> : spg_chain_kernel<__nv_bfloat16, 1, 1, EPI>;
+}
+// terms: of an activation, and three where a weight has two as well
+Kernel variant(int terms, int type16, uint32_t epi) { return epi == 8 ? variant_of<8>(terms, type16) : variant_of<16>(terms, type16); }
+
 // clusters of 1 to 8 CTAs that the device holds at one CTA an SM (0: none)
 struct AtOnce { uint32_t n[MAX_C + 1]; };
 int clusters_at_once(int dev, const SpgDeviceProps &dp, AtOnce &out)
@@ -725,17 +734,18 @@ int clusters_at_once(int dev, const SpgDeviceProps &dp, AtOnce &out)
     static SpgOncePerDevice once;
     static AtOnce known[SPG_MAX_DEVICES];
     const int rc = once.run(dev, [&]() -> int {
-        for (auto kernel : { spg_chain_kernel<__half, 1, 1>, spg_chain_kernel<__half, 2, 1>, spg_chain_kernel<__nv_bfloat16, 1, 1>, spg_chain_kernel<__nv_bfloat16, 2, 1>, spg_chain_kernel<__nv_bfloat16, 2, 2> })
-            SPGK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dp.smem_optin));
+        for (uint32_t terms = 0; terms < 6; terms++)
+            for (uint32_t epi : { 8u, 16u })
+                SPGK_CUDA(cudaFuncSetAttribute(variant((int)(terms >> 1) + 1, terms & 1u ? SPGK_T_F16 : SPGK_T_BF16, epi), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dp.smem_optin));
         for (uint32_t c = 1; c <= MAX_C; c++) {
             cudaLaunchConfig_t cfg = {};
-            cfg.gridDim = dim3(c); cfg.blockDim = dim3(THREADS); cfg.dynamicSmemBytes = 160 * 1024;
+            cfg.gridDim = dim3(c); cfg.blockDim = dim3(threads_of(16)); cfg.dynamicSmemBytes = 160 * 1024;
             cudaLaunchAttribute attr[1];
             attr[0].id = cudaLaunchAttributeClusterDimension;
             attr[0].val.clusterDim.x = c; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
             cfg.attrs = attr; cfg.numAttrs = 1;
             int n = 0;
-            if (cudaOccupancyMaxActiveClusters(&n, spg_chain_kernel<__nv_bfloat16, 2, 1>, &cfg) != cudaSuccess) { cudaGetLastError(); n = 0; }
+            if (cudaOccupancyMaxActiveClusters(&n, spg_chain_kernel<__nv_bfloat16, 2, 1, 16>, &cfg) != cudaSuccess) { cudaGetLastError(); n = 0; }
             known[dev].n[c] = n > 0 ? (uint32_t)n : 0u;
         }
         return SPGK_OK;
@@ -746,20 +756,32 @@ int clusters_at_once(int dev, const SpgDeviceProps &dp, AtOnce &out)
 
 uint32_t ceil_div(uint32_t a, uint32_t b) { return (a + b - 1) / b; }
 
+// Epilogue warps.  A warp finishes eight rows of 32 outputs in one go: sixteen warps would do every row of a block of 16 twice.  Over 2300
+// arrangements of eight nets, time of eight warps against sixteen (median, 5 to 95 %): 16 rows 0.92 (0.84 to 0.96); 32 rows 0.965 (0.93 to
+// 1.05), 48 rows 0.985 (0.94 to 1.02) where the epilogues are plain and the last layer is cut, else 1.03 and 1.02; 64 rows 1.07, 96 rows 1.13.
+uint32_t epilogue_warps(const spgk_layer *layers, uint32_t count, uint32_t R, bool cut)
+{
+    if (R <= 16) return 8;
+    if (R > 48 || !cut) return 16;
+    for (uint32_t l = 0; l + 1 < count; l++) if (layers[l].act == SPG_ACT_TANH || layers[l].act == SPG_ACT_SIGMOID) return 16;
+    return 8;
+}
+
 // How a net's layers are laid out on clusters of C CTAs with blocks of R rows (false: they do not fit), and the cycles of a block.
 // The cycles come from a fit over 2037 arrangements of eight nets (40 to 12000 rows, every size of cluster, one to three products a term):
 // 5 to 95 % of them within 11 %, and the arrangement that it calls the fastest 2 % behind the fastest one on average.
-struct Layout { uint32_t tr[MAX_LAYERS], mt[MAX_LAYERS], mains, SA, SW, a_slot, w_slot, tmem_cols, smem, tail, tail_rows, cycles; };
+struct Layout { uint32_t epi, tr[MAX_LAYERS], mt[MAX_LAYERS], mains, SA, SW, a_slot, w_slot, tmem_cols, smem, tail, tail_rows, cycles; };
 bool lay_out(const spgk_layer *layers, uint32_t count, uint32_t C, uint32_t R, uint32_t a_parts, uint32_t w_parts, bool softmax, bool one_accumulator, size_t smem_max, Layout &o)
 {
-    const uint32_t n = R * a_parts, rounds = ceil_div(R, ROUND), out = layers[count - 1].out;
+    const uint32_t n = R * a_parts, rounds = ceil_div(R, 32), out = layers[count - 1].out;
     if (n > 256) return false;                                 // the widest product
     uint32_t cols = 0, tr_max = 0, kb_max = 0;
     o.tail = out <= TAIL_MAX;
+    o.epi = epilogue_warps(layers, count, R, o.tail != 0);
     if (softmax && !o.tail) return false;
     // a product of K = 16: what it takes to fetch 128 rows of weights (58 cycles), or the tensor pipe's time
     const uint32_t product = (n > 144 ? n / 2 : 58 + n / 10) + (w_parts > 1 ? (R > 144 ? R / 2 : 58 + R / 10) : 0);
-    o.cycles = ceil_div(ceil_div(ceil_div(layers[0].in, TK), KG) * (R / 8), EPI) * 460;
+    o.cycles = ceil_div(ceil_div(ceil_div(layers[0].in, TK), KG) * (R / 8), 16) * 460;
     for (uint32_t l = 0; l < count; l++) {
         const spgk_layer &L = layers[l];
         const bool cut = o.tail && l + 1 == count;
@@ -782,7 +804,8 @@ bool lay_out(const spgk_layer *layers, uint32_t count, uint32_t C, uint32_t R, u
     for (o.tmem_cols = 32; o.tmem_cols < cols; o.tmem_cols <<= 1) { }
     o.a_slot = KG * R * 128 * a_parts; o.w_slot = KG * tr_max * 128 * w_parts;
     o.tail_rows = o.tail ? ceil_div(R, o.tail) : 0;
-    if (o.tail) o.cycles += ceil_div(o.tail_rows, EPI) * (out <= 32 ? 780 : 1330);
+    if (o.tail) o.cycles += ceil_div(o.tail_rows, 16) * (out <= 32 ? 780 : 1330);
+    if (R <= 16) o.cycles -= 2200;                             // (the fit is of sixteen epilogue warps)
     const uint32_t parts = R * 8 + 2 * o.tail * o.tail_rows * out * 4;      // (the table of the rows' owners; sums of two blocks)
     if (parts + BAR_BYTES > smem_max) return false;
     const uint32_t room = (uint32_t)smem_max - BAR_BYTES - parts;
@@ -818,7 +841,7 @@ float layered_us(const spgk_layer *layers, uint32_t count, uint32_t N, uint32_t 
 }
 
 // The cheapest arrangement for a number of rows (0: none): C, R and microseconds.  only: that size of cluster and one accumulator.
-float cheapest(const spgk_layer *layers, uint32_t count, uint32_t rows, uint32_t a_parts, uint32_t w_parts, bool softmax, uint32_t only, const AtOnce &at, size_t smem_max,
+float cheapest(const spgk_layer *layers, uint32_t count, uint32_t rows, uint32_t a_parts, uint32_t w_parts, bool softmax, uint32_t only, const AtOnce &at, const SpgDeviceProps &dp,
                uint32_t &best_C, uint32_t &best_R)
 {
     uint64_t best = ~0ull;
@@ -828,9 +851,11 @@ float cheapest(const spgk_layer *layers, uint32_t count, uint32_t rows, uint32_t
         for (uint32_t waves = 1, tried = 0; waves <= 16 && tried < 3; waves++) {
             const uint32_t R = (ceil_div(rows, at.n[C] * waves) + 15) & ~15u;
             Layout o;
-            if (R > MAX_R || !lay_out(layers, count, C, R, a_parts, w_parts, softmax, only != 0, smem_max, o)) continue;
+            if (R > MAX_R || !lay_out(layers, count, C, R, a_parts, w_parts, softmax, only != 0, dp.smem_optin, o)) continue;
             tried++;
-            const uint64_t cost = (uint64_t)o.cycles * ceil_div(ceil_div(rows, R), at.n[C]);
+            const uint32_t blocks = ceil_div(rows, R), busy = (blocks < at.n[C] ? blocks : at.n[C]) * C;
+            // (on five eighths of the chip or less the next launch's first blocks get started beside this one's last)
+            const uint64_t cost = (uint64_t)o.cycles * ceil_div(blocks, at.n[C]) + (busy * 8 > (uint32_t)dp.sm_count * 5 ? 1000 : 0);
             if (cost < best) { best = cost; best_C = C; best_R = R; }
             if (R == 16) break;
         }
@@ -859,12 +884,12 @@ int spgk_chain_plan(const spgk_layer *layers, uint32_t count, uint32_t N, int w_
     // the net comes here and on clusters of which size, goes by 1024 rows whatever the guess.
     const bool counted = spg_tls_rows_limit != nullptr, softmax = softmax_fused != 0;
     const uint32_t a = (uint32_t)a_parts, w = (uint32_t)w_parts, rows = counted && N > 1024 ? 1024 : N;
-    plan->us = cheapest(layers, count, rows, a, w, softmax, counted ? COUNTED_C : 0, at, dp.smem_optin, plan->C, plan->R);
+    plan->us = cheapest(layers, count, rows, a, w, softmax, counted ? COUNTED_C : 0, at, dp, plan->C, plan->R);
     if (plan->us == 0.0f) return SPGK_E_UNSUPPORTED;
     plan->layered_us = layered_us(layers, count, rows, (uint32_t)dp.sm_count, a, w);
     if (counted) {
         const uint32_t seen = spg_tls_rows_expected ? spg_tls_rows_expected : 1024, likely = seen + 3u * (uint32_t)sqrtf((float)seen);      // (what a selection by chance varies)
-        cheapest(layers, count, likely < N ? likely : N, a, w, softmax, COUNTED_C, at, dp.smem_optin, plan->C, plan->R);
+        cheapest(layers, count, likely < N ? likely : N, a, w, softmax, COUNTED_C, at, dp, plan->C, plan->R);
     }
     const uint32_t blocks = ceil_div(N, plan->R);
     plan->clusters = blocks < at.n[plan->C] ? blocks : at.n[plan->C];
@@ -913,17 +938,14 @@ int spgk_chain_forward(const spgk_chain *plan, const spgk_layer *layers, uint32_
     p.impatient = spg_gemm_impatient() ? 1 : 0;
     p.status = status;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(plan->clusters * plan->C); cfg.blockDim = dim3(THREADS); cfg.dynamicSmemBytes = o.smem; cfg.stream = (cudaStream_t)stream;
+    cfg.gridDim = dim3(plan->clusters * plan->C); cfg.blockDim = dim3(threads_of(o.epi)); cfg.dynamicSmemBytes = o.smem; cfg.stream = (cudaStream_t)stream;
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = plan->C; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
     attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr; cfg.numAttrs = 2;
-    const bool f16 = type16 == SPGK_T_F16;
-    if (w_parts > 1) SPGK_CUDA(cudaLaunchKernelEx(&cfg, spg_chain_kernel<__nv_bfloat16, 2, 2>, p));
-    else if (a_parts > 1) SPGK_CUDA(cudaLaunchKernelEx(&cfg, f16 ? spg_chain_kernel<__half, 2, 1> : spg_chain_kernel<__nv_bfloat16, 2, 1>, p));
-    else SPGK_CUDA(cudaLaunchKernelEx(&cfg, f16 ? spg_chain_kernel<__half, 1, 1> : spg_chain_kernel<__nv_bfloat16, 1, 1>, p));
+    SPGK_CUDA(cudaLaunchKernelEx(&cfg, variant(w_parts > 1 ? 3 : a_parts, type16, o.epi), p));
     tls_arrangement[0] = plan->C; tls_arrangement[1] = plan->R;
     return spgk_check_launch("spg_chain_kernel");
 }
