@@ -169,45 +169,45 @@ template <int ACT, int N> __device__ __forceinline__ void activate(float (&v)[N]
     }
 }
 // A layer's activation is chosen once, outside the loops (a branch inside costs as much as the activation)
-#define SPG_CHAIN_ACTS(act, call)                                                              \
+#define SPG_CHAIN_ACTS(act, both, call)                                                        \
     switch (act) {                                                                             \
-        case SPG_ACT_RELU:  call(SPG_ACT_RELU); break;                                         \
-        case SPG_ACT_LEAKY: call(SPG_ACT_LEAKY); break;                                        \
-        case SPG_ACT_FOO52: call(SPG_ACT_FOO52); break;                                        \
-        case SPG_ACT_NONE:  call(SPG_ACT_NONE); break;                                         \
-        default:            call(CURVED); break;                                               \
+        case SPG_ACT_RELU:  if (both) call(SPG_ACT_RELU, true); else call(SPG_ACT_RELU, false); break;    \
+        case SPG_ACT_LEAKY: if (both) call(SPG_ACT_LEAKY, true); else call(SPG_ACT_LEAKY, false); break;  \
+        case SPG_ACT_FOO52: if (both) call(SPG_ACT_FOO52, true); else call(SPG_ACT_FOO52, false); break;  \
+        case SPG_ACT_NONE:  if (both) call(SPG_ACT_NONE, true); else call(SPG_ACT_NONE, false); break;    \
+        default:            if (both) call(CURVED, true); else call(CURVED, false); break;                \
     }
 
 // One output of eight rows: four from a place in sixteen rows on, and the four sixteen further on, or the first four again where the block has
 // no more.  (A warp's instructions hang on one another: eight rows take little longer than four, 560 cycles.)  The accumulators' sums in
 // their order.
-template <int AP>
+template <int AP, bool BOTH>
 __device__ __forceinline__ void sums8(const Slice &s, uint32_t taddr, uint32_t more, float (&v)[8])
 {
-    // (a layer with one accumulator reads it twice: loads that depend on a condition cost the compiler its registers)
-    const bool both = s.mains > 1;
-    const uint32_t second = both ? AP * s.n : 0;
+    const uint32_t second = AP * s.n;
     uint32_t hi[2][4], lo[2][4], hi2[2][4], lo2[2][4];
 #pragma unroll
     for (int h = 0; h < 2; h++) {
         const uint32_t at = taddr + (h ? more : 0);
         tmem_ld4(at, hi[h]);
-        tmem_ld4(at + second, hi2[h]);
-        if (AP > 1) { tmem_ld4(at + s.n, lo[h]); tmem_ld4(at + second + s.n, lo2[h]); }
+        if (AP > 1) tmem_ld4(at + s.n, lo[h]);
+        if (BOTH) tmem_ld4(at + second, hi2[h]);
+        if (BOTH && AP > 1) tmem_ld4(at + second + s.n, lo2[h]);
     }
     tmem_ld_wait();
 #pragma unroll
     for (int i = 0; i < 8; i++) {
         const int h = i >> 2, j = i & 3;
-        v[i] = __uint_as_float(hi[h][j]) + (both ? __uint_as_float(hi2[h][j]) : 0.0f);
-        if (AP > 1) v[i] += __uint_as_float(lo[h][j]) + (both ? __uint_as_float(lo2[h][j]) : 0.0f);
+        v[i] = __uint_as_float(hi[h][j]);
+        if (BOTH) v[i] += __uint_as_float(hi2[h][j]);
+        if (AP > 1) v[i] += BOTH ? __uint_as_float(lo[h][j]) + __uint_as_float(lo2[h][j]) : __uint_as_float(lo[h][j]);
     }
 }
 // ... scale, bias, activation
-template <int ACT, int AP>
+template <int ACT, int AP, bool BOTH>
 __device__ __forceinline__ void finish8(const Slice &s, uint32_t taddr, uint32_t more, float bias, float (&v)[8])
 {
-    sums8<AP>(s, taddr, more, v);
+    sums8<AP, BOTH>(s, taddr, more, v);
 #pragma unroll
     for (int i = 0; i < 8; i++) v[i] = fmaf(v[i], s.scale, bias);
     activate<ACT>(v, s.act);
@@ -215,7 +215,7 @@ __device__ __forceinline__ void finish8(const Slice &s, uint32_t taddr, uint32_t
 
 // A layer's outputs become the next one's operand: [k-block][plane][row] of 128 bytes.  Lane pairs trade rows so that each writes
 // two neighbouring values at once.  Columns beyond the layer's outputs get the activation of zero, whose weights are zeros.
-template <int ACT, typename T16, int AP, uint32_t EPI>
+template <int ACT, bool BOTH, typename T16, int AP, uint32_t EPI>
 __device__ __forceinline__ void to_operand(const Slice &s, uint8_t *next, uint32_t k0, uint32_t next_k, uint32_t plane)
 {
     const uint32_t odd = s.lane & 1u;
@@ -232,7 +232,7 @@ __device__ __forceinline__ void to_operand(const Slice &s, uint8_t *next, uint32
         for (uint32_t c = 4 * s.g; c < s.n; c += 2 * EPI, taddr += 2 * EPI, dst += 2 * EPI * 128) {
             const bool two = c + EPI < s.n;
             float v[8];
-            finish8<ACT, AP>(s, taddr, two ? EPI : 0, bias, v);
+            finish8<ACT, AP, BOTH>(s, taddr, two ? EPI : 0, bias, v);
 #pragma unroll
             for (int i = 0; i < 8; i += 2) {
                 const float got = __shfl_xor_sync(0xffffffffu, odd ? v[i] : v[i + 1], 1);
@@ -248,7 +248,7 @@ __device__ __forceinline__ void to_operand(const Slice &s, uint8_t *next, uint32
     }
 }
 
-template <int ACT, int AP, uint32_t EPI>
+template <int ACT, bool BOTH, int AP, uint32_t EPI>
 __device__ __forceinline__ void to_output(const ChainParams &p, const Slice &s)
 {
 #pragma unroll 1
@@ -260,7 +260,7 @@ __device__ __forceinline__ void to_output(const ChainParams &p, const Slice &s)
 #pragma unroll 1
         for (uint32_t c = 4 * s.g; c < s.n; c += 2 * EPI) {
             float v[8];
-            finish8<ACT, AP>(s, taddr + c, c + EPI < s.n ? EPI : 0, bias, v);
+            finish8<ACT, AP, BOTH>(s, taddr + c, c + EPI < s.n ? EPI : 0, bias, v);
 #pragma unroll
             for (int i = 0; i < 8; i++) {
                 const uint32_t r = c + (i & 3) + (i >> 2) * EPI, row = s.first + r;
@@ -280,7 +280,7 @@ template <int AP, uint32_t EPI> __device__ __forceinline__ void to_owners(const 
     for (uint32_t c = 4 * s.g; c < s.n; c += 2 * EPI) {
         const uint32_t more = c + EPI < s.n ? EPI : 0;
         float v[8];
-        sums8<AP>(s, s.tmem + c, more, v);                     // (by whole warps)
+        sums8<AP, false>(s, s.tmem + c, more, v);                     // (by whole warps)
         if (s.o < s.out) {
 #pragma unroll
             for (int i = 0; i < 8; i++) {
@@ -340,8 +340,8 @@ __device__ __forceinline__ void put_together(const ChainParams &p, int act, uint
 #pragma unroll
             for (int i = 0; i < PER; i++) if ((uint32_t)i * 32 + lane < out) y[i * 32 + lane] = v[i] * inv;
         } else if (lane < out) {
-#define SPG_CHAIN_CALL(A) activate<A>(v, act)
-            SPG_CHAIN_ACTS(act, SPG_CHAIN_CALL)
+#define SPG_CHAIN_CALL(A, B) activate<A>(v, act)
+            SPG_CHAIN_ACTS(act, false, SPG_CHAIN_CALL)
 #undef SPG_CHAIN_CALL
 #pragma unroll
             for (int i = 0; i < PER; i++) if ((uint32_t)i * 32 + lane < out) y[i * 32 + lane] = v[i];
@@ -639,8 +639,8 @@ spg_chain_kernel(const __grid_constant__ ChainParams p)
                 if (p.tail && l + 1 == last) {
                     if (idle) continue;
                     // (every copy into the activation ring has been used up: its memory holds the CTA's own outputs until they are multiplied)
-#define SPG_CHAIN_CALL(A) to_operand<A, T16, AP, EPI>(s, smem + a_off, o0, tail_k, p.R * 128)
-                    SPG_CHAIN_ACTS(s.act, SPG_CHAIN_CALL)
+#define SPG_CHAIN_CALL(A, B) to_operand<A, B, T16, AP, EPI>(s, smem + a_off, o0, tail_k, p.R * 128)
+                    SPG_CHAIN_ACTS(s.act, s.mains > 1, SPG_CHAIN_CALL)
 #undef SPG_CHAIN_CALL
                     fence_async_smem();
                     tc_fence_before();
@@ -649,8 +649,8 @@ spg_chain_kernel(const __grid_constant__ ChainParams p)
                 } else if (l < last) {
                     const uint32_t next_k = p.l[l + 1].kblocks * TK, plane = p.R * 128;
                     uint8_t *next = p.scratch + (uint64_t)(2 * cluster + (e & 1u)) * p.exchange_bytes;
-#define SPG_CHAIN_CALL(A) to_operand<A, T16, AP, EPI>(s, next, 0, next_k, plane)
-                    SPG_CHAIN_ACTS(s.act, SPG_CHAIN_CALL)
+#define SPG_CHAIN_CALL(A, B) to_operand<A, B, T16, AP, EPI>(s, next, 0, next_k, plane)
+                    SPG_CHAIN_ACTS(s.act, s.mains > 1, SPG_CHAIN_CALL)
 #undef SPG_CHAIN_CALL
                     // columns of the last k-block that no CTA's tiles reach
                     if (ok && me == 0 && L.covered < next_k) {
@@ -683,8 +683,8 @@ spg_chain_kernel(const __grid_constant__ ChainParams p)
                     // (nobody sends its sums of the next block while a row of this one is still read, here or in a neighbour that waits for them)
                     if (b + clusters < blocks) epi_sync<EPI>();
                 } else {
-#define SPG_CHAIN_CALL(A) to_output<A, AP, EPI>(p, s)
-                    SPG_CHAIN_ACTS(s.act, SPG_CHAIN_CALL)
+#define SPG_CHAIN_CALL(A, B) to_output<A, B, AP, EPI>(p, s)
+                    SPG_CHAIN_ACTS(s.act, s.mains > 1, SPG_CHAIN_CALL)
 #undef SPG_CHAIN_CALL
                 }
                 __syncwarp();
