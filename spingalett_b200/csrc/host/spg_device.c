@@ -408,34 +408,50 @@ static bool all_wstream(const spg_net *n, uint32_t N)
 }
 
 /* Up to eight rows of a net of few weights go warp by warp from L2, whatever their precision, widths and alignment.  The lines lie where the
- * kernel meets what serves otherwise (us a call, this kernel / the GEMV or the general kernels), in weights a layer on average, since every
- * layer costs the others a launch or a chain's step: nets of integers at two rows or more 4 Mi (one layer of 4.1 million INT4 weights at
- * four rows 15 / 18, of 5.1 million 23 / 18, of 8.4 million 24 / 19, at one row 12 / 36; two layers of 8.3 million 27 / 28, three 33 / 50);
- * rows of odd lengths, which are loaded one by one, 3 Mi (INT4 in one layer of 4 million 29 / 21 at four rows, two layers of 6.1 million 44
- * / 60), of fp32 at five to seven rows 2 Mi (three layers of 6.5 million 75 / 71, of 8.1 million 99 / 78; 98 / 254 at eight).  Every output is a
- * warp, which is much beside the streaming kernel's way with short rows of integers: 64-65536-32 in INT4 126 / 93 at four rows, 64-32768-100 68 / 62.  25
- * million INT2 weights take 148 / 49 at six rows. */
-#define SPG_ROWS_MAX_WEIGHTS ((uint64_t)8 << 20)
+ * kernel meets what serves otherwise, in weights a layer on average, since every layer costs the others a launch or a chain's step (us a
+ * call, this kernel / the other):
+ * - integers in whole 16 bytes a row, which the streaming kernels take: 8 Mi in all at one row, 4 Mi a layer beyond (one layer of 4.1 million
+ *   INT4 weights at four rows 15 / 18, of 5.1 million 23 / 18, of 8.4 million 24 / 19, at one row 12 / 36; 2048-2048-2048-2048-100 at two
+ *   rows 27 / 33, at four 42 / 42, at six 52 / 44).  Every output is a warp, which is much beside the streaming kernel's way with short
+ *   rows: 64-65536-32 in INT4 126 / 93 at four rows, 64-32768-100 68 / 62.
+ * - floats that the GEMV takes: at one row up to 32 Mi in a layer (8192-4096 in fp32 29 / 34, 16000-4000 in BF16 45 / 31), beyond 8 Mi in all, or
+ *   10 Mi a layer in three and more (2048-2048-2048-2048-100 in FP16 at three rows 38 / 58, at eight 64 / 121; 2048-4096-4096-512 in fp32 44 / 56 at
+ *   two, 117 / 159 at eight; 3000-6000-2056-5000-304 in BF16 at two 69 / 64, at four 113 / 93; one layer of 16 Mi at four 34 / 25); where a row ends
+ *   on half a lane's values 3 Mi (2000-1900-1800-1700-100 in fp32 33 / 45 at two, 67 / 129 at eight).
+ * - rows for the general kernel, whose reads are uneven: up to 18 Mi in a layer (2000-1900-1800-1700-100 in INT8 at one row 25 / 37, at eight 58 / 362;
+ *   3000-6000-2056-5000-304 in INT4 45 / 80 and 155 / 898; 8000-3000-10, 23 Mi, in INT2 at one row 27 / 25, at six 74 / 68).
+ * - rows of odd lengths, loaded one by one: 3 Mi a layer (2001-1901-1803-1707-101 in INT4 at one row 37 / 43, at eight 125 / 424; INT4 in one layer of 4 million
+ *   at four rows 24 / 23, at six 32 / 25); at two, three and eight rows 12 Mi in several layers (3001-6001-2051-5003-301 in INT8 131 / 272, 195 / 322 and
+ *   392 / 948; at one row 76 / 62).  fp32: 3 Mi, at five to seven rows 2 Mi (three layers of 6.5 million 75 / 71, of 8.1 million 99 / 78; 98 / 254 at eight),
+ *   and at one and four no more than 8 Mi in all (the 2001-...-101 net 39 / 36 and 110 / 107). */
 #define SPG_ROWS_MAX_OUTPUTS 65535u                 /* of a layer of integers */
 
 static bool few_weights(const spg_net *n, uint32_t N)
 {
     const PrecisionMode prec = n->klayers[0].precision;
-    const bool integers = prec >= PRECISION_INT8;
-    uint64_t count = 0;
+    const bool integers = prec >= PRECISION_INT8, fp32 = prec == PRECISION_FLOAT32;
+    const uint32_t line = prec == PRECISION_FLOAT32 ? 4 : !integers ? 8 : 16u << (prec - PRECISION_INT8);       /* weights in 16 bytes */
+    const uint64_t mi = (uint64_t)1 << 20, layers = n->dev_layers;
+    uint64_t count = 0, largest = 0;
     uint32_t widest = 0;
-    bool odd = false, streams = true;           /* some rows are no multiple of a lane's eight values; all are whole 16 bytes of integers */
+    bool odd = false, streams = true;           /* some rows are no multiple of a lane's eight values; all are whole 16 bytes */
     for (uint32_t l = 0; l < n->dev_layers; l++) {
         const spgk_layer *L = &n->klayers[l];
+        const uint64_t weights = (uint64_t)L->in * L->out;
         odd = odd || L->in % 8;
-        streams = streams && integers && L->in % (16u << (prec - PRECISION_INT8)) == 0;
+        streams = streams && L->in % line == 0;
         if (L->out > widest) widest = L->out;
-        count += (uint64_t)L->in * L->out;
+        if (weights > largest) largest = weights;
+        count += weights;
     }
-    if (streams && widest > SPG_ROWS_MAX_OUTPUTS) return false;
-    const uint64_t mi = (uint64_t)1 << 20;
-    const uint64_t each = odd ? (prec == PRECISION_FLOAT32 && N > 4 && N < 8 ? 2 * mi : 3 * mi) : integers && N > 1 ? 4 * mi : SPG_ROWS_MAX_WEIGHTS;
-    return count <= SPG_ROWS_MAX_WEIGHTS && count <= each * n->dev_layers;
+    if (streams && integers && widest > SPG_ROWS_MAX_OUTPUTS) return false;
+    if (count <= 8 * mi && count <= (odd ? (fp32 && N > 4 && N < 8 ? 2 : 3) : integers && N > 1 ? 4 : 8) * mi * layers) return true;
+    if (streams && integers) return (N == 2 || N == 3) && count <= 16 * mi && count <= 4 * mi * layers;
+    if (streams && N == 1 && !odd) return largest <= 32 * mi;
+    if (streams) return layers > 2 && count <= (odd ? 3 : 10) * mi * layers;
+    if (!odd) return largest <= 18 * mi;
+    if (fp32) return N != 1 && N != 4 && count <= (N > 4 && N < 8 ? 2 : 3) * mi * layers;
+    return count <= (layers > 1 && (N == 2 || N == 3 || N == 8) ? 12 : 3) * mi * layers;
 }
 
 /* Small / medium batches (fp32 activations between layers; every layer streams its packed weights once).
