@@ -89,8 +89,11 @@ KERNEL_OF_PATH = {"rows": "spg_rows_kernel", "gemv": "spg_gemv_kernel", "istream
 
 
 def kernels(path, topo, batch):
-    """The path's kernel, and with it the one on pairs of CTAs where layers have more 128 x 256 tiles than the GPU has SMs."""
+    """The path's kernel, and with it the one on pairs of CTAs where layers have more 128 x 256 tiles than the GPU has SMs.  Nets of up to some
+    thousand rows whose layers a cluster can share out run in one launch where an estimate says so."""
     name = KERNEL_OF_PATH.get(path, path)
+    if path.startswith("tcgen05") and batch <= 8192 and max(topo[1:]) <= 4096:
+        return "spg_chain_kernel or " + name
     pairs = path == "tcgen05" and any(-(-batch // 128) * -(-b // 256) > 148 and a >= 512 and b > 128 for a, b in zip(topo, topo[1:]))
     return "spg_gemm_pair_kernel, " + name if pairs else name
 
@@ -596,7 +599,7 @@ def main():
                             "whole_step_frac": flops / (dev_ms * args.steps * 1e-3) / 1e12 / pk["bf16_tflops"],
                             "note": ("frac: the one launch per step that computes all three layers of all rows (event pair around it); "
                                      "whole_step_frac: the same FLOPs over ms_per_step, which in AUTO also holds the exact "
-                                     "recomputation of the low-margin rows (per-layer kernels on a percent or two of the rows)")
+                                     "recomputation of the low-margin rows (one launch of spg_chain_kernel on a percent or two of the rows)")
                                     if fused else "frac: summed device time of the layer kernels (event pairs); whole_step_frac: over ms_per_step"}
     elif k_cnt:
         nbytes = algorithmic_bytes(topo, args.dtype, batch)      # per step, all layers (one kernel launch per layer)

@@ -330,9 +330,9 @@ SPINGALETT_API int spingalett_synchronize(NeuralNetwork *net);
  * AUTO runs batches of up to 512 rows in EXACT: a chain that is bound by
  * streaming the weights pays next to nothing for the second term.
  * Integer files (INT8, INT4, INT2) at 1 to 24 rows, and outside EXACT at up to
- * 256: a layer's inputs are fixed-point numbers of 28 bits with exact products
+ * 448: a layer's inputs are fixed-point numbers of 28 bits with exact products
  * and sums, a row's scale being at least its largest magnitude (at 7 rows or
- * more just that).  From 7 rows on, when more than an eighth of a row's
+ * more, outside EXACT at 3, just that).  From there on, when more than an eighth of a row's
  * non-zero values would keep less than 16 bits that way, those values are held
  * in 28 bits of their own; fewer such values keep 2^-28 of the maximum. */
 typedef enum { SPINGALETT_MATH_FAST = 0, SPINGALETT_MATH_EXACT = 1, SPINGALETT_MATH_AUTO = 2 } SpingalettMathMode;

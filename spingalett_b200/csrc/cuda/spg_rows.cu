@@ -15,7 +15,7 @@
 // weight-streaming GEMV, made to keep HBM busy, or the general kernel where rows are no multiple of 16 bytes) and now, us a call:
 // 784-512-1000-10 at one row fp32 31.6 -> 8.0, INT8 46 -> 7.8, INT4 26 -> 7.9; at eight rows fp32 90 -> 12, INT4 118 -> 10.4;
 // 301-777-333-129-37 fp32 at one row 22.6 -> 12 to 17, at eight 103 -> 19; 1024-1024-1024-1024-16 BF16 35 -> 12.5 and 117 -> 23.
-// forward() of one sample 57 -> 36 (28 of them launches, device time and the wait).  Error against 64 bits 5e-8 to 2e-7 (before:
+// forward() of one sample 57 -> 36, and 22 since its launches are replayed as a graph and the answer is taken as it arrives.  Error against 64 bits 5e-8 to 2e-7 (before:
 // 1e-7 to 5e-6).  An input that travels as a parameter of the first launch instead of through the fetch kernel: level.
 //
 // Reference: forward's layer step, Src/Spingalett.Network.c:218-247; decode of Src/Spingalett.Serialize.c:222-294.

@@ -2,11 +2,12 @@
  *
  * The weights go to the GPU exactly as stored (packed INT8/INT4/INT2, FP16,
  * BF16 or FP32 images, one 256-byte aligned allocation per matrix); biases go
- * as fp32.  Two chains exist: the small-batch chain (fused dequant-GEMV per
- * layer, fp32 activations) and the large-batch chain (tcgen05 GEMM per layer,
- * 16-bit activations between layers).  Shapes a fast kernel does not take run
- * on the general SIMT kernel -- still on the GPU; nothing here computes on
- * the CPU. */
+ * as fp32.  A few rows go through kernels that read the packed weights (small
+ * nets from L2, the GEMV, the streaming kernels), more through a whole net in
+ * one launch (spg_chain.cu, or the three-layer kernel on large batches) or the
+ * tcgen05 GEMM layer by layer, on 16-bit operands.  Shapes a fast kernel does
+ * not take run on the general SIMT kernel -- still on the GPU; nothing here
+ * computes on the CPU. */
 #include "spg_internal.h"
 #include <pthread.h>
 #include <stdlib.h>
@@ -907,7 +908,7 @@ static int large_chain(spg_net *n, const float *d_x, uint32_t N, float *d_out, b
 
 #define SPG_AUTO_EXACT_ROWS 512u     /* AUTO runs batches of up to this many rows in EXACT */
 #define SPG_AUTO_RECAL 1024u         /* large AUTO calls between two measurements of the margin */
-#define SPG_FUSED_MIN_ROWS 1024u     /* below this a handful of 128-row tiles cannot fill the GPU: the per-layer chain spreads better */
+#define SPG_FUSED_MIN_ROWS 1024u     /* below this a handful of 128-row tiles cannot fill the GPU (spg_chain.cu, where it takes the net, up to what its estimate says) */
 
 /* 16-bit flavour of the one-term pass: fp16, except for a BF16 file with weights beyond fp16's range */
 static int fast_type(spg_net *n)
@@ -1072,7 +1073,7 @@ int spg_dev_forward_large(spg_net *n, const float *d_x, uint32_t N, float *d_out
         if ((rc = reserve((void **)&n->d_rep_out, &n->rep_out_bytes, (size_t)N * outw * 4, "repair outputs"))) return rc;
     }
     /* The flagged rows are a percent or two of the batch, so either repair is one latency-bound pass over a handful of
-     * tiles.  Measured on the benchmark MLP at 65536 rows: the per-layer exact chain takes 30 us, the one-launch kernel
+     * tiles.  Measured on the benchmark MLP at 65536 rows: the exact chain takes 30 us layer by layer, 26 in one launch (spg_chain.cu), the one-launch kernel
      * in pair mode 93 us (a single 128-row tile runs its 13 + 32 k-blocks and six epilogues back to back), so the chain
      * is the default; SPINGALETT_REPAIR=fused selects the other for comparisons. */
     static int repair_fused = -1;
