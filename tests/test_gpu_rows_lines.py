@@ -1,6 +1,7 @@
 """Which nets of more than 8 Mi weights the small-net kernel takes (one to eight rows): on either side of the lines, and right on both."""
 import pytest
 
+from test_gpu_rows import test_a_sample_from_host_memory_gives_what_a_batch_of_one_gives as check_sample
 from test_gpu_rows import test_which_nets_go_there as check
 
 pytestmark = pytest.mark.gpu
@@ -20,3 +21,8 @@ pytestmark = pytest.mark.gpu
     ([5003, 5029, 13], "int4", 8, False), ([1777, 1770, 1770, 1770], "fp32", 8, True), ([1777, 1770, 1770, 1770], "fp32", 4, False), ([1777, 1770, 1770, 1770], "fp32", 6, False)])
 def test_which_large_nets_go_there(spg, tmp_path, topo, precision, n, rows):
     check(spg, tmp_path, topo, precision, n, rows)
+
+
+@pytest.mark.parametrize("topo", [[2048, 2048, 2048, 1000], [4096, 2560, 100]])
+def test_a_sample_of_a_large_net(spg, topo):
+    check_sample(spg, topo, 5)
