@@ -593,7 +593,7 @@ spg_chain_kernel(const __grid_constant__ ChainParams p)
             }
     } else if (warp >= 4) {
         // ---- the input's terms, then every layer's outputs --------------------------------------------------------------------
-        // (all sixteen warps come to every epi_sync: one that has given up goes through the loops without doing anything)
+        // (all EPI warps come to every epi_sync: one that has given up goes through the loops without doing anything)
         const uint32_t w = warp - 4;
         Ring ring;
         uint32_t e = 0, finished = 0, round = 0;
@@ -681,11 +681,17 @@ spg_chain_kernel(const __grid_constant__ ChainParams p)
                     else if (ok) put_together<TAIL_MAX / 32, EPI>(p, s.act, s.out, s.scale, s.bias, parts, s.first + row0, row_count, s.end, w, lane);
                     __syncwarp();
                     // (nobody sends its sums of the next block while a row of this one is still read, here or in a neighbour that waits for them)
+                    tc_fence_before();
                     if (b + clusters < blocks) epi_sync<EPI>();
                 } else {
 #define SPG_CHAIN_CALL(A, B) to_output<A, B, AP, EPI>(p, s)
                     SPG_CHAIN_ACTS(s.act, s.mains > 1, SPG_CHAIN_CALL)
 #undef SPG_CHAIN_CALL
+                    // The next block's first products take the place of these sums as soon as the first R / 8 warps have rounded a stage of its input:
+                    // no warp begins with that before all of them have read theirs.
+                    tc_fence_before();
+                    __syncwarp();
+                    if (b + clusters < blocks) epi_sync<EPI>();
                 }
                 __syncwarp();
                 tc_fence_before();
