@@ -180,9 +180,10 @@ template <int ACT, int N> __device__ __forceinline__ void activate(float (&v)[N]
 
 // One output of eight rows: four from a place in sixteen rows on, and the four sixteen further on, or the first four again where the block has
 // no more.  (A warp's instructions hang on one another: eight rows take little longer than four, 560 cycles.)  The accumulators' sums in
-// their order.
+// their order; zeros where the output is a dead one of a warp that has some (edge: masks in every warp cost 3001 rows of 301-777-333-129-37 0.8 us of
+// 31, a branch behind the wait 0.1; zeros stored afterwards 0.7 to 3.5).
 template <int AP, bool BOTH>
-__device__ __forceinline__ void sums8(const Slice &s, uint32_t taddr, uint32_t more, float (&v)[8])
+__device__ __forceinline__ void sums8(const Slice &s, uint32_t taddr, uint32_t more, bool edge, bool dead, float (&v)[8])
 {
     const uint32_t second = AP * s.n;
     uint32_t hi[2][4], lo[2][4], hi2[2][4], lo2[2][4];
@@ -195,6 +196,17 @@ __device__ __forceinline__ void sums8(const Slice &s, uint32_t taddr, uint32_t m
         if (BOTH && AP > 1) tmem_ld4(at + second + s.n, lo2[h]);
     }
     tmem_ld_wait();
+    if (edge) {
+        const uint32_t keep = dead ? 0u : 0xFFFFFFFFu;
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+            const int h = i >> 2, j = i & 3;
+            hi[h][j] &= keep;
+            if (AP > 1) lo[h][j] &= keep;
+            if (BOTH) hi2[h][j] &= keep;
+            if (BOTH && AP > 1) lo2[h][j] &= keep;
+        }
+    }
 #pragma unroll
     for (int i = 0; i < 8; i++) {
         const int h = i >> 2, j = i & 3;
@@ -205,16 +217,17 @@ __device__ __forceinline__ void sums8(const Slice &s, uint32_t taddr, uint32_t m
 }
 // ... scale, bias, activation
 template <int ACT, int AP, bool BOTH>
-__device__ __forceinline__ void finish8(const Slice &s, uint32_t taddr, uint32_t more, float bias, float (&v)[8])
+__device__ __forceinline__ void finish8(const Slice &s, uint32_t taddr, uint32_t more, float bias, bool edge, bool dead, float (&v)[8])
 {
-    sums8<AP, BOTH>(s, taddr, more, v);
+    sums8<AP, BOTH>(s, taddr, more, edge, dead, v);
 #pragma unroll
     for (int i = 0; i < 8; i++) v[i] = fmaf(v[i], s.scale, bias);
     activate<ACT>(v, s.act);
 }
 
 // A layer's outputs become the next one's operand: [k-block][plane][row] of 128 bytes.  Lane pairs trade rows so that each writes
-// two neighbouring values at once.  Columns beyond the layer's outputs get the activation of zero, whose weights are zeros.
+// two neighbouring values at once.  Columns beyond the layer's outputs get the activation of zero, whose weights are zeros.  Their own sums are not taken
+// for it: a row with an infinity times weights of zero is NaN, and so it would be with the next layer's zeros.
 template <int ACT, bool BOTH, typename T16, int AP, uint32_t EPI>
 __device__ __forceinline__ void to_operand(const Slice &s, uint8_t *next, uint32_t k0, uint32_t next_k, uint32_t plane)
 {
@@ -223,6 +236,7 @@ __device__ __forceinline__ void to_operand(const Slice &s, uint8_t *next, uint32
     for (uint32_t t = 0; t < s.tiles; t++) {
         const uint32_t k = ((s.o + t * s.tr) & ~1u) - k0;      // (k0: the operand's first column)
         const bool in = s.q * 32 + s.lane < s.tr && k < next_k;                               // (tr, next_k: even)
+        const bool dead = s.o + t * s.tr >= s.out, edge = __any_sync(0xffffffffu, dead);
         const float bias = t == 0 ? s.bias[0] : t == 1 ? s.bias[1] : t == 2 ? s.bias[2] : s.bias[3];
         uint32_t taddr = s.tmem + t * s.mains * AP * s.n + 4 * s.g;
         uint8_t *dst = next + (k >> 6) * (AP * plane) + 4 * s.g * 128;
@@ -232,7 +246,7 @@ __device__ __forceinline__ void to_operand(const Slice &s, uint8_t *next, uint32
         for (uint32_t c = 4 * s.g; c < s.n; c += 2 * EPI, taddr += 2 * EPI, dst += 2 * EPI * 128) {
             const bool two = c + EPI < s.n;
             float v[8];
-            finish8<ACT, AP, BOTH>(s, taddr, two ? EPI : 0, bias, v);
+            finish8<ACT, AP, BOTH>(s, taddr, two ? EPI : 0, bias, edge, dead, v);
 #pragma unroll
             for (int i = 0; i < 8; i += 2) {
                 const float got = __shfl_xor_sync(0xffffffffu, odd ? v[i] : v[i + 1], 1);
@@ -260,7 +274,7 @@ __device__ __forceinline__ void to_output(const ChainParams &p, const Slice &s)
 #pragma unroll 1
         for (uint32_t c = 4 * s.g; c < s.n; c += 2 * EPI) {
             float v[8];
-            finish8<ACT, AP, BOTH>(s, taddr + c, c + EPI < s.n ? EPI : 0, bias, v);
+            finish8<ACT, AP, BOTH>(s, taddr + c, c + EPI < s.n ? EPI : 0, bias, false, false, v);
 #pragma unroll
             for (int i = 0; i < 8; i++) {
                 const uint32_t r = c + (i & 3) + (i >> 2) * EPI, row = s.first + r;
@@ -280,7 +294,7 @@ template <int AP, uint32_t EPI> __device__ __forceinline__ void to_owners(const 
     for (uint32_t c = 4 * s.g; c < s.n; c += 2 * EPI) {
         const uint32_t more = c + EPI < s.n ? EPI : 0;
         float v[8];
-        sums8<AP, false>(s, s.tmem + c, more, v);                     // (by whole warps)
+        sums8<AP, false>(s, s.tmem + c, more, false, false, v);                     // (by whole warps)
         if (s.o < s.out) {
 #pragma unroll
             for (int i = 0; i < 8; i++) {

@@ -237,3 +237,33 @@ def test_which_calls_come_here(spg, name, rows, auto_path, tmp_path):
             spg.lib().spgk_chain_arrangement(out)
             assert out[0] >= 1 and out[1] % 16 == 0 and out[1] > 0
     net.free()
+
+
+@pytest.mark.parametrize("t16,a_parts,w_parts", [(0, 1, 1), (1, 1, 1), (0, 2, 1), (1, 2, 1), (1, 2, 2)])
+@pytest.mark.parametrize("act", [0, 1, 2, 3, 4, 6])
+@pytest.mark.parametrize("topology", [[70, 100, 91, 33], [70, 100, 91, 200], [129, 45, 6], [40, 7, 9, 11, 131]], ids=lambda t: "-".join(map(str, t)))
+def test_infinities_stay_in_their_rows_and_columns(spg, lib, topology, act, t16, a_parts, w_parts):
+    """Widths that are no multiple of 16, of positive weights: an infinity is an infinity in every sum, and what an activation makes of it behind.
+    With one term that is the answer; an infinity has no second term (its row is NaN, in every output).  Other rows are as they were."""
+    import torch
+    acts = [act] * (len(topology) - 1)
+    n = Net(spg, lib, topology, acts, t16, a_parts, w_parts, seed=act)
+    for w in n.w16:
+        w.abs_()
+    x, xd = inputs(301, topology[0])
+    bad = np.arange(0, 301, 9)
+    x[bad, 3] = np.inf if t16 else 1e6                         # beyond fp16: an infinity as well
+    xd.copy_(torch.from_numpy(x))
+    y, _ = n.run(xd)
+    good = np.setdiff1d(np.arange(301), bad)
+    want, err = n.want(x[good])
+    assert np.all(np.abs(y[good] - want) <= err)
+    x[bad, 3] = np.inf
+    with np.errstate(all="ignore"):
+        far, _ = n.want(x[bad])
+    if a_parts > 1:
+        assert act == 1 or np.isnan(y[bad]).all()              # (a NaN is not above zero: ReLU makes 0 of it)
+    elif act in (1, 3, 4, 6):
+        assert np.isposinf(far).all() and np.array_equal(y[bad], far.astype(np.float32))
+    else:
+        assert np.isfinite(far).all() and np.abs(y[bad] - far).max() <= 0.02        # (hidden values of exactly 1 or a half, sums of 100 or fewer)
