@@ -324,8 +324,9 @@ SPGK_API int spgk_layer_gemm_tc_head(const spgk_layer *L,
                                      const spgk_layer *head, const float *head_w, float *out32, uint32_t ldo32,
                                      uint32_t N, int32_t *status, void *stream);
 /* A whole net of 2 to SPGK_CHAIN_MAX_LAYERS layers on N rows in one launch (spg_chain.cu), for batches too small to fill the device layer by
- * layer.  spgk_chain_plan decides how (SPGK_E_UNSUPPORTED: not at all) and says how much scratch that takes and what it is estimated
- * to cost; spgk_chain_forward launches it.
+ * layer.  spgk_chain_plan decides how (SPGK_E_UNSUPPORTED: not at all) and says how much scratch that takes (which goes by the net,
+ * the terms and N alone, whatever the guess of a count, and is never less for more rows) and what it is estimated to cost;
+ * spgk_chain_forward launches it.
  *   w16/ldw/w_plane/w_parts: every layer's 16-bit weight operand as for spgk_layer_gemm_tc; a_parts: terms of an activation (type16);
  *   x: fp32 rows, row r of the batch at x_rows[r] where x_rows is given; y: fp32 rows (spgk_set_output_rows);
  *   softmax_fused: the last layer's softmax is applied here (at most 128 columns), else a softmax layer leaves logits;

@@ -916,7 +916,13 @@ int spgk_chain_plan(const spgk_layer *layers, uint32_t count, uint32_t N, int w_
     uint32_t kb = 0;
     for (uint32_t l = 1; l < count; l++) if (ceil_div(layers[l].in, TK) > kb) kb = ceil_div(layers[l].in, TK);
     plan->exchange_bytes = plan->R * 128 * (uint32_t)a_parts * kb;
-    plan->scratch_bytes = (uint64_t)plan->clusters * 2 * plan->exchange_bytes;
+    // What clusters * R rows take, whichever of the plans for so many rows or fewer it is: a call of another guess or of fewer rows never wants a larger
+    // scratch, which would free the one that a captured call refers to.  (R rows of a block at most, and as many blocks as there are or as are at work.)
+    const uint32_t most = 256 / a < MAX_R ? 256 / a : MAX_R;
+    uint64_t held = 0;
+    for (uint32_t C = 1; C <= MAX_C; C++) if ((!counted || C == COUNTED_C) && (uint64_t)at.n[C] * most > held) held = (uint64_t)at.n[C] * most;
+    const uint64_t in_blocks = (uint64_t)N + most;
+    plan->scratch_bytes = (in_blocks < held ? in_blocks : held) * 2 * 128 * a * kb;
     return SPGK_OK;
 }
 

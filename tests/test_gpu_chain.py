@@ -267,3 +267,32 @@ def test_infinities_stay_in_their_rows_and_columns(spg, lib, topology, act, t16,
         assert np.isposinf(far).all() and np.array_equal(y[bad], far.astype(np.float32))
     else:
         assert np.isfinite(far).all() and np.abs(y[bad] - far).max() <= 0.02        # (hidden values of exactly 1 or a half, sums of 100 or fewer)
+
+
+@pytest.mark.parametrize("a_parts", [1, 2])
+@pytest.mark.parametrize("topology", [[784, 512, 1000, 10], [301, 777, 333, 129, 37], [64, 80, 200], [512, 1500, 1500, 64]])
+def test_scratch_goes_by_the_rows_alone(spg, lib, topology, a_parts):
+    """Whatever the guess of a count, and never less for more rows: a workspace that has served a call serves every later one of as many rows or fewer."""
+    import torch
+    n = Net(spg, lib, topology, [1] * (len(topology) - 1), 1, a_parts, 1)
+    plan, c = Plan(), torch.zeros(1, dtype=torch.int32, device="cuda")
+
+    def scratch(rows):
+        if lib.spgk_chain_plan(n.layers, len(n.layers), rows, 1, a_parts, 0, C.byref(plan)) != 0:
+            return None                                        # (more rows than this net's blocks hold)
+        assert plan.scratch_bytes >= 2 * plan.clusters * plan.exchange_bytes
+        return plan.scratch_bytes
+
+    sizes = [size for size in (scratch(rows) for rows in [*range(1, 5000, 37), *range(5000, 66000, 611)]) if size]
+    assert len(sizes) > 100 and sizes == sorted(sizes)
+    try:
+        last = 0
+        for rows in (600, 1024, 1500, 8192, 65536):
+            met = set()
+            for guess in (0, 1, 20, 333, 950, 3000, 10000, rows):
+                lib.spgk_set_dynamic_rows(c.data_ptr(), guess)
+                met.add(scratch(rows))
+            assert len(met) == 1 and max(met) >= last, (rows, met)
+            last = max(met)
+    finally:
+        lib.spgk_set_dynamic_rows(None, 0)

@@ -73,3 +73,33 @@ def test_replays_between_direct_calls(spg, topo, acts):
         assert count == expected_other and torch.equal(got, want_other)
     del graph
     net.free()
+
+
+@pytest.mark.parametrize("topo,acts", NETS)
+def test_replays_after_calls_that_list_more_rows(spg, topo, acts):
+    """A call is captured when few rows are listed; direct ones of as many rows then list all of them.  What the graph refers to is still there."""
+    import torch
+    net = build(spg, topo, acts)
+    stream = torch.cuda.Stream()
+    net.set_stream(stream.cuda_stream)
+    x, ties = torch.randn(3000, 64, device="cuda") * 40, torch.zeros(3000, 64, device="cuda")
+    y, z = torch.empty(3000, 10, device="cuda"), torch.empty(3000, 10, device="cuda")
+    torch.cuda.synchronize()
+    for _ in range(2):                                         # (the second goes by the first one's count)
+        want, few = call(spg, net, x, y)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        net.forward_batch_ptr(x.data_ptr(), 3000, y.data_ptr())
+    for _ in range(3):
+        _, many = call(spg, net, ties, z)
+        assert few < 600 and many == 3000, (few, many)
+        keep = [torch.randn(1 << 18, device="cuda") for _ in range(8)]      # (what would lie in memory that was given back)
+        y.zero_()
+        torch.cuda.synchronize()
+        with torch.cuda.stream(stream):
+            graph.replay()
+        net.synchronize()
+        assert torch.equal(y, want)
+        del keep
+    del graph
+    net.free()
