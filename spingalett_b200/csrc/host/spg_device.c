@@ -455,6 +455,14 @@ static bool few_weights(const spg_net *n, uint32_t N)
     return count <= (layers > 1 && (N == 2 || N == 3 || N == 8) ? 12 : 3) * mi * layers;
 }
 
+/* Outputs in the place of inputs (rows of in and out floats).  A launch that reads rows of the input while it writes outputs of others is not for
+ * such a call; kernels that make an operand of the whole input first, and chains of launches, take it. */
+static bool overlapping(const float *x, uint32_t in, const float *y, uint32_t out, uint32_t N)
+{
+    const uintptr_t x0 = (uintptr_t)x, y0 = (uintptr_t)y;
+    return x && y && x0 < y0 + (size_t)N * out * sizeof(float) && y0 < x0 + (size_t)N * in * sizeof(float);
+}
+
 /* Small / medium batches (fp32 activations between layers; every layer streams its packed weights once).
  * Nets of few weights on up to 8 rows: spg_rows.cu.  Otherwise per layer, in order of preference: the weight-streaming
  * tcgen05 kernel, the mma.sync GEMV (<= 8 rows), the general SIMT kernel.  d_x == NULL means the caller already placed the input rows in slot 0 of the
@@ -462,7 +470,7 @@ static bool few_weights(const spg_net *n, uint32_t N)
 int spg_dev_forward_small(spg_net *n, const float *d_x, uint32_t ldx, uint32_t N, float **d_last, float *d_final)
 {
     NeuralNetwork *p = &n->pub;
-    const bool rows = N <= SPGK_ROWS_MAX_BATCH && few_weights(n, N);
+    const bool rows = N <= SPGK_ROWS_MAX_BATCH && few_weights(n, N) && !(n->dev_layers == 1 && overlapping(d_x, ldx, d_final, n->klayers[0].out, N));
     int rc = rows ? activations_reserve(n, N) : small_reserve(n, N);
     if (rc) return rc;
     if (!d_last) return SPINGALETT_OK;          /* reservation only */
@@ -763,16 +771,16 @@ static int chain_type(spg_net *n, bool exact)
 }
 
 /* The whole net in one launch: whether it takes this net and as many rows sooner than the layers one by one would, and how.  (Weights that
- * are not kept as 16-bit operands, and softmax rows that do not end in it, stay with those.) */
+ * are not kept as 16-bit operands, softmax rows that do not end in it, and outputs in the place of inputs stay with those.) */
 #define SPG_CHAIN_SOFTMAX 128u
-static int whole_plan(spg_net *n, uint32_t N, bool exact, spgk_chain *plan, bool *takes)
+static int whole_plan(spg_net *n, const float *d_x, uint32_t N, const float *d_out, bool exact, spgk_chain *plan, bool *takes)
 {
     *takes = false;
     *plan = (spgk_chain){ 0 };
     const uint32_t layers = n->dev_layers;
     const spgk_layer *last = &n->klayers[layers - 1];
     const bool softmax = last->act == ACT_SOFTMAX;
-    if (layers > SPGK_CHAIN_MAX_LAYERS || (softmax && last->out > SPG_CHAIN_SOFTMAX)) return SPINGALETT_OK;
+    if (layers > SPGK_CHAIN_MAX_LAYERS || (softmax && last->out > SPG_CHAIN_SOFTMAX) || overlapping(d_x, n->klayers[0].in, d_out, last->out, N)) return SPINGALETT_OK;
     for (uint32_t l = 0; l + 1 < layers; l++) if (n->klayers[l].act == ACT_SOFTMAX) return SPINGALETT_OK;
     if (!weights_keepable(n, chain_type(n, exact), exact)) return SPINGALETT_OK;
     const int rc = spgk_chain_plan(n->klayers, layers, N, exact && last->precision == PRECISION_FLOAT32 ? 2 : 1, exact ? 2 : 1, softmax, plan);
@@ -819,7 +827,7 @@ static int large_chain(spg_net *n, const float *d_x, uint32_t N, float *d_out, b
 
     spgk_chain whole;
     bool takes;
-    int rc = whole_plan(n, N, exact, &whole, &takes);
+    int rc = whole_plan(n, d_x, N, d_out, exact, &whole, &takes);
     if (rc) return rc;
     if (takes) return whole_net(n, &whole, d_x, N, d_out, exact);
     const int type = chain_type(n, exact), parts = exact ? 2 : 1;
@@ -987,7 +995,7 @@ int spg_dev_forward_large(spg_net *n, const float *d_x, uint32_t N, float *d_out
     const float fused_us = fused ? spgk_mlp3_us(&n->klayers[0], &n->klayers[1], N) : 0.0f;
     if (fused && mode != SPINGALETT_MATH_EXACT) {
         /* some thousand rows are too few pairs of tiles for it: 2000 rows of the benchmark MLP 31 us there, 18 as a chain of one launch */
-        if ((rc = whole_plan(n, N, false, &whole, &takes))) return rc;
+        if ((rc = whole_plan(n, d_x, N, d_out, false, &whole, &takes))) return rc;
         if (takes && whole.us < fused_us) fused = false;
     }
     if (mode == SPINGALETT_MATH_FAST && fused) return fused_pass(n, d_x, N, d_out, false, NULL, NULL, 0, 0.0f, NULL, NULL);

@@ -296,3 +296,23 @@ def test_scratch_goes_by_the_rows_alone(spg, lib, topology, a_parts):
             last = max(met)
     finally:
         lib.spgk_set_dynamic_rows(None, 0)
+
+
+@pytest.mark.parametrize("topology,rows", [([64, 128, 16], 20000), ([64, 128, 64], 3000), ([4096, 4096], 2)])
+def test_outputs_in_the_place_of_inputs(spg, topology, rows):
+    import torch
+    a = spg.abi
+    net = spg.Network.build(topology, [a.ACT_RELU] * (len(topology) - 2) + [a.ACT_SIGMOID], a.WEIGHT_INITIALIZATION_NONE)
+    net.weights[:] = np.random.default_rng(1).standard_normal(net.weights.size, dtype=np.float32) / 8
+    x = torch.randn(rows, topology[0], device="cuda")
+    y, both = torch.empty(rows, topology[-1], device="cuda"), x.clone()
+    spg.set_math_mode(a.MATH_EXACT)
+    try:
+        net.forward_batch_ptr(x.data_ptr(), rows, y.data_ptr())
+        net.forward_batch_ptr(both.data_ptr(), rows, both.data_ptr())
+        net.synchronize()
+    finally:
+        spg.set_math_mode(a.MATH_AUTO)
+    got = both.reshape(-1)[:y.numel()].reshape(y.shape)
+    assert float((got - y).abs().max()) <= 2e-4                # (logits of some units, two 16-bit terms of either operand)
+    net.free()

@@ -107,6 +107,11 @@ def test_streamed_layers_write_operands_that_have_room(tmp_path):
     assert r.returncode == 0 and r.stdout == "every operand fits\n", (r.returncode, r.stdout, r.stderr)
 
 
+def test_outputs_where_the_inputs_lie(tmp_path):
+    r = subprocess.run([on_fake_kernels(tmp_path, "in_place")], capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0 and r.stdout == "every call on its kernel\n", (r.returncode, r.stdout, r.stderr)
+
+
 def test_a_net_of_very_many_layers(tmp_path):
     r = subprocess.run([on_fake_kernels(tmp_path, "deep_net")], capture_output=True, text=True, timeout=120)
     assert r.returncode == 0 and r.stdout == "every layer\n", (r.returncode, r.stdout, r.stderr)
