@@ -88,13 +88,11 @@ KERNEL_OF_PATH = {"rows": "spg_rows_kernel", "gemv": "spg_gemv_kernel", "istream
                   "tcgen05-fused": "spg_mlp3_fused_kernel", "simt": "spg_layer_simt_kernel"}
 
 
-def kernels(path, topo, batch):
-    """The path's kernel, and with it the one on pairs of CTAs where layers have more 128 x 256 tiles than the GPU has SMs.  Nets of up to some
-    thousand rows whose layers a cluster can share out run in one launch where an estimate says so."""
-    name = KERNEL_OF_PATH.get(path, path)
-    if path.startswith("tcgen05") and batch <= 8192 and max(topo[1:]) <= 4096:
-        return "spg_chain_kernel or " + name
-    pairs = path == "tcgen05" and any(-(-batch // 128) * -(-b // 256) > 148 and a >= 512 and b > 128 for a, b in zip(topo, topo[1:]))
+def kernels(path, kernel, topo, batch):
+    """The kernel that ran (of those that serve a path, the one that spingalett_last_kernel names), and with the one of the layers the one on pairs of
+    CTAs where layers have more 128 x 256 tiles than the GPU has SMs."""
+    name = KERNEL_OF_PATH.get(kernel, kernel)
+    pairs = path == "tcgen05" and name == "spg_gemm_tc_kernel" and any(-(-batch // 128) * -(-b // 256) > 148 and a >= 512 and b > 128 for a, b in zip(topo, topo[1:]))
     return "spg_gemm_pair_kernel, " + name if pairs else name
 
 
@@ -557,11 +555,11 @@ def main():
         net = spg.Network.load(path)
         net.set_stream(torch.cuda.current_stream().cuda_stream)
         res = measure(spg, net, torch, x_dev, y_dev, x_pin, y_pin, batch, steps, warmup, dist, local_rank)
-        path_taken = spg.last_path()
+        taken = spg.last_path(), spg.last_kernel()
         net.free()
-        return path, res, path_taken
+        return path, res, taken
 
-    path, (dev_ms, e2e_ms, k_ms, k_cnt, launches, clocks), path_taken = run_dtype(args.dtype, args.steps, args.warmup)
+    path, (dev_ms, e2e_ms, k_ms, k_cnt, launches, clocks), (path_taken, kernel_taken) = run_dtype(args.dtype, args.steps, args.warmup)
     value = batch * world / (dev_ms * 1e-3)
     e2e_value = batch * world / (e2e_ms * 1e-3)
     passes = 2 if args.math == "exact" else 1
@@ -582,17 +580,17 @@ def main():
         "clocks": clocks,
     }
     if k_cnt and path_taken.startswith("tcgen05"):
-        fused = path_taken == "tcgen05-fused"
+        fused, whole = kernel_taken == "spg_mlp3_fused_kernel", kernel_taken == "spg_chain_kernel"
         flops = flops_per_sample(topo) * batch * args.steps      # algorithmic: 2*N*sum(in*out), one term per product
         k_ms_eff = min(k_ms, dev_ms * args.steps)                # event pairs around single launches cannot undercut the timed loop
         achieved = flops / (k_ms_eff * 1e-3) / 1e12
         traffic = None
         tpath = os.path.join(ROOT, "profiles", "mlp3_fused_traffic.json" if fused else "gemm_tc_traffic.json")
-        if os.path.exists(tpath):
+        if not whole and os.path.exists(tpath):
             traffic = json.load(open(tpath)).get(f"{args.workload}_{args.dtype}_{args.math}_{batch}")
         line["roofline"] = {"bound": "tensor", "achieved": achieved, "peak": pk["bf16_tflops"], "unit": "TFLOP/s",
                             "frac": achieved / pk["bf16_tflops"], "traffic": traffic,
-                            "kernel": kernels(path_taken, args.topo, batch),
+                            "kernel": kernels(path_taken, kernel_taken, args.topo, batch),
                             "launches": int(k_cnt), "kernel_ms_per_step": k_ms_eff / args.steps,
                             "peak_source": pk["source"] + " burst bf16", "tensor_passes_per_product": passes,
                             "executed_frac": achieved * passes / pk["bf16_tflops"],
@@ -600,7 +598,7 @@ def main():
                             "note": ("frac: the one launch per step that computes all three layers of all rows (event pair around it); "
                                      "whole_step_frac: the same FLOPs over ms_per_step, which in AUTO also holds the exact "
                                      "recomputation of the low-margin rows (one launch of spg_chain_kernel on a percent or two of the rows)")
-                                    if fused else "frac: summed device time of the layer kernels (event pairs); whole_step_frac: over ms_per_step"}
+                                    if fused or whole else "frac: summed device time of the layer kernels (event pairs); whole_step_frac: over ms_per_step"}
     elif k_cnt:
         nbytes = algorithmic_bytes(topo, args.dtype, batch)      # per step, all layers (one kernel launch per layer)
         achieved = nbytes * args.steps / (k_ms * 1e-3) / 1e9
@@ -610,7 +608,7 @@ def main():
             traffic = json.load(open(tpath)).get(f"{args.workload}_{args.dtype}_{batch}")
         line["roofline"] = {"bound": "hbm", "achieved": achieved, "peak": pk["hbm_gbs"], "unit": "GB/s",
                             "frac": achieved / pk["hbm_gbs"], "traffic": traffic,
-                            "kernel": kernels(path_taken, args.topo, batch),
+                            "kernel": kernels(path_taken, kernel_taken, args.topo, batch),
                             "launches": int(k_cnt), "kernel_ms_per_step": k_ms / args.steps,
                             "algorithmic_bytes_per_step": nbytes, "peak_source": pk["source"] + " copy bandwidth",
                             "whole_step_frac": nbytes / (dev_ms * 1e-3) / 1e9 / pk["hbm_gbs"],

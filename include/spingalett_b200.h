@@ -408,9 +408,12 @@ SPINGALETT_API void spingalett_profile_read(NeuralNetwork *net, double *kernel_m
  * name of the compute path the last batched/forward call took ("gemv",
  * "rows" -- nets of few weights on up to eight rows --,
  * "istream" -- integer files through the 8-bit integer tensor path --, "wstream",
- * "tcgen05", "tcgen05-fused" -- the one-term pass of a three-layer net in one launch --, "simt").  For benchmarks and tests. */
+ * "tcgen05", "tcgen05-fused" -- the one-term pass of a three-layer net in one launch --, "simt").  Where several kernels serve a
+ * path, spingalett_last_kernel says which one ran the batch ("tcgen05" and "tcgen05-fused": "spg_chain_kernel" -- a whole net by
+ * clusters --, "spg_mlp3_fused_kernel", "spg_gemm_tc_kernel" -- layer by layer --); elsewhere it is the path's name.  For benchmarks and tests. */
 SPINGALETT_API uint64_t spingalett_kernel_launches(void);
 SPINGALETT_API const char *spingalett_last_path(void);
+SPINGALETT_API const char *spingalett_last_kernel(void);
 
 #ifdef __cplusplus
 }

@@ -232,5 +232,9 @@ def last_path():
     return lib().spingalett_last_path().decode()
 
 
+def last_kernel():
+    return lib().spingalett_last_kernel().decode()
+
+
 def kernel_launches():
     return int(lib().spingalett_kernel_launches())

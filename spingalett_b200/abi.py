@@ -137,7 +137,7 @@ def bind_reference_abi(lib):
 EXTENSION_SYMBOLS = [
     "forward_batch_struct_arguments", "spingalett_set_math_mode", "spingalett_get_math_mode",
     "spingalett_set_device", "spingalett_get_device_count", "spingalett_set_stream", "spingalett_sync_weights",
-    "spingalett_seed", "spingalett_kernel_launches", "spingalett_last_path",
+    "spingalett_seed", "spingalett_kernel_launches", "spingalett_last_path", "spingalett_last_kernel",
     "spingalett_profile", "spingalett_profile_read", "spingalett_synchronize",
     "spingalett_set_auto_margin", "spingalett_get_auto_margin", "spingalett_last_repaired", "spingalett_net_margin",
     "spingalett_dist_unique_id", "spingalett_dist_init", "spingalett_dist_shutdown", "spingalett_dist_world",
@@ -166,6 +166,7 @@ def bind_extensions(lib):
     lib.spingalett_seed.restype = None
     lib.spingalett_kernel_launches.restype = C.c_uint64
     lib.spingalett_last_path.restype = C.c_char_p
+    lib.spingalett_last_kernel.restype = C.c_char_p
     lib.spingalett_set_auto_margin.argtypes = [C.c_float]
     lib.spingalett_set_auto_margin.restype = None
     lib.spingalett_get_auto_margin.restype = C.c_float

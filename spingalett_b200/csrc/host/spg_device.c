@@ -813,7 +813,7 @@ static int whole_net(spg_net *n, const spgk_chain *plan, const float *d_x, uint3
     if (!dynamic_rows) prof_mark(n);
     if (rc) return rc;
     n->status_pending = true;
-    spg_note_path("tcgen05");
+    spg_note_kernel("tcgen05", "spg_chain_kernel");
     return SPINGALETT_OK;
 }
 
@@ -908,7 +908,7 @@ static int large_chain(spg_net *n, const float *d_x, uint32_t N, float *d_out, b
             (rc = spg_map_kernel_error(spgk_softmax_rows(d_out, L->out, N, L->out, n->stream), "softmax"))) return rc;
     }
     n->status_pending = true;
-    spg_note_path("tcgen05");
+    spg_note_kernel("tcgen05", "spg_gemm_tc_kernel");
     return SPINGALETT_OK;
 }
 
@@ -974,7 +974,7 @@ static int fused_pass(spg_net *n, const float *d_x, uint32_t N, float *d_out, bo
     if (rc) return rc;
     n->status_pending = true;
     n->fused_ran = true;
-    spg_note_path("tcgen05-fused");
+    spg_note_kernel("tcgen05-fused", "spg_mlp3_fused_kernel");
     return SPINGALETT_OK;
 }
 
@@ -1001,7 +1001,7 @@ int spg_dev_forward_large(spg_net *n, const float *d_x, uint32_t N, float *d_out
     if (mode == SPINGALETT_MATH_FAST && fused) return fused_pass(n, d_x, N, d_out, false, NULL, NULL, 0, 0.0f, NULL, NULL);
     if (mode != SPINGALETT_MATH_AUTO) {
         rc = large_chain(n, d_x, N, d_out, mode == SPINGALETT_MATH_EXACT);
-        if (!rc && mode == SPINGALETT_MATH_FAST && whole.clusters) spg_note_path(one_launch);
+        if (!rc && mode == SPINGALETT_MATH_FAST && whole.clusters) spg_note_kernel(one_launch, spingalett_last_kernel());
         return rc;
     }
     if (!softmax_out) return large_chain(n, d_x, N, d_out, true);
@@ -1034,6 +1034,7 @@ int spg_dev_forward_large(spg_net *n, const float *d_x, uint32_t N, float *d_out
     }
     if (rc) return rc;
     if (strncmp(spingalett_last_path(), "tcgen05", 7) != 0) return SPINGALETT_OK;  /* the fp32 chain ran: nothing to repair */
+    const char *const pass_kernel = spingalett_last_kernel();
     theta = spingalett_get_auto_margin();
     if (theta <= 0.0f) {
         /* Self-calibration, once per device image of the net: run both modes on up to 2048 rows, measure the
@@ -1111,7 +1112,7 @@ int spg_dev_forward_large(spg_net *n, const float *d_x, uint32_t N, float *d_out
     if (rc) return rc;
     if ((rc = spg_map_kernel_error(spgk_count_take(d_count, h_slot, n->stream), "repair count"))) return rc;
     n->count_pending = true; n->count_seen = true; n->count_clean = captured ? clean_before : true;
-    spg_note_path(one_launch);
+    spg_note_kernel(one_launch, pass_kernel);
     return SPINGALETT_OK;
 }
 

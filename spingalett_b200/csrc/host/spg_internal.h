@@ -108,6 +108,7 @@ SPG_HIDDEN const char *spg_act_name(unsigned a);
 SPG_HIDDEN const char *spg_precision_name(unsigned p);
 SPG_HIDDEN const char *spg_loss_name(unsigned l);
 SPG_HIDDEN void spg_note_path(const char *name);
+SPG_HIDDEN void spg_note_kernel(const char *path, const char *kernel);
 /* rng.c */
 SPG_HIDDEN float spg_rand_uniform_pm1(void);
 SPG_HIDDEN float spg_rand_normal(void);

@@ -16,7 +16,7 @@ static _Atomic bool     s_verbose = true;
 static _Atomic int      s_math = SPINGALETT_MATH_AUTO;
 static _Atomic float    s_margin = 0.0f;                /* 0 = calibrate per net */
 static _Atomic bool     s_mode_note_done = false;
-static _Thread_local const char *t_path = "none";
+static _Thread_local const char *t_path = "none", *t_kernel = "none";
 
 ComputeMode spingalett_get_compute_mode(void) { return (ComputeMode)atomic_load(&s_mode); }
 
@@ -43,8 +43,10 @@ SpingalettMathMode spingalett_get_math_mode(void) { return (SpingalettMathMode)a
 void spingalett_set_auto_margin(float log_gap) { atomic_store(&s_margin, log_gap > 0.0f ? log_gap : 0.0f); }
 float spingalett_get_auto_margin(void) { return atomic_load(&s_margin); }
 
-void spg_note_path(const char *name) { t_path = name; }
+void spg_note_kernel(const char *path, const char *kernel) { t_path = path; t_kernel = kernel; }
+void spg_note_path(const char *name) { spg_note_kernel(name, name); }
 const char *spingalett_last_path(void) { return t_path; }
+const char *spingalett_last_kernel(void) { return t_kernel; }
 uint64_t spingalett_kernel_launches(void) { return spgk_launch_count(); }
 
 void spg_log(LogLevel level, const char *fmt, ...)

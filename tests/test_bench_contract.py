@@ -48,6 +48,15 @@ def test_the_line_names_what_the_path_runs():
         assert bench.KERNEL_OF_PATH[path] == kernel and bench.arithmetic(path, "int4", "auto").startswith(dtype)
 
 
+def test_the_line_names_the_kernel_that_ran():
+    import bench
+    assert bench.kernels("tcgen05-fused", "spg_chain_kernel", bench.TOPO, 2048) == "spg_chain_kernel"
+    assert bench.kernels("tcgen05-fused", "spg_mlp3_fused_kernel", bench.TOPO, 65536) == "spg_mlp3_fused_kernel"
+    assert bench.kernels("tcgen05", "spg_gemm_tc_kernel", [784, 512, 10], 2048) == "spg_gemm_tc_kernel"
+    assert bench.kernels("tcgen05", "spg_gemm_tc_kernel", [4096, 4096, 4096], 16384) == "spg_gemm_pair_kernel, spg_gemm_tc_kernel"
+    assert bench.kernels("istream", "istream", [8192, 1000], 64) == "spg_istream_kernel"
+
+
 def test_defaults_follow_the_workload():
     sys.path.insert(0, ROOT)
     import bench
