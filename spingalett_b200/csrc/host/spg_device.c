@@ -801,7 +801,7 @@ static int whole_net(spg_net *n, const spgk_chain *plan, const float *d_x, uint3
     uint64_t w_plane[SPGK_CHAIN_MAX_LAYERS];
     bool ready = true;                          /* no operand is made in front of this launch */
     for (uint32_t l = 0; l < layers; l++) {
-        const bool there = spgk_weights16_direct(&n->klayers[l], type) || (n->d_w16c[type] && n->d_w16c[type][l]);
+        const bool there = spgk_weights16_direct(&n->klayers[l], type) || (n->d_w16c[type] && n->d_w16c[type][l] && n->w16c_parts[type][l] == w_parts);
         if ((rc = kept_weight_operand(n, type, l, w_parts, true, &w16[l], &ldw[l], &w_plane[l]))) return rc;
         ready = ready && there;
     }

@@ -112,6 +112,11 @@ def test_outputs_where_the_inputs_lie(tmp_path):
     assert r.returncode == 0 and r.stdout == "every call on its kernel\n", (r.returncode, r.stdout, r.stderr)
 
 
+def test_weights_are_read_early_only_when_they_are_there(tmp_path):
+    r = subprocess.run([on_fake_kernels(tmp_path, "ready_weights")], capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0 and r.stdout == "only when they are there\n", (r.returncode, r.stdout, r.stderr)
+
+
 def test_a_net_of_very_many_layers(tmp_path):
     r = subprocess.run([on_fake_kernels(tmp_path, "deep_net")], capture_output=True, text=True, timeout=120)
     assert r.returncode == 0 and r.stdout == "every layer\n", (r.returncode, r.stdout, r.stderr)
