@@ -245,7 +245,10 @@ SPINGALETT_API float derivative(float x, ActivationFunction act_func);
  * topology[0] floats in host memory.  Returns a pointer into net->neurons
  * (the last layer's slice), valid until the next call on this net.  NULL net
  * or input returns NULL without touching the error state; fewer than two
- * layers is ERR_INVALID (reference Network.c:207-212). */
+ * layers is ERR_INVALID (reference Network.c:207-212).  The answer of a small
+ * net is taken as it arrives: everything issued on the net's stream before has
+ * run then, and the call itself writes no device memory any more, but the
+ * stream may not be idle yet. */
 SPINGALETT_API float *forward_struct_arguments(ForwardArgs args);
 
 /* :230 -- training.  Supported on the GPU: MODE_ARRAY with

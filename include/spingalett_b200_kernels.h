@@ -106,7 +106,8 @@ SPGK_API int spgk_layer_simt(const spgk_layer *L, const float *x, uint32_t ldx,
 SPGK_API int spgk_rows_forward(const spgk_layer *layers, uint32_t count, const float *x, uint32_t ldx, float *const *ys, uint32_t N,
                                void *stream);
 /* One sample the same way, from and to page-locked host memory: host and dev hold the input and then every layer's outputs, one behind the
- * other; the input is read from host, the outputs are written to dev and to host (there once the stream has been waited for).
+ * other; the input is read from host, the outputs are written to host, those of all layers but the last to dev as well.  When every output is there
+ * nothing in device memory is written any more.
  * SPGK_E_UNSUPPORTED, and nothing launched, for a softmax that needs a launch of its own (more than 128 outputs, or too many products for a CTA). */
 #define SPGK_ROWS_MAX_LAYERS 64u
 SPGK_API int spgk_rows_sample(const spgk_layer *layers, uint32_t count, float *host, float *dev, void *stream);

@@ -294,6 +294,9 @@ extern "C" int spgk_rows_sample(const spgk_layer *layers, uint32_t count, float 
         ys[l] = dev + at; copies[l] = host + at;
         at += layers[l].out;
     }
+    // The last outputs go to the host alone: a caller that has seen every output may go on before the stream is idle, and nothing in device memory is
+    // written any more then (the layers before have been read by the one behind them).
+    ys[count - 1] = copies[count - 1]; copies[count - 1] = nullptr;
     SPGK_CUDA(spg_launch_chained(spg_rows_fetch_kernel, dim3((layers[0].in + 255) / 256), dim3(256), 0, (cudaStream_t)stream, host, dev, layers[0].in));
     const int rc = spgk_check_launch("spg_rows_fetch_kernel");
     return rc ? rc : rows_chain(layers, count, dev, layers[0].in, ys, copies, 1, stream);

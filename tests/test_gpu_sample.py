@@ -84,3 +84,29 @@ def test_many_nets_side_by_side(spg, has_gpu):
     for t in threads:
         t.join()
     assert not failed
+
+
+@pytest.mark.parametrize("topology,acts", [([784, 512, 1000, 10], [1, 1, 5]), ([33, 100, 7], [1, 2]), ([4096, 24], [0])])
+def test_last_outputs_go_to_the_host_alone(spg, has_gpu, topology, acts):
+    """Whoever has seen every output may go on before the stream is idle: no store to device memory may be under way then."""
+    import torch
+    lib = spg.lib()
+    lib.spgk_rows_sample.argtypes = [C.c_void_p, C.c_uint32, C.c_void_p, C.c_void_p, C.c_void_p]
+    pairs = list(zip(topology, topology[1:]))
+    gen = torch.Generator().manual_seed(1)
+    w = [(torch.randn(b, a, generator=gen) / a ** 0.5).cuda() for a, b in pairs]
+    bias = [torch.randn(b, generator=gen).cuda() for _, b in pairs]
+    layers = (spg.abi.KLayer * len(pairs))(*[spg.abi.KLayer(m.data_ptr(), v.data_ptr(), 1.0, a, b, 0, act) for (a, b), m, v, act in zip(pairs, w, bias, acts)])
+    host = torch.full((sum(topology),), -7.0).pin_memory()
+    host[:topology[0]] = torch.randn(topology[0], generator=gen)
+    dev = torch.full((sum(topology),), -7.0, device="cuda")
+    torch.cuda.synchronize()
+    assert lib.spgk_rows_sample(layers, len(pairs), host.data_ptr(), dev.data_ptr(), None) == 0
+    torch.cuda.synchronize()
+    last = topology[-1]
+    assert torch.equal(dev[:-last].cpu(), host[:-last]) and bool((dev[-last:] == -7.0).all())
+    a = host[:topology[0]].double()
+    for m, v, act in zip(w, bias, acts):
+        z = m.double().cpu() @ a + v.double().cpu()
+        a = {0: torch.sigmoid, 1: torch.relu, 2: torch.tanh, 5: lambda t: torch.softmax(t, 0)}[act](z)
+    assert float((host[-last:].double() - a).abs().max()) <= 2e-5
