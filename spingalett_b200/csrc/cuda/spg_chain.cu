@@ -69,7 +69,8 @@ struct ChainParams {
     uint8_t *scratch; uint32_t exchange_bytes;
     uint32_t rows; const uint32_t *limit;
     int impatient;
-    int early;                        // the weights and the number of rows are known before the kernel before this one has ended
+    int ready;                        // no kernel before this one makes the weights
+    int early;                        // ... and the number of rows is known before it has ended
     int32_t *status;
 };
 
@@ -458,6 +459,7 @@ spg_chain_kernel(const __grid_constant__ ChainParams p)
     cluster_sync();                                            // every barrier of the cluster is set up
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
+    if (!p.ready) spg_grid_wait();                             // the launch behind this one may read weights that are still being made, before its own wait
     spg_grid_trigger();
     const uint32_t last = p.layers - 1;
     // what this CTA does of layer l: tiles (0: nothing) from output o0 on; of a last layer cut along K all outputs
@@ -960,6 +962,7 @@ int spgk_chain_forward(const spgk_chain *plan, const spgk_layer *layers, uint32_
     if (softmax_fused && spg_tls_margin_idx) { p.margin_theta = spg_tls_margin_theta; p.margin_idx = spg_tls_margin_idx; p.margin_count = spg_tls_margin_count; }
     p.scratch = (uint8_t *)scratch; p.exchange_bytes = plan->exchange_bytes;
     p.rows = N; p.limit = spg_tls_rows_limit;
+    p.ready = weights_ready;
     p.early = weights_ready && !p.limit;
     p.impatient = spg_gemm_impatient() ? 1 : 0;
     p.status = status;
