@@ -845,6 +845,10 @@ bool lay_out(const spgk_layer *layers, uint32_t count, uint32_t C, uint32_t R, u
     // the tensor core reads 128 rows from wherever a tile begins
     const uint32_t reach = sw * o.w_slot - tr_max * 128 + TM * 128;
     if (reach > o.smem) o.smem = reach;
+    // Tensor memory is waited for without a bound, in front of the cluster's first barrier: two clusters that each held what the other wants would wait
+    // for good.  Two CTAs fit an SM only where both have eight epilogue warps, one term and small rings (three never: 384 threads of 80 registers); with
+    // 256 columns each at most they get them.  A CTA of more columns takes an SM to itself (its rings nearly fill the shared memory as it is).
+    if (o.tmem_cols > 256) o.smem = (uint32_t)smem_max;
     return o.smem <= smem_max;
 }
 
