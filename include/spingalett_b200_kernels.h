@@ -317,6 +317,10 @@ SPGK_API void spgk_gemm_tc_arrangement(uint32_t out[4]);
  * spgk_head_weights (spgk_head_weights_bytes bytes; it depends only on the head's weights and can be kept).
  * Replaces the last two iterations of the layer loop of batch_forward (Training.c:327-343). */
 SPGK_API int spgk_gemm_tc_head_supported(const spgk_layer *L, const spgk_layer *head);
+/* Products of 16 inputs that follow one another in an accumulator of spgk_layer_gemm_tc; of the weight-streaming kernel, which keeps a value's terms
+ * apart (0: not taken).  What a sum loses goes by them: the tensor core cuts off after each. */
+SPGK_API uint32_t spgk_layer_gemm_sum_steps(const spgk_layer *L, uint32_t N, int a_parts, int w_parts, int softmax_fused);
+SPGK_API uint32_t spgk_wstream_sum_steps(const spgk_layer *L, uint32_t N);
 SPGK_API size_t spgk_head_weights_bytes(const spgk_layer *head);
 SPGK_API int spgk_head_weights(const spgk_layer *head, float *dst, void *stream);
 SPGK_API int spgk_layer_gemm_tc_head(const spgk_layer *L,
@@ -332,7 +336,11 @@ SPGK_API int spgk_layer_gemm_tc_head(const spgk_layer *L,
  *   x: fp32 rows, row r of the batch at x_rows[r] where x_rows is given; y: fp32 rows (spgk_set_output_rows);
  *   softmax_fused: the last layer's softmax is applied here (at most 128 columns), else a softmax layer leaves logits;
  *   weights_ready: no kernel in front of this one in the stream writes w16 or a bias (they are read under its tail).
- * Honours spgk_set_dynamic_rows and spgk_set_margin_sink.  A row's result depends on neither N nor the plan. */
+ * Its accumulators add up no more products in a row, all layers together, than spgk_layer_gemm_tc's would; where there is no such arrangement, layered_us
+ * is 0.
+ * Honours spgk_set_dynamic_rows and spgk_set_margin_sink.  The order in which a row's products are added up goes by the number of rows and what
+ * the plan says (the size of a cluster, the accumulators that tensor memory has room for), not by the other rows.  With rows counted on the device it goes by the
+ * net alone: the same bits whatever the count, its guess, and the row's place. */
 #define SPGK_CHAIN_MAX_LAYERS 8
 typedef struct { uint32_t C, R, clusters, exchange_bytes; uint64_t scratch_bytes; float us, layered_us; } spgk_chain;
 SPGK_API int spgk_chain_plan(const spgk_layer *layers, uint32_t count, uint32_t N, int w_parts, int a_parts, int softmax_fused, spgk_chain *plan);

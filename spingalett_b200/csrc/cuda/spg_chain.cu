@@ -12,8 +12,15 @@
 // The input is rounded to its terms on the way into shared memory.  The weight ring runs ahead of the layers, and starts before
 // the kernel in front has ended.
 //
-// A row's sums depend on the size of the cluster where the last layer is cut, and on whether tensor memory has room for two
-// accumulators a tile, but not on the other rows, nor on R otherwise.
+// The tensor core cuts off what of a product does not fit the sum, so what a sum loses goes by how many products follow one another in an
+// accumulator.  A tile has two accumulators where there is room, and up to eight (the stages of K in turn, or one a k-block) where it takes more for all
+// layers together to add no more in a row than the layer kernels do, which cut K over CTAs (`steps_allowed`); a net that does not fit with so many
+// stays with those.  Error against 64 bits, positive values and weights, layer kernels / two accumulators / now: 4096-512-64 in FP16 at
+// 200 rows 3.3e-6 / 11.7e-6 / 2.7e-6, 8192-512-64 in BF16 at 1000 rows 7.2e-6 / 12.7e-6 / 4.5e-6, 784-512-1000-10 in FP16 at 256 rows 2.2e-6 / 3.4e-6 /
+// 1.9e-6; values of either sign half of the layer kernels'.  An accumulator more costs 250 cycles a layer and 32 rows: FP16 at 256 rows 13.7 -> 14.5 us.
+//
+// A row's sums depend on the size of the cluster where the last layer is cut, and on the accumulators of a tile, which go by the number of rows,
+// but not on the other rows, nor on R otherwise.
 //
 // What bounds it: latency.  256 rows of 784-512-1000-10 in INT4, clusters of 8 on 32 rows each, in cycles: first rows of the input
 // 2700, all of them in shared memory 6000, first layer multiplied 9800 (a product of 128 x 64 x 16 takes 65 cycles, 58 of them whatever
@@ -43,6 +50,7 @@ constexpr uint32_t KG = 2;                                     // k-blocks that 
 constexpr uint32_t MAX_LAYERS = SPGK_CHAIN_MAX_LAYERS, MAX_C = 8, MAX_R = 256, MAX_RING = 12;
 constexpr uint32_t threads_of(uint32_t epi) { return 128 + 32 * epi; }
 constexpr uint32_t TAIL_MAX = 128, MAX_MT = 4;                 // outputs of a last layer whose sums are put together
+constexpr uint32_t MAX_ACC = 8;                                // accumulators of a tile
 constexpr uint32_t COUNTED_C = 4;                              // CTAs of a cluster where only the device knows the number of rows
 constexpr uint32_t BAR_BYTES = 8 * (5 * MAX_RING + 6) + 32;
 
@@ -52,7 +60,7 @@ struct ChainLayer {
     int act;
     uint32_t in, out, kblocks, stages;  // stages: of KG k-blocks
     uint32_t tr, mt;                  // rows of a weight tile, tiles of a CTA
-    uint32_t mains;                   // accumulators of a tile (each of 16-bit terms times n columns)
+    uint32_t mains, run;              // accumulators of a tile (each of 16-bit terms times n columns), stages of one of them (0: a k-block)
     uint32_t covered;                 // outputs of all tiles together: the next layer's columns from here on are nobody's
 };
 struct ChainParams {
@@ -169,58 +177,95 @@ template <int ACT, int N> __device__ __forceinline__ void activate(float (&v)[N]
         for (int i = 0; i < N; i++) v[i] = spg_activate(v[i], ACT);
     }
 }
-// A layer's activation is chosen once, outside the loops (a branch inside costs as much as the activation)
-#define SPG_CHAIN_ACTS(act, both, call)                                                        \
+constexpr int MANY = 0;
+// A layer's activation is chosen once, outside the loops (a branch inside costs as much as the activation),
+// and so is the number of accumulators: 1, 2, or MANY
+#define SPG_CHAIN_ACCS(act, accs, call)                                                         \
+    if ((accs) == 1) call(act, 1); else if ((accs) == 2) call(act, 2); else call(act, MANY)
+#define SPG_CHAIN_ACTS(act, accs, call)                                                         \
     switch (act) {                                                                             \
-        case SPG_ACT_RELU:  if (both) call(SPG_ACT_RELU, true); else call(SPG_ACT_RELU, false); break;    \
-        case SPG_ACT_LEAKY: if (both) call(SPG_ACT_LEAKY, true); else call(SPG_ACT_LEAKY, false); break;  \
-        case SPG_ACT_FOO52: if (both) call(SPG_ACT_FOO52, true); else call(SPG_ACT_FOO52, false); break;  \
-        case SPG_ACT_NONE:  if (both) call(SPG_ACT_NONE, true); else call(SPG_ACT_NONE, false); break;    \
-        default:            if (both) call(CURVED, true); else call(CURVED, false); break;                \
+        case SPG_ACT_RELU:  SPG_CHAIN_ACCS(SPG_ACT_RELU, accs, call); break;                     \
+        case SPG_ACT_LEAKY: SPG_CHAIN_ACCS(SPG_ACT_LEAKY, accs, call); break;                    \
+        case SPG_ACT_FOO52: SPG_CHAIN_ACCS(SPG_ACT_FOO52, accs, call); break;                    \
+        case SPG_ACT_NONE:  SPG_CHAIN_ACCS(SPG_ACT_NONE, accs, call); break;                     \
+        default:            SPG_CHAIN_ACCS(CURVED, accs, call); break;                           \
     }
 
 // One output of eight rows: four from a place in sixteen rows on, and the four sixteen further on, or the first four again where the block has
 // no more.  (A warp's instructions hang on one another: eight rows take little longer than four, 560 cycles.)  The accumulators' sums in
 // their order; zeros where the output is a dead one of a warp that has some (edge: masks in every warp cost 3001 rows of 301-777-333-129-37 0.8 us of
 // 31, a branch behind the wait 0.1; zeros stored afterwards 0.7 to 3.5).
-template <int AP, bool BOTH>
+template <int AP, int ACC>
 __device__ __forceinline__ void sums8(const Slice &s, uint32_t taddr, uint32_t more, bool edge, bool dead, float (&v)[8])
 {
-    const uint32_t second = AP * s.n;
-    uint32_t hi[2][4], lo[2][4], hi2[2][4], lo2[2][4];
+    if constexpr (ACC == MANY) {
+        // (two a turn; where their number is odd the last one's place is read again and left out)
+        float low[8];
 #pragma unroll
-    for (int h = 0; h < 2; h++) {
-        const uint32_t at = taddr + (h ? more : 0);
-        tmem_ld4(at, hi[h]);
-        if (AP > 1) tmem_ld4(at + s.n, lo[h]);
-        if (BOTH) tmem_ld4(at + second, hi2[h]);
-        if (BOTH && AP > 1) tmem_ld4(at + second + s.n, lo2[h]);
-    }
-    tmem_ld_wait();
-    if (edge) {
-        const uint32_t keep = dead ? 0u : 0xFFFFFFFFu;
+        for (int i = 0; i < 8; i++) v[i] = low[i] = 0.0f;
+#pragma unroll 1
+        for (uint32_t a = 0; a < s.mains; a += 2) {
+            const bool pair = a + 1 < s.mains;
+            uint32_t hi[2][2][4], lo[2][2][4];
+#pragma unroll
+            for (int b = 0; b < 2; b++)
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                    const uint32_t at = taddr + (a + (b && pair ? 1 : 0)) * AP * s.n + (h ? more : 0);
+                    tmem_ld4(at, hi[b][h]);
+                    if (AP > 1) tmem_ld4(at + s.n, lo[b][h]);
+                }
+            tmem_ld_wait();
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+                const int h = i >> 2, j = i & 3;
+                v[i] += __uint_as_float(hi[0][h][j]) + (pair ? __uint_as_float(hi[1][h][j]) : 0.0f);
+                if (AP > 1) low[i] += __uint_as_float(lo[0][h][j]) + (pair ? __uint_as_float(lo[1][h][j]) : 0.0f);
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+            if (AP > 1) v[i] += low[i];
+            if (edge && dead) v[i] = 0.0f;
+        }
+    } else {
+        constexpr bool BOTH = ACC == 2;
+        const uint32_t second = AP * s.n;
+        uint32_t hi[2][4], lo[2][4], hi2[2][4], lo2[2][4];
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            const uint32_t at = taddr + (h ? more : 0);
+            tmem_ld4(at, hi[h]);
+            if (AP > 1) tmem_ld4(at + s.n, lo[h]);
+            if (BOTH) tmem_ld4(at + second, hi2[h]);
+            if (BOTH && AP > 1) tmem_ld4(at + second + s.n, lo2[h]);
+        }
+        tmem_ld_wait();
+        if (edge) {
+            const uint32_t keep = dead ? 0u : 0xFFFFFFFFu;
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+                const int h = i >> 2, j = i & 3;
+                hi[h][j] &= keep;
+                if (AP > 1) lo[h][j] &= keep;
+                if (BOTH) hi2[h][j] &= keep;
+                if (BOTH && AP > 1) lo2[h][j] &= keep;
+            }
+        }
 #pragma unroll
         for (int i = 0; i < 8; i++) {
             const int h = i >> 2, j = i & 3;
-            hi[h][j] &= keep;
-            if (AP > 1) lo[h][j] &= keep;
-            if (BOTH) hi2[h][j] &= keep;
-            if (BOTH && AP > 1) lo2[h][j] &= keep;
+            v[i] = __uint_as_float(hi[h][j]);
+            if (BOTH) v[i] += __uint_as_float(hi2[h][j]);
+            if (AP > 1) v[i] += BOTH ? __uint_as_float(lo[h][j]) + __uint_as_float(lo2[h][j]) : __uint_as_float(lo[h][j]);
         }
-    }
-#pragma unroll
-    for (int i = 0; i < 8; i++) {
-        const int h = i >> 2, j = i & 3;
-        v[i] = __uint_as_float(hi[h][j]);
-        if (BOTH) v[i] += __uint_as_float(hi2[h][j]);
-        if (AP > 1) v[i] += BOTH ? __uint_as_float(lo[h][j]) + __uint_as_float(lo2[h][j]) : __uint_as_float(lo[h][j]);
     }
 }
 // ... scale, bias, activation
-template <int ACT, int AP, bool BOTH>
+template <int ACT, int AP, int ACC>
 __device__ __forceinline__ void finish8(const Slice &s, uint32_t taddr, uint32_t more, float bias, bool edge, bool dead, float (&v)[8])
 {
-    sums8<AP, BOTH>(s, taddr, more, edge, dead, v);
+    sums8<AP, ACC>(s, taddr, more, edge, dead, v);
 #pragma unroll
     for (int i = 0; i < 8; i++) v[i] = fmaf(v[i], s.scale, bias);
     activate<ACT>(v, s.act);
@@ -229,7 +274,7 @@ __device__ __forceinline__ void finish8(const Slice &s, uint32_t taddr, uint32_t
 // A layer's outputs become the next one's operand: [k-block][plane][row] of 128 bytes.  Lane pairs trade rows so that each writes
 // two neighbouring values at once.  Columns beyond the layer's outputs get the activation of zero, whose weights are zeros.  Their own sums are not taken
 // for it: a row with an infinity times weights of zero is NaN, and so it would be with the next layer's zeros.
-template <int ACT, bool BOTH, typename T16, int AP, uint32_t EPI>
+template <int ACT, int ACC, typename T16, int AP, uint32_t EPI>
 __device__ __forceinline__ void to_operand(const Slice &s, uint8_t *next, uint32_t k0, uint32_t next_k, uint32_t plane)
 {
     const uint32_t odd = s.lane & 1u;
@@ -247,7 +292,7 @@ __device__ __forceinline__ void to_operand(const Slice &s, uint8_t *next, uint32
         for (uint32_t c = 4 * s.g; c < s.n; c += 2 * EPI, taddr += 2 * EPI, dst += 2 * EPI * 128) {
             const bool two = c + EPI < s.n;
             float v[8];
-            finish8<ACT, AP, BOTH>(s, taddr, two ? EPI : 0, bias, edge, dead, v);
+            finish8<ACT, AP, ACC>(s, taddr, two ? EPI : 0, bias, edge, dead, v);
 #pragma unroll
             for (int i = 0; i < 8; i += 2) {
                 const float got = __shfl_xor_sync(0xffffffffu, odd ? v[i] : v[i + 1], 1);
@@ -263,7 +308,7 @@ __device__ __forceinline__ void to_operand(const Slice &s, uint8_t *next, uint32
     }
 }
 
-template <int ACT, bool BOTH, int AP, uint32_t EPI>
+template <int ACT, int ACC, int AP, uint32_t EPI>
 __device__ __forceinline__ void to_output(const ChainParams &p, const Slice &s)
 {
 #pragma unroll 1
@@ -275,7 +320,7 @@ __device__ __forceinline__ void to_output(const ChainParams &p, const Slice &s)
 #pragma unroll 1
         for (uint32_t c = 4 * s.g; c < s.n; c += 2 * EPI) {
             float v[8];
-            finish8<ACT, AP, BOTH>(s, taddr + c, c + EPI < s.n ? EPI : 0, bias, false, false, v);
+            finish8<ACT, AP, ACC>(s, taddr + c, c + EPI < s.n ? EPI : 0, bias, false, false, v);
 #pragma unroll
             for (int i = 0; i < 8; i++) {
                 const uint32_t r = c + (i & 3) + (i >> 2) * EPI, row = s.first + r;
@@ -295,7 +340,8 @@ template <int AP, uint32_t EPI> __device__ __forceinline__ void to_owners(const 
     for (uint32_t c = 4 * s.g; c < s.n; c += 2 * EPI) {
         const uint32_t more = c + EPI < s.n ? EPI : 0;
         float v[8];
-        sums8<AP, false>(s, s.tmem + c, more, false, false, v);                     // (by whole warps)
+        if (s.mains == 1) sums8<AP, 1>(s, s.tmem + c, more, false, false, v);         // (by whole warps)
+        else sums8<AP, MANY>(s, s.tmem + c, more, false, false, v);
         if (s.o < s.out) {
 #pragma unroll
             for (int i = 0; i < 8; i++) {
@@ -356,7 +402,7 @@ __device__ __forceinline__ void put_together(const ChainParams &p, int act, uint
             for (int i = 0; i < PER; i++) if ((uint32_t)i * 32 + lane < out) y[i * 32 + lane] = v[i] * inv;
         } else if (lane < out) {
 #define SPG_CHAIN_CALL(A, B) activate<A>(v, act)
-            SPG_CHAIN_ACTS(act, false, SPG_CHAIN_CALL)
+            SPG_CHAIN_ACTS(act, 1, SPG_CHAIN_CALL)
 #undef SPG_CHAIN_CALL
 #pragma unroll
             for (int i = 0; i < PER; i++) if ((uint32_t)i * 32 + lane < out) y[i * 32 + lane] = v[i];
@@ -524,12 +570,15 @@ spg_chain_kernel(const __grid_constant__ ChainParams p)
                 const bool cut = p.tail && l == last;
                 const uint32_t n = p.R, stages = cut ? (tail_k + KG * TK - 1) / (KG * TK) : p.l[l].stages, w_lo = p.l[l].tr * (128 >> 4), mains = p.l[l].mains;
                 const uint32_t idesc = p.idesc_base | ((AP * n >> 3) << 17), idesc_lo = p.idesc_base | ((n >> 3) << 17);
-                const uint32_t half = mains > 1 ? (stages + 1) / 2 : stages, from = l == 0 ? a_conv : a_full;
+                const uint32_t run = p.l[l].run, from = l == 0 ? a_conv : a_full, apart = run ? 0u : AP * n;      // (run 0: an accumulator a k-block)
+                uint32_t done_stages = 0, first = tmem;                    // of an accumulator, and where it is
                 uint32_t ph = l == 0 ? conv_ph : full_ph, steps = cut ? tail_k / 16 : (p.l[l].in + 15) / 16;      // of 16 values that are left
                 if (cut) { mbar_wait_uniform(own, own_ph, abort_addr, p.status, 72); own_ph ^= 1u; }
                 for (uint32_t st = 0; st < stages; st++) {
-                    const uint32_t fresh = st == 0 || st == half ? 0u : 1u;
-                    uint32_t d = tmem + (st >= half ? AP * n : 0u);
+                    if (apart) { done_stages = 0; if (st) first += KG * apart; }
+                    else if (done_stages == run) { done_stages = 0; first += AP * n; }
+                    const uint32_t fresh = done_stages++ ? 1u : 0u, fresh2 = apart ? 0u : 1u;
+                    uint32_t d = first;
                     const uint64_t da = smem_desc_sw128(base + a_off + (cut ? st : ra.slot) * a_slot);
                     if (!cut) {
                         mbar_wait_uniform(from + 8 * ra.slot, (ph >> ra.slot) & 1u, abort_addr, p.status, 62);
@@ -547,14 +596,14 @@ spg_chain_kernel(const __grid_constant__ ChainParams p)
 #pragma unroll
                                 for (uint32_t k = 0; k < KG * TK / 16; k++) {
                                     const uint32_t j = k / (TK / 16), i = 2 * (k % (TK / 16));
-                                    umma_f16(d, dw + j * w_next + i, da + j * a_next + i, idesc, k ? 1u : fresh);
-                                    if (WP > 1) umma_f16(d + n, dw + j * w_next + w_lo + i, da + j * a_next + i, idesc_lo, 1u);
+                                    umma_f16(d + j * apart, dw + j * w_next + i, da + j * a_next + i, idesc, k == 0 ? fresh : k == TK / 16 ? fresh2 : 1u);
+                                    if (WP > 1) umma_f16(d + j * apart + n, dw + j * w_next + w_lo + i, da + j * a_next + i, idesc_lo, 1u);
                                 }
                             } else {
                                 for (uint32_t k = 0; k < steps; k++) {
                                     const uint32_t j = k / (TK / 16), i = 2 * (k % (TK / 16));
-                                    umma_f16(d, dw + j * w_next + i, da + j * a_next + i, idesc, k ? 1u : fresh);
-                                    if (WP > 1) umma_f16(d + n, dw + j * w_next + w_lo + i, da + j * a_next + i, idesc_lo, 1u);
+                                    umma_f16(d + j * apart, dw + j * w_next + i, da + j * a_next + i, idesc, k == 0 ? fresh : k == TK / 16 ? fresh2 : 1u);
+                                    if (WP > 1) umma_f16(d + j * apart + n, dw + j * w_next + w_lo + i, da + j * a_next + i, idesc_lo, 1u);
                                 }
                             }
                             umma_commit(w_empty + 8 * rw.slot);
@@ -633,6 +682,7 @@ spg_chain_kernel(const __grid_constant__ ChainParams p)
                 s.tiles = share(l, o0); s.o = o0 + s.q * 32 + lane; s.tr = L.tr; s.n = p.R; s.mains = L.mains; s.out = L.out; s.act = L.act; s.scale = L.scale;
                 s.first = b * p.R; s.end = rows < (b + 1) * p.R ? rows : (b + 1) * p.R;
                 s.tmem = tmem + ((s.q * 32) << 16);
+                if (p.tail && l == last && s.mains > 1) s.mains = L.run ? ((tail_k + KG * TK - 1) / (KG * TK) + L.run - 1) / L.run : (tail_k + TK - 1) / TK;      // (those of its part of K)
                 const bool idle = s.tiles == 0;
 #pragma unroll
                 for (uint32_t t = 0; t < MAX_MT; t++) {
@@ -656,7 +706,7 @@ spg_chain_kernel(const __grid_constant__ ChainParams p)
                     if (idle) continue;
                     // (every copy into the activation ring has been used up: its memory holds the CTA's own outputs until they are multiplied)
 #define SPG_CHAIN_CALL(A, B) to_operand<A, B, T16, AP, EPI>(s, smem + a_off, o0, tail_k, p.R * 128)
-                    SPG_CHAIN_ACTS(s.act, s.mains > 1, SPG_CHAIN_CALL)
+                    SPG_CHAIN_ACTS(s.act, s.mains, SPG_CHAIN_CALL)
 #undef SPG_CHAIN_CALL
                     fence_async_smem();
                     tc_fence_before();
@@ -666,7 +716,7 @@ spg_chain_kernel(const __grid_constant__ ChainParams p)
                     const uint32_t next_k = p.l[l + 1].kblocks * TK, plane = p.R * 128;
                     uint8_t *next = p.scratch + (uint64_t)(2 * cluster + (e & 1u)) * p.exchange_bytes;
 #define SPG_CHAIN_CALL(A, B) to_operand<A, B, T16, AP, EPI>(s, next, 0, next_k, plane)
-                    SPG_CHAIN_ACTS(s.act, s.mains > 1, SPG_CHAIN_CALL)
+                    SPG_CHAIN_ACTS(s.act, s.mains, SPG_CHAIN_CALL)
 #undef SPG_CHAIN_CALL
                     // columns of the last k-block that no CTA's tiles reach
                     if (ok && me == 0 && L.covered < next_k) {
@@ -701,7 +751,7 @@ spg_chain_kernel(const __grid_constant__ ChainParams p)
                     if (b + clusters < blocks) epi_sync<EPI>();
                 } else {
 #define SPG_CHAIN_CALL(A, B) to_output<A, B, AP, EPI>(p, s)
-                    SPG_CHAIN_ACTS(s.act, s.mains > 1, SPG_CHAIN_CALL)
+                    SPG_CHAIN_ACTS(s.act, s.mains, SPG_CHAIN_CALL)
 #undef SPG_CHAIN_CALL
                     // The next block's first products take the place of these sums as soon as the first R / 8 warps have rounded a stage of its input:
                     // no warp begins with that before all of them have read theirs.
@@ -789,15 +839,17 @@ uint32_t epilogue_warps(const spgk_layer *layers, uint32_t count, uint32_t R, bo
     return 8;
 }
 
-// How a net's layers are laid out on clusters of C CTAs with blocks of R rows (false: they do not fit), and the cycles of a block.
+// How a net's layers are laid out on clusters of C CTAs with blocks of R rows (false: they do not fit), and the cycles of a block.  steps: products of K = 16
+// that an accumulator may add up one after the other, all layers together (0: any number).
 // The cycles come from a fit over 2037 arrangements of eight nets (40 to 12000 rows, every size of cluster, one to three products a term):
 // 5 to 95 % of them within 11 %, and the arrangement that it calls the fastest 2 % behind the fastest one on average.
-struct Layout { uint32_t epi, tr[MAX_LAYERS], mt[MAX_LAYERS], mains, SA, SW, a_slot, w_slot, tmem_cols, smem, tail, tail_rows, cycles; };
-bool lay_out(const spgk_layer *layers, uint32_t count, uint32_t C, uint32_t R, uint32_t a_parts, uint32_t w_parts, bool softmax, bool one_accumulator, size_t smem_max, Layout &o)
+struct Layout { uint32_t epi, tr[MAX_LAYERS], mt[MAX_LAYERS], mains[MAX_LAYERS], run[MAX_LAYERS], SA, SW, a_slot, w_slot, tmem_cols, smem, tail, tail_rows, cycles; };
+bool lay_out(const spgk_layer *layers, uint32_t count, uint32_t C, uint32_t R, uint32_t a_parts, uint32_t w_parts, bool softmax, bool counted, uint32_t steps,
+             size_t smem_max, Layout &o)
 {
     const uint32_t n = R * a_parts, rounds = ceil_div(R, 32), out = layers[count - 1].out;
     if (n > 256) return false;                                 // the widest product
-    uint32_t cols = 0, tr_max = 0, kb_max = 0;
+    uint32_t cols = 0, inputs[MAX_LAYERS], tr_max = 0, kb_max = 0;
     o.tail = out <= TAIL_MAX;
     o.epi = epilogue_warps(layers, count, R, o.tail != 0);
     if (softmax && !o.tail) return false;
@@ -813,6 +865,7 @@ bool lay_out(const spgk_layer *layers, uint32_t count, uint32_t C, uint32_t R, u
         if (o.mt[l] > MAX_MT) return false;
         if (round == 16) o.tail = ceil_div(L.out, o.mt[l] * o.tr[l]);
         if (o.mt[l] * n > cols) cols = o.mt[l] * n;
+        o.mains[l] = 1; o.run[l] = ceil_div(kb, KG); inputs[l] = in;
         if (o.tr[l] > tr_max) tr_max = o.tr[l];
         if (!cut && kb > kb_max) kb_max = kb;
         o.cycles += 2760 + ceil_div(in, 16) * o.mt[l] * product * 11 / 10;
@@ -820,9 +873,35 @@ bool lay_out(const spgk_layer *layers, uint32_t count, uint32_t C, uint32_t R, u
         else o.cycles += o.mt[l] * rounds * (L.act == SPG_ACT_TANH || L.act == SPG_ACT_SIGMOID ? 1960 : 1300) + (l ? R * kb * 128 * a_parts / 44 : 0);
     }
     if (cols > 512) return false;
-    // two accumulators where tensor memory has room: half as many additions in a row
-    o.mains = cols <= 256 && !one_accumulator ? 2 : 1;
-    cols *= o.mains;
+    // two accumulators where tensor memory has room: half as many additions in a row.  (Not where R may be another one in the next call.)
+    const auto stages_of = [&](uint32_t l) { return ceil_div(ceil_div(inputs[l], TK), KG); };
+    if (cols <= 256 && !counted) {
+        for (uint32_t l = 0; l + (o.tail ? 1 : 0) < count; l++) if (stages_of(l) > 1) { o.run[l] = (stages_of(l) + 1) / 2; o.mains[l] = 2; }
+        cols *= 2;
+    }
+    // more where the sums would be too long: for the layer with the longest ones that may have more, a k-block each at the most (run: 0)
+    const auto longest = [&](uint32_t l) { const uint32_t all = ceil_div(inputs[l], 16), one = o.run[l] ? o.run[l] * (KG * TK / 16) : TK / 16; return all < one ? all : one; };
+    for (;;) {
+        uint32_t total = 0, at = count, at_mains = 0, at_run = 0;
+        for (uint32_t l = 0; l < count; l++) {
+            total += longest(l);
+            uint32_t run = o.run[l], mains = o.mains[l];
+            if (run == 0 || (at < count && longest(l) <= longest(at))) continue;
+            while (mains <= o.mains[l] && run > 1) mains = ceil_div(stages_of(l), --run);
+            if (mains <= o.mains[l]) { run = 0; mains = ceil_div(inputs[l], TK); }
+            if (mains <= o.mains[l] || mains > MAX_ACC || (!counted && o.mt[l] * n * mains > 512)) continue;
+            at = l; at_mains = mains; at_run = run;
+        }
+        if (!steps || total <= steps) break;
+        if (at == count) return false;
+        o.mains[at] = at_mains; o.run[at] = at_run;
+    }
+    for (uint32_t l = 0; l < count; l++) {
+        const uint32_t took = o.mt[l] * n * o.mains[l];
+        if (took > cols) cols = took;
+        if (o.mains[l] > 2) o.cycles += o.mt[l] * rounds * (o.mains[l] - 2) * 250;
+    }
+    if (cols > 512) return false;
     for (o.tmem_cols = 32; o.tmem_cols < cols; o.tmem_cols <<= 1) { }
     o.a_slot = KG * R * 128 * a_parts; o.w_slot = KG * tr_max * 128 * w_parts;
     o.tail_rows = o.tail ? ceil_div(R, o.tail) : 0;
@@ -866,9 +945,9 @@ float layered_us(const spgk_layer *layers, uint32_t count, uint32_t N, uint32_t 
     return us;
 }
 
-// The cheapest arrangement for a number of rows (0: none): C, R and microseconds.  only: that size of cluster and one accumulator.
-float cheapest(const spgk_layer *layers, uint32_t count, uint32_t rows, uint32_t a_parts, uint32_t w_parts, bool softmax, uint32_t only, const AtOnce &at, const SpgDeviceProps &dp,
-               uint32_t &best_C, uint32_t &best_R)
+// The cheapest arrangement for a number of rows (0: none): C, R and microseconds.  only: that size of cluster, no more accumulators than `steps` asks for.
+float cheapest(const spgk_layer *layers, uint32_t count, uint32_t rows, uint32_t a_parts, uint32_t w_parts, bool softmax, uint32_t only, uint32_t steps, const AtOnce &at,
+               const SpgDeviceProps &dp, uint32_t &best_C, uint32_t &best_R)
 {
     uint64_t best = ~0ull;
     for (uint32_t C = only ? only : 1; C <= (only ? only : MAX_C); C++) {
@@ -877,7 +956,7 @@ float cheapest(const spgk_layer *layers, uint32_t count, uint32_t rows, uint32_t
         for (uint32_t waves = 1, tried = 0; waves <= 16 && tried < 3; waves++) {
             const uint32_t R = (ceil_div(rows, at.n[C] * waves) + 15) & ~15u;
             Layout o;
-            if (R > MAX_R || !lay_out(layers, count, C, R, a_parts, w_parts, softmax, only != 0, dp.smem_optin, o)) continue;
+            if (R > MAX_R || !lay_out(layers, count, C, R, a_parts, w_parts, softmax, only != 0, steps, dp.smem_optin, o)) continue;
             tried++;
             const uint32_t blocks = ceil_div(rows, R), busy = (blocks < at.n[C] ? blocks : at.n[C]) * C;
             // (on five eighths of the chip or less the next launch's first blocks get started beside this one's last)
@@ -887,6 +966,25 @@ float cheapest(const spgk_layer *layers, uint32_t count, uint32_t rows, uint32_t
         }
     }
     return best == ~0ull ? 0.0f : 3.2f + (float)best / 1965.0f;
+}
+
+// Products that may follow one another in the accumulators, all layers together: as many as in the layer kernels' (what a layer cuts off goes
+// through the ones behind it, so it is their sum that counts).  Those add the products of all terms to the same
+// one; of 8-bit terms and up to 1024 inputs a product's bits mostly fit the sum, and the second terms' are what is cut off: all are counted
+// there, only the first terms' beyond, and of 11-bit terms.  One term of a value loses more than sixteen sums do.
+// Not asked (0) of INT4 and INT2 files, whose products are short enough for the sums to hold nearly all of them.
+uint32_t steps_allowed(const spgk_layer *layers, uint32_t count, uint32_t N, uint32_t a_parts, uint32_t w_parts, bool softmax, const SpgDeviceProps &dp, int dev)
+{
+    const int prec = layers[0].precision;
+    if (prec == SPG_P_I4 || prec == SPG_P_I2) return 0;
+    const uint32_t passes = a_parts + w_parts - 1;
+    uint32_t total = 0;
+    for (uint32_t l = 0; l < count; l++) {
+        uint32_t steps = spg_gemm_steps(&layers[l], N, a_parts, w_parts, softmax && l + 1 == count, dp, dev);
+        if (prec == SPG_P_F16 || layers[l].in > 1024) steps /= passes;
+        total += passes == 1 && steps < 16 ? 16 : steps;
+    }
+    return total;
 }
 
 thread_local uint32_t tls_arrangement[2] = { 0, 0 };
@@ -910,12 +1008,18 @@ int spgk_chain_plan(const spgk_layer *layers, uint32_t count, uint32_t N, int w_
     // the net comes here and on clusters of which size, goes by 1024 rows whatever the guess.
     const bool counted = spg_tls_rows_limit != nullptr, softmax = softmax_fused != 0;
     const uint32_t a = (uint32_t)a_parts, w = (uint32_t)w_parts, rows = counted && N > 1024 ? 1024 : N;
-    plan->us = cheapest(layers, count, rows, a, w, softmax, counted ? COUNTED_C : 0, at, dp, plan->C, plan->R);
-    if (plan->us == 0.0f) return SPGK_E_UNSUPPORTED;
+    uint32_t steps = steps_allowed(layers, count, N, a, w, softmax, dp, dev);
     plan->layered_us = layered_us(layers, count, rows, (uint32_t)dp.sm_count, a, w);
+    plan->us = cheapest(layers, count, rows, a, w, softmax, counted ? COUNTED_C : 0, steps, at, dp, plan->C, plan->R);
+    if (plan->us == 0.0f && steps) {
+        steps = 0;
+        plan->layered_us = 0.0f;
+        plan->us = cheapest(layers, count, rows, a, w, softmax, counted ? COUNTED_C : 0, steps, at, dp, plan->C, plan->R);
+    }
+    if (plan->us == 0.0f) return SPGK_E_UNSUPPORTED;
     if (counted) {
         const uint32_t seen = spg_tls_rows_expected ? spg_tls_rows_expected : 1024, likely = seen + 3u * (uint32_t)sqrtf((float)seen);      // (what a selection by chance varies)
-        cheapest(layers, count, likely < N ? likely : N, a, w, softmax, COUNTED_C, at, dp, plan->C, plan->R);
+        cheapest(layers, count, likely < N ? likely : N, a, w, softmax, COUNTED_C, steps, at, dp, plan->C, plan->R);
     }
     const uint32_t blocks = ceil_div(N, plan->R);
     plan->clusters = blocks < at.n[plan->C] ? blocks : at.n[plan->C];
@@ -944,8 +1048,13 @@ int spgk_chain_forward(const spgk_chain *plan, const spgk_layer *layers, uint32_
     SpgDeviceProps dp;
     int rc = spg_device_props(&dp);
     if (rc) return rc;
+    int dev = 0;
+    SPGK_CUDA(cudaGetDevice(&dev));
     Layout o;
-    if (!lay_out(layers, count, plan->C, plan->R, (uint32_t)a_parts, (uint32_t)w_parts, softmax_fused != 0, spg_tls_rows_limit != nullptr, dp.smem_optin, o)) { spgk_set_error("spgk_chain_forward", "plan of another net"); return SPGK_E_ARG; }
+    const bool counted = spg_tls_rows_limit != nullptr;
+    const auto fits = [&](uint32_t steps) { return lay_out(layers, count, plan->C, plan->R, (uint32_t)a_parts, (uint32_t)w_parts, softmax_fused != 0, counted, steps, dp.smem_optin, o); };
+    // (as the plan was made: one that no arrangement with as many accumulators was found for has as few as there is room for)
+    if (!fits(steps_allowed(layers, count, N, (uint32_t)a_parts, (uint32_t)w_parts, softmax_fused != 0, dp, dev)) && !fits(0)) { spgk_set_error("spgk_chain_forward", "plan of another net"); return SPGK_E_ARG; }
     ChainParams p{};
     for (uint32_t l = 0; l < count; l++) {
         const spgk_layer &L = layers[l];
@@ -953,7 +1062,7 @@ int spgk_chain_forward(const spgk_chain *plan, const spgk_layer *layers, uint32_
         c.bias = L.bias; c.scale = L.w_scale; c.act = L.act == SPG_ACT_SOFTMAX ? SPG_ACT_NONE : L.act;
         c.in = L.in; c.out = L.out; c.kblocks = ceil_div(L.in, TK); c.stages = ceil_div(c.kblocks, KG);
         c.tr = o.tr[l]; c.mt = o.mt[l];
-        c.mains = c.stages > 1 && !(o.tail && l + 1 == count) ? o.mains : 1;
+        c.mains = o.mains[l]; c.run = o.run[l];
         c.covered = ceil_div(L.out, c.tr) * c.tr;
         if ((rc = spg_gemm_map(&p.w[l], w16[l], type16, L.in, L.out, ldw[l], w_plane[l], w_parts, c.tr, (uint32_t)w_parts))) return rc;
     }

@@ -27,5 +27,8 @@ int spg_gemm_map(CUtensorMap *map, const void *base, int type16, uint32_t K, uin
 // row counts above `served` (0: for all, nothing was launched).
 int spg_gemm_split_try(const SpgGemmArgs &a, const SpgDeviceProps &dp, int dev, uint32_t &served);
 
+// Products of K = 16 that a layer's accumulators add up one after the other, whichever kernel its product runs on
+uint32_t spg_gemm_steps(const spgk_layer *L, uint32_t N, uint32_t a_parts, uint32_t w_parts, bool softmax_fused, const SpgDeviceProps &dp, int dev);
+
 // spgk_selftest_impatient
 bool spg_gemm_impatient();

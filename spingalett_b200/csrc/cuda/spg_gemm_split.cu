@@ -344,6 +344,10 @@ int clusters_at_once(int dev, AtOnce &out)
     static SpgOncePerDevice once;
     static AtOnce known[SPG_MAX_DEVICES];
     const int rc = once.run(dev, [&]() -> int {
+        SpgDeviceProps dp;
+        const int prc = spg_device_props(&dp);
+        if (prc) return prc;
+        SPGK_CUDA(cudaFuncSetAttribute(spg_gemm_split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dp.smem_optin));
         for (int i = 0; i < 4; i++) {
             cudaLaunchConfig_t cfg = {};
             cfg.gridDim = dim3(1u << i); cfg.blockDim = dim3(THREADS); cfg.dynamicSmemBytes = 160 * 1024;
@@ -497,14 +501,9 @@ int spg_gemm_split_try(const SpgGemmArgs &a, const SpgDeviceProps &dp, int dev, 
 {
     served = 0;
     if (a.w_type16 != a.type16) return SPGK_E_UNSUPPORTED;
-    static SpgOncePerDevice once;
-    int rc = once.run(dev, [&]() -> int {
-        SPGK_CUDA(cudaFuncSetAttribute(spg_gemm_split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dp.smem_optin));
-        return SPGK_OK;
-    });
-    if (rc) return rc;
     AtOnce at;
-    if ((rc = clusters_at_once(dev, at))) return rc;
+    int rc = clusters_at_once(dev, at);
+    if (rc) return rc;
     const uint32_t N = a.L->out, kblocks = (a.L->in + TK - 1) / TK, a_parts = (uint32_t)a.a_parts, w_parts = (uint32_t)a.w_parts;
     const bool softmax = a.softmax_fused != 0;
     SplitPlan plan;
@@ -537,6 +536,33 @@ int spg_gemm_split_try(const SpgGemmArgs &a, const SpgDeviceProps &dp, int dev, 
     if (!softmax) return SPGK_E_UNSUPPORTED;
     if (!split_plan(at, rows, N, kblocks, a_parts, w_parts, true, 0, false, dp.smem_optin, plan)) return SPGK_E_UNSUPPORTED;
     return split_launch(a, at, plan, { limit, ~0u, ~0u });
+}
+
+// (asked for every layer of every call of some kernels: 1 us to find out, so the last few answers are kept, which hang on the arguments alone)
+uint32_t spg_gemm_steps(const spgk_layer *L, uint32_t rows, uint32_t a_parts, uint32_t w_parts, bool softmax_fused, const SpgDeviceProps &dp, int dev)
+{
+    const uint32_t N = L->out, kblocks = (L->in + TK - 1) / TK, passes = a_parts + w_parts - 1;
+    const auto steps = [&](uint32_t S) { return passes * ((kblocks + S - 1) / S) * (TK / 16); };
+    if (spg_tls_rows_limit) return steps(fixed_split(N, kblocks, (uint32_t)dp.sm_count));
+    struct Answer { int dev; uint32_t rows, N, kblocks, form, S; };
+    static thread_local Answer known[64];                       // S == 0: none yet
+    const uint32_t form = a_parts * 4 + w_parts * 2 + (softmax_fused ? 1 : 0);
+    Answer &k = known[(rows * 0x9E3779B1u ^ N * 0x85EBCA6Bu ^ kblocks * 0xC2B2AE35u ^ form * 0x27D4EB2Fu) >> 26];
+    if (!k.S || k.dev != dev || k.rows != rows || k.N != N || k.kblocks != kblocks || k.form != form) {
+        AtOnce at;
+        SplitPlan plan;
+        if (clusters_at_once(dev, at) != SPGK_OK) return steps(1);
+        k = { dev, rows, N, kblocks, form, split_plan(at, rows, N, kblocks, a_parts, w_parts, softmax_fused, -1, true, dp.smem_optin, plan) ? plan.S : 1 };
+    }
+    return steps(k.S);
+}
+
+extern "C" uint32_t spgk_layer_gemm_sum_steps(const spgk_layer *L, uint32_t N, int a_parts, int w_parts, int softmax_fused)
+{
+    SpgDeviceProps dp;
+    int dev = 0;
+    if (!L || a_parts < 1 || w_parts < 1 || spg_device_props(&dp) != SPGK_OK || cudaGetDevice(&dev) != cudaSuccess) return 0;
+    return spg_gemm_steps(L, N, (uint32_t)a_parts, (uint32_t)w_parts, softmax_fused != 0, dp, dev);
 }
 
 bool spg_gemm_impatient() { return spg_tls_impatient; }

@@ -580,6 +580,8 @@ int ws_map(const void *ptr, CUtensorMapDataType dt, uint32_t esize, uint64_t d0,
 
 extern "C" {
 
+uint32_t spgk_wstream_sum_steps(const spgk_layer *L, uint32_t N) { return ws_plan(L, N).kb_per_split * 4; }
+
 size_t spgk_wstream_scratch_bytes(const spgk_layer *L, uint32_t N)
 {
     WsPlan pl = ws_plan(L, N);

@@ -932,6 +932,32 @@ static bool fused_eligible(spg_net *n, const float *d_x, uint32_t N)
     return weights_keepable(n, fast_type(n), false);
 }
 
+/* What takes rows of a net of small operands that the 16-bit streaming kernel would take: the net in one launch where that is said to be the faster, or
+ * the layers one by one, as long as sums do not get longer by it (in one launch they are no longer than layer by layer, or than their inputs).  Of INT4 and
+ * INT2 the streaming kernel's sums hold everything, and so do those in one launch, since second terms have accumulators of their own there;
+ * the layer kernels' do not (256-4096-300 of positive values in INT4 at 33 rows: 1.3e-7 of the result lost, and 9e-7; 64-4096-64 2.9e-7 either way).  Sums half as
+ * long are asked of them (16384-512-64 in INT8: 256 products of both terms in a row 4.3e-6, 344 of one 3.6e-6). */
+typedef enum { LIGHT_STREAMED, LIGHT_LAYERS, LIGHT_WHOLE } LightRoute;
+static int light_route(spg_net *n, const float *d_x, uint32_t N, const float *d_out, spgk_chain *plan, LightRoute *route)
+{
+    bool takes;
+    const int rc = whole_plan(n, d_x, N, d_out, true, plan, &takes);
+    if (rc) return rc;
+    const PrecisionMode prec = n->klayers[0].precision;
+    bool whole = plan->clusters != 0, layers = prec != PRECISION_INT4 && prec != PRECISION_INT2;
+    for (uint32_t l = 0; l < n->dev_layers; l++) {
+        const spgk_layer *L = &n->klayers[l];
+        const int softmax = L->act == ACT_SOFTMAX && spgk_gemm_tc_softmax_fusable(L->out, N, 0);
+        const uint32_t streamed = spgk_wstream_sum_steps(L, N), layered = spgk_layer_gemm_sum_steps(L, N, 2, 1, softmax);
+        if (2 * layered > streamed) {
+            layers = false;
+            if ((L->in + 15u) / 16u > streamed) whole = false;
+        }
+    }
+    *route = whole && (takes || !layers) ? LIGHT_WHOLE : layers ? LIGHT_LAYERS : LIGHT_STREAMED;
+    return SPINGALETT_OK;
+}
+
 /* Nets that the chains take at any number of rows: every layer on the tensor cores, 16-bit operands well inside L2 */
 #define SPG_LIGHT_BYTES ((uint64_t)64 << 20)
 static bool light_operands(spg_net *n)
@@ -1310,7 +1336,11 @@ static float *forward_batch_on(spg_net *n, ForwardBatchArgs a)
     /* ... and at any number of rows when those operands are small: the streaming kernel's groups take 100 to 350 us (three layers of 2048: 137 us at
      * 33 rows, 264 at 96, against 27 on the chain; 784-512-1000-10 in bf16 114 and 240 against 13).  Like that kernel they then use two terms
      * in any mode. */
-    const bool light = N > SPGK_GEMV_MAX_BATCH && light_operands(n), light_exact = light && N <= 96 && all_wstream(n, N);
+    const bool small = N > SPGK_GEMV_MAX_BATCH && light_operands(n), light_exact = small && N <= 96 && !gemv_groups && all_wstream(n, N);
+    LightRoute route = LIGHT_LAYERS;
+    spgk_chain whole = { 0 };
+    if (light_exact && light_route(n, d_x, N, out_dev ? result : NULL, &whole, &route)) return NULL;
+    const bool light = small && route != LIGHT_STREAMED;
     const bool chain_kept = light || (N > 96 && weights_keepable(n, fast_type(n), false) && weights_keepable(n, SPGK_T_BF16, true));
     if (N <= SPGK_GEMV_MAX_BATCH || gemv_groups || (N <= 512 && !chain_kept && all_wstream(n, N < group ? N : group))) {
         for (uint32_t r0 = 0; r0 < N; r0 += group) {
@@ -1364,7 +1394,8 @@ static float *forward_batch_on(spg_net *n, ForwardBatchArgs a)
                     if (rc) return NULL;
                 }
             }
-        } else if (light_exact ? large_chain(n, d_x, N, d_out, true) : spg_dev_forward_large(n, d_x, N, d_out)) return NULL;
+        } else if (!light_exact ? spg_dev_forward_large(n, d_x, N, d_out)
+                   : route == LIGHT_WHOLE ? whole_net(n, &whole, d_x, N, d_out, true) : large_chain(n, d_x, N, d_out, true)) return NULL;
         if (!out_dev && spg_map_kernel_error(spgk_memcpy_d2h(result, d_out, out_bytes, n->stream), "forward_batch: output copy")) return NULL;
     }
     /* device-to-device calls are stream-ordered like any CUDA library call: the caller
