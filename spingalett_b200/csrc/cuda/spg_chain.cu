@@ -592,15 +592,15 @@ spg_chain_kernel(const __grid_constant__ ChainParams p)
                             // the high and the low terms of the rows lie one behind the other: one product for both, side by side in tensor
                             // memory; then hi*lo of the weights on top of the corrections (lo*lo is below fp32 resolution)
                             const uint32_t a_next = AP * n * (128 >> 4), w_next = WP * w_lo;          // the second k-block of a stage
-                            if (steps >= KG * TK / 16) {
+                            if (steps >= KG * TK / 16 && !apart) {
 #pragma unroll
                                 for (uint32_t k = 0; k < KG * TK / 16; k++) {
                                     const uint32_t j = k / (TK / 16), i = 2 * (k % (TK / 16));
-                                    umma_f16(d + j * apart, dw + j * w_next + i, da + j * a_next + i, idesc, k == 0 ? fresh : k == TK / 16 ? fresh2 : 1u);
-                                    if (WP > 1) umma_f16(d + j * apart + n, dw + j * w_next + w_lo + i, da + j * a_next + i, idesc_lo, 1u);
+                                    umma_f16(d, dw + j * w_next + i, da + j * a_next + i, idesc, k ? 1u : fresh);
+                                    if (WP > 1) umma_f16(d + n, dw + j * w_next + w_lo + i, da + j * a_next + i, idesc_lo, 1u);
                                 }
                             } else {
-                                for (uint32_t k = 0; k < steps; k++) {
+                                for (uint32_t k = 0; k < (steps < KG * TK / 16 ? steps : KG * TK / 16); k++) {
                                     const uint32_t j = k / (TK / 16), i = 2 * (k % (TK / 16));
                                     umma_f16(d + j * apart, dw + j * w_next + i, da + j * a_next + i, idesc, k == 0 ? fresh : k == TK / 16 ? fresh2 : 1u);
                                     if (WP > 1) umma_f16(d + j * apart + n, dw + j * w_next + w_lo + i, da + j * a_next + i, idesc_lo, 1u);
@@ -888,6 +888,7 @@ bool lay_out(const spgk_layer *layers, uint32_t count, uint32_t C, uint32_t R, u
             uint32_t run = o.run[l], mains = o.mains[l];
             if (run == 0 || (at < count && longest(l) <= longest(at))) continue;
             while (mains <= o.mains[l] && run > 1) mains = ceil_div(stages_of(l), --run);
+            if (run) run = ceil_div(stages_of(l), mains);       // (as even as they come)
             if (mains <= o.mains[l]) { run = 0; mains = ceil_div(inputs[l], TK); }
             if (mains <= o.mains[l] || mains > MAX_ACC || (!counted && o.mt[l] * n * mains > 512)) continue;
             at = l; at_mains = mains; at_run = run;
