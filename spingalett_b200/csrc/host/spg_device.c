@@ -423,7 +423,8 @@ static bool all_wstream(const spg_net *n, uint32_t N)
  *   3000-6000-2056-5000-304 in INT4 45 / 80 and 155 / 898; 8000-3000-10, 23 Mi, in INT2 at one row 27 / 25, at six 74 / 68).
  * - rows of odd lengths, loaded one by one: 3 Mi a layer (2001-1901-1803-1707-101 in INT4 at one row 37 / 43, at eight 125 / 424; INT4 in one layer of 4 million
  *   at four rows 24 / 23, at six 32 / 25); at two, three and eight rows 12 Mi in several layers (3001-6001-2051-5003-301 in INT8 131 / 272, 195 / 322 and
- *   392 / 948; at one row 76 / 62).  fp32: 3 Mi, at five to seven rows 2 Mi (three layers of 6.5 million 75 / 71, of 8.1 million 99 / 78; 98 / 254 at eight),
+ *   392 / 948; at one row 76 / 62; at four to six a fifth ahead at most, INT8 234 / 303, 307 / 355 and 312 / 355, INT4 237 / 252, 300 / 308
+ *   and 306 / 309, BF16 273 / 299, 334 / 359 and 339 / 361; at seven INT8 385 / 360, INT4 385 / 311, BF16 437 / 373).  fp32: 3 Mi, at five to seven rows 2 Mi (three layers of 6.5 million 75 / 71, of 8.1 million 99 / 78; 98 / 254 at eight),
  *   and at one and four no more than 8 Mi in all (the 2001-...-101 net 39 / 36 and 110 / 107). */
 #define SPG_ROWS_MAX_OUTPUTS 65535u                 /* of a layer of integers */
 
