@@ -28,8 +28,8 @@
 // second layer 17400, last layer's sums 20000, rows put together 23500 (with sixteen epilogue warps; eight save 1200); 2 us from the end to the next launch's first load.  With
 // more rows the epilogues' instructions weigh: 3001 rows of 301-777-333-129-37, clusters of 4 on 96 rows, spend half of the time there.
 //
-// Measured against layer by layer (us): 784-512-1000-10 at 256 rows 22.9 -> 13.7 (INT4), 22.0 -> 16.9 (fp32, three products a term), 1500 rows
-// 29 -> 20; 301-777-333-129-37 at 3001 rows 39.2 -> 32.1; 100-65-130-7 at 3000 rows 25.5 -> 13.4; 1024-256-256-256-10 at 12000 rows 76 -> 38;
+// Measured against layer by layer (us): 784-512-1000-10 at 256 rows 22.9 -> 13.9 (INT4), 22.0 -> 17.7 (fp32, three products a term), 1500 rows
+// 29 -> 20; 301-777-333-129-37 in FP16 at 3001 rows 39.2 -> 32.2; 100-65-130-7 at 3000 rows 25.5 -> 13.4; 1024-256-256-256-10 at 12000 rows 76 -> 38;
 // 128-128-128-128-128-128 at 256 rows 39 -> 14.  Against the 16-bit streaming kernel at 33 rows: 784-512-1000-10 in BF16 114 -> 12.
 // Tried: four rows a round of the epilogue instead of eight (560 cycles a round of four, eight little more), the input's loads ahead of the
 // fence that hands a tile on (the fence waits for them), one k-block a stage (waits and commits, 400 cycles a stage, twice as often).

@@ -21,7 +21,7 @@
 // Measured against the persistent kernel, a layer with two terms an activation (us): 256 rows 784 -> 512 19.3 -> 6.5 and
 // 1000 -> 10 11.6 -> 6.2; 1000 rows 784 -> 512 19.6 -> 8.8 and 2048 -> 2048 32.1 -> 23.7; 3000 rows 301 -> 777 14.7 -> 9.5 and
 // 777 -> 333 19.7 -> 10.2.  Whole nets of up to some thousand rows go through spg_chain.cu in one launch (784-512-1000-10 at 256 rows
-// 49.8 in the persistent kernel, 22.8 here, 13.7 there); this kernel has those that do not fit it, and larger ones' products of few tiles.
+// 49.8 in the persistent kernel, 22.8 here, 13.9 there); this kernel has those that do not fit it, and larger ones' products of few tiles.
 //
 // Every wait on an mbarrier is bounded as in spg_gemm_tc.cu; the cluster barriers are reached by every thread on every path, by
 // whole warps (they are of the aligned kind).  A wait that gave up in one CTA is known to its whole cluster before anybody finishes
